@@ -77,7 +77,11 @@ enum {
    * projection reads, replacing its transpose + contiguous copy
    * (qwen_lora_experiment/attention/common.py:575-596) -- instead of [B, Hq, N, 64].  num and den keep the
    * head-first layout.  bf16_tensorcore with at most 8 groups per head only. */
-  OAL_FLAG_OUT_TOKEN_MAJOR = 1
+  OAL_FLAG_OUT_TOKEN_MAJOR = 1,
+  /* the sequences start here (no state_in, no dstate_in in this call or its counterpart): the forward and the
+   * backward of a call, which must both carry the flag or both not, leave out the state work of the chunks that
+   * only meet a zero state */
+  OAL_FLAG_ZERO_STATE_IN = 2
 };
 
 typedef struct OalProblem {
@@ -152,6 +156,24 @@ int oal_backward(const OalProblem* problem, const void* q, const void* k, const 
                  size_t workspace_bytes, int32_t* status, void* stream);
 
 /*
+ * The same forward and backward for coefficients given as the packed factor (see oal_expand_factor for its layout),
+ * the form a training step has in hand: expansion, coefficient tables and factor gradient run inside the call's own
+ * kernels.  coefs: fp32 [q_heads * (1 + G + G * G)], written by the forward (A, then B, then C) and read by the
+ * backward.  status: two words, cleared by the call itself.  ticket (may be NULL: the status stays on the device):
+ * the last kernel also writes the word to pinned host memory, to be read with oal_status_poll; a ticket stays valid
+ * for the next 1023 such calls on its device.
+ */
+int oal_forward_packed(const OalProblem* problem, const void* q, const void* k, const void* v, const int32_t* dim_perm,
+                       const int32_t* group_start, const float* factor, int factor_rows, float kernel_eps, float* coefs,
+                       void* out, float* num, float* den, void* saved_state, void* workspace, size_t workspace_bytes,
+                       int32_t* status, int64_t* ticket, void* stream);
+int oal_backward_packed(const OalProblem* problem, const void* q, const void* k, const void* v, const int32_t* dim_perm,
+                        const int32_t* group_start, const float* factor, int factor_rows, const float* coefs,
+                        const float* num, const float* den, const void* saved_state, const void* grad_out,
+                        const float* grad_num, const float* grad_den, void* dq, void* dk, void* dv, float* d_factor,
+                        void* workspace, size_t workspace_bytes, int32_t* status, int64_t* ticket, void* stream);
+
+/*
  * Sequence parallelism (new; the reference is single-GPU, there is nothing to be compatible with).
  * A rank that owns a contiguous token range first computes the sum of its own chunk-state
  * increments, the ranks exchange these (one all-gather of batch*kv_heads*OAL_STATE_ROWS*OAL_E_PAD
@@ -181,7 +203,7 @@ int oal_backward_local_state(const OalProblem* problem, const void* q, const int
  * memory is frozen after start-up (serving processes with a pre-carved pool, plugins run from
  * allocator-free callbacks).
  *   Limits: batch * kv_heads * ceil(seq_len / 128) <= 16 and q_heads <= 64; larger problems return
- *   OAL_ERR_WORKSPACE.  The array (about 13.1 MB) is resident on every GPU that loads the library.
+ *   OAL_ERR_WORKSPACE.  The array (about 12.5 MB) is resident on every GPU that loads the library.
  *   The first call on each device resolves the array's device address; make that call outside any
  *   stream capture, with the device current.
  *   All calls on a device share the array and it keeps the previous call's contents; every element

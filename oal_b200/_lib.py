@@ -23,6 +23,7 @@ PRECISION_CODES = {"fp32_ieee": 0, "bf16_tensorcore": 1}
 GRAD_Q, GRAD_K, GRAD_V, GRAD_COEF, GRAD_REUSE_STATE_STAGE = 1, 2, 4, 8, 16
 STATE_ROWS = 2432
 FLAG_OUT_TOKEN_MAJOR = 1
+FLAG_ZERO_STATE_IN = 2
 STATUS_NONFINITE, STATUS_DENOMINATOR, STATUS_WAIT_TIMEOUT, STATUS_BAD_LAYOUT = 1, 2, 4, 8
 
 # every symbol include/oal_b200.h declares
@@ -30,6 +31,8 @@ EXPORTED_SYMBOLS = (
     "oal_workspace_bytes",
     "oal_forward",
     "oal_backward",
+    "oal_forward_packed",
+    "oal_backward_packed",
     "oal_last_error_string",
     "oal_version_string",
     "oal_selftest_umma",
@@ -71,6 +74,7 @@ class OalProblem(ctypes.Structure):
 
 
 _lib = None
+_host = None
 
 
 def load() -> ctypes.CDLL:
@@ -102,6 +106,13 @@ def load() -> ctypes.CDLL:
                                  f32p, vp, vp, vp, f32p, f32p, f32p, f32p, vp, ctypes.c_size_t, i32p, vp]
     lib.oal_backward.restype = ctypes.c_int
     ci = ctypes.c_int
+    i64p = ctypes.POINTER(ctypes.c_int64)
+    lib.oal_forward_packed.argtypes = [pp, vp, vp, vp, i32p, i32p, f32p, ci, ctypes.c_float, f32p, vp, f32p, f32p, vp, vp,
+                                       ctypes.c_size_t, i32p, i64p, vp]
+    lib.oal_forward_packed.restype = ctypes.c_int
+    lib.oal_backward_packed.argtypes = [pp, vp, vp, vp, i32p, i32p, f32p, ci, f32p, f32p, f32p, vp, vp, f32p, f32p, vp, vp,
+                                        vp, f32p, vp, ctypes.c_size_t, i32p, i64p, vp]
+    lib.oal_backward_packed.restype = ctypes.c_int
     lib.oal_rope_pack.argtypes = [vp, vp, vp, f32p, f32p, vp, vp, vp, ci, ci, ci, ci, vp]
     lib.oal_rope_pack.restype = ctypes.c_int
     lib.oal_rope_unpack_grad.argtypes = [vp, vp, vp, f32p, f32p, vp, vp, vp, ci, ci, ci, ci, vp]
@@ -131,6 +142,30 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+def host():
+    """The native host path (``_host.so``: autograd node, allocation and status queue of the prepared call)."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as module
+        except ImportError as exc:
+            raise RuntimeError(f"the native host path does not load ({exc}): build it with `python -m oal_b200.build`") from exc
+        _host = module
+    return _host
+
+
+class _NullGuard:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NULL_GUARD = _NullGuard()
+
+
 def ptr(t: torch.Tensor | None):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
@@ -141,6 +176,11 @@ def device_guard(t: torch.Tensor):
     The kernels launch on the calling thread's current device while the stream that is passed in
     belongs to the tensors' device; the reference is plain torch code and follows the tensors, so
     every entry into the library goes through this guard."""
+    if t.device.type != "cuda":
+        return _NULL_GUARD              # host-only work (argument checks on CPU tensors)
+    index = t.device.index
+    if index is not None and torch.cuda.is_initialized() and torch._C._cuda_getDevice() == index:
+        return _NULL_GUARD              # already current: nothing to set or to restore
     return torch.cuda.device(t.device)
 
 

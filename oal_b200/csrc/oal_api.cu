@@ -3,6 +3,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <chrono>
 #include <map>
 #include <mutex>
 #include <string>
@@ -10,6 +11,7 @@
 
 #include "oal_intra.cuh"
 #include "oal_kernels.h"
+#include "oal_prologue.cuh"
 
 namespace {
 
@@ -76,6 +78,59 @@ struct StatusRing {
 std::mutex g_status_mutex;
 StatusRing g_status[64];
 
+// ---- delivered status words -----------------------------------------------------------------------
+// A call that takes a ticket has its last kernel write the status word straight into a ring of pinned, mapped host
+// words: no copy, no event, nothing queued beside the call, and a waiting host sees it a microsecond after the
+// kernel has written it.
+constexpr int DELIVERY_RING = 1024;
+struct DeliveryRing {
+  int32_t* host = nullptr;
+  long long next = 0;
+};
+DeliveryRing g_delivery[64];
+constexpr int64_t TICKET_DELIVERED = (int64_t)1 << 62;
+
+// Spins on a delivered word; past the limit it lets the device drain once.  False: the word never came.
+bool wait_delivered(const int32_t* word, int dev) {
+  const volatile int32_t* w = word;
+  const auto t0 = std::chrono::steady_clock::now();
+  for (unsigned spin = 1;; ++spin) {
+    if (*w & oal::STATUS_DELIVERED) return true;
+    if ((spin & 1023) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) break;
+  }
+  int current = dev;
+  cudaGetDevice(&current);
+  if (current != dev) cudaSetDevice(dev);
+  cudaDeviceSynchronize();
+  if (current != dev) cudaSetDevice(current);
+  return (*w & oal::STATUS_DELIVERED) != 0;
+}
+
+// A fresh word of the current device's ring and its ticket.
+int take_delivery(int32_t** word, int64_t* ticket) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return fail_cuda(e, "status delivery");
+  if (dev < 0 || dev >= 64) return fail(OAL_ERR_ARGUMENT, "status delivery: device index out of range");
+  std::lock_guard<std::mutex> lock(g_status_mutex);
+  DeliveryRing& r = g_delivery[dev];
+  if (!r.host) {
+    e = cudaHostAlloc(reinterpret_cast<void**>(&r.host), DELIVERY_RING * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+      r.host = nullptr;
+      return fail_cuda(e, "status delivery");
+    }
+    for (int i = 0; i < DELIVERY_RING; ++i) r.host[i] = oal::STATUS_DELIVERED;
+  }
+  int32_t* slot = r.host + r.next % DELIVERY_RING;
+  if (!wait_delivered(slot, dev)) *slot = 0;      // its call, 1024 calls ago, died: the device reported that elsewhere
+  *static_cast<volatile int32_t*>(slot) = 0;
+  *word = slot;
+  *ticket = TICKET_DELIVERED | ((int64_t)dev << 48) | (int64_t)r.next;
+  ++r.next;
+  return OAL_OK;
+}
+
 // ---- side streams ------------------------------------------------------------------------------
 // Small kernels that nothing on the main chain waits for (the per-head factor table of the forward, the
 // coefficient-gradient reductions, the reverse state scan and the whole key/value chain of the backward)
@@ -89,14 +144,16 @@ struct SideStreams {
   cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
   bool ok = false;
 };
-std::mutex g_side_mutex;
+std::mutex g_side_mutex[64];
 SideStreams g_side[64];
 
-SideStreams* side_streams() {
+// `lock` is held while the call queues its forks and joins: an event that a second thread records again between a
+// record and the wait that belongs to it would order the wrong streams.
+SideStreams* side_streams(std::unique_lock<std::mutex>& lock) {
   if (!g_overlap.load()) return nullptr;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(g_side_mutex);
+  lock = std::unique_lock<std::mutex>(g_side_mutex[dev]);
   SideStreams& x = g_side[dev];
   if (!x.ok) {
     bool good = cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming) == cudaSuccess;
@@ -152,18 +209,48 @@ int check_problem(const OalProblem* p) {
     if (p->chunk != 128) return fail(OAL_ERR_ARGUMENT, "bf16_tensorcore requires chunk == 128");
   }
   if (!(p->floor > 0.f)) return fail(OAL_ERR_ARGUMENT, "floor must be positive");
-  if (p->flags & ~OAL_FLAG_OUT_TOKEN_MAJOR) return fail(OAL_ERR_ARGUMENT, "unknown bits in flags");
+  if (p->flags & ~(OAL_FLAG_OUT_TOKEN_MAJOR | OAL_FLAG_ZERO_STATE_IN)) return fail(OAL_ERR_ARGUMENT, "unknown bits in flags");
   if ((p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) &&
       (p->precision != OAL_PRECISION_BF16_TENSORCORE || p->groups + 1 > oal::intra_coef_terms()))
     return fail(OAL_ERR_ARGUMENT, "token-major out needs bf16_tensorcore and at most 8 groups per head");
   return OAL_OK;
 }
 
+// Where a call's coefficients come from: the packed factor (expanded on the device into A, B, C), or A, B, C.
+struct CoefSource {
+  const float* factor;      // null: A, B, C are inputs
+  int factor_rows;
+  float eps;
+  float *A, *B, *C;
+};
+
+CoefSource explicit_coefs(const float* a, const float* b, const float* c) {
+  return CoefSource{nullptr, 0, 0.f, const_cast<float*>(a), const_cast<float*>(b), const_cast<float*>(c)};
+}
+CoefSource packed_coefs(const OalProblem* p, const float* factor, int factor_rows, float eps, float* coefs) {
+  float* b = coefs + p->q_heads;
+  return CoefSource{factor, factor_rows, eps, coefs, b, b + (size_t)p->q_heads * p->groups};
+}
+
+// Gradient of the coefficients: dA, dB, dC, and the packed factor's when it was the source.
+struct CoefSink {
+  float *dA, *dB, *dC, *dfactor;
+};
+
+oal::PrologueArgs prologue_args(const OalProblem* p, const CoefSource& src, const int32_t* dim_perm, const int32_t* group_start,
+                                float* coef_table, void* factors, int32_t* status, int32_t* counter) {
+  return oal::PrologueArgs{src.factor, src.factor_rows, p->groups, src.eps, p->scale, dim_perm, group_start, src.A, src.B, src.C,
+                           coef_table, static_cast<oal::HeadFactor*>(factors), status, counter};
+}
+
 struct BackwardSpace {
   float* g;
   float* coef_pairs;
+  float* dcoefs;
   size_t bytes;
 };
+
+size_t coef_floats(const OalProblem* p) { return (size_t)p->q_heads * (1 + p->groups + p->groups * p->groups); }
 
 BackwardSpace carve_backward(const OalProblem* p, void* ws) {
   Carver c(ws);
@@ -171,6 +258,7 @@ BackwardSpace carve_backward(const OalProblem* p, void* ws) {
   const size_t rows = (size_t)p->batch * p->q_heads * p->seq_len;
   s.g = c.take<float>(rows * oal::EP);
   s.coef_pairs = c.take<float>((size_t)p->batch * p->q_heads * oal::pairs_tiles(p->seq_len) * oal::NCOEF);
+  s.dcoefs = c.take<float>(coef_floats(p));
   s.bytes = c.off;
   return s;
 }
@@ -179,8 +267,21 @@ constexpr int kChunk = 128;
 
 int chunk_count(const OalProblem* p) { return (p->seq_len + kChunk - 1) / kChunk; }
 
+// Chunks that meet a state.  Without a state from earlier tokens the first chunk of a sequence reads none and
+// nothing needs the increment of the last one, and the other way round in the backward: a share of 1 / chunks of
+// the state work, all of it for a sequence of one chunk.
+struct ChunkRange {
+  bool trim;
+  int n;         // chunks that read a state: the last n (forward), the first n (key side of the backward)
+  int first;     // first chunk that reads a carry
+};
+ChunkRange chunk_range(const OalProblem* p, const void* state_in, const void* dstate_in) {
+  const bool trim = (p->flags & OAL_FLAG_ZERO_STATE_IN) && !state_in && !dstate_in && !(p->grad_mask & OAL_GRAD_REUSE_STATE_STAGE);
+  const int nb = chunk_count(p);
+  return ChunkRange{trim, trim ? nb - 1 : nb, trim ? 1 : 0};
+}
+
 struct ForwardSpaceTC {
-  float* coef_table;
   float* ds;
   size_t bytes;
 };
@@ -200,7 +301,6 @@ ForwardSpaceTC carve_forward_tc(const OalProblem* p, void* ws) {
   Carver c(ws);
   ForwardSpaceTC s;
   const size_t units = (size_t)p->batch * p->kv_heads;
-  s.coef_table = c.take<float>((size_t)p->q_heads * oal::state_rows());
   s.ds = c.take<float>(units * chunk_count(p) * oal::state_rows() * oal::EP);
   s.bytes = c.off;
   return s;
@@ -208,24 +308,28 @@ ForwardSpaceTC carve_forward_tc(const OalProblem* p, void* ws) {
 
 // The buffer the forward hands to the backward: the bf16 carry images of every chunk (the MMA operand),
 // the images of their rounding remainders (read only by the coefficient-gradient dot products), then the
-// per-head factor table of the intra-chunk kernels (the backward of the same call sees the same
-// coefficients, so it does not factor them again).
+// per-head factor table of the intra-chunk kernels and the per-feature coefficient table of the state kernels
+// (the backward of the same call sees the same coefficients).
 size_t saved_images_bytes_tc(const OalProblem* p) {
   return align_up((size_t)p->batch * p->kv_heads * chunk_count(p) * oal::state_image_bytes_per_chunk());
 }
-size_t saved_state_bytes_tc(const OalProblem* p) { return 2 * saved_images_bytes_tc(p) + oal::head_factor_bytes(p->q_heads); }
-void* saved_remainders(const OalProblem* p, const void* saved_state) {
-  return const_cast<char*>(static_cast<const char*>(saved_state)) + saved_images_bytes_tc(p);
+size_t saved_factors_bytes_tc(const OalProblem* p) { return align_up(oal::head_factor_bytes(p->q_heads)); }
+size_t saved_state_bytes_tc(const OalProblem* p) {
+  return 2 * saved_images_bytes_tc(p) + saved_factors_bytes_tc(p) + align_up((size_t)p->q_heads * oal::state_rows() * sizeof(float));
 }
-void* saved_factors(const OalProblem* p, const void* saved_state) {
-  return const_cast<char*>(static_cast<const char*>(saved_state)) + 2 * saved_images_bytes_tc(p);
+char* saved_at(const void* saved_state, size_t offset) {
+  return const_cast<char*>(static_cast<const char*>(saved_state)) + offset;
+}
+void* saved_remainders(const OalProblem* p, const void* saved_state) { return saved_at(saved_state, saved_images_bytes_tc(p)); }
+void* saved_factors(const OalProblem* p, const void* saved_state) { return saved_at(saved_state, 2 * saved_images_bytes_tc(p)); }
+float* saved_coef_table(const OalProblem* p, const void* saved_state) {
+  return reinterpret_cast<float*>(saved_at(saved_state, 2 * saved_images_bytes_tc(p) + saved_factors_bytes_tc(p)));
 }
 
 struct BackwardSpaceTC {
   float* g;
   float* coef_pairs;
   void* gimg;
-  float* coef_table;
   float* dcarry;
   void* dt_img;
   float* dcoef_partial;
@@ -233,6 +337,7 @@ struct BackwardSpaceTC {
   float* slots;
   float *dq_cross, *dk_cross, *dv_cross;
   float *dk_part, *dv_part;      // per-query-head intra-chunk shares of dk / dv
+  float* dcoefs;                 // dA, dB, dC of a call whose caller asks for the factor's gradient
   size_t bytes;
 };
 
@@ -246,7 +351,6 @@ BackwardSpaceTC carve_backward_tc(const OalProblem* p, void* ws) {
   s.g = c.take<float>(qrows * oal::EP);
   s.coef_pairs = c.take<float>((size_t)p->batch * p->q_heads * oal::pairs_tiles(p->seq_len) * oal::NCOEF);
   s.gimg = c.take<char>(2 * (size_t)p->batch * p->q_heads * nb * slab_image);   // hi image, then lo image
-  s.coef_table = c.take<float>((size_t)p->q_heads * oal::state_rows());
   s.dcarry = c.take<float>(units * nb * oal::state_rows() * oal::EP);
   s.dt_img = c.take<char>(units * nb * oal::state_image_bytes_per_chunk());
   s.dcoef_partial = c.take<float>(2 * (size_t)p->batch * nb * p->q_heads * oal::state_rows());   // two column halves
@@ -257,44 +361,36 @@ BackwardSpaceTC carve_backward_tc(const OalProblem* p, void* ws) {
   s.dv_cross = c.take<float>(krows * oal::VD);
   s.dk_part = c.take<float>(qrows * oal::HD);
   s.dv_part = c.take<float>(qrows * oal::VD);
+  s.dcoefs = c.take<float>(coef_floats(p));
   s.bytes = c.off;
   return s;
 }
 
 // Stage A of the tensor-core backward: everything that does not depend on later tokens' state
-// gradient (normalisation VJP, coefficient table, per-chunk dCarry and coefficient partial sums).
-int backward_state_stage(const OalProblem* p, const void* q, const int32_t* dim_perm, const int32_t* group_start,
-                         const float* coef_a, const float* coef_b, const float* coef_c, const float* num,
-                         const float* den, const void* saved_state, const void* grad_out, const float* grad_num,
-                         const float* grad_den, const BackwardSpaceTC& s, int32_t* status, cudaStream_t st) {
-  const int nb = chunk_count(p);
-  const int mask = p->grad_mask;
-  const bool want_c = mask & OAL_GRAD_COEF;
-  cudaError_t e;
-  { LaunchScope scope("norm_vjp", st);
-    // the fp32 rows of g are read by the token-pair kernels only (heads with more than 8 groups)
-    e = oal::norm_vjp_image(grad_out, p->out_dtype, grad_num, grad_den, num, den, p->floor,
-                            tc_intra(p) ? nullptr : s.g, s.gimg,
-                            p->batch * p->q_heads, p->seq_len, nb,
-                            (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) ? p->q_heads : 0, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "normalisation VJP kernel");
-  { LaunchScope scope("coef_table", st);
-    e = oal::build_coef_table(dim_perm, group_start, coef_a, coef_b, coef_c, p->q_heads, p->groups, p->scale, s.coef_table, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
-  if (mask & (OAL_GRAD_K | OAL_GRAD_V | OAL_GRAD_COEF)) {
-    { LaunchScope scope("dstate_heads", st);
-      e = oal::dstate_heads(q, s.gimg, want_c ? saved_state : nullptr, want_c ? saved_remainders(p, saved_state) : nullptr,
-                            s.coef_table, s.dcarry,
-                            want_c ? s.dcoef_partial : nullptr, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb,
-                            p->scale, status, st); }
-    if (e != cudaSuccess) return fail_cuda(e, "state gradient kernel");
-  }
-  return OAL_OK;
+// gradient (normalisation VJP, per-chunk dCarry and coefficient partial sums).
+int backward_vjp(const OalProblem* p, const float* num, const float* den, const void* grad_out, const float* grad_num,
+                 const float* grad_den, const BackwardSpaceTC& s, int32_t* clear_status, cudaStream_t st) {
+  LaunchScope scope("norm_vjp", st);
+  // the fp32 rows of g are read by the token-pair kernels only (heads with more than 8 groups)
+  const cudaError_t e = oal::norm_vjp_image(grad_out, p->out_dtype, grad_num, grad_den, num, den, p->floor,
+                                            tc_intra(p) ? nullptr : s.g, s.gimg, p->batch * p->q_heads, p->seq_len, chunk_count(p),
+                                            (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) ? p->q_heads : 0, clear_status, st);
+  return e == cudaSuccess ? OAL_OK : fail_cuda(e, "normalisation VJP kernel");
+}
+int backward_dstate(const OalProblem* p, const void* q, const void* saved_state, const ChunkRange& cr, const BackwardSpaceTC& s,
+                    int32_t* status, cudaStream_t st) {
+  const bool want_c = p->grad_mask & OAL_GRAD_COEF;
+  if (!(p->grad_mask & (OAL_GRAD_K | OAL_GRAD_V | OAL_GRAD_COEF)) || cr.n == 0) return OAL_OK;
+  LaunchScope scope("dstate_heads", st);
+  const cudaError_t e = oal::dstate_heads(q, s.gimg, want_c ? saved_state : nullptr,
+                                          want_c ? saved_remainders(p, saved_state) : nullptr, saved_coef_table(p, saved_state),
+                                          s.dcarry, want_c ? s.dcoef_partial : nullptr, p->batch, p->q_heads, p->kv_heads,
+                                          p->seq_len, chunk_count(p), cr.first, cr.n, p->scale, status, st);
+  return e == cudaSuccess ? OAL_OK : fail_cuda(e, "state gradient kernel");
 }
 
 oal::PairArgs base_args(const OalProblem* p, const void* q, const void* k, const void* v,
-                        const int32_t* perm, const int32_t* gstart, const float* A, const float* B,
-                        const float* C, int32_t* status) {
+                        const int32_t* perm, const int32_t* gstart, const CoefSource& src, int32_t* status) {
   oal::PairArgs a;
   memset(&a, 0, sizeof(a));
   a.B = p->batch; a.Hq = p->q_heads; a.Hkv = p->kv_heads; a.N = p->seq_len; a.G = p->groups;
@@ -303,9 +399,255 @@ oal::PairArgs base_args(const OalProblem* p, const void* q, const void* k, const
   a.scale = p->scale; a.floor = p->floor;
   a.q = q; a.k = k; a.v = v;
   a.dim_perm = perm; a.group_start = gstart;
-  a.A = A; a.Bc = B; a.Cc = C;
+  a.A = src.A; a.Bc = src.B; a.Cc = src.C;
   a.status = status;
   return a;
+}
+
+// ---- forward ------------------------------------------------------------------------------------
+int forward_core(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
+                 const int32_t* group_start, const CoefSource& src, void* out, float* num, float* den, void* saved_state,
+                 const float* state_in, float* ds, int32_t* status, oal::StatusSink sink, bool timing, cudaStream_t st) {
+  cudaError_t e;
+  const bool tc_mode = p->precision == OAL_PRECISION_BF16_TENSORCORE, tc = tc_mode && tc_intra(p);
+  const int units = p->batch * p->kv_heads, nb = chunk_count(p);
+  const ChunkRange cr = chunk_range(p, state_in, nullptr);
+  const bool reuse = p->grad_mask & OAL_GRAD_REUSE_STATE_STAGE;      // increments left by oal_forward_local_state
+  const bool update = tc_mode && !reuse && cr.n > 0;
+  void* factors = tc ? saved_factors(p, saved_state) : nullptr;
+  float* coef_table = tc_mode ? saved_coef_table(p, saved_state) : nullptr;
+  std::unique_lock<std::mutex> side_lock;
+  SideStreams* side = nullptr;
+  cudaStream_t s0 = st;
+  oal::PrologueArgs pro{};
+  if (src.factor) {
+    pro = prologue_args(p, src, dim_perm, group_start, coef_table, factors, status, sink.host ? sink.counter : nullptr);
+    if (!update) {
+      LaunchScope scope("head_prologue", st, 1, timing);
+      if ((e = oal::launch_head_prologue(pro, p->q_heads, st)) != cudaSuccess) return fail_cuda(e, "prologue kernel");
+    }
+  } else if (tc_mode) {
+    // explicit coefficients: the factor table (rotations of a possibly indefinite matrix, 50 us) is needed by the
+    // last kernel only and is computed beside the state kernels
+    if (tc) {
+      if (timing) side = side_streams(side_lock);
+      s0 = fork_to(side, 0, st);
+      if (int rc = make_head_factors(p, dim_perm, group_start, src.A, src.B, src.C, factors, s0, timing)) return rc;
+      join_mark(side, 0, s0, st);
+    }
+    LaunchScope scope("coef_table", st, 1, timing);
+    e = oal::build_coef_table(dim_perm, group_start, src.A, src.B, src.C, p->q_heads, p->groups, p->scale, coef_table, st);
+    if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
+  }
+  if (update) {
+    LaunchScope scope("state_update", st, 1, timing);
+    e = oal::state_update(k, v, ds, units, p->seq_len, nb, cr.n, src.factor ? &pro : nullptr, p->q_heads, status, st);
+    if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
+  }
+  if (tc_mode && cr.n > 0) {
+    { LaunchScope scope("state_scan", st, 1, timing);
+      e = oal::state_scan(ds, saved_state, saved_remainders(p, saved_state), state_in, nullptr, units, nb, 0, cr.trim, st); }
+    if (e != cudaSuccess) return fail_cuda(e, "state scan kernel");
+    { LaunchScope scope("cross_read_q", st, 1, timing);
+      e = oal::cross_read(true, q, saved_state, coef_table, num, den, p->batch, p->q_heads, p->q_heads / p->kv_heads,
+                          p->seq_len, nb, cr.first, cr.n, status, st); }
+    if (e != cudaSuccess) return fail_cuda(e, "cross read kernel");
+  }
+  if (tc) {
+    join_wait(side, 0, s0, st);
+    LaunchScope scope("intra_forward", st, 1, timing);
+    e = oal::intra_forward(q, k, v, factors, out, num, den, status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb,
+                           p->out_dtype, p->floor, (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) != 0, cr.first, sink, st);
+    return e == cudaSuccess ? OAL_OK : fail_cuda(e, "intra-chunk forward kernel");
+  }
+  oal::PairArgs a = base_args(p, q, k, v, dim_perm, group_start, src, status);
+  a.window = tc_mode ? kChunk : 0;
+  a.out = out; a.num = num; a.den = den;
+  a.accumulate = tc_mode ? 1 : 0;
+  a.accumulate_from = cr.first * kChunk;
+  a.sink = sink;
+  LaunchScope scope("pairs_forward", st, 1, timing);
+  e = oal::pairs_forward(a, st);
+  return e == cudaSuccess ? OAL_OK : fail_cuda(e, "forward pair kernel");
+}
+
+// ---- backward -----------------------------------------------------------------------------------
+// sums of the coefficient partials -> dA, dB, dC, and on to the packed factor
+int finish_coefs(const OalProblem* p, const CoefSource& src, const CoefSink& sink, const float* partial, const float* slots,
+                 const void* factors, cudaStream_t st) {
+  cudaError_t e;
+  const bool fused = factors && sink.dfactor && src.factor_rows == p->q_heads;
+  { LaunchScope scope("reduce_coefs", st);
+    const int rm = oal::intra_coef_terms();
+    e = factors ? oal::intra_coef_finish(partial, chunk_count(p), rm * (rm + 1) / 2 + rm + 1, rm, factors, slots, p->batch,
+                                         p->q_heads, p->groups, sink.dA, sink.dB, sink.dC, fused ? src.factor : nullptr,
+                                         fused ? sink.dfactor : nullptr, st)
+                : oal::reduce_coefs(partial, oal::pairs_tiles(p->seq_len), slots, p->batch, p->q_heads, p->groups,
+                                    sink.dA, sink.dB, sink.dC, st); }
+  if (e != cudaSuccess) return fail_cuda(e, "coefficient reduction kernel");
+  if (sink.dfactor && !fused) {
+    LaunchScope scope("expand_factor_grad", st);
+    e = oal::expand_factor_grad(src.factor, src.factor_rows, p->q_heads, p->groups, sink.dA, sink.dB, sink.dC, sink.dfactor, st);
+    if (e != cudaSuccess) return fail_cuda(e, "factor gradient kernel");
+  }
+  return OAL_OK;
+}
+
+struct BackwardArgs {
+  const void *q, *k, *v;
+  const int32_t *dim_perm, *group_start;
+  const float *num, *den;
+  const void *saved_state, *grad_out;
+  const float *grad_num, *grad_den;
+  void *dq, *dk, *dv;
+  const float* dstate_in;
+  void* workspace;
+  size_t workspace_bytes;
+  int32_t* status;
+  bool clear_status;          // the first kernel zeroes the word
+};
+
+int backward_core_fp32(const OalProblem* p, const BackwardArgs& x, const CoefSource& src, CoefSink sink, cudaStream_t st) {
+  if (x.dstate_in) return fail(OAL_ERR_ARGUMENT, "fp32_ieee mode keeps no chunk state: dstate_in must be NULL");
+  BackwardSpace s = carve_backward(p, x.workspace);
+  if (!x.workspace || x.workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_backward: workspace too small");
+  const int mask = p->grad_mask;
+  if (sink.dfactor) {
+    sink.dA = s.dcoefs; sink.dB = sink.dA + p->q_heads; sink.dC = sink.dB + (size_t)p->q_heads * p->groups;
+  }
+  const size_t rows = (size_t)p->batch * p->q_heads * p->seq_len;
+  cudaError_t e;
+  { LaunchScope scope("norm_vjp", st);
+    e = oal::norm_vjp(x.grad_out, p->out_dtype, x.grad_num, x.grad_den, x.num, x.den, p->floor, s.g, rows,
+                      x.clear_status ? x.status : nullptr, st); }
+  if (e != cudaSuccess) return fail_cuda(e, "normalisation VJP kernel");
+  oal::PairArgs a = base_args(p, x.q, x.k, x.v, x.dim_perm, x.group_start, src, x.status);
+  a.g = s.g;
+  if (mask & (OAL_GRAD_Q | OAL_GRAD_COEF)) {
+    a.dq = (mask & OAL_GRAD_Q) ? x.dq : nullptr;
+    a.coef_partial = (mask & OAL_GRAD_COEF) ? s.coef_pairs : nullptr;
+    { LaunchScope scope("pairs_backward_q", st); e = oal::pairs_backward_q(a, st); }
+    if (e != cudaSuccess) return fail_cuda(e, "backward query-side pair kernel");
+    if (mask & OAL_GRAD_COEF)
+      if (int rc = finish_coefs(p, src, sink, s.coef_pairs, nullptr, nullptr, st)) return rc;
+  }
+  if (mask & (OAL_GRAD_K | OAL_GRAD_V)) {
+    a.dq = nullptr; a.coef_partial = nullptr;
+    a.dk = (mask & OAL_GRAD_K) ? x.dk : nullptr;
+    a.dv = (mask & OAL_GRAD_V) ? x.dv : nullptr;
+    { LaunchScope scope("pairs_backward_kv", st); e = oal::pairs_backward_kv(a, st); }
+    if (e != cudaSuccess) return fail_cuda(e, "backward key/value-side pair kernel");
+  }
+  return OAL_OK;
+}
+
+int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& src, CoefSink sink, cudaStream_t st) {
+  if (p->precision == OAL_PRECISION_FP32_IEEE) return backward_core_fp32(p, x, src, sink, st);
+  if (!x.saved_state) return fail(OAL_ERR_ARGUMENT, "oal_backward: saved_state is NULL");
+  BackwardSpaceTC s = carve_backward_tc(p, x.workspace);
+  if (!x.workspace || x.workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_backward: workspace too small");
+  if (sink.dfactor) {
+    sink.dA = s.dcoefs; sink.dB = sink.dA + p->q_heads; sink.dC = sink.dB + (size_t)p->q_heads * p->groups;
+  }
+  const int mask = p->grad_mask;
+  const int nb = chunk_count(p), units = p->batch * p->kv_heads, rep = p->q_heads / p->kv_heads;
+  const bool want_q = mask & OAL_GRAD_Q, want_k = mask & OAL_GRAD_K, want_v = mask & OAL_GRAD_V, want_kv = want_k || want_v;
+  const bool want_c = mask & OAL_GRAD_COEF;
+  const bool tc = tc_intra(p);                // intra-chunk term on the tensor cores (else token-pair kernels)
+  const bool reuse = mask & OAL_GRAD_REUSE_STATE_STAGE;
+  const ChunkRange cr = chunk_range(p, nullptr, x.dstate_in);
+  const void* factors = saved_factors(p, x.saved_state);      // written by the forward of this call
+  const float* coef_table = saved_coef_table(p, x.saved_state);
+  cudaError_t e;
+  if (!reuse) {
+    if (int rc = backward_vjp(p, x.num, x.den, x.grad_out, x.grad_num, x.grad_den, s, x.clear_status ? x.status : nullptr, st)) return rc;
+    if (int rc = backward_dstate(p, x.q, x.saved_state, cr, s, x.status, st)) return rc;
+  }
+  // Three chains leave the state stage: the query side (on the caller's stream), the key/value side and
+  // the reduction of the cross-chunk coefficient gradient.  They share no buffer, so the last two run on
+  // the library's side streams and are joined before this function returns.
+  std::unique_lock<std::mutex> side_lock;
+  SideStreams* side = side_streams(side_lock);
+  const bool cross = cr.n > 0;
+  cudaStream_t skv = want_kv ? fork_to(side, 0, st) : st;
+  cudaStream_t sc = want_c && cross ? fork_to(side, 1, st) : st;
+  oal::PairArgs a = base_args(p, x.q, x.k, x.v, x.dim_perm, x.group_start, src, x.status);
+  a.window = kChunk;
+  a.g = s.g;
+  a.q_init_from = cr.first * kChunk;
+  a.kv_init_end = cr.n * kChunk;
+  if (want_c && cross) {
+    { LaunchScope scope("dcoef_reduce", sc, 2);
+      e = oal::dcoef_reduce(s.dcoef_partial, 2 * p->batch * cr.n, p->q_heads, p->groups, x.dim_perm, x.group_start, s.dcoef, s.slots, sc); }
+    if (e != cudaSuccess) return fail_cuda(e, "coefficient gradient reduction kernels");
+    join_mark(side, 1, sc, st);
+  }
+  if (want_kv && cross) {
+    { LaunchScope scope("state_scan_reverse", skv);
+      e = oal::state_scan(s.dcarry, s.dt_img, nullptr, x.dstate_in, nullptr, units, nb, 1, cr.trim, skv); }
+    if (e != cudaSuccess) return fail_cuda(e, "reverse state scan kernel");
+    if (want_k) {
+      { LaunchScope scope("feature_grad_k", skv);
+        e = oal::feature_grad(false, x.k, nullptr, x.v, s.dt_img, nullptr, s.dk_cross, p->batch, p->kv_heads, 1,
+                              p->seq_len, nb, 0, cr.n, x.status, skv); }
+      if (e != cudaSuccess) return fail_cuda(e, "key feature gradient kernel");
+    }
+    if (want_v) {
+      { LaunchScope scope("cross_read_k", skv);
+        e = oal::cross_read(false, x.k, s.dt_img, nullptr, s.dv_cross, nullptr, p->batch, p->kv_heads, 1, p->seq_len,
+                            nb, 0, cr.n, x.status, skv); }
+      if (e != cudaSuccess) return fail_cuda(e, "key cross read kernel");
+    }
+  }
+  if (want_q && cross) {
+    { LaunchScope scope("feature_grad_q", st);
+      e = oal::feature_grad(true, x.q, s.gimg, nullptr, x.saved_state, coef_table, s.dq_cross, p->batch, p->q_heads,
+                            rep, p->seq_len, nb, cr.first, cr.n, x.status, st); }
+    if (e != cudaSuccess) return fail_cuda(e, "query feature gradient kernel");
+  }
+  if (want_q || want_c) {
+    if (tc) {
+      { LaunchScope scope("intra_backward_q", st);
+        e = oal::intra_backward_q(x.q, x.k, x.v, s.gimg, factors, want_q ? x.dq : nullptr, want_q ? s.dq_cross : nullptr,
+                                  want_c ? s.coef_pairs : nullptr, x.status, p->batch, p->q_heads, p->kv_heads,
+                                  p->seq_len, nb, cr.first, st); }
+      if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward query-side kernel");
+    } else {
+      a.dq = want_q ? x.dq : nullptr;
+      a.dq_init = want_q ? s.dq_cross : nullptr;
+      a.coef_partial = want_c ? s.coef_pairs : nullptr;
+      { LaunchScope scope("pairs_backward_q", st); e = oal::pairs_backward_q(a, st); }
+      if (e != cudaSuccess) return fail_cuda(e, "backward query-side pair kernel");
+    }
+  }
+  if (want_kv) {
+    // the two intra-chunk kernels each fill the machine: the key/value one is queued after the query one
+    if (tc) {
+      { LaunchScope scope("intra_backward_kv", skv);
+        e = oal::intra_backward_kv(x.q, x.k, x.v, s.gimg, factors, want_k ? s.dk_part : nullptr, want_v ? s.dv_part : nullptr,
+                                   x.status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb, skv); }
+      if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward key/value-side kernel");
+      { LaunchScope scope("kv_head_reduce", skv);
+        e = oal::kv_head_reduce(s.dk_part, s.dv_part, s.dk_cross, s.dv_cross, want_k ? x.dk : nullptr, want_v ? x.dv : nullptr,
+                                p->batch, p->q_heads, p->kv_heads, p->seq_len, cr.n * kChunk, skv); }
+      if (e != cudaSuccess) return fail_cuda(e, "key/value head reduction kernel");
+    } else {
+      a.dq = nullptr; a.dq_init = nullptr; a.coef_partial = nullptr;
+      a.dk = want_k ? x.dk : nullptr;
+      a.dv = want_v ? x.dv : nullptr;
+      a.dk_init = want_k ? s.dk_cross : nullptr;
+      a.dv_init = want_v ? s.dv_cross : nullptr;
+      { LaunchScope scope("pairs_backward_kv", skv); e = oal::pairs_backward_kv(a, skv); }
+      if (e != cudaSuccess) return fail_cuda(e, "backward key/value-side pair kernel");
+    }
+    join_mark(side, 0, skv, st);
+  }
+  if (want_c) {
+    if (cross) join_wait(side, 1, sc, st);
+    if (int rc = finish_coefs(p, src, sink, s.coef_pairs, cross ? s.slots : nullptr, tc ? factors : nullptr, st)) return rc;
+  }
+  if (want_kv) join_wait(side, 0, skv, st);
+  return OAL_OK;
 }
 
 }  // namespace
@@ -404,67 +746,104 @@ int64_t oal_workspace_bytes(const OalProblem* p, int phase) {
   return (int64_t)carve_backward_tc(p, nullptr).bytes;
 }
 
+static int forward_entry(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
+                         const int32_t* group_start, const CoefSource& src, void* out, float* num, float* den, void* saved_state,
+                         const float* state_in, void* workspace, size_t workspace_bytes, int32_t* status, oal::StatusSink sink,
+                         void* stream) {
+  if (!q || !k || !v || !dim_perm || !group_start || !src.A || !src.B || !src.C || !out || !num || !den || !status)
+    return fail(OAL_ERR_ARGUMENT, "oal_forward: NULL tensor pointer");
+  float* ds = nullptr;
+  if (p->precision == OAL_PRECISION_FP32_IEEE) {
+    if (state_in) return fail(OAL_ERR_ARGUMENT, "fp32_ieee mode keeps no chunk state: state_in must be NULL");
+  } else {
+    ForwardSpaceTC s = carve_forward_tc(p, workspace);
+    if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_forward: workspace too small");
+    if (!saved_state) return fail(OAL_ERR_ARGUMENT, "oal_forward: saved_state is NULL");
+    ds = s.ds;
+  }
+  return forward_core(p, q, k, v, dim_perm, group_start, src, out, num, den, saved_state, state_in, ds, status, sink, true,
+                      static_cast<cudaStream_t>(stream));
+}
+
 int oal_forward(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
                 const int32_t* group_start, const float* coef_a, const float* coef_b, const float* coef_c,
                 void* out, float* num, float* den, void* saved_state, const float* state_in,
                 void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
-  int rc = check_problem(p);
-  if (rc) return rc;
-  if (!q || !k || !v || !dim_perm || !group_start || !coef_a || !coef_b || !coef_c || !out || !num || !den || !status)
-    return fail(OAL_ERR_ARGUMENT, "oal_forward: NULL tensor pointer");
-  (void)saved_state; (void)workspace; (void)workspace_bytes;
+  if (int rc = check_problem(p)) return rc;
+  return forward_entry(p, q, k, v, dim_perm, group_start, explicit_coefs(coef_a, coef_b, coef_c), out, num, den, saved_state,
+                       state_in, workspace, workspace_bytes, status, oal::StatusSink{nullptr, nullptr}, stream);
+}
+
+int oal_forward_packed(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
+                       const int32_t* group_start, const float* factor, int factor_rows, float kernel_eps, float* coefs, void* out,
+                       float* num, float* den, void* saved_state, void* workspace, size_t workspace_bytes, int32_t* status,
+                       int64_t* ticket, void* stream) {
+  if (int rc = check_problem(p)) return rc;
+  if (!factor || !coefs) return fail(OAL_ERR_ARGUMENT, "oal_forward_packed: NULL pointer");
+  if (factor_rows != 1 && factor_rows != p->q_heads) return fail(OAL_ERR_ARGUMENT, "oal_forward_packed: factor_rows must be 1 or q_heads");
+  oal::StatusSink sink{nullptr, nullptr};
+  if (ticket) {
+    int32_t* word = nullptr;
+    if (int rc = take_delivery(&word, ticket)) return rc;
+    sink = oal::StatusSink{status + 1, word};
+  }
+  int rc = forward_entry(p, q, k, v, dim_perm, group_start, packed_coefs(p, factor, factor_rows, kernel_eps, coefs), out, num, den,
+                         saved_state, nullptr, workspace, workspace_bytes, status, sink, stream);
+  if (rc && sink.host) *sink.host = oal::STATUS_DELIVERED;      // nothing will write it
+  return rc;
+}
+
+int oal_backward(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
+                 const int32_t* group_start, const float* coef_a, const float* coef_b, const float* coef_c,
+                 const float* num, const float* den, const void* saved_state, const void* grad_out,
+                 const float* grad_num, const float* grad_den, void* dq, void* dk, void* dv,
+                 float* d_coef_a, float* d_coef_b, float* d_coef_c, const float* dstate_in, void* workspace,
+                 size_t workspace_bytes, int32_t* status, void* stream) {
+  if (int rc = check_problem(p)) return rc;
+  if (!q || !k || !v || !dim_perm || !group_start || !coef_a || !coef_b || !coef_c || !num || !den || !status)
+    return fail(OAL_ERR_ARGUMENT, "oal_backward: NULL tensor pointer");
+  const int mask = p->grad_mask;
+  if ((mask & OAL_GRAD_Q) && !dq) return fail(OAL_ERR_ARGUMENT, "dq requested but NULL");
+  if ((mask & OAL_GRAD_K) && !dk) return fail(OAL_ERR_ARGUMENT, "dk requested but NULL");
+  if ((mask & OAL_GRAD_V) && !dv) return fail(OAL_ERR_ARGUMENT, "dv requested but NULL");
+  if ((mask & OAL_GRAD_COEF) && (!d_coef_a || !d_coef_b || !d_coef_c))
+    return fail(OAL_ERR_ARGUMENT, "coefficient gradients requested but NULL");
+  BackwardArgs x{q, k, v, dim_perm, group_start, num, den, saved_state, grad_out, grad_num, grad_den, dq, dk, dv, dstate_in,
+                 workspace, workspace_bytes, status, false};
+  return backward_core(p, x, explicit_coefs(coef_a, coef_b, coef_c), CoefSink{d_coef_a, d_coef_b, d_coef_c, nullptr},
+                       static_cast<cudaStream_t>(stream));
+}
+
+int oal_backward_packed(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
+                        const int32_t* group_start, const float* factor, int factor_rows, const float* coefs, const float* num,
+                        const float* den, const void* saved_state, const void* grad_out, const float* grad_num,
+                        const float* grad_den, void* dq, void* dk, void* dv, float* d_factor, void* workspace,
+                        size_t workspace_bytes, int32_t* status, int64_t* ticket, void* stream) {
+  if (int rc = check_problem(p)) return rc;
+  if (!q || !k || !v || !dim_perm || !group_start || !factor || !coefs || !num || !den || !status)
+    return fail(OAL_ERR_ARGUMENT, "oal_backward_packed: NULL tensor pointer");
+  if (factor_rows != 1 && factor_rows != p->q_heads) return fail(OAL_ERR_ARGUMENT, "oal_backward_packed: factor_rows must be 1 or q_heads");
+  const int mask = p->grad_mask;
+  if (((mask & OAL_GRAD_Q) && !dq) || ((mask & OAL_GRAD_K) && !dk) || ((mask & OAL_GRAD_V) && !dv) || ((mask & OAL_GRAD_COEF) && !d_factor))
+    return fail(OAL_ERR_ARGUMENT, "oal_backward_packed: a requested gradient is NULL");
+  oal::StatusSink sink{nullptr, nullptr};
+  if (ticket) {
+    int32_t* word = nullptr;
+    if (int rc = take_delivery(&word, ticket)) return rc;
+    sink = oal::StatusSink{nullptr, word};
+  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (p->precision == OAL_PRECISION_FP32_IEEE) {
-    if (state_in) return fail(OAL_ERR_ARGUMENT, "fp32_ieee mode keeps no chunk state: state_in must be NULL");
-    oal::PairArgs a = base_args(p, q, k, v, dim_perm, group_start, coef_a, coef_b, coef_c, status);
-    a.out = out; a.num = num; a.den = den; a.accumulate = 0;
-    cudaError_t e;
-    { LaunchScope scope("pairs_forward", st); e = oal::pairs_forward(a, st); }
-    if (e != cudaSuccess) return fail_cuda(e, "forward pair kernel");
-    return OAL_OK;
+  BackwardArgs x{q, k, v, dim_perm, group_start, num, den, saved_state, grad_out, grad_num, grad_den, dq, dk, dv, nullptr,
+                 workspace, workspace_bytes, status, true};
+  CoefSource src = packed_coefs(p, factor, factor_rows, 0.f, const_cast<float*>(coefs));
+  int rc = backward_core(p, x, src, CoefSink{nullptr, nullptr, nullptr, (mask & OAL_GRAD_COEF) ? d_factor : nullptr}, st);
+  if (!rc && sink.host) {
+    LaunchScope scope("deliver_status", st);
+    const cudaError_t e = oal::deliver_status(status, sink, st);
+    if (e != cudaSuccess) rc = fail_cuda(e, "status delivery kernel");
   }
-  // bf16_tensorcore: chunk states on the tensor cores, intra-chunk term from token pairs
-  ForwardSpaceTC s = carve_forward_tc(p, workspace);
-  if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_forward: workspace too small");
-  if (!saved_state) return fail(OAL_ERR_ARGUMENT, "oal_forward: saved_state is NULL");
-  const int units = p->batch * p->kv_heads, nb = chunk_count(p);
-  cudaError_t e;
-  // the factor table is needed by the last kernel only: it is computed beside the state kernels
-  SideStreams* side = tc_intra(p) ? side_streams() : nullptr;
-  void* factors = saved_factors(p, saved_state);
-  cudaStream_t s0 = st;
-  if (tc_intra(p)) {
-    s0 = fork_to(side, 0, st);
-    if (int rc2 = make_head_factors(p, dim_perm, group_start, coef_a, coef_b, coef_c, factors, s0)) return rc2;
-    join_mark(side, 0, s0, st);
-  }
-  { LaunchScope scope("coef_table", st);
-    e = oal::build_coef_table(dim_perm, group_start, coef_a, coef_b, coef_c, p->q_heads, p->groups, p->scale, s.coef_table, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
-  if (!(p->grad_mask & OAL_GRAD_REUSE_STATE_STAGE)) {      // else: left in this workspace by oal_forward_local_state
-    { LaunchScope scope("state_update", st); e = oal::state_update(k, v, s.ds, units, p->seq_len, nb, status, st); }
-    if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
-  }
-  { LaunchScope scope("state_scan", st); e = oal::state_scan(s.ds, saved_state, saved_remainders(p, saved_state), state_in, nullptr, units, nb, 0, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "state scan kernel");
-  { LaunchScope scope("cross_read_q", st);
-    e = oal::cross_read(true, q, saved_state, s.coef_table, num, den, p->batch, p->q_heads,
-                        p->q_heads / p->kv_heads, p->seq_len, nb, status, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "cross read kernel");
-  if (tc_intra(p)) {
-    join_wait(side, 0, s0, st);
-    { LaunchScope scope("intra_forward", st);
-      e = oal::intra_forward(q, k, v, factors, out, num, den, status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb,
-                             p->out_dtype, p->floor, (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) != 0, st); }
-    if (e != cudaSuccess) return fail_cuda(e, "intra-chunk forward kernel");
-    return OAL_OK;
-  }
-  oal::PairArgs a = base_args(p, q, k, v, dim_perm, group_start, coef_a, coef_b, coef_c, status);
-  a.window = kChunk;
-  a.out = out; a.num = num; a.den = den; a.accumulate = 1;
-  { LaunchScope scope("pairs_forward", st); e = oal::pairs_forward(a, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "forward pair kernel");
-  return OAL_OK;
+  if (rc && sink.host) *sink.host = oal::STATUS_DELIVERED;
+  return rc;
 }
 
 void oal_set_overlap(int enable) { g_overlap.store(enable ? 1 : 0); }
@@ -503,8 +882,28 @@ int oal_status_defer(const int32_t* status, void* stream, int64_t* ticket) {
 
 int oal_status_poll(int64_t ticket, int block, int32_t* value) {
   if (!value) return fail(OAL_ERR_ARGUMENT, "oal_status_poll: NULL pointer");
-  const int dev = (int)(ticket >> 48);
+  const bool delivered = ticket & TICKET_DELIVERED;
+  const int dev = (int)((ticket & ~TICKET_DELIVERED) >> 48);
   const long long seq = (long long)(ticket & (((int64_t)1 << 48) - 1));
+  if (dev >= 0 && dev < 64 && delivered) {
+    const int32_t* word;
+    {
+      std::lock_guard<std::mutex> lock(g_status_mutex);
+      const DeliveryRing& r = g_delivery[dev];
+      if (seq >= r.next || seq + DELIVERY_RING <= r.next) return fail(OAL_ERR_ARGUMENT, "oal_status_poll: ticket expired or unknown");
+      word = r.host + seq % DELIVERY_RING;
+    }
+    if (block) {
+      if (!wait_delivered(word, dev)) {
+        const cudaError_t e = cudaGetLastError();
+        return e != cudaSuccess ? fail_cuda(e, "oal_status_poll") : fail(OAL_ERR_CUDA, "oal_status_poll: the call's status word was never written");
+      }
+    } else if (!(*static_cast<const volatile int32_t*>(word) & oal::STATUS_DELIVERED)) {
+      return 0;
+    }
+    *value = *static_cast<const volatile int32_t*>(word) & ~oal::STATUS_DELIVERED;
+    return 1;
+  }
   if (dev < 0 || dev >= 64) return fail(OAL_ERR_ARGUMENT, "oal_status_poll: bad ticket");
   cudaEvent_t done;
   int32_t* word;
@@ -550,158 +949,6 @@ int oal_expand_factor_grad(const float* factor, int factor_rows, int q_heads, in
   return e == cudaSuccess ? OAL_OK : fail_cuda(e, "oal_expand_factor_grad");
 }
 
-int oal_backward(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
-                 const int32_t* group_start, const float* coef_a, const float* coef_b, const float* coef_c,
-                 const float* num, const float* den, const void* saved_state, const void* grad_out,
-                 const float* grad_num, const float* grad_den, void* dq, void* dk, void* dv,
-                 float* d_coef_a, float* d_coef_b, float* d_coef_c, const float* dstate_in, void* workspace,
-                 size_t workspace_bytes, int32_t* status, void* stream) {
-  int rc = check_problem(p);
-  if (rc) return rc;
-  if (!q || !k || !v || !dim_perm || !group_start || !coef_a || !coef_b || !coef_c || !num || !den || !status)
-    return fail(OAL_ERR_ARGUMENT, "oal_backward: NULL tensor pointer");
-  const int mask = p->grad_mask;
-  if ((mask & OAL_GRAD_Q) && !dq) return fail(OAL_ERR_ARGUMENT, "dq requested but NULL");
-  if ((mask & OAL_GRAD_K) && !dk) return fail(OAL_ERR_ARGUMENT, "dk requested but NULL");
-  if ((mask & OAL_GRAD_V) && !dv) return fail(OAL_ERR_ARGUMENT, "dv requested but NULL");
-  if ((mask & OAL_GRAD_COEF) && (!d_coef_a || !d_coef_b || !d_coef_c))
-    return fail(OAL_ERR_ARGUMENT, "coefficient gradients requested but NULL");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (p->precision == OAL_PRECISION_FP32_IEEE) {
-    if (dstate_in) return fail(OAL_ERR_ARGUMENT, "fp32_ieee mode keeps no chunk state: dstate_in must be NULL");
-    BackwardSpace s = carve_backward(p, workspace);
-    if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_backward: workspace too small");
-    const size_t rows = (size_t)p->batch * p->q_heads * p->seq_len;
-    cudaError_t e;
-    { LaunchScope scope("norm_vjp", st);
-      e = oal::norm_vjp(grad_out, p->out_dtype, grad_num, grad_den, num, den, p->floor, s.g, rows, st); }
-    if (e != cudaSuccess) return fail_cuda(e, "normalisation VJP kernel");
-    oal::PairArgs a = base_args(p, q, k, v, dim_perm, group_start, coef_a, coef_b, coef_c, status);
-    a.g = s.g;
-    if (mask & (OAL_GRAD_Q | OAL_GRAD_COEF)) {
-      a.dq = (mask & OAL_GRAD_Q) ? dq : nullptr;
-      a.coef_partial = (mask & OAL_GRAD_COEF) ? s.coef_pairs : nullptr;
-      { LaunchScope scope("pairs_backward_q", st); e = oal::pairs_backward_q(a, st); }
-      if (e != cudaSuccess) return fail_cuda(e, "backward query-side pair kernel");
-      if (mask & OAL_GRAD_COEF) {
-        { LaunchScope scope("reduce_coefs", st);
-          e = oal::reduce_coefs(s.coef_pairs, oal::pairs_tiles(p->seq_len), nullptr, p->batch, p->q_heads,
-                                p->groups, d_coef_a, d_coef_b, d_coef_c, st); }
-        if (e != cudaSuccess) return fail_cuda(e, "coefficient reduction kernel");
-      }
-    }
-    if (mask & (OAL_GRAD_K | OAL_GRAD_V)) {
-      a.dq = nullptr; a.coef_partial = nullptr;
-      a.dk = (mask & OAL_GRAD_K) ? dk : nullptr;
-      a.dv = (mask & OAL_GRAD_V) ? dv : nullptr;
-      { LaunchScope scope("pairs_backward_kv", st); e = oal::pairs_backward_kv(a, st); }
-      if (e != cudaSuccess) return fail_cuda(e, "backward key/value-side pair kernel");
-    }
-    return OAL_OK;
-  }
-  // bf16_tensorcore
-  if (!saved_state) return fail(OAL_ERR_ARGUMENT, "oal_backward: saved_state is NULL");
-  BackwardSpaceTC s = carve_backward_tc(p, workspace);
-  if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_backward: workspace too small");
-  const int nb = chunk_count(p), units = p->batch * p->kv_heads, rep = p->q_heads / p->kv_heads;
-  const bool want_q = mask & OAL_GRAD_Q, want_k = mask & OAL_GRAD_K, want_v = mask & OAL_GRAD_V;
-  const bool want_c = mask & OAL_GRAD_COEF;
-  const bool tc = tc_intra(p);                // intra-chunk term on the tensor cores (else token-pair kernels)
-  cudaError_t e;
-  if (!(mask & OAL_GRAD_REUSE_STATE_STAGE)) {
-    rc = backward_state_stage(p, q, dim_perm, group_start, coef_a, coef_b, coef_c, num, den, saved_state, grad_out,
-                              grad_num, grad_den, s, status, st);
-    if (rc) return rc;
-  }
-  const void* factors = saved_factors(p, saved_state);      // written by the forward of this call
-  // Three chains leave the state stage: the query side (on the caller's stream), the key/value side and
-  // the reduction of the cross-chunk coefficient gradient.  They share no buffer, so the last two run on
-  // the library's side streams and are joined before this function returns.
-  SideStreams* side = side_streams();
-  cudaStream_t skv = (want_k || want_v) ? fork_to(side, 0, st) : st;
-  cudaStream_t sc = want_c ? fork_to(side, 1, st) : st;
-  oal::PairArgs a = base_args(p, q, k, v, dim_perm, group_start, coef_a, coef_b, coef_c, status);
-  a.window = kChunk;
-  a.g = s.g;
-  if (want_c) {
-    { LaunchScope scope("dcoef_reduce", sc, 2);
-      e = oal::dcoef_reduce(s.dcoef_partial, 2 * p->batch * nb, p->q_heads, dim_perm, group_start, s.dcoef, s.slots, sc); }
-    if (e != cudaSuccess) return fail_cuda(e, "coefficient gradient reduction kernels");
-    join_mark(side, 1, sc, st);
-  }
-  if (want_k || want_v) {
-    { LaunchScope scope("state_scan_reverse", skv);
-      e = oal::state_scan(s.dcarry, s.dt_img, nullptr, dstate_in, nullptr, units, nb, 1, skv); }
-    if (e != cudaSuccess) return fail_cuda(e, "reverse state scan kernel");
-    if (want_k) {
-      { LaunchScope scope("feature_grad_k", skv);
-        e = oal::feature_grad(false, k, nullptr, v, s.dt_img, nullptr, s.dk_cross, p->batch, p->kv_heads, 1,
-                              p->seq_len, nb, status, skv); }
-      if (e != cudaSuccess) return fail_cuda(e, "key feature gradient kernel");
-    }
-    if (want_v) {
-      { LaunchScope scope("cross_read_k", skv);
-        e = oal::cross_read(false, k, s.dt_img, nullptr, s.dv_cross, nullptr, p->batch, p->kv_heads, 1, p->seq_len,
-                            nb, status, skv); }
-      if (e != cudaSuccess) return fail_cuda(e, "key cross read kernel");
-    }
-  }
-  if (want_q || want_c) {
-    if (want_q) {
-      { LaunchScope scope("feature_grad_q", st);
-        e = oal::feature_grad(true, q, s.gimg, nullptr, saved_state, s.coef_table, s.dq_cross, p->batch, p->q_heads,
-                              rep, p->seq_len, nb, status, st); }
-      if (e != cudaSuccess) return fail_cuda(e, "query feature gradient kernel");
-    }
-    if (tc) {
-      { LaunchScope scope("intra_backward_q", st);
-        e = oal::intra_backward_q(q, k, v, s.gimg, factors, want_q ? dq : nullptr, want_q ? s.dq_cross : nullptr,
-                                  want_c ? s.coef_pairs : nullptr, status, p->batch, p->q_heads, p->kv_heads,
-                                  p->seq_len, nb, st); }
-      if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward query-side kernel");
-    } else {
-      a.dq = want_q ? dq : nullptr;
-      a.dq_init = want_q ? s.dq_cross : nullptr;
-      a.coef_partial = want_c ? s.coef_pairs : nullptr;
-      { LaunchScope scope("pairs_backward_q", st); e = oal::pairs_backward_q(a, st); }
-      if (e != cudaSuccess) return fail_cuda(e, "backward query-side pair kernel");
-    }
-    if (want_c) {
-      join_wait(side, 1, sc, st);
-      { LaunchScope scope("reduce_coefs", st);
-        const int rm = oal::intra_coef_terms();
-        e = tc ? oal::intra_coef_finish(s.coef_pairs, nb, rm * (rm + 1) / 2 + rm + 1, rm, factors, s.slots, p->batch,
-                                        p->q_heads, p->groups, d_coef_a, d_coef_b, d_coef_c, st)
-               : oal::reduce_coefs(s.coef_pairs, oal::pairs_tiles(p->seq_len), s.slots, p->batch, p->q_heads,
-                                   p->groups, d_coef_a, d_coef_b, d_coef_c, st); }
-      if (e != cudaSuccess) return fail_cuda(e, "coefficient reduction kernel");
-    }
-  } else if (want_c) {
-    join_wait(side, 1, sc, st);
-  }
-  if (want_k || want_v) {
-    // the two intra-chunk kernels each fill the machine: the key/value one is queued after the query one
-    if (tc) {
-      { LaunchScope scope("intra_backward_kv", skv, 1 + (want_k ? 1 : 0) + (want_v ? 1 : 0));
-        e = oal::intra_backward_kv(q, k, v, s.gimg, factors, want_k ? dk : nullptr, want_v ? dv : nullptr,
-                                   want_k ? s.dk_cross : nullptr, want_v ? s.dv_cross : nullptr, s.dk_part, s.dv_part,
-                                   status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb, skv); }
-      if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward key/value-side kernel");
-    } else {
-      a.dq = nullptr; a.dq_init = nullptr; a.coef_partial = nullptr;
-      a.dk = want_k ? dk : nullptr;
-      a.dv = want_v ? dv : nullptr;
-      a.dk_init = want_k ? s.dk_cross : nullptr;
-      a.dv_init = want_v ? s.dv_cross : nullptr;
-      { LaunchScope scope("pairs_backward_kv", skv); e = oal::pairs_backward_kv(a, skv); }
-      if (e != cudaSuccess) return fail_cuda(e, "backward key/value-side pair kernel");
-    }
-    join_mark(side, 0, skv, st);
-    join_wait(side, 0, skv, st);
-  }
-  return OAL_OK;
-}
-
 int oal_forward_local_state(const OalProblem* p, const void* k, const void* v, float* state_total, void* workspace,
                             size_t workspace_bytes, int32_t* status, void* stream) {
   int rc = check_problem(p);
@@ -714,9 +961,9 @@ int oal_forward_local_state(const OalProblem* p, const void* k, const void* v, f
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int units = p->batch * p->kv_heads, nb = chunk_count(p);
   cudaError_t e;
-  { LaunchScope scope("state_update", st); e = oal::state_update(k, v, s.ds, units, p->seq_len, nb, status, st); }
+  { LaunchScope scope("state_update", st); e = oal::state_update(k, v, s.ds, units, p->seq_len, nb, nb, nullptr, 0, status, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
-  { LaunchScope scope("state_total", st); e = oal::state_scan(s.ds, nullptr, nullptr, nullptr, state_total, units, nb, 0, st); }
+  { LaunchScope scope("state_total", st); e = oal::state_scan(s.ds, nullptr, nullptr, nullptr, state_total, units, nb, 0, false, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state total kernel");
   return OAL_OK;
 }
@@ -737,12 +984,11 @@ int oal_backward_local_state(const OalProblem* p, const void* q, const int32_t* 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   OalProblem local = *p;
   local.grad_mask |= OAL_GRAD_K;      // dCarry is needed whatever the caller finally asks for
-  rc = backward_state_stage(&local, q, dim_perm, group_start, coef_a, coef_b, coef_c, num, den, saved_state, grad_out,
-                            grad_num, grad_den, s, status, st);
-  if (rc) return rc;
+  if ((rc = backward_vjp(&local, num, den, grad_out, grad_num, grad_den, s, nullptr, st))) return rc;
+  if ((rc = backward_dstate(&local, q, saved_state, ChunkRange{false, chunk_count(p), 0}, s, status, st))) return rc;
   cudaError_t e;
   { LaunchScope scope("state_total", st);
-    e = oal::state_scan(s.dcarry, nullptr, nullptr, nullptr, dstate_total, p->batch * p->kv_heads, chunk_count(p), 1, st); }
+    e = oal::state_scan(s.dcarry, nullptr, nullptr, nullptr, dstate_total, p->batch * p->kv_heads, chunk_count(p), 1, false, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state gradient total kernel");
   return OAL_OK;
 }
@@ -753,17 +999,16 @@ int oal_backward_local_state(const OalProblem* p, const void* q, const int32_t* 
 // Some hosts of this library cannot obtain device memory at call time: an inference server whose
 // memory pool was carved up and frozen at start-up, a plugin that runs inside someone else's
 // allocator-free execution callback, a process near its memory limit where cudaMalloc may fail or
-// stall.  For them the tensor-core forward keeps its two scratch buffers -- the per-head coefficient
-// table and the per-chunk state increments -- in the file-scope device array below.  The array has
+// stall.  For them the tensor-core forward keeps its scratch buffer -- the per-chunk
+// state increments -- in the file-scope device array below.  The array has
 // a fixed size, so the entry point only accepts problems up to kStaticMaxUnitChunks (batch x KV heads
 // x 128-token chunks) and kStaticMaxHeads query heads; every GPU that loads the library holds the
-// array (about 13.1 MB) until the process exits.
+// array (about 12.5 MB) until the process exits.
 // ---------------------------------------------------------------------------------------------
 constexpr int kStaticMaxUnitChunks = 16;
 constexpr int kStaticMaxHeads = 64;
 constexpr size_t kStaticStateFloats = (size_t)kStaticMaxUnitChunks * OAL_STATE_ROWS * OAL_E_PAD;
-constexpr size_t kStaticTableFloats = (size_t)kStaticMaxHeads * OAL_STATE_ROWS;
-static __device__ __align__(256) float g_static_scratch[kStaticTableFloats + kStaticStateFloats];
+static __device__ __align__(256) float g_static_scratch[kStaticStateFloats];
 
 namespace {
 constexpr int kMaxDevices = 64;
@@ -807,36 +1052,8 @@ int oal_forward_static_scratch(const OalProblem* p, const void* q, const void* k
   float* scratch = nullptr;
   rc = static_scratch_address(&scratch);
   if (rc) return rc;
-  float* coef_table = scratch;
-  float* ds = scratch + kStaticTableFloats;
-  void* factors = saved_factors(p, saved_state);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e;
-  { LaunchScope scope("coef_table", st, 1, false);
-    e = oal::build_coef_table(dim_perm, group_start, coef_a, coef_b, coef_c, p->q_heads, p->groups, p->scale, coef_table, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
-  { LaunchScope scope("state_update", st, 1, false); e = oal::state_update(k, v, ds, units, p->seq_len, nb, status, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
-  { LaunchScope scope("state_scan", st, 1, false); e = oal::state_scan(ds, saved_state, saved_remainders(p, saved_state), nullptr, nullptr, units, nb, 0, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "state scan kernel");
-  { LaunchScope scope("cross_read_q", st, 1, false);
-    e = oal::cross_read(true, q, saved_state, coef_table, num, den, p->batch, p->q_heads, p->q_heads / p->kv_heads,
-                        p->seq_len, nb, status, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "cross read kernel");
-  if (tc_intra(p)) {
-    if (int rc2 = make_head_factors(p, dim_perm, group_start, coef_a, coef_b, coef_c, factors, st, false)) return rc2;
-    { LaunchScope scope("intra_forward", st, 1, false);
-      e = oal::intra_forward(q, k, v, factors, out, num, den, status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb,
-                             p->out_dtype, p->floor, (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) != 0, st); }
-    if (e != cudaSuccess) return fail_cuda(e, "intra-chunk forward kernel");
-    return OAL_OK;
-  }
-  oal::PairArgs a = base_args(p, q, k, v, dim_perm, group_start, coef_a, coef_b, coef_c, status);
-  a.window = kChunk;
-  a.out = out; a.num = num; a.den = den; a.accumulate = 1;
-  { LaunchScope scope("pairs_forward", st, 1, false); e = oal::pairs_forward(a, st); }
-  if (e != cudaSuccess) return fail_cuda(e, "forward pair kernel");
-  return OAL_OK;
+  return forward_core(p, q, k, v, dim_perm, group_start, explicit_coefs(coef_a, coef_b, coef_c), out, num, den, saved_state,
+                      nullptr, scratch, status, oal::StatusSink{nullptr, nullptr}, false, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

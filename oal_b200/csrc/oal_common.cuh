@@ -6,7 +6,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/oal_b200.h"
+#include "oal_kernels.h"
 
 namespace oal {
 
@@ -68,6 +71,45 @@ __device__ __forceinline__ void load_head_groups(HeadGroups& hg, const int32_t* 
     while (g < GMAX - 1 && x >= hg.start[g + 1]) ++g;
     hg.group_of[x] = g;
   }
+}
+
+// End of a block of a call's last kernel (one thread, after the block's own status bits are in): the last block to
+// come here hands the word to the host.
+__device__ __forceinline__ void sink_status(const int32_t* status, const StatusSink& sink) {
+  if (!sink.host) return;
+  const int blocks = gridDim.x * gridDim.y * gridDim.z;
+  __threadfence();
+  if (atomicAdd(sink.counter, 1) == blocks - 1) {
+    __threadfence();
+    *sink.host = *const_cast<volatile const int32_t*>(status) | STATUS_DELIVERED;
+    __threadfence_system();
+  }
+}
+
+// Host side: raise a kernel's shared-memory limit once per device (the attribute call costs as much as the launch
+// it precedes), and the number of SMs of the current device.
+template <auto Kernel>
+inline cudaError_t allow_smem(int bytes) {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (dev < 64 && (done.load(std::memory_order_relaxed) & bit)) return cudaSuccess;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
+inline int sm_count() {
+  static std::atomic<int> count[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  int n = count[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 1;
+    count[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 }  // namespace oal

@@ -16,6 +16,7 @@
 // (oal_attention/hd_block_gemm_feature_backward.py:59-131 coefficient partials).
 #include "oal_intra.cuh"
 #include "oal_kernels.h"
+#include "oal_prologue.cuh"
 
 namespace oal {
 namespace {
@@ -162,7 +163,8 @@ __global__ void __launch_bounds__(32) head_factor_kernel(const int32_t* dim_perm
     for (int r = 0; r < n; ++r) lam[r] = sqrtf(fmaxf(fabsf(sig[order[r]]), floor_v));
     table[h].rank = n;
     table[h].rpos = rpos;
-    table[h].pad[0] = table[h].pad[1] = 0;
+    table[h].w0 = 0.f;
+    table[h].pad = 0;
   }
   __syncwarp();
   HeadFactor& out = table[h];
@@ -179,63 +181,101 @@ __global__ void __launch_bounds__(32) head_factor_kernel(const int32_t* dim_perm
 
 __device__ __forceinline__ int tri_all(int g, int g2) { return g * GMAX - (g * (g - 1)) / 2 + (g2 - g); }
 
+// The prologue on its own, where no state kernel runs whose launch it could share (state_update_kernel).
+__global__ void __launch_bounds__(256) head_prologue_kernel(const PrologueArgs a) {
+  __shared__ PrologueSmem s;
+  head_prologue(a, blockIdx.x, s, threadIdx.x, 256);
+}
+
+__global__ void deliver_status_kernel(const int32_t* status, StatusSink sink) {
+  *sink.host = *status | STATUS_DELIVERED;
+  __threadfence_system();
+}
+
 // partial: [B][Hq][tiles][nu_stride]: entries r <= r' in row-major upper-triangle order of an rm x rm
-// matrix, then the rm sums n'[r], then s'.
-__global__ void __launch_bounds__(128) intra_coef_finish_kernel(const float* partial, int tiles, int nu_stride, int rm,
+// matrix, then the rm sums n'[r], then s'.  One block per head; FINISH_SEGS threads share the tiles of a sum (a
+// serial walk over 512 tiles is 60 us of dependent loads), their parts are added in fixed order.  With `factor`
+// the block goes on from dM to the gradient of its own packed factor row: dL = (S + S^T) L, see
+// expand_factor_grad_kernel.
+constexpr int FINISH_THREADS = 1024, FINISH_SEGS = 16;
+__global__ void __launch_bounds__(FINISH_THREADS) intra_coef_finish_kernel(const float* partial, int tiles, int nu_stride, int rm,
                                                                 const HeadFactor* table, const float* extra, int B,
-                                                                int Hq, int G, float* dA, float* dB, float* dC) {
+                                                                int Hq, int G, float* dA, float* dB, float* dC,
+                                                                const float* factor, float* dfactor) {
   __shared__ float D[RMAX_ALL][RMAX_ALL];
   __shared__ float T[RMAX_ALL][RMAX_ALL];
-  __shared__ float X[RMAX_ALL][RMAX_ALL];       // t D'
+  __shared__ float X[RMAX_ALL][RMAX_ALL];       // t D', later S + S^T
   __shared__ float N1[RMAX_ALL + 1];            // n'[r], then s'
+  __shared__ float seg_sum[FINISH_SEGS][NU_ALL + RMAX_ALL + 1];
   const int h = blockIdx.x, tid = threadIdx.x;
   const int n = G + 1;
-  for (int x = tid; x < RMAX_ALL * RMAX_ALL; x += 128) {
+  for (int x = tid; x < RMAX_ALL * RMAX_ALL; x += FINISH_THREADS) {
     D[x / RMAX_ALL][x % RMAX_ALL] = 0.f;
     T[x / RMAX_ALL][x % RMAX_ALL] = table[h].t[x / RMAX_ALL][x % RMAX_ALL];
   }
-  __syncthreads();
-  const int nu = rm * (rm + 1) / 2;
-  for (int x = tid; x < nu; x += 128) {
-    int r = 0, rest = x;
-    while (rest >= rm - r) { rest -= rm - r; ++r; }
-    const int r2 = r + rest;
+  if (tid <= RMAX_ALL) N1[tid] = 0.f;
+  const int nu = rm * (rm + 1) / 2, nv = nu + rm + 1;
+  const int outer = B * tiles, per = (outer + FINISH_SEGS - 1) / FINISH_SEGS;
+  for (int x = tid; x < nv * FINISH_SEGS; x += FINISH_THREADS) {
+    const int v = x % nv, seg = x / nv, o0 = seg * per, o1 = min(outer, o0 + per);
     float t = 0.f;
-    if (partial)
-      for (int b = 0; b < B; ++b)
-        for (int i = 0; i < tiles; ++i) t += partial[((size_t)(b * Hq + h) * tiles + i) * nu_stride + x];
-    if (r < RMAX_ALL && r2 < RMAX_ALL) { D[r][r2] = t; D[r2][r] = t; }
-  }
-  for (int x = tid; x < RMAX_ALL + 1; x += 128) {
-    float t = 0.f;
-    const int src = x < RMAX_ALL ? nu + x : nu + rm;
-    if (partial && (x < rm || x == RMAX_ALL))
-      for (int b = 0; b < B; ++b)
-        for (int i = 0; i < tiles; ++i) t += partial[((size_t)(b * Hq + h) * tiles + i) * nu_stride + src];
-    N1[x] = t;
+#pragma unroll 8
+    for (int o = o0; o < o1; ++o) {
+      const int b = o / tiles, i = o - b * tiles;
+      t += partial[((size_t)(b * Hq + h) * tiles + i) * nu_stride + v];
+    }
+    seg_sum[seg][v] = t;
   }
   __syncthreads();
-  for (int x = tid; x < n * n; x += 128) {
+  for (int v = tid; v < nv; v += FINISH_THREADS) {
+    float t = 0.f;
+#pragma unroll
+    for (int seg = 0; seg < FINISH_SEGS; ++seg) t += seg_sum[seg][v];
+    if (v < nu) {
+      int r = 0, rest = v;
+      while (rest >= rm - r) { rest -= rm - r; ++r; }
+      D[r][r + rest] = t;
+      D[r + rest][r] = t;
+    } else {
+      N1[v < nu + rm ? v - nu : RMAX_ALL] = t;
+    }
+  }
+  __syncthreads();
+  for (int x = tid; x < n * n; x += FINISH_THREADS) {
     const int a = x / n, r2 = x % n;
     float t = 0.f;
     for (int r = 0; r < n; ++r) t += T[a][r] * D[r][r2];
     X[a][r2] = t;
   }
   __syncthreads();
-  for (int x = tid; x < n * n; x += 128) {
+  for (int x = tid; x < n * n; x += FINISH_THREADS) {
     const int a = x / n, b = x % n;
     float t = 0.f;
     if (a == 0 && b == 0) t = N1[RMAX_ALL];
     else if (a == 0 || b == 0) { for (int r = 0; r < n; ++r) t += T[a + b][r] * N1[r]; }
     else { for (int r2 = 0; r2 < n; ++r2) t += X[a][r2] * T[b][r2]; }
     t *= 0.5f;
-    if (a == 0 && b == 0) dA[h] = t + (extra ? extra[(size_t)h * NCOEF] : 0.f);
-    else if (a == 0) dB[h * G + b - 1] = t + (extra ? extra[(size_t)h * NCOEF + b] : 0.f);
-    else if (b > 0) {
+    if (a == 0 || b == 0) {
+      t += extra ? extra[(size_t)h * NCOEF + a + b] : 0.f;
+    } else {
       const int g = a - 1, g2 = b - 1;
-      const int slot = 1 + GMAX + (g <= g2 ? tri_all(g, g2) : tri_all(g2, g));
-      dC[((size_t)h * G + g) * G + g2] = t + (extra ? extra[(size_t)h * NCOEF + slot] : 0.f);
+      t += extra ? extra[(size_t)h * NCOEF + 1 + GMAX + (g <= g2 ? tri_all(g, g2) : tri_all(g2, g))] : 0.f;
     }
+    if (a == 0 && b == 0) dA[h] = t;
+    else if (a == 0) dB[h * G + b - 1] = t;
+    else if (b > 0) dC[((size_t)h * G + a - 1) * G + b - 1] = t;
+    D[a][b] = a == 0 && b > 0 ? 2.f * t : (b == 0 && a > 0 ? 0.f : t);      // S
+  }
+  if (!factor) return;
+  __syncthreads();
+  const int P = n * (n + 1) / 2;
+  for (int x = tid; x < P; x += FINISH_THREADS) {
+    int i = 0, rest = x;
+    while (rest > i) { rest -= i + 1; ++i; }
+    const int k = rest;
+    float t = 0.f;
+    for (int j = k; j < n; ++j) t = fmaf(D[i][j] + D[j][i], factor[(size_t)h * P + j * (j + 1) / 2 + k], t);
+    dfactor[(size_t)h * P + x] = t;
   }
 }
 
@@ -295,11 +335,21 @@ cudaError_t build_head_factors(const int32_t* dim_perm, const int32_t* group_sta
   return cudaGetLastError();
 }
 
+cudaError_t launch_head_prologue(const PrologueArgs& a, int Hq, cudaStream_t st) {
+  head_prologue_kernel<<<Hq, 256, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t deliver_status(const int32_t* status, StatusSink sink, cudaStream_t st) {
+  deliver_status_kernel<<<1, 1, 0, st>>>(status, sink);
+  return cudaGetLastError();
+}
+
 cudaError_t intra_coef_finish(const float* partial, int tiles, int nu_stride, int rm, const void* table,
                               const float* extra, int B, int Hq, int G, float* dA, float* dB, float* dC,
-                              cudaStream_t st) {
-  intra_coef_finish_kernel<<<Hq, 128, 0, st>>>(partial, tiles, nu_stride, rm, static_cast<const HeadFactor*>(table),
-                                               extra, B, Hq, G, dA, dB, dC);
+                              const float* factor, float* dfactor, cudaStream_t st) {
+  intra_coef_finish_kernel<<<Hq, FINISH_THREADS, 0, st>>>(partial, tiles, nu_stride, rm, static_cast<const HeadFactor*>(table),
+                                                          extra, B, Hq, G, dA, dB, dC, factor, dfactor);
   return cudaGetLastError();
 }
 

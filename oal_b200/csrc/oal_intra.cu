@@ -27,6 +27,8 @@ struct IntraFwdArgs {
   int N, Hq, Hkv, out_dt;
   float floor;
   int out_token_major;      // out is [B, N, Hq, 64] instead of [B, Hq, N, 64]
+  int cross_from;           // first chunk that has a cross-chunk part in num / den
+  StatusSink sink;
 };
 
 constexpr int FWD_SMEM = XA_BYTES + X_BYTES + SLAB_S_BYTES + 2 * ST_BYTES;
@@ -72,6 +74,8 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
   __syncthreads();
   const int tiles = min(CT / KT, (a.N - c * CT + KT - 1) / KT);
   const int rank = hf.rank, rpos = hf.rpos;
+  const f32x2 w0 = f2_bcast(hf.w0);
+  const bool cross = c >= a.cross_from;
   init_stack_constants(St, hf, tid, CTHREADS);
   init_stack_constants(St + ST_BYTES, hf, tid, CTHREADS);
   if (tid < CTHREADS && (tid >> 7) < tiles) build_stack_piece(St + (tid >> 7) * ST_BYTES, Kimg, (tid >> 7) * KT, hf, tid & 127);
@@ -97,7 +101,10 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
     const bool warp_active = 32 * (warp & 3) + 31 >= kt * KT;       // else every pair of the warp is masked
     f32x2 wp[4], wn[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) wp[j] = wn[j] = 0ull;
+    for (int j = 0; j < 4; ++j) {
+      wp[j] = w0;
+      wn[j] = 0ull;
+    }
     w.wait(&u_done, kt & 1, 0x14);
     fence_after_sync();
     // two batches of terms: the loads of the second overlap the arithmetic of the first.  A positive
@@ -236,7 +243,7 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
         } else {
           float den = vv[0];                    // column 64
           if (i < a.N && !dead) {
-            den += a.den[orow];
+            if (cross) den += a.den[orow];
             a.den[orow] = den;
             if (!finite_f(den)) flags |= OAL_STATUS_NONFINITE;
             else if (!(den > 0.f)) flags |= OAL_STATUS_DENOMINATOR;
@@ -256,7 +263,8 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
 #pragma unroll
     for (int it = 0; it < PER; ++it) {
       const int x = tid + it * CTHREADS, r = x >> 3, seg = x & 7, ii = c * CT + r;
-      if (ii < a.N) {
+      o0[it] = o1[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (cross && ii < a.N) {
         const float* np = a.num + (qoff + ii) * VD + seg * 8;
         o0[it] = *reinterpret_cast<const float4*>(np);
         o1[it] = *reinterpret_cast<const float4*>(np + 4);
@@ -296,19 +304,23 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
   if (flags) atomicOr(a.status, flags);
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, 256);
-  if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
+  if (tid == 0) {
+    if (dead) atomicOr(a.status, w.status_bits());
+    sink_status(a.status, a.sink);
+  }
 }
 
 }  // namespace
 
 cudaError_t OAL_INTRA_NAME(intra_forward)(const void* q, const void* k, const void* v, const void* factors, void* out,
                                           float* num, float* den, int32_t* status, int B, int Hq, int Hkv, int N, int NB,
-                                          int out_dt, float floor_v, bool out_token_major, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(intra_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM);
+                                          int out_dt, float floor_v, bool out_token_major, int cross_from, StatusSink sink,
+                                          cudaStream_t st) {
+  cudaError_t e = allow_smem<intra_fwd_kernel>(FWD_SMEM);
   if (e != cudaSuccess) return e;
   IntraFwdArgs a{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                  static_cast<const __nv_bfloat16*>(v), static_cast<const HeadFactor*>(factors), out, num, den, status,
-                 N, Hq, Hkv, out_dt, floor_v, out_token_major ? 1 : 0};
+                 N, Hq, Hkv, out_dt, floor_v, out_token_major ? 1 : 0, cross_from, sink};
   intra_fwd_kernel<<<dim3(NB, Hq, B), CTHREADS, FWD_SMEM, st>>>(a);
   return cudaGetLastError();
 }

@@ -5,7 +5,7 @@
 //     w = v^T M v,   M = [[A, B/2], [B/2, C]]          (oal_attention/grouped_reference.py:61-99)
 // With the eigen-decomposition M = V diag(sigma) V^T (head_factor_kernel, one per call) and
 // lambda_r = sqrt|sigma_r| the weight is a signed sum of squares
-//     w = sum_r sgn_r u_r^2,   u_r(i,j) = c_r + sum_d q_i[d] (l_r[d] k_j[d]),
+//     w = w0 + sum_r sgn_r u_r^2,   u_r(i,j) = c_r + sum_d q_i[d] (l_r[d] k_j[d]),
 //     c_r = lambda_r V[0][r],  l_r[d] = scale lambda_r V[1 + g(d)][r],
 // so every u_r is one plain 64-long dot product of the query row with a per-dimension scaled copy
 // of the key row.  The kernels stack the R = G + 1 scaled copies of a 16-key tile as the N rows of
@@ -48,7 +48,8 @@ struct HeadFactor {
   float t[RMAX_ALL][RMAX_ALL];       // t[a][r] = V[a][r] / lambda_r  (v = t u)
   int rank;                          // R = G + 1
   int rpos;                          // terms r < rpos enter with +, the others with -
-  int pad[2];
+  float w0;                          // constant added to the weight (the packed-factor form keeps its eps out of the terms)
+  int pad;
 };
 
 // The part of it a kernel keeps in shared memory.
@@ -56,6 +57,7 @@ struct HeadFactorS {
   float l[RM][HD];
   float c[RM];
   int rank, rpos;
+  float w0;
 };
 
 __device__ __forceinline__ void load_head_factor(HeadFactorS& s, const HeadFactor* table, int h, int tid, int nthreads) {
@@ -65,6 +67,7 @@ __device__ __forceinline__ void load_head_factor(HeadFactorS& s, const HeadFacto
   if (tid == 0) {
     s.rank = min(f.rank, RM);
     s.rpos = min(f.rpos, RM);
+    s.w0 = f.w0;
   }
 }
 

@@ -36,6 +36,7 @@ struct IntraBwdArgs {
   float* coef_partial;              // [B][Hq][NB][NQ] or null: D upper triangle, sum t_r, sum 2 dW
   int32_t* status;
   int N, NB, Hq, Hkv;
+  int cross_from;                   // first chunk that has a cross-chunk part in dq_init
 };
 
 constexpr int STAGE_OUT_FLOATS = CT * 65 + 3;   // one [128][65] fp32 output staging tile (padded to 16 bytes)
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) intra_bwd_q_kernel(const IntraBwd
     for (int it = 0; it < PER; ++it) {
       const int x = tid + it * CTHREADS, r = x >> 3, seg = x & 7, i = c * CT + r;
       i0[it] = i1[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (i < a.N && a.dq_init) {
+      if (i < a.N && a.dq_init && c >= a.cross_from) {
         const float* ip = a.dq_init + (qoff + i) * HD + seg * 8;
         i0[it] = *reinterpret_cast<const float4*>(ip);
         i1[it] = *reinterpret_cast<const float4*>(ip + 4);
@@ -356,6 +357,7 @@ __global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const Intra
   __syncthreads();
   const int tiles = min(CT / KT, (a.N - c * CT + KT - 1) / KT);
   const int rank = hf.rank, rpos = hf.rpos;
+  const f32x2 w0 = f2_bcast(hf.w0);
   for (int s = 0; s < 3; ++s) init_stack_constants(St + s * ST_BYTES, hf, tid, KV_THREADS);
   if (tid < 256 && (tid >> 7) < tiles)
     build_stack_piece(St + (tid >> 7) * ST_BYTES, Qimg, (tid >> 7) * KT, hf, tid & 127, Lo + (tid >> 7) * STLO_BYTES);
@@ -420,7 +422,8 @@ __global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const Intra
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         dw2[j] = f2_pack(keep[2 * j] ? 2.f * dw[2 * j] : 0.f, keep[2 * j + 1] ? 2.f * dw[2 * j + 1] : 0.f);
-        wp[j] = wn[j] = 0ull;
+        wp[j] = w0;
+        wn[j] = 0ull;
       }
 #pragma unroll
       for (int r = 0; r < RM; ++r) {
@@ -512,21 +515,29 @@ __global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const Intra
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
 
-// dk / dv = cross-chunk part + sum over the query heads of the KV head of the per-head shares,
-// fixed order, cast to bf16.  One thread per 4 consecutive dims of one key token.
-__global__ void __launch_bounds__(256) kv_head_reduce_kernel(const float* part, const float* cross,
-                                                            __nv_bfloat16* out, int B, int Hq, int Hkv, int N) {
+// dk / dv = cross-chunk part (tokens before cross_end) + sum over the query heads of the KV head of the per-head
+// shares, fixed order, cast to bf16.  One thread per 4 consecutive dims of one key token; blockIdx.y: dk, then dv.
+struct KvReduceArgs {
+  const float *part[2], *cross[2];
+  __nv_bfloat16* out[2];
+  int B, Hq, Hkv, N, cross_end;
+};
+__global__ void __launch_bounds__(256) kv_head_reduce_kernel(const KvReduceArgs a) {
   const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x;       // over B*Hkv*N*16
-  const size_t total = (size_t)B * Hkv * N * 16;
-  if (idx >= total) return;
+  const size_t total = (size_t)a.B * a.Hkv * a.N * 16;
+  __nv_bfloat16* out = a.out[blockIdx.y];
+  if (idx >= total || !out) return;
+  const float *part = a.part[blockIdx.y], *cross = a.cross[blockIdx.y];
   const int d4 = (int)(idx & 15);
   const size_t tok = idx >> 4;                                     // (b*Hkv + kvh)*N + n
-  const int n = (int)(tok % N);
-  const size_t bk = tok / N;
-  const int kvh = (int)(bk % Hkv), b = (int)(bk / Hkv), rep = Hq / Hkv;
-  float4 acc = cross ? *reinterpret_cast<const float4*>(cross + tok * HD + 4 * d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int n = (int)(tok % a.N);
+  const size_t bk = tok / a.N;
+  const int kvh = (int)(bk % a.Hkv), b = (int)(bk / a.Hkv), rep = a.Hq / a.Hkv;
+  float4 acc = n < a.cross_end ? *reinterpret_cast<const float4*>(cross + tok * HD + 4 * d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* src = part + (((size_t)b * a.Hq + kvh * rep) * a.N + n) * HD + 4 * d4;
+#pragma unroll 8
   for (int r = 0; r < rep; ++r) {
-    const float4 t = *reinterpret_cast<const float4*>(part + (((size_t)b * Hq + kvh * rep + r) * N + n) * HD + 4 * d4);
+    const float4 t = *reinterpret_cast<const float4*>(src + (size_t)r * a.N * HD);
     acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
   }
   *reinterpret_cast<uint2*>(out + tok * HD + 4 * d4) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
@@ -536,42 +547,48 @@ __global__ void __launch_bounds__(256) kv_head_reduce_kernel(const float* part, 
 
 int OAL_INTRA_NAME(intra_coef_terms)() { return RM; }
 
-cudaError_t OAL_INTRA_NAME(intra_backward_q)(const void* q, const void* k, const void* v, const void* gimg,
-                                             const void* factors, void* dq, const float* dq_init, float* coef_partial,
-                                             int32_t* status, int B, int Hq, int Hkv, int N, int NB, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(intra_bwd_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BQ_SMEM);
-  if (e != cudaSuccess) return e;
+static IntraBwdArgs bwd_args(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
+                             int32_t* status, int B, int Hq, int Hkv, int N, int NB) {
   IntraBwdArgs a{};
   a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k);
   a.v = static_cast<const __nv_bfloat16*>(v); a.gimg = static_cast<const __nv_bfloat16*>(gimg);
   a.factors = static_cast<const HeadFactor*>(factors);
-  a.dq = dq; a.dq_init = dq_init; a.coef_partial = coef_partial; a.status = status;
+  a.status = status;
   a.N = N; a.NB = NB; a.Hq = Hq; a.Hkv = Hkv;
   a.gimg_lo_offset = (size_t)B * Hq * NB * SLAB_S_BYTES;
+  return a;
+}
+
+cudaError_t OAL_INTRA_NAME(intra_backward_q)(const void* q, const void* k, const void* v, const void* gimg,
+                                             const void* factors, void* dq, const float* dq_init, float* coef_partial,
+                                             int32_t* status, int B, int Hq, int Hkv, int N, int NB, int cross_from,
+                                             cudaStream_t st) {
+  cudaError_t e = allow_smem<intra_bwd_q_kernel>(BQ_SMEM);
+  if (e != cudaSuccess) return e;
+  IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB);
+  a.dq = dq; a.dq_init = dq_init; a.coef_partial = coef_partial; a.cross_from = cross_from;
   intra_bwd_q_kernel<<<dim3(NB, Hq, B), CTHREADS, BQ_SMEM, st>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t OAL_INTRA_NAME(intra_backward_kv)(const void* q, const void* k, const void* v, const void* gimg,
-                                              const void* factors, void* dk, void* dv, const float* dk_cross,
-                                              const float* dv_cross, float* dk_part, float* dv_part, int32_t* status,
+                                              const void* factors, float* dk_part, float* dv_part, int32_t* status,
                                               int B, int Hq, int Hkv, int N, int NB, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(intra_bwd_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BKV_SMEM);
+  cudaError_t e = allow_smem<intra_bwd_kv_kernel>(BKV_SMEM);
   if (e != cudaSuccess) return e;
-  IntraBwdArgs a{};
-  a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k);
-  a.v = static_cast<const __nv_bfloat16*>(v); a.gimg = static_cast<const __nv_bfloat16*>(gimg);
-  a.factors = static_cast<const HeadFactor*>(factors);
-  a.dk_part = dk ? dk_part : nullptr; a.dv_part = dv ? dv_part : nullptr; a.status = status;
-  a.N = N; a.NB = NB; a.Hq = Hq; a.Hkv = Hkv;
-  a.gimg_lo_offset = (size_t)B * Hq * NB * SLAB_S_BYTES;
+  IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB);
+  a.dk_part = dk_part; a.dv_part = dv_part;
   intra_bwd_kv_kernel<<<dim3(NB, Hq, B), KV_THREADS, BKV_SMEM, st>>>(a);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  return cudaGetLastError();
+}
+
+// dk, dv: null where not requested; *_cross: fp32 cross-chunk parts of the tokens before cross_end
+cudaError_t OAL_INTRA_NAME(kv_head_reduce)(const float* dk_part, const float* dv_part, const float* dk_cross, const float* dv_cross,
+                                           void* dk, void* dv, int B, int Hq, int Hkv, int N, int cross_end, cudaStream_t st) {
+  KvReduceArgs a{{dk_part, dv_part}, {dk_cross, dv_cross}, {static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv)},
+                 B, Hq, Hkv, N, cross_end};
   const size_t total = (size_t)B * Hkv * N * 16;
-  const unsigned blocks = (unsigned)((total + 255) / 256);
-  if (dk) kv_head_reduce_kernel<<<blocks, 256, 0, st>>>(dk_part, dk_cross, static_cast<__nv_bfloat16*>(dk), B, Hq, Hkv, N);
-  if (dv) kv_head_reduce_kernel<<<blocks, 256, 0, st>>>(dv_part, dv_cross, static_cast<__nv_bfloat16*>(dv), B, Hq, Hkv, N);
+  kv_head_reduce_kernel<<<dim3((unsigned)((total + 255) / 256), 2), 256, 0, st>>>(a);
   return cudaGetLastError();
 }
 

@@ -8,6 +8,16 @@
 namespace oal {
 
 // Arguments of the token-pair kernels (oal_pairs.cu).
+struct PrologueArgs;      // oal_prologue.cuh
+
+// Delivery of a call's status word to pinned host memory by the last block of its last kernel: `counter` (device, zero
+// at the start of that kernel) counts finished blocks.  host == null: not delivered.
+struct StatusSink {
+  int32_t* counter;
+  volatile int32_t* host;
+};
+constexpr int32_t STATUS_DELIVERED = (int32_t)0x80000000;
+
 struct PairArgs {
   int B, Hq, Hkv, N, G;
   int window;            // 0: whole causal prefix; >0: keys of the query's own chunk only (multiple of 64)
@@ -20,11 +30,14 @@ struct PairArgs {
   // forward
   void* out;
   float *num, *den;
-  int accumulate;        // num/den already hold the cross-chunk term
+  int accumulate;        // num/den of tokens from `accumulate_from` on already hold the cross-chunk term
+  int accumulate_from;
+  StatusSink sink;       // forward
   // backward
   const float* g;        // [B,Hq,N,80] augmented upstream gradient
   void *dq, *dk, *dv;
   const float *dq_init, *dk_init, *dv_init;   // fp32 cross-chunk parts to add, or null
+  int q_init_from, kv_init_end;               // ... of query tokens from the first on, of key tokens before the second
   float* coef_partial;   // [B][Hq][tiles][NCOEF] or null
 };
 
@@ -35,7 +48,7 @@ int pairs_tiles(int n);
 
 cudaError_t norm_vjp(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                      const float* num, const float* den, float floor_v, float* g, size_t rows,
-                     cudaStream_t st);
+                     int32_t* clear_status, cudaStream_t st);
 
 // extra: [Hq][NCOEF] slots already summed over the batch (cross-chunk term), or null
 cudaError_t reduce_coefs(const float* p0, int tiles0, const float* extra, int B, int Hq, int G,
@@ -55,28 +68,31 @@ size_t state_slab_image_bytes();           // bytes of one slab image [10][128][
 cudaError_t build_coef_table(const int32_t* dim_perm, const int32_t* group_start, const float* A,
                              const float* Bc, const float* Cc, int Hq, int G, float scale, float* table,
                              cudaStream_t st);
-cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int32_t* status,
-                         cudaStream_t st);
-// image_lo: optional second image holding bf16(state - bf16(state))
+// increments of the first NC chunks; `prologue` (optional): its blocks ride in the same launch
+cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, const PrologueArgs* prologue,
+                         int q_heads, int32_t* status, cudaStream_t st);
+// image_lo: optional second image holding bf16(state - bf16(state)); trim: see state_scan_kernel
 cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float* state_in, float* state_total,
-                       int units, int NB, int reverse, cudaStream_t st);
+                       int units, int NB, int reverse, bool trim, cudaStream_t st);
+// chunks [c0, c0 + NC) of every sequence; the other rows of out64 / out1 are not written
 cudaError_t cross_read(bool query, const void* x, const void* image, const float* coef_table, float* out64,
-                       float* out1, int B, int H, int rep, int N, int NB, int32_t* status, cudaStream_t st);
+                       float* out1, int B, int H, int rep, int N, int NB, int c0, int NC, int32_t* status, cudaStream_t st);
 
 
-// ---- tensor-core backward kernels (oal_state_bwd.cu) ----------------------------------
+// ---- tensor-core backward kernels (oal_state_bwd.cu): chunks [c0, c0 + NC) of every sequence ----------
 // carry_img / carry_lo: the saved state image and its remainder image (both or neither)
 cudaError_t dstate_heads(const void* q, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
-                         float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, float scale,
+                         float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, int c0, int NC, float scale,
                          int32_t* status, cudaStream_t st);
 cudaError_t feature_grad(bool query, const void* x, const void* gimg, const void* v, const void* image,
-                         const float* coef_table, float* dx, int B, int H, int rep, int N, int NB, int32_t* status,
-                         cudaStream_t st);
-cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, const int32_t* dim_perm,
+                         const float* coef_table, float* dx, int B, int H, int rep, int N, int NB, int c0, int NC,
+                         int32_t* status, cudaStream_t st);
+cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, int G, const int32_t* dim_perm,
                          const int32_t* group_start, float* dcoef, float* slots, cudaStream_t st);
 cudaError_t norm_vjp_image(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                            const float* num, const float* den, float floor_v, float* g, void* gimg, int heads,
-                           int N, int NB, int token_major_heads, cudaStream_t st);   // > 0: grad_out is [B, N, Hq, 64]
+                           int N, int NB, int token_major_heads /* > 0: grad_out is [B, N, Hq, 64] */,
+                           int32_t* clear_status, cudaStream_t st);
 
 
 // ---- factored intra-chunk weight (oal_factor.cu) -----------------------------------------
@@ -93,18 +109,23 @@ cudaError_t build_head_factors(const int32_t* dim_perm, const int32_t* group_sta
 // upper triangle) + extra ([Hq][NCOEF] slots of the cross-chunk term, or null).
 cudaError_t intra_coef_finish(const float* partial, int tiles, int nu_stride, int rm, const void* table,
                               const float* extra, int B, int Hq, int G, float* dA, float* dB, float* dC,
-                              cudaStream_t st);
+                              const float* factor, float* dfactor, cudaStream_t st);
+cudaError_t launch_head_prologue(const PrologueArgs& a, int Hq, cudaStream_t st);
+// writes *status | STATUS_DELIVERED to the sink's host word
+cudaError_t deliver_status(const int32_t* status, StatusSink sink, cudaStream_t st);
 
 // ---- tensor-core intra-chunk kernels (oal_intra.cu, oal_intra_bwd.cu): heads with at most 8 groups ----
 int intra_coef_terms();          // terms per head this build handles (rows of the partial-sum triangle)
 cudaError_t intra_forward(const void* q, const void* k, const void* v, const void* factors, void* out, float* num,
                           float* den, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int out_dt,
-                          float floor_v, bool out_token_major, cudaStream_t st);
+                          float floor_v, bool out_token_major, int cross_from, StatusSink sink, cudaStream_t st);
 cudaError_t intra_backward_q(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
                              void* dq, const float* dq_init, float* coef_partial, int32_t* status, int B, int Hq,
-                             int Hkv, int N, int NB, cudaStream_t st);
+                             int Hkv, int N, int NB, int cross_from, cudaStream_t st);
 cudaError_t intra_backward_kv(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
-                              void* dk, void* dv, const float* dk_cross, const float* dv_cross, float* dk_part,
-                              float* dv_part, int32_t* status, int B, int Hq, int Hkv, int N, int NB, cudaStream_t st);
+                              float* dk_part, float* dv_part, int32_t* status, int B, int Hq, int Hkv, int N, int NB,
+                              cudaStream_t st);
+cudaError_t kv_head_reduce(const float* dk_part, const float* dv_part, const float* dk_cross, const float* dv_cross,
+                           void* dk, void* dv, int B, int Hq, int Hkv, int N, int cross_end, cudaStream_t st);
 
 }  // namespace oal

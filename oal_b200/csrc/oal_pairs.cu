@@ -158,12 +158,13 @@ __global__ void __launch_bounds__(256) fwd_pairs_kernel(const PairArgs a) {
     const int r = x >> 4, c4 = (x & 15) * 4, i = i0 + r;
     if (i >= N) continue;
     const size_t row = (size_t)(b * a.Hq + h) * N + i;
+    const bool add = a.accumulate && i >= a.accumulate_from;
     float den = Ys[r * EP + VD];
-    if (a.accumulate) den += a.den[row];
+    if (add) den += a.den[row];
     float nv[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) nv[c] = Ys[r * EP + c4 + c];
-    if (a.accumulate) {
+    if (add) {
       const float4 o = *reinterpret_cast<const float4*>(a.num + row * VD + c4);
       nv[0] += o.x; nv[1] += o.y; nv[2] += o.z; nv[3] += o.w;
     }
@@ -185,10 +186,12 @@ __global__ void __launch_bounds__(256) fwd_pairs_kernel(const PairArgs a) {
     if (i >= N) continue;
     const size_t row = (size_t)(b * a.Hq + h) * N + i;
     float den = Ys[r * EP + VD];
-    if (a.accumulate) den += a.den[row];
+    if (a.accumulate && i >= a.accumulate_from) den += a.den[row];
     a.den[row] = den;
   }
   if (flags) atomicOr(a.status, flags);
+  __syncthreads();
+  if (tid == 0) sink_status(a.status, a.sink);
 }
 
 // ---------------------------------------------------------------------------
@@ -380,7 +383,7 @@ __global__ void __launch_bounds__(256) bwd_q_pairs_kernel(const PairArgs a) {
       for (int c = 0; c < 4; ++c) {
         const size_t o = qbase + (size_t)i * HD + hg.perm[4 * tx + c];
         float v = a.scale * acc[r][c];
-        if (a.dq_init) v += a.dq_init[o];
+        if (a.dq_init && i >= a.q_init_from) v += a.dq_init[o];
         store_elem(a.dq, o, a.io_dt, v);
       }
     }
@@ -555,7 +558,7 @@ __global__ void __launch_bounds__(256) bwd_kv_pairs_kernel(const PairArgs a) {
       if (j >= N) continue;
       const size_t o = kbase + (size_t)j * HD + (x & 63);
       float v = dkacc[x];
-      if (a.dk_init) v += a.dk_init[o];
+      if (a.dk_init && j < a.kv_init_end) v += a.dk_init[o];
       store_elem(a.dk, o, a.io_dt, v);
     }
   }
@@ -570,7 +573,7 @@ __global__ void __launch_bounds__(256) bwd_kv_pairs_kernel(const PairArgs a) {
         if (e >= VD) continue;
         const size_t o = kbase + (size_t)j * VD + e;
         float v = adu[r][c];
-        if (a.dv_init) v += a.dv_init[o];
+        if (a.dv_init && j < a.kv_init_end) v += a.dv_init[o];
         store_elem(a.dv, o, a.io_dt, v);
       }
     }
@@ -586,7 +589,8 @@ __global__ void __launch_bounds__(256) bwd_kv_pairs_kernel(const PairArgs a) {
 __global__ void __launch_bounds__(256) norm_vjp_kernel(const void* grad_out, int out_dt,
                                                        const float* grad_num, const float* grad_den,
                                                        const float* num, const float* den,
-                                                       float floor_v, float* g, size_t rows) {
+                                                       float floor_v, float* g, size_t rows, int32_t* clear_status) {
+  if (clear_status && blockIdx.x == 0 && threadIdx.x == 0) *clear_status = 0;     // first kernel of the backward
   const size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -657,18 +661,15 @@ cudaError_t launch_pairs(const PairArgs& a, int which, cudaStream_t st) {
   const int tiles = (a.N + TP - 1) / TP;
   cudaError_t e;
   if (which == 0) {
-    e = cudaFuncSetAttribute(fwd_pairs_kernel<GCAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)fwd_smem<GCAP>());
+    e = allow_smem<fwd_pairs_kernel<GCAP>>((int)fwd_smem<GCAP>());
     if (e != cudaSuccess) return e;
     fwd_pairs_kernel<GCAP><<<dim3(tiles, a.Hq, a.B), 256, fwd_smem<GCAP>(), st>>>(a);
   } else if (which == 1) {
-    e = cudaFuncSetAttribute(bwd_q_pairs_kernel<GCAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bwd_q_smem<GCAP>());
+    e = allow_smem<bwd_q_pairs_kernel<GCAP>>((int)bwd_q_smem<GCAP>());
     if (e != cudaSuccess) return e;
     bwd_q_pairs_kernel<GCAP><<<dim3(tiles, a.Hq, a.B), 256, bwd_q_smem<GCAP>(), st>>>(a);
   } else {
-    e = cudaFuncSetAttribute(bwd_kv_pairs_kernel<GCAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bwd_kv_smem<GCAP>());
+    e = allow_smem<bwd_kv_pairs_kernel<GCAP>>((int)bwd_kv_smem<GCAP>());
     if (e != cudaSuccess) return e;
     bwd_kv_pairs_kernel<GCAP><<<dim3(tiles, a.Hkv, a.B), 256, bwd_kv_smem<GCAP>(), st>>>(a);
   }
@@ -690,9 +691,9 @@ int pairs_tiles(int n) { return (n + TP - 1) / TP; }
 
 cudaError_t norm_vjp(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                      const float* num, const float* den, float floor_v, float* g, size_t rows,
-                     cudaStream_t st) {
+                     int32_t* clear_status, cudaStream_t st) {
   norm_vjp_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(grad_out, out_dt, grad_num, grad_den, num,
-                                                             den, floor_v, g, rows);
+                                                             den, floor_v, g, rows, clear_status);
   return cudaGetLastError();
 }
 

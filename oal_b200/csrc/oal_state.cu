@@ -12,6 +12,7 @@
 // async copies.  Every mbarrier wait is bounded (oal_umma.cuh).
 #include "oal_features.cuh"
 #include "oal_kernels.h"
+#include "oal_prologue.cuh"
 
 namespace oal {
 namespace {
@@ -55,24 +56,32 @@ __global__ void coef_table_kernel(const int32_t* dim_perm, const int32_t* group_
 
 // ---------------------------------------------------------------------------
 // state_update: dS[u,c][slab rows] = phi_k^T U
-//   grid (4 slab groups, chunks, units); 256 threads, thread = (token, half of the slab's chunks)
+//   one block per (slab group of 4, chunk, unit); 256 threads, thread = (token, half of the slab's chunks).
+//   The first `n_prologue` blocks compute the per-head prologue instead (oal_prologue.cuh): it has no input in
+//   common with this kernel, both are needed next, and one launch costs less than two and a fork.
 // ---------------------------------------------------------------------------
 struct StateUpdateArgs {
   const __nv_bfloat16 *k, *v;   // [units, N, 64]
   float* ds;                    // [units, NB] chunks of F_ROWS x EP floats in state_inc_offset order
-  int N, NB;
+  int N, NB, NC;                // chunks of the sequence; chunks whose increment is computed (the first NC)
   int32_t* status;
 };
 
-__global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const StateUpdateArgs a) {
+__global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const StateUpdateArgs a, const PrologueArgs pro,
+                                                                      int n_prologue) {
   extern __shared__ __align__(128) unsigned char smem[];
+  if ((int)blockIdx.x < n_prologue) {
+    head_prologue(pro, blockIdx.x, *reinterpret_cast<PrologueSmem*>(smem), threadIdx.x, GEN_THREADS);
+    return;
+  }
   unsigned char* Abuf = smem;                          // 2 x SLAB_A_BYTES
   unsigned char* Uimg = smem + 2 * SLAB_A_BYTES;       // [10][128 tokens][8 e]
   __shared__ uint64_t mma_done[2];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int grp = blockIdx.x, c = blockIdx.y, u = blockIdx.z;
+  const int item = (int)blockIdx.x - n_prologue;
+  const int grp = item % SU_GROUPS, c = (item / SU_GROUPS) % a.NC, u = item / SU_GROUPS / a.NC;
   const int token = tid & 127, half = tid >> 7;
   if (warp == 0) tmem_alloc(&tmem_base, 256);
   if (tid == 0) {
@@ -146,54 +155,54 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
 // ---------------------------------------------------------------------------
 // state_scan: exclusive prefix over chunks (forward) or suffix (reverse), fp32 running sum,
 // result stored as the bf16 MMA operand image  [u][c][slab][e/8][128 rows][8 e].
-//   thread = (feature row f, e chunk): grid (F_ROWS*10/256, units)
-// ---------------------------------------------------------------------------
+//   Increments and images have the same element order, so a thread owns four consecutive elements and walks the
+//   chunks: grid (F_ROWS * EP / 4 / 256, units).  Bound by HBM at many units, by the latency of the walk at few:
+//   the loads of SCAN_AHEAD chunks are in flight together.  `trim`: the first chunk visited meets a zero state and
+//   nothing reads its image, and the increment of the last one visited reaches no image: neither is touched.
 // image_lo (optional): a second image of the rounding remainders, bf16(state - bf16(state)); the
 // coefficient-gradient dot products of the backward read state = image + image_lo.
+// ---------------------------------------------------------------------------
+constexpr int SCAN_AHEAD = 4;
+
 __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_bfloat16* image,
                                                          __nv_bfloat16* image_lo, const float* state_in,
-                                                         float* state_total, int NB, int reverse) {
-  const int x = blockIdx.x * 256 + threadIdx.x;     // 0 .. F_ROWS*10
-  const int u = blockIdx.y;
-  if (x >= F_ROWS * (EP / 8)) return;
-  const int ec = x / F_ROWS, f = x % F_ROWS;
-  const int slab = f >> 7, fr = f & 127;
-  float run[8];
-  if (state_in) {
-    const float4* p = reinterpret_cast<const float4*>(state_in + ((size_t)u * F_ROWS + f) * EP + 8 * ec);
-    const float4 a0 = p[0], a1 = p[1];
-    run[0] = a0.x; run[1] = a0.y; run[2] = a0.z; run[3] = a0.w;
-    run[4] = a1.x; run[5] = a1.y; run[6] = a1.z; run[7] = a1.w;
-  } else {
+                                                         float* state_total, int NB, int reverse, int trim) {
+  constexpr size_t CHUNK = (size_t)F_ROWS * EP;
+  static_assert(CHUNK % 1024 == 0, "the grid covers a chunk exactly");
+  const size_t x = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;      // element inside a chunk, image order
+  const size_t u = blockIdx.y;
+  // row-major position of the same element in state_in / state_total
+  const int tile = (int)(x >> 10), within = (int)(x & 1023);          // 1024 = 128 rows x 8 columns
+  const size_t rm = (size_t)((tile / (EP / 8)) * 128 + (within >> 3)) * EP + (tile % (EP / 8)) * 8 + (within & 7);
+  float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (state_in) run = *reinterpret_cast<const float4*>(state_in + u * CHUNK + rm);
+  const float* src = ds + u * NB * CHUNK + x;
+  const size_t dst = u * NB * CHUNK + x;
+  for (int n0 = 0; n0 < NB; n0 += SCAN_AHEAD) {
+    float4 inc[SCAN_AHEAD];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) run[j] = 0.f;
-  }
-  for (int n = 0; n < NB; ++n) {
-    const int c = reverse ? NB - 1 - n : n;
-    const float4* p =
-        reinterpret_cast<const float4*>(ds + ((size_t)u * NB + c) * F_ROWS * EP + state_inc_offset(f, 8 * ec));
-    const float4 a0 = p[0], a1 = p[1];
-    if (image) {
-      uint4 o = make_uint4(pack_bf16(run[0], run[1]), pack_bf16(run[2], run[3]), pack_bf16(run[4], run[5]),
-                           pack_bf16(run[6], run[7]));
-      const size_t at = ((((size_t)u * NB + c) * F_SLABS + slab) * (EP / 8) + ec) * 128 + fr;
-      reinterpret_cast<uint4*>(image)[at] = o;
-      if (image_lo) {
-        const uint32_t w[4] = {o.x, o.y, o.z, o.w};
-        uint32_t l[4];
+    for (int k = 0; k < SCAN_AHEAD; ++k) {
+      const int n = n0 + k, c = reverse ? NB - 1 - n : n;
+      if (n < NB - trim) inc[k] = __ldcs(reinterpret_cast<const float4*>(src + c * CHUNK));
+    }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) l[k] = pack_bf16(run[2 * k] - bf16_lo(w[k]), run[2 * k + 1] - bf16_hi(w[k]));
-        reinterpret_cast<uint4*>(image_lo)[at] = make_uint4(l[0], l[1], l[2], l[3]);
+    for (int k = 0; k < SCAN_AHEAD; ++k) {
+      const int n = n0 + k, c = reverse ? NB - 1 - n : n;
+      if (n >= NB) break;
+      if (image && n >= trim) {
+        const uint2 hi = make_uint2(pack_bf16(run.x, run.y), pack_bf16(run.z, run.w));
+        *reinterpret_cast<uint2*>(image + dst + c * CHUNK) = hi;
+        if (image_lo)
+          *reinterpret_cast<uint2*>(image_lo + dst + c * CHUNK) =
+              make_uint2(pack_bf16(run.x - bf16_lo(hi.x), run.y - bf16_hi(hi.x)),
+                         pack_bf16(run.z - bf16_lo(hi.y), run.w - bf16_hi(hi.y)));
+      }
+      if (n < NB - trim) {
+        run.x += inc[k].x; run.y += inc[k].y; run.z += inc[k].z; run.w += inc[k].w;
       }
     }
-    run[0] += a0.x; run[1] += a0.y; run[2] += a0.z; run[3] += a0.w;
-    run[4] += a1.x; run[5] += a1.y; run[6] += a1.z; run[7] += a1.w;
   }
-  if (state_total) {
-    float4* p = reinterpret_cast<float4*>(state_total + ((size_t)u * F_ROWS + f) * EP + 8 * ec);
-    p[0] = make_float4(run[0], run[1], run[2], run[3]);
-    p[1] = make_float4(run[4], run[5], run[6], run[7]);
-  }
+  if (state_total) *reinterpret_cast<float4*>(state_total + u * CHUNK + rm) = run;
 }
 
 // ---------------------------------------------------------------------------
@@ -208,6 +217,7 @@ struct CrossReadArgs {
   float* out64;                  // [B,H,N,64]
   float* out1;                   // [B,H,N] (QUERY: denominator)
   int N, NB, H, rep, B;          // rep = heads per state unit (Hq/Hkv for QUERY, 1 otherwise)
+  int c0, NC;                    // chunks [c0, c0 + NC) of each sequence (the others meet a zero state)
   int32_t* status;
 };
 
@@ -229,11 +239,11 @@ struct CrItem {
   int b, h, c;
 };
 // item index -> (batch, head, chunk): the `rep` heads of a state unit are adjacent, then chunks
-__device__ __forceinline__ CrItem cr_item(int item, int H, int rep, int NB) {
+__device__ __forceinline__ CrItem cr_item(int item, int H, int rep, int NC, int c0) {
   CrItem r;
   const int hh = item % rep, t = item / rep;
-  r.c = t % NB;
-  const int unit = t / NB, units_per_b = H / rep;
+  r.c = c0 + t % NC;
+  const int unit = t / NC, units_per_b = H / rep;
   r.b = unit / units_per_b;
   r.h = (unit % units_per_b) * rep + hh;
   return r;
@@ -249,7 +259,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_items = a.B * a.H * a.NB;
+  const int n_items = a.B * a.H * a.NC;
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   if (warp == CR_ISSUER) tmem_alloc(&tmem_base, 256);
   if (tid == 0) {
@@ -280,7 +290,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
     const int token = tid & 127, half = tid >> 7;
     int s3 = 0, use = 0;
     for (int k = 0; k < my_items; ++k) {
-      const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NB);
+      const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
       // this head's coefficient table, brought in by the loader warp (two buffers)
       const float* coef = reinterpret_cast<const float*>(Sbuf + CR_SRING * SLAB_S_BYTES) + (k & 1) * F_ROWS;
       if constexpr (QUERY) w.wait(&coef_full[k & 1], (k >> 1) & 1, 0x47);
@@ -312,7 +322,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
     // ---------------- accumulator -> HBM ----------------
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
     for (int k = 0; k < my_items; ++k) {
-      const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NB);
+      const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
       const int row = it.c * CT + 32 * (warp & 3) + lane;
       const size_t orow = (size_t)(it.b * a.H + it.h) * a.N + row;
       w.wait(&acc_full[k & 1], (k >> 1) & 1, 0x42);
@@ -372,7 +382,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
     if (lane == 0) {
       int gs = 0, guse = 0;
       for (int k = 0; k < my_items; ++k) {
-        const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NB);
+        const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         const int unit = (it.b * a.H + it.h) / a.rep;
         const unsigned char* img = reinterpret_cast<const unsigned char*>(a.image) +
                                    ((size_t)unit * a.NB + it.c) * F_SLABS * SLAB_S_BYTES;
@@ -410,41 +420,38 @@ cudaError_t build_coef_table(const int32_t* dim_perm, const int32_t* group_start
   return cudaGetLastError();
 }
 
-cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int32_t* status,
-                         cudaStream_t st) {
+cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, const PrologueArgs* prologue,
+                         int q_heads, int32_t* status, cudaStream_t st) {
   const int smem = 2 * SLAB_A_BYTES + SLAB_S_BYTES;
-  cudaError_t e = cudaFuncSetAttribute(state_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = allow_smem<state_update_kernel>(smem);
   if (e != cudaSuccess) return e;
-  StateUpdateArgs a{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ds, N, NB, status};
-  state_update_kernel<<<dim3(SU_GROUPS, NB, units), GEN_THREADS, smem, st>>>(a);
+  StateUpdateArgs a{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ds, N, NB, NC, status};
+  const int n_pro = prologue ? q_heads : 0;
+  state_update_kernel<<<n_pro + SU_GROUPS * NC * units, GEN_THREADS, smem, st>>>(a, prologue ? *prologue : PrologueArgs{}, n_pro);
   return cudaGetLastError();
 }
 
 cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float* state_in, float* state_total,
-                       int units, int NB, int reverse, cudaStream_t st) {
-  state_scan_kernel<<<dim3((F_ROWS * (EP / 8) + 255) / 256, units), 256, 0, st>>>(
-      ds, static_cast<__nv_bfloat16*>(image), static_cast<__nv_bfloat16*>(image_lo), state_in, state_total, NB, reverse);
+                       int units, int NB, int reverse, bool trim, cudaStream_t st) {
+  state_scan_kernel<<<dim3(F_ROWS * EP / 1024, units), 256, 0, st>>>(
+      ds, static_cast<__nv_bfloat16*>(image), static_cast<__nv_bfloat16*>(image_lo), state_in, state_total, NB, reverse,
+      trim ? 1 : 0);
   return cudaGetLastError();
 }
 
 cudaError_t cross_read(bool query, const void* x, const void* image, const float* coef_table, float* out64,
-                       float* out1, int B, int H, int rep, int N, int NB, int32_t* status,
+                       float* out1, int B, int H, int rep, int N, int NB, int c0, int NC, int32_t* status,
                        cudaStream_t st) {
   const int smem = CR_ARING * SLAB_A_BYTES + CR_SRING * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float);
   CrossReadArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(image), coef_table,
-                  out64, out1, N, NB, H, rep, B, status};
+                  out64, out1, N, NB, H, rep, B, c0, NC, status};
   cudaError_t e;
-  int dev = 0, sms = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  const int items = B * H * NB, grid = items < sms ? items : sms;
+  const int sms = sm_count(), items = B * H * NC, grid = items < sms ? items : sms;
   if (query) {
-    e = cudaFuncSetAttribute(cross_read_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+    if ((e = allow_smem<cross_read_kernel<true>>(smem)) != cudaSuccess) return e;
     cross_read_kernel<true><<<grid, CR_THREADS, smem, st>>>(a);
   } else {
-    e = cudaFuncSetAttribute(cross_read_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+    if ((e = allow_smem<cross_read_kernel<false>>(smem)) != cudaSuccess) return e;
     cross_read_kernel<false><<<grid, CR_THREADS, smem, st>>>(a);
   }
   return cudaGetLastError();

@@ -40,8 +40,9 @@ struct DStateArgs {
                                    // because they are sums of strongly cancelling terms
   const float* coef_table;         // [Hq, F_ROWS]
   float* dcarry;                   // [units, NB] chunks of F_ROWS x EP floats in state_inc_offset order
-  float* dcoef_partial;            // [B, NB, 2 column halves, Hq, F_ROWS] or null
+  float* dcoef_partial;            // [B, NC, 2 column halves, Hq, F_ROWS] or null
   int N, NB, Hq, Hkv, units;
+  int c0, NC;                      // chunks [c0, c0 + NC) of each sequence (no one reads dCarry of the others)
   float scale;
   int32_t* status;
 };
@@ -71,23 +72,23 @@ static_assert(DS_GEN_WARPS % 4 == 0, "drain warp w must sit on tensor-memory lan
 struct DsCursor {
   int u, c, slab, hh, item;
   int b, h0;          // batch row and first query head of the item's KV head
-  __device__ __forceinline__ void set_item(int it_item, int NB, int Hkv, int rep) {
+  __device__ __forceinline__ void set_item(int it_item, int c0, int NC, int Hkv, int rep) {
     item = it_item;
     slab = item % F_SLABS;
     const int r = item / F_SLABS;
-    c = r % NB;
-    u = r / NB;
+    c = c0 + r % NC;
+    u = r / NC;
     b = u / Hkv;
     h0 = (u - b * Hkv) * rep;
   }
-  __device__ __forceinline__ void start(int NB, int Hkv, int rep) {
+  __device__ __forceinline__ void start(int c0, int NC, int Hkv, int rep) {
     hh = 0;
-    set_item(blockIdx.x, NB, Hkv, rep);
+    set_item(blockIdx.x, c0, NC, Hkv, rep);
   }
-  __device__ __forceinline__ void next(int rep, int NB, int Hkv) {
+  __device__ __forceinline__ void next(int rep, int c0, int NC, int Hkv) {
     if (++hh == rep) {
       hh = 0;
-      set_item(item + gridDim.x, NB, Hkv, rep);
+      set_item(item + gridDim.x, c0, NC, Hkv, rep);
     }
   }
 };
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
   __shared__ int dead;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rep = a.Hq / a.Hkv;
-  const int n_items = F_SLABS * a.NB * a.units;
+  const int n_items = F_SLABS * a.NC * a.units;
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   const int T = my_items * rep;
   if (warp == DS_ISSUER) tmem_alloc(&tmem_base, 256);
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
       }
     };
     DsCursor cur;
-    cur.start(a.NB, a.Hkv, rep);
+    cur.start(a.c0, a.NC, a.Hkv, rep);
     if (T > 0) fetch(cur);
     int s = 0, use = 0;                       // ring slot of `it` and how often it has been used before
     for (int it = 0; it < T; ++it) {
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
         xp[4 * j + 2] = nx[j].z;
         xp[4 * j + 3] = nx[j].w;
       }
-      cur.next(rep, a.NB, a.Hkv);
+      cur.next(rep, a.c0, a.NC, a.Hkv);
       if (it + 1 < T) fetch(cur);             // in flight while this slab is generated
       if (use > 0) w.wait(&mma_done[s], (use - 1) & 1, 0x31);   // the MMA that read A[s] has completed
       write_slab_raw(slab, xp, reinterpret_cast<uint4*>(Abuf + s * SLAB_A_BYTES) + token);
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
 #pragma unroll
     for (int j = 0; j < DS_COLS / 2; ++j) carry[j] = 0ull;
     DsCursor d, dn;
-    d.start(a.NB, a.Hkv, rep);
+    d.start(a.c0, a.NC, a.Hkv, rep);
     dn = d;
     int s = 0, use = 0;
     float cf_next = T > 0 ? a.coef_table[(size_t)d.h0 * F_ROWS + d.slab * 128 + fr] : 0.f;
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
       const int b = d.b, h = d.h0 + d.hh, f = d.slab * 128 + fr;
       const float fs = feature_scale_factor(f, a.scale);   // d(table entry) / d(coefficient)
       const float cf = cf_next;
-      dn.next(rep, a.NB, a.Hkv);
+      dn.next(rep, a.c0, a.NC, a.Hkv);
       if (it + 1 < T)       // coefficient of the next (item, head): in flight during this drain
         cf_next = a.coef_table[(size_t)(dn.h0 + dn.hh) * F_ROWS + dn.slab * 128 + fr];
       if (d.hh == 0 && a.carry_img) {
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
       f2_unpack(dot[1], d2, d3);
       const float dot_sum = (d0 + d2) + (d1 + d3);
       if (a.dcoef_partial)      // one partial per column half, summed by the reduction over (batch, chunk, half)
-        a.dcoef_partial[((((size_t)b * a.NB + d.c) * 2 + ch) * a.Hq + h) * F_ROWS + f] =
+        a.dcoef_partial[((((size_t)b * a.NC + d.c - a.c0) * 2 + ch) * a.Hq + h) * F_ROWS + f] =
             fs * dot_sum;
       if (d.hh == rep - 1) {
         // dCarry rows of this slab -> HBM; the next group of 8 columns of a row lies one 128-row block further
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
     // ---------------- G image stream ----------------
     if (lane == 0) {
       DsCursor d;
-      d.start(a.NB, a.Hkv, rep);
+      d.start(a.c0, a.NC, a.Hkv, rep);
       int gs = 0, guse = 0;
       for (int it = 0; it < T; ++it) {
         const int h = d.h0 + d.hh;
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
         if (guse > 0) w.wait(&g_free[gs], (guse - 1) & 1, 0x36);
         mbar_arrive_expect_tx(&g_full[gs], SLAB_S_BYTES);
         bulk_g2s(Gbuf + gs * SLAB_S_BYTES, src, SLAB_S_BYTES, &g_full[gs]);
-        d.next(rep, a.NB, a.Hkv);
+        d.next(rep, a.c0, a.NC, a.Hkv);
         if (++gs == DS_GRING) { gs = 0; ++guse; }
       }
     }
@@ -408,6 +409,7 @@ struct FeatGradArgs {
   const float* coef_table;       // QUERY
   float* dx;                     // [B,H,N,64] fp32
   int N, NB, H, rep, B;
+  int c0, NC;                    // chunks [c0, c0 + NC) of each sequence (the others meet a zero state)
   int32_t* status;
 };
 
@@ -418,11 +420,11 @@ constexpr int FG_SRING = 4, FG_DRING = 3;
 struct FgItem {
   int b, h, c;
 };
-__device__ __forceinline__ FgItem fg_item(int item, int H, int rep, int NB) {
+__device__ __forceinline__ FgItem fg_item(int item, int H, int rep, int NC, int c0) {
   FgItem r;
   const int hh = item % rep, t = item / rep;
-  r.c = t % NB;
-  const int unit = t / NB, units_per_b = H / rep;
+  r.c = c0 + t % NC;
+  const int unit = t / NC, units_per_b = H / rep;
   r.b = unit / units_per_b;
   r.h = (unit % units_per_b) * rep + hh;
   return r;
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_items = a.B * a.H * a.NB;
+  const int n_items = a.B * a.H * a.NC;
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   if (warp == FG_ISSUER) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
@@ -472,7 +474,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
     int ds = 0, duse = 0;
     for (int k = 0; k < my_items; ++k) {
-      const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NB);
+      const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
       const int i = it.c * CT + token;
       const size_t head_off = (size_t)(it.b * a.H + it.h) * a.N;
       f32x2 xq[HD / 2], dxq[HD / 2];
@@ -561,7 +563,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
     if (lane == 0) {
       int gs = 0, guse = 0;
       for (int k = 0; k < my_items; ++k) {
-        const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NB);
+        const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         const int unit = (it.b * a.H + it.h) / a.rep;
         const unsigned char* img = reinterpret_cast<const unsigned char*>(a.image) +
                                    ((size_t)unit * a.NB + it.c) * F_SLABS * SLAB_S_BYTES;
@@ -598,7 +600,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
 // coefficient gradients of the cross-chunk term: per-feature sums -> (A, B_g, C_gg') slots
 // ---------------------------------------------------------------------------
 // block = 32 feature rows x 8 segments of the outer index; the segments are added in fixed order
-__global__ void __launch_bounds__(256) dcoef_sum_kernel(const float* partial, int outer /* B*NB*2 */, int Hq,
+__global__ void __launch_bounds__(256) dcoef_sum_kernel(const float* partial, int outer /* B*NC*2 */, int Hq,
                                                         float* dcoef) {
   __shared__ float seg_sum[8][32];
   const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
@@ -619,12 +621,16 @@ __global__ void __launch_bounds__(256) dcoef_sum_kernel(const float* partial, in
 
 __device__ __forceinline__ int tri_slot(int g, int g2) { return g * GMAX - (g * (g - 1)) / 2 + (g2 - g); }
 
-__global__ void dcoef_slots_kernel(const float* dcoef, const int32_t* dim_perm, const int32_t* group_start,
-                                   float* slots /* [Hq][NCOEF] */) {
+// One block per head.  A warp walks all features once per coefficient slot, so the sums need no atomics and
+// their order is fixed: lane partial sums over features lane, lane + 32, ..., then the butterfly.
+constexpr int SLOT_WARPS = 32;
+__global__ void __launch_bounds__(32 * SLOT_WARPS) dcoef_slots_kernel(const float* dcoef, const int32_t* dim_perm,
+                                                                      const int32_t* group_start, int G,
+                                                                      float* slots /* [Hq][NCOEF] */) {
   __shared__ int gdim[HD];
   __shared__ short fslot[F_ROWS];
   __shared__ float fval[F_ROWS];
-  const int h = blockIdx.x;
+  const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x < HD) {
     const int p = threadIdx.x;
     int g = 0;
@@ -634,7 +640,7 @@ __global__ void dcoef_slots_kernel(const float* dcoef, const int32_t* dim_perm, 
   __syncthreads();
   for (int f = threadIdx.x; f < F_ROWS; f += blockDim.x) {
     int slot = -1;
-    float wgt = 1.f;
+    float wgt = 0.f;
     const FeatureId id = feature_id(f);
     if (id.kind == 0 && id.live) {
       const int ga = min(gdim[id.r], gdim[id.c]), gb = max(gdim[id.r], gdim[id.c]);
@@ -642,18 +648,29 @@ __global__ void dcoef_slots_kernel(const float* dcoef, const int32_t* dim_perm, 
       wgt = (ga == gb && id.r != id.c) ? 2.f : 1.f;
     } else if (id.kind == 1) {
       slot = 1 + gdim[id.r];
+      wgt = 1.f;
     } else if (id.kind == 2) {
       slot = 0;
+      wgt = 1.f;
     }
     fslot[f] = (short)slot;
     fval[f] = slot >= 0 ? wgt * dcoef[(size_t)h * F_ROWS + f] : 0.f;
   }
   __syncthreads();
-  for (int s = threadIdx.x; s < NCOEF; s += blockDim.x) {
+  const int live = 1 + G + G * (G + 1) / 2;      // slots that groups 0 .. G-1 can reach, in (A, B, C rows) order
+  for (int x = warp; x < live; x += SLOT_WARPS) {
+    int s = x;
+    if (x > G) {
+      int g = 0, rest = x - 1 - G;
+      while (rest >= G - g) { rest -= G - g; ++g; }
+      s = 1 + GMAX + tri_slot(g, g + rest);
+    }
     float t = 0.f;
-    for (int f = 0; f < F_ROWS; ++f)
-      if (fslot[f] == s) t += fval[f];
-    slots[(size_t)h * NCOEF + s] = t;
+#pragma unroll 4
+    for (int f = lane; f < F_ROWS; f += 32) t += fslot[f] == s ? fval[f] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) slots[(size_t)h * NCOEF + s] = t;
   }
 }
 
@@ -665,8 +682,9 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
                                                              const float* grad_den, const float* num,
                                                              const float* den, float floor_v, float* g,
                                                              __nv_bfloat16* gimg, int N, int NB, int heads,
-                                                             int tm_heads) {
+                                                             int tm_heads, int32_t* status) {
   __shared__ float part[8][32];
+  if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;     // first kernel of the backward
   const int ec = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t per_head = (size_t)NB * CT;
   const size_t r = (size_t)blockIdx.x * 32 + lane;          // grid covers heads * per_head rows exactly
@@ -751,64 +769,55 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
 }  // namespace
 
 cudaError_t dstate_heads(const void* q, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
-                         float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, float scale,
+                         float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, int c0, int NC, float scale,
                          int32_t* status, cudaStream_t st) {
   const int smem = DS_RING * SLAB_A_BYTES + DS_GRING * SLAB_S_BYTES;
-  cudaError_t e = cudaFuncSetAttribute(dstate_heads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = allow_smem<dstate_heads_kernel>(smem);
   if (e != cudaSuccess) return e;
-  int dev = 0, sms = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  const int items = F_SLABS * NB * B * Hkv;
+  const int sms = sm_count(), items = F_SLABS * NC * B * Hkv;
   DStateArgs a{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(gimg),
                static_cast<const __nv_bfloat16*>(carry_img), static_cast<const __nv_bfloat16*>(carry_lo), coef_table,
-               dcarry, dcoef_partial, N, NB, Hq, Hkv,
-               B * Hkv, scale, status};
+               dcarry, dcoef_partial, N, NB, Hq, Hkv, B * Hkv, c0, NC, scale, status};
   dstate_heads_kernel<<<items < sms ? items : sms, DS_THREADS, smem, st>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t feature_grad(bool query, const void* x, const void* gimg, const void* v, const void* image,
-                         const float* coef_table, float* dx, int B, int H, int rep, int N, int NB, int32_t* status,
-                         cudaStream_t st) {
+                         const float* coef_table, float* dx, int B, int H, int rep, int N, int NB, int c0, int NC,
+                         int32_t* status, cudaStream_t st) {
   const int smem = FG_SRING * SLAB_S_BYTES + 2 * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float) +
                    128 * 65 * (int)sizeof(float);
   FeatGradArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gimg),
                  static_cast<const __nv_bfloat16*>(v), static_cast<const __nv_bfloat16*>(image), coef_table, dx,
-                 N, NB, H, rep, B, status};
+                 N, NB, H, rep, B, c0, NC, status};
   cudaError_t e;
-  int dev = 0, sms = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  const int items = B * H * NB, grid = items < sms ? items : sms;
+  const int sms = sm_count(), items = B * H * NC, grid = items < sms ? items : sms;
   if (query) {
-    e = cudaFuncSetAttribute(feature_grad_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+    if ((e = allow_smem<feature_grad_kernel<true>>(smem)) != cudaSuccess) return e;
     feature_grad_kernel<true><<<grid, FG_THREADS, smem, st>>>(a);
   } else {
-    e = cudaFuncSetAttribute(feature_grad_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+    if ((e = allow_smem<feature_grad_kernel<false>>(smem)) != cudaSuccess) return e;
     feature_grad_kernel<false><<<grid, FG_THREADS, smem, st>>>(a);
   }
   return cudaGetLastError();
 }
 
-cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, const int32_t* dim_perm,
+cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, int G, const int32_t* dim_perm,
                          const int32_t* group_start, float* dcoef, float* slots, cudaStream_t st) {
   dcoef_sum_kernel<<<dim3(F_ROWS / 32, Hq), 256, 0, st>>>(partial, outer, Hq, dcoef);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  dcoef_slots_kernel<<<Hq, 256, 0, st>>>(dcoef, dim_perm, group_start, slots);
+  dcoef_slots_kernel<<<Hq, 32 * SLOT_WARPS, 0, st>>>(dcoef, dim_perm, group_start, G, slots);
   return cudaGetLastError();
 }
 
 cudaError_t norm_vjp_image(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                            const float* num, const float* den, float floor_v, float* g, void* gimg, int heads,
-                           int N, int NB, int token_major_heads, cudaStream_t st) {
+                           int N, int NB, int token_major_heads, int32_t* clear_status, cudaStream_t st) {
   const size_t rows = (size_t)heads * NB * CT;      // a multiple of 32
   norm_vjp_image_kernel<<<(unsigned)(rows / 32), 256, 0, st>>>(grad_out, out_dt, grad_num, grad_den, num, den,
                                                                    floor_v, g, static_cast<__nv_bfloat16*>(gimg), N,
-                                                                   NB, heads, token_major_heads);
+                                                                   NB, heads, token_major_heads, clear_status);
   return cudaGetLastError();
 }
 

@@ -106,6 +106,15 @@ def _validate_factor(factor: object, *, query_heads: int, q_device: torch.device
 def _canonicalize_dim_groups(dim_groups: object, *, query_heads: int, head_dimension: int, gmax: int,
                              q_device: torch.device) -> torch.Tensor:
     """int32 ``[D]`` or ``[Hq, D]``; ids of every head must form the prefix 0..G_h-1, G_h <= gmax."""
+    return _canonical_groups_and_tables(dim_groups, query_heads=query_heads, head_dimension=head_dimension, gmax=gmax,
+                                        q_device=q_device)[0]
+
+
+def _canonical_groups_and_tables(dim_groups: object, *, query_heads: int, head_dimension: int, gmax: int,
+                                 q_device: torch.device):
+    """The same, with the device tables (``dim_perm``, ``group_start``) the kernels read."""
+    from . import _lib
+
     if not isinstance(dim_groups, torch.Tensor):
         raise TypeError("dim_groups must be a torch.Tensor")
     if dim_groups.dtype not in {torch.int32, torch.int64}:
@@ -124,15 +133,14 @@ def _canonicalize_dim_groups(dim_groups: object, *, query_heads: int, head_dimen
         per_head = dim_groups
     else:
         raise ValueError("dim_groups must have shape [D] or [Hq, D]")
-    # one device-to-host copy instead of the reference's per-head torch.unique loop
-    table = per_head.detach().to("cpu", torch.int64)
-    if not bool(((table >= 0) & (table < gmax)).all()):
+    # one copy to the host instead of the reference's per-head torch.unique loop; the tables go back in one copy
+    with _lib.device_guard(per_head):
+        problem, dim_perm, group_start = _lib.host().group_tables(per_head, query_heads, gmax)
+    if problem == 1:
         raise ValueError("dim_groups IDs must satisfy 0 <= id < Gmax")
-    for row in table:
-        used = torch.unique(row, sorted=True)
-        if used.numel() == 0 or not torch.equal(used, torch.arange(used.numel())):
-            raise ValueError("dim_groups IDs for every query head must form a continuous prefix")
-    return dim_groups.to(dtype=torch.int32).contiguous()
+    if problem:
+        raise ValueError("dim_groups IDs for every query head must form a continuous prefix")
+    return dim_groups.to(dtype=torch.int32).contiguous(), dim_perm, group_start
 
 
 class _ExpandFactorOnDevice(torch.autograd.Function):
@@ -249,7 +257,7 @@ def oal_attention(
     ``"bf16_tensorcore"`` (default for bf16 inputs) or ``"fp32_ieee"`` (default
     otherwise).
     """
-    from .hd_block_gemm_adapters import grouped_causal_attention
+    from .hd_block_gemm_adapters import _prepare, run_prepared_grouped_hd_block_gemm
 
     q, k, v = _validate_qkv(q, k, v)
     causal, execution = _validate_public_options(causal=causal, execution=execution,
@@ -258,8 +266,8 @@ def oal_attention(
     factor, gmax = _validate_factor(factor, query_heads=q.shape[1], q_device=q.device)
     working_dtype = _resolve_working_dtype(q.dtype, factor.dtype)
     _validate_kernel_eps(kernel_eps, working_dtype=working_dtype)
-    _canonicalize_dim_groups(dim_groups, query_heads=q.shape[1], head_dimension=q.shape[-1], gmax=gmax,
-                             q_device=q.device)
+    checked = _canonical_groups_and_tables(dim_groups, query_heads=q.shape[1], head_dimension=q.shape[-1], gmax=gmax,
+                                           q_device=q.device)
     _resolve_scale(scale, q.shape[-1])
     if execution == "reference":
         raise RuntimeError("execution='reference' (the pure-torch statement) is not part of oal_b200")
@@ -271,9 +279,9 @@ def oal_attention(
         raise ValueError("oal_b200 grouped quadratic attention supports D<=64")
     if precision is None:
         precision = "bf16_tensorcore" if q.dtype == torch.bfloat16 else "fp32_ieee"
-    output, numerator, denominator = grouped_causal_attention(
-        q, k, v, dim_groups, factor, scale=scale, kernel_eps=kernel_eps, precision=precision,
-        output_dtype=output_dtype)
+    prepared = _prepare(q, k, v, checked, factor, gmax, scale=scale, kernel_eps=float(kernel_eps), precision=precision,
+                        output_dtype=output_dtype, keep_groups=False)
+    output, numerator, denominator = run_prepared_grouped_hd_block_gemm(prepared, q, k, v, factor)
     if return_unnormalized:
         return output, numerator, denominator
     return output

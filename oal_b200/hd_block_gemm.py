@@ -17,6 +17,8 @@ from __future__ import annotations
 
 import hashlib
 import json
+import threading
+from collections import OrderedDict
 from dataclasses import dataclass, field
 from math import ceil
 from typing import Sequence
@@ -247,6 +249,36 @@ def build_hd_block_gemm_plan(
     groups: int = 1,
 ) -> HDParallelBlockPlan:
     """Validate one invocation and size its workspaces (no device allocation)."""
+    arguments = locals()
+    try:      # a plan is a function of the geometry and the options alone: keep the latest ones
+        options = tuple((type(x), x) for name, x in arguments.items() if name not in ("q", "k", "v"))
+        key = (_validate_geometry(q, k, v), q.dtype, q.device, options)
+        with _PLANS_LOCK:
+            if (plan := _PLANS.get(key)) is not None:
+                _PLANS.move_to_end(key)
+                return plan
+    except (TypeError, ValueError):
+        key = None
+    plan = _build_plan(**arguments)
+    if key is not None:
+        with _PLANS_LOCK:
+            _PLANS[key] = plan
+            if len(_PLANS) > _PLANS_LIMIT:
+                _PLANS.popitem(last=False)
+    return plan
+
+
+_PLANS: OrderedDict = OrderedDict()
+_PLANS_LOCK = threading.Lock()
+_PLANS_LIMIT = 64
+
+
+def _build_plan(q, k, v, *, token_block, feature_wave_blocks, precision, result_contract, key_feature_impl, key_fold_impl,
+                query_feature_impl, query_feature_token_tile, query_fold_impl, query_fold_token_tile, query_fold_input,
+                query_gradient_flow, query_producer_fold_strategy, query_producer_partition_count, query_consumer_stages,
+                query_consumer_fusion, backward_schedule, gradient_staging, forward_normalize_impl, backward_normalize_impl,
+                kv_cross_impl, save_local_score, key_retention, output_dtype, requested_gradient_mask, memory_budget_bytes,
+                model_residency_bytes, strict_backend, feature_padding, groups) -> HDParallelBlockPlan:
     if not isinstance(result_contract, str):
         raise TypeError("result_contract must be a string")
     if result_contract != _FULL_AUX_RESULT_CONTRACT:

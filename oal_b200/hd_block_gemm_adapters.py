@@ -3,8 +3,8 @@
 Same three entry points, keyword names and return triple as the reference
 (oal_attention/hd_block_gemm_adapters.py:120-415):
 ``prepare_grouped_hd_block_gemm`` freezes geometry, groups and the plan once,
-``run_prepared_grouped_hd_block_gemm`` expands the live ``factor`` into (A, B, C)
-with differentiable torch ops and enters the autograd Function,
+``run_prepared_grouped_hd_block_gemm`` runs it on live tensors: one native autograd
+node from (q, k, v, factor) to the result triple (``csrc/oal_host.cpp``),
 ``grouped_causal_attention`` does both.
 """
 
@@ -15,6 +15,7 @@ from dataclasses import dataclass
 import torch
 
 from .grouped_quadratic import (
+    _canonical_groups_and_tables,
     _canonicalize_dim_groups,
     _expand_factor_coefficients,
     _resolve_scale,
@@ -23,14 +24,17 @@ from .grouped_quadratic import (
     _validate_kernel_eps,
     _validate_qkv,
 )
-from .hd_block_gemm import HDParallelBlockPlan, build_hd_block_gemm_plan
+from . import _lib
+from .hd_block_gemm import HDParallelBlockPlan, build_hd_block_gemm_plan, make_problem
 from .hd_block_gemm_autograd import (
     GroupTables,
+    _grad_bits,
     build_group_tables,
     hd_parallel_block_gemm,
     hd_parallel_block_gemm_autograd,
 )
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
 # oal_attention/hd_block_gemm_adapters.py:24
 _POSITIVE_FP32_FLOOR = float(torch.finfo(torch.float32).tiny * torch.finfo(torch.float32).eps)
 
@@ -54,6 +58,7 @@ class _PreparedGroupedHdBlockGemm:
     kernel_eps: float
     normalization_floor: float
     out_token_major: bool = False      # `out` is [B, N, Hq, 64] (an addition: see prepare_grouped_hd_block_gemm)
+    native: object = None              # the call as the native host path keeps it
 
 
 def prepare_grouped_hd_block_gemm(
@@ -107,15 +112,13 @@ def prepare_grouped_hd_block_gemm(
     if working_dtype != torch.float32:
         raise TypeError("grouped HD Block-GEMM requires FP32 working precision")
     resolved_eps = _validate_kernel_eps(kernel_eps, working_dtype=working_dtype)
-    canonical_groups = _canonicalize_dim_groups(dim_groups, query_heads=q.shape[1],
-                                                head_dimension=q.shape[-1], gmax=gmax, q_device=q.device)
-    gradient_mask = _requested_gradient_mask(q, k, v, coefficient_source_requires_grad=factor.requires_grad)
-    plan = build_hd_block_gemm_plan(
-        q, k, v,
+    checked = _canonical_groups_and_tables(dim_groups, query_heads=q.shape[1], head_dimension=q.shape[-1], gmax=gmax,
+                                           q_device=q.device)
+    return _prepare(
+        q, k, v, checked, factor, gmax, scale=scale, kernel_eps=resolved_eps, output_layout=output_layout,
         token_block=token_block, feature_wave_blocks=feature_wave_blocks,
         memory_budget_bytes=memory_budget_bytes, model_residency_bytes=model_residency_bytes,
-        requested_gradient_mask=gradient_mask, precision=precision,
-        key_feature_impl=key_feature_impl, key_fold_impl=key_fold_impl,
+        precision=precision, key_feature_impl=key_feature_impl, key_fold_impl=key_fold_impl,
         query_feature_impl=query_feature_impl, query_feature_token_tile=query_feature_token_tile,
         query_fold_impl=query_fold_impl, query_fold_token_tile=query_fold_token_tile,
         query_fold_input=query_fold_input, query_gradient_flow=query_gradient_flow,
@@ -124,20 +127,56 @@ def prepare_grouped_hd_block_gemm(
         backward_schedule=backward_schedule, gradient_staging=gradient_staging,
         forward_normalize_impl=forward_normalize_impl, backward_normalize_impl=backward_normalize_impl,
         kv_cross_impl=kv_cross_impl, save_local_score=save_local_score, key_retention=key_retention,
-        feature_padding=feature_padding, output_dtype=output_dtype, groups=gmax,
-    )
+        feature_padding=feature_padding, output_dtype=output_dtype)
+
+
+def _prepare(q, k, v, checked, factor, gmax, *, scale, kernel_eps, output_layout="heads_first", keep_groups=True,
+             **plan_options):
+    """The preparation of validated arguments; ``checked``: canonical groups and their device tables.
+    ``keep_groups``: the preparation outlives this call, so it takes a copy of the caller's group ids."""
+    canonical_groups, dim_perm, group_start = checked
+    gradient_mask = _requested_gradient_mask(q, k, v, coefficient_source_requires_grad=factor.requires_grad)
+    plan = build_hd_block_gemm_plan(q, k, v, requested_gradient_mask=gradient_mask, groups=gmax, **plan_options)
     groups = (canonical_groups.unsqueeze(0).expand(q.shape[1], -1)
-              if canonical_groups.ndim == 1 else canonical_groups).detach().clone()
+              if canonical_groups.ndim == 1 else canonical_groups).detach()
+    if keep_groups:
+        groups = groups.clone()
+    tables, resolved_eps = GroupTables(dim_perm, group_start, gmax), kernel_eps
+    resolved_scale, token_major = _resolve_scale(scale, q.shape[-1]), output_layout == "tokens_first"
     return _PreparedGroupedHdBlockGemm(
-        plan=plan, groups=groups, tables=build_group_tables(groups, gmax), gmax=gmax,
-        scale=_resolve_scale(scale, q.shape[-1]), kernel_eps=resolved_eps,
-        normalization_floor=_POSITIVE_FP32_FLOOR, out_token_major=output_layout == "tokens_first")
+        plan=plan, groups=groups, tables=tables, gmax=gmax, scale=resolved_scale, kernel_eps=resolved_eps,
+        normalization_floor=_POSITIVE_FP32_FLOOR, out_token_major=token_major,
+        native=_native_call(plan, tables, resolved_scale, resolved_eps, token_major, q))
+
+
+def _native_call(plan, tables, scale, kernel_eps, token_major, q):
+    """Hand the frozen call to the native host path; None for tensors it does not run on."""
+    if q.device.type != "cuda":
+        return None
+    out_dtype = getattr(torch, plan.output_dtype)
+    mask = plan.requested_gradient_mask
+    problem = make_problem(plan.geometry, groups=tables.group_count, io_dtype=q.dtype,
+                           out_dtype=out_dtype if out_dtype != torch.float64 else torch.float32, precision=plan.precision,
+                           chunk=plan.chunk_tokens, scale=scale, floor=_POSITIVE_FP32_FLOOR, grad_mask=_grad_bits(mask),
+                           flags=_lib.FLAG_ZERO_STATE_IN | (_lib.FLAG_OUT_TOKEN_MAJOR if token_major else 0))
+    if token_major and plan.geometry[5] != _lib.HEAD_DIM:
+        return None                     # refused where the call runs
+    return _lib.host().prepare(bytes(problem), list(plan.geometry), tables.group_count, q.dtype, out_dtype, q.device.index,
+                               tables.dim_perm, tables.group_start, kernel_eps,
+                               [plan.forward_workspace_bytes, plan.backward_workspace_bytes, plan.saved_state_bytes],
+                               [mask[0], mask[1], mask[2], any(mask[3:])])
 
 
 def run_prepared_grouped_hd_block_gemm(prepared, q, k, v, factor):
     """Run one live invocation against an explicit immutable preparation."""
     if not isinstance(prepared, _PreparedGroupedHdBlockGemm):
         raise TypeError("prepared must be an explicit grouped HD Block-GEMM preparation")
+    if prepared.native is not None and all(type(t) in _PLAIN for t in (q, k, v, factor)):
+        with _lib.device_guard(q):
+            result = _lib.host().run(prepared.native, q, k, v, factor)
+        if result is not None:
+            return result
+    # not the prepared call (or not plain tensors): find out what does not match
     q, k, v = _validate_qkv(q, k, v)
     factor, gmax = _validate_factor(factor, query_heads=q.shape[1], q_device=q.device)
     if gmax != prepared.gmax:

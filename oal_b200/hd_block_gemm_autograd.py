@@ -15,7 +15,6 @@ the adapters, as in the reference (hd_block_gemm_adapters.py:278-301).
 from __future__ import annotations
 
 import ctypes
-import itertools
 import threading
 from dataclasses import dataclass
 from typing import Any
@@ -109,7 +108,6 @@ def raise_on_status(status: torch.Tensor) -> None:
 # make before an optimizer step consumes the gradients.  Every error names the call it belongs to.
 _PENDING: dict = {}
 _PENDING_LOCK = threading.Lock()
-_CALL_IDS = itertools.count(1)
 _PENDING_LIMIT = 256          # a ticket stays valid for 1023 later ones on its device: drain well before that
 
 
@@ -142,9 +140,17 @@ class PendingStatus:
 _CAPTURED: dict = {}
 
 
+def _collect_captured() -> None:
+    """Take over the words of calls that the native host path recorded."""
+    for index, word, what in _lib.host().take_captured():
+        with _PENDING_LOCK:
+            _CAPTURED.setdefault(index, []).append((word, what))
+
+
 def check_captured_status(device=None) -> None:
     """One host synchronisation: raise if any call recorded into a CUDA graph on ``device`` (default: every
     device) reported a problem in the replays so far.  Call it where a training loop synchronises anyway."""
+    _collect_captured()
     with _PENDING_LOCK:
         keys = list(_CAPTURED) if device is None else [torch.device(device).index if not isinstance(device, int) else device]
         words = [(w, what) for key in keys for w, what in _CAPTURED.get(key, [])]
@@ -157,6 +163,7 @@ def check_captured_status(device=None) -> None:
 
 def forget_captured_status(device=None) -> None:
     """Drop the recorded words (when the graphs that own them are destroyed)."""
+    _collect_captured()
     with _PENDING_LOCK:
         if device is None:
             _CAPTURED.clear()
@@ -185,7 +192,7 @@ def defer_status(status: torch.Tensor, what: str = "forward", *, guarded: bool =
         with _lib.device_guard(status):
             rc = lib.oal_status_defer(_lib.ptr(status), _stream_ptr(device), ctypes.byref(ticket))
     _lib.check(rc)
-    entry = PendingStatus(int(ticket.value), next(_CALL_IDS), what, device_word=status)
+    entry = PendingStatus(int(ticket.value), _lib.host().next_call_id(), what, device_word=status)
     with _PENDING_LOCK:
         queue = _PENDING.setdefault(device.index, [])
         queue.append(entry)
@@ -202,6 +209,8 @@ def check_pending_status(block: bool = False, device=None) -> None:
     drained completely (call it before an optimizer step when a forward ran without its backward)."""
     if torch.cuda.is_current_stream_capturing():
         return                  # no event may be queried while a stream is capturing
+    index = device if device is None or isinstance(device, int) else torch.device(device).index
+    _lib.host().check_pending(block, -1 if index is None else index)
     with _PENDING_LOCK:
         keys = list(_PENDING) if device is None else [torch.device(device).index if not isinstance(device, int) else device]
     for key in keys:
