@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   __shared__ float den_s[CT];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int kvh = h / (a.Hq / a.Hkv);
   const int half = (warp >> 2) & 1, row = 32 * (warp & 3) + lane;
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
   async_copies_wait();
   __syncthreads();
   const int tiles = min(CT / KT, (a.N - c * CT + KT - 1) / KT);
-  const int rank = hf.rank, rpos = hf.rpos;
+  const int rank = uniform(hf.rank), rpos = uniform(hf.rpos);
   const f32x2 w0 = f2_bcast(hf.w0);
   const bool cross = c >= a.cross_from;
   init_stack_constants(St, hf, tid, CTHREADS);
@@ -84,13 +84,14 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
-  const uint32_t tU = tmem_base + FWD_TMEM_U, tY = tmem_base + FWD_TMEM_Y, tWt = tmem_base + FWD_TMEM_W;
+  const uint32_t tmem = uniform(tmem_base);
+  const uint32_t tU = tmem + FWD_TMEM_U, tY = tmem + FWD_TMEM_Y, tWt = tmem + FWD_TMEM_W;
   const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
 
   const uint32_t q_addr = smem_u32(Qa), u_addr = smem_u32(Uimg), st_addr = smem_u32(St);
   const uint32_t idesc_y = instr_desc_bf16(128, EP, 0, 1);
   if (issuer) {
-    if (lane == 0) {
+    if (elect_one()) {
       issue_stack_scores(tU, q_addr, st_addr, rank);
       mma_commit(&u_done);
     }
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
     fence_before_sync();
     warp_arrive(&u_free, lane);
     if (issuer && kt + 1 < tiles) {
-      if (lane == 0) {
+      if (elect_one()) {
         w.wait(&u_free, kt & 1, 0x11);                                   // every warp holds U(kt)
         if (kt + 1 >= 2) w.wait(&st_ready[(kt + 1) & 1], ((kt - 1) >> 1) & 1, 0x12);
         fence_after_sync();
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(CTHREADS, 2) intra_fwd_kernel(const IntraFwdAr
       warp_arrive(&st_ready[buf], lane);
     }
     if (issuer) {
-      if (lane == 0) {
+      if (elect_one()) {
         w.wait(&w_ready[buf], (kt >> 1) & 1, 0x13);
         fence_after_sync();
         mma_bf16_ts(tY, tWt + buf * (KT / 2), smem_desc(u_addr + kt * KT * 16, 128, CT * 16), idesc_y, kt > 0);

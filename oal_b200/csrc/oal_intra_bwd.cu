@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) intra_bwd_q_kernel(const IntraBwd
   __shared__ uint64_t gfull, dw_done, u_done, u_free, p_ready[2], p_done[2], st_ready[3];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int kvh = h / (a.Hq / a.Hkv);
   const int half = (warp >> 2) & 1, row = 32 * (warp & 3) + lane;
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) intra_bwd_q_kernel(const IntraBwd
   async_copies_wait();
   __syncthreads();
   const int tiles = min(CT / KT, (a.N - c * CT + KT - 1) / KT);
-  const int rank = hf.rank, rpos = hf.rpos;
+  const int rank = uniform(hf.rank), rpos = uniform(hf.rpos);
   for (int s = 0; s < 3; ++s) init_stack_constants(St + s * ST_BYTES, hf, tid, CTHREADS);
   if ((tid >> 7) < tiles)
     build_stack_piece(St + (tid >> 7) * ST_BYTES, Kimg, (tid >> 7) * KT, hf, tid & 127, Lo + (tid >> 7) * STLO_BYTES);
@@ -112,7 +112,8 @@ __global__ void __launch_bounds__(CTHREADS, 1) intra_bwd_q_kernel(const IntraBwd
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
-  const uint32_t tU = tmem_base, tW = tmem_base + RM * KT, tQ = tW + CT, tP = tQ + HD;
+  const uint32_t tmem = uniform(tmem_base);
+  const uint32_t tU = tmem, tW = tmem + RM * KT, tQ = tW + CT, tP = tQ + HD;
   const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
   f32x2 D2[NU], N2[RM], S2 = 0ull;
 #pragma unroll
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) intra_bwd_q_kernel(const IntraBwd
 
   const uint32_t q_addr = smem_u32(Qa), st_addr = smem_u32(St), lo_addr = smem_u32(Lo);
   if (issuer) {
-    if (lane == 0) {
+    if (elect_one()) {
       w.wait(&gfull, 0, 0x20);
       fence_after_sync();
       issue_dw(tW, smem_u32(Gimg), true, smem_u32(Uimg), false);
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) intra_bwd_q_kernel(const IntraBwd
     fence_before_sync();
     warp_arrive(&u_free, lane);
     if (issuer && kt + 1 < tiles) {
-      if (lane == 0) {
+      if (elect_one()) {
         w.wait(&u_free, kt & 1, 0x21);                 // every warp holds U(kt)
         if (kt + 1 >= 2) w.wait(&st_ready[(kt + 1) % 3], ((kt - 1) / 3) & 1, 0x22);
         fence_after_sync();
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) intra_bwd_q_kernel(const IntraBwd
       warp_arrive(&st_ready[(kt + 2) % 3], lane);
     }
     if (issuer) {
-      if (lane == 0) {
+      if (elect_one()) {
         w.wait(&p_ready[buf], (kt >> 1) & 1, 0x23);     // P tile of tile kt is in shared memory
         fence_after_sync();
         issue_stack_grad(tQ, tP + buf * P_COLS, st_addr + (kt % 3) * ST_BYTES, rank, kt > 0);
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const Intra
   __shared__ uint64_t gfull, dw_done, u_done, u_free, p_ready, p_done, st_ready[3];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int kvh = h / (a.Hq / a.Hkv);
   const int part = warp >> 2, row = 32 * (warp & 3) + lane;       // row = key index inside the chunk; part = 4 queries of a tile
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const Intra
   async_copies_wait();
   __syncthreads();
   const int tiles = min(CT / KT, (a.N - c * CT + KT - 1) / KT);
-  const int rank = hf.rank, rpos = hf.rpos;
+  const int rank = uniform(hf.rank), rpos = uniform(hf.rpos);
   const f32x2 w0 = f2_bcast(hf.w0);
   for (int s = 0; s < 3; ++s) init_stack_constants(St + s * ST_BYTES, hf, tid, KV_THREADS);
   if (tid < 256 && (tid >> 7) < tiles)
@@ -366,13 +367,14 @@ __global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const Intra
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
-  const uint32_t tU = tmem_base, tW = tmem_base + RM * KT, tK = tW + CT, tV = tK + HD, tP = tV + EP, tWt = tP + P_COLS;
+  const uint32_t tmem = uniform(tmem_base);
+  const uint32_t tU = tmem, tW = tmem + RM * KT, tK = tW + CT, tV = tK + HD, tP = tV + EP, tWt = tP + P_COLS;
   const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
 
   const uint32_t k_addr = smem_u32(Ka), st_addr = smem_u32(St), g_addr = smem_u32(Ghi), lo_addr = smem_u32(Lo);
   const uint32_t idesc_du = instr_desc_bf16(128, EP, 0, 1);
   if (issuer) {
-    if (lane == 0) {
+    if (elect_one()) {
       w.wait(&gfull, 0, 0x30);
       fence_after_sync();
       // dW^T[j, i] = [v|1]_j . g_i: rows from the U image, columns from the hi and lo images of G
@@ -400,7 +402,7 @@ __global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const Intra
     fence_before_sync();
     warp_arrive(&u_free, lane);
     if (issuer && qt + 1 < tiles) {
-      if (lane == 0) {
+      if (elect_one()) {
         w.wait(&u_free, qt & 1, 0x31);
         if (qt + 1 >= 2) w.wait(&st_ready[(qt + 1) % 3], ((qt - 1) / 3) & 1, 0x32);
         fence_after_sync();
@@ -469,7 +471,7 @@ __global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const Intra
       warp_arrive(&st_ready[(qt + 2) % 3], lane);
     }
     if (issuer) {
-      if (lane == 0) {
+      if (elect_one()) {
         w.wait(&p_ready, qt & 1, 0x33);
         fence_after_sync();
         issue_stack_grad(tK, tP, st_addr + (qt % 3) * ST_BYTES, rank, qt > 0);

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   __shared__ uint64_t mma_done[2];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int item = (int)blockIdx.x - n_prologue;
   const int grp = item % SU_GROUPS, c = (item / SU_GROUPS) % a.NC, u = item / SU_GROUPS / a.NC;
   const int token = tid & 127, half = tid >> 7;
@@ -103,7 +103,8 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
-  const uint32_t tacc = tmem_base;
+  const uint32_t tmem = uniform(tmem_base);
+  const uint32_t tacc = tmem;
   const int s0 = group_first_slab(grp), ns = group_slab_count(grp);
   const uint32_t idesc = instr_desc_bf16(128, EP, 1, 1);
   const uint32_t u_addr = smem_u32(Uimg);
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
     write_half_slab_raw(s0 + it, half, xp, reinterpret_cast<uint4*>(Abuf + buf * SLAB_A_BYTES) + token);
     fence_async_smem();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       fence_after_sync();
       const uint64_t da = smem_desc(smem_u32(Abuf + buf * SLAB_A_BYTES), 128, CT * 16);
       const uint64_t du = smem_desc(u_addr, 128, CT * 16);
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
   __shared__ uint64_t coef_full[2], coef_free[2];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int n_items = a.B * a.H * a.NC;
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   if (warp == CR_ISSUER) tmem_alloc(&tmem_base, 256);
@@ -284,6 +285,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
+  const uint32_t tmem = uniform(tmem_base);
 
   if (warp < CR_GEN_WARPS) {
     // ---------------- generators: thread = (token, half of the slab's chunks) ----------------
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
       const size_t orow = (size_t)(it.b * a.H + it.h) * a.N + row;
       w.wait(&acc_full[k & 1], (k >> 1) & 1, 0x42);
       fence_after_sync();
-      const uint32_t t = tmem_base + (k & 1) * EP + lane_off;
+      const uint32_t t = tmem + (k & 1) * EP + lane_off;
 #pragma unroll
       for (int cc = 0; cc < EP; cc += 16) {
         if (cc < VD || QUERY) {
@@ -352,13 +354,13 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
     }
   } else if (warp == CR_ISSUER) {
     // ---------------- MMA issue ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc_bf16(128, EP, 0, 1);
       // descriptors of slot 0 of both rings, advanced by adds: this thread is the serial path of every slab
       const uint64_t da0 = smem_desc(smem_u32(Abuf), CT * 16, 128), ds0 = smem_desc(smem_u32(Sbuf), 128, 128 * 16);
       int s3 = 0, use = 0, gs = 0, guse = 0;
       for (int k = 0; k < my_items; ++k) {
-        const uint32_t tacc = tmem_base + (k & 1) * EP;
+        const uint32_t tacc = tmem + (k & 1) * EP;
         if (k >= 2) w.wait(&acc_free[k & 1], ((k >> 1) - 1) & 1, 0x43);   // item k-2 has left this accumulator
         for (int s = 0; s < F_SLABS; ++s) {
           const uint64_t da = desc_advance(da0, s3 * SLAB_A_BYTES), dsl = desc_advance(ds0, gs * SLAB_S_BYTES);
@@ -379,7 +381,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
     __syncwarp();
   } else {
     // ---------------- state image stream ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int gs = 0, guse = 0;
       for (int k = 0; k < my_items; ++k) {
         const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);

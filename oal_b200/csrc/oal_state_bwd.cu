@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
   __shared__ uint64_t full_a[DS_RING], mma_done[DS_RING], z_free[DS_RING], g_full[DS_GRING], g_free[DS_GRING];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int rep = a.Hq / a.Hkv;
   const int n_items = F_SLABS * a.NC * a.units;
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
+  const uint32_t tmem = uniform(tmem_base);
 
   if (warp < DS_GEN_WARPS) {
     // ---------------- generators ----------------
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
       }
       w.wait(&mma_done[s], use & 1, 0x32);
       fence_after_sync();
-      const uint32_t tz = tmem_base + EP * s + col0;
+      const uint32_t tz = tmem + EP * s + col0;
       if (d.hh == 0) {
 #pragma unroll
         for (int j = 0; j < DS_COLS / 2; ++j) acc[j] = 0ull;
@@ -253,14 +254,14 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
     }
   } else if (warp == DS_ISSUER) {
     // ---------------- MMA issue ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc_bf16(128, EP, 1, 1);
       // descriptors of slot 0 of both rings, advanced by adds: this thread is the serial path of every slab
       const uint64_t da0 = smem_desc(smem_u32(Abuf), 128, CT * 16), dg0 = smem_desc(smem_u32(Gbuf), 128, CT * 16);
       int s = 0, use = 0, gs = 0, guse = 0;
       for (int it = 0; it < T; ++it) {
         const uint64_t da = desc_advance(da0, s * SLAB_A_BYTES), dg = desc_advance(dg0, gs * SLAB_S_BYTES);
-        const uint32_t tz = tmem_base + EP * s;
+        const uint32_t tz = tmem + EP * s;
         w.wait(&full_a[s], use & 1, 0x33);
         w.wait(&g_full[gs], guse & 1, 0x34);
         if (use > 0) w.wait(&z_free[s], (use - 1) & 1, 0x35);
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
     __syncwarp();
   } else {
     // ---------------- G image stream ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       DsCursor d;
       d.start(a.c0, a.NC, a.Hkv, rep);
       int gs = 0, guse = 0;
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
   __shared__ uint64_t d_full[FG_DRING], d_free[FG_DRING];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int n_items = a.B * a.H * a.NC;
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   if (warp == FG_ISSUER) tmem_alloc(&tmem_base, 512);
@@ -467,6 +468,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
+  const uint32_t tmem = uniform(tmem_base);
 
   if (warp < FG_FOLD_WARPS) {
     // ---------------- fold warps ----------------
@@ -502,7 +504,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
       for (int s = 0; s < F_SLABS; ++s) {
         w.wait(&d_full[ds], duse & 1, 0x53);
         fence_after_sync();
-        fold_half_slab<QUERY>(s, wg, tmem_base + ds * 128 + lane_off, xq, coef, dxq);
+        fold_half_slab<QUERY>(s, wg, tmem + ds * 128 + lane_off, xq, coef, dxq);
         fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&d_free[ds]);
@@ -533,7 +535,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
     }
   } else if (warp == FG_ISSUER) {
     // ---------------- MMA issue ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc_bf16(128, 128, 0, 0);
       const uint64_t da0 = smem_desc(smem_u32(Aimg), CT * 16, 128), ds0 = smem_desc(smem_u32(Sbuf), 128 * 16, 128);
       int gs = 0, guse = 0, ds = 0, duse = 0;
@@ -547,7 +549,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
           fence_after_sync();
 #pragma unroll
           for (int ks = 0; ks < EP / 16; ++ks)
-            mma_bf16_ss(tmem_base + ds * 128, desc_advance(da, ks * 2 * CT * 16), desc_advance(dsl, ks * 2 * 128 * 16), idesc,
+            mma_bf16_ss(tmem + ds * 128, desc_advance(da, ks * 2 * CT * 16), desc_advance(dsl, ks * 2 * 128 * 16), idesc,
                         ks > 0);
           mma_commit(&d_full[ds]);
           mma_commit(&s_free[gs]);
@@ -560,7 +562,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
     __syncwarp();
   } else {
     // ---------------- image / table stream ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int gs = 0, guse = 0;
       for (int k = 0; k < my_items; ++k) {
         const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);

@@ -51,6 +51,28 @@ __host__ __device__ constexpr uint32_t instr_desc_bf16(int m, int n, int a_major
          | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// The operands of the tensor-core and bulk-copy instructions (descriptors, tensor-memory and barrier addresses) are
+// warp-uniform registers.  A thread that issues them should therefore run in code the compiler can see to be
+// warp-uniform: one elected lane of a converged warp, the warp index and everything read from shared memory passed
+// through uniform().  Measured, one warp issuing back to back: 154 clocks per MMA of any size when the address
+// comes from a shared-memory load in a branch on threadIdx, 41 / 53 / 72 / 123 clocks for N = 16 / 80 / 144 / 256
+// (A and B in shared memory, M = 128, K = 16) when it does not, which is what the operand reads (128 bytes per
+// clock) and the tensor pipe allow.
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t yes;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(yes));
+  return yes != 0;
+}
+
 // ---- TMEM ----------------------------------------------------------------------
 // One full warp allocates `cols` (power of two >= 32) columns; the base address is
 // written to *dst_smem.
