@@ -210,9 +210,8 @@ int check_problem(const OalProblem* p) {
   }
   if (!(p->floor > 0.f)) return fail(OAL_ERR_ARGUMENT, "floor must be positive");
   if (p->flags & ~(OAL_FLAG_OUT_TOKEN_MAJOR | OAL_FLAG_ZERO_STATE_IN)) return fail(OAL_ERR_ARGUMENT, "unknown bits in flags");
-  if ((p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) &&
-      (p->precision != OAL_PRECISION_BF16_TENSORCORE || p->groups + 1 > oal::intra_coef_terms()))
-    return fail(OAL_ERR_ARGUMENT, "token-major out needs bf16_tensorcore and at most 8 groups per head");
+  if ((p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) && p->precision != OAL_PRECISION_BF16_TENSORCORE)
+    return fail(OAL_ERR_ARGUMENT, "token-major out needs bf16_tensorcore");
   return OAL_OK;
 }
 
@@ -286,9 +285,6 @@ struct ForwardSpaceTC {
   size_t bytes;
 };
 
-// the intra-chunk term runs on the tensor cores for heads with at most 8 groups (else token-pair kernels)
-bool tc_intra(const OalProblem* p) { return p->groups + 1 <= oal::intra_coef_terms(); }
-
 int make_head_factors(const OalProblem* p, const int32_t* dim_perm, const int32_t* group_start, const float* coef_a,
                       const float* coef_b, const float* coef_c, void* factors, cudaStream_t st, bool timing = true) {
   LaunchScope scope("head_factors", st, 1, timing);
@@ -327,8 +323,7 @@ float* saved_coef_table(const OalProblem* p, const void* saved_state) {
 }
 
 struct BackwardSpaceTC {
-  float* g;
-  float* coef_pairs;
+  float* coef_blocks;            // coefficient partial sums of the query row blocks
   void* gimg;
   float* dcarry;
   void* dt_img;
@@ -336,7 +331,7 @@ struct BackwardSpaceTC {
   float* dcoef;
   float* slots;
   float *dq_cross, *dk_cross, *dv_cross;
-  float *dk_part, *dv_part;      // per-query-head intra-chunk shares of dk / dv
+  float *dk_part, *dv_part;      // shares of dk / dv of groups of query heads
   float* dcoefs;                 // dA, dB, dC of a call whose caller asks for the factor's gradient
   size_t bytes;
 };
@@ -348,8 +343,7 @@ BackwardSpaceTC carve_backward_tc(const OalProblem* p, void* ws) {
   const size_t qrows = (size_t)p->batch * p->q_heads * p->seq_len;
   const size_t krows = (size_t)p->batch * p->kv_heads * p->seq_len;
   const size_t slab_image = oal::state_slab_image_bytes();
-  s.g = c.take<float>(qrows * oal::EP);
-  s.coef_pairs = c.take<float>((size_t)p->batch * p->q_heads * oal::pairs_tiles(p->seq_len) * oal::NCOEF);
+  s.coef_blocks = c.take<float>((size_t)p->batch * p->q_heads * oal::intra_row_blocks(p->seq_len) * oal::NQ_ALL);
   s.gimg = c.take<char>(2 * (size_t)p->batch * p->q_heads * nb * slab_image);   // hi image, then lo image
   s.dcarry = c.take<float>(units * nb * oal::state_rows() * oal::EP);
   s.dt_img = c.take<char>(units * nb * oal::state_image_bytes_per_chunk());
@@ -371,9 +365,8 @@ BackwardSpaceTC carve_backward_tc(const OalProblem* p, void* ws) {
 int backward_vjp(const OalProblem* p, const float* num, const float* den, const void* grad_out, const float* grad_num,
                  const float* grad_den, const BackwardSpaceTC& s, int32_t* clear_status, cudaStream_t st) {
   LaunchScope scope("norm_vjp", st);
-  // the fp32 rows of g are read by the token-pair kernels only (heads with more than 8 groups)
   const cudaError_t e = oal::norm_vjp_image(grad_out, p->out_dtype, grad_num, grad_den, num, den, p->floor,
-                                            tc_intra(p) ? nullptr : s.g, s.gimg, p->batch * p->q_heads, p->seq_len, chunk_count(p),
+                                            s.gimg, p->batch * p->q_heads, p->seq_len, chunk_count(p),
                                             (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) ? p->q_heads : 0, clear_status, st);
   return e == cudaSuccess ? OAL_OK : fail_cuda(e, "normalisation VJP kernel");
 }
@@ -394,7 +387,6 @@ oal::PairArgs base_args(const OalProblem* p, const void* q, const void* k, const
   oal::PairArgs a;
   memset(&a, 0, sizeof(a));
   a.B = p->batch; a.Hq = p->q_heads; a.Hkv = p->kv_heads; a.N = p->seq_len; a.G = p->groups;
-  a.window = 0;
   a.io_dt = p->io_dtype; a.out_dt = p->out_dtype;
   a.scale = p->scale; a.floor = p->floor;
   a.q = q; a.k = k; a.v = v;
@@ -409,13 +401,13 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
                  const int32_t* group_start, const CoefSource& src, void* out, float* num, float* den, void* saved_state,
                  const float* state_in, float* ds, int32_t* status, oal::StatusSink sink, bool timing, cudaStream_t st) {
   cudaError_t e;
-  const bool tc_mode = p->precision == OAL_PRECISION_BF16_TENSORCORE, tc = tc_mode && tc_intra(p);
+  const bool tc = p->precision == OAL_PRECISION_BF16_TENSORCORE;
   const int units = p->batch * p->kv_heads, nb = chunk_count(p);
   const ChunkRange cr = chunk_range(p, state_in, nullptr);
   const bool reuse = p->grad_mask & OAL_GRAD_REUSE_STATE_STAGE;      // increments left by oal_forward_local_state
-  const bool update = tc_mode && !reuse && cr.n > 0;
+  const bool update = tc && !reuse && cr.n > 0;
   void* factors = tc ? saved_factors(p, saved_state) : nullptr;
-  float* coef_table = tc_mode ? saved_coef_table(p, saved_state) : nullptr;
+  float* coef_table = tc ? saved_coef_table(p, saved_state) : nullptr;
   std::unique_lock<std::mutex> side_lock;
   SideStreams* side = nullptr;
   cudaStream_t s0 = st;
@@ -426,15 +418,13 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
       LaunchScope scope("head_prologue", st, 1, timing);
       if ((e = oal::launch_head_prologue(pro, p->q_heads, st)) != cudaSuccess) return fail_cuda(e, "prologue kernel");
     }
-  } else if (tc_mode) {
+  } else if (tc) {
     // explicit coefficients: the factor table (rotations of a possibly indefinite matrix, 50 us) is needed by the
     // last kernel only and is computed beside the state kernels
-    if (tc) {
-      if (timing) side = side_streams(side_lock);
-      s0 = fork_to(side, 0, st);
-      if (int rc = make_head_factors(p, dim_perm, group_start, src.A, src.B, src.C, factors, s0, timing)) return rc;
-      join_mark(side, 0, s0, st);
-    }
+    if (timing) side = side_streams(side_lock);
+    s0 = fork_to(side, 0, st);
+    if (int rc = make_head_factors(p, dim_perm, group_start, src.A, src.B, src.C, factors, s0, timing)) return rc;
+    join_mark(side, 0, s0, st);
     LaunchScope scope("coef_table", st, 1, timing);
     e = oal::build_coef_table(dim_perm, group_start, src.A, src.B, src.C, p->q_heads, p->groups, p->scale, coef_table, st);
     if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
@@ -444,7 +434,7 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
     e = oal::state_update(k, v, ds, units, p->seq_len, nb, cr.n, src.factor ? &pro : nullptr, p->q_heads, status, st);
     if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
   }
-  if (tc_mode && cr.n > 0) {
+  if (tc && cr.n > 0) {
     { LaunchScope scope("state_scan", st, 1, timing);
       e = oal::state_scan(ds, saved_state, saved_remainders(p, saved_state), state_in, nullptr, units, nb, 0, cr.trim, st); }
     if (e != cudaSuccess) return fail_cuda(e, "state scan kernel");
@@ -456,15 +446,12 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
   if (tc) {
     join_wait(side, 0, s0, st);
     LaunchScope scope("intra_forward", st, 1, timing);
-    e = oal::intra_forward(q, k, v, factors, out, num, den, status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb,
+    e = oal::intra_forward(q, k, v, factors, out, num, den, status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb, p->groups,
                            p->out_dtype, p->floor, (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) != 0, cr.first, sink, st);
     return e == cudaSuccess ? OAL_OK : fail_cuda(e, "intra-chunk forward kernel");
   }
   oal::PairArgs a = base_args(p, q, k, v, dim_perm, group_start, src, status);
-  a.window = tc_mode ? kChunk : 0;
   a.out = out; a.num = num; a.den = den;
-  a.accumulate = tc_mode ? 1 : 0;
-  a.accumulate_from = cr.first * kChunk;
   a.sink = sink;
   LaunchScope scope("pairs_forward", st, 1, timing);
   e = oal::pairs_forward(a, st);
@@ -478,8 +465,8 @@ int finish_coefs(const OalProblem* p, const CoefSource& src, const CoefSink& sin
   cudaError_t e;
   const bool fused = factors && sink.dfactor && src.factor_rows == p->q_heads;
   { LaunchScope scope("reduce_coefs", st);
-    const int rm = oal::intra_coef_terms();
-    e = factors ? oal::intra_coef_finish(partial, chunk_count(p), rm * (rm + 1) / 2 + rm + 1, rm, factors, slots, p->batch,
+    const int rm = p->groups + 1;
+    e = factors ? oal::intra_coef_finish(partial, oal::intra_row_blocks(p->seq_len), rm * (rm + 1) / 2 + rm + 1, rm, factors, slots, p->batch,
                                          p->q_heads, p->groups, sink.dA, sink.dB, sink.dC, fused ? src.factor : nullptr,
                                          fused ? sink.dfactor : nullptr, st)
                 : oal::reduce_coefs(partial, oal::pairs_tiles(p->seq_len), slots, p->batch, p->q_heads, p->groups,
@@ -553,7 +540,6 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   const int nb = chunk_count(p), units = p->batch * p->kv_heads, rep = p->q_heads / p->kv_heads;
   const bool want_q = mask & OAL_GRAD_Q, want_k = mask & OAL_GRAD_K, want_v = mask & OAL_GRAD_V, want_kv = want_k || want_v;
   const bool want_c = mask & OAL_GRAD_COEF;
-  const bool tc = tc_intra(p);                // intra-chunk term on the tensor cores (else token-pair kernels)
   const bool reuse = mask & OAL_GRAD_REUSE_STATE_STAGE;
   const ChunkRange cr = chunk_range(p, nullptr, x.dstate_in);
   const void* factors = saved_factors(p, x.saved_state);      // written by the forward of this call
@@ -571,11 +557,6 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   const bool cross = cr.n > 0;
   cudaStream_t skv = want_kv ? fork_to(side, 0, st) : st;
   cudaStream_t sc = want_c && cross ? fork_to(side, 1, st) : st;
-  oal::PairArgs a = base_args(p, x.q, x.k, x.v, x.dim_perm, x.group_start, src, x.status);
-  a.window = kChunk;
-  a.g = s.g;
-  a.q_init_from = cr.first * kChunk;
-  a.kv_init_end = cr.n * kChunk;
   if (want_c && cross) {
     { LaunchScope scope("dcoef_reduce", sc, 2);
       e = oal::dcoef_reduce(s.dcoef_partial, 2 * p->batch * cr.n, p->q_heads, p->groups, x.dim_perm, x.group_start, s.dcoef, s.slots, sc); }
@@ -606,45 +587,24 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
     if (e != cudaSuccess) return fail_cuda(e, "query feature gradient kernel");
   }
   if (want_q || want_c) {
-    if (tc) {
-      { LaunchScope scope("intra_backward_q", st);
-        e = oal::intra_backward_q(x.q, x.k, x.v, s.gimg, factors, want_q ? x.dq : nullptr, want_q ? s.dq_cross : nullptr,
-                                  want_c ? s.coef_pairs : nullptr, x.status, p->batch, p->q_heads, p->kv_heads,
-                                  p->seq_len, nb, cr.first, st); }
-      if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward query-side kernel");
-    } else {
-      a.dq = want_q ? x.dq : nullptr;
-      a.dq_init = want_q ? s.dq_cross : nullptr;
-      a.coef_partial = want_c ? s.coef_pairs : nullptr;
-      { LaunchScope scope("pairs_backward_q", st); e = oal::pairs_backward_q(a, st); }
-      if (e != cudaSuccess) return fail_cuda(e, "backward query-side pair kernel");
-    }
+    { LaunchScope scope("intra_backward_q", st);
+      e = oal::intra_backward_q(x.q, x.k, x.v, s.gimg, factors, want_q ? x.dq : nullptr, want_q ? s.dq_cross : nullptr,
+                                want_c ? s.coef_blocks : nullptr, x.status, p->batch, p->q_heads, p->kv_heads,
+                                p->seq_len, nb, p->groups, cr.first, st); }
+    if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward query-side kernel");
   }
   if (want_kv) {
     // the two intra-chunk kernels each fill the machine: the key/value one is queued after the query one
-    if (tc) {
-      { LaunchScope scope("intra_backward_kv", skv);
-        e = oal::intra_backward_kv(x.q, x.k, x.v, s.gimg, factors, want_k ? s.dk_part : nullptr, want_v ? s.dv_part : nullptr,
-                                   x.status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb, skv); }
-      if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward key/value-side kernel");
-      { LaunchScope scope("kv_head_reduce", skv);
-        e = oal::kv_head_reduce(s.dk_part, s.dv_part, s.dk_cross, s.dv_cross, want_k ? x.dk : nullptr, want_v ? x.dv : nullptr,
-                                p->batch, p->q_heads, p->kv_heads, p->seq_len, cr.n * kChunk, skv); }
-      if (e != cudaSuccess) return fail_cuda(e, "key/value head reduction kernel");
-    } else {
-      a.dq = nullptr; a.dq_init = nullptr; a.coef_partial = nullptr;
-      a.dk = want_k ? x.dk : nullptr;
-      a.dv = want_v ? x.dv : nullptr;
-      a.dk_init = want_k ? s.dk_cross : nullptr;
-      a.dv_init = want_v ? s.dv_cross : nullptr;
-      { LaunchScope scope("pairs_backward_kv", skv); e = oal::pairs_backward_kv(a, skv); }
-      if (e != cudaSuccess) return fail_cuda(e, "backward key/value-side pair kernel");
-    }
+    { LaunchScope scope("intra_backward_kv", skv, oal::intra_kv_parts(p->batch, p->q_heads, p->kv_heads, nb) > 1 ? 2 : 1);
+      e = oal::intra_backward_kv(x.q, x.k, x.v, s.gimg, factors, want_k ? x.dk : nullptr, want_v ? x.dv : nullptr, s.dk_cross,
+                                 s.dv_cross, cr.n * kChunk, s.dk_part, s.dv_part, x.status, p->batch, p->q_heads, p->kv_heads,
+                                 p->seq_len, nb, p->groups, skv); }
+    if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward key/value-side kernels");
     join_mark(side, 0, skv, st);
   }
   if (want_c) {
     if (cross) join_wait(side, 1, sc, st);
-    if (int rc = finish_coefs(p, src, sink, s.coef_pairs, cross ? s.slots : nullptr, tc ? factors : nullptr, st)) return rc;
+    if (int rc = finish_coefs(p, src, sink, s.coef_blocks, cross ? s.slots : nullptr, factors, st)) return rc;
   }
   if (want_kv) join_wait(side, 0, skv, st);
   return OAL_OK;

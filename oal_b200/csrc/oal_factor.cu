@@ -161,14 +161,13 @@ __global__ void __launch_bounds__(32) head_factor_kernel(const int32_t* dim_perm
     const int rpos = k;
     for (int r = 0; r < n; ++r) if (sig[r] < 0.f) order[k++] = r;
     for (int r = 0; r < n; ++r) lam[r] = sqrtf(fmaxf(fabsf(sig[order[r]]), floor_v));
-    table[h].rank = n;
-    table[h].rpos = rpos;
-    table[h].w0 = 0.f;
-    table[h].pad = 0;
+    table[h].s.rank = n;
+    table[h].s.rpos = rpos;
+    table[h].s.w0 = 0.f;
   }
   __syncwarp();
   HeadFactor& out = table[h];
-  if (lane < RMAX_ALL) out.c[lane] = lane < n ? lam[lane] * V[0][order[lane]] : 0.f;
+  if (lane < RMAX_ALL) out.s.c[lane] = lane < n ? lam[lane] * V[0][order[lane]] : 0.f;
   for (int r = 0; r < RMAX_ALL; ++r) {
     const bool live = r < n;
     const float sl = live ? scale * lam[r] : 0.f;

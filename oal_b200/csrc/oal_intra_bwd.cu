@@ -1,21 +1,27 @@
 // Intra-chunk term of the chunked scan on the tensor cores (tcgen05 / TMEM), backward.
 //
-// Query side, per 16-key tile of a 128-token chunk (rows are queries):
-//   U  = Q . stack(K)^T,  dW = G [v|1]^T (whole chunk, G as hi + lo bf16)      MMAs into tensor memory
-//   P_r = 2 sgn_r dW u_r  (bf16 tile),  D[r][r'] += 2 dW u_r u_r'               registers
-//     (here the stack is carried as bf16 value + bf16 remainder, two MMA chains: the coefficient
-//      gradient is a sum of strongly cancelling terms -- sum_j dW_ij w_ij = 0 for every row -- and
-//      needs u to more than 8 bits; sum dW and sum dW u_r are accumulated on their own for dA, dB)
-//   dq += P . stack(K)                                                           MMA, K = 16 R
-// Key / value side (rows are keys, 16 queries per tile): the same with q and k exchanged,
-//   dk += P^T-tile . stack(Q),  dU += W^T G   with W = sum_r sgn_r u_r^2,
-// per query head into fp32 partials that kv_head_reduce_kernel sums over the heads of a KV head in
-// fixed order.  The stacked scaled tile (oal_intra.cuh) is rebuilt per tile in a three-slot ring by
-// the warps themselves; lane 0 of one compute warp (the one whose rows the causal mask idles most) also issues
-// every MMA, between that warp's own steps, driven by warp-granular mbarrier arrivals.  The cross-chunk parts computed by the state kernels arrive as fp32 buffers and are added
-// before the final cast.  Reference stages replaced: oal_attention/hd_block_gemm_backward_wave.py:253-476
-// (dS, local dphi_q / dphi_k / dU GEMMs) and the folds / coefficient partials of
-// oal_attention/hd_block_gemm_feature_backward.py:59-474.
+// Both kernels walk the terms r of the factored weight (oal_intra.cuh).  The scaled rows are carried as bf16
+// value + bf16 remainder, two MMA chains into u_r: the coefficient gradient is a sum of strongly cancelling terms
+// (sum_j dW_ij w_ij = 0 for every row) and needs u to more than 8 bits, and on the key side the rounding of the
+// scaled keys would act like a perturbation that is the same for every query.
+//
+// Query side (rows are query rows, columns are keys), dW = G [v|1]^T once (G as hi + lo bf16), then per term:
+//   P_r = 2 dW u_r             registers -> tensor memory, bf16 value + remainder
+//   Z_r = P_r K                one accumulator per term;  n_r = sum of P_r, registers
+//   dq  += sgn_r l_r * Z_r     registers (element-wise in the dimension)
+//   y_r  = sum over rows of q * Z_r, one 64-vector per row block
+// The coefficient gradient needs D'[r][r'] = sum_ij 2 dW u_r u_r' = sum_d l_r'[d] y_r[d] + c_r' n_r: 64 sums per
+// term instead of R (R + 1) / 2 products per pair.  P_r's remainder keeps these sums at the 16 bits they had when
+// they were formed from fp32 products.
+//
+// Key / value side (rows are keys, columns are the queries of one head): per head and term
+//   P_r^T as above (bf16 value),  Z_r = P_r^T Q,  dk += sgn_r l_r * Z_r,  w += sgn_r u_r^2 in registers,
+// and after the last term dU += W^T G.  A CTA walks several query heads of its KV head; dk stays in registers, dU
+// in tensor memory, and the next head's operands arrive while the current one is worked on.
+//
+// The cross-chunk parts computed by the state kernels arrive as fp32 buffers and are added before the final cast.
+// Reference stages replaced: oal_attention/hd_block_gemm_backward_wave.py:253-476 (dS, local dphi_q / dphi_k / dU
+// GEMMs) and the folds / coefficient partials of oal_attention/hd_block_gemm_feature_backward.py:59-474.
 #include "oal_intra.cuh"
 #include "oal_kernels.h"
 
@@ -29,500 +35,693 @@ struct IntraBwdArgs {
   const __nv_bfloat16* gimg;        // [2][B*Hq, NB, 10, 128, 8]: bf16(g) image, then the image of g - bf16(g)
   size_t gimg_lo_offset;            // bytes from the hi image to the lo image
   const HeadFactor* factors;
-  void* dq;                         // io dtype (bf16), may be null
+  __nv_bfloat16* dq;                // may be null
   const float* dq_init;             // fp32 cross part, or null
-  float* dk_part;                   // fp32 [B,Hq,N,64]: this query head's intra-chunk share of dk
-  float* dv_part;                   // fp32 [B,Hq,N,64]: this query head's intra-chunk share of dv
-  float* coef_partial;              // [B][Hq][NB][NQ] or null: D upper triangle, sum t_r, sum 2 dW
+  float* coef_partial;              // [B][Hq][row blocks][NQ] or null: D upper triangle, n_r, sum 2 dW
+  // key / value side: fp32 partials [B, Hkv * parts, N, 64] when the heads are spread over `parts` CTAs, else the
+  // results with the cross parts of the tokens before cross_end added
+  float *dk_part, *dv_part;
+  const float *dk_cross, *dv_cross;
+  __nv_bfloat16 *dk, *dv;
+  int cross_end, heads_per_cta, parts;
   int32_t* status;
-  int N, NB, Hq, Hkv;
+  int N, NB, Hq, Hkv, rep, rank;    // rank = groups + 1, the same for every head of a call
   int cross_from;                   // first chunk that has a cross-chunk part in dq_init
 };
 
-constexpr int STAGE_OUT_FLOATS = CT * 65 + 3;   // one [128][65] fp32 output staging tile (padded to 16 bytes)
+// Warps 0..15 compute, warp 16 issues; 17..19 only fill the issuer's warpgroup, whose registers the compute warps
+// take: 640 threads x 96 at launch = 512 x 112 + 128 x 24 and 1024 to spare.
+constexpr int BW_COMPUTE = 16, BW_ISSUER = BW_COMPUTE, BW_THREADS = (BW_COMPUTE + 4) * 32;
 
-// the G images (hi, lo) of one (batch row, query head, chunk): two bulk copies on one barrier
-__device__ __forceinline__ void fetch_g_images(const IntraBwdArgs& a, unsigned char* ghi, unsigned char* glo,
-                                               uint64_t* bar, int b, int h, int c) {
-  const size_t item = (size_t)(b * a.Hq + h) * a.NB + c;
-  const unsigned char* gsrc = reinterpret_cast<const unsigned char*>(a.gimg) + item * SLAB_S_BYTES;
-  mbar_arrive_expect_tx(bar, 2 * SLAB_S_BYTES);
-  bulk_g2s(ghi, gsrc, SLAB_S_BYTES, bar);
-  bulk_g2s(glo, gsrc + a.gimg_lo_offset, SLAB_S_BYTES, bar);
+// dW[128, n] = rows . cols^T over the 80-long augmented value axis; the side given as hi + lo is walked twice.
+__device__ __forceinline__ void issue_dw(uint32_t tmem_dw, uint64_t rows_hi, uint64_t rows_lo, uint32_t rows_step, uint64_t cols_hi,
+                                         uint64_t cols_lo, uint32_t cols_step, int n) {
+  const uint32_t idesc = instr_desc_bf16(128, n, 0, 0);
+#pragma unroll
+  for (int ks = 0; ks < 2 * (EP / 16); ++ks) {
+    const int lo = ks / (EP / 16), kk = ks % (EP / 16);
+    mma_bf16_ss(tmem_dw, desc_advance(lo ? rows_lo : rows_hi, kk * rows_step), desc_advance(lo ? cols_lo : cols_hi, kk * cols_step),
+                idesc, ks > 0);
+  }
+}
+
+// hi / lo bf16 pairs of eight products
+__device__ __forceinline__ void split8(const f32x2 (&t)[4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a, b;
+    f2_unpack(t[j], a, b);
+    hi[j] = pack_bf16(a, b);
+    lo[j] = pack_bf16(a - bf16_lo(hi[j]), b - bf16_hi(hi[j]));
+  }
 }
 
 // ---------------------------------------------------------------------------
 // query side
 // ---------------------------------------------------------------------------
-// shared memory: Qa | Kimg | 3 stacks | 2 remainder stacks | G hi, G lo, U (dead once dW is complete)
-// tensor memory: U (16 R columns) | dW (128) | dq (64) | two P tiles (8 R columns each)
-constexpr int BQ_SMEM = XA_BYTES + X_BYTES + 3 * ST_BYTES + 2 * STLO_BYTES + 3 * SLAB_S_BYTES;
-constexpr int NQ = NU + RM + 1;                 // partial sums per CTA: D (upper triangle), sum t_r, sum 2 dW
-static_assert(RM * KT + CT + HD + 2 * P_COLS <= 512, "tensor-memory columns of the query-side kernel");
-static_assert(CT * 65 * 4 <= XA_BYTES + X_BYTES + 3 * ST_BYTES, "dq staging tile");
+// tensor memory: U (two halves of 64; first dW) | P hi (64) | P lo (64) | two Z (64) | two term slots (64)
+constexpr uint32_t BQ_U = 0, BQ_P = 128, BQ_PLO = 192, BQ_Z = 256, BQ_TERM = 384;
+static_assert(BQ_TERM + 2 * TERM_COLS <= 512, "tensor-memory columns of the query-side kernel");
+constexpr int BQ_L_FLOATS = 4 * RMAX_ALL * HD;
+constexpr int BQ_SMEM = 2 * X_BYTES + 3 * XA_BYTES + BQ_L_FLOATS * 4;
+static_assert(BQ_L_FLOATS * 4 <= XA_BYTES, "the y sums take the place of an image of G");
 
-
-__global__ void __launch_bounds__(CTHREADS, 1) intra_bwd_q_kernel(const IntraBwdArgs a) {
+__global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_q_kernel(const IntraBwdArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* Qa = smem;
-  unsigned char* Kimg = Qa + XA_BYTES;
-  unsigned char* St = Kimg + X_BYTES;                     // 3 x ST_BYTES
-  unsigned char* Lo = St + 3 * ST_BYTES;                  // 2 x STLO_BYTES
-  unsigned char* Gimg = Lo + 2 * STLO_BYTES;              // hi, lo
-  unsigned char* Uimg = Gimg + 2 * SLAB_S_BYTES;
-  __shared__ HeadFactorS hf;
-  __shared__ uint64_t gfull, dw_done, u_done, u_free, p_ready[2], p_done[2], st_ready[3];
+  unsigned char* Qimg = smem;
+  unsigned char* Kimg = Qimg + X_BYTES;
+  unsigned char* Uimg = Kimg + X_BYTES;
+  unsigned char* Gimg = Uimg + XA_BYTES;                        // hi, lo; dead once dW is complete
+  float* lq = reinterpret_cast<float*>(Gimg + 2 * XA_BYTES);    // [quadrant][term][64]
+  float* ys = reinterpret_cast<float*>(Gimg);                   // [quadrant][term][64]
+  __shared__ __align__(16) HeadScalars sc[4];
+  __shared__ float nq[BW_COMPUTE][RMAX_ALL], sq[BW_COMPUTE];
+  __shared__ uint64_t dw_full, dw_free, u_full[2], u_free[2], term_full[2], p_full[2], z_half[2], z_free[2];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
-  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  const int kvh = h / (a.Hq / a.Hkv);
-  const int half = (warp >> 2) & 1, row = 32 * (warp & 3) + lane;
-  const bool issuer = warp == 0;
+  const QueryTile tile(a.Hkv, a.N, a.rep);
+  if (tile.empty()) return;
+  const int qd = warp & 3, sub = (warp >> 2) & 3, row = 32 * qd + lane;
+  const int tok0 = tile.c * CT, cols = tile.columns(), rank = a.rank;
+  const int my_rb = tile.rb(qd), my_head = tile.head(qd);
+  {
+    const size_t koff = ((size_t)tile.b * a.Hkv + tile.kvh) * a.N + tok0;
+    const size_t qoff = ((size_t)tile.b * a.Hq + my_head) * a.N + tok0 + min(32 * my_rb, tile.nc - 1);
+    const int fifth = (warp >> 2) * 32 + lane;                  // five warps load a quadrant's rows and table
+    const unsigned char* gsrc = reinterpret_cast<const unsigned char*>(a.gimg) +
+                                (((size_t)tile.b * a.Hq + my_head) * a.NB + tile.c) * SLAB_S_BYTES + 32 * my_rb * 16;
+    for (int x = fifth; x < 2 * (EP / 8) * 32; x += 160) {
+      const int r = x & 31, e = (x >> 5) % (EP / 8), lo = x >= (EP / 8) * 32;
+      async_copy16(Gimg + lo * XA_BYTES + e * CP + (32 * qd + r) * 16, gsrc + lo * a.gimg_lo_offset + e * (CT * 16) + r * 16, true);
+    }
+    load_rows(Uimg, 0, a.v + koff * VD, cols, tile.nc, tid, BW_THREADS);
+    load_rows(Qimg, 32 * qd, a.q + qoff * HD, 32, max(tile.nc - 32 * my_rb, 0), fifth, 160);
+    load_rows(Kimg, 0, a.k + koff * HD, cols, tile.nc, tid, BW_THREADS);
+    load_head(lq + qd * RMAX_ALL * HD, &sc[qd], a.factors + my_head, rank, fifth, 160);
+  }
+  augment_rows(Uimg, tile.nc, tid, BW_THREADS);
   if (warp == 0) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
-    mbar_init(&gfull, 1);
-    mbar_init(&dw_done, 1);
-    mbar_init(&u_done, 1);
-    mbar_init(&u_free, CWARPS);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&p_ready[s], CWARPS);
-      mbar_init(&p_done[s], 1);
+      mbar_init(&u_full[s], 1);
+      mbar_init(&u_free[s], BW_COMPUTE);
+      mbar_init(&term_full[s], BW_COMPUTE);
+      mbar_init(&p_full[s], BW_COMPUTE);
+      mbar_init(&z_half[s], 1);
+      mbar_init(&z_free[s], BW_COMPUTE);
     }
-    for (int s = 0; s < 3; ++s) mbar_init(&st_ready[s], CWARPS);
+    mbar_init(&dw_full, 1);
+    mbar_init(&dw_free, BW_COMPUTE);
     mbar_fence_init();
     dead = 0;
   }
-  __syncthreads();
-  if (tid == 0) fetch_g_images(a, Gimg, Gimg + SLAB_S_BYTES, &gfull, b, h, c);
-  const size_t qoff = (size_t)(b * a.Hq + h) * a.N, koff = (size_t)(b * a.Hkv + kvh) * a.N;
-  load_head_factor(hf, a.factors, h, tid, CTHREADS);
-  load_operand_image(Qa, a.q + qoff * HD, c * CT, a.N, true, tid, CTHREADS);
-  load_operand_image(Kimg, a.k + koff * HD, c * CT, a.N, false, tid, CTHREADS);
-  load_u_image(Uimg, a.v + koff * VD, c * CT, a.N, tid, CTHREADS);
   async_copies_wait();
-  __syncthreads();
-  const int tiles = min(CT / KT, (a.N - c * CT + KT - 1) / KT);
-  const int rank = uniform(hf.rank), rpos = uniform(hf.rpos);
-  for (int s = 0; s < 3; ++s) init_stack_constants(St + s * ST_BYTES, hf, tid, CTHREADS);
-  if ((tid >> 7) < tiles)
-    build_stack_piece(St + (tid >> 7) * ST_BYTES, Kimg, (tid >> 7) * KT, hf, tid & 127, Lo + (tid >> 7) * STLO_BYTES);
   fence_async_smem();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
   const uint32_t tmem = uniform(tmem_base);
-  const uint32_t tU = tmem, tW = tmem + RM * KT, tQ = tW + CT, tP = tQ + HD;
-  const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
-  f32x2 D2[NU], N2[RM], S2 = 0ull;
-#pragma unroll
-  for (int x = 0; x < NU; ++x) D2[x] = 0ull;
-#pragma unroll
-  for (int x = 0; x < RM; ++x) N2[x] = 0ull;
+  const uint32_t lane_off = (uint32_t)(32 * qd) << 16;
+  const int na = min(cols, 64), nb2 = cols - na;              // columns of the two halves
+  const bool want_coef = a.coef_partial != nullptr;
 
-  const uint32_t q_addr = smem_u32(Qa), st_addr = smem_u32(St), lo_addr = smem_u32(Lo);
-  if (issuer) {
-    if (elect_one()) {
-      w.wait(&gfull, 0, 0x20);
-      fence_after_sync();
-      issue_dw(tW, smem_u32(Gimg), true, smem_u32(Uimg), false);
-      mma_commit(&dw_done);
-      issue_stack_scores(tU, q_addr, st_addr, rank, lo_addr);
-      mma_commit(&u_done);
-    }
-    __syncwarp();
-  }
-  w.wait(&dw_done, 0, 0x24);
-  for (int kt = 0; kt < tiles; ++kt) {
-    const int buf = kt & 1;
-    const bool warp_active = 32 * (warp & 3) + 31 >= kt * KT;
-    float u[RM][8], dw[8];
-    w.wait(&u_done, kt & 1, 0x25);
-    fence_after_sync();
-    if (warp_active) {
-#pragma unroll
-      for (int r = 0; r < RM; ++r)
-        if (r < rank) tmem_ld8(tU + lane_off + r * KT + 8 * half, u[r]);
-      tmem_ld8(tW + lane_off + kt * KT + 8 * half, dw);
-      tmem_ld_wait();
-    }
-    fence_before_sync();
-    warp_arrive(&u_free, lane);
-    if (issuer && kt + 1 < tiles) {
+  if (warp >= BW_ISSUER) {
+    registers_down_to<24>();
+    if (warp == BW_ISSUER) {
+      const uint32_t k_addr = smem_u32(Kimg), g_addr = smem_u32(Gimg), u_addr = smem_u32(Uimg);
       if (elect_one()) {
-        w.wait(&u_free, kt & 1, 0x21);                 // every warp holds U(kt)
-        if (kt + 1 >= 2) w.wait(&st_ready[(kt + 1) % 3], ((kt - 1) / 3) & 1, 0x22);
-        fence_after_sync();
-        issue_stack_scores(tU, q_addr, st_addr + ((kt + 1) % 3) * ST_BYTES, rank, lo_addr + ((kt + 1) & 1) * STLO_BYTES);
-        mma_commit(&u_done);
+        const uint64_t du = smem_desc(u_addr, CP, 128), dk = smem_desc(k_addr, 128, CP);
+        issue_dw(tmem + BQ_U, smem_desc(g_addr, CP, 128), smem_desc(g_addr + XA_BYTES, CP, 128), 2 * CP, du, du, 2 * CP, cols);
+        mma_commit(&dw_full);
+        // half hf of the keys of Z_r = (P hi + P lo) K
+        const auto issue_z = [&](int r, int hf) {
+          w.wait(&p_full[hf], r & 1, 0x21);
+          if (hf == 0 && r >= 2) w.wait(&z_free[r & 1], ((r >> 1) - 1) & 1, 0x22);
+          fence_after_sync();
+          const uint32_t z = tmem + BQ_Z + (r & 1) * HD, idesc = instr_desc_bf16(128, HD, 0, 1);
+          const int k0 = hf ? 4 : 0, k1 = hf ? 4 + nb2 / 16 : na / 16;
+          for (int ks = k0; ks < k1; ++ks) {
+            mma_bf16_ts(z, tmem + BQ_P + 8 * ks, desc_advance(dk, ks * 256), idesc, ks > 0);
+            mma_bf16_ts(z, tmem + BQ_PLO + 8 * ks, desc_advance(dk, ks * 256), idesc, 1);
+          }
+          mma_commit(&z_half[hf]);
+        };
+        for (int r = 0; r < rank; ++r) {
+          const uint32_t slot = tmem + BQ_TERM + (r & 1) * TERM_COLS;
+          w.wait(&term_full[r & 1], (r >> 1) & 1, 0x23);
+          if (r > 0) w.wait(&u_free[0], (r - 1) & 1, 0x24);
+          else w.wait(&dw_free, 0, 0x25);
+          fence_after_sync();
+          issue_term(tmem + BQ_U, slot, k_addr, na);
+          mma_commit(&u_full[0]);
+          if (r > 0) {
+            issue_z(r - 1, 0);
+            w.wait(&u_free[1], (r - 1) & 1, 0x26);
+          }
+          if (nb2) {
+            fence_after_sync();
+            issue_term(tmem + BQ_U + 64, slot, k_addr + 64 * 16, nb2);
+          }
+          mma_commit(&u_full[1]);            // also: the term's slot has been read
+          if (r > 0) issue_z(r - 1, 1);
+        }
+        issue_z(rank - 1, 0);
+        issue_z(rank - 1, 1);
       }
       __syncwarp();
     }
-    if (kt >= 2) w.wait(&p_done[buf], ((kt - 2) >> 1) & 1, 0x26);
+  } else {
+    registers_up_to<112>();
+    const unsigned char* xrow = Qimg + row * 16;
+    const float* l = lq + qd * RMAX_ALL * HD;
+    const int rpos = uniform(sc[qd].rpos);
+    const int last_key = 32 * my_rb + 31, my_key = 32 * my_rb + lane;
+    const int d0 = 16 * sub;
+    const auto build = [&](int r) {
+      build_term16(tmem + BQ_TERM + (r & 1) * TERM_COLS + lane_off, xrow, l + r * HD, d0);
+      tmem_st_wait();
+      fence_before_sync();
+      warp_arrive(&term_full[r & 1], lane);
+    };
+    build(0);
+    // this warp's keys: a quarter of each half, in blocks of 8; blocks behind the diagonal stay zero in P
+    const auto key_of = [&](int hf, int x) { return 64 * hf + sub * ((hf ? nb2 : na) / 4) + 8 * x; };
+    const auto exists = [&](int hf, int x) { return 32 * x < (hf ? nb2 : na); };
+    const auto on = [&](int hf, int x) { return exists(hf, x) && key_of(hf, x) <= last_key; };
+    f32x2 dw[2][2][4];
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+        if (exists(hf, x) && !on(hf, x)) {
+          tmem_st4(tmem + BQ_P + lane_off + key_of(hf, x) / 2, 0u, 0u, 0u, 0u);
+          tmem_st4(tmem + BQ_PLO + lane_off + key_of(hf, x) / 2, 0u, 0u, 0u, 0u);
+        }
+    w.wait(&dw_full, 0, 0x27);
     fence_after_sync();
-    const uint32_t pt = tP + lane_off + buf * P_COLS;
-    if (warp_active) {
-      f32x2 dw2[4];
+    f32x2 sum2 = 0ull;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float d0 = dw[2 * j], d1 = dw[2 * j + 1];
-        if (kt * KT + 8 * half + 2 * j > row) d0 = 0.f;
-        if (kt * KT + 8 * half + 2 * j + 1 > row) d1 = 0.f;
-        dw2[j] = f2_pack(2.f * d0, 2.f * d1);
-        S2 = f2_add(S2, dw2[j]);
-      }
-      f32x2 u2[RM][4];
+    for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
-      for (int r = 0; r < RM; ++r)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) u2[r][j] = f2_pack(u[r][2 * j], u[r][2 * j + 1]);
-      int idx = 0;
-#pragma unroll
-      for (int r = 0; r < RM; ++r) {
-        if (r < rank) {
-          f32x2 t[4];
+      for (int x = 0; x < 2; ++x)
+        if (on(hf, x)) {
+          float d[8];
+          tmem_ld8(tmem + BQ_U + lane_off + key_of(hf, x), d);
+          tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            t[j] = f2_mul(dw2[j], u2[r][j]);
-            N2[r] = f2_add(N2[r], t[j]);
-          }
-          store_tile8(pt, r, half, t, r >= rpos);
-#pragma unroll
-          for (int r2 = r; r2 < RM; ++r2) {
-            if (r2 < rank) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) D2[idx + r2 - r] = f2_fma(t[j], u2[r2][j], D2[idx + r2 - r]);
-            }
+            const int kj = key_of(hf, x) + 2 * j;
+            dw[hf][x][j] = f2_pack(kj <= my_key ? 2.f * d[2 * j] : 0.f, kj + 1 <= my_key ? 2.f * d[2 * j + 1] : 0.f);
+            sum2 = f2_add(sum2, dw[hf][x][j]);
           }
         }
-        idx += RM - r;
-      }
-    } else {
-      const f32x2 zero[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-      for (int r = 0; r < RM; ++r)
-        if (r < rank) store_tile8(pt, r, half, zero, false);
-    }
-    tmem_st_wait();
     fence_before_sync();
-    warp_arrive(&p_ready[buf], lane);
-    // stack of tile kt + 2 into the slot whose last reader was the dq MMA of tile kt - 1
-    if (kt + 2 < tiles) {
-      if (kt >= 1) w.wait(&p_done[(kt - 1) & 1], ((kt - 1) >> 1) & 1, 0x27);
-      // (the remainder tile of slot kt & 1 was last read by U(kt), complete since u_done(kt))
-      if (half == (kt & 1))
-        build_stack_piece(St + ((kt + 2) % 3) * ST_BYTES, Kimg, (kt + 2) * KT, hf, tid & 127, Lo + buf * STLO_BYTES);
-      fence_async_smem();
-      warp_arrive(&st_ready[(kt + 2) % 3], lane);
-    }
-    if (issuer) {
-      if (elect_one()) {
-        w.wait(&p_ready[buf], (kt >> 1) & 1, 0x23);     // P tile of tile kt is in shared memory
+    warp_arrive(&dw_free, lane);
+    f32x2 dq[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dq[j] = 0ull;
+    // Z of term r: dq, and the sums over the 32 rows of q * Z (one warp holds all rows of its block)
+    const auto drain = [&](int r) {
+      float z[16];
+      tmem_ld16(tmem + BQ_Z + (r & 1) * HD + lane_off + d0, z);
+      tmem_ld_wait();
+      fence_before_sync();
+      warp_arrive(&z_free[r & 1], lane);
+      const f32x2 sgn = f2_bcast(r < rpos ? 1.f : -1.f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const ulonglong2 lv = *reinterpret_cast<const ulonglong2*>(l + r * HD + d0 + 4 * j);
+        dq[2 * j] = f2_fma(f2_mul(lv.x, sgn), f2_pack(z[4 * j], z[4 * j + 1]), dq[2 * j]);
+        dq[2 * j + 1] = f2_fma(f2_mul(lv.y, sgn), f2_pack(z[4 * j + 2], z[4 * j + 3]), dq[2 * j + 1]);
+      }
+      if (!want_coef) return;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(xrow + (d0 / 8 + k) * CP);
+        const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          z[8 * k + 2 * j] *= bf16_lo(rw[j]);
+          z[8 * k + 2 * j + 1] *= bf16_hi(rw[j]);
+        }
+      }
+      // butterfly that halves the values it carries: 16 shuffles for 16 sums over 32 lanes
+#pragma unroll
+      for (int o = 16; o >= 2; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < o / 2; ++j) {
+          const float send = up ? z[j] : z[j + o / 2], keep = up ? z[j + o / 2] : z[j];
+          z[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+      z[0] += __shfl_xor_sync(0xffffffffu, z[0], 1);
+      if ((lane & 1) == 0) ys[(qd * RMAX_ALL + r) * HD + d0 + (lane >> 1)] = z[0];
+    };
+    for (int r = 0; r < rank; ++r) {
+      // the next term is built while the MMAs of this one run; its slot's last reader was term r - 1, complete
+      // since u_full[1](r - 1)
+      if (r + 1 < rank) build(r + 1);
+      const f32x2 c2 = f2_bcast(sc[qd].c[r]);
+      f32x2 n2 = 0ull;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        w.wait(&u_full[hf], r & 1, 0x28 + hf);
         fence_after_sync();
-        issue_stack_grad(tQ, tP + buf * P_COLS, st_addr + (kt % 3) * ST_BYTES, rank, kt > 0);
-        mma_commit(&p_done[buf]);
-      }
-      __syncwarp();
-    }
-  }
-  if (tiles >= 2) w.wait(&p_done[(tiles - 2) & 1], ((tiles - 2) >> 1) & 1, 0x28);
-  w.wait(&p_done[(tiles - 1) & 1], ((tiles - 1) >> 1) & 1, 0x29);
-  fence_after_sync();
-  // every MMA has completed: all shared-memory operands are free
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
-  float* stage_out = reinterpret_cast<float*>(smem);              // [128][65] fp32 over Qa / Kimg / stacks
-  float* red = reinterpret_cast<float*>(smem + CT * 65 * 4 + 256);   // [NQ][CTHREADS] behind it
-  static_assert(CT * 65 * 4 + 256 + NQ * CTHREADS * 4 <= BQ_SMEM, "staging tile and partial sums");
-  {
-    if (a.dq) {
+        float u[2][8];
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        float vv[16];
-        tmem_ld16(tQ + lane_off + 32 * half + 16 * cc, vv);
+        for (int x = 0; x < 2; ++x)
+          if (on(hf, x)) tmem_ld8(tmem + BQ_U + lane_off + key_of(hf, x), u[x]);
         tmem_ld_wait();
+        fence_before_sync();
+        warp_arrive(&u_free[hf], lane);
+        uint32_t hi[2][4], lo[2][4];
 #pragma unroll
-        for (int x = 0; x < 16; ++x) stage_out[row * 65 + 32 * half + 16 * cc + x] = vv[x];
+        for (int x = 0; x < 2; ++x)
+          if (on(hf, x)) {
+            f32x2 t[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              t[j] = f2_mul(dw[hf][x][j], f2_add(f2_pack(u[x][2 * j], u[x][2 * j + 1]), c2));
+              n2 = f2_add(n2, t[j]);
+            }
+            split8(t, hi[x], lo[x]);
+          }
+        if (r > 0) {                           // the previous term's P has been read
+          w.wait(&z_half[hf], (r - 1) & 1, 0x2A + hf);
+          fence_after_sync();
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          if (on(hf, x)) {
+            tmem_st4(tmem + BQ_P + lane_off + key_of(hf, x) / 2, hi[x][0], hi[x][1], hi[x][2], hi[x][3]);
+            tmem_st4(tmem + BQ_PLO + lane_off + key_of(hf, x) / 2, lo[x][0], lo[x][1], lo[x][2], lo[x][3]);
+          }
+        tmem_st_wait();
+        fence_before_sync();
+        warp_arrive(&p_full[hf], lane);
+      }
+      if (r > 0) drain(r - 1);
+      if (want_coef) {
+        float n, n1;
+        f2_unpack(n2, n, n1);
+        n += n1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+        if (lane == 0) nq[warp][r] = n;
       }
     }
-    if (a.coef_partial) {
+    w.wait(&z_half[0], (rank - 1) & 1, 0x2C);
+    w.wait(&z_half[1], (rank - 1) & 1, 0x2D);
+    fence_after_sync();
+    drain(rank - 1);
+    if (want_coef) {
+      float s0, s1;
+      f2_unpack(sum2, s0, s1);
+      s0 += s1;
 #pragma unroll
-      for (int x = 0; x < NQ; ++x) {
-        float lo, hi;
-        f2_unpack(x < NU ? D2[x < NU ? x : 0] : (x < NU + RM ? N2[x >= NU && x < NU + RM ? x - NU : 0] : S2), lo, hi);
-        red[x * CTHREADS + tid] = lo + hi;
+      for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      if (lane == 0) sq[warp] = s0;
+    }
+    if (a.dq && my_key < tile.nc && !dead) {
+      // 16 consecutive dims of a row per thread: whole 32- and 64-byte sectors
+      const size_t o = (((size_t)tile.b * a.Hq + my_head) * a.N + tok0 + my_key) * HD + d0;
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f2_unpack(dq[j], v[2 * j], v[2 * j + 1]);
+      if (a.dq_init && tile.c >= a.cross_from) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 t = *reinterpret_cast<const float4*>(a.dq_init + o + 4 * j);
+          v[4 * j] += t.x; v[4 * j + 1] += t.y; v[4 * j + 2] += t.z; v[4 * j + 3] += t.w;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        *reinterpret_cast<uint4*>(a.dq + o + 8 * j) =
+            make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
+                       pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
+    }
+    if (want_coef) {
+      // the quadrant's four warps turn its sums into D' (symmetrised: both orders are the same sum), n', s'
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + qd) : "memory");
+      const auto n_of = [&](int r) { return (nq[qd][r] + nq[4 + qd][r]) + (nq[8 + qd][r] + nq[12 + qd][r]); };
+      const int nu = rank * (rank + 1) / 2, stride = nu + rank + 1, blocks = (a.N + 31) / 32;
+      float* dst = a.coef_partial + (((size_t)tile.b * a.Hq + my_head) * blocks + tile.c * 4 + my_rb) * stride;
+      const float* y = ys + qd * RMAX_ALL * HD;
+      for (int x = sub * 32 + lane; x < stride && 32 * my_rb < tile.nc; x += 128) {
+        float t;
+        if (x < nu) {
+          int r = 0, rest = x;
+          while (rest >= rank - r) { rest -= rank - r; ++r; }
+          const int r2 = r + rest;
+          t = fmaf(sc[qd].c[r2], n_of(r), sc[qd].c[r] * n_of(r2));
+#pragma unroll 4
+          for (int d = 0; d < HD; d += 4) {
+            const float4 la = *reinterpret_cast<const float4*>(l + r * HD + d), lb = *reinterpret_cast<const float4*>(l + r2 * HD + d);
+            const float4 ya = *reinterpret_cast<const float4*>(y + r * HD + d), yb = *reinterpret_cast<const float4*>(y + r2 * HD + d);
+            t = fmaf(lb.x, ya.x, fmaf(lb.y, ya.y, fmaf(lb.z, ya.z, fmaf(lb.w, ya.w, t))));
+            t = fmaf(la.x, yb.x, fmaf(la.y, yb.y, fmaf(la.z, yb.z, fmaf(la.w, yb.w, t))));
+          }
+          t *= 0.5f;
+        } else if (x < nu + rank) {
+          t = n_of(x - nu);
+        } else {
+          t = (sq[qd] + sq[4 + qd]) + (sq[8 + qd] + sq[12 + qd]);
+        }
+        dst[x] = t;
       }
     }
   }
   fence_before_sync();
-  __syncthreads();
-  if (a.dq && !dead) {
-    // coalesced write-out: 8 consecutive dims per thread, cross-chunk part added, one 16-byte store
-    constexpr int PER = CT * 8 / CTHREADS;
-    float4 i0[PER], i1[PER];
-#pragma unroll
-    for (int it = 0; it < PER; ++it) {
-      const int x = tid + it * CTHREADS, r = x >> 3, seg = x & 7, i = c * CT + r;
-      i0[it] = i1[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (i < a.N && a.dq_init && c >= a.cross_from) {
-        const float* ip = a.dq_init + (qoff + i) * HD + seg * 8;
-        i0[it] = *reinterpret_cast<const float4*>(ip);
-        i1[it] = *reinterpret_cast<const float4*>(ip + 4);
-      }
-    }
-#pragma unroll
-    for (int it = 0; it < PER; ++it) {
-      const int x = tid + it * CTHREADS, r = x >> 3, seg = x & 7, i = c * CT + r;
-      if (i >= a.N) continue;
-      const size_t o = (qoff + i) * HD + seg * 8;
-      const float* sp = stage_out + r * 65 + seg * 8;
-      const float val[8] = {sp[0] + i0[it].x, sp[1] + i0[it].y, sp[2] + i0[it].z, sp[3] + i0[it].w,
-                            sp[4] + i1[it].x, sp[5] + i1[it].y, sp[6] + i1[it].z, sp[7] + i1[it].w};
-      *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.dq) + o) =
-          make_uint4(pack_bf16(val[0], val[1]), pack_bf16(val[2], val[3]), pack_bf16(val[4], val[5]), pack_bf16(val[6], val[7]));
-    }
-  }
-  if (a.coef_partial) {
-    // column sums of the per-thread partials: red[value][thread], one warp per value, fixed order
-    float* dst = a.coef_partial + ((size_t)(b * a.Hq + h) * a.NB + c) * NQ;
-    for (int v = warp; v < NQ; v += CWARPS) {
-      float t = 0.f;
-#pragma unroll
-      for (int x = 0; x < CTHREADS / 32; ++x) t += red[v * CTHREADS + 32 * x + lane];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) dst[v] = t;
-    }
-  }
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, 512);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
 
 // ---------------------------------------------------------------------------
-// key / value side: one CTA per (chunk, query head, batch row); rows are keys
+// key / value side: one CTA per (chunk, KV head, batch row) and group of query heads; rows are keys
 // ---------------------------------------------------------------------------
-constexpr int KV_WARPS = 16, KV_THREADS = KV_WARPS * 32;   // 128 key rows x 4 quarters of a 16-query tile
-// shared memory: Ka | Qimg | G hi | G lo | 3 stacks | 2 remainder stacks | U   (G lo and U are dead once dW
-// is complete).  The stack is carried as value + remainder here too: its rounding acts like a perturbation
-// of the query rows that is the same for every key, and with large cancelling dimensions that alone costs
-// dk / dv more than the tolerance.
-// tensor memory: U (16 R columns) | dW^T (128) | dk (64) | dU (80) | one P tile (8 R) | one W^T tile (8)
-constexpr int BKV_SMEM = XA_BYTES + X_BYTES + SLAB_S_BYTES + 3 * ST_BYTES + 2 * STLO_BYTES + 2 * SLAB_S_BYTES;
-static_assert(RM * KT + CT + HD + EP + P_COLS + KT / 2 <= 512, "tensor-memory columns of the key/value-side kernel");
-static_assert(2 * STAGE_OUT_FLOATS * 4 <= XA_BYTES + X_BYTES + 2 * SLAB_S_BYTES + 3 * ST_BYTES, "staging tiles");
+// tensor memory: U (two halves of 64; first dW^T of a head) | P^T (64), later W^T | Z (64) | dU (80) | two term slots (64)
+constexpr uint32_t BK_U = 0, BK_P = 128, BK_Z = 192, BK_V = 256, BK_TERM = 336;
+static_assert(BK_TERM + 2 * TERM_COLS <= 512, "tensor-memory columns of the key/value-side kernel");
+constexpr int BK_HEAD_L = RMAX_ALL * HD * 4;
+constexpr int BK_HEAD_BYTES = X_BYTES + 2 * SLAB_S_BYTES + BK_HEAD_L;       // Q image, G hi, G lo, l: one head's operands
+constexpr int BK_SMEM = X_BYTES + XA_BYTES + 2 * BK_HEAD_BYTES;
+static_assert(BK_HEAD_BYTES % 16 == 0 && BK_SMEM <= 227 * 1024, "shared memory of the key/value-side kernel");
 
-__global__ void __launch_bounds__(KV_THREADS, 1) intra_bwd_kv_kernel(const IntraBwdArgs a) {
+__global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const IntraBwdArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* Ka = smem;                               // augmented k image (rows are keys)
-  unsigned char* Qimg = Ka + XA_BYTES;
-  unsigned char* Ghi = Qimg + X_BYTES;
-  unsigned char* Glo = Ghi + SLAB_S_BYTES;                // dead once dW is complete
-  unsigned char* St = Glo + SLAB_S_BYTES;                 // 3 x ST_BYTES: stacked scaled query tiles
-  unsigned char* Lo = St + 3 * ST_BYTES;                  // 2 x STLO_BYTES
-  unsigned char* Uimg = Lo + 2 * STLO_BYTES;              // dead once dW is complete
-  __shared__ HeadFactorS hf;
-  __shared__ uint64_t gfull, dw_done, u_done, u_free, p_ready, p_done, st_ready[3];
+  unsigned char* Kimg = smem;
+  unsigned char* Uimg = Kimg + X_BYTES;
+  unsigned char* heads = Uimg + XA_BYTES;                       // two sets of a head's operands
+  __shared__ __align__(16) HeadScalars sc[2];
+  __shared__ uint64_t q_full[2], g_full[2], dw_full, dw_free, u_full[2], u_free[2], term_full[2], p_full[2], z_half[2], z_free, w_full, v_full;
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
-  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  const int kvh = h / (a.Hq / a.Hkv);
-  const int part = warp >> 2, row = 32 * (warp & 3) + lane;       // row = key index inside the chunk; part = 4 queries of a tile
-  // Key rows 96..127 (warps 3, 7, 11, 15) are masked out of every tile but the last two, and every stack is
-  // built before those: these four warps are the builders, so the warps of rows 0..31, which work in every
-  // tile, never build.  Rows 64..95 are idle for the first four tiles: warp 2 issues the MMAs.
-  const bool issuer = warp == 2, builder = (warp & 3) == 3;
+  const int part = blockIdx.z, c = blockIdx.x, b = blockIdx.y / a.Hkv, kvh = blockIdx.y - b * a.Hkv;
+  const int h0 = part * a.heads_per_cta, n_heads = min(a.heads_per_cta, a.rep - h0), rank = a.rank;
+  const int qd = warp & 3, sub = (warp >> 2) & 3, row = 32 * qd + lane;     // row: key index inside the chunk
+  const int tok0 = c * CT, nc = min(CT, a.N - tok0), cols = (nc + 31) & ~31;
+  const size_t koff = ((size_t)b * a.Hkv + kvh) * a.N + tok0;
+  const auto head_of = [&](int i) { return kvh * a.rep + h0 + i; };
+  // Q image, l and scalars of head i: asynchronous copies by threads tid of n
+  const auto fetch_q = [&](int i, int n) {
+    unsigned char* set = heads + (i & 1) * BK_HEAD_BYTES;
+    load_rows(set, 0, a.q + (((size_t)b * a.Hq + head_of(i)) * a.N + tok0) * HD, cols, nc, tid, n);
+    load_head(reinterpret_cast<float*>(set + X_BYTES + 2 * SLAB_S_BYTES), &sc[i & 1], a.factors + head_of(i), rank, tid, n);
+  };
+  load_rows(Kimg, 0, a.k + koff * HD, CT, nc, tid, BW_THREADS);
+  load_rows(Uimg, 0, a.v + koff * VD, CT, nc, tid, BW_THREADS);
+  if (warp < BW_COMPUTE) fetch_q(0, BW_COMPUTE * 32);
+  augment_rows(Uimg, nc, tid, BW_THREADS);
   if (warp == 0) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
-    mbar_init(&gfull, 1);
-    mbar_init(&dw_done, 1);
-    mbar_init(&u_done, 1);
-    mbar_init(&u_free, KV_WARPS);
-    mbar_init(&p_ready, KV_WARPS);
-    mbar_init(&p_done, 1);
-    for (int s = 0; s < 3; ++s) mbar_init(&st_ready[s], KV_WARPS);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], BW_COMPUTE);
+      mbar_init(&g_full[s], 1);
+      mbar_init(&u_full[s], 1);
+      mbar_init(&u_free[s], BW_COMPUTE);
+      mbar_init(&term_full[s], BW_COMPUTE);
+      mbar_init(&p_full[s], BW_COMPUTE);
+      mbar_init(&z_half[s], 1);
+    }
+    mbar_init(&dw_full, 1);
+    mbar_init(&dw_free, BW_COMPUTE);
+    mbar_init(&z_free, BW_COMPUTE);
+    mbar_init(&w_full, BW_COMPUTE);
+    mbar_init(&v_full, 1);
     mbar_fence_init();
     dead = 0;
   }
-  __syncthreads();
-  if (tid == 0) fetch_g_images(a, Ghi, Glo, &gfull, b, h, c);
-  const size_t qoff = (size_t)(b * a.Hq + h) * a.N, koff = (size_t)(b * a.Hkv + kvh) * a.N;
-  load_head_factor(hf, a.factors, h, tid, KV_THREADS);
-  load_operand_image(Ka, a.k + koff * HD, c * CT, a.N, true, tid, KV_THREADS);
-  load_operand_image(Qimg, a.q + qoff * HD, c * CT, a.N, false, tid, KV_THREADS);
-  load_u_image(Uimg, a.v + koff * VD, c * CT, a.N, tid, KV_THREADS);
   async_copies_wait();
-  __syncthreads();
-  const int tiles = min(CT / KT, (a.N - c * CT + KT - 1) / KT);
-  const int rank = uniform(hf.rank), rpos = uniform(hf.rpos);
-  const f32x2 w0 = f2_bcast(hf.w0);
-  for (int s = 0; s < 3; ++s) init_stack_constants(St + s * ST_BYTES, hf, tid, KV_THREADS);
-  if (tid < 256 && (tid >> 7) < tiles)
-    build_stack_piece(St + (tid >> 7) * ST_BYTES, Qimg, (tid >> 7) * KT, hf, tid & 127, Lo + (tid >> 7) * STLO_BYTES);
   fence_async_smem();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   Waiter w{&dead};
   const uint32_t tmem = uniform(tmem_base);
-  const uint32_t tU = tmem, tW = tmem + RM * KT, tK = tW + CT, tV = tK + HD, tP = tV + EP, tWt = tP + P_COLS;
-  const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
+  const uint32_t lane_off = (uint32_t)(32 * qd) << 16;
+  const int na = min(cols, 64), nb2 = cols - na;              // columns of the two halves
 
-  const uint32_t k_addr = smem_u32(Ka), st_addr = smem_u32(St), g_addr = smem_u32(Ghi), lo_addr = smem_u32(Lo);
-  const uint32_t idesc_du = instr_desc_bf16(128, EP, 0, 1);
-  if (issuer) {
-    if (elect_one()) {
-      w.wait(&gfull, 0, 0x30);
-      fence_after_sync();
-      // dW^T[j, i] = [v|1]_j . g_i: rows from the U image, columns from the hi and lo images of G
-      issue_dw(tW, smem_u32(Uimg), false, g_addr, true);
-      mma_commit(&dw_done);
-      issue_stack_scores(tU, k_addr, st_addr, rank, lo_addr);
-      mma_commit(&u_done);
-    }
-    __syncwarp();
-  }
-  w.wait(&dw_done, 0, 0x34);
-  for (int qt = 0; qt < tiles; ++qt) {
-    // keys of this warp are all later than the tile's queries -> nothing survives the mask
-    const bool warp_active = 32 * (warp & 3) <= qt * KT + KT - 1;
-    float u[RM][4], dw[4];
-    w.wait(&u_done, qt & 1, 0x35);
-    fence_after_sync();
-    if (warp_active) {
-#pragma unroll
-      for (int r = 0; r < RM; ++r)
-        if (r < rank) tmem_ld4(tU + lane_off + r * KT + 4 * part, u[r]);
-      tmem_ld4(tW + lane_off + qt * KT + 4 * part, dw);
-      tmem_ld_wait();
-    }
-    fence_before_sync();
-    warp_arrive(&u_free, lane);
-    if (issuer && qt + 1 < tiles) {
+  if (warp >= BW_ISSUER) {
+    registers_down_to<24>();
+    if (warp == BW_ISSUER) {
       if (elect_one()) {
-        w.wait(&u_free, qt & 1, 0x31);
-        if (qt + 1 >= 2) w.wait(&st_ready[(qt + 1) % 3], ((qt - 1) / 3) & 1, 0x32);
-        fence_after_sync();
-        issue_stack_scores(tU, k_addr, st_addr + ((qt + 1) % 3) * ST_BYTES, rank, lo_addr + ((qt + 1) & 1) * STLO_BYTES);
-        mma_commit(&u_done);
-      }
-      __syncwarp();
-    }
-    // one P tile and one W^T tile in tensor memory: the MMAs of the previous tile must have read them
-    if (qt >= 1) w.wait(&p_done, (qt - 1) & 1, 0x36);
-    fence_after_sync();
-    const uint32_t pt = tP + lane_off + 2 * part;
-    f32x2 wv[2] = {0ull, 0ull};
-    if (warp_active) {
-      f32x2 dw2[2], wp[2], wn[2];
-      bool keep[4];
-#pragma unroll
-      for (int x = 0; x < 4; ++x) keep[x] = qt * KT + 4 * part + x >= row;      // query not earlier than the key
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        dw2[j] = f2_pack(keep[2 * j] ? 2.f * dw[2 * j] : 0.f, keep[2 * j + 1] ? 2.f * dw[2 * j + 1] : 0.f);
-        wp[j] = w0;
-        wn[j] = 0ull;
-      }
-#pragma unroll
-      for (int r = 0; r < RM; ++r) {
-        if (r < rank) {
-          const f32x2 ua = f2_pack(u[r][0], u[r][1]), ub = f2_pack(u[r][2], u[r][3]);
-          const f32x2 ta = f2_mul(dw2[0], ua), tb = f2_mul(dw2[1], ub);
-          if (r < rpos) { wp[0] = f2_fma(ua, ua, wp[0]); wp[1] = f2_fma(ub, ub, wp[1]); }
-          else { wn[0] = f2_fma(ua, ua, wn[0]); wn[1] = f2_fma(ub, ub, wn[1]); }
-          float a0, a1, b0, b1;
-          f2_unpack(ta, a0, a1);
-          f2_unpack(tb, b0, b1);
-          uint32_t lo = pack_bf16(a0, a1), hi = pack_bf16(b0, b1);
-          if (r >= rpos) { lo ^= 0x80008000u; hi ^= 0x80008000u; }
-          tmem_st2(pt + r * (KT / 2), lo, hi);
+        const uint32_t u_addr = smem_u32(Uimg);
+        const auto fetch_g = [&](int i) {                     // both G images of head i (bulk copies)
+          unsigned char* dst = heads + (i & 1) * BK_HEAD_BYTES + X_BYTES;
+          const unsigned char* src = reinterpret_cast<const unsigned char*>(a.gimg) + (((size_t)b * a.Hq + head_of(i)) * a.NB + c) * SLAB_S_BYTES;
+          mbar_arrive_expect_tx(&g_full[i & 1], 2 * SLAB_S_BYTES);
+          bulk_g2s(dst, src, SLAB_S_BYTES, &g_full[i & 1]);
+          bulk_g2s(dst + SLAB_S_BYTES, src + a.gimg_lo_offset, SLAB_S_BYTES, &g_full[i & 1]);
+        };
+        fetch_g(0);
+        int T = 0;                                            // terms issued so far, over all heads
+        for (int i = 0; i < n_heads; ++i) {
+          const uint32_t q_addr = smem_u32(heads + (i & 1) * BK_HEAD_BYTES), g_addr = q_addr + X_BYTES;
+          if (i + 1 < n_heads) {
+            if (i > 0) w.wait(&v_full, (i - 1) & 1, 0x30);    // head i - 1 no longer reads the set that head i + 1 takes
+            fetch_g(i + 1);
+          }
+          w.wait(&g_full[i & 1], (i >> 1) & 1, 0x31);
+          w.wait(&q_full[i & 1], (i >> 1) & 1, 0x32);
+          if (T > 0) {
+            w.wait(&u_free[0], (T - 1) & 1, 0x33);
+            w.wait(&u_free[1], (T - 1) & 1, 0x34);
+          }
+          fence_after_sync();
+          // dW^T[j, i] = [v|1]_j . g_i: rows from the U image, columns from the hi and lo images of G
+          const uint64_t du = smem_desc(u_addr, CP, 128);
+          issue_dw(tmem + BK_U, du, du, 2 * CP, smem_desc(g_addr, CT * 16, 128), smem_desc(g_addr + SLAB_S_BYTES, CT * 16, 128),
+                   2 * CT * 16, cols);
+          mma_commit(&dw_full);
+          const uint64_t dq = smem_desc(q_addr, 128, CP), dg = smem_desc(g_addr, 128, CT * 16);
+          const auto issue_z = [&](int t, int hf) {
+            w.wait(&p_full[hf], t & 1, 0x35);
+            if (hf == 0 && t > 0) w.wait(&z_free, (t - 1) & 1, 0x36);
+            fence_after_sync();
+            const int k0 = hf ? 4 : 0, k1 = hf ? 4 + nb2 / 16 : na / 16;
+            for (int ks = k0; ks < k1; ++ks)
+              mma_bf16_ts(tmem + BK_Z, tmem + BK_P + 8 * ks, desc_advance(dq, ks * 256), instr_desc_bf16(128, HD, 0, 1), ks > 0);
+            mma_commit(&z_half[hf]);
+          };
+          for (int r = 0; r < rank; ++r, ++T) {
+            const uint32_t slot = tmem + BK_TERM + (T & 1) * TERM_COLS;
+            w.wait(&term_full[T & 1], (T >> 1) & 1, 0x37);
+            if (r > 0) w.wait(&u_free[0], (T - 1) & 1, 0x38);
+            else w.wait(&dw_free, i & 1, 0x39);
+            fence_after_sync();
+            issue_term(tmem + BK_U, slot, q_addr, na);
+            mma_commit(&u_full[0]);
+            if (r > 0) {
+              issue_z(T - 1, 0);
+              w.wait(&u_free[1], (T - 1) & 1, 0x3A);
+            }
+            if (nb2) {
+              fence_after_sync();
+              issue_term(tmem + BK_U + 64, slot, q_addr + 64 * 16, nb2);
+            }
+            mma_commit(&u_full[1]);            // also: the term's slot has been read
+            if (r > 0) issue_z(T - 1, 1);
+          }
+          issue_z(T - 1, 0);
+          issue_z(T - 1, 1);
+          w.wait(&w_full, i & 1, 0x3B);
+          fence_after_sync();
+          for (int ks = 0; ks < cols / 16; ++ks)      // dU (+)= W^T G
+            mma_bf16_ts(tmem + BK_V, tmem + BK_P + 8 * ks, desc_advance(dg, ks * 256), instr_desc_bf16(128, EP, 0, 1), i + ks > 0);
+          mma_commit(&v_full);
         }
       }
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        float p0, p1, n0, n1;
-        f2_unpack(wp[j], p0, p1);
-        f2_unpack(wn[j], n0, n1);
-        wv[j] = f2_pack(keep[2 * j] ? p0 - n0 : 0.f, keep[2 * j + 1] ? p1 - n1 : 0.f);
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < RM; ++r)
-        if (r < rank) tmem_st2(pt + r * (KT / 2), 0u, 0u);
-    }
-    {
-      float a0, a1, b0, b1;
-      f2_unpack(wv[0], a0, a1);
-      f2_unpack(wv[1], b0, b1);
-      tmem_st2(tWt + lane_off + 2 * part, pack_bf16(a0, a1), pack_bf16(b0, b1));
-    }
-    tmem_st_wait();
-    fence_before_sync();
-    warp_arrive(&p_ready, lane);
-    // stack of tile qt + 2 into the slot whose last reader was the dk MMA of tile qt - 1 (complete: see above)
-    if (qt + 2 < tiles) {
-      if (builder)
-        build_stack_piece(St + ((qt + 2) % 3) * ST_BYTES, Qimg, (qt + 2) * KT, hf, 32 * part + lane, Lo + (qt & 1) * STLO_BYTES);
-      fence_async_smem();
-      warp_arrive(&st_ready[(qt + 2) % 3], lane);
-    }
-    if (issuer) {
-      if (elect_one()) {
-        w.wait(&p_ready, qt & 1, 0x33);
-        fence_after_sync();
-        issue_stack_grad(tK, tP, st_addr + (qt % 3) * ST_BYTES, rank, qt > 0);
-        mma_bf16_ts(tV, tWt, smem_desc(g_addr + qt * KT * 16, 128, CT * 16), idesc_du, qt > 0);
-        mma_commit(&p_done);
-      }
       __syncwarp();
     }
-  }
-  w.wait(&p_done, (tiles - 1) & 1, 0x39);
-  fence_after_sync();
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
-  // tensor-memory loads are warp-collective: every thread of a compute warp executes them; rows
-  // beyond N are dropped at the write-out
-  float* stage_out = reinterpret_cast<float*>(smem);    // two [128][65] fp32 staging tiles: dk, then dv
-  {
-    float vv[16];
-    tmem_ld16(tK + lane_off + 16 * part, vv);
+  } else {
+    registers_up_to<112>();
+    const unsigned char* xrow = Kimg + row * 16;
+    const int d0 = 16 * sub;
+    // this warp's queries: a quarter of each half, in blocks of 8; blocks before the diagonal stay zero in P^T and W^T
+    const auto col_of = [&](int hf, int x) { return 64 * hf + sub * ((hf ? nb2 : na) / 4) + 8 * x; };
+    const auto exists = [&](int hf, int x) { return 32 * x < (hf ? nb2 : na); };
+    const auto on = [&](int hf, int x) { return exists(hf, x) && col_of(hf, x) + 7 >= 32 * qd; };
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+        if (exists(hf, x) && !on(hf, x)) tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, 0u, 0u, 0u, 0u);
+    f32x2 dk[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dk[j] = 0ull;
+    int T = 0;
+    for (int i = 0; i < n_heads; ++i) {
+      const float* l = reinterpret_cast<const float*>(heads + (i & 1) * BK_HEAD_BYTES + X_BYTES + 2 * SLAB_S_BYTES);
+      const HeadScalars& hs = sc[i & 1];
+      async_copies_wait();
+      fence_async_smem();
+      warp_arrive(&q_full[i & 1], lane);
+      // every warp reads l and the scalars below: all copies have arrived
+      w.wait(&q_full[i & 1], (i >> 1) & 1, 0x3C);
+      if (i > 0) w.wait(&v_full, (i - 1) & 1, 0x3D);          // W^T of the previous head has been read; so has its operand set
+      if (i + 1 < n_heads) fetch_q(i + 1, BW_COMPUTE * 32);
+      const int rpos = uniform(hs.rpos);
+      const auto build = [&](int r) {
+        build_term16(tmem + BK_TERM + ((T + r) & 1) * TERM_COLS + lane_off, xrow, l + r * HD, d0);
+        tmem_st_wait();
+        fence_before_sync();
+        warp_arrive(&term_full[(T + r) & 1], lane);
+      };
+      build(0);
+      f32x2 dw[2][2][4], wt[2][2][4];
+      w.wait(&dw_full, i & 1, 0x3E);
+      fence_after_sync();
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          if (on(hf, x)) {
+            float d[8];
+            tmem_ld8(tmem + BK_U + lane_off + col_of(hf, x), d);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int i0 = col_of(hf, x) + 2 * j;             // query not earlier than the key
+              dw[hf][x][j] = f2_pack(i0 >= row ? 2.f * d[2 * j] : 0.f, i0 + 1 >= row ? 2.f * d[2 * j + 1] : 0.f);
+              wt[hf][x][j] = f2_bcast(hs.w0);
+            }
+          }
+      fence_before_sync();
+      warp_arrive(&dw_free, lane);
+      const auto drain = [&](int r) {
+        float z[16];
+        tmem_ld16(tmem + BK_Z + lane_off + d0, z);
+        tmem_ld_wait();
+        fence_before_sync();
+        warp_arrive(&z_free, lane);
+        const f32x2 sgn = f2_bcast(r < rpos ? 1.f : -1.f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const ulonglong2 lv = *reinterpret_cast<const ulonglong2*>(l + r * HD + d0 + 4 * j);
+          dk[2 * j] = f2_fma(f2_mul(lv.x, sgn), f2_pack(z[4 * j], z[4 * j + 1]), dk[2 * j]);
+          dk[2 * j + 1] = f2_fma(f2_mul(lv.y, sgn), f2_pack(z[4 * j + 2], z[4 * j + 3]), dk[2 * j + 1]);
+        }
+      };
+      for (int r = 0; r < rank; ++r) {
+        // the next term is built while the MMAs of this one run; its slot's last reader was term r - 1, complete
+        // since u_full[1](r - 1)
+        if (r + 1 < rank) build(r + 1);
+        const f32x2 c2 = f2_bcast(hs.c[r]), sgn = f2_bcast(r < rpos ? 1.f : -1.f);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          w.wait(&u_full[hf], (T + r) & 1, 0x40 + hf);
+          fence_after_sync();
+          float u[2][8];
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            if (on(hf, x)) tmem_ld8(tmem + BK_U + lane_off + col_of(hf, x), u[x]);
+          tmem_ld_wait();
+          fence_before_sync();
+          warp_arrive(&u_free[hf], lane);
+          uint32_t p[2][4];
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            if (on(hf, x)) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const f32x2 u2 = f2_add(f2_pack(u[x][2 * j], u[x][2 * j + 1]), c2);
+                float t0, t1;
+                f2_unpack(f2_mul(dw[hf][x][j], u2), t0, t1);
+                p[x][j] = pack_bf16(t0, t1);
+                wt[hf][x][j] = f2_fma(rpos == rank ? u2 : f2_mul(u2, sgn), u2, wt[hf][x][j]);
+              }
+            }
+          if (r > 0) {                         // the previous term's P^T has been read
+            w.wait(&z_half[hf], (T + r - 1) & 1, 0x42 + hf);
+            fence_after_sync();
+          }
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            if (on(hf, x)) tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, p[x][0], p[x][1], p[x][2], p[x][3]);
+          tmem_st_wait();
+          fence_before_sync();
+          // the whole Z of the previous term is complete: out of the way before the next one starts
+          if (hf == 1 && r > 0) drain(r - 1);
+          warp_arrive(&p_full[hf], lane);
+        }
+      }
+      w.wait(&z_half[0], (T + rank - 1) & 1, 0x44);
+      w.wait(&z_half[1], (T + rank - 1) & 1, 0x45);
+      fence_after_sync();
+      drain(rank - 1);
+      // W^T in the place of P^T, whose last reader is complete
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          if (on(hf, x)) {
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float w_lo, w_hi;
+              f2_unpack(wt[hf][x][j], w_lo, w_hi);
+              const int i0 = col_of(hf, x) + 2 * j;
+              o[j] = pack_bf16(i0 >= row ? w_lo : 0.f, i0 + 1 >= row ? w_hi : 0.f);
+            }
+            tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, o[0], o[1], o[2], o[3]);
+          }
+      tmem_st_wait();
+      fence_before_sync();
+      warp_arrive(&w_full, lane);
+      T += rank;
+    }
+    w.wait(&v_full, (n_heads - 1) & 1, 0x46);
+    fence_after_sync();
+    float z[16], v[16];
+    tmem_ld16(tmem + BK_V + lane_off + d0, z);
     tmem_ld_wait();
 #pragma unroll
-    for (int x = 0; x < 16; ++x) stage_out[row * 65 + 16 * part + x] = vv[x];
-    tmem_ld16(tV + lane_off + 16 * part, vv);
-    tmem_ld_wait();
+    for (int j = 0; j < 8; ++j) f2_unpack(dk[j], v[2 * j], v[2 * j + 1]);
+    if (row < nc && !dead) {
+      // 16 consecutive dims of a row per thread: whole sectors
+      const auto write = [&](float (&x)[16], float* partial, const float* cross, __nv_bfloat16* out) {
+        if (partial) {
+          float* dst = partial + ((((size_t)b * a.Hkv + kvh) * a.parts + part) * a.N + tok0 + row) * HD + d0;
 #pragma unroll
-    for (int x = 0; x < 16; ++x) stage_out[STAGE_OUT_FLOATS + row * 65 + 16 * part + x] = vv[x];
-  }
-  fence_before_sync();
-  __syncthreads();
-  if (!dead) {
-    for (int x = tid; x < 2 * CT * 16; x += KV_THREADS) {   // coalesced write-out, four dims per thread: dk, then dv
-      const int which = x >= CT * 16, xx = x - which * CT * 16;
-      const int r = xx >> 4, seg = xx & 15, j = c * CT + r;
-      float* dst = which ? a.dv_part : a.dk_part;
-      if (j >= a.N || dst == nullptr) continue;
-      const float* sp = stage_out + which * STAGE_OUT_FLOATS + r * 65 + seg * 4;
-      *reinterpret_cast<float4*>(dst + (qoff + j) * HD + seg * 4) = make_float4(sp[0], sp[1], sp[2], sp[3]);
+          for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(dst + 4 * j) = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+        } else if (out) {
+          const size_t o = (koff + row) * HD + d0;
+          if (cross && tok0 + row < a.cross_end) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float4 t = *reinterpret_cast<const float4*>(cross + o + 4 * j);
+              x[4 * j] += t.x; x[4 * j + 1] += t.y; x[4 * j + 2] += t.z; x[4 * j + 3] += t.w;
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            *reinterpret_cast<uint4*>(out + o + 8 * j) =
+                make_uint4(pack_bf16(x[8 * j], x[8 * j + 1]), pack_bf16(x[8 * j + 2], x[8 * j + 3]),
+                           pack_bf16(x[8 * j + 4], x[8 * j + 5]), pack_bf16(x[8 * j + 6], x[8 * j + 7]));
+        }
+      };
+      write(v, a.dk_part, a.dk_cross, a.dk);
+      write(z, a.dv_part, a.dv_cross, a.dv);
     }
   }
+  fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, 512);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
 
-// dk / dv = cross-chunk part (tokens before cross_end) + sum over the query heads of the KV head of the per-head
-// shares, fixed order, cast to bf16.  One thread per 4 consecutive dims of one key token; blockIdx.y: dk, then dv.
+// dk / dv = cross-chunk part (tokens before cross_end) + sum over the parts (groups of query heads of the KV head) of
+// their shares, fixed order, cast to bf16.  One thread per 4 consecutive dims of one key token; blockIdx.y: dk, then dv.
 struct KvReduceArgs {
   const float *part[2], *cross[2];
   __nv_bfloat16* out[2];
-  int B, Hq, Hkv, N, cross_end;
+  int B, Hkv, parts, N, cross_end;
 };
 __global__ void __launch_bounds__(256) kv_head_reduce_kernel(const KvReduceArgs a) {
   const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x;       // over B*Hkv*N*16
@@ -534,63 +733,84 @@ __global__ void __launch_bounds__(256) kv_head_reduce_kernel(const KvReduceArgs 
   const size_t tok = idx >> 4;                                     // (b*Hkv + kvh)*N + n
   const int n = (int)(tok % a.N);
   const size_t bk = tok / a.N;
-  const int kvh = (int)(bk % a.Hkv), b = (int)(bk / a.Hkv), rep = a.Hq / a.Hkv;
   float4 acc = n < a.cross_end ? *reinterpret_cast<const float4*>(cross + tok * HD + 4 * d4) : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float* src = part + (((size_t)b * a.Hq + kvh * rep) * a.N + n) * HD + 4 * d4;
+  const float* src = part + ((bk * a.parts) * a.N + n) * HD + 4 * d4;
 #pragma unroll 8
-  for (int r = 0; r < rep; ++r) {
+  for (int r = 0; r < a.parts; ++r) {
     const float4 t = *reinterpret_cast<const float4*>(src + (size_t)r * a.N * HD);
     acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
   }
   *reinterpret_cast<uint2*>(out + tok * HD + 4 * d4) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
 }
 
-}  // namespace
-
-int OAL_INTRA_NAME(intra_coef_terms)() { return RM; }
-
-static IntraBwdArgs bwd_args(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
-                             int32_t* status, int B, int Hq, int Hkv, int N, int NB) {
+IntraBwdArgs bwd_args(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
+                      int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups) {
   IntraBwdArgs a{};
   a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k);
   a.v = static_cast<const __nv_bfloat16*>(v); a.gimg = static_cast<const __nv_bfloat16*>(gimg);
   a.factors = static_cast<const HeadFactor*>(factors);
   a.status = status;
-  a.N = N; a.NB = NB; a.Hq = Hq; a.Hkv = Hkv;
+  a.N = N; a.NB = NB; a.Hq = Hq; a.Hkv = Hkv; a.rep = Hq / Hkv; a.rank = groups + 1;
   a.gimg_lo_offset = (size_t)B * Hq * NB * SLAB_S_BYTES;
   return a;
 }
 
-cudaError_t OAL_INTRA_NAME(intra_backward_q)(const void* q, const void* k, const void* v, const void* gimg,
-                                             const void* factors, void* dq, const float* dq_init, float* coef_partial,
-                                             int32_t* status, int B, int Hq, int Hkv, int N, int NB, int cross_from,
-                                             cudaStream_t st) {
+}  // namespace
+
+int intra_row_blocks(int N) { return (N + 31) / 32; }
+
+cudaError_t intra_backward_q(const void* q, const void* k, const void* v, const void* gimg,
+                             const void* factors, void* dq, const float* dq_init, float* coef_partial,
+                             int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups, int cross_from,
+                             cudaStream_t st) {
   cudaError_t e = allow_smem<intra_bwd_q_kernel>(BQ_SMEM);
   if (e != cudaSuccess) return e;
-  IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB);
-  a.dq = dq; a.dq_init = dq_init; a.coef_partial = coef_partial; a.cross_from = cross_from;
-  intra_bwd_q_kernel<<<dim3(NB, Hq, B), CTHREADS, BQ_SMEM, st>>>(a);
+  IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB, groups);
+  a.dq = static_cast<__nv_bfloat16*>(dq); a.dq_init = dq_init; a.coef_partial = coef_partial; a.cross_from = cross_from;
+  intra_bwd_q_kernel<<<dim3(NB, B * Hkv, Hq / Hkv), BW_THREADS, BQ_SMEM, st>>>(a);
   return cudaGetLastError();
 }
 
-cudaError_t OAL_INTRA_NAME(intra_backward_kv)(const void* q, const void* k, const void* v, const void* gimg,
-                                              const void* factors, float* dk_part, float* dv_part, int32_t* status,
-                                              int B, int Hq, int Hkv, int N, int NB, cudaStream_t st) {
-  cudaError_t e = allow_smem<intra_bwd_kv_kernel>(BKV_SMEM);
+// Heads of a KV head per CTA of the key/value side: all of them when that still fills the machine (dk and dv then
+// leave the kernel finished: no fp32 partials of every head, no reduction kernel), else the fewest parts that do.
+int intra_kv_parts(int B, int Hq, int Hkv, int NB) {
+  const int rep = Hq / Hkv, groups = B * Hkv * NB, sms = sm_count();
+  int best = 1;
+  double best_cost = 1e30;
+  for (int parts = 1; parts <= rep; ++parts) {
+    const int heads = (rep + parts - 1) / parts;
+    if (parts > 1 && (rep + heads - 1) / heads != parts) continue;       // the same split with fewer parts
+    const int waves = (groups * parts + sms - 1) / sms;
+    // a head costs one unit, the CTA's own prologue and epilogue about half of one, partials another third per head
+    const double cost = waves * (heads + 0.5) + (parts > 1 ? 0.3 * groups * parts / sms : 0.);
+    if (cost < best_cost) { best_cost = cost; best = parts; }
+  }
+  return best;
+}
+
+cudaError_t intra_backward_kv(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
+                              void* dk, void* dv, const float* dk_cross, const float* dv_cross, int cross_end, float* dk_part,
+                              float* dv_part, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups,
+                              cudaStream_t st) {
+  cudaError_t e = allow_smem<intra_bwd_kv_kernel>(BK_SMEM);
   if (e != cudaSuccess) return e;
-  IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB);
-  a.dk_part = dk_part; a.dv_part = dv_part;
-  intra_bwd_kv_kernel<<<dim3(NB, Hq, B), KV_THREADS, BKV_SMEM, st>>>(a);
-  return cudaGetLastError();
-}
-
-// dk, dv: null where not requested; *_cross: fp32 cross-chunk parts of the tokens before cross_end
-cudaError_t OAL_INTRA_NAME(kv_head_reduce)(const float* dk_part, const float* dv_part, const float* dk_cross, const float* dv_cross,
-                                           void* dk, void* dv, int B, int Hq, int Hkv, int N, int cross_end, cudaStream_t st) {
-  KvReduceArgs a{{dk_part, dv_part}, {dk_cross, dv_cross}, {static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv)},
-                 B, Hq, Hkv, N, cross_end};
+  IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB, groups);
+  a.parts = intra_kv_parts(B, Hq, Hkv, NB);
+  a.heads_per_cta = (Hq / Hkv + a.parts - 1) / a.parts;
+  a.cross_end = cross_end;
+  if (a.parts > 1) {
+    a.dk_part = dk ? dk_part : nullptr;
+    a.dv_part = dv ? dv_part : nullptr;
+  } else {
+    a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
+    a.dk_cross = dk_cross; a.dv_cross = dv_cross;
+  }
+  intra_bwd_kv_kernel<<<dim3(NB, B * Hkv, a.parts), BW_THREADS, BK_SMEM, st>>>(a);
+  if (a.parts == 1 || (e = cudaGetLastError()) != cudaSuccess) return cudaGetLastError();
+  KvReduceArgs r{{dk_part, dv_part}, {dk_cross, dv_cross}, {static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv)},
+                 B, Hkv, a.parts, N, cross_end};
   const size_t total = (size_t)B * Hkv * N * 16;
-  kv_head_reduce_kernel<<<dim3((unsigned)((total + 255) / 256), 2), 256, 0, st>>>(a);
+  kv_head_reduce_kernel<<<dim3((unsigned)((total + 255) / 256), 2), 256, 0, st>>>(r);
   return cudaGetLastError();
 }
 

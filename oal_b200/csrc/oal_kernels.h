@@ -20,7 +20,6 @@ constexpr int32_t STATUS_DELIVERED = (int32_t)0x80000000;
 
 struct PairArgs {
   int B, Hq, Hkv, N, G;
-  int window;            // 0: whole causal prefix; >0: keys of the query's own chunk only (multiple of 64)
   int io_dt, out_dt;
   float scale, floor;
   const void *q, *k, *v;
@@ -30,14 +29,10 @@ struct PairArgs {
   // forward
   void* out;
   float *num, *den;
-  int accumulate;        // num/den of tokens from `accumulate_from` on already hold the cross-chunk term
-  int accumulate_from;
   StatusSink sink;       // forward
   // backward
   const float* g;        // [B,Hq,N,80] augmented upstream gradient
   void *dq, *dk, *dv;
-  const float *dq_init, *dk_init, *dv_init;   // fp32 cross-chunk parts to add, or null
-  int q_init_from, kv_init_end;               // ... of query tokens from the first on, of key tokens before the second
   float* coef_partial;   // [B][Hq][tiles][NCOEF] or null
 };
 
@@ -90,7 +85,7 @@ cudaError_t feature_grad(bool query, const void* x, const void* gimg, const void
 cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, int G, const int32_t* dim_perm,
                          const int32_t* group_start, float* dcoef, float* slots, cudaStream_t st);
 cudaError_t norm_vjp_image(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
-                           const float* num, const float* den, float floor_v, float* g, void* gimg, int heads,
+                           const float* num, const float* den, float floor_v, void* gimg, int heads,
                            int N, int NB, int token_major_heads /* > 0: grad_out is [B, N, Hq, 64] */,
                            int32_t* clear_status, cudaStream_t st);
 
@@ -114,18 +109,20 @@ cudaError_t launch_head_prologue(const PrologueArgs& a, int Hq, cudaStream_t st)
 // writes *status | STATUS_DELIVERED to the sink's host word
 cudaError_t deliver_status(const int32_t* status, StatusSink sink, cudaStream_t st);
 
-// ---- tensor-core intra-chunk kernels (oal_intra.cu, oal_intra_bwd.cu): heads with at most 8 groups ----
-int intra_coef_terms();          // terms per head this build handles (rows of the partial-sum triangle)
+// ---- tensor-core intra-chunk kernels (oal_intra.cu, oal_intra_bwd.cu) ----------------------------
+// cross_from: first chunk that has a cross-chunk part in num / den (dq_init)
 cudaError_t intra_forward(const void* q, const void* k, const void* v, const void* factors, void* out, float* num,
-                          float* den, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int out_dt,
+                          float* den, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups, int out_dt,
                           float floor_v, bool out_token_major, int cross_from, StatusSink sink, cudaStream_t st);
+int intra_row_blocks(int N);     // row blocks per head: partial sums of the coefficient gradient
 cudaError_t intra_backward_q(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
                              void* dq, const float* dq_init, float* coef_partial, int32_t* status, int B, int Hq,
-                             int Hkv, int N, int NB, int cross_from, cudaStream_t st);
+                             int Hkv, int N, int NB, int groups, int cross_from, cudaStream_t st);
+int intra_kv_parts(int B, int Hq, int Hkv, int NB);     // CTAs the heads of a KV head are spread over
+// dk, dv: null where not requested; *_cross: fp32 cross-chunk parts of the tokens before cross_end; *_part: scratch of
+// B * Hq * N * 64 floats
 cudaError_t intra_backward_kv(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
-                              float* dk_part, float* dv_part, int32_t* status, int B, int Hq, int Hkv, int N, int NB,
-                              cudaStream_t st);
-cudaError_t kv_head_reduce(const float* dk_part, const float* dv_part, const float* dk_cross, const float* dv_cross,
-                           void* dk, void* dv, int B, int Hq, int Hkv, int N, int cross_end, cudaStream_t st);
+                              void* dk, void* dv, const float* dk_cross, const float* dv_cross, int cross_end, float* dk_part,
+                              float* dv_part, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups, cudaStream_t st);
 
 }  // namespace oal

@@ -5,15 +5,9 @@
 //     s_g(i,j) = sum_{d in g} (scale q_i[d]) k_j[d]
 //     w(i,j)   = A + sum_g B_g s_g + sum_{g,g'} C_gg' s_g s_g'
 // and accumulate  num_i, den_i = sum_{j<=i} w(i,j) [v_j, 1]  together with the
-// first-order gradients.  `window` selects the key range of a query:
-//   window == 0 : the whole causal prefix -> the exact fp32 mode of the operator
-//                 (reference semantics: oal_attention/grouped_reference.py:102-178,
-//                 dense statement tests/operators/test_grouped_quadratic.py:31-84);
-//   window  > 0 : only keys in the query's own chunk of `window` tokens -> the
-//                 intra-chunk term of the chunked scan, added onto the cross-chunk
-//                 term that the state kernels left in num/den (reference:
-//                 oal_attention/hd_block_gemm_runtime.py:530-597 local score, tril,
-//                 score x U; backward oal_attention/hd_block_gemm_backward_wave.py:253-476).
+// first-order gradients, over the whole causal prefix of every query: the exact fp32 mode of the operator
+// (reference semantics: oal_attention/grouped_reference.py:102-178, dense statement
+// tests/operators/test_grouped_quadratic.py:31-84).
 // Dimensions of a head are visited in group-sorted order (dim_perm), so a group is
 // a contiguous range and s_g needs no gather.
 #include "oal_common.cuh"
@@ -87,9 +81,8 @@ __global__ void __launch_bounds__(256) fwd_pairs_kernel(const PairArgs a) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) acc[r][c] = 0.f;
 
-  const int jt_begin = a.window ? ((i0 / a.window) * a.window) / TP : 0;
   const int il = tid & 63, jb = tid >> 6;
-  for (int jt = jt_begin; jt <= it; ++jt) {
+  for (int jt = 0; jt <= it; ++jt) {
     const int j0 = jt * TP;
     load_tile_perm(Ks, a.k, kbase, j0, N, a.io_dt, 1.f, hg.perm, tid);
     for (int x = tid; x < TP * EP; x += 256) {
@@ -158,16 +151,10 @@ __global__ void __launch_bounds__(256) fwd_pairs_kernel(const PairArgs a) {
     const int r = x >> 4, c4 = (x & 15) * 4, i = i0 + r;
     if (i >= N) continue;
     const size_t row = (size_t)(b * a.Hq + h) * N + i;
-    const bool add = a.accumulate && i >= a.accumulate_from;
-    float den = Ys[r * EP + VD];
-    if (add) den += a.den[row];
+    const float den = Ys[r * EP + VD];
     float nv[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) nv[c] = Ys[r * EP + c4 + c];
-    if (add) {
-      const float4 o = *reinterpret_cast<const float4*>(a.num + row * VD + c4);
-      nv[0] += o.x; nv[1] += o.y; nv[2] += o.z; nv[3] += o.w;
-    }
     *reinterpret_cast<float4*>(a.num + row * VD + c4) = make_float4(nv[0], nv[1], nv[2], nv[3]);
     const float dn = fmaxf(den, a.floor);
 #pragma unroll
@@ -180,14 +167,11 @@ __global__ void __launch_bounds__(256) fwd_pairs_kernel(const PairArgs a) {
       else if (!(den > 0.f)) flags |= OAL_STATUS_DENOMINATOR;
     }
   }
-  __syncthreads();           // every thread has read its old den before any is overwritten
   for (int r = tid; r < TP; r += 256) {
     const int i = i0 + r;
     if (i >= N) continue;
     const size_t row = (size_t)(b * a.Hq + h) * N + i;
-    float den = Ys[r * EP + VD];
-    if (a.accumulate && i >= a.accumulate_from) den += a.den[row];
-    a.den[row] = den;
+    a.den[row] = Ys[r * EP + VD];
   }
   if (flags) atomicOr(a.status, flags);
   __syncthreads();
@@ -282,9 +266,8 @@ __global__ void __launch_bounds__(256) bwd_q_pairs_kernel(const PairArgs a) {
 #pragma unroll
   for (int x = 0; x < GCAP * (GCAP + 1) / 2; ++x) cC[x] = 0.f;
 
-  const int jt_begin = a.window ? ((i0 / a.window) * a.window) / TP : 0;
   const int il = tid & 63, jb = tid >> 6;
-  for (int jt = jt_begin; jt <= it; ++jt) {
+  for (int jt = 0; jt <= it; ++jt) {
     const int j0 = jt * TP;
     load_tile_perm(Ks, a.k, kbase, j0, N, a.io_dt, 1.f, hg.perm, tid);
     for (int x = tid; x < E1 * TP; x += 256) {
@@ -382,9 +365,7 @@ __global__ void __launch_bounds__(256) bwd_q_pairs_kernel(const PairArgs a) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const size_t o = qbase + (size_t)i * HD + hg.perm[4 * tx + c];
-        float v = a.scale * acc[r][c];
-        if (a.dq_init && i >= a.q_init_from) v += a.dq_init[o];
-        store_elem(a.dq, o, a.io_dt, v);
+        store_elem(a.dq, o, a.io_dt, a.scale * acc[r][c]);
       }
     }
   }
@@ -429,7 +410,6 @@ __global__ void __launch_bounds__(256) bwd_kv_pairs_kernel(const PairArgs a) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) adu[r][c] = 0.f;
   const int last_tile = (N - 1) / TP;
-  const int it_end = a.window ? min(last_tile, ((j0 / a.window + 1) * a.window) / TP - 1) : last_tile;
   const int jl = tid & 63, ib = tid >> 6;
 
   for (int hh = 0; hh < rep; ++hh) {
@@ -449,7 +429,7 @@ __global__ void __launch_bounds__(256) bwd_kv_pairs_kernel(const PairArgs a) {
       for (int c = 0; c < 4; ++c) adk[r][c] = 0.f;
     const size_t qbase = (size_t)(b * a.Hq + h) * N * HD;
     const size_t gbase = (size_t)(b * a.Hq + h) * N * EP;
-    for (int it = jt; it <= it_end; ++it) {
+    for (int it = jt; it <= last_tile; ++it) {
       const int i0 = it * TP;
       load_tile_perm(Qs, a.q, qbase, i0, N, a.io_dt, a.scale, hg.perm, tid);
       for (int x = tid; x < TP * EP; x += 256) {
@@ -557,9 +537,7 @@ __global__ void __launch_bounds__(256) bwd_kv_pairs_kernel(const PairArgs a) {
       const int r = x >> 6, j = j0 + r;
       if (j >= N) continue;
       const size_t o = kbase + (size_t)j * HD + (x & 63);
-      float v = dkacc[x];
-      if (a.dk_init && j < a.kv_init_end) v += a.dk_init[o];
-      store_elem(a.dk, o, a.io_dt, v);
+      store_elem(a.dk, o, a.io_dt, dkacc[x]);
     }
   }
   if (a.dv) {
@@ -572,9 +550,7 @@ __global__ void __launch_bounds__(256) bwd_kv_pairs_kernel(const PairArgs a) {
         const int e = 5 * tx + c;
         if (e >= VD) continue;
         const size_t o = kbase + (size_t)j * VD + e;
-        float v = adu[r][c];
-        if (a.dv_init && j < a.kv_init_end) v += a.dv_init[o];
-        store_elem(a.dv, o, a.io_dt, v);
+        store_elem(a.dv, o, a.io_dt, adu[r][c]);
       }
     }
   }

@@ -159,12 +159,11 @@ __device__ __forceinline__ void head_prologue(const PrologueArgs& a, int h, Prol
     const int q = x / RMAX_ALL, r = x % RMAX_ALL;
     out.t[q][r] = (q < n && r < n) ? s.V[q][r] / s.lam[r] : 0.f;
   }
-  if (tid < RMAX_ALL) out.c[tid] = tid < n ? s.lam[tid] * s.V[0][tid] : 0.f;
+  if (tid < RMAX_ALL) out.s.c[tid] = tid < n ? s.lam[tid] * s.V[0][tid] : 0.f;
   if (tid == 0) {
-    out.rank = n;
-    out.rpos = n;
-    out.w0 = a.eps;
-    out.pad = 0;
+    out.s.rank = n;
+    out.s.rpos = n;
+    out.s.w0 = a.eps;
   }
 }
 

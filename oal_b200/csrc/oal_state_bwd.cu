@@ -676,14 +676,13 @@ __global__ void __launch_bounds__(32 * SLOT_WARPS) dcoef_slots_kernel(const floa
   }
 }
 
-// normalisation VJP writing the bf16 operand images of G (hi, lo) and, when `g` is given, its fp32 rows
+// normalisation VJP writing the bf16 operand images of G (hi, lo)
 //   CTA = 32 consecutive tokens of one (head, chunk); warp = 8 consecutive columns, lane = token, so a
 //   warp stores 512 contiguous bytes of an image chunk.  Rows are enumerated over padded chunks so
 //   that tail tokens of the last chunk are zeroed.
 __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_out, int out_dt, const float* grad_num,
                                                              const float* grad_den, const float* num,
-                                                             const float* den, float floor_v, float* g,
-                                                             __nv_bfloat16* gimg, int N, int NB, int heads,
+                                                             const float* den, float floor_v, __nv_bfloat16* gimg, int N, int NB, int heads,
                                                              int tm_heads, int32_t* status) {
   __shared__ float part[8][32];
   if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;     // first kernel of the backward
@@ -744,10 +743,6 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
     img[ec * CT + tl] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     img_lo[ec * CT + tl] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
-  if (g && live) {
-    *reinterpret_cast<float4*>(g + row * EP + 8 * ec) = make_float4(gv[0], gv[1], gv[2], gv[3]);
-    *reinterpret_cast<float4*>(g + row * EP + 8 * ec + 4) = make_float4(gv[4], gv[5], gv[6], gv[7]);
-  }
   __syncthreads();
   if (ec < 2) {            // columns 64..79: [d den, 0 x 15]
     float gd = 0.f;
@@ -761,10 +756,6 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
     const __nv_bfloat16 h0 = __float2bfloat16_rn(gd);
     img[(VD / 8 + ec) * CT + tl] = make_uint4((uint32_t)__bfloat16_as_ushort(h0), 0u, 0u, 0u);
     img_lo[(VD / 8 + ec) * CT + tl] = make_uint4(pack_bf16(gd - __bfloat162float(h0), 0.f), 0u, 0u, 0u);
-    if (g && live) {
-      *reinterpret_cast<float4*>(g + row * EP + VD + 8 * ec) = make_float4(gd, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(g + row * EP + VD + 8 * ec + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
   }
 }
 
@@ -814,11 +805,11 @@ cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, int G, const i
 }
 
 cudaError_t norm_vjp_image(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
-                           const float* num, const float* den, float floor_v, float* g, void* gimg, int heads,
+                           const float* num, const float* den, float floor_v, void* gimg, int heads,
                            int N, int NB, int token_major_heads, int32_t* clear_status, cudaStream_t st) {
   const size_t rows = (size_t)heads * NB * CT;      // a multiple of 32
   norm_vjp_image_kernel<<<(unsigned)(rows / 32), 256, 0, st>>>(grad_out, out_dt, grad_num, grad_den, num, den,
-                                                                   floor_v, g, static_cast<__nv_bfloat16*>(gimg), N,
+                                                                   floor_v, static_cast<__nv_bfloat16*>(gimg), N,
                                                                    NB, heads, token_major_heads, clear_status);
   return cudaGetLastError();
 }
