@@ -246,8 +246,13 @@ struct BackwardSpace {
   float* g;
   float* coef_pairs;
   float* dcoefs;
+  float *dk_part, *dv_part;
   size_t bytes;
 };
+
+int coef_slots_pairs(const OalProblem* p) {
+  return oal::pairs_tiles(p->seq_len) * oal::pairs_split(p->batch, p->q_heads, p->seq_len);
+}
 
 size_t coef_floats(const OalProblem* p) { return (size_t)p->q_heads * (1 + p->groups + p->groups * p->groups); }
 
@@ -256,8 +261,11 @@ BackwardSpace carve_backward(const OalProblem* p, void* ws) {
   BackwardSpace s;
   const size_t rows = (size_t)p->batch * p->q_heads * p->seq_len;
   s.g = c.take<float>(rows * oal::EP);
-  s.coef_pairs = c.take<float>((size_t)p->batch * p->q_heads * oal::pairs_tiles(p->seq_len) * oal::NCOEF);
+  s.coef_pairs = c.take<float>((size_t)p->batch * p->q_heads * coef_slots_pairs(p) * oal::NCOEF);
   s.dcoefs = c.take<float>(coef_floats(p));
+  const size_t shares = p->q_heads > p->kv_heads ? rows * oal::HD : 0;
+  s.dk_part = c.take<float>(shares);
+  s.dv_part = c.take<float>(shares);
   s.bytes = c.off;
   return s;
 }
@@ -469,7 +477,7 @@ int finish_coefs(const OalProblem* p, const CoefSource& src, const CoefSink& sin
     e = factors ? oal::intra_coef_finish(partial, oal::intra_row_blocks(p->seq_len), rm * (rm + 1) / 2 + rm + 1, rm, factors, slots, p->batch,
                                          p->q_heads, p->groups, sink.dA, sink.dB, sink.dC, fused ? src.factor : nullptr,
                                          fused ? sink.dfactor : nullptr, st)
-                : oal::reduce_coefs(partial, oal::pairs_tiles(p->seq_len), slots, p->batch, p->q_heads, p->groups,
+                : oal::reduce_coefs(partial, coef_slots_pairs(p), slots, p->batch, p->q_heads, p->groups,
                                     sink.dA, sink.dB, sink.dC, st); }
   if (e != cudaSuccess) return fail_cuda(e, "coefficient reduction kernel");
   if (sink.dfactor && !fused) {
@@ -510,21 +518,30 @@ int backward_core_fp32(const OalProblem* p, const BackwardArgs& x, const CoefSou
   if (e != cudaSuccess) return fail_cuda(e, "normalisation VJP kernel");
   oal::PairArgs a = base_args(p, x.q, x.k, x.v, x.dim_perm, x.group_start, src, x.status);
   a.g = s.g;
+  const bool want_kv = mask & (OAL_GRAD_K | OAL_GRAD_V);
+  // The two sides share no buffer: the key/value side fills the SMs that the last blocks of the query side leave idle
+  // (all but a few SMs in a short call).
+  std::unique_lock<std::mutex> side_lock;
+  SideStreams* side = side_streams(side_lock);
+  cudaStream_t skv = want_kv ? fork_to(side, 0, st) : st;
   if (mask & (OAL_GRAD_Q | OAL_GRAD_COEF)) {
     a.dq = (mask & OAL_GRAD_Q) ? x.dq : nullptr;
     a.coef_partial = (mask & OAL_GRAD_COEF) ? s.coef_pairs : nullptr;
     { LaunchScope scope("pairs_backward_q", st); e = oal::pairs_backward_q(a, st); }
     if (e != cudaSuccess) return fail_cuda(e, "backward query-side pair kernel");
-    if (mask & OAL_GRAD_COEF)
-      if (int rc = finish_coefs(p, src, sink, s.coef_pairs, nullptr, nullptr, st)) return rc;
   }
-  if (mask & (OAL_GRAD_K | OAL_GRAD_V)) {
+  if (want_kv) {
     a.dq = nullptr; a.coef_partial = nullptr;
+    a.dk_part = s.dk_part; a.dv_part = s.dv_part;
     a.dk = (mask & OAL_GRAD_K) ? x.dk : nullptr;
     a.dv = (mask & OAL_GRAD_V) ? x.dv : nullptr;
-    { LaunchScope scope("pairs_backward_kv", st); e = oal::pairs_backward_kv(a, st); }
-    if (e != cudaSuccess) return fail_cuda(e, "backward key/value-side pair kernel");
+    { LaunchScope scope("pairs_backward_kv", skv, p->q_heads > p->kv_heads ? 2 : 1); e = oal::pairs_backward_kv(a, skv); }
+    if (e != cudaSuccess) return fail_cuda(e, "backward key/value-side pair kernels");
+    join_mark(side, 0, skv, st);
   }
+  if (mask & OAL_GRAD_COEF)
+    if (int rc = finish_coefs(p, src, sink, s.coef_pairs, nullptr, nullptr, st)) return rc;
+  if (want_kv) join_wait(side, 0, skv, st);
   return OAL_OK;
 }
 

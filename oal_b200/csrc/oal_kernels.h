@@ -33,13 +33,17 @@ struct PairArgs {
   // backward
   const float* g;        // [B,Hq,N,80] augmented upstream gradient
   void *dq, *dk, *dv;
-  float* coef_partial;   // [B][Hq][tiles][NCOEF] or null
+  float* coef_partial;   // [B][Hq][tiles][split][NCOEF] or null
+  float *dk_part, *dv_part;      // [B,Hq,N,64] fp32, where a KV head has several query heads
+  // set by the launch: 64-token tiles, CTAs that share a tile, which of q, k, v (bits) allow loads of four elements
+  int tiles, split, vec;
 };
 
 cudaError_t pairs_forward(const PairArgs& a, cudaStream_t st);
 cudaError_t pairs_backward_q(const PairArgs& a, cudaStream_t st);
 cudaError_t pairs_backward_kv(const PairArgs& a, cudaStream_t st);
 int pairs_tiles(int n);
+int pairs_split(int B, int Hq, int N);      // partial sums of the coefficient gradient per tile
 
 cudaError_t norm_vjp(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                      const float* num, const float* den, float floor_v, float* g, size_t rows,
