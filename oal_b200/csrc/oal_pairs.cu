@@ -15,14 +15,14 @@
 //   * tiles are stored transposed, [dimension in group order][token], row pitch 68: a warp of 8 x 4 threads reads
 //     four owner tokens per thread and JP others in one wavefront each, JP x 4 FMAs per dimension; threads that
 //     walk tokens of one dimension (lanes over dimensions) read four tokens per conflict-free load;
-//   * a thread keeps all group scores of its 4 x JP pairs in registers, JP such that they are 64;
+//   * a thread keeps all group scores of its 4 x JP pairs in registers, 64 or 128 of them;
 //   * per-group weight gradients go through shared memory once, and a thread then owns 16 tokens of ONE
 //     dimension, so that the group of its dimension is fixed.
 // Clusters of up to 8 CTAs share an owner tile when there are too few tiles to fill the chip: each takes every
 // S-th tile of the other side, and the partial sums meet through distributed shared memory in rank order.
 //
 // Measured against one pair per (thread, key slot) with scalar shared-memory reads, us: 14 / 2 heads, N = 2048,
-// 8 groups: forward 955 -> 398, query side 2500 -> 750, key/value side 8124 -> 867 with its reduction; 2 heads,
+// 8 groups: forward 955 -> 398, query side 2500 -> 681, key/value side 8124 -> 867 with its reduction; 2 heads,
 // N = 256, 4 groups: 76 -> 22, 119 -> 21, 126 -> 25.
 // Dimensions of a head are visited in group-sorted order (dim_perm), so a group is
 // a contiguous range and s_g needs no gather.
@@ -46,9 +46,14 @@ __device__ __forceinline__ int tri_index(int g, int g2) {   // g <= g2 < GMAX
   return g * GMAX - (g * (g - 1)) / 2 + (g2 - g);
 }
 
-template <int GCAP>
+// JP by group capacity.  At 8 groups the query side takes 4 (128 scores, 255 registers: 681 us at N = 2048, 14 heads,
+// against 750 with 2); the forward is faster with 2 and two CTAs per SM (398 us against 451 with 4 and one), the
+// key/value side spills with 4.
+constexpr int jp(int gcap) { return gcap <= 4 ? 4 : gcap <= 8 ? 2 : 1; }
+constexpr int jp_q(int gcap) { return gcap <= 8 ? 4 : 1; }
+template <int GCAP, int JPT>
 struct PairCfg {
-  static constexpr int JP = GCAP <= 4 ? 4 : GCAP <= 8 ? 2 : 1;     // 4 x JP pairs per thread: 64 scores in registers
+  static constexpr int JP = JPT;     // 4 x JP pairs per thread
   static constexpr int SUB = 16 * JP;                              // tokens of the other side per pass
   static constexpr int GS = SUB * TP + 4;                          // group stride of the weight gradients
 };
@@ -261,7 +266,7 @@ __device__ __forceinline__ void sync_ranks(int split) {
 // ---------------------------------------------------------------------------
 template <int GCAP>
 __global__ void __launch_bounds__(THREADS, 2) fwd_pairs_kernel(const PairArgs a) {
-  using Cfg = PairCfg<GCAP>;
+  using Cfg = PairCfg<GCAP, jp(GCAP)>;
   constexpr int JP = Cfg::JP;
   extern __shared__ __align__(16) float sm[];
   float* Qt = sm;                 // [64 d][68]  scaled, group order
@@ -408,7 +413,7 @@ __device__ __forceinline__ void block_reduce_coefs(float cA, const float (&cB)[G
 
 template <int GCAP>
 __global__ void __launch_bounds__(THREADS, 1) bwd_q_pairs_kernel(const PairArgs a) {
-  using Cfg = PairCfg<GCAP>;
+  using Cfg = PairCfg<GCAP, jp_q(GCAP)>;
   constexpr int JP = Cfg::JP, SUB = Cfg::SUB, GS = Cfg::GS;
   extern __shared__ __align__(16) float sm[];
   float* Qt = sm;                     // [64 d][68]  scaled, group order; at the end the sums [64 i][64 d]
@@ -535,7 +540,7 @@ __global__ void __launch_bounds__(THREADS, 1) bwd_q_pairs_kernel(const PairArgs 
 // ---------------------------------------------------------------------------
 template <int GCAP>
 __global__ void __launch_bounds__(THREADS, 1) bwd_kv_pairs_kernel(const PairArgs a) {
-  using Cfg = PairCfg<GCAP>;
+  using Cfg = PairCfg<GCAP, jp(GCAP)>;
   constexpr int IP = Cfg::JP, SUB = Cfg::SUB, GS = Cfg::GS;
   extern __shared__ __align__(16) float sm[];
   float* Kt = sm;                     // [64 d][68]  group order; at the end the sums of dk [64 j][64 d]
@@ -744,10 +749,10 @@ __global__ void reduce_coefs_kernel(const float* p0, int tiles0, const float* ex
 template <int GCAP>
 constexpr size_t fwd_smem() { return sizeof(float) * (2 * TT + 2 * TP * TP); }
 template <int GCAP>
-constexpr size_t bwd_q_smem() { return sizeof(float) * (4 * TT + TP + GCAP * PairCfg<GCAP>::GS); }
+constexpr size_t bwd_q_smem() { return sizeof(float) * (4 * TT + TP + GCAP * PairCfg<GCAP, jp_q(GCAP)>::GS); }
 template <int GCAP>
 constexpr size_t bwd_kv_smem() {
-  return sizeof(float) * (4 * TT + TP * TP + TP + PairCfg<GCAP>::SUB * TP + GCAP * PairCfg<GCAP>::GS);
+  return sizeof(float) * (4 * TT + TP * TP + TP + PairCfg<GCAP, jp(GCAP)>::SUB * TP + GCAP * PairCfg<GCAP, jp(GCAP)>::GS);
 }
 
 // Launch with clusters of a.split CTAs.
