@@ -210,8 +210,8 @@ int check_problem(const OalProblem* p) {
   }
   if (!(p->floor > 0.f)) return fail(OAL_ERR_ARGUMENT, "floor must be positive");
   if (p->flags & ~(OAL_FLAG_OUT_TOKEN_MAJOR | OAL_FLAG_ZERO_STATE_IN)) return fail(OAL_ERR_ARGUMENT, "unknown bits in flags");
-  if ((p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) && p->precision != OAL_PRECISION_BF16_TENSORCORE)
-    return fail(OAL_ERR_ARGUMENT, "token-major out needs bf16_tensorcore");
+  if ((p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) && (p->precision != OAL_PRECISION_BF16_TENSORCORE || p->groups > 8))
+    return fail(OAL_ERR_ARGUMENT, "token-major out needs bf16_tensorcore and at most 8 groups per head");
   return OAL_OK;
 }
 
@@ -425,6 +425,19 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
     if (!update) {
       LaunchScope scope("head_prologue", st, 1, timing);
       if ((e = oal::launch_head_prologue(pro, p->q_heads, st)) != cudaSuccess) return fail_cuda(e, "prologue kernel");
+    } else if (timing && (side = side_streams(side_lock))) {
+      // The rotations (11 us at 8 groups, 45 at 16) are needed by the call's last kernel only, the coefficients by the
+      // next but one: with both in the state kernel's launch the scan waited for the rotations.  Beside the state
+      // kernels they cost the host a launch and two events.  14 / 2 heads, B = 1, both forms in us: forward + backward
+      // N = 256 169 -> 160, N = 1024 198 -> 190, replayed 203 -> 192, 16 groups N = 4096 663 -> 647.
+      s0 = fork_to(side, 0, st);
+      oal::PrologueArgs own = pro;
+      own.A = own.B = own.C = own.coef_table = nullptr;
+      own.status = own.counter = nullptr;
+      pro.factors = nullptr;
+      LaunchScope scope("head_prologue", s0, 1, timing);
+      if ((e = oal::launch_head_prologue(own, p->q_heads, s0)) != cudaSuccess) return fail_cuda(e, "prologue kernel");
+      join_mark(side, 0, s0, st);
     }
   } else if (tc) {
     // explicit coefficients: the factor table (rotations of a possibly indefinite matrix, 50 us) is needed by the

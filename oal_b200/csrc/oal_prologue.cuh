@@ -1,4 +1,5 @@
-// Per-head prologue of a forward call, one block per query head: packed factor row L (lower triangular,
+// Per-head prologue of a forward call, one block per query head, in one launch or in two (coefficients and their table
+// beside the state update's blocks, the factor table on a side stream): packed factor row L (lower triangular,
 // M = L L^T + eps e0 e0^T) -> coefficients A, B, C, the coefficient table of the state kernels and the
 // factor table of the intra-chunk kernels.
 //
@@ -20,7 +21,7 @@ struct PrologueArgs {
   int factor_rows, G;
   float eps, scale;
   const int32_t *dim_perm, *group_start;
-  float *A, *B, *C;                  // outputs [Hq], [Hq,G], [Hq,G,G]
+  float *A, *B, *C;                  // outputs [Hq], [Hq,G], [Hq,G,G], or all null
   float* coef_table;                 // output [Hq, F_ROWS], or null (no state kernels follow)
   HeadFactor* factors;               // output, or null (no tensor-core intra-chunk kernels follow)
   int32_t *status, *counter;         // cleared by block 0 (each may be null)
@@ -128,6 +129,7 @@ __device__ __forceinline__ void head_prologue(const PrologueArgs& a, int h, Prol
     float m = 0.f;
     for (int k = 0; k <= min(i, j); ++k) m = fmaf(s.L[i][k], s.L[j][k], m);
     s.M[i][j] = m;
+    if (!a.A) continue;
     if (i == 0 && j == 0) a.A[h] = m + a.eps;
     else if (i == 0) a.B[(size_t)h * a.G + j - 1] = 2.f * m;
     else if (j > 0) a.C[((size_t)h * a.G + i - 1) * a.G + j - 1] = m;
