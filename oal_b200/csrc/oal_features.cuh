@@ -184,10 +184,21 @@ __device__ __forceinline__ void raw_chunks_impl(const uint32_t (&xp)[HD / 2], ui
                                                 std::integer_sequence<int, J...>) {
   ((tile[(J0 + J) * CT] = raw_chunk<S * 16 + J0 + J>(xp)), ...);
 }
-template <int S, int J0, int... J>
-__device__ __forceinline__ void coef_chunks_impl(const f32x2 (&xq)[HD / 2], const float* coef, uint4* tile,
-                                                 std::integer_sequence<int, J...>) {
-  ((tile[(J0 + J) * CT] = coef_chunk<S * 16 + J0 + J>(xq, coef)), ...);
+// Four chunks of slab S of one token, from chunk J0, as columns of the MMA's A operand in tensor memory (a feature pair
+// per column; `slot`: the slab's first column at this warp's lanes).
+template <int S, int J0>
+__device__ __forceinline__ void coef_chunks_to_tmem(uint32_t slot, const f32x2 (&xq)[HD / 2], const float* coef) {
+  const uint4 c0 = coef_chunk<S * 16 + J0>(xq, coef), c1 = coef_chunk<S * 16 + J0 + 1>(xq, coef);
+  const uint4 c2 = coef_chunk<S * 16 + J0 + 2>(xq, coef), c3 = coef_chunk<S * 16 + J0 + 3>(xq, coef);
+  const uint32_t w[16] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w, c2.x, c2.y, c2.z, c2.w, c3.x, c3.y, c3.z, c3.w};
+  umma::tmem_st16(slot + 4 * J0, w);
+}
+template <int S, int J0>
+__device__ __forceinline__ void raw_chunks_to_tmem(uint32_t slot, const uint32_t (&xp)[HD / 2]) {
+  const uint4 c0 = raw_chunk<S * 16 + J0>(xp), c1 = raw_chunk<S * 16 + J0 + 1>(xp);
+  const uint4 c2 = raw_chunk<S * 16 + J0 + 2>(xp), c3 = raw_chunk<S * 16 + J0 + 3>(xp);
+  const uint32_t w[16] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w, c2.x, c2.y, c2.z, c2.w, c3.x, c3.y, c3.z, c3.w};
+  umma::tmem_st16(slot + 4 * J0, w);
 }
 
 #define OAL_SLAB_SWITCH(s, CASE)                                                                      \
@@ -215,12 +226,31 @@ __device__ __forceinline__ void write_half_slab_raw(int s, int half, const uint3
   if (half == 0) write_half_slab_raw_impl<0>(s, xp, tile);
   else write_half_slab_raw_impl<8>(s, xp, tile);
 }
-__device__ __forceinline__ void write_half_slab_coef(int s, int half, const f32x2 (&xq)[HD / 2], const float* coef,
-                                                     uint4* tile) {
-#define OAL_CASE(S)                                                                                 \
-  case S:                                                                                           \
-    if (half == 0) coef_chunks_impl<S, 0>(xq, coef, tile, std::make_integer_sequence<int, 8>{});    \
-    else coef_chunks_impl<S, 8>(xq, coef, tile, std::make_integer_sequence<int, 8>{});              \
+// The same half as columns of the A operand in tensor memory; `half` is the same for the lanes of a warp.
+__device__ __forceinline__ void store_half_slab_raw(int s, int half, const uint32_t (&xp)[HD / 2], uint32_t slot) {
+#define OAL_CASE(S)                        \
+  case S:                                  \
+    if (half == 0) {                       \
+      raw_chunks_to_tmem<S, 0>(slot, xp);  \
+      raw_chunks_to_tmem<S, 4>(slot, xp);  \
+    } else {                               \
+      raw_chunks_to_tmem<S, 8>(slot, xp);  \
+      raw_chunks_to_tmem<S, 12>(slot, xp); \
+    }                                      \
+    break;
+  OAL_SLAB_SWITCH(s, OAL_CASE)
+#undef OAL_CASE
+}
+__device__ __forceinline__ void store_half_slab_coef(int s, int half, const f32x2 (&xq)[HD / 2], const float* coef, uint32_t slot) {
+#define OAL_CASE(S)                               \
+  case S:                                         \
+    if (half == 0) {                              \
+      coef_chunks_to_tmem<S, 0>(slot, xq, coef);  \
+      coef_chunks_to_tmem<S, 4>(slot, xq, coef);  \
+    } else {                                      \
+      coef_chunks_to_tmem<S, 8>(slot, xq, coef);  \
+      coef_chunks_to_tmem<S, 12>(slot, xq, coef); \
+    }                                             \
     break;
   OAL_SLAB_SWITCH(s, OAL_CASE)
 #undef OAL_CASE

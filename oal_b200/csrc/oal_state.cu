@@ -225,15 +225,24 @@ struct CrossReadArgs {
 // Persistent, warp-specialised kernel.  Work items are (batch, head, chunk) with the heads of one
 // state unit adjacent, so CTAs running at the same time read the same state image from L2.  CTA k
 // takes items k, k + gridDim.x, ...; the flat iteration `it` = (item, slab) drives four roles:
-//   warps 0-7   generate feature slab `slab` of the item's 128 tokens into A[it % 3]
-//   warp  13    lane 0 streams the state slab images into a 4-slot ring and the head's coefficient
+//   warps 0-7   generate feature slab `slab` of the item's 128 tokens into tensor memory, A[it % 4]
+//   warp  13    lane 0 streams the state slab images into a 6-slot ring and the head's coefficient
 //               table into one of two buffers (bulk copies)
 //   warp  12    lane 0 issues the MMAs  acc[item & 1] += A . S  once both are full
 //   warps 8-11  after the item's last slab: accumulator -> HBM, then release it
+// What bounded it: shared memory.  With the slabs there an MMA of 128 x 80 x 16 reads 6.5 KB (53 clocks at 128 bytes
+// per clock), a slab is written and read at 32 KB each beside the 20 KB of state that arrive and are read: 970 of the
+// 1550 clocks a slab took.  A token is a tensor-memory lane and its thread writes the slab's columns itself, which
+// leaves the state image alone in shared memory.  Generating with 16 warps
+// and copying a quarter of the state changed nothing before that.  14 / 2 heads, B = 4, N = 4096: 187 -> 156 us
+// (QUERY), 32 -> 26 (not).
 constexpr int CR_GEN_WARPS = 8, CR_EPI_WARPS = 4;
 constexpr int CR_ISSUER = CR_GEN_WARPS + CR_EPI_WARPS, CR_LOADER = CR_ISSUER + 1;
 constexpr int CR_THREADS = (CR_LOADER + 1) * 32;
-constexpr int CR_ARING = 3, CR_SRING = 4;
+constexpr int CR_ARING = 4, CR_SRING = 6;
+// tensor memory: ring of feature slabs (128 features of the 128 tokens, two per column), two accumulators
+constexpr uint32_t CR_SLAB_COLS = 64, CR_ACC = CR_ARING * CR_SLAB_COLS;
+static_assert(CR_ACC + 2 * EP <= 512, "tensor-memory columns of the cross-read kernel");
 static_assert(CR_GEN_WARPS * 32 == GEN_THREADS, "the slab generator is written for GEN_THREADS threads");
 
 struct CrItem {
@@ -253,8 +262,7 @@ __device__ __forceinline__ CrItem cr_item(int item, int H, int rep, int NC, int 
 template <bool QUERY>
 __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossReadArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* Abuf = smem;                                   // CR_ARING x SLAB_A_BYTES
-  unsigned char* Sbuf = smem + CR_ARING * SLAB_A_BYTES;         // CR_SRING x SLAB_S_BYTES, then the head's coefficient table
+  unsigned char* Sbuf = smem;                                   // CR_SRING x SLAB_S_BYTES, then the head's coefficient table
   __shared__ uint64_t full_a[CR_ARING], a_free[CR_ARING], s_full[CR_SRING], s_free[CR_SRING], acc_full[2], acc_free[2];
   __shared__ uint64_t coef_full[2], coef_free[2];
   __shared__ uint32_t tmem_base;
@@ -262,7 +270,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int n_items = a.B * a.H * a.NC;
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-  if (warp == CR_ISSUER) tmem_alloc(&tmem_base, 256);
+  if (warp == CR_ISSUER) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
     for (int s = 0; s < CR_ARING; ++s) {
       mbar_init(&full_a[s], CR_GEN_WARPS);
@@ -289,7 +297,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
 
   if (warp < CR_GEN_WARPS) {
     // ---------------- generators: thread = (token, half of the slab's chunks) ----------------
-    const int token = tid & 127, half = tid >> 7;
+    const int token = tid & 127, half = warp >> 2;
     int s3 = 0, use = 0;
     for (int k = 0; k < my_items; ++k) {
       const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
@@ -302,15 +310,18 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
       if constexpr (QUERY) unpack_row(xp, xq);
       for (int s = 0; s < F_SLABS; ++s) {
         if (use > 0) w.wait(&a_free[s3], (use - 1) & 1, 0x41);      // the MMAs that read A[s3] have completed
-        uint4* tile = reinterpret_cast<uint4*>(Abuf + s3 * SLAB_A_BYTES) + token;
+        __syncwarp();
+        fence_after_sync();
+        const uint32_t slot = tmem + s3 * CR_SLAB_COLS + ((uint32_t)(32 * (warp & 3)) << 16);
         if constexpr (QUERY) {
           keep_in_loop(xq);
-          write_half_slab_coef(s, half, xq, coef, tile);
+          store_half_slab_coef(s, half, xq, coef, slot);
         } else {
           keep_in_loop(xp);
-          write_half_slab_raw(s, half, xp, tile);
+          store_half_slab_raw(s, half, xp, slot);
         }
-        fence_async_smem();
+        tmem_st_wait();
+        fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&full_a[s3]);
         if (++s3 == CR_ARING) { s3 = 0; ++use; }
@@ -329,7 +340,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
       const size_t orow = (size_t)(it.b * a.H + it.h) * a.N + row;
       w.wait(&acc_full[k & 1], (k >> 1) & 1, 0x42);
       fence_after_sync();
-      const uint32_t t = tmem + (k & 1) * EP + lane_off;
+      const uint32_t t = tmem + CR_ACC + (k & 1) * EP + lane_off;
 #pragma unroll
       for (int cc = 0; cc < EP; cc += 16) {
         if (cc < VD || QUERY) {
@@ -356,20 +367,21 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
     // ---------------- MMA issue ----------------
     if (elect_one()) {
       const uint32_t idesc = instr_desc_bf16(128, EP, 0, 1);
-      // descriptors of slot 0 of both rings, advanced by adds: this thread is the serial path of every slab
-      const uint64_t da0 = smem_desc(smem_u32(Abuf), CT * 16, 128), ds0 = smem_desc(smem_u32(Sbuf), 128, 128 * 16);
+      // descriptor of slot 0 of the image ring, advanced by adds: this thread is the serial path of every slab
+      const uint64_t ds0 = smem_desc(smem_u32(Sbuf), 128, 128 * 16);
       int s3 = 0, use = 0, gs = 0, guse = 0;
       for (int k = 0; k < my_items; ++k) {
-        const uint32_t tacc = tmem + (k & 1) * EP;
+        const uint32_t tacc = tmem + CR_ACC + (k & 1) * EP;
         if (k >= 2) w.wait(&acc_free[k & 1], ((k >> 1) - 1) & 1, 0x43);   // item k-2 has left this accumulator
         for (int s = 0; s < F_SLABS; ++s) {
-          const uint64_t da = desc_advance(da0, s3 * SLAB_A_BYTES), dsl = desc_advance(ds0, gs * SLAB_S_BYTES);
+          const uint64_t dsl = desc_advance(ds0, gs * SLAB_S_BYTES);
+          const uint32_t slab = tmem + s3 * CR_SLAB_COLS;
           w.wait(&full_a[s3], use & 1, 0x44);
           w.wait(&s_full[gs], guse & 1, 0x45);
           fence_after_sync();
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks)       // 16 features per step
-            mma_bf16_ss(tacc, desc_advance(da, ks * 2 * CT * 16), desc_advance(dsl, ks * 256), idesc, (s > 0 || ks > 0));
+            mma_bf16_ts(tacc, slab + 8 * ks, desc_advance(dsl, ks * 256), idesc, (s > 0 || ks > 0));
           mma_commit(&a_free[s3]);
           mma_commit(&s_free[gs]);
           if (s == F_SLABS - 1) mma_commit(&acc_full[k & 1]);
@@ -406,7 +418,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
   }
   fence_before_sync();
   __syncthreads();
-  if (warp == CR_ISSUER) tmem_dealloc(tmem_base, 256);
+  if (warp == CR_ISSUER) tmem_dealloc(tmem_base, 512);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
 
@@ -444,7 +456,7 @@ cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float
 cudaError_t cross_read(bool query, const void* x, const void* image, const float* coef_table, float* out64,
                        float* out1, int B, int H, int rep, int N, int NB, int c0, int NC, int32_t* status,
                        cudaStream_t st) {
-  const int smem = CR_ARING * SLAB_A_BYTES + CR_SRING * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float);
+  const int smem = CR_SRING * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float);
   CrossReadArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(image), coef_table,
                   out64, out1, N, NB, H, rep, B, c0, NC, status};
   cudaError_t e;
