@@ -582,15 +582,16 @@ def run_gpu_arm(args) -> None:
             "intra_backward_q": intra,         # dW and dq
             "intra_backward_kv": intra,        # dk and dv
         }
-        # MMA FLOPs the intra-chunk kernels really execute per launch: stacked tile of 16 (G + 1) columns per
-        # 16-key tile, 8 tiles per 128-token chunk under the causal mask as full 128-row tiles, the constant K
-        # step (64 + 16), value + remainder chains on the backward side, dW over the 80-long value axis twice
-        nr, ctas = 16 * (w["g"] + 1), w["batch"] * w["hq"] * (w["n"] // KERNEL_CHUNK)
-        u_hi, u_lo = 2 * 128 * nr * 80, 2 * 128 * nr * 64
+        # MMA FLOPs the intra-chunk kernels really execute per launch, per 128-token chunk: G + 1 terms, each a chain
+        # over K = 64 of value + remainder against the other side's rows.  Query-side tiles hold four 32-row blocks
+        # and see only the keys of the last one; the key/value side walks all 128 queries of a head.
+        terms, rep, chunks = w["g"] + 1, w["hq"] // w["hkv"], w["batch"] * w["hkv"] * (w["n"] // KERNEL_CHUNK)
+        seen = chunks * sum(32 * (4 - 4 * x // rep) for x in range(rep))       # key columns of all query-side tiles
+        rows = chunks * rep * 128                                             # query columns of the key/value side
         executed_flops = {
-            "intra_forward": ctas * 8 * (u_hi + 2 * 128 * 80 * 16),
-            "intra_backward_q": ctas * (2 * 2 * 128 * 128 * 80 + 8 * (u_hi + u_lo + 2 * 128 * 64 * nr)),
-            "intra_backward_kv": ctas * (2 * 2 * 128 * 128 * 80 + 8 * (u_hi + u_lo + 2 * 128 * 64 * nr + 2 * 128 * 80 * 16)),
+            "intra_forward": seen * 2 * 128 * (terms * 128 + 80),
+            "intra_backward_q": seen * 2 * 128 * (2 * 80 + terms * (128 + 2 * 64)),
+            "intra_backward_kv": rows * 2 * 128 * (2 * 80 + terms * (128 + 64) + 80),
         }
         kernels = {name: dict(launches=cnt, ms_per_launch=ms / max(cnt, 1), share=None)
                    for name, (cnt, ms) in report.items()}

@@ -70,7 +70,7 @@ def sweep(ns, gs, steps: int, warmup: int) -> None:
             captured.check_status()
             print(json.dumps(dict(benchmark="sweep", n=n, groups=g, ms_per_step=ms, ns_per_token=ms * 1e6 / n,
                                   tokens_per_s=n / (ms * 1e-3), cuda_graph_ms_per_step=graph_ms,
-                                  intra_chunk="tcgen05" if g <= 8 else "token-pair kernels")), flush=True)
+                                  intra_chunk="tcgen05")), flush=True)
             del q, k, v, dout, prepared, captured
             torch.cuda.empty_cache()
 
