@@ -6,7 +6,7 @@
 //   U_r = term . K^T     one MMA chain per half of the keys (64 columns each, so that one half is read
 //                        while the other is computed),
 //   w += sgn_r u_r^2     in registers, 64 keys per thread.
-// Then the causal mask, the bf16 weight tile W into tensor memory, Y = W [v | 1] (one MMA chain), and the epilogue
+// Then the causal mask, the weight tile W into tensor memory (bf16 value + remainder), Y = W [v | 1] (one MMA chain), and the epilogue
 // adds the cross-chunk part left in num / den by cross_read, normalises and writes out / num / den and the status
 // flags.  Eight compute warps (quadrant x 2), one warp issues the MMAs; two CTAs share an SM.  Replaces, per chunk,
 // the reference's F-wide local score GEMM, tril, bf16 cast, score x U GEMM, merge and normalise stages
@@ -130,8 +130,10 @@ __global__ void __launch_bounds__(FW_THREADS, 2) intra_fwd_kernel(const IntraFwd
         w.wait(&w_full, 0, 0x14);
         fence_after_sync();
         const uint64_t du = smem_desc(u_addr, 128, CP);
-        for (int ks = 0; ks < cols / 16; ++ks)
-          mma_bf16_ts(tmem + FW_U, tmem + FW_TERM + 8 * ks, desc_advance(du, ks * 256), instr_desc_bf16(128, EP, 0, 1), ks > 0);
+        for (int part = 0; part < 2; ++part)                    // the weights' bf16 values, then their remainders
+          for (int ks = 0; ks < cols / 16; ++ks)
+            mma_bf16_ts(tmem + FW_U, tmem + FW_TERM + part * TERM_COLS + 8 * ks, desc_advance(du, ks * 256),
+                        instr_desc_bf16(128, EP, 0, 1), part + ks > 0);
         mma_commit(&y_full);
       }
       __syncwarp();
@@ -200,7 +202,11 @@ __global__ void __launch_bounds__(FW_THREADS, 2) intra_fwd_kernel(const IntraFwd
         if (on(hf, 1)) add(u, acc[hf][1]);
       }
     }
-    // weight tile over the term slots (every MMA that read them is complete): masked, bf16, 16 keys = 8 columns
+    // weight tile over the term slots (every MMA that read them is complete): masked, 16 keys = 8 columns, bf16 values
+    // over the first slot and their rounding remainders over the second.  Without the remainders a numerator is off by
+    // 2^-9 of its largest weight, which the first rows of a sequence, where few weights are summed and gradients are
+    // large, turn into errors of a third of dq's rms (B = 4, N = 4096, 8 groups, gains of 20; with them
+    // under a tenth).
     const int my_key = 32 * my_rb + lane;
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf)
@@ -208,14 +214,18 @@ __global__ void __launch_bounds__(FW_THREADS, 2) intra_fwd_kernel(const IntraFwd
       for (int x = 0; x < 2; ++x)
         if (32 * x < (hf ? nb2 : na)) {
           const int key = key_of(hf, x);
-          uint32_t o[8];
+          uint32_t o[8], rest[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            float lo, hi;
-            f2_unpack(acc[hf][x][j], lo, hi);
-            o[j] = pack_bf16(key + 2 * j <= my_key ? lo : 0.f, key + 2 * j + 1 <= my_key ? hi : 0.f);
+            float w_a, w_b;
+            f2_unpack(acc[hf][x][j], w_a, w_b);
+            if (key + 2 * j > my_key) w_a = 0.f;
+            if (key + 2 * j + 1 > my_key) w_b = 0.f;
+            o[j] = pack_bf16(w_a, w_b);
+            rest[j] = pack_bf16(w_a - bf16_lo(o[j]), w_b - bf16_hi(o[j]));
           }
           tmem_st8(tmem + FW_TERM + lane_off + key / 2, o);
+          tmem_st8(tmem + FW_TERM + TERM_COLS + lane_off + key / 2, rest);
         }
     tmem_st_wait();
     fence_before_sync();

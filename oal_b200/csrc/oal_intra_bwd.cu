@@ -16,7 +16,8 @@
 //
 // Key / value side (rows are keys, columns are the queries of one head): per head and term
 //   P_r^T as above (bf16 value),  Z_r = P_r^T Q,  dk += sgn_r l_r * Z_r,  w += sgn_r u_r^2 in registers,
-// and after the last term dU += W^T G.  A CTA walks several query heads of its KV head; dk stays in registers, dU
+// and after the last term dU += W^T G (W as value + remainder, as in the forward: a row's weights and its denominator
+// then agree to 16 bits).  A CTA walks several query heads of its KV head; dk stays in registers, dU
 // in tensor memory, and the next head's operands arrive while the current one is worked on.
 //
 // The cross-chunk parts computed by the state kernels arrive as fp32 buffers and are added before the final cast.
@@ -532,8 +533,10 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
           issue_z(T - 1, 1);
           w.wait(&w_full, i & 1, 0x3B);
           fence_after_sync();
-          for (int ks = 0; ks < cols / 16; ++ks)      // dU (+)= W^T G
-            mma_bf16_ts(tmem + BK_V, tmem + BK_P + 8 * ks, desc_advance(dg, ks * 256), instr_desc_bf16(128, EP, 0, 1), i + ks > 0);
+          for (int part = 0; part < 2; ++part)        // dU (+)= W^T G: the weights' bf16 values, then their remainders
+            for (int ks = 0; ks < cols / 16; ++ks)
+              mma_bf16_ts(tmem + BK_V, tmem + (part ? BK_TERM : BK_P) + 8 * ks, desc_advance(dg, ks * 256),
+                          instr_desc_bf16(128, EP, 0, 1), i + part + ks > 0);
           mma_commit(&v_full);
         }
       }
@@ -655,21 +658,30 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
       w.wait(&z_half[1], (T + rank - 1) & 1, 0x45);
       fence_after_sync();
       drain(rank - 1);
-      // W^T in the place of P^T, whose last reader is complete
+      // W^T in the place of P^T, whose last reader is complete, and its remainders over the first term slot (so are
+      // the slot's readers, and the next head builds no term before v_full)
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
         for (int x = 0; x < 2; ++x)
-          if (on(hf, x)) {
-            uint32_t o[4];
+          if (exists(hf, x)) {
+            const uint32_t at = lane_off + col_of(hf, x) / 2;
+            uint32_t rest[4] = {0u, 0u, 0u, 0u};
+            if (on(hf, x)) {
+              uint32_t o[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float w_lo, w_hi;
-              f2_unpack(wt[hf][x][j], w_lo, w_hi);
-              const int i0 = col_of(hf, x) + 2 * j;
-              o[j] = pack_bf16(i0 >= row ? w_lo : 0.f, i0 + 1 >= row ? w_hi : 0.f);
+              for (int j = 0; j < 4; ++j) {
+                float w_a, w_b;
+                f2_unpack(wt[hf][x][j], w_a, w_b);
+                const int i0 = col_of(hf, x) + 2 * j;
+                if (i0 < row) w_a = 0.f;
+                if (i0 + 1 < row) w_b = 0.f;
+                o[j] = pack_bf16(w_a, w_b);
+                rest[j] = pack_bf16(w_a - bf16_lo(o[j]), w_b - bf16_hi(o[j]));
+              }
+              tmem_st4(tmem + BK_P + at, o[0], o[1], o[2], o[3]);
             }
-            tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, o[0], o[1], o[2], o[3]);
+            tmem_st4(tmem + BK_TERM + at, rest[0], rest[1], rest[2], rest[3]);
           }
       tmem_st_wait();
       fence_before_sync();

@@ -49,3 +49,24 @@ def test_token_major_output_stays_limited_to_eight_groups():
         else:
             with pytest.raises(ValueError, match="at most 8 groups"):
                 _lib.workspace_bytes(p, 1)
+
+
+# the first chunk of a sequence (nothing from the state kernels): full, partial and one-block tiles, rep 7 / 1 / 3
+@pytest.mark.parametrize("n,hq,hkv,g", [(128, 14, 2, 8), (33, 2, 2, 1), (100, 3, 1, 16)])
+def test_numerators_of_the_first_chunk_value_by_value(n, hq, hkv, g):
+    case = _case(1, n, hq, hkv, g)
+    num = run_operator(case, precision="bf16_tensorcore", io_dtype=torch.bfloat16, need=())["num"].double()
+    q, k, v = (t[0].double() for t in (case.q, case.k, case.v))
+    k, v = (t.repeat_interleave(hq // hkv, 0) for t in (k, v))
+    rows, cols = torch.tril_indices(g + 1, g + 1)
+    lower = torch.zeros(hq, g + 1, g + 1, dtype=torch.double)
+    lower[:, rows, cols] = case.factor.double()
+    per_dim = case.scale * lower[:, 1:].gather(1, case.dim_groups.long()[..., None].expand(-1, -1, g + 1))    # [hq, 64, r]
+    u = lower[:, 0, None, None] + torch.einsum("hid,hdr,hjd->hijr", q, per_dim, k)
+    w = ((u ** 2).sum(-1) + case.kernel_eps).tril()
+    # Weights enter as bf16 value + remainder (2^-17 of w) and u_r = c_r + sum_d l_r[d] q_d k_d from products with one
+    # factor rounded the same way: |du_r| <= 2^-17 a_r, a_r the sum of magnitudes, so dw <= 2^-16 |u| |a|; both norms over r
+    # are those of any rotation of the terms, |a| <= |L_0| + sum_d |l[d]| |q_d k_d|.  Doubled for the fp32 roundings.
+    a = lower[:, 0].norm(dim=-1)[:, None, None] + torch.einsum("hid,hd,hjd->hij", q.abs(), per_dim.norm(dim=-1), k.abs())
+    bound = (2.0 ** -16 * w + 2.0 ** -15 * w.sqrt() * a).tril() @ v.abs()
+    assert ((num[0] - w @ v).abs() <= bound).all()
