@@ -159,8 +159,11 @@ __global__ void __launch_bounds__(32) head_factor_kernel(const int32_t* dim_perm
     int k = 0;
     for (int r = 0; r < n; ++r) if (sig[r] >= 0.f) order[k++] = r;
     const int rpos = k;
-    for (int r = 0; r < n; ++r) if (sig[r] < 0.f) order[k++] = r;
-    for (int r = 0; r < n; ++r) lam[r] = sqrtf(fmaxf(fabsf(sig[order[r]]), floor_v));
+    for (int r = 0; r < n; ++r) if (!(sig[r] >= 0.f)) order[k++] = r;      // negative or not a number: all n entries are indices
+    for (int r = 0; r < n; ++r) {
+      const float size = fabsf(sig[order[r]]);
+      lam[r] = sqrtf(size < floor_v ? floor_v : size);                     // a NaN stays one and reaches the status word
+    }
     table[h].s.rank = n;
     table[h].s.rpos = rpos;
     table[h].s.w0 = 0.f;

@@ -1,0 +1,35 @@
+"""What a call reports: non-finite coefficients and factors end in the documented error, at every place where they
+could get lost (one chunk, a chunk edge, several chunks), and leave the context usable."""
+
+import pytest
+import torch
+
+import oal_b200
+
+pytestmark = pytest.mark.gpu
+
+BAD = [float("nan"), float("inf"), -float("inf")]
+ERROR = "denominator must be finite and strictly positive"
+
+
+def _inputs(n, g, hq=4, hkv=2):
+    gen = torch.Generator().manual_seed(n + g)
+    q, k, v = (torch.randn(1, h, n, 64, generator=gen).bfloat16().cuda() for h in (hq, hkv, hkv))
+    groups = (torch.arange(64) % g).to(torch.int32).cuda()
+    return q, k, v, groups
+
+
+# the per-head factorisation of explicit coefficients orders its terms by sign: a NaN has none
+@pytest.mark.parametrize("n", [64, 128, 129, 300])
+@pytest.mark.parametrize("g", [1, 8, 16])
+@pytest.mark.parametrize("value", BAD)
+def test_non_finite_explicit_coefficients_raise(n, g, value):
+    q, k, v, groups = _inputs(n, g)
+    for which in range(3):
+        coefs = [torch.ones(4), torch.ones(4, g), torch.eye(g).expand(4, g, g).clone()]
+        coefs[which].view(4, -1)[1, -1] = value
+        with pytest.raises(RuntimeError, match=ERROR):
+            oal_b200.grouped_coefficient_attention(q, k, v, groups, *(c.cuda() for c in coefs), precision="bf16_tensorcore")
+    coefs = [torch.ones(4), torch.ones(4, g), torch.eye(g).expand(4, g, g).clone()]
+    out, _, _ = oal_b200.grouped_coefficient_attention(q, k, v, groups, *(c.cuda() for c in coefs), precision="bf16_tensorcore")
+    assert torch.isfinite(out).all()
