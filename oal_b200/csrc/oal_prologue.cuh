@@ -97,8 +97,9 @@ __device__ __forceinline__ void one_sided_jacobi(PrologueSmem& s, int n, int lan
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
   if (lane < n) {
     // a vanishing term keeps its direction at a negligible weight, so that the coefficient gradient of a
-    // singular factor can be rotated back
-    s.lam[lane] = sqrtf(fmaxf(norm, fmaxf(1e-12f * top, 1e-30f)));
+    // singular factor can be rotated back; a NaN (which fmaxf would drop) stays one and reaches weights and status
+    const float least = fmaxf(1e-12f * top, 1e-30f);
+    s.lam[lane] = sqrtf(norm < least ? least : norm);
 #pragma unroll
     for (int i = 0; i < NM; ++i)
       if (i < n) s.V[i][lane] = v[i];

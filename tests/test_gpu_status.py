@@ -33,3 +33,37 @@ def test_non_finite_explicit_coefficients_raise(n, g, value):
     coefs = [torch.ones(4), torch.ones(4, g), torch.eye(g).expand(4, g, g).clone()]
     out, _, _ = oal_b200.grouped_coefficient_attention(q, k, v, groups, *(c.cuda() for c in coefs), precision="bf16_tensorcore")
     assert torch.isfinite(out).all()
+
+
+# a factor that is not finite: the one-call form, a prepared inference and training call, a recorded step
+@pytest.mark.parametrize("n", [1, 64, 128, 129, 300])
+@pytest.mark.parametrize("g", [1, 8, 16])
+@pytest.mark.parametrize("value", BAD)
+def test_non_finite_factors_raise(n, g, value):
+    from oal_b200 import hd_block_gemm_autograd as hd
+    from oal_b200.captured_step import CapturedStep
+
+    q, k, v, groups = _inputs(n, g)
+    good = torch.full((4, (g + 1) * (g + 2) // 2), 0.5, device="cuda")
+    for entry in (0, 1, good.shape[1] - 1):
+        factor = good.clone()
+        factor[1, entry] = value
+        with pytest.raises(RuntimeError, match=ERROR):
+            oal_b200.oal_attention(q, k, v, groups, factor)
+        prepared = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, good, precision="bf16_tensorcore")
+        with pytest.raises(RuntimeError, match=ERROR):
+            oal_b200.run_prepared_grouped_hd_block_gemm(prepared, q, k, v, factor)
+        leaves = [t.clone().requires_grad_() for t in (q, k, v, factor)]
+        prepared = oal_b200.prepare_grouped_hd_block_gemm(*leaves[:3], groups, leaves[3], precision="bf16_tensorcore")
+        with pytest.raises(RuntimeError, match=ERROR):
+            oal_b200.run_prepared_grouped_hd_block_gemm(prepared, *leaves)[0].sum().backward()
+            hd.check_pending_status(block=True)
+    leaves = [t.clone().requires_grad_() for t in (q, k, v, good)]
+    prepared = oal_b200.prepare_grouped_hd_block_gemm(*leaves[:3], groups, leaves[3], precision="bf16_tensorcore")
+    step = CapturedStep(prepared, *leaves, torch.ones_like(leaves[0]))
+    step.replay(*(t.detach() for t in leaves), torch.ones_like(q))
+    step.check_status()
+    step.replay(q, k, v, factor, torch.ones_like(q))
+    with pytest.raises(RuntimeError, match=ERROR):
+        step.check_status()
+    hd.forget_captured_status()
