@@ -76,8 +76,10 @@ def _grad_bits(mask) -> int:
 
 
 def _pad_last(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as the kernels read it: 64 columns, row-major (a live tensor may have other strides than the one its
+    call was prepared with)."""
     d = t.shape[-1]
-    return t if d == _lib.HEAD_DIM else F.pad(t, (0, _lib.HEAD_DIM - d)).contiguous()
+    return (t if d == _lib.HEAD_DIM else F.pad(t, (0, _lib.HEAD_DIM - d))).contiguous()
 
 
 def _raise_for_bits(bits: int, where: str = "") -> None:
