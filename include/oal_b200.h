@@ -13,6 +13,9 @@
  * and the library never allocates or frees device memory: the caller owns the
  * inputs, the outputs and one workspace blob whose size is returned by
  * oal_workspace_bytes().  All launches go to the stream that is passed in.
+ * Tensors of bf16_tensorcore calls and of the rotary moves, and every workspace,
+ * start on a 16-byte boundary; others are refused with OAL_ERR_ARGUMENT.
+ * (coefficients, packed factors, den, grad_den and status words need 4 bytes.)
  *
  * Return value of every int function: 0 on success, a negative OAL_ERR_* code
  * on a contract violation (oal_last_error_string() describes it).  Numerical

@@ -64,11 +64,11 @@ class _RopePackFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q_flat, k_flat, v_flat, cos, sin, q_heads: int, kv_heads: int):
         from . import _lib
-        from .hd_block_gemm_autograd import _stream_ptr
+        from .hd_block_gemm_autograd import _stream_ptr, on_boundary
 
         b, n, _ = q_flat.shape
-        q_flat, k_flat, v_flat = q_flat.contiguous(), k_flat.contiguous(), v_flat.contiguous()
-        cos, sin = cos.float().contiguous(), sin.float().contiguous()
+        q_flat, k_flat, v_flat = (on_boundary(t.contiguous()) for t in (q_flat, k_flat, v_flat))
+        cos, sin = (on_boundary(t.float().contiguous()) for t in (cos, sin))
         q = torch.empty(b, q_heads, n, 64, dtype=q_flat.dtype, device=q_flat.device)
         k = torch.empty(b, kv_heads, n, 64, dtype=q_flat.dtype, device=q_flat.device)
         v = torch.empty(b, kv_heads, n, 64, dtype=q_flat.dtype, device=q_flat.device)
@@ -84,12 +84,12 @@ class _RopePackFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dq, dk, dv):
         from . import _lib
-        from .hd_block_gemm_autograd import _stream_ptr
+        from .hd_block_gemm_autograd import _stream_ptr, on_boundary
 
-        cos, sin = ctx.saved_tensors
+        cos, sin = (on_boundary(t) for t in ctx.saved_tensors)
         b, n, hq, hkv = ctx.geometry
         mk = lambda g, h: None if g is None else torch.empty(b, n, h * 64, dtype=g.dtype, device=g.device)
-        dq, dk, dv = (None if g is None else g.contiguous() for g in (dq, dk, dv))
+        dq, dk, dv = (None if g is None else on_boundary(g.contiguous()) for g in (dq, dk, dv))
         dq_flat, dk_flat, dv_flat = mk(dq, hq), mk(dk, hkv), mk(dv, hkv)
         dev = next(g for g in (dq, dk, dv) if g is not None).device
         with torch.cuda.device(dev):

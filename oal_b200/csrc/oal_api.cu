@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <chrono>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -214,6 +215,15 @@ int check_problem(const OalProblem* p) {
     return fail(OAL_ERR_ARGUMENT, "token-major out needs bf16_tensorcore and at most 8 groups per head");
   return OAL_OK;
 }
+
+// The tensor-core kernels and the row moves read and write these tensors in 16-byte pieces.  (The exact fp32 kernels
+// look at the alignment themselves and fall back to single elements; they ask it of the workspace only.)
+bool misaligned(std::initializer_list<const void*> tensors) {
+  uintptr_t bits = 0;
+  for (const void* t : tensors) bits |= reinterpret_cast<uintptr_t>(t);
+  return bits & 15;
+}
+constexpr const char* kMisaligned = "%s: tensors must start on a 16-byte boundary";
 
 // Where a call's coefficients come from: the packed factor (expanded on the device into A, B, C), or A, B, C.
 struct CoefSource {
@@ -519,6 +529,7 @@ int backward_core_fp32(const OalProblem* p, const BackwardArgs& x, const CoefSou
   if (x.dstate_in) return fail(OAL_ERR_ARGUMENT, "fp32_ieee mode keeps no chunk state: dstate_in must be NULL");
   BackwardSpace s = carve_backward(p, x.workspace);
   if (!x.workspace || x.workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_backward: workspace too small");
+  if (misaligned({x.workspace})) return fail(OAL_ERR_ARGUMENT, kMisaligned, "oal_backward");
   const int mask = p->grad_mask;
   if (sink.dfactor) {
     sink.dA = s.dcoefs; sink.dB = sink.dA + p->q_heads; sink.dC = sink.dB + (size_t)p->q_heads * p->groups;
@@ -561,6 +572,8 @@ int backward_core_fp32(const OalProblem* p, const BackwardArgs& x, const CoefSou
 int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& src, CoefSink sink, cudaStream_t st) {
   if (p->precision == OAL_PRECISION_FP32_IEEE) return backward_core_fp32(p, x, src, sink, st);
   if (!x.saved_state) return fail(OAL_ERR_ARGUMENT, "oal_backward: saved_state is NULL");
+  if (misaligned({x.q, x.k, x.v, x.num, x.saved_state, x.grad_out, x.grad_num, x.dq, x.dk, x.dv, x.dstate_in, x.workspace}))
+    return fail(OAL_ERR_ARGUMENT, kMisaligned, "oal_backward");
   BackwardSpaceTC s = carve_backward_tc(p, x.workspace);
   if (!x.workspace || x.workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_backward: workspace too small");
   if (sink.dfactor) {
@@ -648,6 +661,7 @@ int oal_rope_pack(const void* q_flat, const void* k_flat, const void* v_flat, co
                   void* q, void* k, void* v, int batch, int seq_len, int q_heads, int kv_heads, void* stream) {
   if (batch < 0 || seq_len < 0 || q_heads < 1 || kv_heads < 1) return fail(OAL_ERR_ARGUMENT, "oal_rope_pack: bad geometry");
   if ((q_flat || k_flat) && (!cosv || !sinv)) return fail(OAL_ERR_ARGUMENT, "oal_rope_pack: cos / sin are required");
+  if (misaligned({q_flat, k_flat, v_flat, cosv, sinv, q, k, v})) return fail(OAL_ERR_ARGUMENT, kMisaligned, "oal_rope_pack");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
   LaunchScope scope("rope_pack", st, (q_flat ? 1 : 0) + (k_flat ? 1 : 0) + (v_flat ? 1 : 0));
@@ -666,6 +680,7 @@ int oal_rope_unpack_grad(const void* dq, const void* dk, const void* dv, const f
   if (batch < 0 || seq_len < 0 || q_heads < 1 || kv_heads < 1)
     return fail(OAL_ERR_ARGUMENT, "oal_rope_unpack_grad: bad geometry");
   if ((dq || dk) && (!cosv || !sinv)) return fail(OAL_ERR_ARGUMENT, "oal_rope_unpack_grad: cos / sin are required");
+  if (misaligned({dq, dk, dv, cosv, sinv, dq_flat, dk_flat, dv_flat})) return fail(OAL_ERR_ARGUMENT, kMisaligned, "oal_rope_unpack_grad");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
   LaunchScope scope("rope_unpack_grad", st, (dq ? 1 : 0) + (dk ? 1 : 0) + (dv ? 1 : 0));
@@ -746,6 +761,7 @@ static int forward_entry(const OalProblem* p, const void* q, const void* k, cons
   if (p->precision == OAL_PRECISION_FP32_IEEE) {
     if (state_in) return fail(OAL_ERR_ARGUMENT, "fp32_ieee mode keeps no chunk state: state_in must be NULL");
   } else {
+    if (misaligned({q, k, v, out, num, saved_state, state_in, workspace})) return fail(OAL_ERR_ARGUMENT, kMisaligned, "oal_forward");
     ForwardSpaceTC s = carve_forward_tc(p, workspace);
     if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_forward: workspace too small");
     if (!saved_state) return fail(OAL_ERR_ARGUMENT, "oal_forward: saved_state is NULL");
@@ -946,6 +962,7 @@ int oal_forward_local_state(const OalProblem* p, const void* k, const void* v, f
   if (p->precision != OAL_PRECISION_BF16_TENSORCORE)
     return fail(OAL_ERR_DTYPE, "oal_forward_local_state: chunk states exist only in bf16_tensorcore mode");
   if (!k || !v || !state_total || !status) return fail(OAL_ERR_ARGUMENT, "oal_forward_local_state: NULL tensor pointer");
+  if (misaligned({k, v, state_total, workspace})) return fail(OAL_ERR_ARGUMENT, kMisaligned, "oal_forward_local_state");
   ForwardSpaceTC s = carve_forward_tc(p, workspace);
   if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_forward_local_state: workspace too small");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -969,6 +986,8 @@ int oal_backward_local_state(const OalProblem* p, const void* q, const int32_t* 
     return fail(OAL_ERR_DTYPE, "oal_backward_local_state: chunk states exist only in bf16_tensorcore mode");
   if (!q || !dim_perm || !group_start || !coef_a || !coef_b || !coef_c || !num || !den || !saved_state || !dstate_total || !status)
     return fail(OAL_ERR_ARGUMENT, "oal_backward_local_state: NULL tensor pointer");
+  if (misaligned({q, num, saved_state, grad_out, grad_num, dstate_total, workspace}))
+    return fail(OAL_ERR_ARGUMENT, kMisaligned, "oal_backward_local_state");
   BackwardSpaceTC s = carve_backward_tc(p, workspace);
   if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_backward_local_state: workspace too small");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1034,6 +1053,7 @@ int oal_forward_static_scratch(const OalProblem* p, const void* q, const void* k
     return fail(OAL_ERR_DTYPE, "oal_forward_static_scratch: only bf16_tensorcore uses scratch memory (fp32_ieee forward needs none: call oal_forward)");
   if (!q || !k || !v || !dim_perm || !group_start || !coef_a || !coef_b || !coef_c || !out || !num || !den || !status || !saved_state)
     return fail(OAL_ERR_ARGUMENT, "oal_forward_static_scratch: NULL tensor pointer");
+  if (misaligned({q, k, v, out, num, saved_state})) return fail(OAL_ERR_ARGUMENT, kMisaligned, "oal_forward_static_scratch");
   const int units = p->batch * p->kv_heads, nb = chunk_count(p);
   if ((long long)units * nb > kStaticMaxUnitChunks)
     return fail(OAL_ERR_WORKSPACE, "oal_forward_static_scratch: batch x kv_heads x ceil(seq_len/128) exceeds the static scratch limit of 16; use oal_forward with a caller workspace");

@@ -143,9 +143,15 @@ struct Prepared {
   }
 };
 
-Tensor pad_last(const Tensor& t) {
+// A contiguous tensor may start anywhere in its storage; the tensor-core kernels read 16 bytes at a time.  (The exact
+// fp32 kernels look at the alignment themselves.)
+Tensor on_boundary(const Prepared& p, const Tensor& t) {
+  const bool off = p.problem.precision == OAL_PRECISION_BF16_TENSORCORE && t.defined() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15);
+  return off ? t.clone() : t;
+}
+Tensor pad_last(const Prepared& p, const Tensor& t) {
   const int64_t d = t.size(-1);
-  return d == OAL_HEAD_DIM ? t : at::constant_pad_nd(t, {0, OAL_HEAD_DIM - d}).contiguous();
+  return d == OAL_HEAD_DIM ? on_boundary(p, t) : at::constant_pad_nd(t, {0, OAL_HEAD_DIM - d}).contiguous();
 }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
@@ -163,9 +169,9 @@ Forward forward_call(const Prepared& p, const Tensor& q, const Tensor& k, const 
   const bool recording = capturing();
   if (!recording) drain(dev, false);
   Forward r;
-  r.q = pad_last(q);
-  r.k = pad_last(k);
-  r.v = pad_last(v);
+  r.q = pad_last(p, q);
+  r.k = pad_last(p, k);
+  r.v = pad_last(p, v);
   r.factor = f.contiguous();
   const auto opt = q.options().requires_grad(false);
   r.out = at::empty(p.token_major ? at::IntArrayRef({p.B, p.N, p.Hq, OAL_HEAD_DIM}) : at::IntArrayRef({p.B, p.Hq, p.N, OAL_HEAD_DIM}),
@@ -203,11 +209,11 @@ Forward forward_call(const Prepared& p, const Tensor& q, const Tensor& k, const 
 }
 
 // gradients of the outputs as the kernels read them
-Tensor upstream(const Tensor& g, at::ScalarType dtype, bool pad) {
+Tensor upstream(const Prepared& p, const Tensor& g, at::ScalarType dtype, bool pad) {
   if (!g.defined()) return g;
   Tensor t = g.to(dtype);
   if (pad && t.size(-1) != OAL_HEAD_DIM) t = at::constant_pad_nd(t, {0, OAL_HEAD_DIM - t.size(-1)});
-  return t.contiguous();
+  return on_boundary(p, t.contiguous());
 }
 
 struct PackedNode : torch::autograd::Function<PackedNode> {
@@ -236,12 +242,15 @@ struct PackedNode : torch::autograd::Function<PackedNode> {
     auto holder = ctx->saved_data["prepared"].toCapsule();
     const Prepared& p = *static_cast<Holder*>(holder.get())->p;
     const variable_list s = ctx->get_saved_variables();
-    const Tensor &q = s[0], &k = s[1], &v = s[2], &factor = s[3], &num = s[4], &den = s[5], &saved = s[6], &meta = s[7];
+    // saved-tensor hooks may hand back copies that start elsewhere
+    const Tensor q = on_boundary(p, s[0]), k = on_boundary(p, s[1]), v = on_boundary(p, s[2]), num = on_boundary(p, s[4]),
+                 saved = on_boundary(p, s[6]);
+    const Tensor &factor = s[3], &den = s[5], &meta = s[7];
     const int dev = p.device.index();
     c10::cuda::CUDAGuard guard(p.device);
     const bool recording = capturing();
     if (!recording) drain(dev, false);
-    const Tensor go = upstream(grads[0], p.kernel_out, true), gn = upstream(grads[1], at::kFloat, true), gd = upstream(grads[2], at::kFloat, false);
+    const Tensor go = upstream(p, grads[0], p.kernel_out, true), gn = upstream(p, grads[1], at::kFloat, true), gd = upstream(p, grads[2], at::kFloat, false);
     Tensor d[4];
     if (p.grad[0]) d[0] = at::empty_like(q);
     if (p.grad[1]) d[1] = at::empty_like(k);

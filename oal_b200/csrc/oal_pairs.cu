@@ -352,10 +352,11 @@ __global__ void __launch_bounds__(THREADS, 2) fwd_pairs_kernel(const PairArgs a)
     float nv[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) nv[c] = sum_ranks(WT + r * TP + c4 + c, a.split);
-    *reinterpret_cast<float4*>(a.num + row * VD + c4) = make_float4(nv[0], nv[1], nv[2], nv[3]);
+    if (a.vec & 8) *reinterpret_cast<float4*>(a.num + row * VD + c4) = make_float4(nv[0], nv[1], nv[2], nv[3]);
     const float dn = fmaxf(dsum, a.floor);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
+      if (!(a.vec & 8)) a.num[row * VD + c4 + c] = nv[c];
       if (!finite_f(nv[c])) flags |= OAL_STATUS_NONFINITE;
       store_elem(a.out, row * VD + c4 + c, a.out_dt, nv[c] / dn);
     }
@@ -789,6 +790,7 @@ cudaError_t dispatch_pairs(const PairArgs& args, int which, cudaStream_t st) {
   const void* in[3] = {a.q, a.k, a.v};
   a.vec = 0;
   for (int x = 0; x < 3; ++x) a.vec |= reinterpret_cast<uintptr_t>(in[x]) % quad == 0 ? 1 << x : 0;
+  a.vec |= reinterpret_cast<uintptr_t>(a.num) % 16 == 0 ? 8 : 0;
   a.tiles = pairs_tiles(a.N);
   a.split = pairs_split(a.B, a.Hq, a.N);
   if (a.G <= 4) return launch_pairs<4>(a, which, st);

@@ -75,11 +75,17 @@ def _grad_bits(mask) -> int:
     return bits
 
 
+def on_boundary(t):
+    """``t``, or its copy when it does not start on the 16-byte boundary that the tensor-core kernels need."""
+    return t if t is None or t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _pad_last(t: torch.Tensor) -> torch.Tensor:
     """``t`` as the kernels read it: 64 columns, row-major (a live tensor may have other strides than the one its
-    call was prepared with)."""
+    call was prepared with), bf16 on a 16-byte boundary (the fp32 kernels look at the alignment themselves)."""
     d = t.shape[-1]
-    return (t if d == _lib.HEAD_DIM else F.pad(t, (0, _lib.HEAD_DIM - d))).contiguous()
+    t = (t if d == _lib.HEAD_DIM else F.pad(t, (0, _lib.HEAD_DIM - d))).contiguous()
+    return on_boundary(t) if t.dtype == torch.bfloat16 else t
 
 
 def _raise_for_bits(bits: int, where: str = "") -> None:
@@ -303,7 +309,7 @@ def backward_operands(plan: HDParallelBlockPlan, num, den, grad_out, grad_num, g
         gt = gt.to(dtype)
         if gt.shape[-1] != width and width == _lib.HEAD_DIM:
             gt = F.pad(gt, (0, width - gt.shape[-1]))
-        return gt.contiguous()
+        return on_boundary(gt.contiguous())
 
     return (kernel_out, prep(num, torch.float32, _lib.HEAD_DIM), den.contiguous(),
             prep(grad_out, kernel_out, _lib.HEAD_DIM), prep(grad_num, torch.float32, _lib.HEAD_DIM),
@@ -319,7 +325,9 @@ def backward_impl(saved_inputs, num, den, saved_state, tables: GroupTables, scal
     ``workspace`` / ``reuse_state_stage``: sequence parallelism passes the workspace that
     ``oal_backward_local_state`` has just filled so that stage is not computed twice."""
     lib = _lib.load()
-    qp, kp, vp, a32, b32, c32 = saved_inputs
+    qp, kp, vp = (on_boundary(t) for t in saved_inputs[:3])      # saved-tensor hooks may hand back copies that start elsewhere
+    a32, b32, c32 = saved_inputs[3:]
+    saved_state = on_boundary(saved_state)
     B, Hq, Hkv, N, D, Dv = plan.geometry
     dev = qp.device
     if forward_status is not None and not torch.cuda.is_current_stream_capturing():

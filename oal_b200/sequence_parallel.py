@@ -34,6 +34,7 @@ from .hd_block_gemm_autograd import (
     backward_operands,
     defer_status,
     forward_impl,
+    on_boundary,
 )
 
 
@@ -84,7 +85,7 @@ def local_dstate_total(saved_inputs, num, den, saved_state, tables, scale, floor
                        grad_num, grad_den, workspace):
     """Stage A of the backward into ``workspace``; returns this rank's state-gradient sum."""
     lib = _lib.load()
-    qp, kp, vp, a32, b32, c32 = saved_inputs
+    qp, (a32, b32, c32), saved_state = on_boundary(saved_inputs[0]), saved_inputs[3:], on_boundary(saved_state)
     B, Hq, Hkv, N, D, Dv = plan.geometry
     # the same padded operands and kernel-side output dtype as the backward proper: the stage it leaves in
     # the workspace is reused there
