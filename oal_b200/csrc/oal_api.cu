@@ -300,6 +300,7 @@ ChunkRange chunk_range(const OalProblem* p, const void* state_in, const void* ds
 
 struct ForwardSpaceTC {
   float* ds;
+  int32_t* update_status;
   size_t bytes;
 };
 
@@ -316,6 +317,7 @@ ForwardSpaceTC carve_forward_tc(const OalProblem* p, void* ws) {
   ForwardSpaceTC s;
   const size_t units = (size_t)p->batch * p->kv_heads;
   s.ds = c.take<float>(units * chunk_count(p) * oal::state_rows() * oal::EP);
+  s.update_status = c.take<int32_t>(oal::state_update_blocks((int)units, chunk_count(p)));
   s.bytes = c.off;
   return s;
 }
@@ -417,7 +419,8 @@ oal::PairArgs base_args(const OalProblem* p, const void* q, const void* k, const
 // ---- forward ------------------------------------------------------------------------------------
 int forward_core(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
                  const int32_t* group_start, const CoefSource& src, void* out, float* num, float* den, void* saved_state,
-                 const float* state_in, float* ds, int32_t* status, oal::StatusSink sink, bool timing, cudaStream_t st) {
+                 const float* state_in, float* ds, int32_t* update_status, int32_t* status, oal::StatusSink sink, bool timing,
+                 cudaStream_t st) {
   cudaError_t e;
   const bool tc = p->precision == OAL_PRECISION_BF16_TENSORCORE;
   const int units = p->batch * p->kv_heads, nb = chunk_count(p);
@@ -462,12 +465,14 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
   }
   if (update) {
     LaunchScope scope("state_update", st, 1, timing);
-    e = oal::state_update(k, v, ds, units, p->seq_len, nb, cr.n, src.factor ? &pro : nullptr, p->q_heads, status, st);
+    e = oal::state_update(k, v, ds, units, p->seq_len, nb, cr.n, src.factor ? &pro : nullptr, p->q_heads, status,
+                          src.factor ? update_status : nullptr, st);
     if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
   }
   if (tc && cr.n > 0) {
     { LaunchScope scope("state_scan", st, 1, timing);
-      e = oal::state_scan(ds, saved_state, saved_remainders(p, saved_state), state_in, nullptr, units, nb, 0, cr.trim, st); }
+      e = oal::state_scan(ds, saved_state, saved_remainders(p, saved_state), state_in, nullptr, units, nb, 0, cr.trim,
+                          update && src.factor ? update_status : nullptr, oal::state_update_blocks(units, cr.n), status, st); }
     if (e != cudaSuccess) return fail_cuda(e, "state scan kernel");
     { LaunchScope scope("cross_read_q", st, 1, timing);
       e = oal::cross_read(true, q, saved_state, coef_table, num, den, p->batch, p->q_heads, p->q_heads / p->kv_heads,
@@ -608,7 +613,7 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   }
   if (want_kv && cross) {
     { LaunchScope scope("state_scan_reverse", skv);
-      e = oal::state_scan(s.dcarry, s.dt_img, nullptr, x.dstate_in, nullptr, units, nb, 1, cr.trim, skv); }
+      e = oal::state_scan(s.dcarry, s.dt_img, nullptr, x.dstate_in, nullptr, units, nb, 1, cr.trim, nullptr, 0, nullptr, skv); }
     if (e != cudaSuccess) return fail_cuda(e, "reverse state scan kernel");
     if (want_k) {
       { LaunchScope scope("feature_grad_k", skv);
@@ -758,6 +763,7 @@ static int forward_entry(const OalProblem* p, const void* q, const void* k, cons
   if (!q || !k || !v || !dim_perm || !group_start || !src.A || !src.B || !src.C || !out || !num || !den || !status)
     return fail(OAL_ERR_ARGUMENT, "oal_forward: NULL tensor pointer");
   float* ds = nullptr;
+  int32_t* update_status = nullptr;
   if (p->precision == OAL_PRECISION_FP32_IEEE) {
     if (state_in) return fail(OAL_ERR_ARGUMENT, "fp32_ieee mode keeps no chunk state: state_in must be NULL");
   } else {
@@ -766,8 +772,9 @@ static int forward_entry(const OalProblem* p, const void* q, const void* k, cons
     if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_forward: workspace too small");
     if (!saved_state) return fail(OAL_ERR_ARGUMENT, "oal_forward: saved_state is NULL");
     ds = s.ds;
+    update_status = s.update_status;
   }
-  return forward_core(p, q, k, v, dim_perm, group_start, src, out, num, den, saved_state, state_in, ds, status, sink, true,
+  return forward_core(p, q, k, v, dim_perm, group_start, src, out, num, den, saved_state, state_in, ds, update_status, status, sink, true,
                       static_cast<cudaStream_t>(stream));
 }
 
@@ -968,9 +975,9 @@ int oal_forward_local_state(const OalProblem* p, const void* k, const void* v, f
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int units = p->batch * p->kv_heads, nb = chunk_count(p);
   cudaError_t e;
-  { LaunchScope scope("state_update", st); e = oal::state_update(k, v, s.ds, units, p->seq_len, nb, nb, nullptr, 0, status, st); }
+  { LaunchScope scope("state_update", st); e = oal::state_update(k, v, s.ds, units, p->seq_len, nb, nb, nullptr, 0, status, nullptr, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
-  { LaunchScope scope("state_total", st); e = oal::state_scan(s.ds, nullptr, nullptr, nullptr, state_total, units, nb, 0, false, st); }
+  { LaunchScope scope("state_total", st); e = oal::state_scan(s.ds, nullptr, nullptr, nullptr, state_total, units, nb, 0, false, nullptr, 0, nullptr, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state total kernel");
   return OAL_OK;
 }
@@ -997,7 +1004,8 @@ int oal_backward_local_state(const OalProblem* p, const void* q, const int32_t* 
   if ((rc = backward_dstate(&local, q, saved_state, ChunkRange{false, chunk_count(p), 0}, s, status, st))) return rc;
   cudaError_t e;
   { LaunchScope scope("state_total", st);
-    e = oal::state_scan(s.dcarry, nullptr, nullptr, nullptr, dstate_total, p->batch * p->kv_heads, chunk_count(p), 1, false, st); }
+    e = oal::state_scan(s.dcarry, nullptr, nullptr, nullptr, dstate_total, p->batch * p->kv_heads, chunk_count(p), 1, false, nullptr, 0,
+                        nullptr, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state gradient total kernel");
   return OAL_OK;
 }
@@ -1063,7 +1071,7 @@ int oal_forward_static_scratch(const OalProblem* p, const void* q, const void* k
   rc = static_scratch_address(&scratch);
   if (rc) return rc;
   return forward_core(p, q, k, v, dim_perm, group_start, explicit_coefs(coef_a, coef_b, coef_c), out, num, den, saved_state,
-                      nullptr, scratch, status, oal::StatusSink{nullptr, nullptr}, false, static_cast<cudaStream_t>(stream));
+                      nullptr, scratch, nullptr, status, oal::StatusSink{nullptr, nullptr}, false, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

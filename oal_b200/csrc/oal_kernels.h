@@ -67,12 +67,15 @@ size_t state_slab_image_bytes();           // bytes of one slab image [10][128][
 cudaError_t build_coef_table(const int32_t* dim_perm, const int32_t* group_start, const float* A,
                              const float* Bc, const float* Cc, int Hq, int G, float scale, float* table,
                              cudaStream_t st);
-// increments of the first NC chunks; `prologue` (optional): its blocks ride in the same launch
+// increments of the first NC chunks; `prologue` (optional): its blocks ride in the same launch.  block_status: words
+// [state_update_blocks] for state_scan to merge, or null where no prologue clears `status` in this launch
+int state_update_blocks(int units, int NC);
 cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, const PrologueArgs* prologue,
-                         int q_heads, int32_t* status, cudaStream_t st);
+                         int q_heads, int32_t* status, int32_t* block_status, cudaStream_t st);
 // image_lo: optional second image holding bf16(state - bf16(state)); trim: see state_scan_kernel
 cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float* state_in, float* state_total,
-                       int units, int NB, int reverse, bool trim, cudaStream_t st);
+                       int units, int NB, int reverse, bool trim, const int32_t* block_status, int n_status, int32_t* status,
+                       cudaStream_t st);
 // chunks [c0, c0 + NC) of every sequence; the other rows of out64 / out1 are not written
 cudaError_t cross_read(bool query, const void* x, const void* image, const float* coef_table, float* out64,
                        float* out1, int B, int H, int rep, int N, int NB, int c0, int NC, int32_t* status, cudaStream_t st);

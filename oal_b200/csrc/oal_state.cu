@@ -65,6 +65,7 @@ struct StateUpdateArgs {
   float* ds;                    // [units, NB] chunks of F_ROWS x EP floats in state_inc_offset order
   int N, NB, NC;                // chunks of the sequence; chunks whose increment is computed (the first NC)
   int32_t* status;
+  int32_t* block_status;        // with a prologue that clears `status` in this launch: a word per block instead, see state_scan
 };
 
 __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const StateUpdateArgs a, const PrologueArgs pro,
@@ -150,7 +151,11 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   epilogue(ns - 1);
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, 256);
-  if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
+  if (tid == 0) {
+    const int32_t bits = dead ? w.status_bits() : 0;
+    if (a.block_status) a.block_status[item] = bits;
+    else if (bits) atomicOr(a.status, bits);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -162,12 +167,15 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
 //   nothing reads its image, and the increment of the last one visited reaches no image: neither is touched.
 // image_lo (optional): a second image of the rounding remainders, bf16(state - bf16(state)); the
 // coefficient-gradient dot products of the backward read state = image + image_lo.
+// block_status (optional): words left by the blocks of a state update whose launch also cleared `status`; nothing orders
+// that store against an atomic of the same launch, so they are merged into it here.
 // ---------------------------------------------------------------------------
 constexpr int SCAN_AHEAD = 4;
 
 __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_bfloat16* image,
                                                          __nv_bfloat16* image_lo, const float* state_in,
-                                                         float* state_total, int NB, int reverse, int trim) {
+                                                         float* state_total, int NB, int reverse, int trim,
+                                                         const int32_t* block_status, int n_status, int32_t* status) {
   constexpr size_t CHUNK = (size_t)F_ROWS * EP;
   static_assert(CHUNK % 1024 == 0, "the grid covers a chunk exactly");
   const size_t x = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;      // element inside a chunk, image order
@@ -175,6 +183,8 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_b
   // row-major position of the same element in state_in / state_total
   const int tile = (int)(x >> 10), within = (int)(x & 1023);          // 1024 = 128 rows x 8 columns
   const size_t rm = (size_t)((tile / (EP / 8)) * 128 + (within >> 3)) * EP + (tile % (EP / 8)) * 8 + (within & 7);
+  for (size_t b = (size_t)blockIdx.y * (CHUNK / 4) + x / 4; b < (size_t)n_status; b += (size_t)gridDim.y * (CHUNK / 4))
+    if (block_status[b]) atomicOr(status, block_status[b]);
   float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
   if (state_in) run = *reinterpret_cast<const float4*>(state_in + u * CHUNK + rm);
   const float* src = ds + u * NB * CHUNK + x;
@@ -434,22 +444,25 @@ cudaError_t build_coef_table(const int32_t* dim_perm, const int32_t* group_start
   return cudaGetLastError();
 }
 
+int state_update_blocks(int units, int NC) { return SU_GROUPS * NC * units; }
+
 cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, const PrologueArgs* prologue,
-                         int q_heads, int32_t* status, cudaStream_t st) {
+                         int q_heads, int32_t* status, int32_t* block_status, cudaStream_t st) {
   const int smem = 2 * SLAB_A_BYTES + SLAB_S_BYTES;
   cudaError_t e = allow_smem<state_update_kernel>(smem);
   if (e != cudaSuccess) return e;
-  StateUpdateArgs a{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ds, N, NB, NC, status};
+  StateUpdateArgs a{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ds, N, NB, NC, status, block_status};
   const int n_pro = prologue ? q_heads : 0;
-  state_update_kernel<<<n_pro + SU_GROUPS * NC * units, GEN_THREADS, smem, st>>>(a, prologue ? *prologue : PrologueArgs{}, n_pro);
+  state_update_kernel<<<n_pro + state_update_blocks(units, NC), GEN_THREADS, smem, st>>>(a, prologue ? *prologue : PrologueArgs{}, n_pro);
   return cudaGetLastError();
 }
 
 cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float* state_in, float* state_total,
-                       int units, int NB, int reverse, bool trim, cudaStream_t st) {
+                       int units, int NB, int reverse, bool trim, const int32_t* block_status, int n_status, int32_t* status,
+                       cudaStream_t st) {
   state_scan_kernel<<<dim3(F_ROWS * EP / 1024, units), 256, 0, st>>>(
       ds, static_cast<__nv_bfloat16*>(image), static_cast<__nv_bfloat16*>(image_lo), state_in, state_total, NB, reverse,
-      trim ? 1 : 0);
+      trim ? 1 : 0, block_status, block_status ? n_status : 0, status);
   return cudaGetLastError();
 }
 

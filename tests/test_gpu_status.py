@@ -67,3 +67,41 @@ def test_non_finite_factors_raise(n, g, value):
     with pytest.raises(RuntimeError, match=ERROR):
         step.check_status()
     hd.forget_captured_status()
+
+
+# one chunk (prologue alone), several (prologue in the state update's launch, its rotations beside it or in it)
+@pytest.mark.parametrize("n", [100, 300, 1000])
+@pytest.mark.parametrize("overlap", [1, 0])
+def test_packed_forward_owns_its_status_words(n, overlap):
+    """Status words and workspace hold anything before the call; a clean call leaves zero, delivers it and counts no
+    word of an earlier one."""
+    import ctypes
+
+    from oal_b200 import _lib
+    from oal_b200.hd_block_gemm import make_problem
+    from oal_b200.hd_block_gemm_autograd import build_group_tables
+
+    lib = _lib.load()
+    q, k, v, groups = _inputs(n, 8)
+    tables = build_group_tables(groups.expand(4, -1), 8)
+    factor = torch.full((4, 45), 0.5, device="cuda")
+    problem = make_problem((1, 4, 2, n, 64, 64), groups=8, io_dtype=torch.bfloat16, out_dtype=torch.bfloat16,
+                           precision="bf16_tensorcore", chunk=128, scale=0.125, floor=1e-38, flags=_lib.FLAG_ZERO_STATE_IN)
+    out, num, den = torch.empty_like(q), torch.empty(q.shape, device="cuda"), torch.empty(q.shape[:3], device="cuda")
+    ws, saved = (torch.full((_lib.workspace_bytes(problem, phase),), 255, dtype=torch.uint8, device="cuda") for phase in (0, 2))
+    coefs, status = torch.empty(4 * 73, device="cuda"), torch.full((2,), 0x55555555, dtype=torch.int32, device="cuda")
+    ticket, word = ctypes.c_int64(0), ctypes.c_int32(-1)
+    torch.cuda.synchronize()
+    lib.oal_set_overlap(overlap)
+    try:
+        _lib.check(lib.oal_forward_packed(
+            ctypes.byref(problem), *(_lib.ptr(t) for t in (q, k, v, tables.dim_perm, tables.group_start, factor)), 4, 1e-6,
+            *(_lib.ptr(t) for t in (coefs, out, num, den, saved, ws)), ws.numel(), _lib.ptr(status), ctypes.byref(ticket),
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        assert lib.oal_status_poll(ticket.value, 1, ctypes.byref(word)) == 1 and word.value == 0
+    finally:
+        lib.oal_set_overlap(1)
+    torch.cuda.synchronize()
+    assert status[0].item() == 0 and torch.isfinite(out).all()
+    want = oal_b200.oal_attention(q, k, v, groups, factor, scale=0.125)
+    assert torch.equal(out, want)
