@@ -164,7 +164,7 @@ int oal_backward(const OalProblem* problem, const void* q, const void* k, const 
  * kernels.  coefs: fp32 [q_heads * (1 + G + G * G)], written by the forward (A, then B, then C) and read by the
  * backward.  status: two words, cleared by the call itself.  ticket (may be NULL: the status stays on the device):
  * the last kernel also writes the word to pinned host memory, to be read with oal_status_poll; a ticket stays valid
- * for the next 1023 such calls on its device.
+ * for the next 1023 such calls on its device, and until it has been read while fewer than 4096 are unread.
  */
 int oal_forward_packed(const OalProblem* problem, const void* q, const void* k, const void* v, const int32_t* dim_perm,
                        const int32_t* group_start, const float* factor, int factor_rows, float kernel_eps, float* coefs,

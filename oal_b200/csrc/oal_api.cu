@@ -4,10 +4,12 @@
 
 #include <atomic>
 #include <chrono>
+#include <deque>
 #include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "oal_intra.cuh"
@@ -80,56 +82,150 @@ std::mutex g_status_mutex;
 StatusRing g_status[64];
 
 // ---- delivered status words -----------------------------------------------------------------------
-// A call that takes a ticket has its last kernel write the status word straight into a ring of pinned, mapped host
-// words: no copy, no event, nothing queued beside the call, and a waiting host sees it a microsecond after the
-// kernel has written it.
-constexpr int DELIVERY_RING = 1024;
-struct DeliveryRing {
-  int32_t* host = nullptr;
-  long long next = 0;
+// A call that takes a ticket has its last kernel write the status word straight into a pinned, mapped host word: no
+// copy, and a waiting host sees it a microsecond after the kernel has written it.  A ticket names a slot (word, event
+// behind the call) and the slot's use.  A slot is taken again only when its call's word is in, at least
+// DELIVERY_KEEP later calls have taken one, and the word has been read -- or, at the limit of slots, unread (a caller
+// that never polls).  A call still in flight keeps its slot whatever the others do: a late word never lands in
+// another call's ticket.
+constexpr int DELIVERY_KEEP = 1024, DELIVERY_LIMIT = 4 * DELIVERY_KEEP, DELIVERY_LOOK = 64;
+struct DeliverySlot {
+  volatile int32_t* word = nullptr;
+  cudaEvent_t done = nullptr;
+  long long use = 0, taken = 0;      // uses of this slot so far; the device's count of takes at its last one
+  bool recorded = false, read = false;
 };
-DeliveryRing g_delivery[64];
+struct DeliverySlots {
+  std::vector<DeliverySlot> slots;   // reserved at the first take: never moves
+  std::deque<int> order;             // by take, oldest first
+  int32_t* block = nullptr;          // pinned words that have no slot yet
+  long long takes = 0;
+};
+std::mutex g_delivery_mutex;
+DeliverySlots g_delivery[64];
 constexpr int64_t TICKET_DELIVERED = (int64_t)1 << 62;
+constexpr int TICKET_SLOT_BITS = 12;
+static_assert(DELIVERY_LIMIT <= 1 << TICKET_SLOT_BITS, "slot index of a ticket");
 
-// Spins on a delivered word; past the limit it lets the device drain once.  False: the word never came.
-bool wait_delivered(const int32_t* word, int dev) {
-  const volatile int32_t* w = word;
+// Calls that another thread's stream capture would not allow (event waits) in this scope.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Waits for one call's word, without any lock: on the word itself for a while (a short call is over in that time), then
+// on the event behind the call -- never on the device, which may have other work queued for seconds.
+cudaError_t wait_delivered(const volatile int32_t* word, cudaEvent_t done) {
   const auto t0 = std::chrono::steady_clock::now();
-  for (unsigned spin = 1;; ++spin) {
-    if (*w & oal::STATUS_DELIVERED) return true;
-    if ((spin & 1023) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) break;
-  }
-  int current = dev;
-  cudaGetDevice(&current);
-  if (current != dev) cudaSetDevice(dev);
-  cudaDeviceSynchronize();
-  if (current != dev) cudaSetDevice(current);
-  return (*w & oal::STATUS_DELIVERED) != 0;
+  for (unsigned spin = 1; !(*word & oal::STATUS_DELIVERED); ++spin)
+    if ((spin & 1023) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) {
+      if (!done) return cudaSuccess;
+      RelaxedCapture scope;
+      cudaError_t e;      // an event that puts the thread to sleep itself raises an interrupt in every call
+      while ((e = cudaEventQuery(done)) == cudaErrorNotReady) std::this_thread::sleep_for(std::chrono::microseconds(20));
+      return e;
+    }
+  return cudaSuccess;
 }
 
-// A fresh word of the current device's ring and its ticket.
+int add_delivery_slot(DeliverySlots& d) {
+  const int n = (int)d.slots.size();
+  if (n == 0) d.slots.reserve(DELIVERY_LIMIT);
+  if (n % DELIVERY_KEEP == 0) {
+    const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&d.block), DELIVERY_KEEP * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) return fail_cuda(e, "status delivery");
+  }
+  DeliverySlot s;
+  s.word = d.block + n % DELIVERY_KEEP;
+  const cudaError_t e = cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming);
+  if (e != cudaSuccess) return fail_cuda(e, "status delivery");
+  d.slots.push_back(s);
+  return n;
+}
+
+// A word of the current device for one call, and its ticket.
 int take_delivery(int32_t** word, int64_t* ticket) {
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  const cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return fail_cuda(e, "status delivery");
   if (dev < 0 || dev >= 64) return fail(OAL_ERR_ARGUMENT, "status delivery: device index out of range");
-  std::lock_guard<std::mutex> lock(g_status_mutex);
-  DeliveryRing& r = g_delivery[dev];
-  if (!r.host) {
-    e = cudaHostAlloc(reinterpret_cast<void**>(&r.host), DELIVERY_RING * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped);
-    if (e != cudaSuccess) {
-      r.host = nullptr;
-      return fail_cuda(e, "status delivery");
+  std::lock_guard<std::mutex> lock(g_delivery_mutex);
+  DeliverySlots& d = g_delivery[dev];
+  const bool at_limit = d.slots.size() == DELIVERY_LIMIT;
+  int slot = -1, looked = 0;
+  for (auto it = d.order.begin(); it != d.order.end() && (at_limit || looked < DELIVERY_LOOK); ++it, ++looked) {
+    const DeliverySlot& s = d.slots[*it];
+    if (d.takes - s.taken < DELIVERY_KEEP) break;
+    if ((*s.word & oal::STATUS_DELIVERED) && (s.read || at_limit)) {
+      slot = *it;
+      d.order.erase(it);
+      break;
     }
-    for (int i = 0; i < DELIVERY_RING; ++i) r.host[i] = oal::STATUS_DELIVERED;
   }
-  int32_t* slot = r.host + r.next % DELIVERY_RING;
-  if (!wait_delivered(slot, dev)) *slot = 0;      // its call, 1024 calls ago, died: the device reported that elsewhere
-  *static_cast<volatile int32_t*>(slot) = 0;
-  *word = slot;
-  *ticket = TICKET_DELIVERED | ((int64_t)dev << 48) | (int64_t)r.next;
-  ++r.next;
+  if (slot < 0) {
+    if (at_limit) return fail(OAL_ERR_CUDA, "status delivery: too many calls in flight");
+    if ((slot = add_delivery_slot(d)) < 0) return slot;
+  }
+  DeliverySlot& s = d.slots[slot];
+  *s.word = 0;
+  s.recorded = s.read = false;
+  s.taken = d.takes++;
+  ++s.use;
+  d.order.push_back(slot);
+  *word = const_cast<int32_t*>(s.word);
+  *ticket = TICKET_DELIVERED | ((int64_t)dev << 48) | (int64_t)((s.use << TICKET_SLOT_BITS | slot) & (((int64_t)1 << 48) - 1));
   return OAL_OK;
+}
+
+// The slot of a ticket, or null when the slot has been taken again since; g_delivery_mutex held.
+DeliverySlot* delivery_slot(int64_t ticket) {
+  const int dev = (int)((ticket & ~TICKET_DELIVERED) >> 48);
+  const size_t slot = (size_t)(ticket & ((1 << TICKET_SLOT_BITS) - 1));
+  const long long use = (ticket & (((int64_t)1 << 48) - 1)) >> TICKET_SLOT_BITS;
+  if (dev < 0 || dev >= 64 || slot >= g_delivery[dev].slots.size()) return nullptr;
+  DeliverySlot& s = g_delivery[dev].slots[slot];
+  return s.use == use ? &s : nullptr;
+}
+
+// After a call's last launch, or its failure: an event behind it, or a word that nothing else will write.
+void finish_delivery(int64_t ticket, int rc, cudaStream_t st) {
+  std::lock_guard<std::mutex> lock(g_delivery_mutex);
+  DeliverySlot* s = delivery_slot(ticket);
+  if (!s) return;
+  if (rc) {
+    *s->word = oal::STATUS_DELIVERED;
+    s->read = true;
+    return;
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  s->recorded = cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
+                cudaEventRecord(s->done, st) == cudaSuccess;
+}
+
+int poll_delivery(int64_t ticket, bool block, int32_t* value) {
+  constexpr const char* kExpired = "oal_status_poll: ticket expired or unknown";
+  const volatile int32_t* word;
+  cudaEvent_t done;
+  {
+    std::lock_guard<std::mutex> lock(g_delivery_mutex);
+    DeliverySlot* s = delivery_slot(ticket);
+    if (!s) return fail(OAL_ERR_ARGUMENT, kExpired);
+    word = s->word;
+    done = s->recorded ? s->done : nullptr;
+  }
+  if (block) {
+    const cudaError_t e = wait_delivered(word, done);
+    if (e != cudaSuccess) return fail_cuda(e, "oal_status_poll");
+  }
+  std::lock_guard<std::mutex> lock(g_delivery_mutex);
+  DeliverySlot* s = delivery_slot(ticket);
+  if (!s) return fail(OAL_ERR_ARGUMENT, kExpired);
+  const int32_t seen = *s->word;
+  if (!(seen & oal::STATUS_DELIVERED)) return block ? fail(OAL_ERR_CUDA, "oal_status_poll: the call's status word was never written") : 0;
+  s->read = true;
+  *value = seen & ~oal::STATUS_DELIVERED;
+  return 1;
 }
 
 // ---- side streams ------------------------------------------------------------------------------
@@ -802,7 +898,7 @@ int oal_forward_packed(const OalProblem* p, const void* q, const void* k, const 
   }
   int rc = forward_entry(p, q, k, v, dim_perm, group_start, packed_coefs(p, factor, factor_rows, kernel_eps, coefs), out, num, den,
                          saved_state, nullptr, workspace, workspace_bytes, status, sink, stream);
-  if (rc && sink.host) *sink.host = oal::STATUS_DELIVERED;      // nothing will write it
+  if (ticket) finish_delivery(*ticket, rc, static_cast<cudaStream_t>(stream));
   return rc;
 }
 
@@ -855,7 +951,7 @@ int oal_backward_packed(const OalProblem* p, const void* q, const void* k, const
     const cudaError_t e = oal::deliver_status(status, sink, st);
     if (e != cudaSuccess) rc = fail_cuda(e, "status delivery kernel");
   }
-  if (rc && sink.host) *sink.host = oal::STATUS_DELIVERED;
+  if (ticket) finish_delivery(*ticket, rc, st);
   return rc;
 }
 
@@ -895,28 +991,9 @@ int oal_status_defer(const int32_t* status, void* stream, int64_t* ticket) {
 
 int oal_status_poll(int64_t ticket, int block, int32_t* value) {
   if (!value) return fail(OAL_ERR_ARGUMENT, "oal_status_poll: NULL pointer");
-  const bool delivered = ticket & TICKET_DELIVERED;
-  const int dev = (int)((ticket & ~TICKET_DELIVERED) >> 48);
+  if (ticket & TICKET_DELIVERED) return poll_delivery(ticket, block != 0, value);
+  const int dev = (int)(ticket >> 48);
   const long long seq = (long long)(ticket & (((int64_t)1 << 48) - 1));
-  if (dev >= 0 && dev < 64 && delivered) {
-    const int32_t* word;
-    {
-      std::lock_guard<std::mutex> lock(g_status_mutex);
-      const DeliveryRing& r = g_delivery[dev];
-      if (seq >= r.next || seq + DELIVERY_RING <= r.next) return fail(OAL_ERR_ARGUMENT, "oal_status_poll: ticket expired or unknown");
-      word = r.host + seq % DELIVERY_RING;
-    }
-    if (block) {
-      if (!wait_delivered(word, dev)) {
-        const cudaError_t e = cudaGetLastError();
-        return e != cudaSuccess ? fail_cuda(e, "oal_status_poll") : fail(OAL_ERR_CUDA, "oal_status_poll: the call's status word was never written");
-      }
-    } else if (!(*static_cast<const volatile int32_t*>(word) & oal::STATUS_DELIVERED)) {
-      return 0;
-    }
-    *value = *static_cast<const volatile int32_t*>(word) & ~oal::STATUS_DELIVERED;
-    return 1;
-  }
   if (dev < 0 || dev >= 64) return fail(OAL_ERR_ARGUMENT, "oal_status_poll: bad ticket");
   cudaEvent_t done;
   int32_t* word;

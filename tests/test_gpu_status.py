@@ -105,3 +105,91 @@ def test_packed_forward_owns_its_status_words(n, overlap):
     assert status[0].item() == 0 and torch.isfinite(out).all()
     want = oal_b200.oal_attention(q, k, v, groups, factor, scale=0.125)
     assert torch.equal(out, want)
+
+
+SLEEP = 1_000_000_000      # clocks of torch.cuda._sleep: about half a second
+
+
+def _warm(prepared, *leaves):
+    """Memory and slots of a call on the current stream, before anything is timed or captured."""
+    for _ in range(3):
+        oal_b200.run_prepared_grouped_hd_block_gemm(prepared, *leaves)
+    torch.cuda.current_stream().synchronize()
+
+
+def test_a_stalled_call_keeps_its_status_word_and_delays_no_other_stream():
+    """A training call behind half a second of other work, then more inference calls on another stream than there are
+    slots: they finish first, and the stalled call's error is still reported."""
+    from oal_b200 import hd_block_gemm_autograd as hd
+
+    q, k, v, groups = _inputs(64, 4)
+    bad = torch.full((4, 15), float("nan"), device="cuda").requires_grad_()
+    good = torch.full((4, 15), 0.5, device="cuda")
+    train = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, bad, precision="bf16_tensorcore")
+    infer = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, good, precision="bf16_tensorcore")
+    stalled, other = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(other):
+        _warm(infer, q, k, v, good)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stalled):
+        torch.cuda._sleep(2 * SLEEP)
+        oal_b200.run_prepared_grouped_hd_block_gemm(train, q, k, v, bad)
+        end = stalled.record_event()
+    with torch.cuda.stream(other):
+        for _ in range(1100):
+            oal_b200.run_prepared_grouped_hd_block_gemm(infer, q, k, v, good)
+            assert not end.query()
+    with pytest.raises(RuntimeError, match=ERROR):
+        hd.check_pending_status(block=True)
+    assert end.query()
+    for _ in range(5000):      # and the slots do not run out
+        oal_b200.run_prepared_grouped_hd_block_gemm(infer, q, k, v, good)
+
+
+def test_a_long_inference_call_waits_for_its_own_stream_only():
+    q, k, v, groups = _inputs(64, 4)
+    factor = torch.full((4, 15), 0.5, device="cuda")
+    prepared = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, factor, precision="bf16_tensorcore")
+    own, other = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(own):
+        _warm(prepared, q, k, v, factor)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(2 * SLEEP)
+        end = other.record_event()
+    with torch.cuda.stream(own):
+        torch.cuda._sleep(SLEEP // 5)
+        oal_b200.run_prepared_grouped_hd_block_gemm(prepared, q, k, v, factor)
+    assert not end.query()
+
+
+def test_a_long_inference_call_beside_a_capture():
+    """One thread records a graph while another waits for a call of 100 ms: both come through."""
+    import threading
+
+    q, k, v, groups = _inputs(64, 4)
+    factor = torch.full((4, 15), 0.5, device="cuda")
+    prepared = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, factor, precision="bf16_tensorcore")
+    want = oal_b200.run_prepared_grouped_hd_block_gemm(prepared, q, k, v, factor)[0]
+    stream, started, got = torch.cuda.Stream(), threading.Event(), []
+
+    def wait_for_a_call():
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(SLEEP // 5)
+            started.set()
+            got.append(oal_b200.run_prepared_grouped_hd_block_gemm(prepared, q, k, v, factor)[0])
+
+    with torch.cuda.stream(stream):
+        _warm(prepared, q, k, v, factor)
+    x = torch.zeros(8, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    thread = threading.Thread(target=wait_for_a_call)
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):      # other threads may allocate
+        thread.start()
+        started.wait()
+        thread.join()
+        x += 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.eq(1).all() and torch.equal(got[0], want)
