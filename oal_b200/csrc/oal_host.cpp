@@ -17,6 +17,7 @@
 #include <deque>
 #include <map>
 #include <mutex>
+#include <optional>
 
 #include "../../include/oal_b200.h"
 
@@ -44,7 +45,7 @@ struct Pending {
 std::mutex g_pending_mutex;
 std::map<int, std::deque<Pending>> g_pending;
 std::atomic<int64_t> g_call_ids{1};
-constexpr size_t kPendingLimit = 256;      // a ticket stays valid for 1023 later ones on its device
+constexpr size_t kPendingLimit = 256;
 
 void raise_for_bits(int bits, const std::string& where) {
   if (bits & OAL_STATUS_WAIT_TIMEOUT) {
@@ -58,18 +59,21 @@ void raise_for_bits(int bits, const std::string& where) {
                              ")" + where);
 }
 
-// Finished entries in order; the first that reports a problem is dropped and raised.
-void drain(int device, bool block) {
+// Finished entries in order; the first that reports a problem is dropped and raised.  With `block` also unfinished ones,
+// until `leave` are left.  Called without the GIL (see Unlocked).
+void drain(int device, bool block, size_t leave = 0) {
   for (;;) {
     Pending e;
+    bool wait;
     {
       std::lock_guard<std::mutex> lock(g_pending_mutex);
       auto it = g_pending.find(device);
       if (it == g_pending.end() || it->second.empty()) return;
       e = it->second.front();
+      wait = block && it->second.size() > leave;
     }
     int32_t word = 0;
-    const int rc = oal_status_poll(e.ticket, block ? 1 : 0, &word);
+    const int rc = oal_status_poll(e.ticket, wait ? 1 : 0, &word);
     if (rc == 0) return;
     {
       std::lock_guard<std::mutex> lock(g_pending_mutex);
@@ -90,8 +94,17 @@ void enqueue(int device, int64_t ticket, const char* what) {
     q.push_back(Pending{ticket, g_call_ids++, what});
     full = q.size() > kPendingLimit;
   }
-  if (full) drain(device, true);
+  if (full) drain(device, true, kPendingLimit);
 }
+
+// Gives up the GIL where it is held (a call from Python; the autograd engine's threads come without it): this file
+// waits for calls, and the work that they wait for may need another Python thread's launch.
+struct Unlocked {
+  std::optional<py::gil_scoped_release> release;
+  Unlocked() {
+    if (PyGILState_Check()) release.emplace();
+  }
+};
 
 void check_pending(bool block, int device) {
   std::vector<int> devices;
@@ -193,12 +206,7 @@ Forward forward_call(const Prepared& p, const Tensor& q, const Tensor& k, const 
     g_captured.emplace_back(dev, r.meta.view(at::kInt).slice(0, 0, 1), "forward");
   } else if (blocking) {
     int32_t word = 0;
-    int rc;
-    {
-      py::gil_scoped_release release;
-      rc = oal_status_poll(ticket, 1, &word);
-    }
-    check_rc(rc);
+    check_rc(oal_status_poll(ticket, 1, &word));
     if (word) raise_for_bits(word, "");
   } else {
     enqueue(dev, ticket, "forward");
@@ -284,14 +292,20 @@ struct PackedNode : torch::autograd::Function<PackedNode> {
 // (out, numerator, denominator), or None when the arguments are not those of the preparation
 py::object run(const std::shared_ptr<Prepared>& p, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& f) {
   if (!p->takes(q, k, v, f)) return py::none();
-  if (p->grad[0] || p->grad[1] || p->grad[2] || p->grad[3]) {
-    variable_list o = PackedNode::apply(q, k, v, f, p);
-    return py::make_tuple(o[0], o[1], o[2]);
+  Tensor out, num, den;
+  {
+    Unlocked unlocked;
+    if (p->grad[0] || p->grad[1] || p->grad[2] || p->grad[3]) {
+      variable_list o = PackedNode::apply(q, k, v, f, p);
+      out = o[0], num = o[1], den = o[2];
+    } else {
+      at::AutoDispatchBelowADInplaceOrView below;
+      Forward r = forward_call(*p, q, k, v, f, true);
+      out = r.out, den = r.den;
+      num = p->Dv != OAL_HEAD_DIM ? r.num.slice(-1, 0, p->Dv).contiguous() : r.num;
+    }
   }
-  at::AutoDispatchBelowADInplaceOrView below;
-  Forward r = forward_call(*p, q, k, v, f, true);
-  if (p->Dv != OAL_HEAD_DIM) r.num = r.num.slice(-1, 0, p->Dv).contiguous();
-  return py::make_tuple(r.out, r.num, r.den);
+  return py::make_tuple(out, num, den);
 }
 
 std::shared_ptr<Prepared> prepare(py::bytes problem, std::vector<int64_t> geometry, int64_t groups, at::ScalarType dtype,
@@ -324,7 +338,11 @@ std::shared_ptr<Prepared> prepare(py::bytes problem, std::vector<int64_t> geomet
 // stands for every head.  Dimensions beyond D are padding and belong to group 0.
 std::tuple<int, Tensor, Tensor> group_tables(const Tensor& ids, int64_t hq, int64_t gmax) {
   const c10::Device device = ids.device();
-  const Tensor host = ids.detach().to(at::kCPU, at::kLong).contiguous();
+  Tensor host;
+  {
+    Unlocked unlocked;      // waits for the work that writes the ids
+    host = ids.detach().to(at::kCPU, at::kLong).contiguous();
+  }
   const int64_t rows = host.size(0), d = host.size(1);
   const int64_t* id = host.data_ptr<int64_t>();
   for (int64_t r = 0; r < rows; ++r) {

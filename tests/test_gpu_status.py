@@ -193,3 +193,105 @@ def test_a_long_inference_call_beside_a_capture():
     graph.replay()
     torch.cuda.synchronize()
     assert x.eq(1).all() and torch.equal(got[0], want)
+
+
+def _ticks(run):
+    """The longest pause of another Python thread while ``run()`` is under way."""
+    import threading
+    import time
+
+    stop, pauses = threading.Event(), [0.0]
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            pauses.append(now - last)
+            last = now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        run()
+    finally:
+        stop.set()
+        thread.join()
+    return max(pauses)
+
+
+def test_waiting_leaves_other_python_threads_running():
+    """A full queue of unfinished training calls, an inference call and group ids that are not there yet: each waits
+    for half a second or more of device work, without the interpreter's lock."""
+    from oal_b200 import hd_block_gemm_autograd as hd
+
+    q, k, v, groups = _inputs(64, 4)
+    factor = torch.full((4, 15), 0.5, device="cuda")
+    trained = factor.clone().requires_grad_()
+    train = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, trained, precision="bf16_tensorcore")
+    infer = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, factor, precision="bf16_tensorcore")
+    stream = torch.cuda.Stream()
+
+    def full_queue():
+        torch.cuda._sleep(2 * SLEEP)
+        for _ in range(260):
+            oal_b200.run_prepared_grouped_hd_block_gemm(train, q, k, v, trained)
+
+    def inference():
+        torch.cuda._sleep(2 * SLEEP)
+        oal_b200.run_prepared_grouped_hd_block_gemm(infer, q, k, v, factor)
+
+    def late_ids():
+        torch.cuda._sleep(2 * SLEEP)
+        oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups + 0, factor, precision="bf16_tensorcore")
+
+    with torch.cuda.stream(stream):
+        _warm(train, q, k, v, trained)
+        _warm(infer, q, k, v, factor)
+        for run in (full_queue, inference, late_ids):
+            assert _ticks(run) < 0.4, run.__name__
+            torch.cuda.synchronize()
+    hd.check_pending_status(block=True)
+
+
+def test_one_preparation_from_two_threads_on_two_streams():
+    import threading
+
+    from oal_b200 import hd_block_gemm_autograd as hd
+
+    q, k, v, groups = _inputs(300, 8)
+    factor = torch.full((4, 45), 0.5, device="cuda")
+    leaves = [t.clone().requires_grad_() for t in (q, k, v, factor)]
+    prepared = oal_b200.prepare_grouped_hd_block_gemm(*leaves[:3], groups, leaves[3], precision="bf16_tensorcore")
+
+    def step(scale):
+        own = [(t * scale).detach().requires_grad_() for t in (q, k, v, factor)]
+        out = oal_b200.run_prepared_grouped_hd_block_gemm(prepared, *own)[0]
+        out.backward(torch.ones_like(out))
+        return [out.detach(), *(t.grad for t in own)]
+
+    want = {scale: step(scale) for scale in (1.0, 0.5)}
+    torch.cuda.synchronize()
+    got, errors = {1.0: [], 0.5: []}, []
+
+    def work(scale):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for _ in range(50):
+                    got[scale].append(step(scale))
+            stream.synchronize()
+        except Exception as exc:
+            errors.append(exc)
+
+    threads = [threading.Thread(target=work, args=(scale,)) for scale in got]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    hd.check_pending_status(block=True)
+    assert not errors
+    for scale, passes in got.items():
+        for one in passes:
+            for x, y in zip(one, want[scale]):
+                assert torch.equal(x, y)
