@@ -251,7 +251,7 @@ def build_hd_block_gemm_plan(
     """Validate one invocation and size its workspaces (no device allocation)."""
     arguments = locals()
     try:      # a plan is a function of the geometry and the options alone: keep the latest ones
-        options = tuple((type(x), x) for name, x in arguments.items() if name not in ("q", "k", "v"))
+        options = tuple(_typed(x) for name, x in arguments.items() if name not in ("q", "k", "v"))
         key = (_validate_geometry(q, k, v), q.dtype, q.device, options)
         with _PLANS_LOCK:
             if (plan := _PLANS.get(key)) is not None:
@@ -266,6 +266,11 @@ def build_hd_block_gemm_plan(
             if len(_PLANS) > _PLANS_LIMIT:
                 _PLANS.popitem(last=False)
     return plan
+
+
+def _typed(x):
+    """An option as a key: 1, 1.0 and True are equal and hash alike, in a tuple too, but not all of them are legal."""
+    return (type(x), tuple(_typed(y) for y in x) if isinstance(x, tuple) else x)
 
 
 _PLANS: OrderedDict = OrderedDict()

@@ -177,3 +177,15 @@ def test_packed_pair_count_is_triangular():
         assert _infer_gmax((gmax + 1) * (gmax + 2) // 2) == gmax
     with pytest.raises(ValueError):
         _infer_gmax(7)
+
+
+def test_a_kept_plan_does_not_answer_for_options_of_other_types():
+    """Equal and of equal hash, but refused: whatever plan of the geometry has been built before."""
+    q, k, v = _case()
+    build_hd_block_gemm_plan(q, k, v, requested_gradient_mask=(True,) * 6, save_local_score=False, token_block=1)
+    with pytest.raises(TypeError, match="entries must be bool"):
+        build_hd_block_gemm_plan(q, k, v, requested_gradient_mask=(1,) * 6, save_local_score=False, token_block=1)
+    with pytest.raises(TypeError):
+        build_hd_block_gemm_plan(q, k, v, requested_gradient_mask=(True,) * 6, save_local_score=0, token_block=1)
+    with pytest.raises((TypeError, ValueError)):
+        build_hd_block_gemm_plan(q, k, v, requested_gradient_mask=(True,) * 6, save_local_score=False, token_block=True)
