@@ -10,7 +10,7 @@ node from (q, k, v, factor) to the result triple (``csrc/oal_host.cpp``),
 
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 
 import torch
 
@@ -58,7 +58,18 @@ class _PreparedGroupedHdBlockGemm:
     kernel_eps: float
     normalization_floor: float
     out_token_major: bool = False      # `out` is [B, N, Hq, 64] (an addition: see prepare_grouped_hd_block_gemm)
-    native: object = None              # the call as the native host path keeps it
+    # the call as the native host path keeps it: made from the fields above, also those of a changed or unpickled copy
+    native: object = field(init=False, repr=False, compare=False, default=None)
+
+    def __post_init__(self):
+        object.__setattr__(self, "native", _native_call(self))
+
+    def __getstate__(self):
+        return {name: value for name, value in self.__dict__.items() if name != "native"}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        self.__post_init__()
 
 
 def prepare_grouped_hd_block_gemm(
@@ -145,24 +156,26 @@ def _prepare(q, k, v, checked, factor, gmax, *, scale, kernel_eps, output_layout
     resolved_scale, token_major = _resolve_scale(scale, q.shape[-1]), output_layout == "tokens_first"
     return _PreparedGroupedHdBlockGemm(
         plan=plan, groups=groups, tables=tables, gmax=gmax, scale=resolved_scale, kernel_eps=resolved_eps,
-        normalization_floor=_POSITIVE_FP32_FLOOR, out_token_major=token_major,
-        native=_native_call(plan, tables, resolved_scale, resolved_eps, token_major, q))
+        normalization_floor=_POSITIVE_FP32_FLOOR, out_token_major=token_major)
 
 
-def _native_call(plan, tables, scale, kernel_eps, token_major, q):
+def _native_call(prepared):
     """Hand the frozen call to the native host path; None for tensors it does not run on."""
-    if q.device.type != "cuda":
+    plan, tables, token_major = prepared.plan, prepared.tables, prepared.out_token_major
+    device = torch.device(plan.device)
+    if device.type != "cuda" or tables.dim_perm.device != device or tables.group_start.device != device:
         return None
-    out_dtype = getattr(torch, plan.output_dtype)
+    io_dtype, out_dtype = getattr(torch, plan.input_dtype), getattr(torch, plan.output_dtype)
     mask = plan.requested_gradient_mask
-    problem = make_problem(plan.geometry, groups=tables.group_count, io_dtype=q.dtype,
+    problem = make_problem(plan.geometry, groups=tables.group_count, io_dtype=io_dtype,
                            out_dtype=out_dtype if out_dtype != torch.float64 else torch.float32, precision=plan.precision,
-                           chunk=plan.chunk_tokens, scale=scale, floor=_POSITIVE_FP32_FLOOR, grad_mask=_grad_bits(mask),
+                           chunk=plan.chunk_tokens, scale=prepared.scale, floor=prepared.normalization_floor,
+                           grad_mask=_grad_bits(mask),
                            flags=_lib.FLAG_ZERO_STATE_IN | (_lib.FLAG_OUT_TOKEN_MAJOR if token_major else 0))
     if token_major and plan.geometry[5] != _lib.HEAD_DIM:
         return None                     # refused where the call runs
-    return _lib.host().prepare(bytes(problem), list(plan.geometry), tables.group_count, q.dtype, out_dtype, q.device.index,
-                               tables.dim_perm, tables.group_start, kernel_eps,
+    return _lib.host().prepare(bytes(problem), list(plan.geometry), tables.group_count, io_dtype, out_dtype, device.index,
+                               tables.dim_perm, tables.group_start, prepared.kernel_eps,
                                [plan.forward_workspace_bytes, plan.backward_workspace_bytes, plan.saved_state_bytes],
                                [mask[0], mask[1], mask[2], any(mask[3:])])
 

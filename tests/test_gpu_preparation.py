@@ -1,0 +1,60 @@
+"""A preparation as a value: copies, pickles and changed copies run what their fields say."""
+
+import copy
+import dataclasses
+import io
+import pickle
+
+import pytest
+import torch
+
+import oal_b200
+
+pytestmark = pytest.mark.gpu
+
+
+def _prepared(n=150, **options):
+    gen = torch.Generator().manual_seed(7)
+    q, k, v = (torch.randn(1, h, n, 64, generator=gen).bfloat16().cuda() for h in (4, 2, 2))
+    groups = (torch.arange(64) % 4).to(torch.int32).cuda()
+    factor = (torch.rand(4, 15, generator=gen) * 0.9 + 0.1).cuda()
+    make = lambda **more: oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, factor, precision="bf16_tensorcore", **options, **more)
+    return make, (q, k, v, factor)
+
+
+def test_copies_and_pickles_run_the_same_call():
+    make, live = _prepared()
+    prepared = make()
+    want = oal_b200.run_prepared_grouped_hd_block_gemm(prepared, *live)
+    for other in (copy.copy(prepared), copy.deepcopy(prepared), pickle.loads(pickle.dumps(prepared))):
+        for got, x in zip(oal_b200.run_prepared_grouped_hd_block_gemm(other, *live), want):
+            assert torch.equal(got, x)
+
+
+def test_a_changed_copy_runs_its_own_options():
+    make, live = _prepared()
+    prepared = make()
+    for change in (dict(kernel_eps=0.5), dict(scale=0.3)):
+        changed = dataclasses.replace(prepared, **change)
+        for got, x in zip(oal_b200.run_prepared_grouped_hd_block_gemm(changed, *live),
+                          oal_b200.run_prepared_grouped_hd_block_gemm(make(**change), *live)):
+            assert torch.equal(got, x)
+    assert not torch.equal(oal_b200.run_prepared_grouped_hd_block_gemm(changed, *live)[0],
+                           oal_b200.run_prepared_grouped_hd_block_gemm(prepared, *live)[0])
+
+
+def test_a_layer_is_copied_and_saved_after_its_first_call():
+    from oal_b200 import attention_shell as shell
+
+    geo = shell.ModelGeometry(num_query_heads=4, num_kv_heads=2, hidden_size=256, head_dim=64)
+    groups = (torch.arange(64) % 4).to(torch.int32).expand(4, 64).clone()
+    torch.manual_seed(1)
+    layer = shell.OalAttentionLayer(0, groups, torch.full((4, 15), 0.5), cache=shell.PreparedCallCache(), geometry=geo,
+                                    dtype=torch.bfloat16).cuda()
+    x, rope = torch.randn(1, 130, 256, device="cuda").bfloat16(), shell.rope_tables(130, 64, device="cuda")
+    want = layer(x, rope)
+    file = io.BytesIO()
+    torch.save(layer, file)
+    file.seek(0)
+    for other in (copy.deepcopy(layer), torch.load(file, weights_only=False)):
+        assert torch.equal(other(x, rope), want)
