@@ -262,19 +262,34 @@ SideStreams* side_streams(std::unique_lock<std::mutex>& lock) {
   }
   return &x;
 }
-// side stream i starts after everything queued on `st` so far
-cudaStream_t fork_to(SideStreams* x, int i, cudaStream_t st) {
-  if (!x) return st;
-  if (cudaEventRecord(x->fork, st) != cudaSuccess || cudaStreamWaitEvent(x->s[i], x->fork, 0) != cudaSuccess) return st;
-  return x->s[i];
-}
-// mark the end of what was queued on side stream i; `st` waits for that mark in join_wait
-void join_mark(SideStreams* x, int i, cudaStream_t side, cudaStream_t st) {
-  if (x && side != st) cudaEventRecord(x->join[i], side);
-}
-void join_wait(SideStreams* x, int i, cudaStream_t side, cudaStream_t st) {
-  if (x && side != st) cudaStreamWaitEvent(st, x->join[i], 0);
-}
+// Work of one call on side stream i: starts after everything queued on `st` when it forks; mark() ends it, wait() makes
+// `st` wait for that mark.  Whatever way the call is left, an error return included, the caller's stream waits: it may
+// free the buffers or end a capture next.
+class SideWork {
+ public:
+  ~SideWork() { wait(); }
+  cudaStream_t fork(SideStreams* x, int i, cudaStream_t st) {
+    if (!x || cudaEventRecord(x->fork, st) != cudaSuccess || cudaStreamWaitEvent(x->s[i], x->fork, 0) != cudaSuccess) return st;
+    side_ = x->s[i];
+    st_ = st;
+    join_ = x->join[i];
+    open_ = true;
+    return side_;
+  }
+  void mark() {
+    if (open_ && !marked_) marked_ = cudaEventRecord(join_, side_) == cudaSuccess;
+  }
+  void wait() {
+    mark();
+    if (open_) cudaStreamWaitEvent(st_, join_, 0);
+    open_ = false;
+  }
+
+ private:
+  cudaStream_t side_ = nullptr, st_ = nullptr;
+  cudaEvent_t join_ = nullptr;
+  bool open_ = false, marked_ = false;
+};
 
 struct Carver {
   char* base;
@@ -527,6 +542,7 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
   float* coef_table = tc ? saved_coef_table(p, saved_state) : nullptr;
   std::unique_lock<std::mutex> side_lock;
   SideStreams* side = nullptr;
+  SideWork beside;
   cudaStream_t s0 = st;
   oal::PrologueArgs pro{};
   if (src.factor) {
@@ -539,22 +555,22 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
       // next but one: with both in the state kernel's launch the scan waited for the rotations.  Beside the state
       // kernels they cost the host a launch and two events.  14 / 2 heads, B = 1, both forms in us: forward + backward
       // N = 256 169 -> 160, N = 1024 198 -> 190, replayed 203 -> 192, 16 groups N = 4096 663 -> 647.
-      s0 = fork_to(side, 0, st);
+      s0 = beside.fork(side, 0, st);
       oal::PrologueArgs own = pro;
       own.A = own.B = own.C = own.coef_table = nullptr;
       own.status = own.counter = nullptr;
       pro.factors = nullptr;
       LaunchScope scope("head_prologue", s0, 1, timing);
       if ((e = oal::launch_head_prologue(own, p->q_heads, s0)) != cudaSuccess) return fail_cuda(e, "prologue kernel");
-      join_mark(side, 0, s0, st);
+      beside.mark();
     }
   } else if (tc) {
     // explicit coefficients: the factor table (rotations of a possibly indefinite matrix, 50 us) is needed by the
     // last kernel only and is computed beside the state kernels
     if (timing) side = side_streams(side_lock);
-    s0 = fork_to(side, 0, st);
+    s0 = beside.fork(side, 0, st);
     if (int rc = make_head_factors(p, dim_perm, group_start, src.A, src.B, src.C, factors, s0, timing)) return rc;
-    join_mark(side, 0, s0, st);
+    beside.mark();
     LaunchScope scope("coef_table", st, 1, timing);
     e = oal::build_coef_table(dim_perm, group_start, src.A, src.B, src.C, p->q_heads, p->groups, p->scale, coef_table, st);
     if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
@@ -576,7 +592,7 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
     if (e != cudaSuccess) return fail_cuda(e, "cross read kernel");
   }
   if (tc) {
-    join_wait(side, 0, s0, st);
+    beside.wait();
     LaunchScope scope("intra_forward", st, 1, timing);
     e = oal::intra_forward(q, k, v, factors, out, num, den, status, p->batch, p->q_heads, p->kv_heads, p->seq_len, nb, p->groups,
                            p->out_dtype, p->floor, (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) != 0, cr.first, sink, st);
@@ -648,7 +664,8 @@ int backward_core_fp32(const OalProblem* p, const BackwardArgs& x, const CoefSou
   // (all but a few SMs in a short call).
   std::unique_lock<std::mutex> side_lock;
   SideStreams* side = side_streams(side_lock);
-  cudaStream_t skv = want_kv ? fork_to(side, 0, st) : st;
+  SideWork kv;
+  cudaStream_t skv = want_kv ? kv.fork(side, 0, st) : st;
   if (mask & (OAL_GRAD_Q | OAL_GRAD_COEF)) {
     a.dq = (mask & OAL_GRAD_Q) ? x.dq : nullptr;
     a.coef_partial = (mask & OAL_GRAD_COEF) ? s.coef_pairs : nullptr;
@@ -662,11 +679,11 @@ int backward_core_fp32(const OalProblem* p, const BackwardArgs& x, const CoefSou
     a.dv = (mask & OAL_GRAD_V) ? x.dv : nullptr;
     { LaunchScope scope("pairs_backward_kv", skv, p->q_heads > p->kv_heads ? 2 : 1); e = oal::pairs_backward_kv(a, skv); }
     if (e != cudaSuccess) return fail_cuda(e, "backward key/value-side pair kernels");
-    join_mark(side, 0, skv, st);
+    kv.mark();
   }
   if (mask & OAL_GRAD_COEF)
     if (int rc = finish_coefs(p, src, sink, s.coef_pairs, nullptr, nullptr, st)) return rc;
-  if (want_kv) join_wait(side, 0, skv, st);
+  kv.wait();
   return OAL_OK;
 }
 
@@ -699,13 +716,14 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   std::unique_lock<std::mutex> side_lock;
   SideStreams* side = side_streams(side_lock);
   const bool cross = cr.n > 0;
-  cudaStream_t skv = want_kv ? fork_to(side, 0, st) : st;
-  cudaStream_t sc = want_c && cross ? fork_to(side, 1, st) : st;
+  SideWork kv, cross_coefs;
+  cudaStream_t skv = want_kv ? kv.fork(side, 0, st) : st;
+  cudaStream_t sc = want_c && cross ? cross_coefs.fork(side, 1, st) : st;
   if (want_c && cross) {
     { LaunchScope scope("dcoef_reduce", sc, 2);
       e = oal::dcoef_reduce(s.dcoef_partial, 2 * p->batch * cr.n, p->q_heads, p->groups, x.dim_perm, x.group_start, s.dcoef, s.slots, sc); }
     if (e != cudaSuccess) return fail_cuda(e, "coefficient gradient reduction kernels");
-    join_mark(side, 1, sc, st);
+    cross_coefs.mark();
   }
   if (want_kv && cross) {
     { LaunchScope scope("state_scan_reverse", skv);
@@ -744,13 +762,13 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
                                  s.dv_cross, cr.n * kChunk, s.dk_part, s.dv_part, x.status, p->batch, p->q_heads, p->kv_heads,
                                  p->seq_len, nb, p->groups, skv); }
     if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward key/value-side kernels");
-    join_mark(side, 0, skv, st);
+    kv.mark();
   }
   if (want_c) {
-    if (cross) join_wait(side, 1, sc, st);
+    cross_coefs.wait();
     if (int rc = finish_coefs(p, src, sink, s.coef_blocks, cross ? s.slots : nullptr, factors, st)) return rc;
   }
-  if (want_kv) join_wait(side, 0, skv, st);
+  kv.wait();
   return OAL_OK;
 }
 
