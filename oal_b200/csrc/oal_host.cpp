@@ -150,6 +150,12 @@ struct Prepared {
     if (!shape(q, Hq, D) || !shape(k, Hkv, D) || !shape(v, Hkv, Dv)) return false;
     if (f.scalar_type() != at::kFloat || f.device() != device || f.dim() < 1 || f.dim() > 2 || f.size(-1) != P) return false;
     if (f.dim() == 2 && f.size(0) != Hq) return false;
+    // forward-mode tangents: the operator has none, and the Python layer says so
+    const auto tangent = [](const Tensor& t) {
+      const auto* meta = torch::autograd::impl::get_autograd_meta(t);
+      return meta && meta->fw_grad(/*level=*/0, t).defined();
+    };
+    if (tangent(q) || tangent(k) || tangent(v) || tangent(f)) return false;
     const bool live = at::GradMode::is_enabled();
     return (live && q.requires_grad()) == grad[0] && (live && k.requires_grad()) == grad[1] &&
            (live && v.requires_grad()) == grad[2] && (live && f.requires_grad()) == grad[3];

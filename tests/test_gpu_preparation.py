@@ -58,3 +58,23 @@ def test_a_layer_is_copied_and_saved_after_its_first_call():
     file.seek(0)
     for other in (copy.deepcopy(layer), torch.load(file, weights_only=False)):
         assert torch.equal(other(x, rope), want)
+
+
+def test_transforms_that_the_operator_does_not_support_raise():
+    """Forward-mode tangents, vmap and functional gradients never come back as plain outputs."""
+    import torch.autograd.forward_ad as fw
+
+    make, (q, k, v, factor) = _prepared()
+    prepared = make()
+    with fw.dual_level():
+        dual = fw.make_dual(factor, torch.ones_like(factor))
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            oal_b200.run_prepared_grouped_hd_block_gemm(prepared, q, k, v, dual)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda x: oal_b200.run_prepared_grouped_hd_block_gemm(prepared, x, k, v, factor)[0])(q.expand(2, *q.shape))
+    trained = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, (torch.arange(64) % 4).to(torch.int32).cuda(),
+                                                     factor.clone().requires_grad_(), precision="bf16_tensorcore")
+    for call in (prepared, trained):      # refused as another gradient mode, and as a transform
+        with pytest.raises((RuntimeError, ValueError)):
+            torch.func.grad(lambda x: oal_b200.run_prepared_grouped_hd_block_gemm(call, q, k, v, x)[0].float().sum())(factor)
+    assert torch.isfinite(oal_b200.run_prepared_grouped_hd_block_gemm(prepared, q, k, v, factor)[0]).all()
