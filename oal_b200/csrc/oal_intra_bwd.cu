@@ -405,14 +405,20 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_q_kernel(const IntraB
 // ---------------------------------------------------------------------------
 // key / value side: one CTA per (chunk, KV head, batch row) and group of query heads; rows are keys
 // ---------------------------------------------------------------------------
-// tensor memory: U (two halves of 64; first dW^T of a head) | P^T (64), later W^T | Z (64) | dU (80) | two term slots (64)
-constexpr uint32_t BK_U = 0, BK_P = 128, BK_Z = 192, BK_V = 256, BK_TERM = 336;
+// tensor memory: U (two halves of 64; first dW^T of a head) | P^T (64), later W^T | their remainders (64) | Z (64) | dU (64) |
+// two term slots (64)
+constexpr uint32_t BK_U = 0, BK_P = 128, BK_PLO = 192, BK_Z = 256, BK_V = 320, BK_TERM = 384;
 static_assert(BK_TERM + 2 * TERM_COLS <= 512, "tensor-memory columns of the key/value-side kernel");
 constexpr int BK_HEAD_L = RMAX_ALL * HD * 4;
 constexpr int BK_HEAD_BYTES = X_BYTES + 2 * SLAB_S_BYTES + BK_HEAD_L;       // Q image, G hi, G lo, l: one head's operands
 constexpr int BK_SMEM = X_BYTES + XA_BYTES + 2 * BK_HEAD_BYTES;
 static_assert(BK_HEAD_BYTES % 16 == 0 && BK_SMEM <= 227 * 1024, "shared memory of the key/value-side kernel");
 
+// FINE: P^T with its remainders and W^T against both images of G, for heads of more than 8 groups.  Their weights were
+// formed and summed in fp32 (oal_pairs.cu) before these kernels took them over, and the bf16 values alone were up to 1.24
+// times as far from 64 bits in dv and 1.18 times in dk (14 / 2 heads, N = 347, 16 groups: 2.13e-3 -> 2.64e-3 and 2.14e-3 ->
+// 2.52e-3); up to 8 groups the bf16 values are nearer than the tiles that they replaced (dk 3.3e-3 -> 2.8e-3).
+template <bool FINE>
 __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const IntraBwdArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* Kimg = smem;
@@ -501,13 +507,16 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
                    2 * CT * 16, cols);
           mma_commit(&dw_full);
           const uint64_t dq = smem_desc(q_addr, 128, CP), dg = smem_desc(g_addr, 128, CT * 16);
+          const uint64_t dg_lo = smem_desc(g_addr + SLAB_S_BYTES, 128, CT * 16);
           const auto issue_z = [&](int t, int hf) {
             w.wait(&p_full[hf], t & 1, 0x35);
             if (hf == 0 && t > 0) w.wait(&z_free, (t - 1) & 1, 0x36);
             fence_after_sync();
             const int k0 = hf ? 4 : 0, k1 = hf ? 4 + nb2 / 16 : na / 16;
-            for (int ks = k0; ks < k1; ++ks)
-              mma_bf16_ts(tmem + BK_Z, tmem + BK_P + 8 * ks, desc_advance(dq, ks * 256), instr_desc_bf16(128, HD, 0, 1), ks > 0);
+            for (int part = 0; part < (FINE ? 2 : 1); ++part)
+              for (int ks = k0; ks < k1; ++ks)
+                mma_bf16_ts(tmem + BK_Z, tmem + (part ? BK_PLO : BK_P) + 8 * ks, desc_advance(dq, ks * 256),
+                            instr_desc_bf16(128, HD, 0, 1), part + ks > 0);
             mma_commit(&z_half[hf]);
           };
           for (int r = 0; r < rank; ++r, ++T) {
@@ -533,10 +542,11 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
           issue_z(T - 1, 1);
           w.wait(&w_full, i & 1, 0x3B);
           fence_after_sync();
-          for (int part = 0; part < 2; ++part)        // dU (+)= W^T G: the weights' bf16 values, then their remainders
+          // dU (+)= W^T G: the weights' bf16 values, then their remainders, then the values against G's remainders
+          for (int part = 0; part < (FINE ? 3 : 2); ++part)
             for (int ks = 0; ks < cols / 16; ++ks)
-              mma_bf16_ts(tmem + BK_V, tmem + (part ? BK_TERM : BK_P) + 8 * ks, desc_advance(dg, ks * 256),
-                          instr_desc_bf16(128, EP, 0, 1), i + part + ks > 0);
+              mma_bf16_ts(tmem + BK_V, tmem + (part == 1 ? BK_PLO : BK_P) + 8 * ks, desc_advance(part == 2 ? dg_lo : dg, ks * 256),
+                          instr_desc_bf16(128, HD, 0, 1), i + part + ks > 0);
           mma_commit(&v_full);
         }
       }
@@ -554,7 +564,10 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
     for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
       for (int x = 0; x < 2; ++x)
-        if (exists(hf, x) && !on(hf, x)) tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, 0u, 0u, 0u, 0u);
+        if (exists(hf, x) && !on(hf, x)) {
+          tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, 0u, 0u, 0u, 0u);
+          tmem_st4(tmem + BK_PLO + lane_off + col_of(hf, x) / 2, 0u, 0u, 0u, 0u);
+        }
     f32x2 dk[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) dk[j] = 0ull;
@@ -627,7 +640,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
           tmem_ld_wait();
           fence_before_sync();
           warp_arrive(&u_free[hf], lane);
-          uint32_t p[2][4];
+          uint32_t p[2][4], rest[2][4];
 #pragma unroll
           for (int x = 0; x < 2; ++x)
             if (on(hf, x)) {
@@ -637,6 +650,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
                 float t0, t1;
                 f2_unpack(f2_mul(dw[hf][x][j], u2), t0, t1);
                 p[x][j] = pack_bf16(t0, t1);
+                if (FINE) rest[x][j] = pack_bf16(t0 - bf16_lo(p[x][j]), t1 - bf16_hi(p[x][j]));
                 wt[hf][x][j] = f2_fma(rpos == rank ? u2 : f2_mul(u2, sgn), u2, wt[hf][x][j]);
               }
             }
@@ -646,7 +660,11 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
           }
 #pragma unroll
           for (int x = 0; x < 2; ++x)
-            if (on(hf, x)) tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, p[x][0], p[x][1], p[x][2], p[x][3]);
+            if (on(hf, x)) {
+              const uint32_t at = lane_off + col_of(hf, x) / 2;
+              tmem_st4(tmem + BK_P + at, p[x][0], p[x][1], p[x][2], p[x][3]);
+              if (FINE) tmem_st4(tmem + BK_PLO + at, rest[x][0], rest[x][1], rest[x][2], rest[x][3]);
+            }
           tmem_st_wait();
           fence_before_sync();
           // the whole Z of the previous term is complete: out of the way before the next one starts
@@ -658,30 +676,26 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
       w.wait(&z_half[1], (T + rank - 1) & 1, 0x45);
       fence_after_sync();
       drain(rank - 1);
-      // W^T in the place of P^T, whose last reader is complete, and its remainders over the first term slot (so are
-      // the slot's readers, and the next head builds no term before v_full)
+      // W^T and its remainders in the place of P^T and its, whose last readers are complete
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
         for (int x = 0; x < 2; ++x)
-          if (exists(hf, x)) {
-            const uint32_t at = lane_off + col_of(hf, x) / 2;
-            uint32_t rest[4] = {0u, 0u, 0u, 0u};
-            if (on(hf, x)) {
-              uint32_t o[4];
+          if (on(hf, x)) {
+            uint32_t o[4], rest[4];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float w_a, w_b;
-                f2_unpack(wt[hf][x][j], w_a, w_b);
-                const int i0 = col_of(hf, x) + 2 * j;
-                if (i0 < row) w_a = 0.f;
-                if (i0 + 1 < row) w_b = 0.f;
-                o[j] = pack_bf16(w_a, w_b);
-                rest[j] = pack_bf16(w_a - bf16_lo(o[j]), w_b - bf16_hi(o[j]));
-              }
-              tmem_st4(tmem + BK_P + at, o[0], o[1], o[2], o[3]);
+            for (int j = 0; j < 4; ++j) {
+              float w_a, w_b;
+              f2_unpack(wt[hf][x][j], w_a, w_b);
+              const int i0 = col_of(hf, x) + 2 * j;
+              if (i0 < row) w_a = 0.f;
+              if (i0 + 1 < row) w_b = 0.f;
+              o[j] = pack_bf16(w_a, w_b);
+              rest[j] = pack_bf16(w_a - bf16_lo(o[j]), w_b - bf16_hi(o[j]));
             }
-            tmem_st4(tmem + BK_TERM + at, rest[0], rest[1], rest[2], rest[3]);
+            const uint32_t at = lane_off + col_of(hf, x) / 2;
+            tmem_st4(tmem + BK_P + at, o[0], o[1], o[2], o[3]);
+            tmem_st4(tmem + BK_PLO + at, rest[0], rest[1], rest[2], rest[3]);
           }
       tmem_st_wait();
       fence_before_sync();
@@ -804,7 +818,8 @@ cudaError_t intra_backward_kv(const void* q, const void* k, const void* v, const
                               void* dk, void* dv, const float* dk_cross, const float* dv_cross, int cross_end, float* dk_part,
                               float* dv_part, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups,
                               cudaStream_t st) {
-  cudaError_t e = allow_smem<intra_bwd_kv_kernel>(BK_SMEM);
+  const bool fine = groups > 8;
+  cudaError_t e = fine ? allow_smem<intra_bwd_kv_kernel<true>>(BK_SMEM) : allow_smem<intra_bwd_kv_kernel<false>>(BK_SMEM);
   if (e != cudaSuccess) return e;
   IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB, groups);
   a.parts = intra_kv_parts(B, Hq, Hkv, NB);
@@ -817,7 +832,9 @@ cudaError_t intra_backward_kv(const void* q, const void* k, const void* v, const
     a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
     a.dk_cross = dk_cross; a.dv_cross = dv_cross;
   }
-  intra_bwd_kv_kernel<<<dim3(NB, B * Hkv, a.parts), BW_THREADS, BK_SMEM, st>>>(a);
+  const dim3 grid(NB, B * Hkv, a.parts);
+  if (fine) intra_bwd_kv_kernel<true><<<grid, BW_THREADS, BK_SMEM, st>>>(a);
+  else intra_bwd_kv_kernel<false><<<grid, BW_THREADS, BK_SMEM, st>>>(a);
   if (a.parts == 1 || (e = cudaGetLastError()) != cudaSuccess) return cudaGetLastError();
   KvReduceArgs r{{dk_part, dv_part}, {dk_cross, dv_cross}, {static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv)},
                  B, Hkv, a.parts, N, cross_end};

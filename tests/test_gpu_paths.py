@@ -70,3 +70,13 @@ def test_numerators_of_the_first_chunk_value_by_value(n, hq, hkv, g):
     a = lower[:, 0].norm(dim=-1)[:, None, None] + torch.einsum("hid,hd,hjd->hij", q.abs(), per_dim.norm(dim=-1), k.abs())
     bound = (2.0 ** -16 * w + 2.0 ** -15 * w.sqrt() * a).tril() @ v.abs()
     assert ((num[0] - w @ v).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("n,hq,hkv,g", [(128, 14, 2, 9), (100, 2, 2, 12), (128, 4, 1, 16)])
+def test_key_value_gradients_above_eight_groups_are_as_exact_as_their_dtype(n, hq, hkv, g):
+    """One chunk, every product as value + remainder (2^-16): what is left is the rounding of the results to bf16, at most
+    2^-9 of each value and so of the 2-norm."""
+    case = _case(2, n, hq, hkv, g)
+    res, ref = run_operator(case, precision="bf16_tensorcore", io_dtype=torch.bfloat16), oracle_dense(case)
+    for key in ("dq", "dk", "dv"):
+        assert (res[key].double() - ref[key]).norm() <= 1.01 * 2.0 ** -9 * ref[key].norm(), key
