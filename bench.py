@@ -584,14 +584,15 @@ def run_gpu_arm(args) -> None:
         }
         # MMA FLOPs the intra-chunk kernels really execute per launch, per 128-token chunk: G + 1 terms, each a chain
         # over K = 64 of value + remainder against the other side's rows.  Query-side tiles hold four 32-row blocks
-        # and see only the keys of the last one; the key/value side walks all 128 queries of a head.
+        # and see only the keys of the last one; the key/value side walks all 128 queries of a head.  The weights meet
+        # the values (80 columns) and G (64) as value + remainder.
         terms, rep, chunks = w["g"] + 1, w["hq"] // w["hkv"], w["batch"] * w["hkv"] * (w["n"] // KERNEL_CHUNK)
         seen = chunks * sum(32 * (4 - 4 * x // rep) for x in range(rep))       # key columns of all query-side tiles
         rows = chunks * rep * 128                                             # query columns of the key/value side
         executed_flops = {
-            "intra_forward": seen * 2 * 128 * (terms * 128 + 80),
+            "intra_forward": seen * 2 * 128 * (terms * 128 + 2 * 80),
             "intra_backward_q": seen * 2 * 128 * (2 * 80 + terms * (128 + 2 * 64)),
-            "intra_backward_kv": rows * 2 * 128 * (2 * 80 + terms * (128 + 64) + 80),
+            "intra_backward_kv": rows * 2 * 128 * (2 * 80 + terms * (128 + 64) + 2 * 64),
         }
         kernels = {name: dict(launches=cnt, ms_per_launch=ms / max(cnt, 1), share=None)
                    for name, (cnt, ms) in report.items()}

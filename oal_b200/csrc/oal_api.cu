@@ -323,6 +323,7 @@ int check_problem(const OalProblem* p) {
   if (!(p->floor > 0.f)) return fail(OAL_ERR_ARGUMENT, "floor must be positive");
   if (p->flags & ~(OAL_FLAG_OUT_TOKEN_MAJOR | OAL_FLAG_ZERO_STATE_IN)) return fail(OAL_ERR_ARGUMENT, "unknown bits in flags");
   if ((p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) && (p->precision != OAL_PRECISION_BF16_TENSORCORE || p->groups > 8))
+    // (the limit of 8 groups is the flag's contract; the kernels have none)
     return fail(OAL_ERR_ARGUMENT, "token-major out needs bf16_tensorcore and at most 8 groups per head");
   return OAL_OK;
 }

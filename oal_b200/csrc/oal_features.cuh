@@ -290,27 +290,6 @@ __device__ __forceinline__ void unpack_row(const uint32_t (&xp)[HD / 2], f32x2 (
   for (int w = 0; w < HD / 2; ++w) xq[w] = f2_pack(bf16_lo(xp[w]), bf16_hi(xp[w]));
 }
 
-// Row `i` (or zeros when i >= N) of a bf16 [.., N, 64] tensor into registers, times mul.
-__device__ __forceinline__ void load_row_bf16(float (&x)[HD], const __nv_bfloat16* base, int i, int N, float mul) {
-  if (i < N) {
-    const uint4* p = reinterpret_cast<const uint4*>(base + (size_t)i * HD);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const uint4 t = p[c];
-      const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&w[j]);
-        x[8 * c + 2 * j] = mul * __low2float(h);
-        x[8 * c + 2 * j + 1] = mul * __high2float(h);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int d = 0; d < HD; ++d) x[d] = 0.f;
-  }
-}
-
 // Bounded mbarrier waits for one CTA: the first wait that expires raises a shared flag and every
 // later wait returns at once, so a kernel always terminates; the flag ends up in the status word.
 struct Waiter {

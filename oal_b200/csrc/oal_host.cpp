@@ -2,7 +2,8 @@
 //
 // At one or two (batch row, KV head) units the kernels of a step take less time than Python needs to marshal its
 // calls, so everything a repeated call does between the caller's tensors and the launches is here: one pass over
-// the arguments, one allocation each for the outputs that live on and for the workspace, one C call.  The argument
+// the arguments, one allocation per result, saved buffer and workspace (six forward, up to five backward, all from the
+// caching allocator), one C call.  The argument
 // checks of this file only decide whether the call is the prepared one; when they say no, the Python layer goes
 // through the full validation and raises what it always raised.
 //

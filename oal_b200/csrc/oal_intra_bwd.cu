@@ -15,7 +15,7 @@
 // they were formed from fp32 products.
 //
 // Key / value side (rows are keys, columns are the queries of one head): per head and term
-//   P_r^T as above (bf16 value),  Z_r = P_r^T Q,  dk += sgn_r l_r * Z_r,  w += sgn_r u_r^2 in registers,
+//   P_r^T as above (bf16 value; with its remainder above 8 groups),  Z_r = P_r^T Q,  dk += sgn_r l_r * Z_r,  w += sgn_r u_r^2 in registers,
 // and after the last term dU += W^T G (W as value + remainder, as in the forward: a row's weights and its denominator
 // then agree to 16 bits).  A CTA walks several query heads of its KV head; dk stays in registers, dU
 // in tensor memory, and the next head's operands arrive while the current one is worked on.

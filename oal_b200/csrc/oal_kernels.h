@@ -7,7 +7,6 @@
 
 namespace oal {
 
-// Arguments of the token-pair kernels (oal_pairs.cu).
 struct PrologueArgs;      // oal_prologue.cuh
 
 // Delivery of a call's status word to pinned host memory by the last block of its last kernel: `counter` (device, zero
@@ -18,6 +17,7 @@ struct StatusSink {
 };
 constexpr int32_t STATUS_DELIVERED = (int32_t)0x80000000;
 
+// Arguments of the token-pair kernels (oal_pairs.cu).
 struct PairArgs {
   int B, Hq, Hkv, N, G;
   int io_dt, out_dt;
@@ -35,7 +35,7 @@ struct PairArgs {
   void *dq, *dk, *dv;
   float* coef_partial;   // [B][Hq][tiles][split][NCOEF] or null
   float *dk_part, *dv_part;      // [B,Hq,N,64] fp32, where a KV head has several query heads
-  // set by the launch: 64-token tiles, CTAs that share a tile, which of q, k, v (bits) allow loads of four elements
+  // set by the launch: 64-token tiles, CTAs that share a tile, which of q, k, v, num (bits) allow accesses of four elements
   int tiles, split, vec;
 };
 

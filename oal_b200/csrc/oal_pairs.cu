@@ -810,12 +810,14 @@ cudaError_t pairs_backward_kv(const PairArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 int pairs_tiles(int n) { return (n + TP - 1) / TP; }
-// CTAs that share an owner tile: doubled while the chip's 148 SMs would not get two blocks each, up to the number of
-// tiles there are to share and the portable cluster size.
+// CTAs that share an owner tile: doubled while the chip's SMs would not get two blocks each, up to the number of
+// tiles there are to share and the portable cluster size.  The number of SMs is a constant here: workspace sizes follow
+// the split, and they are asked for without a device too.
+constexpr int B200_SMS = 148;
 int pairs_split(int B, int Hq, int N) {
   const long long tiles = pairs_tiles(N), blocks = tiles * Hq * B;
   int s = 1;
-  while (s < 8 && 2 * s <= tiles && blocks * s < 2 * 148) s *= 2;
+  while (s < 8 && 2 * s <= tiles && blocks * s < 2 * B200_SMS) s *= 2;
   return s;
 }
 

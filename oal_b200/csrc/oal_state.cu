@@ -7,7 +7,8 @@
 //   state_scan   : carry[u,c] = state_in + sum_{c'<c} dS[u,c'] (fp32), stored as the bf16
 //                  operand image the MMAs read
 //   cross_read   : Y[i,:] = phi_q(i) . carry[u,c(i)]           (tokens are the MMA M dimension)
-// Feature tiles are generated in shared memory (oal_features.cuh) and never touch HBM.
+// Feature tiles are generated on chip (oal_features.cuh), in shared memory or, for the cross read, straight in tensor
+// memory, and never touch HBM.
 // The fp32 accumulators live in tensor memory; state images are streamed with 1-D bulk
 // async copies.  Every mbarrier wait is bounded (oal_umma.cuh).
 #include "oal_features.cuh"
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_b
 // ---------------------------------------------------------------------------
 struct CrossReadArgs {
   const __nv_bfloat16* x;        // q [B,Hq,N,64] or k [B,Hkv,N,64]
-  const __nv_bfloat16* image;    // [units, NB, 17, 10, 128, 8]
+  const __nv_bfloat16* image;    // [units, NB, 19, 10, 128, 8]
   const float* coef_table;       // [Hq, F_ROWS] (QUERY)
   float* out64;                  // [B,H,N,64]
   float* out1;                   // [B,H,N] (QUERY: denominator)

@@ -55,8 +55,7 @@ _RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
-    """The device's current stream as a raw handle (the accessor without the Stream object when torch has it:
-    this runs four times per training step on the host's critical path)."""
+    """The device's current stream as a raw handle (the accessor without the Stream object when torch has it)."""
     if _RAW_STREAM is not None and device.index is not None:
         return ctypes.c_void_p(_RAW_STREAM(device.index))
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
@@ -103,17 +102,16 @@ def raise_on_status(status: torch.Tensor) -> None:
     _raise_for_bits(int(status.item()))
 
 
-# Deferred status words.  The reference synchronises after every forward because "a device-side
-# assertion can poison a CUDA context ... until a safe asynchronous status mechanism is available"
-# (hd_block_gemm_runtime.py:395-398).  The status word is that mechanism: when autograd will run a
-# backward anyway, the forward only queues an asynchronous copy of its status word to pinned host
-# memory (``oal_status_defer``: a ring of pinned words and a copy stream inside the library) and keeps the
-# ticket.  The backward of the same call looks at exactly that ticket before it launches anything --
-# without waiting: the host normally runs ahead of the GPU, and a wait here would serialise host and
-# device in every step (measured: it costs the whole forward time per step and stalls input pipelines).
-# A ticket that is not finished yet stays on a per-device list that every later entry into the library
-# drains without blocking; ``check_pending_status(block=True)`` drains it completely and is the call to
-# make before an optimizer step consumes the gradients.  Every error names the call it belongs to.
+# Status words of calls whose result is looked at later.  The reference synchronises after every forward because "a
+# device-side assertion can poison a CUDA context ... until a safe asynchronous status mechanism is available"
+# (hd_block_gemm_runtime.py:395-398).  The status word is that mechanism.  A prepared call on plain tensors has its
+# last kernel write the word to pinned host memory (csrc/oal_host.cpp keeps the tickets); the calls of this file, with
+# explicit coefficients, queue an asynchronous copy instead (``oal_status_defer``) and keep the ticket here.  Later
+# entries into the library look at the tickets without waiting: the host normally runs ahead of the GPU, and a wait here
+# would serialise host and device in every step (measured: it costs the whole forward time per step and stalls input
+# pipelines).  The backward of a call looks at its own forward's ticket first.
+# ``check_pending_status(block=True)`` drains both lists and is the call to make before an optimizer step consumes the
+# gradients.  Every error names the call it belongs to.
 _PENDING: dict = {}
 _PENDING_LOCK = threading.Lock()
 _PENDING_LIMIT = 256          # a ticket stays valid for 1023 later ones on its device: drain well before that
