@@ -4,38 +4,38 @@
 // phi_q = [A, B_{g(d)} q_d, m C_{g(r)g(c)} q_r q_c] as [tokens, 2145] matrices in HBM
 // (oal_attention/hd_block_gemm_feature_forward.py:225-253, :373-385; pair order
 // oal_attention/hd_block_gemm_cache.py:105-121).  Here a feature tile only ever exists in
-// shared memory, as 16-byte chunks of 8 features in bf16.  The feature order is internal (the
-// running state is never exposed) and chosen so that a chunk multiplies one row element with eight
-// adjacent column elements, which the packed bf16 / fp32 multiplies do two at a time:
-//   pair chunk (cb, r), r = 8 cb .. 63:  features x[r] * x[8 cb + j], j = 0..7, zero where
-//       8 cb + j > r.  Chunks are ordered by cb, then r: while cb stays the same the eight
-//       column values stay in registers and only x[r] changes.
-//       chunk index = 64 cb - 4 cb (cb - 1) + (r - 8 cb); 288 pair chunks
-//   chunks 288..295  linear features d = 8 (chunk - 288) + j
-//   chunk  296       [constant, 0 x 7]
-//   chunks 297..303  zero padding
-// 16 chunks (128 features) form a slab: 19 slabs, 2432 feature rows.
-// Each thread owns one token and keeps its row in registers; every index in the generated code is a
-// compile-time constant.  Pairs (x[8 cb + 2k], x[8 cb + 2k + 1]) are adjacent in the packed row, so a
-// chunk is one broadcast of x[r] and four packed multiplies.
+// shared memory or tensor memory, in bf16.  The feature order is internal (the running state is never exposed): 64
+// consecutive features are one 8 x 8 block of x x^T,
+//   features 64 hs + 16 (c / 2) + 2 r + c % 2:  x[8 rb + r] * x[8 cb + c],  r, c = 0 .. 7,  rb >= cb
+//   blocks hs = 0 .. 35 by cb, then rb; in a diagonal block the entries above the diagonal (c > r) have no meaning
+//   features 2304 + d: linear, x[d];   feature 2368: constant;   zeros up to 2432
+// Two blocks (128 features) form a slab: 19 slabs, 2432 feature rows.  What the order is for:
+//   * a block needs 16 of a token's 64 values, so a thread reads two 16-byte pieces of the token's row from shared memory;
+//   * pairs of features (2 r + 16 i, + 1) share r and take adjacent columns: one broadcast and one packed multiply;
+//   * in tensor memory an accumulator fragment (.16x256b: thread t of a warp holds, of 16 rows, rows t / 4 and t / 4 + 8,
+//     and of every 8 columns, columns 2 (t % 4) and + 1) gives a thread two rows r and all eight columns c of a block for
+//     each of four tokens, as bf16 operand (two features per column) and as fp32 accumulator: the coefficients that a thread
+//     reads serve four tokens, and sums over c need no exchange.
 #pragma once
-
-#include <utility>
 
 #include "oal_common.cuh"
 #include "oal_umma.cuh"
 
 namespace oal {
 
-constexpr int F_PAIR_CHUNKS = 288;
-constexpr int F_LIN_CHUNK0 = 288;
-constexpr int F_CONST_CHUNK = 296;
-constexpr int F_CHUNKS = 304;
+constexpr int F_BLOCK = 64;                    // features of a block of x x^T, or half slab
+constexpr int F_PAIR_BLOCKS = 36;
+constexpr int F_LINEAR = F_PAIR_BLOCKS * F_BLOCK, F_CONST = F_LINEAR + HD;
 constexpr int F_SLABS = 19;
 constexpr int F_ROWS = F_SLABS * 128;          // 2432
+constexpr int LAST_STEPS = (F_CONST - 128 * (F_SLABS - 1)) / 16 + 1;      // 16-feature steps of the last slab before its padding
 constexpr int CT = 128;                        // tokens per chunk of the scan
 constexpr int SLAB_A_BYTES = 128 * CT * 2;     // feature slab tile  [16 chunks][128 tokens][8] bf16
 constexpr int SLAB_S_BYTES = (EP / 8) * 128 * 16;   // state slab image [10][128 features][8 e] bf16
+// Columns of [v | 1 | 0] that can be other than zero, in whole blocks of 8.  The last block of an image or increment only
+// completes the extent that the MMA wants (a multiple of 16): it is never written, copied or read.
+constexpr int EU = (E1 + 7) / 8 * 8;
+constexpr int SLAB_U_BYTES = (EU / 8) * 128 * 16;
 
 // Per-chunk fp32 state increments (and state-gradient increments) are stored like the bf16 state
 // image, [slab][e / 8][128 rows][8 e], so that a warp whose lanes are consecutive feature rows writes
@@ -44,47 +44,39 @@ __host__ __device__ constexpr size_t state_inc_offset(int f, int e) {
   return ((size_t)((f >> 7) * (EP / 8) + (e >> 3)) * 128 + (f & 127)) * 8 + (e & 7);
 }
 
-// Position in the pair-chunk order.
-struct PairCursor {
-  int r, cb;
-  __host__ __device__ constexpr void seek(int q) {      // q < F_PAIR_CHUNKS
-    cb = 0;
-    int base = 0;
-    while (q >= base + HD - 8 * cb) {
-      base += HD - 8 * cb;
-      ++cb;
-    }
-    r = 8 * cb + (q - base);
-  }
-  // number of features of the chunk that exist (c <= r); 8 or more means all
-  __host__ __device__ constexpr int valid() const { return r - 8 * cb + 1; }
+// Row and column block of half slab hs < F_PAIR_BLOCKS.
+struct HalfBlock {
+  int rb, cb;
 };
-__host__ __device__ constexpr PairCursor pair_pos(int q) {
-  PairCursor pc{0, 0};
-  pc.seek(q);
-  return pc;
+__host__ __device__ constexpr HalfBlock half_pos(int hs) {
+  int cb = 0;
+  while (hs >= 8 - cb) {
+    hs -= 8 - cb;
+    ++cb;
+  }
+  return HalfBlock{cb + hs, cb};
 }
 
-// What feature row f is: kind 0 pair (r, c; `live` false for the zero entries above the diagonal),
+// What feature row f is: kind 0 pair (r, c; `live` false for the repeated entries above the diagonal),
 // 1 linear (r = dimension), 2 constant, 3 padding.
 struct FeatureId {
   int kind, r, c;
   bool live;
 };
 __host__ __device__ inline FeatureId feature_id(int f) {
-  const int q = f >> 3, j = f & 7;
   FeatureId id{3, 0, 0, false};
-  if (q < F_PAIR_CHUNKS) {
-    const PairCursor pc = pair_pos(q);
+  if (f < F_LINEAR) {
+    const HalfBlock blk = half_pos(f / F_BLOCK);
+    const int y = f % F_BLOCK;
     id.kind = 0;
-    id.r = pc.r;
-    id.c = 8 * pc.cb + j;
+    id.r = 8 * blk.rb + ((y >> 1) & 7);
+    id.c = 8 * blk.cb + 2 * (y >> 4) + (y & 1);
     id.live = id.c <= id.r;
-  } else if (q < F_CONST_CHUNK) {
+  } else if (f < F_CONST) {
     id.kind = 1;
-    id.r = 8 * (q - F_LIN_CHUNK0) + j;
+    id.r = f - F_LINEAR;
     id.live = true;
-  } else if (q == F_CONST_CHUNK && j == 0) {
+  } else if (f == F_CONST) {
     id.kind = 2;
     id.live = true;
   }
@@ -94,7 +86,7 @@ __host__ __device__ inline FeatureId feature_id(int f) {
 // Power of the query scale folded into the per-head coefficient table: the query-side kernels work
 // on the unscaled q, so pair coefficients carry scale^2 and linear ones scale.
 __host__ __device__ inline float feature_scale_factor(int f, float scale) {
-  return f < 8 * F_PAIR_CHUNKS ? scale * scale : (f < 8 * F_CONST_CHUNK ? scale : 1.f);
+  return f < F_LINEAR ? scale * scale : (f < F_CONST ? scale : 1.f);
 }
 
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
@@ -105,189 +97,158 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
-// ---- coefficient-free chunk from the packed bf16 row  xp[k] = (x[2k], x[2k+1]) -------------------
-// The product of two bf16 values rounded once to bf16 is what an fp32 multiply followed by a
-// conversion gives, so the packed multiply yields those bits at two features per instruction.
-template <int Q>
-__device__ __forceinline__ uint4 raw_chunk(const uint32_t (&xp)[HD / 2]) {
-  if constexpr (Q < F_PAIR_CHUNKS) {
-    constexpr PairCursor pc = pair_pos(Q);
-    constexpr int nv = pc.valid();
-    const uint32_t w = xp[pc.r / 2];
-    const uint32_t xr2 = __byte_perm(w, w, (pc.r & 1) ? 0x3232u : 0x1010u);
-    uint32_t o[4];
+// ---- rows in shared memory -----------------------------------------------------------------------
+// Chunk planes of an operand image that threads write: 128 rows of 16 bytes and 16 bytes of padding, so that eight
+// threads that copy one 128-byte row (coalesced) hit eight different bank groups.
+constexpr int CP = CT * 16 + 16;
+constexpr int X_BYTES = 8 * CP;
+
+// 16-byte asynchronous copy global -> shared (zero fill when `valid` is false); completion with
+// async_copies_wait().  All copies of a thread are in flight together, so an image costs one memory
+// latency instead of one per 16 bytes.
+__device__ __forceinline__ void async_copy16(void* dst_smem, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(dst_smem)), "l"(src),
+               "r"(valid ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void async_copies_wait() {
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+// `rows` rows of 64 bf16 from `src` (consecutive, the first `valid` exist) -> operand image [8][rows][8] at row `row0`,
+// plane pitch CP, by threads tid of nthreads (a multiple of 8).  A tile of rows is contiguous: a thread keeps its column
+// piece and advances both addresses by constants (with the row computed for every piece, the address arithmetic took
+// longer than the copies).
+__device__ __forceinline__ void load_rows(unsigned char* img, int row0, const __nv_bfloat16* src, int rows, int valid, int tid,
+                                          int nthreads) {
+  const int step = nthreads >> 3;
+  unsigned char* dst = img + (tid & 7) * CP + (row0 + (tid >> 3)) * 16;
+  const __nv_bfloat16* from = src + (size_t)tid * 8;
+  for (int r = tid >> 3; r < rows; r += step, dst += step * 16, from += (size_t)nthreads * 8)
+    async_copy16(dst, r < valid ? from : src, r < valid);
+}
+
+// ---- half slabs -------------------------------------------------------------------------------------
+// The code is the same for every half slab.  (The form this replaces, one specialised piece of code per 8 features and the
+// row in registers, was 60 to 100 KB of straight-line code and needed the whole row where a half slab uses a quarter of it.)
+// Entries above the diagonal are generated too: their coefficients are zero, so they reach no result.
+constexpr int HALF_LINEAR = F_PAIR_BLOCKS, HALF_CONST = F_PAIR_BLOCKS + 1;
+static_assert(HALF_CONST == 2 * F_SLABS - 1, "the constant starts the last half slab");
+constexpr uint64_t half_slab_rows(int word) {          // 4 bits per half slab, 16 half slabs per word
+  uint64_t w = 0;
+  for (int h = 16 * word; h < 16 * word + 16 && h < F_PAIR_BLOCKS; ++h) w |= (uint64_t)half_pos(h).rb << (4 * (h - 16 * word));
+  return w;
+}
+constexpr uint64_t half_slab_columns(int word) {
+  uint64_t w = 0;
+  for (int h = 16 * word; h < 16 * word + 16 && h < F_PAIR_BLOCKS; ++h) w |= (uint64_t)half_pos(h).cb << (4 * (h - 16 * word));
+  return w;
+}
+static __constant__ uint64_t kHalfRow[3] = {half_slab_rows(0), half_slab_rows(1), half_slab_rows(2)};
+static __constant__ uint64_t kHalfCol[3] = {half_slab_columns(0), half_slab_columns(1), half_slab_columns(2)};
+__device__ __forceinline__ HalfBlock half_block(int hs) {      // hs < F_PAIR_BLOCKS, warp-uniform
+  const int sh = 4 * (hs & 15);
+  return HalfBlock{(int)(kHalfRow[hs >> 4] >> sh) & 15, (int)(kHalfCol[hs >> 4] >> sh) & 15};
+}
+__device__ __forceinline__ uint32_t bf16_twice(uint32_t word, int high) { return __byte_perm(word, word, high ? 0x3232u : 0x1010u); }
+
+// Coefficient-free features of half slab hs of one token, eight at a time: emit(j, 16 bytes), j = 0 .. 7, from the pieces of
+// the token's row that hold the block's rows and columns (`r4`, `c4`) or, for the linear features, piece(j).  The product of
+// two bf16 values rounded once to bf16 is what an fp32 multiply followed by a conversion gives, so the packed multiply
+// yields those bits at two features per instruction.
+template <class Piece, class Emit>
+__device__ __forceinline__ void raw_half_slab(int hs, const uint4 r4, const uint4 c4, Piece piece, Emit emit) {
+  if (hs < F_PAIR_BLOCKS) {
+    const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w};
+    uint32_t r[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t mask = (2 * k < nv ? 0x0000FFFFu : 0u) | (2 * k + 1 < nv ? 0xFFFF0000u : 0u);
-      o[k] = mask == 0u ? 0u : (mul_bf16x2(xr2, xp[4 * pc.cb + k]) & mask);
+    for (int j = 0; j < 8; ++j) r[j] = bf16_twice(rw[j / 2], j & 1);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t* rr = r + 4 * (j & 1);
+      emit(j, make_uint4(mul_bf16x2(rr[0], c[j / 2]), mul_bf16x2(rr[1], c[j / 2]), mul_bf16x2(rr[2], c[j / 2]), mul_bf16x2(rr[3], c[j / 2])));
     }
-    return make_uint4(o[0], o[1], o[2], o[3]);
-  } else if constexpr (Q < F_CONST_CHUNK) {
-    constexpr int k = 4 * (Q - F_LIN_CHUNK0);
-    return make_uint4(xp[k], xp[k + 1], xp[k + 2], xp[k + 3]);
-  } else if constexpr (Q == F_CONST_CHUNK) {
-    return make_uint4(0x00003F80u, 0u, 0u, 0u);   // bf16(1.0) in element 0
+  } else if (hs == HALF_LINEAR) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) emit(j, piece(j));
   } else {
-    return make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) emit(j, make_uint4(j == 0 ? 0x00003F80u : 0u, 0u, 0u, 0u));   // bf16(1.0) first
   }
 }
 
-// ---- chunk times the per-head coefficient table (query side of the forward) -----------------------
-//   xq   : fp32 row as packed pairs, xq[k] = (x[2k], x[2k+1]), unscaled
-//   coef : table of the head in feature order, query scale folded in, zero above the diagonal and in
-//          the padding; every lane reads the same address, so global memory through L1 is fine
-__device__ __forceinline__ uint4 pack_pairs_bf16(const f32x2 (&f)[4]) {
-  uint32_t o[4];
+// Features of half slab hs for the 32 tokens of a warp as the MMA's A operand in tensor memory (32 columns, a feature pair
+// each).  A lane works on rows r = 2 (lane % 4) and + 1 of the block for the tokens lane / 4 + 8 t, t = 0 .. 3.  `xlane`
+// points at token lane / 4 of the warp in plane 0 of the row image, `slot` at the half slab's first column at the warp's
+// lanes.  COEF: times the per-head coefficient table (feature order, query scale folded in, zero above the diagonal and in
+// the padding), in fp32 and rounded once.
+template <bool COEF>
+__device__ __forceinline__ void store_half_slab(int hs, const unsigned char* xlane, const float* coef, uint32_t slot, int lane) {
+  const int m = lane & 3;
+  const float* cf = coef + F_BLOCK * hs + 4 * m;
+  uint32_t o[2][16];                       // [tokens 0, 8 | 16, 24][column pair i: (token, column 2 m), (token, + 1), (token + 8, ..) ..]
+  f32x2 ca[4], cb[4];
+  const auto load_coefs = [&]() {
+    if constexpr (COEF) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
+      for (int i = 0; i < 4; ++i) {
+        const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(cf + 16 * i);
+        ca[i] = c.x;
+        cb[i] = c.y;
+      }
+    }
+  };
+  const auto pack = [](f32x2 f) {
     float lo, hi;
-    f2_unpack(f[k], lo, hi);
-    o[k] = umma::pack_bf16(lo, hi);
-  }
-  return make_uint4(o[0], o[1], o[2], o[3]);
-}
-
-template <int Q>
-__device__ __forceinline__ uint4 coef_chunk(const f32x2 (&xq)[HD / 2], const float* coef) {
-  if constexpr (Q <= F_CONST_CHUNK) {
-    const ulonglong2 ca = *reinterpret_cast<const ulonglong2*>(coef + 8 * Q);
-    const ulonglong2 cb2 = *reinterpret_cast<const ulonglong2*>(coef + 8 * Q + 4);
-    const f32x2 cf[4] = {ca.x, ca.y, cb2.x, cb2.y};
-    f32x2 f[4];
-    if constexpr (Q < F_PAIR_CHUNKS) {
-      constexpr PairCursor pc = pair_pos(Q);
-      float lo, hi;
-      f2_unpack(xq[pc.r / 2], lo, hi);
-      const f32x2 xr2 = f2_bcast((pc.r & 1) ? hi : lo);
+    f2_unpack(f, lo, hi);
+    return umma::pack_bf16(lo, hi);
+  };
+  if (hs < F_PAIR_BLOCKS) {
+    const HalfBlock blk = half_block(hs);
+    load_coefs();
 #pragma unroll
-      for (int k = 0; k < 4; ++k) f[k] = f2_mul(f2_mul(xr2, xq[4 * pc.cb + k]), cf[k]);
-    } else if constexpr (Q < F_CONST_CHUNK) {
+    for (int t = 0; t < 4; ++t) {
+      const unsigned char* x = xlane + 128 * t;
+      uint32_t* out = &o[t >> 1][2 * (t & 1)];
+      const uint32_t r = *reinterpret_cast<const uint32_t*>(x + blk.rb * CP + 4 * m);
+      const uint4 c4 = *reinterpret_cast<const uint4*>(x + blk.cb * CP);
+      const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+      if constexpr (COEF) {
+        const f32x2 xa = f2_bcast(bf16_lo(r)), xb = f2_bcast(bf16_hi(r));
 #pragma unroll
-      for (int k = 0; k < 4; ++k) f[k] = f2_mul(xq[4 * (Q - F_LIN_CHUNK0) + k], cf[k]);
-    } else {
-      f[0] = cf[0];          // (A, 0): the table is zero in the padding
-      f[1] = f[2] = f[3] = 0ull;
+        for (int i = 0; i < 4; ++i) {
+          const f32x2 xc = f2_pack(bf16_lo(c[i]), bf16_hi(c[i]));
+          out[4 * i] = pack(f2_mul(f2_mul(xa, xc), ca[i]));
+          out[4 * i + 1] = pack(f2_mul(f2_mul(xb, xc), cb[i]));
+        }
+      } else {
+        const uint32_t xa = bf16_twice(r, 0), xb = bf16_twice(r, 1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          out[4 * i] = mul_bf16x2(xa, c[i]);
+          out[4 * i + 1] = mul_bf16x2(xb, c[i]);
+        }
+      }
     }
-    return pack_pairs_bf16(f);
-  } else {
-    return make_uint4(0u, 0u, 0u, 0u);
-  }
-}
-
-// Threads per CTA of the kernels whose threads split a slab as (token, half of the 16 chunks).
-constexpr int GEN_THREADS = 256;
-
-// Chunks [J0, J0 + NJ) of slab S of one token into the slab tile ([16 chunks][128 tokens] x 16 bytes);
-// `tile` points at the token's column.
-template <int S, int J0, int... J>
-__device__ __forceinline__ void raw_chunks_impl(const uint32_t (&xp)[HD / 2], uint4* tile,
-                                                std::integer_sequence<int, J...>) {
-  ((tile[(J0 + J) * CT] = raw_chunk<S * 16 + J0 + J>(xp)), ...);
-}
-// Four chunks of slab S of one token, from chunk J0, as columns of the MMA's A operand in tensor memory (a feature pair
-// per column; `slot`: the slab's first column at this warp's lanes).
-template <int S, int J0>
-__device__ __forceinline__ void coef_chunks_to_tmem(uint32_t slot, const f32x2 (&xq)[HD / 2], const float* coef) {
-  const uint4 c0 = coef_chunk<S * 16 + J0>(xq, coef), c1 = coef_chunk<S * 16 + J0 + 1>(xq, coef);
-  const uint4 c2 = coef_chunk<S * 16 + J0 + 2>(xq, coef), c3 = coef_chunk<S * 16 + J0 + 3>(xq, coef);
-  const uint32_t w[16] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w, c2.x, c2.y, c2.z, c2.w, c3.x, c3.y, c3.z, c3.w};
-  umma::tmem_st16(slot + 4 * J0, w);
-}
-template <int S, int J0>
-__device__ __forceinline__ void raw_chunks_to_tmem(uint32_t slot, const uint32_t (&xp)[HD / 2]) {
-  const uint4 c0 = raw_chunk<S * 16 + J0>(xp), c1 = raw_chunk<S * 16 + J0 + 1>(xp);
-  const uint4 c2 = raw_chunk<S * 16 + J0 + 2>(xp), c3 = raw_chunk<S * 16 + J0 + 3>(xp);
-  const uint32_t w[16] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w, c2.x, c2.y, c2.z, c2.w, c3.x, c3.y, c3.z, c3.w};
-  umma::tmem_st16(slot + 4 * J0, w);
-}
-
-#define OAL_SLAB_SWITCH(s, CASE)                                                                      \
-  switch (s) {                                                                                        \
-    CASE(0) CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10) CASE(11) \
-    CASE(12) CASE(13) CASE(14) CASE(15) CASE(16) CASE(17) CASE(18)                                    \
-    default: break;                                                                                   \
-  }
-static_assert(F_SLABS == 19, "OAL_SLAB_SWITCH enumerates the slabs");
-
-// All 16 chunks of slab s (s is a run-time value; the bodies are static).
-__device__ __forceinline__ void write_slab_raw(int s, const uint32_t (&xp)[HD / 2], uint4* tile) {
-#define OAL_CASE(S) case S: raw_chunks_impl<S, 0>(xp, tile, std::make_integer_sequence<int, 16>{}); break;
-  OAL_SLAB_SWITCH(s, OAL_CASE)
-#undef OAL_CASE
-}
-// Half of the chunks of slab s: half 0 = chunks 0..7, half 1 = chunks 8..15.
-template <int J0>
-__device__ __forceinline__ void write_half_slab_raw_impl(int s, const uint32_t (&xp)[HD / 2], uint4* tile) {
-#define OAL_CASE(S) case S: raw_chunks_impl<S, J0>(xp, tile, std::make_integer_sequence<int, 8>{}); break;
-  OAL_SLAB_SWITCH(s, OAL_CASE)
-#undef OAL_CASE
-}
-__device__ __forceinline__ void write_half_slab_raw(int s, int half, const uint32_t (&xp)[HD / 2], uint4* tile) {
-  if (half == 0) write_half_slab_raw_impl<0>(s, xp, tile);
-  else write_half_slab_raw_impl<8>(s, xp, tile);
-}
-// The same half as columns of the A operand in tensor memory; `half` is the same for the lanes of a warp.
-__device__ __forceinline__ void store_half_slab_raw(int s, int half, const uint32_t (&xp)[HD / 2], uint32_t slot) {
-#define OAL_CASE(S)                        \
-  case S:                                  \
-    if (half == 0) {                       \
-      raw_chunks_to_tmem<S, 0>(slot, xp);  \
-      raw_chunks_to_tmem<S, 4>(slot, xp);  \
-    } else {                               \
-      raw_chunks_to_tmem<S, 8>(slot, xp);  \
-      raw_chunks_to_tmem<S, 12>(slot, xp); \
-    }                                      \
-    break;
-  OAL_SLAB_SWITCH(s, OAL_CASE)
-#undef OAL_CASE
-}
-__device__ __forceinline__ void store_half_slab_coef(int s, int half, const f32x2 (&xq)[HD / 2], const float* coef, uint32_t slot) {
-#define OAL_CASE(S)                               \
-  case S:                                         \
-    if (half == 0) {                              \
-      coef_chunks_to_tmem<S, 0>(slot, xq, coef);  \
-      coef_chunks_to_tmem<S, 4>(slot, xq, coef);  \
-    } else {                                      \
-      coef_chunks_to_tmem<S, 8>(slot, xq, coef);  \
-      coef_chunks_to_tmem<S, 12>(slot, xq, coef); \
-    }                                             \
-    break;
-  OAL_SLAB_SWITCH(s, OAL_CASE)
-#undef OAL_CASE
-}
-
-// The row stays the same while a kernel walks the slabs, and every feature is a pure function of it:
-// without this barrier the compiler hoists the features of all slabs out of the slab loop and spills
-// them.  Costs no instruction.
-__device__ __forceinline__ void keep_in_loop(uint32_t (&xp)[HD / 2]) {
+  } else if (hs == HALF_LINEAR) {
+    load_coefs();
 #pragma unroll
-  for (int w = 0; w < HD / 2; ++w) asm volatile("" : "+r"(xp[w]));
-}
-__device__ __forceinline__ void keep_in_loop(f32x2 (&xq)[HD / 2]) {
+    for (int t = 0; t < 4; ++t) {
+      uint32_t* out = &o[t >> 1][2 * (t & 1)];
 #pragma unroll
-  for (int w = 0; w < HD / 2; ++w) asm volatile("" : "+l"(xq[w]));
-}
-
-// Row `i` (or zeros when i >= N) of a bf16 [.., N, 64] tensor as packed words / as fp32 pairs.
-__device__ __forceinline__ void load_row_packed(uint32_t (&xp)[HD / 2], const __nv_bfloat16* base, int i, int N) {
-  if (i < N) {
-    const uint4* p = reinterpret_cast<const uint4*>(base + (size_t)i * HD);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const uint4 t = p[c];
-      xp[4 * c] = t.x;
-      xp[4 * c + 1] = t.y;
-      xp[4 * c + 2] = t.z;
-      xp[4 * c + 3] = t.w;
+      for (int i = 0; i < 4; ++i) {
+        const uint2 d = *reinterpret_cast<const uint2*>(xlane + 128 * t + (2 * i + (m >> 1)) * CP + 8 * (m & 1));
+        out[4 * i] = COEF ? pack(f2_mul(f2_pack(bf16_lo(d.x), bf16_hi(d.x)), ca[i])) : d.x;
+        out[4 * i + 1] = COEF ? pack(f2_mul(f2_pack(bf16_lo(d.y), bf16_hi(d.y)), cb[i])) : d.y;
+      }
     }
   } else {
+    const uint32_t first = COEF ? umma::pack_bf16(cf[0], 0.f) : 0x00003F80u;
 #pragma unroll
-    for (int w = 0; w < HD / 2; ++w) xp[w] = 0u;
+    for (int x = 0; x < 16; ++x) o[0][x] = o[1][x] = (m == 0 && (x == 0 || x == 2)) ? first : 0u;
   }
-}
-__device__ __forceinline__ void unpack_row(const uint32_t (&xp)[HD / 2], f32x2 (&xq)[HD / 2]) {
-#pragma unroll
-  for (int w = 0; w < HD / 2; ++w) xq[w] = f2_pack(bf16_lo(xp[w]), bf16_hi(xp[w]));
+  umma::tmem_st_rows16(slot, o[0]);
+  umma::tmem_st_rows16(slot + (16u << 16), o[1]);
 }
 
 // Bounded mbarrier waits for one CTA: the first wait that expires raises a shared flag and every
@@ -306,6 +267,13 @@ struct Waiter {
   }
 };
 
+
+// One arrival per warp on an mbarrier after every lane has finished what precedes (shared-memory
+// stores made visible to the async proxy, or tensor-memory accesses).
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) umma::mbar_arrive(bar);
+}
 
 // 16-byte image chunk (8 consecutive e of one token) of U = [v | 1 | 0]
 __device__ __forceinline__ uint4 u_image_chunk(const __nv_bfloat16* vrow, int ec, bool valid) {

@@ -27,11 +27,7 @@ namespace oal {
 constexpr int RMAX_ALL = OAL_MAX_GROUPS + 1;         // 17: extent of the per-head factor table
 constexpr int NU_ALL = RMAX_ALL * (RMAX_ALL + 1) / 2;
 constexpr int NQ_ALL = NU_ALL + RMAX_ALL + 1;        // coefficient partial sums of a row block: D upper triangle, n, s
-// Chunk planes of an operand image that threads write: 128 rows of 16 bytes and 16 bytes of padding, so that eight
-// threads that copy one 128-byte row (coalesced) hit eight different bank groups.
-constexpr int CP = CT * 16 + 16;
 constexpr int XA_BYTES = 10 * CP;                    // [v | 1 | 0]
-constexpr int X_BYTES = 8 * CP;
 
 // What a kernel keeps of a head's table besides l.
 struct HeadScalars {
@@ -49,27 +45,6 @@ struct alignas(16) HeadFactor {
   float t[RMAX_ALL][RMAX_ALL];       // t[a][r] = V[a][r] / lambda_r  (v = t u)
 };
 
-// 16-byte asynchronous copy global -> shared (zero fill when `valid` is false); completion with
-// async_copies_wait().  All copies of a thread are in flight together, so an image costs one memory
-// latency instead of one per 16 bytes.
-__device__ __forceinline__ void async_copy16(void* dst_smem, const void* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(dst_smem)), "l"(src),
-               "r"(valid ? 16 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void async_copies_wait() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
-// `rows` rows of 64 bf16 from `src` (consecutive, the first `valid` exist) -> operand image [8][rows][8] at row `row0`,
-// plane pitch CP, by threads tid of nthreads.
-__device__ __forceinline__ void load_rows(unsigned char* img, int row0, const __nv_bfloat16* src, int rows, int valid, int tid,
-                                          int nthreads) {
-  for (int x = tid; x < rows * 8; x += nthreads) {
-    const int r = x >> 3, c8 = x & 7;
-    async_copy16(img + c8 * CP + (row0 + r) * 16, src + (size_t)max(min(r, valid - 1), 0) * HD + c8 * 8, r < valid);
-  }
-}
 // Chunks 8 and 9 of the image of [v | 1 | 0]: one in the first element of rows below `valid`, zeros elsewhere.
 __device__ __forceinline__ void augment_rows(unsigned char* img, int valid, int tid, int nthreads) {
   for (int x = tid; x < 2 * CT; x += nthreads) {
@@ -84,13 +59,6 @@ __device__ __forceinline__ void load_head(float* l, HeadScalars* sc, const HeadF
     if (y < 0) async_copy16(reinterpret_cast<unsigned char*>(sc) + x * 16, reinterpret_cast<const unsigned char*>(&f->s) + x * 16, true);
     else async_copy16(l + 4 * y, &f->l[0][0] + 4 * y, true);
   }
-}
-
-// One arrival per warp on an mbarrier after every lane has finished what precedes (shared-memory
-// stores made visible to the async proxy, or tensor-memory accesses).
-__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
-  __syncwarp();
-  if (lane == 0) umma::mbar_arrive(bar);
 }
 
 // Term r of this thread's row as the MMA's A operand in tensor memory: bf16(l_r[d] x[d]) for 16 dimensions from d0

@@ -69,6 +69,8 @@ struct StateUpdateArgs {
   int32_t* block_status;        // with a prologue that clears `status` in this launch: a word per block instead, see state_scan
 };
 
+constexpr int GEN_THREADS = 256;      // (token, half of a slab)
+
 __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const StateUpdateArgs a, const PrologueArgs pro,
                                                                       int n_prologue) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -78,6 +80,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   }
   unsigned char* Abuf = smem;                          // 2 x SLAB_A_BYTES
   unsigned char* Uimg = smem + 2 * SLAB_A_BYTES;       // [10][128 tokens][8 e]
+  unsigned char* Ximg = Uimg + SLAB_S_BYTES;           // rows of k
   __shared__ uint64_t mma_done[2];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
@@ -92,15 +95,13 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
     mbar_fence_init();
     dead = 0;
   }
-  const int i = c * CT + token;
-  const __nv_bfloat16* kbase = a.k + (size_t)u * a.N * HD;
   const __nv_bfloat16* vbase = a.v + (size_t)u * a.N * VD;
-  uint32_t xp[HD / 2];
-  load_row_packed(xp, kbase, i, a.N);
+  load_rows(Ximg, 0, a.k + ((size_t)u * a.N + c * CT) * HD, CT, a.N - c * CT, tid, GEN_THREADS);
   for (int idx = tid; idx < (EP / 8) * CT; idx += GEN_THREADS) {
     const int ec = idx >> 7, t = idx & 127, j = c * CT + t;
     reinterpret_cast<uint4*>(Uimg)[idx] = u_image_chunk(vbase + (size_t)j * VD, ec, j < a.N);
   }
+  async_copies_wait();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -115,18 +116,16 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   auto epilogue = [&](int it) {
     w.wait(&mma_done[it & 1], (it >> 1) & 1);
     fence_after_sync();
-    if (warp >= 8) return;          // warps 0-7 cover the 128 lanes x 80 columns
     const int row = (s0 + it) * 128 + 32 * (warp & 3) + lane;
-    const int col0 = warp < 4 ? 0 : 48, ncol = warp < 4 ? 48 : 32;
+    const int col0 = warp < 4 ? 0 : 40, ncol = warp < 4 ? 40 : EU - 40;
     const uint32_t t = tacc + (uint32_t)((it & 1) * EP) + ((uint32_t)(32 * (warp & 3)) << 16) + col0;
-    for (int cc = 0; cc < ncol; cc += 16) {
-      float vv[16];
-      tmem_ld16(t + cc, vv);
+    for (int cc = 0; cc < ncol; cc += 8) {
+      float vv[8];
+      tmem_ld8(t + cc, vv);
       tmem_ld_wait();
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4)
-        *reinterpret_cast<float4*>(ds_base + state_inc_offset(row, col0 + cc + 4 * q4)) =
-            make_float4(vv[4 * q4], vv[4 * q4 + 1], vv[4 * q4 + 2], vv[4 * q4 + 3]);
+      float* dst = ds_base + state_inc_offset(row, col0 + cc);
+      *reinterpret_cast<float4*>(dst) = make_float4(vv[0], vv[1], vv[2], vv[3]);
+      *reinterpret_cast<float4*>(dst + 4) = make_float4(vv[4], vv[5], vv[6], vv[7]);
     }
     fence_before_sync();
   };
@@ -134,8 +133,11 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   for (int it = 0; it < ns; ++it) {
     const int buf = it & 1;
     // A[buf] and accumulator buf were released by epilogue(it-2), which every thread has passed
-    keep_in_loop(xp);
-    write_half_slab_raw(s0 + it, half, xp, reinterpret_cast<uint4*>(Abuf + buf * SLAB_A_BYTES) + token);
+    uint4* tile = reinterpret_cast<uint4*>(Abuf + buf * SLAB_A_BYTES) + 8 * half * CT + token;
+    const int hs = 2 * (s0 + it) + half;
+    const HalfBlock blk = half_block(min(hs, F_PAIR_BLOCKS - 1));
+    const auto piece = [&](int j) { return *reinterpret_cast<const uint4*>(Ximg + j * CP + token * 16); };
+    raw_half_slab(hs, piece(blk.rb), piece(blk.cb), piece, [&](int j, uint4 f) { tile[j * CT] = f; });
     fence_async_smem();
     __syncthreads();
     if (warp == 0 && elect_one()) {
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
 // state_scan: exclusive prefix over chunks (forward) or suffix (reverse), fp32 running sum,
 // result stored as the bf16 MMA operand image  [u][c][slab][e/8][128 rows][8 e].
 //   Increments and images have the same element order, so a thread owns four consecutive elements and walks the
-//   chunks: grid (F_ROWS * EP / 4 / 256, units).  Bound by HBM at many units, by the latency of the walk at few:
+//   chunks: grid (slabs x used blocks of 8 columns, units), one block of 128 rows x 8 columns per CTA.  Bound by HBM at many units, by the latency of the walk at few:
 //   the loads of SCAN_AHEAD chunks are in flight together.  `trim`: the first chunk visited meets a zero state and
 //   nothing reads its image, and the increment of the last one visited reaches no image: neither is touched.
 // image_lo (optional): a second image of the rounding remainders, bf16(state - bf16(state)); the
@@ -178,13 +180,12 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_b
                                                          float* state_total, int NB, int reverse, int trim,
                                                          const int32_t* block_status, int n_status, int32_t* status) {
   constexpr size_t CHUNK = (size_t)F_ROWS * EP;
-  static_assert(CHUNK % 1024 == 0, "the grid covers a chunk exactly");
-  const size_t x = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;      // element inside a chunk, image order
+  const int slab = blockIdx.x / (EU / 8), e8 = blockIdx.x % (EU / 8), within = threadIdx.x * 4;
+  const size_t x = (size_t)(slab * (EP / 8) + e8) * 1024 + within;    // element inside a chunk, image order
   const size_t u = blockIdx.y;
   // row-major position of the same element in state_in / state_total
-  const int tile = (int)(x >> 10), within = (int)(x & 1023);          // 1024 = 128 rows x 8 columns
-  const size_t rm = (size_t)((tile / (EP / 8)) * 128 + (within >> 3)) * EP + (tile % (EP / 8)) * 8 + (within & 7);
-  for (size_t b = (size_t)blockIdx.y * (CHUNK / 4) + x / 4; b < (size_t)n_status; b += (size_t)gridDim.y * (CHUNK / 4))
+  const size_t rm = (size_t)(slab * 128 + (within >> 3)) * EP + e8 * 8 + (within & 7);
+  for (size_t b = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x; b < (size_t)n_status; b += (size_t)gridDim.y * gridDim.x * 256)
     if (block_status[b]) atomicOr(status, block_status[b]);
   float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
   if (state_in) run = *reinterpret_cast<const float4*>(state_in + u * CHUNK + rm);
@@ -214,7 +215,10 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_b
       }
     }
   }
-  if (state_total) *reinterpret_cast<float4*>(state_total + u * CHUNK + rm) = run;
+  if (state_total) {
+    *reinterpret_cast<float4*>(state_total + u * CHUNK + rm) = run;
+    if (e8 == EU / 8 - 1) *reinterpret_cast<float4*>(state_total + u * CHUNK + rm + 8) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -236,25 +240,30 @@ struct CrossReadArgs {
 // Persistent, warp-specialised kernel.  Work items are (batch, head, chunk) with the heads of one
 // state unit adjacent, so CTAs running at the same time read the same state image from L2.  CTA k
 // takes items k, k + gridDim.x, ...; the flat iteration `it` = (item, slab) drives four roles:
-//   warps 0-7   generate feature slab `slab` of the item's 128 tokens into tensor memory, A[it % 4]
-//   warp  13    lane 0 streams the state slab images into a 6-slot ring and the head's coefficient
+//   generators  write feature slab `slab` of the item's 128 tokens into tensor memory, A[it % 5]; four sets of four
+//               warps (32 tokens each) take the slabs in turn
+//   loader      lane 0 streams the state slab images into slot it % 5 of a ring and the head's coefficient
 //               table into one of two buffers (bulk copies)
-//   warp  12    lane 0 issues the MMAs  acc[item & 1] += A . S  once both are full
-//   warps 8-11  after the item's last slab: accumulator -> HBM, then release it
-// What bounded it: shared memory.  With the slabs there an MMA of 128 x 80 x 16 reads 6.5 KB (53 clocks at 128 bytes
-// per clock), a slab is written and read at 32 KB each beside the 20 KB of state that arrive and are read: 970 of the
-// 1550 clocks a slab took.  A token is a tensor-memory lane and its thread writes the slab's columns itself, which
-// leaves the state image alone in shared memory.  Generating with 16 warps
-// and copying a quarter of the state changed nothing before that.  14 / 2 heads, B = 4, N = 4096: 187 -> 156 us
-// (QUERY), 32 -> 26 (not).
-constexpr int CR_GEN_WARPS = 8, CR_EPI_WARPS = 4;
+//   issuer      lane 0 issues the MMAs  acc[item & 1] += A . S  once both are there
+//   epilogue    after the item's last slab: accumulator -> HBM, then release it
+// A slot of features and a slot of the state share one barrier per direction: every wait and every commit costs the
+// issuing thread 50 to 100 clocks, and with a pair of each it needed 550 clocks per slab without any MMA (a slab's eight
+// MMAs take 480).  The epilogue goes through shared memory: stored by the thread of each row, 64 stores of 32 lines held up
+// every other shared-memory access of the SM for 3000 clocks per item.
+// What bounds it: the issuing thread (about 650 clocks per slab) and a gap of 1500 clocks at each item.  14 / 2 heads, 8 groups,
+// B = 4, N = 4096: 157 -> 116 us (QUERY), 30 -> 25 (not).
+constexpr int CR_SETS = 4, CR_GEN_WARPS = 4 * CR_SETS, CR_EPI_WARPS = 4;     // whole warpgroups
 constexpr int CR_ISSUER = CR_GEN_WARPS + CR_EPI_WARPS, CR_LOADER = CR_ISSUER + 1;
-constexpr int CR_THREADS = (CR_LOADER + 1) * 32;
-constexpr int CR_ARING = 4, CR_SRING = 6;
+// Two warps more only fill the issuer's warpgroup, whose registers the generators take: 768 threads x 80 at launch =
+// 512 x 88 + 128 x 72 + 128 x 40 and 2048 to spare.
+constexpr int CR_THREADS = (CR_LOADER + 3) * 32;
+constexpr int CR_RING = 5;
 // tensor memory: ring of feature slabs (128 features of the 128 tokens, two per column), two accumulators
-constexpr uint32_t CR_SLAB_COLS = 64, CR_ACC = CR_ARING * CR_SLAB_COLS;
+constexpr uint32_t CR_SLAB_COLS = 64, CR_ACC = CR_RING * CR_SLAB_COLS;
 static_assert(CR_ACC + 2 * EP <= 512, "tensor-memory columns of the cross-read kernel");
-static_assert(CR_GEN_WARPS * 32 == GEN_THREADS, "the slab generator is written for GEN_THREADS threads");
+// shared memory: ring of state slabs, two coefficient tables, two row images, the epilogue's rows (fp32, padded)
+constexpr int CR_COEF = CR_RING * SLAB_S_BYTES, CR_X = CR_COEF + 2 * F_ROWS * 4, CR_STAGE = CR_X + 2 * X_BYTES;
+constexpr int CR_PITCH = VD + 4, CR_SMEM = CR_STAGE + CT * CR_PITCH * 4;
 
 struct CrItem {
   int b, h, c;
@@ -273,9 +282,8 @@ __device__ __forceinline__ CrItem cr_item(int item, int H, int rep, int NC, int 
 template <bool QUERY>
 __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossReadArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* Sbuf = smem;                                   // CR_SRING x SLAB_S_BYTES, then the head's coefficient table
-  __shared__ uint64_t full_a[CR_ARING], a_free[CR_ARING], s_full[CR_SRING], s_free[CR_SRING], acc_full[2], acc_free[2];
-  __shared__ uint64_t coef_full[2], coef_free[2];
+  __shared__ uint64_t full[CR_RING], done[CR_RING], acc_full[2], acc_free[2];
+  __shared__ uint64_t coef_full[2], coef_free[2], x_full[2];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -283,19 +291,16 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   if (warp == CR_ISSUER) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
-    for (int s = 0; s < CR_ARING; ++s) {
-      mbar_init(&full_a[s], CR_GEN_WARPS);
-      mbar_init(&a_free[s], 1);
-    }
-    for (int s = 0; s < CR_SRING; ++s) {
-      mbar_init(&s_full[s], 1);
-      mbar_init(&s_free[s], 1);
+    for (int s = 0; s < CR_RING; ++s) {
+      mbar_init(&full[s], 4 + 1);          // the warps of a set, and the loader
+      mbar_init(&done[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&acc_full[s], 1);
       mbar_init(&acc_free[s], CR_EPI_WARPS);
       mbar_init(&coef_full[s], 1);
       mbar_init(&coef_free[s], CR_GEN_WARPS);
+      mbar_init(&x_full[s], CR_GEN_WARPS);
     }
     mbar_fence_init();
     dead = 0;
@@ -307,121 +312,129 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
   const uint32_t tmem = uniform(tmem_base);
 
   if (warp < CR_GEN_WARPS) {
-    // ---------------- generators: thread = (token, half of the slab's chunks) ----------------
-    const int token = tid & 127, half = warp >> 2;
-    int s3 = 0, use = 0;
-    for (int k = 0; k < my_items; ++k) {
+    // ---------------- generators ----------------
+    registers_up_to<88>();
+    const int set = warp >> 2;
+    unsigned char* ximg = smem + CR_X;
+    const auto fetch = [&](int k) {
       const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
+      load_rows(ximg + (k & 1) * X_BYTES, 0, a.x + ((size_t)(it.b * a.H + it.h) * a.N + it.c * CT) * HD, CT, a.N - it.c * CT, tid,
+                CR_GEN_WARPS * 32);
+    };
+    if (my_items > 0) fetch(0);
+    int flat = set;                                      // slab of this set, over all items
+    for (int k = 0; k < my_items; ++k) {
+      async_copies_wait();
+      warp_arrive(&x_full[k & 1], lane);
+      w.wait(&x_full[k & 1], (k >> 1) & 1, 0x49);        // the rows are in, and item k-1 has been generated
+      if (k + 1 < my_items) fetch(k + 1);
       // this head's coefficient table, brought in by the loader warp (two buffers)
-      const float* coef = reinterpret_cast<const float*>(Sbuf + CR_SRING * SLAB_S_BYTES) + (k & 1) * F_ROWS;
+      const float* coef = reinterpret_cast<const float*>(smem + CR_COEF) + (k & 1) * F_ROWS;
       if constexpr (QUERY) w.wait(&coef_full[k & 1], (k >> 1) & 1, 0x47);
-      uint32_t xp[HD / 2];
-      load_row_packed(xp, a.x + (size_t)(it.b * a.H + it.h) * a.N * HD, it.c * CT + token, a.N);
-      f32x2 xq[QUERY ? HD / 2 : 1];
-      if constexpr (QUERY) unpack_row(xp, xq);
-      for (int s = 0; s < F_SLABS; ++s) {
-        if (use > 0) w.wait(&a_free[s3], (use - 1) & 1, 0x41);      // the MMAs that read A[s3] have completed
+      const unsigned char* xlane = ximg + (k & 1) * X_BYTES + (32 * (warp & 3) + (lane >> 2)) * 16;
+      for (; flat < (k + 1) * F_SLABS; flat += CR_SETS) {
+        const int slot_i = flat % CR_RING, use = flat / CR_RING, slab = flat - k * F_SLABS;
+        if (use > 0) w.wait(&done[slot_i], (use - 1) & 1, 0x41);      // the MMAs that read the slot have completed
         __syncwarp();
         fence_after_sync();
-        const uint32_t slot = tmem + s3 * CR_SLAB_COLS + ((uint32_t)(32 * (warp & 3)) << 16);
-        if constexpr (QUERY) {
-          keep_in_loop(xq);
-          store_half_slab_coef(s, half, xq, coef, slot);
-        } else {
-          keep_in_loop(xp);
-          store_half_slab_raw(s, half, xp, slot);
-        }
+        const uint32_t slot = tmem + slot_i * CR_SLAB_COLS + ((uint32_t)(32 * (warp & 3)) << 16);
+        store_half_slab<QUERY>(2 * slab, xlane, coef, slot, lane);
+        store_half_slab<QUERY>(2 * slab + 1, xlane, coef, slot + CR_SLAB_COLS / 2, lane);
         tmem_st_wait();
         fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&full_a[s3]);
-        if (++s3 == CR_ARING) { s3 = 0; ++use; }
+        warp_arrive(&full[slot_i], lane);
       }
-      if constexpr (QUERY) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&coef_free[k & 1]);     // this warp no longer reads the table
-      }
+      if constexpr (QUERY) warp_arrive(&coef_free[k & 1], lane);     // this warp no longer reads the table
     }
   } else if (warp < CR_ISSUER) {
     // ---------------- accumulator -> HBM ----------------
+    registers_down_to<72>();
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
+    float* stage = reinterpret_cast<float*>(smem + CR_STAGE) + 32 * (warp & 3) * CR_PITCH;      // this warp's 32 rows
     for (int k = 0; k < my_items; ++k) {
       const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
-      const int row = it.c * CT + 32 * (warp & 3) + lane;
-      const size_t orow = (size_t)(it.b * a.H + it.h) * a.N + row;
+      const int row0 = it.c * CT + 32 * (warp & 3);
+      const size_t orow = (size_t)(it.b * a.H + it.h) * a.N + row0;
       w.wait(&acc_full[k & 1], (k >> 1) & 1, 0x42);
+      __syncwarp();
       fence_after_sync();
       const uint32_t t = tmem + CR_ACC + (k & 1) * EP + lane_off;
 #pragma unroll
-      for (int cc = 0; cc < EP; cc += 16) {
-        if (cc < VD || QUERY) {
-          float vv[16];
-          tmem_ld16(t + cc, vv);
-          tmem_ld_wait();
-          if (row < a.N && !dead) {
-            if (cc < VD) {
+      for (int cc = 0; cc < VD; cc += 16) {
+        float vv[16];
+        tmem_ld16(t + cc, vv);
+        tmem_ld_wait();
 #pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4)
-                *reinterpret_cast<float4*>(a.out64 + orow * VD + cc + 4 * q4) =
-                    make_float4(vv[4 * q4], vv[4 * q4 + 1], vv[4 * q4 + 2], vv[4 * q4 + 3]);
-            } else if (QUERY) {
-              a.out1[orow] = vv[0];
-            }
-          }
-        }
+        for (int q4 = 0; q4 < 4; ++q4)
+          *reinterpret_cast<float4*>(stage + lane * CR_PITCH + cc + 4 * q4) = make_float4(vv[4 * q4], vv[4 * q4 + 1], vv[4 * q4 + 2], vv[4 * q4 + 3]);
+      }
+      float den[8] = {};
+      if constexpr (QUERY) {
+        tmem_ld8(t + VD, den);
+        tmem_ld_wait();
       }
       fence_before_sync();
+      warp_arrive(&acc_free[k & 1], lane);              // (and the staged rows are visible to the warp)
+      if (!dead) {
+        if (QUERY && row0 + lane < a.N) a.out1[orow + lane] = den[0];
+#pragma unroll 4
+        for (int x = lane; x < 32 * (VD / 4); x += 32) {
+          const int r = x / (VD / 4), c4 = x % (VD / 4);
+          if (row0 + r < a.N)
+            *reinterpret_cast<float4*>(a.out64 + orow * VD + 4 * x) = *reinterpret_cast<const float4*>(stage + r * CR_PITCH + 4 * c4);
+        }
+      }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_free[k & 1]);
     }
-  } else if (warp == CR_ISSUER) {
-    // ---------------- MMA issue ----------------
-    if (elect_one()) {
+  } else {
+    registers_down_to<40>();
+    if (warp == CR_ISSUER && elect_one()) {
+      // ---------------- MMA issue ----------------
       const uint32_t idesc = instr_desc_bf16(128, EP, 0, 1);
       // descriptor of slot 0 of the image ring, advanced by adds: this thread is the serial path of every slab
-      const uint64_t ds0 = smem_desc(smem_u32(Sbuf), 128, 128 * 16);
-      int s3 = 0, use = 0, gs = 0, guse = 0;
+      const uint64_t ds0 = smem_desc(smem_u32(smem), 128, 128 * 16);
+      int slot = 0, use = 0;
       for (int k = 0; k < my_items; ++k) {
         const uint32_t tacc = tmem + CR_ACC + (k & 1) * EP;
         if (k >= 2) w.wait(&acc_free[k & 1], ((k >> 1) - 1) & 1, 0x43);   // item k-2 has left this accumulator
         for (int s = 0; s < F_SLABS; ++s) {
-          const uint64_t dsl = desc_advance(ds0, gs * SLAB_S_BYTES);
-          const uint32_t slab = tmem + s3 * CR_SLAB_COLS;
-          w.wait(&full_a[s3], use & 1, 0x44);
-          w.wait(&s_full[gs], guse & 1, 0x45);
+          const uint64_t dsl = desc_advance(ds0, slot * SLAB_S_BYTES);
+          const uint32_t slab = tmem + slot * CR_SLAB_COLS;
+          w.wait(&full[slot], use & 1, 0x44);
           fence_after_sync();
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks)       // 16 features per step
-            mma_bf16_ts(tacc, slab + 8 * ks, desc_advance(dsl, ks * 256), idesc, (s > 0 || ks > 0));
-          mma_commit(&a_free[s3]);
-          mma_commit(&s_free[gs]);
-          if (s == F_SLABS - 1) mma_commit(&acc_full[k & 1]);
-          if (++s3 == CR_ARING) { s3 = 0; ++use; }
-          if (++gs == CR_SRING) { gs = 0; ++guse; }
+            if (s < F_SLABS - 1 || ks < LAST_STEPS) mma_bf16_ts(tacc, slab + 8 * ks, desc_advance(dsl, ks * 256), idesc, (s > 0 || ks > 0));
+          mma_commit(&done[slot]);
+          if (++slot == CR_RING) { slot = 0; ++use; }
         }
+        mma_commit(&acc_full[k & 1]);
       }
     }
-    __syncwarp();
-  } else {
-    // ---------------- state image stream ----------------
-    if (elect_one()) {
-      int gs = 0, guse = 0;
+    if (warp == CR_LOADER && elect_one()) {
+      // ---------------- state image and coefficient stream ----------------
+      int slot = 0, use = 0;
+      const auto fetch_coef = [&](int k) {
+        const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
+        if (k >= 2) w.wait(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x48);   // item k-2 no longer reads this buffer
+        mbar_arrive_expect_tx(&coef_full[k & 1], F_ROWS * (uint32_t)sizeof(float));
+        bulk_g2s(smem + CR_COEF + (k & 1) * F_ROWS * sizeof(float), a.coef_table + (size_t)it.h * F_ROWS,
+                 F_ROWS * (uint32_t)sizeof(float), &coef_full[k & 1]);
+      };
+      if (QUERY && my_items > 0) fetch_coef(0);
       for (int k = 0; k < my_items; ++k) {
         const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         const int unit = (it.b * a.H + it.h) / a.rep;
         const unsigned char* img = reinterpret_cast<const unsigned char*>(a.image) +
                                    ((size_t)unit * a.NB + it.c) * F_SLABS * SLAB_S_BYTES;
-        if constexpr (QUERY) {
-          if (k >= 2) w.wait(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x48);   // item k-2 no longer reads this buffer
-          mbar_arrive_expect_tx(&coef_full[k & 1], F_ROWS * (uint32_t)sizeof(float));
-          bulk_g2s(Sbuf + CR_SRING * SLAB_S_BYTES + (k & 1) * F_ROWS * sizeof(float),
-                   a.coef_table + (size_t)it.h * F_ROWS, F_ROWS * (uint32_t)sizeof(float), &coef_full[k & 1]);
-        }
         for (int s = 0; s < F_SLABS; ++s) {
-          if (guse > 0) w.wait(&s_free[gs], (guse - 1) & 1, 0x46);
-          mbar_arrive_expect_tx(&s_full[gs], SLAB_S_BYTES);
-          bulk_g2s(Sbuf + gs * SLAB_S_BYTES, img + (size_t)s * SLAB_S_BYTES, SLAB_S_BYTES, &s_full[gs]);
-          if (++gs == CR_SRING) { gs = 0; ++guse; }
+          // the next item's table while there is time: its buffer's last reader was item k-1
+          if (QUERY && s == 2 * F_SLABS / 3 && k + 1 < my_items) fetch_coef(k + 1);
+          if (use > 0) w.wait(&done[slot], (use - 1) & 1, 0x46);
+          // the unused columns of an image only reach unused columns of the accumulator
+          mbar_arrive_expect_tx(&full[slot], SLAB_U_BYTES);
+          bulk_g2s(smem + slot * SLAB_S_BYTES, img + (size_t)s * SLAB_S_BYTES, SLAB_U_BYTES, &full[slot]);
+          if (++slot == CR_RING) { slot = 0; ++use; }
         }
       }
     }
@@ -449,7 +462,7 @@ int state_update_blocks(int units, int NC) { return SU_GROUPS * NC * units; }
 
 cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, const PrologueArgs* prologue,
                          int q_heads, int32_t* status, int32_t* block_status, cudaStream_t st) {
-  const int smem = 2 * SLAB_A_BYTES + SLAB_S_BYTES;
+  const int smem = 2 * SLAB_A_BYTES + SLAB_S_BYTES + X_BYTES;
   cudaError_t e = allow_smem<state_update_kernel>(smem);
   if (e != cudaSuccess) return e;
   StateUpdateArgs a{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ds, N, NB, NC, status, block_status};
@@ -461,7 +474,7 @@ cudaError_t state_update(const void* k, const void* v, float* ds, int units, int
 cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float* state_in, float* state_total,
                        int units, int NB, int reverse, bool trim, const int32_t* block_status, int n_status, int32_t* status,
                        cudaStream_t st) {
-  state_scan_kernel<<<dim3(F_ROWS * EP / 1024, units), 256, 0, st>>>(
+  state_scan_kernel<<<dim3(F_SLABS * (EU / 8), units), 256, 0, st>>>(
       ds, static_cast<__nv_bfloat16*>(image), static_cast<__nv_bfloat16*>(image_lo), state_in, state_total, NB, reverse,
       trim ? 1 : 0, block_status, block_status ? n_status : 0, status);
   return cudaGetLastError();
@@ -470,17 +483,16 @@ cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float
 cudaError_t cross_read(bool query, const void* x, const void* image, const float* coef_table, float* out64,
                        float* out1, int B, int H, int rep, int N, int NB, int c0, int NC, int32_t* status,
                        cudaStream_t st) {
-  const int smem = CR_SRING * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float);
   CrossReadArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(image), coef_table,
                   out64, out1, N, NB, H, rep, B, c0, NC, status};
   cudaError_t e;
   const int sms = sm_count(), items = B * H * NC, grid = items < sms ? items : sms;
   if (query) {
-    if ((e = allow_smem<cross_read_kernel<true>>(smem)) != cudaSuccess) return e;
-    cross_read_kernel<true><<<grid, CR_THREADS, smem, st>>>(a);
+    if ((e = allow_smem<cross_read_kernel<true>>(CR_SMEM)) != cudaSuccess) return e;
+    cross_read_kernel<true><<<grid, CR_THREADS, CR_SMEM, st>>>(a);
   } else {
-    if ((e = allow_smem<cross_read_kernel<false>>(smem)) != cudaSuccess) return e;
-    cross_read_kernel<false><<<grid, CR_THREADS, smem, st>>>(a);
+    if ((e = allow_smem<cross_read_kernel<false>>(CR_SMEM)) != cudaSuccess) return e;
+    cross_read_kernel<false><<<grid, CR_THREADS, CR_SMEM, st>>>(a);
   }
   return cudaGetLastError();
 }

@@ -50,22 +50,34 @@ struct DStateArgs {
 // Persistent, warp-specialised kernel.  Work items are (batch x KV head, chunk, feature slab); CTA k
 // takes items k, k + gridDim.x, ... and walks the query heads of the KV head for each, so the flat
 // iteration `it` = (item, head) drives four pipelined roles:
-//   warps 0-3   thread = token: generate the coefficient-free, unscaled feature slab of (item, head)
-//               from the packed bf16 q row into A[it % 3]
-//   warp  13    lane 0 streams the head's G image into a 4-slot ring (bulk copies)
-//   warp  12    lane 0 issues the MMAs  Z[it % 3] = A^T G  once A and G are full and Z[it % 3] is drained
-//   warps 4-11  drain Z, thread = (feature row, half of the 80 columns): dot with the carry row for
+//   warps 0-7   thread = (token, half of the slab): generate the coefficient-free, unscaled feature slab of (item, head)
+//               from the q rows into A[it % 3]
+//   warp  17    lane 0 streams the head's G image and coefficients into slot it % 3 of a ring and, an item ahead, the
+//               slab's carry and remainder images (bulk copies)
+//   warp  16    lane 0 issues the MMAs  Z[it % 3] = A^T G  once A and G are there and Z[it % 3] is drained
+//   warps 8-15  drain Z, thread = (feature row, part of the used columns): dot with the carry row for
 //               the coefficient gradient, acc += coef_h * Z in registers; after the last head
 //               acc -> dCarry
-// A slot and Z buffer share the index it % 3, so the MMA-completion barrier of that index tells the
-// generators "A is free" and the drain warps "Z is ready".
-constexpr int DS_GEN_WARPS = 4, DS_EPI_WARPS = 8;
+// A, G and Z share the index it % 3 and one barrier per direction: `ready` counts the generator and drain warps and the
+// loader, and the MMA-completion barrier tells the generators "A is free", the loader "G is free" and the drain warps
+// "Z is ready".  (Every wait and every commit costs the issuing thread 50 to 100 clocks.)
+constexpr int DS_GEN_WARPS = 8, DS_EPI_WARPS = 8;
 constexpr int DS_ISSUER = DS_GEN_WARPS + DS_EPI_WARPS, DS_LOADER = DS_ISSUER + 1;
-constexpr int DS_THREADS = (DS_LOADER + 1) * 32;
-constexpr int DS_RING = 3;      // A slots in shared memory = Z buffers in tensor memory
-constexpr int DS_GRING = 4;     // G image slots
-constexpr int DS_COLS = EP / 2; // columns per drain thread
-static_assert(DS_GEN_WARPS * 32 == CT, "one generator thread per token");
+// What bounds it: the drain (about 1400 clocks per iteration) and the generators, latency rather than issue slots.  The carry
+// rows were loaded by the drain warps at the head of an item, 5000 of its 15000 clocks.  14 / 2 heads, B = 4, N = 4096:
+// 268 -> 221 us.
+// Two warps more only fill the issuer's warpgroup, whose registers the drain warps take: 640 threads x 96 at launch =
+// 256 x 80 + 256 x 144 + 128 x 24 and 1024 to spare.
+constexpr int DS_THREADS = (DS_LOADER + 3) * 32;
+constexpr int DS_RING = 3;      // A and G slots in shared memory, Z buffers in tensor memory
+// shared memory: A slots | G slots (the MMA reads 8 columns past the used ones: in bounds, into columns of Z that no one
+// reads) | carry and its remainders | coefficients.  A coefficient slot is written again six iterations later,
+// behind mma_done of the third one after its own: the drain warps had read it before they let that MMA have Z.
+constexpr int DS_G = DS_RING * SLAB_A_BYTES, DS_CARRY = DS_G + DS_RING * SLAB_U_BYTES;
+constexpr int DS_COEF = DS_CARRY + 2 * SLAB_U_BYTES, DS_CRING = 2 * DS_RING;
+constexpr int DS_SMEM = DS_COEF + DS_CRING * 128 * 4;
+constexpr int DS_COLS = EP / 2; // columns per drain thread; the second half has EU - DS_COLS used ones
+static_assert(DS_GEN_WARPS * 32 == 2 * CT, "a generator thread per token and half of a slab");
 static_assert(DS_GEN_WARPS % 4 == 0, "drain warp w must sit on tensor-memory lane quadrant w % 4");
 
 // (item, head) cursor of one role; the divisions happen only when the item changes
@@ -96,8 +108,8 @@ struct DsCursor {
 __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStateArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* Abuf = smem;                              // DS_RING x SLAB_A_BYTES
-  unsigned char* Gbuf = smem + DS_RING * SLAB_A_BYTES;     // DS_GRING x SLAB_S_BYTES  ([10][128 tokens][8 e])
-  __shared__ uint64_t full_a[DS_RING], mma_done[DS_RING], z_free[DS_RING], g_full[DS_GRING], g_free[DS_GRING];
+  unsigned char* Gbuf = smem + DS_G;
+  __shared__ uint64_t ready[DS_RING], mma_done[DS_RING], carry_full, carry_free;
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -108,14 +120,11 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
   if (warp == DS_ISSUER) tmem_alloc(&tmem_base, 256);
   if (tid == 0) {
     for (int s = 0; s < DS_RING; ++s) {
-      mbar_init(&full_a[s], DS_GEN_WARPS);
+      mbar_init(&ready[s], DS_GEN_WARPS + DS_EPI_WARPS + 1);
       mbar_init(&mma_done[s], 1);
-      mbar_init(&z_free[s], DS_EPI_WARPS);
     }
-    for (int s = 0; s < DS_GRING; ++s) {
-      mbar_init(&g_full[s], 1);
-      mbar_init(&g_free[s], 1);
-    }
+    mbar_init(&carry_full, 1);
+    mbar_init(&carry_free, DS_EPI_WARPS);
     mbar_fence_init();
     dead = 0;
   }
@@ -127,44 +136,45 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
 
   if (warp < DS_GEN_WARPS) {
     // ---------------- generators ----------------
-    const int token = tid;
-    uint4 nx[8];                               // packed q row of the next (item, head)
-    auto fetch = [&](const DsCursor& d) {
-      const int h = d.h0 + d.hh, i = d.c * CT + token;
-      if (i < a.N) {
-        const uint4* p = reinterpret_cast<const uint4*>(a.q + ((size_t)(d.b * a.Hq + h) * a.N + i) * HD);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) nx[j] = p[j];
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) nx[j] = make_uint4(0u, 0u, 0u, 0u);
-      }
-    };
+    registers_down_to<80>();
+    // The two pieces of its token's row that a thread needs for (item, head) come straight from global memory, an
+    // iteration ahead.  (The whole row, once per slab: 32 cache lines for each of eight loads, 1000 clocks.  Through shared
+    // memory with cp.async, coalesced: about 1000 clocks too, which the copies of 16 bytes take to issue.)
+    const int half = warp >> 2, token = 32 * (warp & 3) + lane;
     DsCursor cur;
     cur.start(a.c0, a.NC, a.Hkv, rep);
-    if (T > 0) fetch(cur);
+    const __nv_bfloat16* row = nullptr;        // the token's row, or null past the end of the sequence
+    uint4 r4 = make_uint4(0u, 0u, 0u, 0u), c4 = r4;
+    const auto fetch = [&]() {
+      const int i = cur.c * CT + token, hs = 2 * cur.slab + half;
+      const HalfBlock blk = half_block(min(hs, F_PAIR_BLOCKS - 1));
+      row = i < a.N ? a.q + ((size_t)(cur.b * a.Hq + cur.h0 + cur.hh) * a.N + i) * HD : nullptr;
+      if (row) {
+        r4 = __ldg(reinterpret_cast<const uint4*>(row) + blk.rb);
+        c4 = __ldg(reinterpret_cast<const uint4*>(row) + blk.cb);
+      } else {
+        r4 = c4 = make_uint4(0u, 0u, 0u, 0u);
+      }
+    };
+    if (T > 0) fetch();
     int s = 0, use = 0;                       // ring slot of `it` and how often it has been used before
     for (int it = 0; it < T; ++it) {
-      const int slab = cur.slab;
-      uint32_t xp[HD / 2];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        xp[4 * j] = nx[j].x;
-        xp[4 * j + 1] = nx[j].y;
-        xp[4 * j + 2] = nx[j].z;
-        xp[4 * j + 3] = nx[j].w;
-      }
+      const int hs = 2 * cur.slab + half;
+      const uint4 r_now = r4, c_now = c4;
+      const __nv_bfloat16* row_now = row;
       cur.next(rep, a.c0, a.NC, a.Hkv);
-      if (it + 1 < T) fetch(cur);             // in flight while this slab is generated
+      if (it + 1 < T) fetch();
       if (use > 0) w.wait(&mma_done[s], (use - 1) & 1, 0x31);   // the MMA that read A[s] has completed
-      write_slab_raw(slab, xp, reinterpret_cast<uint4*>(Abuf + s * SLAB_A_BYTES) + token);
+      uint4* tile = reinterpret_cast<uint4*>(Abuf + s * SLAB_A_BYTES) + 8 * half * CT + token;
+      raw_half_slab(hs, r_now, c_now, [&](int j) { return row_now ? __ldg(reinterpret_cast<const uint4*>(row_now) + j) : make_uint4(0u, 0u, 0u, 0u); },
+                    [&](int j, uint4 f) { tile[j * CT] = f; });
       fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&full_a[s]);
+      warp_arrive(&ready[s], lane);
       if (++s == DS_RING) { s = 0; ++use; }
     }
   } else if (warp < DS_ISSUER) {
     // ---------------- drain warps ----------------
+    registers_up_to<144>();
     const int fr = 32 * (warp & 3) + lane, ch = (warp - DS_GEN_WARPS) >> 2, col0 = ch * DS_COLS;
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
     // packed fp32 pairs: the drain is bound by issue slots, and a packed multiply-add is one slot for two columns
@@ -176,22 +186,24 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
     d.start(a.c0, a.NC, a.Hkv, rep);
     dn = d;
     int s = 0, use = 0;
-    float cf_next = T > 0 ? a.coef_table[(size_t)d.h0 * F_ROWS + d.slab * 128 + fr] : 0.f;
+    const int blocks = ch == 0 ? DS_COLS / 8 : (EU - DS_COLS) / 8;      // of 8 used columns
+    if (lane == 0)
+      for (int x = 0; x < DS_RING; ++x) mbar_arrive(&ready[x]);         // the Z buffers are empty
+    int items = 0;
     for (int it = 0; it < T; ++it) {
       const int b = d.b, h = d.h0 + d.hh, f = d.slab * 128 + fr;
       const float fs = feature_scale_factor(f, a.scale);   // d(table entry) / d(coefficient)
-      const float cf = cf_next;
       dn.next(rep, a.c0, a.NC, a.Hkv);
-      if (it + 1 < T)       // coefficient of the next (item, head): in flight during this drain
-        cf_next = a.coef_table[(size_t)(dn.h0 + dn.hh) * F_ROWS + dn.slab * 128 + fr];
       if (d.hh == 0 && a.carry_img) {
-        const uint4* cp = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(a.carry_img) +
-                                                         (((size_t)d.u * a.NB + d.c) * F_SLABS + d.slab) * SLAB_S_BYTES);
-        const uint4* cl = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(a.carry_lo) +
-                                                         (((size_t)d.u * a.NB + d.c) * F_SLABS + d.slab) * SLAB_S_BYTES);
+        const uint4* cp = reinterpret_cast<const uint4*>(smem + DS_CARRY);
+        const uint4* cl = reinterpret_cast<const uint4*>(smem + DS_CARRY + SLAB_U_BYTES);
+        w.wait(&carry_full, items & 1, 0x37);
+        ++items;
         uint4 cpk[DS_COLS / 8], cpl[DS_COLS / 8];
 #pragma unroll
         for (int e = 0; e < DS_COLS / 8; ++e) {
+          cpk[e] = cpl[e] = make_uint4(0u, 0u, 0u, 0u);
+          if (e >= blocks) continue;
           cpk[e] = cp[(col0 / 8 + e) * 128 + fr];
           cpl[e] = cl[(col0 / 8 + e) * 128 + fr];
         }
@@ -203,6 +215,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
 #pragma unroll
           for (int j = 0; j < 4; ++j) carry[4 * e + j] = f2_pack(c0[2 * j] + c1[2 * j], c0[2 * j + 1] + c1[2 * j + 1]);
         }
+        warp_arrive(&carry_free, lane);
       }
       w.wait(&mma_done[s], use & 1, 0x32);
       fence_after_sync();
@@ -212,14 +225,15 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
         for (int j = 0; j < DS_COLS / 2; ++j) acc[j] = 0ull;
       }
       f32x2 dot[2] = {0ull, 0ull};
-      const f32x2 cf2 = f2_bcast(cf);
+      const f32x2 cf2 = f2_bcast(reinterpret_cast<const float*>(smem + DS_COEF)[it % DS_CRING * 128 + fr]);
       // two register stages: the loads of the next 8 columns are in flight while these are combined
       float z[2][8];
       tmem_ld8(tz + lane_off, z[0]);
 #pragma unroll
       for (int r = 0; r < DS_COLS / 8; ++r) {
+        if (r >= blocks) continue;
         tmem_ld_wait();
-        if (r + 1 < DS_COLS / 8) tmem_ld8(tz + lane_off + 8 * (r + 1), z[(r + 1) & 1]);
+        if (r + 1 < blocks) tmem_ld8(tz + lane_off + 8 * (r + 1), z[(r + 1) & 1]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const f32x2 z2 = f2_pack(z[r & 1][2 * j], z[r & 1][2 * j + 1]);
@@ -228,8 +242,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
         }
       }
       fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&z_free[s]);      // every lane has its Z values in registers
+      warp_arrive(&ready[s], lane);                // every lane has its Z values in registers
       float d0, d1, d2, d3;
       f2_unpack(dot[0], d0, d1);
       f2_unpack(dot[1], d2, d3);
@@ -242,6 +255,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
         float* dst = a.dcarry + ((size_t)d.u * a.NB + d.c) * F_ROWS * EP + state_inc_offset(f, col0);
 #pragma unroll
         for (int r = 0; r < DS_COLS / 8; ++r) {
+          if (r >= blocks) continue;
           float o[8];
 #pragma unroll
           for (int j = 0; j < 4; ++j) f2_unpack(acc[4 * r + j], o[2 * j], o[2 * j + 1]);
@@ -252,45 +266,52 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
       d = dn;
       if (++s == DS_RING) { s = 0; ++use; }
     }
-  } else if (warp == DS_ISSUER) {
-    // ---------------- MMA issue ----------------
-    if (elect_one()) {
+  } else {
+    registers_down_to<24>();
+    if (warp == DS_ISSUER && elect_one()) {
+      // ---------------- MMA issue ----------------
       const uint32_t idesc = instr_desc_bf16(128, EP, 1, 1);
       // descriptors of slot 0 of both rings, advanced by adds: this thread is the serial path of every slab
       const uint64_t da0 = smem_desc(smem_u32(Abuf), 128, CT * 16), dg0 = smem_desc(smem_u32(Gbuf), 128, CT * 16);
-      int s = 0, use = 0, gs = 0, guse = 0;
+      int s = 0, use = 0;
       for (int it = 0; it < T; ++it) {
-        const uint64_t da = desc_advance(da0, s * SLAB_A_BYTES), dg = desc_advance(dg0, gs * SLAB_S_BYTES);
+        const uint64_t da = desc_advance(da0, s * SLAB_A_BYTES), dg = desc_advance(dg0, s * SLAB_U_BYTES);
         const uint32_t tz = tmem + EP * s;
-        w.wait(&full_a[s], use & 1, 0x33);
-        w.wait(&g_full[gs], guse & 1, 0x34);
-        if (use > 0) w.wait(&z_free[s], (use - 1) & 1, 0x35);
+        w.wait(&ready[s], use & 1, 0x33);
         fence_after_sync();
 #pragma unroll
         for (int ks = 0; ks < CT / 16; ++ks)
           mma_bf16_ss(tz, desc_advance(da, ks * 256), desc_advance(dg, ks * 256), idesc, ks > 0);
         mma_commit(&mma_done[s]);
-        mma_commit(&g_free[gs]);               // the loader may refill this G slot when these MMAs are done
         if (++s == DS_RING) { s = 0; ++use; }
-        if (++gs == DS_GRING) { gs = 0; ++guse; }
       }
     }
-    __syncwarp();
-  } else {
-    // ---------------- G image stream ----------------
-    if (elect_one()) {
+    if (warp == DS_LOADER && elect_one()) {
+      // ---------------- G image, carry and coefficient stream ----------------
       DsCursor d;
       d.start(a.c0, a.NC, a.Hkv, rep);
-      int gs = 0, guse = 0;
+      int s = 0, use = 0, fetched = 0;
+      const auto fetch_carry = [&](const DsCursor& x) {
+        const size_t at = (((size_t)x.u * a.NB + x.c) * F_SLABS + x.slab) * SLAB_S_BYTES;
+        if (fetched > 0) w.wait(&carry_free, (fetched - 1) & 1, 0x38);      // in registers of the drain warps
+        ++fetched;
+        mbar_arrive_expect_tx(&carry_full, 2 * SLAB_U_BYTES);
+        bulk_g2s(smem + DS_CARRY, reinterpret_cast<const unsigned char*>(a.carry_img) + at, SLAB_U_BYTES, &carry_full);
+        bulk_g2s(smem + DS_CARRY + SLAB_U_BYTES, reinterpret_cast<const unsigned char*>(a.carry_lo) + at, SLAB_U_BYTES, &carry_full);
+      };
+      if (T > 0 && a.carry_img) fetch_carry(d);
       for (int it = 0; it < T; ++it) {
         const int h = d.h0 + d.hh;
         const unsigned char* src =
             reinterpret_cast<const unsigned char*>(a.gimg) + ((size_t)(d.b * a.Hq + h) * a.NB + d.c) * SLAB_S_BYTES;
-        if (guse > 0) w.wait(&g_free[gs], (guse - 1) & 1, 0x36);
-        mbar_arrive_expect_tx(&g_full[gs], SLAB_S_BYTES);
-        bulk_g2s(Gbuf + gs * SLAB_S_BYTES, src, SLAB_S_BYTES, &g_full[gs]);
+        if (use > 0) w.wait(&mma_done[s], (use - 1) & 1, 0x36);
+        mbar_arrive_expect_tx(&ready[s], SLAB_U_BYTES + 128 * 4);
+        bulk_g2s(Gbuf + s * SLAB_U_BYTES, src, SLAB_U_BYTES, &ready[s]);
+        bulk_g2s(smem + DS_COEF + it % DS_CRING * 128 * 4, a.coef_table + (size_t)h * F_ROWS + d.slab * 128, 128 * 4, &ready[s]);
+        const bool last = d.hh == rep - 1;
         d.next(rep, a.c0, a.NC, a.Hkv);
-        if (++gs == DS_GRING) { gs = 0; ++guse; }
+        if (last && it + 1 < T && a.carry_img) fetch_carry(d);
+        if (++s == DS_RING) { s = 0; ++use; }
       }
     }
     __syncwarp();
@@ -302,104 +323,121 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
 }
 
 // ---------------------------------------------------------------------------
-// fold of dphi (tensor memory, thread = token, columns = the 128 features of a slab) through the
-// feature map into dx.  x and dx are fp32 rows held as packed pairs (element 2k, 2k+1 in pair k);
-// every index is a compile-time constant.  Per pair chunk (cb, r), with t_j = dphi_j (* coef_j):
-//   dx[r]        += sum_j t_j x[8 cb + j]        dx[8 cb + j] += t_j x[r]
+// fold of dphi (tensor memory, thread = token, columns = the features of a half slab) through the feature map into dx.
+// Per block of x x^T, with t = dphi (* coef):
+//   dx[r] += sum_c t[r][c] x[c]        dx[c] += sum_r t[r][c] x[r]
+// dx lies in shared memory (fp32, this thread's token); the sums of the column block stay in registers while it does
+// not change.  Entries above the diagonal of a diagonal block add zeros: their coefficients are zero, and so are the rows
+// of dCarry that belong to them.
 // ---------------------------------------------------------------------------
-template <int Q, bool QUERY, int OFF>
-__device__ __forceinline__ void fold_chunk(const float (&v)[16], const f32x2 (&xq)[HD / 2], const float* coef,
-                                           f32x2 (&dxq)[HD / 2]) {
-  if constexpr (Q < F_CONST_CHUNK) {
-    f32x2 t[4];
+struct FoldColumns {
+  int cb;                        // column block, < 0: none yet
+  f32x2 x[4], dx[4];
+};
+
+__device__ __forceinline__ void fold_add8(unsigned char* dx_token, int block, const f32x2 (&v)[4]) {
+  ulonglong2* p0 = reinterpret_cast<ulonglong2*>(dx_token + 2 * block * CP);
+  ulonglong2* p1 = reinterpret_cast<ulonglong2*>(dx_token + (2 * block + 1) * CP);
+  ulonglong2 a = *p0, b = *p1;
+  a.x = f2_add(a.x, v[0]); a.y = f2_add(a.y, v[1]);
+  b.x = f2_add(b.x, v[2]); b.y = f2_add(b.y, v[3]);
+  *p0 = a;
+  *p1 = b;
+}
+
+// `taddr`: the half slab's 64 columns at this warp's lanes; `loaded` runs once every lane has its values in registers.
+template <bool QUERY, class Loaded>
+__device__ __forceinline__ void fold_half_slab(int hs, uint32_t taddr, const unsigned char* xrow, const float* coef,
+                                               unsigned char* dx_token, FoldColumns& col, Loaded loaded) {
+  if (hs == HALF_CONST) {                // the constant has no gradient
+    loaded();
+    return;
+  }
+  const float* cf = coef + F_BLOCK * hs;
+  float va[2][16];
+  tmem_ld16(taddr, va[0]);
+  // 16 columns: a pair of columns of the block and its eight rows
+  const auto products = [&](int i, f32x2 (&t)[8]) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) t[k] = f2_pack(v[OFF + 2 * k], v[OFF + 2 * k + 1]);
+    for (int r = 0; r < 8; ++r) t[r] = f2_pack(va[i & 1][2 * r], va[i & 1][2 * r + 1]);
     if constexpr (QUERY) {
-      const ulonglong2 ca = *reinterpret_cast<const ulonglong2*>(coef + 8 * Q);
-      const ulonglong2 cb2 = *reinterpret_cast<const ulonglong2*>(coef + 8 * Q + 4);
-      t[0] = f2_mul(t[0], ca.x);
-      t[1] = f2_mul(t[1], ca.y);
-      t[2] = f2_mul(t[2], cb2.x);
-      t[3] = f2_mul(t[3], cb2.y);
-    }
-    if constexpr (Q < F_PAIR_CHUNKS) {
-      constexpr PairCursor pc = pair_pos(Q);
-      constexpr int nv = pc.valid();
-      float xlo, xhi;
-      f2_unpack(xq[pc.r / 2], xlo, xhi);
-      const f32x2 xr2 = f2_bcast((pc.r & 1) ? xhi : xlo);
-      f32x2 sr2 = 0ull;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (2 * k < nv) {                       // pairs entirely above the diagonal do not exist
-          if (2 * k + 1 >= nv) {                // the pair straddles the diagonal: drop its upper element
-            float lo, hi;
-            f2_unpack(t[k], lo, hi);
-            t[k] = f2_pack(lo, 0.f);
-          }
-          sr2 = f2_fma(t[k], xq[4 * pc.cb + k], sr2);
-          dxq[4 * pc.cb + k] = f2_fma(t[k], xr2, dxq[4 * pc.cb + k]);
-        }
+      for (int r = 0; r < 8; r += 2) {
+        const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(cf + 16 * i + 2 * r);
+        t[r] = f2_mul(t[r], c.x);
+        t[r + 1] = f2_mul(t[r + 1], c.y);
       }
-      float slo, shi, dlo, dhi;
-      f2_unpack(sr2, slo, shi);
-      f2_unpack(dxq[pc.r / 2], dlo, dhi);
-      if (pc.r & 1) dhi += slo + shi;
-      else dlo += slo + shi;
-      dxq[pc.r / 2] = f2_pack(dlo, dhi);
-    } else {
-      const f32x2 one2 = f2_bcast(1.f);
+    }
+  };
+  if (hs == HALF_LINEAR) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        dxq[4 * (Q - F_LIN_CHUNK0) + k] = f2_fma(t[k], one2, dxq[4 * (Q - F_LIN_CHUNK0) + k]);
+    for (int i = 0; i < 4; ++i) {
+      tmem_ld_wait();
+      if (i < 3) tmem_ld16(taddr + 16 * (i + 1), va[(i + 1) & 1]);
+      else loaded();
+      f32x2 t[8];
+      products(i, t);
+      const f32x2 lo[4] = {t[0], t[1], t[2], t[3]}, hi[4] = {t[4], t[5], t[6], t[7]};
+      fold_add8(dx_token, 2 * i, lo);
+      fold_add8(dx_token, 2 * i + 1, hi);
+    }
+    return;
+  }
+  const HalfBlock blk = half_block(hs);
+  if (blk.cb != col.cb) {
+    if (col.cb >= 0) fold_add8(dx_token, col.cb, col.dx);
+    col.cb = blk.cb;
+    const uint4 c4 = *reinterpret_cast<const uint4*>(xrow + blk.cb * CP);
+    const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      col.x[k] = f2_pack(bf16_lo(cw[k]), bf16_hi(cw[k]));
+      col.dx[k] = 0ull;
     }
   }
-}
-
-// Eight chunks = four 16-column loads; the next load is in flight while the previous one is folded.
-template <int S, int HALF, bool QUERY>
-__device__ __forceinline__ void fold_half_slab_impl(uint32_t taddr, const f32x2 (&xq)[HD / 2], const float* coef,
-                                                    f32x2 (&dxq)[HD / 2]) {
-  constexpr int Q0 = S * 16 + HALF * 8;
-  float va[16], vb[16];
-  tmem_ld16(taddr + HALF * 64, va);
-  tmem_ld_wait();
-  tmem_ld16(taddr + HALF * 64 + 16, vb);
-  fold_chunk<Q0 + 0, QUERY, 0>(va, xq, coef, dxq);
-  fold_chunk<Q0 + 1, QUERY, 8>(va, xq, coef, dxq);
-  tmem_ld_wait();
-  tmem_ld16(taddr + HALF * 64 + 32, va);
-  fold_chunk<Q0 + 2, QUERY, 0>(vb, xq, coef, dxq);
-  fold_chunk<Q0 + 3, QUERY, 8>(vb, xq, coef, dxq);
-  tmem_ld_wait();
-  tmem_ld16(taddr + HALF * 64 + 48, vb);
-  fold_chunk<Q0 + 4, QUERY, 0>(va, xq, coef, dxq);
-  fold_chunk<Q0 + 5, QUERY, 8>(va, xq, coef, dxq);
-  tmem_ld_wait();
-  fold_chunk<Q0 + 6, QUERY, 0>(vb, xq, coef, dxq);
-  fold_chunk<Q0 + 7, QUERY, 8>(vb, xq, coef, dxq);
-}
-
-template <bool QUERY>
-__device__ __forceinline__ void fold_half_slab(int s, int half, uint32_t taddr, const f32x2 (&xq)[HD / 2],
-                                               const float* coef, f32x2 (&dxq)[HD / 2]) {
-#define OAL_CASE(S)                                                                    \
-  case S:                                                                              \
-    if (half == 0) fold_half_slab_impl<S, 0, QUERY>(taddr, xq, coef, dxq);             \
-    else fold_half_slab_impl<S, 1, QUERY>(taddr, xq, coef, dxq);                       \
-    break;
-  OAL_SLAB_SWITCH(s, OAL_CASE)
-#undef OAL_CASE
+  const uint4 r4 = *reinterpret_cast<const uint4*>(xrow + blk.rb * CP);
+  const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
+  f32x2 xr[8], sum[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) xr[j] = f2_bcast((j & 1) ? bf16_hi(rw[j / 2]) : bf16_lo(rw[j / 2]));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    tmem_ld_wait();
+    if (i < 3) tmem_ld16(taddr + 16 * (i + 1), va[(i + 1) & 1]);
+    else loaded();
+    f32x2 t[8];
+    products(i, t);
+    f32x2 other = f2_mul(t[7], xr[7]);         // two chains
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      sum[r] = i ? f2_fma(t[r], col.x[i], sum[r]) : f2_mul(t[r], col.x[i]);
+      if (r & 1) { if (r < 7) other = f2_fma(t[r], xr[r], other); }
+      else col.dx[i] = f2_fma(t[r], xr[r], col.dx[i]);
+    }
+    col.dx[i] = f2_add(col.dx[i], other);
+  }
+  f32x2 rows[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float a0, a1, b0, b1;
+    f2_unpack(sum[2 * k], a0, a1);
+    f2_unpack(sum[2 * k + 1], b0, b1);
+    rows[k] = f2_pack(a0 + a1, b0 + b1);
+  }
+  fold_add8(dx_token, blk.rb, rows);
 }
 
 // ---------------------------------------------------------------------------
 // feature_grad: persistent, warp-specialised.  Work items are (batch, head, chunk) with the heads of
 // one state unit adjacent; CTA k takes items k, k + gridDim.x, ...  Roles:
 //   warps 0-7  fold: thread = (token, half of the slab's 128 features); drains dphi of slab `s` from
-//              tensor memory (three buffers) into its packed dx row; halves are combined per item
+//              tensor memory (four buffers) into its dx row in shared memory; halves are combined per item
 //   warp  8    lane 0 issues  dphi[s] = A . S[s]^T  (M = tokens, N = 128 features, K = 80)
-//   warp  9    lane 0 streams the state slab images (4-slot ring) and, per item, the A operand
+//   warp  9    lane 0 streams the state slab images (four slots) and, per item, the A operand
 //              image (QUERY: the image of G) and the head's coefficient table (two buffers each)
+// A state slot and a dphi buffer share their index and one barrier per direction (see cross_read_kernel).
+// What bounds it: the fold's instruction latency (two warps per scheduler, 1500 clocks per slab; the MMAs are four slabs
+// ahead).  14 / 2 heads, B = 4, N = 4096: 187 -> 166 us (QUERY), 38 -> 33 (not).
 // KEY: the A operand [v | 1] is built in shared memory by the fold warps.
 // ---------------------------------------------------------------------------
 struct FeatGradArgs {
@@ -416,7 +454,7 @@ struct FeatGradArgs {
 
 constexpr int FG_FOLD_WARPS = 8, FG_ISSUER = FG_FOLD_WARPS, FG_LOADER = FG_ISSUER + 1;
 constexpr int FG_THREADS = (FG_LOADER + 1) * 32;
-constexpr int FG_SRING = 4, FG_DRING = 3;
+constexpr int FG_RING = 4;
 
 struct FgItem {
   int b, h, c;
@@ -434,12 +472,12 @@ __device__ __forceinline__ FgItem fg_item(int item, int H, int rep, int NC, int 
 template <bool QUERY>
 __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatGradArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* Sbuf = smem;                                        // FG_SRING x SLAB_S_BYTES
-  unsigned char* Aimg = Sbuf + FG_SRING * SLAB_S_BYTES;              // 2 x SLAB_S_BYTES: [10][128 tokens][8 e]
+  unsigned char* Sbuf = smem;                                        // FG_RING x SLAB_S_BYTES
+  unsigned char* Aimg = Sbuf + FG_RING * SLAB_S_BYTES;              // 2 x SLAB_S_BYTES: [10][128 tokens][8 e]
   float* coef_s = reinterpret_cast<float*>(Aimg + 2 * SLAB_S_BYTES); // 2 x F_ROWS
-  float* red = coef_s + 2 * F_ROWS;                                  // [128][65]
-  __shared__ uint64_t s_full[FG_SRING], s_free[FG_SRING], a_full[2], a_free[2], coef_full[2], coef_free[2];
-  __shared__ uint64_t d_full[FG_DRING], d_free[FG_DRING];
+  unsigned char* ximg = reinterpret_cast<unsigned char*>(coef_s + 2 * F_ROWS);     // rows of x
+  unsigned char* dx_s = ximg + X_BYTES;                              // per half: [16][128 tokens][4] fp32, plane pitch CP
+  __shared__ uint64_t ready[FG_RING], done[FG_RING], a_full[2], a_free[2], coef_full[2], coef_free[2];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -447,9 +485,9 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
   const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   if (warp == FG_ISSUER) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
-    for (int s = 0; s < FG_SRING; ++s) {
-      mbar_init(&s_full[s], 1);
-      mbar_init(&s_free[s], 1);
+    for (int s = 0; s < FG_RING; ++s) {
+      mbar_init(&ready[s], FG_FOLD_WARPS + 1);
+      mbar_init(&done[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&a_full[s], QUERY ? 1 : FG_FOLD_WARPS);
@@ -457,13 +495,13 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
       mbar_init(&coef_full[s], 1);
       mbar_init(&coef_free[s], FG_FOLD_WARPS);
     }
-    for (int s = 0; s < FG_DRING; ++s) {
-      mbar_init(&d_full[s], 1);
-      mbar_init(&d_free[s], FG_FOLD_WARPS);
-    }
     mbar_fence_init();
     dead = 0;
   }
+  // the last block of columns is not copied: zeros for both operands
+  for (int x = tid; x < (FG_RING + 2) * CT; x += FG_THREADS)
+    *reinterpret_cast<uint4*>(Sbuf + (x / CT) * SLAB_S_BYTES + SLAB_U_BYTES + (x % CT) * 16) = make_uint4(0u, 0u, 0u, 0u);
+  fence_async_smem();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -472,121 +510,136 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
 
   if (warp < FG_FOLD_WARPS) {
     // ---------------- fold warps ----------------
-    const int wg = warp >> 2, token = 32 * (warp & 3) + lane;
+    constexpr int T = FG_FOLD_WARPS * 32, PIECES = CT * 8 / T;
+    const int half = warp >> 2, token = 32 * (warp & 3) + lane;
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
+    const unsigned char* xrow = ximg + token * 16;
+    unsigned char* dx_token = dx_s + half * 16 * CP + token * 16;
+    uint4 next[PIECES];                                   // this thread's share of the next item's rows
+    const auto fetch = [&](int k) {
+      const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
+      const __nv_bfloat16* src = a.x + ((size_t)(it.b * a.H + it.h) * a.N + it.c * CT) * HD;
+#pragma unroll
+      for (int j = 0; j < PIECES; ++j) {
+        const int x = tid + j * T;
+        next[j] = (x >> 3) < a.N - it.c * CT ? *reinterpret_cast<const uint4*>(src + 8 * x) : make_uint4(0u, 0u, 0u, 0u);
+      }
+    };
+    const auto store_rows = [&]() {
+#pragma unroll
+      for (int j = 0; j < PIECES; ++j) {
+        const int x = tid + j * T;
+        *reinterpret_cast<uint4*>(ximg + (x & 7) * CP + (x >> 3) * 16) = next[j];
+      }
+    };
+    if (my_items > 0) fetch(0);
+    store_rows();
+    for (int x = tid; x < 2 * 16 * CP / 16; x += T) reinterpret_cast<uint4*>(dx_s)[x] = make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
+    if (lane == 0)
+      for (int x = 0; x < FG_RING; ++x) mbar_arrive(&ready[x]);         // the dphi buffers are empty
     int ds = 0, duse = 0;
     for (int k = 0; k < my_items; ++k) {
       const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
-      const int i = it.c * CT + token;
       const size_t head_off = (size_t)(it.b * a.H + it.h) * a.N;
-      f32x2 xq[HD / 2], dxq[HD / 2];
-      {
-        uint32_t xp[HD / 2];
-        load_row_packed(xp, a.x + head_off * HD, i, a.N);
-        unpack_row(xp, xq);
-      }
-#pragma unroll
-      for (int d = 0; d < HD / 2; ++d) dxq[d] = 0ull;
       if (!QUERY) {
         // A operand [v | 1] of this item, once the MMAs of item k-2 have left the buffer
         if (k >= 2) w.wait(&a_free[k & 1], ((k >> 1) - 1) & 1, 0x51);
         uint4* dst = reinterpret_cast<uint4*>(Aimg + (k & 1) * SLAB_S_BYTES);
-        for (int idx = tid; idx < (EP / 8) * CT; idx += FG_FOLD_WARPS * 32) {
+        for (int idx = tid; idx < (EP / 8) * CT; idx += T) {
           const int ec = idx >> 7, t = idx & 127, j = it.c * CT + t;
           dst[idx] = u_image_chunk(a.v + (head_off + j) * VD, ec, j < a.N);
         }
         fence_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&a_full[k & 1]);
+        warp_arrive(&a_full[k & 1], lane);
       }
+      if (k + 1 < my_items) fetch(k + 1);
       const float* coef = coef_s + (k & 1) * F_ROWS;
       if (QUERY) w.wait(&coef_full[k & 1], (k >> 1) & 1, 0x52);
+      FoldColumns col;
+      col.cb = -1;
       for (int s = 0; s < F_SLABS; ++s) {
-        w.wait(&d_full[ds], duse & 1, 0x53);
+        w.wait(&done[ds], duse & 1, 0x53);
+        __syncwarp();
         fence_after_sync();
-        fold_half_slab<QUERY>(s, wg, tmem + ds * 128 + lane_off, xq, coef, dxq);
-        fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&d_free[ds]);
-        if (++ds == FG_DRING) { ds = 0; ++duse; }
+        fold_half_slab<QUERY>(2 * s + half, tmem + ds * 128 + 64 * half + lane_off, xrow, coef, dx_token, col, [&]() {
+          fence_before_sync();
+          warp_arrive(&ready[ds], lane);
+        });
+        if (++ds == FG_RING) { ds = 0; ++duse; }
       }
-      if (QUERY) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&coef_free[k & 1]);
-      }
-      // combine the two halves of every token and write
-      float dx[HD];
+      if (QUERY) warp_arrive(&coef_free[k & 1], lane);
+      fold_add8(dx_token, col.cb, col.dx);
+      asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
+      // the halves of every token together, whole rows per warp, and zeros for the next item
+      store_rows();
 #pragma unroll
-      for (int d = 0; d < HD / 2; ++d) f2_unpack(dxq[d], dx[2 * d], dx[2 * d + 1]);
-      if (wg == 1) {
-#pragma unroll
-        for (int d = 0; d < HD; ++d) red[token * 65 + d] = dx[d];
+      for (int j = 0; j < 2 * PIECES; ++j) {
+        const int x = tid + j * T, row = x >> 4;
+        float4* p = reinterpret_cast<float4*>(dx_s + (x & 15) * CP + row * 16);
+        float4* p2 = reinterpret_cast<float4*>(dx_s + (16 + (x & 15)) * CP + row * 16);
+        const float4 u = *p, v = *p2;
+        *p = *p2 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (it.c * CT + row < a.N && !dead)
+          *reinterpret_cast<float4*>(a.dx + (head_off + it.c * CT) * HD + 4 * x) = make_float4(u.x + v.x, u.y + v.y, u.z + v.z, u.w + v.w);
       }
-      asm volatile("bar.sync 1, %0;" ::"n"(FG_FOLD_WARPS * 32) : "memory");
-      if (wg == 0 && i < a.N && !dead) {
-        float* dst = a.dx + (head_off + i) * HD;
-#pragma unroll
-        for (int d4 = 0; d4 < HD; d4 += 4)
-          *reinterpret_cast<float4*>(dst + d4) =
-              make_float4(dx[d4] + red[token * 65 + d4], dx[d4 + 1] + red[token * 65 + d4 + 1],
-                          dx[d4 + 2] + red[token * 65 + d4 + 2], dx[d4 + 3] + red[token * 65 + d4 + 3]);
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(FG_FOLD_WARPS * 32) : "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
     }
   } else if (warp == FG_ISSUER) {
     // ---------------- MMA issue ----------------
     if (elect_one()) {
       const uint32_t idesc = instr_desc_bf16(128, 128, 0, 0);
       const uint64_t da0 = smem_desc(smem_u32(Aimg), CT * 16, 128), ds0 = smem_desc(smem_u32(Sbuf), 128 * 16, 128);
-      int gs = 0, guse = 0, ds = 0, duse = 0;
+      int s4 = 0, use = 0;
       for (int k = 0; k < my_items; ++k) {
         const uint64_t da = desc_advance(da0, (k & 1) * SLAB_S_BYTES);
         w.wait(&a_full[k & 1], (k >> 1) & 1, 0x54);
         for (int s = 0; s < F_SLABS; ++s) {
-          const uint64_t dsl = desc_advance(ds0, gs * SLAB_S_BYTES);
-          w.wait(&s_full[gs], guse & 1, 0x55);
-          if (duse > 0) w.wait(&d_free[ds], (duse - 1) & 1, 0x56);
+          const uint64_t dsl = desc_advance(ds0, s4 * SLAB_S_BYTES);
+          w.wait(&ready[s4], use & 1, 0x55);
           fence_after_sync();
 #pragma unroll
           for (int ks = 0; ks < EP / 16; ++ks)
-            mma_bf16_ss(tmem + ds * 128, desc_advance(da, ks * 2 * CT * 16), desc_advance(dsl, ks * 2 * 128 * 16), idesc,
+            mma_bf16_ss(tmem + s4 * 128, desc_advance(da, ks * 2 * CT * 16), desc_advance(dsl, ks * 2 * 128 * 16), idesc,
                         ks > 0);
-          mma_commit(&d_full[ds]);
-          mma_commit(&s_free[gs]);
-          if (s == F_SLABS - 1) mma_commit(&a_free[k & 1]);
-          if (++gs == FG_SRING) { gs = 0; ++guse; }
-          if (++ds == FG_DRING) { ds = 0; ++duse; }
+          mma_commit(&done[s4]);
+          if (++s4 == FG_RING) { s4 = 0; ++use; }
         }
+        mma_commit(&a_free[k & 1]);
       }
     }
     __syncwarp();
   } else {
     // ---------------- image / table stream ----------------
     if (elect_one()) {
-      int gs = 0, guse = 0;
+      int s4 = 0, use = 0;
+      const auto fetch_item = [&](int k) {
+        const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
+        if (k >= 2) {
+          w.wait(&a_free[k & 1], ((k >> 1) - 1) & 1, 0x57);
+          w.wait(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x58);
+        }
+        mbar_arrive_expect_tx(&a_full[k & 1], SLAB_U_BYTES);
+        bulk_g2s(Aimg + (k & 1) * SLAB_S_BYTES,
+                 reinterpret_cast<const unsigned char*>(a.gimg) + ((size_t)(it.b * a.H + it.h) * a.NB + it.c) * SLAB_S_BYTES,
+                 SLAB_U_BYTES, &a_full[k & 1]);
+        mbar_arrive_expect_tx(&coef_full[k & 1], F_ROWS * (uint32_t)sizeof(float));
+        bulk_g2s(coef_s + (k & 1) * F_ROWS, a.coef_table + (size_t)it.h * F_ROWS, F_ROWS * (uint32_t)sizeof(float),
+                 &coef_full[k & 1]);
+      };
+      if (QUERY && my_items > 0) fetch_item(0);
       for (int k = 0; k < my_items; ++k) {
         const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         const int unit = (it.b * a.H + it.h) / a.rep;
         const unsigned char* img = reinterpret_cast<const unsigned char*>(a.image) +
                                    ((size_t)unit * a.NB + it.c) * F_SLABS * SLAB_S_BYTES;
-        if (QUERY) {
-          if (k >= 2) {
-            w.wait(&a_free[k & 1], ((k >> 1) - 1) & 1, 0x57);
-            w.wait(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x58);
-          }
-          mbar_arrive_expect_tx(&a_full[k & 1], SLAB_S_BYTES);
-          bulk_g2s(Aimg + (k & 1) * SLAB_S_BYTES,
-                   reinterpret_cast<const unsigned char*>(a.gimg) + ((size_t)(it.b * a.H + it.h) * a.NB + it.c) * SLAB_S_BYTES,
-                   SLAB_S_BYTES, &a_full[k & 1]);
-          mbar_arrive_expect_tx(&coef_full[k & 1], F_ROWS * (uint32_t)sizeof(float));
-          bulk_g2s(coef_s + (k & 1) * F_ROWS, a.coef_table + (size_t)it.h * F_ROWS, F_ROWS * (uint32_t)sizeof(float),
-                   &coef_full[k & 1]);
-        }
         for (int s = 0; s < F_SLABS; ++s) {
-          if (guse > 0) w.wait(&s_free[gs], (guse - 1) & 1, 0x59);
-          mbar_arrive_expect_tx(&s_full[gs], SLAB_S_BYTES);
-          bulk_g2s(Sbuf + gs * SLAB_S_BYTES, img + (size_t)s * SLAB_S_BYTES, SLAB_S_BYTES, &s_full[gs]);
-          if (++gs == FG_SRING) { gs = 0; ++guse; }
+          // the next item's operand and table while there is time: their buffers' last reader was item k-1
+          if (QUERY && s == 2 * F_SLABS / 3 && k + 1 < my_items) fetch_item(k + 1);
+          if (use > 0) w.wait(&done[s4], (use - 1) & 1, 0x59);
+          mbar_arrive_expect_tx(&ready[s4], SLAB_U_BYTES);
+          bulk_g2s(Sbuf + s4 * SLAB_S_BYTES, img + (size_t)s * SLAB_S_BYTES, SLAB_U_BYTES, &ready[s4]);
+          if (++s4 == FG_RING) { s4 = 0; ++use; }
         }
       }
     }
@@ -764,22 +817,20 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
 cudaError_t dstate_heads(const void* q, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
                          float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, int c0, int NC, float scale,
                          int32_t* status, cudaStream_t st) {
-  const int smem = DS_RING * SLAB_A_BYTES + DS_GRING * SLAB_S_BYTES;
-  cudaError_t e = allow_smem<dstate_heads_kernel>(smem);
+  cudaError_t e = allow_smem<dstate_heads_kernel>(DS_SMEM);
   if (e != cudaSuccess) return e;
   const int sms = sm_count(), items = F_SLABS * NC * B * Hkv;
   DStateArgs a{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(gimg),
                static_cast<const __nv_bfloat16*>(carry_img), static_cast<const __nv_bfloat16*>(carry_lo), coef_table,
                dcarry, dcoef_partial, N, NB, Hq, Hkv, B * Hkv, c0, NC, scale, status};
-  dstate_heads_kernel<<<items < sms ? items : sms, DS_THREADS, smem, st>>>(a);
+  dstate_heads_kernel<<<items < sms ? items : sms, DS_THREADS, DS_SMEM, st>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t feature_grad(bool query, const void* x, const void* gimg, const void* v, const void* image,
                          const float* coef_table, float* dx, int B, int H, int rep, int N, int NB, int c0, int NC,
                          int32_t* status, cudaStream_t st) {
-  const int smem = FG_SRING * SLAB_S_BYTES + 2 * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float) +
-                   128 * 65 * (int)sizeof(float);
+  const int smem = FG_RING * SLAB_S_BYTES + 2 * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float) + X_BYTES + 2 * 16 * CP;
   FeatGradArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gimg),
                  static_cast<const __nv_bfloat16*>(v), static_cast<const __nv_bfloat16*>(image), coef_table, dx,
                  N, NB, H, rep, B, c0, NC, status};
