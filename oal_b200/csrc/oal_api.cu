@@ -457,6 +457,7 @@ float* saved_coef_table(const OalProblem* p, const void* saved_state) {
 struct BackwardSpaceTC {
   float* coef_blocks;            // coefficient partial sums of the query row blocks
   void* gimg;
+  void *q_image, *k_image, *u_image;      // rows of q, k and [v | 1] as operand images
   float* dcarry;
   void* dt_img;
   float* dcoef_partial;
@@ -475,8 +476,11 @@ BackwardSpaceTC carve_backward_tc(const OalProblem* p, void* ws) {
   const size_t qrows = (size_t)p->batch * p->q_heads * p->seq_len;
   const size_t krows = (size_t)p->batch * p->kv_heads * p->seq_len;
   const size_t slab_image = oal::state_slab_image_bytes();
-  s.coef_blocks = c.take<float>((size_t)p->batch * p->q_heads * oal::intra_row_blocks(p->seq_len) * oal::NQ_ALL);
+  s.coef_blocks = c.take<float>((size_t)p->batch * p->q_heads * oal::intra_row_blocks(p->seq_len) * (1 + p->groups + p->groups * (p->groups + 1) / 2));
   s.gimg = c.take<char>(2 * (size_t)p->batch * p->q_heads * nb * slab_image);   // hi image, then lo image
+  s.q_image = c.take<char>((size_t)p->batch * p->q_heads * nb * oal::ROW_IMAGE_BYTES);
+  s.k_image = c.take<char>(units * nb * oal::ROW_IMAGE_BYTES);
+  s.u_image = c.take<char>(units * nb * slab_image);
   s.dcarry = c.take<float>(units * nb * oal::state_rows() * oal::EP);
   s.dt_img = c.take<char>(units * nb * oal::state_image_bytes_per_chunk());
   s.dcoef_partial = c.take<float>(2 * (size_t)p->batch * nb * p->q_heads * oal::state_rows());   // two column halves
@@ -494,20 +498,24 @@ BackwardSpaceTC carve_backward_tc(const OalProblem* p, void* ws) {
 
 // Stage A of the tensor-core backward: everything that does not depend on later tokens' state
 // gradient (normalisation VJP, per-chunk dCarry and coefficient partial sums).
+oal::RowImages row_images(const BackwardSpaceTC& s, const void* q, const void* k, const void* v) {
+  return oal::RowImages{q, k, v, s.q_image, s.k_image, s.u_image};
+}
 int backward_vjp(const OalProblem* p, const float* num, const float* den, const void* grad_out, const float* grad_num,
-                 const float* grad_den, const BackwardSpaceTC& s, int32_t* clear_status, cudaStream_t st) {
+                 const float* grad_den, const BackwardSpaceTC& s, const oal::RowImages& rows, int32_t* clear_status, cudaStream_t st) {
   LaunchScope scope("norm_vjp", st);
-  const cudaError_t e = oal::norm_vjp_image(grad_out, p->out_dtype, grad_num, grad_den, num, den, p->floor,
-                                            s.gimg, p->batch * p->q_heads, p->seq_len, chunk_count(p),
-                                            (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) ? p->q_heads : 0, clear_status, st);
+  const cudaError_t e = oal::norm_vjp_image(grad_out, p->out_dtype, grad_num, grad_den, num, den, p->floor, s.gimg,
+                                            rows.q ? p->batch * p->q_heads : 0, p->seq_len, chunk_count(p),
+                                            (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) ? p->q_heads : 0, rows, p->batch * p->kv_heads,
+                                            clear_status, st);
   return e == cudaSuccess ? OAL_OK : fail_cuda(e, "normalisation VJP kernel");
 }
-int backward_dstate(const OalProblem* p, const void* q, const void* saved_state, const ChunkRange& cr, const BackwardSpaceTC& s,
+int backward_dstate(const OalProblem* p, const void* saved_state, const ChunkRange& cr, const BackwardSpaceTC& s,
                     int32_t* status, cudaStream_t st) {
   const bool want_c = p->grad_mask & OAL_GRAD_COEF;
   if (!(p->grad_mask & (OAL_GRAD_K | OAL_GRAD_V | OAL_GRAD_COEF)) || cr.n == 0) return OAL_OK;
   LaunchScope scope("dstate_heads", st);
-  const cudaError_t e = oal::dstate_heads(q, s.gimg, want_c ? saved_state : nullptr,
+  const cudaError_t e = oal::dstate_heads(s.q_image, s.gimg, want_c ? saved_state : nullptr,
                                           want_c ? saved_remainders(p, saved_state) : nullptr, saved_coef_table(p, saved_state),
                                           s.dcarry, want_c ? s.dcoef_partial : nullptr, p->batch, p->q_heads, p->kv_heads,
                                           p->seq_len, chunk_count(p), cr.first, cr.n, p->scale, status, st);
@@ -610,14 +618,12 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
 // ---- backward -----------------------------------------------------------------------------------
 // sums of the coefficient partials -> dA, dB, dC, and on to the packed factor
 int finish_coefs(const OalProblem* p, const CoefSource& src, const CoefSink& sink, const float* partial, const float* slots,
-                 const void* factors, cudaStream_t st) {
+                 bool chunked, cudaStream_t st) {
   cudaError_t e;
-  const bool fused = factors && sink.dfactor && src.factor_rows == p->q_heads;
+  const bool fused = chunked && sink.dfactor && src.factor_rows == p->q_heads;
   { LaunchScope scope("reduce_coefs", st);
-    const int rm = p->groups + 1;
-    e = factors ? oal::intra_coef_finish(partial, oal::intra_row_blocks(p->seq_len), rm * (rm + 1) / 2 + rm + 1, rm, factors, slots, p->batch,
-                                         p->q_heads, p->groups, sink.dA, sink.dB, sink.dC, fused ? src.factor : nullptr,
-                                         fused ? sink.dfactor : nullptr, st)
+    e = chunked ? oal::intra_coef_finish(partial, oal::intra_row_blocks(p->seq_len), slots, p->batch, p->q_heads, p->groups, sink.dA,
+                                         sink.dB, sink.dC, fused ? src.factor : nullptr, fused ? sink.dfactor : nullptr, st)
                 : oal::reduce_coefs(partial, coef_slots_pairs(p), slots, p->batch, p->q_heads, p->groups,
                                     sink.dA, sink.dB, sink.dC, st); }
   if (e != cudaSuccess) return fail_cuda(e, "coefficient reduction kernel");
@@ -683,7 +689,7 @@ int backward_core_fp32(const OalProblem* p, const BackwardArgs& x, const CoefSou
     kv.mark();
   }
   if (mask & OAL_GRAD_COEF)
-    if (int rc = finish_coefs(p, src, sink, s.coef_pairs, nullptr, nullptr, st)) return rc;
+    if (int rc = finish_coefs(p, src, sink, s.coef_pairs, nullptr, false, st)) return rc;
   kv.wait();
   return OAL_OK;
 }
@@ -706,10 +712,14 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   const ChunkRange cr = chunk_range(p, nullptr, x.dstate_in);
   const void* factors = saved_factors(p, x.saved_state);      // written by the forward of this call
   const float* coef_table = saved_coef_table(p, x.saved_state);
+  const oal::RowImages rows = row_images(s, x.q, x.k, x.v);
   cudaError_t e;
   if (!reuse) {
-    if (int rc = backward_vjp(p, x.num, x.den, x.grad_out, x.grad_num, x.grad_den, s, x.clear_status ? x.status : nullptr, st)) return rc;
-    if (int rc = backward_dstate(p, x.q, x.saved_state, cr, s, x.status, st)) return rc;
+    if (int rc = backward_vjp(p, x.num, x.den, x.grad_out, x.grad_num, x.grad_den, s, rows, x.clear_status ? x.status : nullptr, st)) return rc;
+    if (int rc = backward_dstate(p, x.saved_state, cr, s, x.status, st)) return rc;
+  } else {
+    // oal_backward_local_state left the images of q and G; it has not seen k and v
+    if (int rc = backward_vjp(p, x.num, x.den, nullptr, nullptr, nullptr, s, row_images(s, nullptr, x.k, x.v), nullptr, st)) return rc;
   }
   // Three chains leave the state stage: the query side (on the caller's stream), the key/value side and
   // the reduction of the cross-chunk coefficient gradient.  They share no buffer, so the last two run on
@@ -732,7 +742,7 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
     if (e != cudaSuccess) return fail_cuda(e, "reverse state scan kernel");
     if (want_k) {
       { LaunchScope scope("feature_grad_k", skv);
-        e = oal::feature_grad(false, x.k, nullptr, x.v, s.dt_img, nullptr, s.dk_cross, p->batch, p->kv_heads, 1,
+        e = oal::feature_grad(false, s.k_image, s.u_image, s.dt_img, nullptr, s.dk_cross, p->batch, p->kv_heads, 1,
                               p->seq_len, nb, 0, cr.n, x.status, skv); }
       if (e != cudaSuccess) return fail_cuda(e, "key feature gradient kernel");
     }
@@ -745,21 +755,21 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   }
   if (want_q && cross) {
     { LaunchScope scope("feature_grad_q", st);
-      e = oal::feature_grad(true, x.q, s.gimg, nullptr, x.saved_state, coef_table, s.dq_cross, p->batch, p->q_heads,
+      e = oal::feature_grad(true, s.q_image, s.gimg, x.saved_state, coef_table, s.dq_cross, p->batch, p->q_heads,
                             rep, p->seq_len, nb, cr.first, cr.n, x.status, st); }
     if (e != cudaSuccess) return fail_cuda(e, "query feature gradient kernel");
   }
   if (want_q || want_c) {
     { LaunchScope scope("intra_backward_q", st);
-      e = oal::intra_backward_q(x.q, x.k, x.v, s.gimg, factors, want_q ? x.dq : nullptr, want_q ? s.dq_cross : nullptr,
+      e = oal::intra_backward_q(rows, s.gimg, factors, want_q ? x.dq : nullptr, want_q ? s.dq_cross : nullptr,
                                 want_c ? s.coef_blocks : nullptr, x.status, p->batch, p->q_heads, p->kv_heads,
-                                p->seq_len, nb, p->groups, cr.first, st); }
+                                p->seq_len, nb, p->groups, p->scale, cr.first, st); }
     if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward query-side kernel");
   }
   if (want_kv) {
     // the two intra-chunk kernels each fill the machine: the key/value one is queued after the query one
     { LaunchScope scope("intra_backward_kv", skv, oal::intra_kv_parts(p->batch, p->q_heads, p->kv_heads, nb) > 1 ? 2 : 1);
-      e = oal::intra_backward_kv(x.q, x.k, x.v, s.gimg, factors, want_k ? x.dk : nullptr, want_v ? x.dv : nullptr, s.dk_cross,
+      e = oal::intra_backward_kv(rows, s.gimg, factors, want_k ? x.dk : nullptr, want_v ? x.dv : nullptr, s.dk_cross,
                                  s.dv_cross, cr.n * kChunk, s.dk_part, s.dv_part, x.status, p->batch, p->q_heads, p->kv_heads,
                                  p->seq_len, nb, p->groups, skv); }
     if (e != cudaSuccess) return fail_cuda(e, "intra-chunk backward key/value-side kernels");
@@ -767,7 +777,7 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   }
   if (want_c) {
     cross_coefs.wait();
-    if (int rc = finish_coefs(p, src, sink, s.coef_blocks, cross ? s.slots : nullptr, factors, st)) return rc;
+    if (int rc = finish_coefs(p, src, sink, s.coef_blocks, cross ? s.slots : nullptr, true, st)) return rc;
   }
   kv.wait();
   return OAL_OK;
@@ -1096,8 +1106,8 @@ int oal_backward_local_state(const OalProblem* p, const void* q, const int32_t* 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   OalProblem local = *p;
   local.grad_mask |= OAL_GRAD_K;      // dCarry is needed whatever the caller finally asks for
-  if ((rc = backward_vjp(&local, num, den, grad_out, grad_num, grad_den, s, nullptr, st))) return rc;
-  if ((rc = backward_dstate(&local, q, saved_state, ChunkRange{false, chunk_count(p), 0}, s, status, st))) return rc;
+  if ((rc = backward_vjp(&local, num, den, grad_out, grad_num, grad_den, s, row_images(s, q, nullptr, nullptr), nullptr, st))) return rc;
+  if ((rc = backward_dstate(&local, saved_state, ChunkRange{false, chunk_count(p), 0}, s, status, st))) return rc;
   cudaError_t e;
   { LaunchScope scope("state_total", st);
     e = oal::state_scan(s.dcarry, nullptr, nullptr, nullptr, dstate_total, p->batch * p->kv_heads, chunk_count(p), 1, false, nullptr, 0,

@@ -4,15 +4,11 @@
 // diagonalised by cyclic Jacobi rotations (fp32; the eigenvalues are re-evaluated as Rayleigh quotients
 // of the untouched matrix), one warp per query head, the rotations of a round (disjoint index pairs of
 // a round-robin tournament) applied together.  The result is stored as the
-// table the intra-chunk kernels read (oal_intra.cuh): c_r, l_r[d], the back-transform t and the count
-// of positive terms.  Replaces nothing in the reference, which evaluates the direct form
+// table the intra-chunk kernels read (oal_intra.cuh): c_r, l_r[d] and the count of positive terms.  Replaces nothing in the reference, which evaluates the direct form
 // (oal_attention/grouped_reference.py:61-99); the values of w are the same.
 //
-// intra_coef_finish_kernel: sums the per-(batch row, chunk) partial sums of the query-side backward in
-// fixed order -- D'[r][r'] = 2 sum dW u_r u_r', n'[r] = 2 sum dW u_r, s' = 2 sum dW -- and maps them to
-// dM = sum dW v v^T with v = t u:  dM[a][b] = 1/2 (t D' t^T)[a][b] for a, b >= 1, dM[0][b] = 1/2 (t n')[b]
-// and dM[0][0] = s' / 2 (v_0 = 1 is exact, so its row never goes through the rotation); adds the
-// cross-chunk coefficient gradient of the state kernels and writes dA, dB, dC
+// intra_coef_finish_kernel: sums the per-(batch row, row block) partial sums of the query-side backward in
+// fixed order, adds the cross-chunk coefficient gradient of the state kernels and writes dA, dB, dC
 // (oal_attention/hd_block_gemm_feature_backward.py:59-131 coefficient partials).
 #include "oal_intra.cuh"
 #include "oal_kernels.h"
@@ -170,6 +166,8 @@ __global__ void __launch_bounds__(32) head_factor_kernel(const int32_t* dim_perm
   }
   __syncwarp();
   HeadFactor& out = table[h];
+  write_head_groups(out.e, out.mask, out.order, gdim, dim_perm + h * HD, group_start + h * (GMAX + 1), G, scale,
+                    [&](int g) { return coefB[g]; }, [&](int g, int g2) { return coefC[g * G + g2] + coefC[g2 * G + g]; }, lane, 32);
   if (lane < RMAX_ALL) out.s.c[lane] = lane < n ? lam[lane] * V[0][order[lane]] : 0.f;
   for (int r = 0; r < RMAX_ALL; ++r) {
     const bool live = r < n;
@@ -177,7 +175,6 @@ __global__ void __launch_bounds__(32) head_factor_kernel(const int32_t* dim_perm
     const int col = live ? order[r] : 0;
     out.l[r][lane] = live ? sl * V[1 + gdim[lane]][col] : 0.f;
     out.l[r][lane + 32] = live ? sl * V[1 + gdim[lane + 32]][col] : 0.f;
-    if (lane < RMAX_ALL) out.t[lane][r] = (live && lane < n) ? V[lane][col] / lam[r] : 0.f;
   }
 }
 
@@ -194,29 +191,18 @@ __global__ void deliver_status_kernel(const int32_t* status, StatusSink sink) {
   __threadfence_system();
 }
 
-// partial: [B][Hq][tiles][nu_stride]: entries r <= r' in row-major upper-triangle order of an rm x rm
-// matrix, then the rm sums n'[r], then s'.  One block per head; FINISH_SEGS threads share the tiles of a sum (a
-// serial walk over 512 tiles is 60 us of dependent loads), their parts are added in fixed order.  With `factor`
-// the block goes on from dM to the gradient of its own packed factor row: dL = (S + S^T) L, see
-// expand_factor_grad_kernel.
-constexpr int FINISH_THREADS = 1024, FINISH_SEGS = 16;
-__global__ void __launch_bounds__(FINISH_THREADS) intra_coef_finish_kernel(const float* partial, int tiles, int nu_stride, int rm,
-                                                                const HeadFactor* table, const float* extra, int B,
+// partial: [B][Hq][tiles][1 + G + G (G + 1) / 2]: dA, dB, upper triangle of dC in row-major order.  One block per head;
+// FINISH_SEGS threads share the tiles of a sum (a serial walk over 512 tiles is 60 us of dependent loads), their parts are
+// added in fixed order.  With `factor` the block goes on from dM to the gradient of its own packed factor row:
+// dL = (S + S^T) L, see expand_factor_grad_kernel.
+constexpr int FINISH_THREADS = 1024, FINISH_SEGS = 16, FINISH_SUMS = 1 + GMAX + GMAX * (GMAX + 1) / 2;
+__global__ void __launch_bounds__(FINISH_THREADS) intra_coef_finish_kernel(const float* partial, int tiles, const float* extra, int B,
                                                                 int Hq, int G, float* dA, float* dB, float* dC,
                                                                 const float* factor, float* dfactor) {
-  __shared__ float D[RMAX_ALL][RMAX_ALL];
-  __shared__ float T[RMAX_ALL][RMAX_ALL];
-  __shared__ float X[RMAX_ALL][RMAX_ALL];       // t D', later S + S^T
-  __shared__ float N1[RMAX_ALL + 1];            // n'[r], then s'
-  __shared__ float seg_sum[FINISH_SEGS][NU_ALL + RMAX_ALL + 1];
+  __shared__ float S[RMAX_ALL][RMAX_ALL];       // S[0][0] = dA, S[0][b] = 2 dB, S[a][0] = 0, S[a][b] = dC
+  __shared__ float seg_sum[FINISH_SEGS][FINISH_SUMS];
   const int h = blockIdx.x, tid = threadIdx.x;
-  const int n = G + 1;
-  for (int x = tid; x < RMAX_ALL * RMAX_ALL; x += FINISH_THREADS) {
-    D[x / RMAX_ALL][x % RMAX_ALL] = 0.f;
-    T[x / RMAX_ALL][x % RMAX_ALL] = table[h].t[x / RMAX_ALL][x % RMAX_ALL];
-  }
-  if (tid <= RMAX_ALL) N1[tid] = 0.f;
-  const int nu = rm * (rm + 1) / 2, nv = nu + rm + 1;
+  const int n = G + 1, nv = 1 + G + G * (G + 1) / 2;
   const int outer = B * tiles, per = (outer + FINISH_SEGS - 1) / FINISH_SEGS;
   for (int x = tid; x < nv * FINISH_SEGS; x += FINISH_THREADS) {
     const int v = x % nv, seg = x / nv, o0 = seg * per, o1 = min(outer, o0 + per);
@@ -224,7 +210,7 @@ __global__ void __launch_bounds__(FINISH_THREADS) intra_coef_finish_kernel(const
 #pragma unroll 8
     for (int o = o0; o < o1; ++o) {
       const int b = o / tiles, i = o - b * tiles;
-      t += partial[((size_t)(b * Hq + h) * tiles + i) * nu_stride + v];
+      t += partial[((size_t)(b * Hq + h) * tiles + i) * nv + v];
     }
     seg_sum[seg][v] = t;
   }
@@ -233,40 +219,20 @@ __global__ void __launch_bounds__(FINISH_THREADS) intra_coef_finish_kernel(const
     float t = 0.f;
 #pragma unroll
     for (int seg = 0; seg < FINISH_SEGS; ++seg) t += seg_sum[seg][v];
-    if (v < nu) {
-      int r = 0, rest = v;
-      while (rest >= rm - r) { rest -= rm - r; ++r; }
-      D[r][r + rest] = t;
-      D[r + rest][r] = t;
+    if (v <= G) {
+      if (extra) t += extra[(size_t)h * NCOEF + v];
+      if (v == 0) dA[h] = t;
+      else dB[h * G + v - 1] = t;
+      S[0][v] = v ? 2.f * t : t;
+      if (v) S[v][0] = 0.f;
     } else {
-      N1[v < nu + rm ? v - nu : RMAX_ALL] = t;
+      int g = 0, rest = v - 1 - G;
+      while (rest >= G - g) { rest -= G - g; ++g; }
+      const int g2 = g + rest;
+      if (extra) t += extra[(size_t)h * NCOEF + 1 + GMAX + tri_all(g, g2)];
+      dC[((size_t)h * G + g) * G + g2] = dC[((size_t)h * G + g2) * G + g] = t;
+      S[1 + g][1 + g2] = S[1 + g2][1 + g] = t;
     }
-  }
-  __syncthreads();
-  for (int x = tid; x < n * n; x += FINISH_THREADS) {
-    const int a = x / n, r2 = x % n;
-    float t = 0.f;
-    for (int r = 0; r < n; ++r) t += T[a][r] * D[r][r2];
-    X[a][r2] = t;
-  }
-  __syncthreads();
-  for (int x = tid; x < n * n; x += FINISH_THREADS) {
-    const int a = x / n, b = x % n;
-    float t = 0.f;
-    if (a == 0 && b == 0) t = N1[RMAX_ALL];
-    else if (a == 0 || b == 0) { for (int r = 0; r < n; ++r) t += T[a + b][r] * N1[r]; }
-    else { for (int r2 = 0; r2 < n; ++r2) t += X[a][r2] * T[b][r2]; }
-    t *= 0.5f;
-    if (a == 0 || b == 0) {
-      t += extra ? extra[(size_t)h * NCOEF + a + b] : 0.f;
-    } else {
-      const int g = a - 1, g2 = b - 1;
-      t += extra ? extra[(size_t)h * NCOEF + 1 + GMAX + (g <= g2 ? tri_all(g, g2) : tri_all(g2, g))] : 0.f;
-    }
-    if (a == 0 && b == 0) dA[h] = t;
-    else if (a == 0) dB[h * G + b - 1] = t;
-    else if (b > 0) dC[((size_t)h * G + a - 1) * G + b - 1] = t;
-    D[a][b] = a == 0 && b > 0 ? 2.f * t : (b == 0 && a > 0 ? 0.f : t);      // S
   }
   if (!factor) return;
   __syncthreads();
@@ -276,7 +242,7 @@ __global__ void __launch_bounds__(FINISH_THREADS) intra_coef_finish_kernel(const
     while (rest > i) { rest -= i + 1; ++i; }
     const int k = rest;
     float t = 0.f;
-    for (int j = k; j < n; ++j) t = fmaf(D[i][j] + D[j][i], factor[(size_t)h * P + j * (j + 1) / 2 + k], t);
+    for (int j = k; j < n; ++j) t = fmaf(S[i][j] + S[j][i], factor[(size_t)h * P + j * (j + 1) / 2 + k], t);
     dfactor[(size_t)h * P + x] = t;
   }
 }
@@ -347,14 +313,11 @@ cudaError_t deliver_status(const int32_t* status, StatusSink sink, cudaStream_t 
   return cudaGetLastError();
 }
 
-cudaError_t intra_coef_finish(const float* partial, int tiles, int nu_stride, int rm, const void* table,
-                              const float* extra, int B, int Hq, int G, float* dA, float* dB, float* dC,
-                              const float* factor, float* dfactor, cudaStream_t st) {
-  intra_coef_finish_kernel<<<Hq, FINISH_THREADS, 0, st>>>(partial, tiles, nu_stride, rm, static_cast<const HeadFactor*>(table),
-                                                          extra, B, Hq, G, dA, dB, dC, factor, dfactor);
+cudaError_t intra_coef_finish(const float* partial, int tiles, const float* extra, int B, int Hq, int G, float* dA, float* dB,
+                              float* dC, const float* factor, float* dfactor, cudaStream_t st) {
+  intra_coef_finish_kernel<<<Hq, FINISH_THREADS, 0, st>>>(partial, tiles, extra, B, Hq, G, dA, dB, dC, factor, dfactor);
   return cudaGetLastError();
 }
-
 
 cudaError_t expand_factor(const float* factor, int factor_rows, int Hq, int G, float eps, float* A, float* B, float* C,
                           cudaStream_t st) {

@@ -97,6 +97,9 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
+constexpr int ROW_PLANE = CT * 16;             // one 16-byte piece of every row of a chunk
+constexpr int ROW_IMAGE_BYTES = 8 * ROW_PLANE; // a chunk's rows of 64 as an operand image [8][128][8], zeros past the sequence
+
 // ---- rows in shared memory -----------------------------------------------------------------------
 // Chunk planes of an operand image that threads write: 128 rows of 16 bytes and 16 bytes of padding, so that eight
 // threads that copy one 128-byte row (coalesced) hit eight different bank groups.

@@ -25,8 +25,6 @@
 namespace oal {
 
 constexpr int RMAX_ALL = OAL_MAX_GROUPS + 1;         // 17: extent of the per-head factor table
-constexpr int NU_ALL = RMAX_ALL * (RMAX_ALL + 1) / 2;
-constexpr int NQ_ALL = NU_ALL + RMAX_ALL + 1;        // coefficient partial sums of a row block: D upper triangle, n, s
 constexpr int XA_BYTES = 10 * CP;                    // [v | 1 | 0]
 
 // What a kernel keeps of a head's table besides l.
@@ -38,11 +36,38 @@ struct HeadScalars {
 };
 static_assert(sizeof(HeadScalars) == 80, "copied in 16-byte pieces");
 
+// Dimensions sorted by group.
+struct HeadOrder {
+  uint8_t pos[HD];                   // position of a dimension
+  uint8_t start[32];                 // first position of group g; 64 from group G on
+};
+static_assert(sizeof(HeadOrder) == 96, "copied in 16-byte pieces");
+
+// What the query side of the backward reads of the groups and coefficients of a head (HeadFactor::e, mask, order), by
+// threads tid of nthreads; `pos` and `group` of every dimension are known, b_of(g) = B_g, c_of(g, g2) = C_gg2 + C_g2g.
+template <class BOf, class COf>
+__device__ __forceinline__ void write_head_groups(float (&e)[RMAX_ALL][HD], uint32_t (&mask)[GMAX][HD / 2], HeadOrder& order,
+                                                  const int* group, const int32_t* dim_perm, const int32_t* group_start, int G,
+                                                  float scale, BOf b_of, COf c_of, int tid, int nthreads) {
+  for (int x = tid; x < (G + 1) * HD; x += nthreads) {
+    const int r = x / HD, g = group[x % HD];
+    e[r][x % HD] = r == 0 ? scale * b_of(g) : scale * scale * c_of(r - 1, g);
+  }
+  for (int x = tid; x < G * (HD / 2); x += nthreads) {
+    const int g = x / (HD / 2), wd = x % (HD / 2);
+    mask[g][wd] = (group[2 * wd] == g ? 0x0000FFFFu : 0u) | (group[2 * wd + 1] == g ? 0xFFFF0000u : 0u);
+  }
+  for (int p = tid; p < HD; p += nthreads) order.pos[dim_perm[p]] = (uint8_t)p;
+  for (int g = tid; g < 32; g += nthreads) order.start[g] = (uint8_t)(g < G ? group_start[g] : HD);
+}
+
 // Per-head factor table in global memory (written by the prologue or head_factor_kernel).
 struct alignas(16) HeadFactor {
   HeadScalars s;
   float l[RMAX_ALL][HD];             // l_r[d], original dimension order
-  float t[RMAX_ALL][RMAX_ALL];       // t[a][r] = V[a][r] / lambda_r  (v = t u)
+  float e[RMAX_ALL][HD];             // of the dimension's group g: e_0 = scale B_g, e_r = scale^2 (C_rg + C_gr)
+  uint32_t mask[GMAX][HD / 2];       // the dimensions of a group, as words of two bf16
+  HeadOrder order;
 };
 
 // Chunks 8 and 9 of the image of [v | 1 | 0]: one in the first element of rows below `valid`, zeros elsewhere.
@@ -65,11 +90,12 @@ __device__ __forceinline__ void load_head(float* l, HeadScalars* sc, const HeadF
 // (columns d0 / 2 ..) and, 32 columns further, the rounding remainders: the scaled side enters u_r with about 16
 // bits.  xrow points at the thread's row in chunk 0 of an image.
 constexpr uint32_t TERM_COLS = 64;
+template <int PITCH = CP>
 __device__ __forceinline__ void build_term16(uint32_t slot, const unsigned char* xrow, const float* l, int d0) {
   uint32_t hw[8], lw[8];
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(xrow + (d0 / 8 + k) * CP);
+    const uint4 raw = *reinterpret_cast<const uint4*>(xrow + (d0 / 8 + k) * PITCH);
     const ulonglong2 la = *reinterpret_cast<const ulonglong2*>(l + d0 + 8 * k);
     const ulonglong2 lb = *reinterpret_cast<const ulonglong2*>(l + d0 + 8 * k + 4);
     const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -89,12 +115,13 @@ __device__ __forceinline__ void build_term16(uint32_t slot, const unsigned char*
 
 // term . rows^T into 128 x n columns, K = 64 for the value and 64 for the remainder operand: `b_addr` is the first of
 // the n rows in an image.  (The kernels add c_r themselves, in fp32.)
+template <int PITCH = CP>
 __device__ __forceinline__ void issue_term(uint32_t tmem_u, uint32_t slot, uint32_t b_addr, int n) {
   const uint32_t idesc = umma::instr_desc_bf16(128, n, 0, 0);
-  const uint64_t db = umma::smem_desc(b_addr, CP, 128);
+  const uint64_t db = umma::smem_desc(b_addr, PITCH, 128);
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks)
-    umma::mma_bf16_ts(tmem_u, slot + 8 * ks, umma::desc_advance(db, (ks & 3) * 2 * CP), idesc, ks > 0);
+    umma::mma_bf16_ts(tmem_u, slot + 8 * ks, umma::desc_advance(db, (ks & 3) * 2 * PITCH), idesc, ks > 0);
 }
 
 // Query-side tiles.  The 128 rows of a CTA are four blocks of 32 query rows, one per tensor-memory lane quadrant,

@@ -1,21 +1,19 @@
 // Intra-chunk term of the chunked scan on the tensor cores (tcgen05 / TMEM), backward.
 //
-// Both kernels walk the terms r of the factored weight (oal_intra.cuh).  The scaled rows are carried as bf16
-// value + bf16 remainder, two MMA chains into u_r: the coefficient gradient is a sum of strongly cancelling terms
-// (sum_j dW_ij w_ij = 0 for every row) and needs u to more than 8 bits, and on the key side the rounding of the
-// scaled keys would act like a perturbation that is the same for every query.
-//
-// Query side (rows are query rows, columns are keys), dW = G [v|1]^T once (G as hi + lo bf16), then per term:
-//   P_r = 2 dW u_r             registers -> tensor memory, bf16 value + remainder
-//   Z_r = P_r K                one accumulator per term;  n_r = sum of P_r, registers
-//   dq  += sgn_r l_r * Z_r     registers (element-wise in the dimension)
+// Query side (rows are query rows, columns are keys).  dW = G [v|1]^T once (G as hi + lo bf16).  The gradient needs the
+// scores of each group, s_g = sum over the group's dims of q k, and no term of the factored weight: with s_0 = 1,
+//   X_r = dW s_r               registers -> tensor memory, bf16 value + remainder,  r = 0 .. G
+//   Z_r = X_r K                one accumulator per r
+//   dq  += e_r * Z_r           element-wise in the dimension d of group g: e_0 = scale B_g, e_r = 2 scale^2 C_rg
 //   y_r  = sum over rows of q * Z_r, one 64-vector per row block
-// The coefficient gradient needs D'[r][r'] = sum_ij 2 dW u_r u_r' = sum_d l_r'[d] y_r[d] + c_r' n_r: 64 sums per
-// term instead of R (R + 1) / 2 products per pair.  P_r's remainder keeps these sums at the 16 bits they had when
-// they were formed from fp32 products.
+// s_g is one MMA chain over the rows of q with the other groups' dims set to zero, exact in bf16.  dB_g and dC_rg are
+// sums of y_0 and y_r over the dims of g: 64 sums per r instead of G (G + 1) / 2 products per pair.  X_r's remainder
+// keeps these strongly cancelling sums (sum_j dW_ij w_ij = 0 for every row) at 16 bits.
 //
-// Key / value side (rows are keys, columns are the queries of one head): per head and term
-//   P_r^T as above (bf16 value; with its remainder above 8 groups),  Z_r = P_r^T Q,  dk += sgn_r l_r * Z_r,  w += sgn_r u_r^2 in registers,
+// Key / value side (rows are keys, columns are the queries of one head): per head and term r of the factored weight
+// (oal_intra.cuh; the scaled rows as bf16 value + remainder: the rounding of the scaled keys alone would act like a
+// perturbation that is the same for every query)
+//   P_r^T = 2 dW^T u_r^T (bf16 value; with its remainder above 8 groups),  Z_r = P_r^T Q,  dk += sgn_r l_r * Z_r,  w += sgn_r u_r^2 in registers,
 // and after the last term dU += W^T G (W as value + remainder, as in the forward: a row's weights and its denominator
 // then agree to 16 bits).  A CTA walks several query heads of its KV head; dk stays in registers, dU
 // in tensor memory, and the next head's operands arrive while the current one is worked on.
@@ -32,13 +30,15 @@ namespace {
 using namespace umma;
 
 struct IntraBwdArgs {
-  const __nv_bfloat16 *q, *k, *v;
-  const __nv_bfloat16* gimg;        // [2][B*Hq, NB, 10, 128, 8]: bf16(g) image, then the image of g - bf16(g)
-  size_t gimg_lo_offset;            // bytes from the hi image to the lo image
+  // operand images: rows of q, k [heads, NB, 8, 128, 8], [v | 1 | 0] and G [heads, NB, 10, 128, 8]
+  const unsigned char *q_image, *k_image, *u_image;
+  const unsigned char* gimg;        // bf16(G), then (gimg_lo_offset bytes on) the images of G - bf16(G)
+  size_t gimg_lo_offset;
   const HeadFactor* factors;
   __nv_bfloat16* dq;                // may be null
   const float* dq_init;             // fp32 cross part, or null
-  float* coef_partial;              // [B][Hq][row blocks][NQ] or null: D upper triangle, n_r, sum 2 dW
+  float* coef_partial;              // [B][Hq][row blocks][1 + G + G (G + 1) / 2] or null: dA, dB, upper triangle of dC
+  float scale;
   // key / value side: fp32 partials [B, Hkv * parts, N, 64] when the heads are spread over `parts` CTAs, else the
   // results with the cross parts of the tokens before cross_end added
   float *dk_part, *dv_part;
@@ -66,331 +66,330 @@ __device__ __forceinline__ void issue_dw(uint32_t tmem_dw, uint64_t rows_hi, uin
   }
 }
 
-// hi / lo bf16 pairs of eight products
-__device__ __forceinline__ void split8(const f32x2 (&t)[4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    float a, b;
-    f2_unpack(t[j], a, b);
-    hi[j] = pack_bf16(a, b);
-    lo[j] = pack_bf16(a - bf16_lo(hi[j]), b - bf16_hi(hi[j]));
-  }
+__device__ __forceinline__ f32x2 f2_shfl_xor(f32x2 v, int o) {
+  float lo, hi;
+  f2_unpack(v, lo, hi);
+  return f2_pack(__shfl_xor_sync(0xffffffffu, lo, o), __shfl_xor_sync(0xffffffffu, hi, o));
 }
 
 // ---------------------------------------------------------------------------
 // query side
 // ---------------------------------------------------------------------------
-// tensor memory: U (two halves of 64; first dW) | P hi (64) | P lo (64) | two Z (64) | two term slots (64)
-constexpr uint32_t BQ_U = 0, BQ_P = 128, BQ_PLO = 192, BQ_Z = 256, BQ_TERM = 384;
-static_assert(BQ_TERM + 2 * TERM_COLS <= 512, "tensor-memory columns of the query-side kernel");
-constexpr int BQ_L_FLOATS = 4 * RMAX_ALL * HD;
-constexpr int BQ_SMEM = 2 * X_BYTES + 3 * XA_BYTES + BQ_L_FLOATS * 4;
-static_assert(BQ_L_FLOATS * 4 <= XA_BYTES, "the y sums take the place of an image of G");
+// What bounds it: the chain score chain -> products -> X -> Z of each r (about 2000 clocks; the MMAs of an r are 1250) and the
+// first and last phase of a tile.  Eight compute warps with 64 keys each, one barrier of theirs per r: it says at once that
+// the scores have been read, X is written, the next masked rows are in place and the Z before last has been drained.
+// 14 / 2 heads, 8 groups, B = 4, N = 4096: 353 -> 204 us against walking the terms of the factored weight (scaled rows as value +
+// remainder, twice the MMA steps, 16 warps with 32 keys each and six barriers per term); of a tile's 32000 clocks 20000 are the
+// loop.
+// Warps 0..7 compute, warp 8 issues; 9..11 only help to load and fill the issuer's warpgroup, whose registers the compute
+// warps take: 384 threads x 168 at launch = 256 x 224 + 128 x 40 and 2048 to spare.
+constexpr int BQ_COMPUTE = 8, BQ_ISSUER = BQ_COMPUTE, BQ_THREADS = (BQ_COMPUTE + 4) * 32;
+// tensor memory: scores (128; first dW) | X hi (64) | X lo (64) | two Z (64) | two slots of masked rows (32)
+constexpr uint32_t BQ_S = 0, BQ_X = 128, BQ_XLO = 192, BQ_Z = 256, BQ_ROWS = 384, BQ_ROW_COLS = 32;
+static_assert(BQ_ROWS + 2 * BQ_ROW_COLS <= 512, "tensor-memory columns of the query-side kernel");
+// shared memory: images of q, k, [v | 1] and G (hi, lo), then of each quadrant's head
+constexpr int BQ_K = ROW_IMAGE_BYTES, BQ_U = BQ_K + ROW_IMAGE_BYTES, BQ_G = BQ_U + SLAB_S_BYTES;
+constexpr int BQ_E = BQ_G + 2 * SLAB_S_BYTES;                           // e_r[d], [quadrant][r][64] fp32
+constexpr int BQ_MASK = BQ_E + 4 * RMAX_ALL * HD * 4;                   // dims of a group, [quadrant][group][32] words of two bf16
+constexpr int BQ_ORDER = BQ_MASK + 4 * GMAX * (HD / 2) * 4;
+constexpr int BQ_SMEM = BQ_ORDER + 4 * (int)sizeof(HeadOrder);
+static_assert(4 * RMAX_ALL * HD * 4 <= 2 * SLAB_S_BYTES, "the y sums take the place of the images of G");
 
-__global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_q_kernel(const IntraBwdArgs a) {
+__global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraBwdArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* Qimg = smem;
-  unsigned char* Kimg = Qimg + X_BYTES;
-  unsigned char* Uimg = Kimg + X_BYTES;
-  unsigned char* Gimg = Uimg + XA_BYTES;                        // hi, lo; dead once dW is complete
-  float* lq = reinterpret_cast<float*>(Gimg + 2 * XA_BYTES);    // [quadrant][term][64]
-  float* ys = reinterpret_cast<float*>(Gimg);                   // [quadrant][term][64]
-  __shared__ __align__(16) HeadScalars sc[4];
-  __shared__ float nq[BW_COMPUTE][RMAX_ALL], sq[BW_COMPUTE];
-  __shared__ uint64_t dw_full, dw_free, u_full[2], u_free[2], term_full[2], p_full[2], z_half[2], z_free[2];
+  float* e_s = reinterpret_cast<float*>(smem + BQ_E);
+  uint32_t* mask_s = reinterpret_cast<uint32_t*>(smem + BQ_MASK);
+  float* ys = reinterpret_cast<float*>(smem + BQ_G);            // [quadrant][r][64], dims sorted by group; G is dead once dW is complete
+  __shared__ float sum_s[BQ_COMPUTE], cls_s[4][RMAX_ALL * GMAX];
+  __shared__ uint64_t in_full, dw_full, s_full, x_full, z_full;
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const QueryTile tile(a.Hkv, a.N, a.rep);
   if (tile.empty()) return;
-  const int qd = warp & 3, sub = (warp >> 2) & 3, row = 32 * qd + lane;
-  const int tok0 = tile.c * CT, cols = tile.columns(), rank = a.rank;
+  const int qd = warp & 3, row = 32 * qd + lane;
+  const int tok0 = tile.c * CT, cols = tile.columns(), G = a.rank - 1;
   const int my_rb = tile.rb(qd), my_head = tile.head(qd);
-  {
-    const size_t koff = ((size_t)tile.b * a.Hkv + tile.kvh) * a.N + tok0;
-    const size_t qoff = ((size_t)tile.b * a.Hq + my_head) * a.N + tok0 + min(32 * my_rb, tile.nc - 1);
-    const int fifth = (warp >> 2) * 32 + lane;                  // five warps load a quadrant's rows and table
-    const unsigned char* gsrc = reinterpret_cast<const unsigned char*>(a.gimg) +
-                                (((size_t)tile.b * a.Hq + my_head) * a.NB + tile.c) * SLAB_S_BYTES + 32 * my_rb * 16;
-    for (int x = fifth; x < 2 * (EP / 8) * 32; x += 160) {
-      const int r = x & 31, e = (x >> 5) % (EP / 8), lo = x >= (EP / 8) * 32;
-      async_copy16(Gimg + lo * XA_BYTES + e * CP + (32 * qd + r) * 16, gsrc + lo * a.gimg_lo_offset + e * (CT * 16) + r * 16, true);
-    }
-    load_rows(Uimg, 0, a.v + koff * VD, cols, tile.nc, tid, BW_THREADS);
-    load_rows(Qimg, 32 * qd, a.q + qoff * HD, 32, max(tile.nc - 32 * my_rb, 0), fifth, 160);
-    load_rows(Kimg, 0, a.k + koff * HD, cols, tile.nc, tid, BW_THREADS);
-    load_head(lq + qd * RMAX_ALL * HD, &sc[qd], a.factors + my_head, rank, fifth, 160);
-  }
-  augment_rows(Uimg, tile.nc, tid, BW_THREADS);
   if (warp == 0) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&u_full[s], 1);
-      mbar_init(&u_free[s], BW_COMPUTE);
-      mbar_init(&term_full[s], BW_COMPUTE);
-      mbar_init(&p_full[s], BW_COMPUTE);
-      mbar_init(&z_half[s], 1);
-      mbar_init(&z_free[s], BW_COMPUTE);
-    }
+    mbar_init(&in_full, 1);
     mbar_init(&dw_full, 1);
-    mbar_init(&dw_free, BW_COMPUTE);
+    mbar_init(&s_full, 1);
+    mbar_init(&x_full, BQ_COMPUTE);
+    mbar_init(&z_full, 1);
     mbar_fence_init();
+    mbar_arrive_expect_tx(&in_full, ROW_IMAGE_BYTES + SLAB_S_BYTES +
+                                        4 * ((8 + 2 * (EP / 8)) * 512 + a.rank * HD * 4 + G * (HD / 2) * 4 + (int)sizeof(HeadOrder)));
     dead = 0;
   }
-  async_copies_wait();
-  fence_async_smem();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
+  if (warp >= BQ_ISSUER) {
+    // a copy per thread: the key side whole, 32 rows of a plane at a time of each quadrant's rows and G, its head's tables
+    constexpr int PER = 8 + 2 * (EP / 8) + 3;
+    static_assert(4 * PER + 2 <= 128, "a copy per thread");
+    const int x = tid - BQ_ISSUER * 32, quadrant = x & 3, y = x >> 2;
+    const size_t unit = ((size_t)tile.b * a.Hkv + tile.kvh) * a.NB + tile.c;
+    const size_t head = ((size_t)tile.b * a.Hq + tile.head(quadrant)) * a.NB + tile.c, rows = 32 * tile.rb(quadrant) * 16;
+    const HeadFactor* f = a.factors + tile.head(quadrant);
+    const int dst = 32 * quadrant * 16;
+    if (y < 8) bulk_g2s(smem + y * ROW_PLANE + dst, a.q_image + head * ROW_IMAGE_BYTES + y * ROW_PLANE + rows, 512, &in_full);
+    else if (y < 8 + 2 * (EP / 8)) {
+      const int lo = y - 8 >= EP / 8, e = y - 8 - lo * (EP / 8);
+      bulk_g2s(smem + BQ_G + lo * SLAB_S_BYTES + e * ROW_PLANE + dst, a.gimg + lo * a.gimg_lo_offset + head * SLAB_S_BYTES + e * ROW_PLANE + rows,
+               512, &in_full);
+    } else if (y == PER - 3) bulk_g2s(e_s + quadrant * RMAX_ALL * HD, &f->e[0][0], a.rank * HD * 4, &in_full);
+    else if (y == PER - 2) bulk_g2s(mask_s + quadrant * GMAX * (HD / 2), &f->mask[0][0], G * (HD / 2) * 4, &in_full);
+    else if (y == PER - 1) bulk_g2s(smem + BQ_ORDER + quadrant * (int)sizeof(HeadOrder), &f->order, (int)sizeof(HeadOrder), &in_full);
+    else if (x == 4 * PER) bulk_g2s(smem + BQ_K, a.k_image + unit * ROW_IMAGE_BYTES, ROW_IMAGE_BYTES, &in_full);
+    else if (x == 4 * PER + 1) bulk_g2s(smem + BQ_U, a.u_image + unit * SLAB_S_BYTES, SLAB_S_BYTES, &in_full);
+  }
   Waiter w{&dead};
   const uint32_t tmem = uniform(tmem_base);
   const uint32_t lane_off = (uint32_t)(32 * qd) << 16;
-  const int na = min(cols, 64), nb2 = cols - na;              // columns of the two halves
   const bool want_coef = a.coef_partial != nullptr;
+  w.wait(&in_full, 0, 0x20);
+  __syncwarp();
 
-  if (warp >= BW_ISSUER) {
-    registers_down_to<24>();
-    if (warp == BW_ISSUER) {
-      const uint32_t k_addr = smem_u32(Kimg), g_addr = smem_u32(Gimg), u_addr = smem_u32(Uimg);
-      if (elect_one()) {
-        const uint64_t du = smem_desc(u_addr, CP, 128), dk = smem_desc(k_addr, 128, CP);
-        issue_dw(tmem + BQ_U, smem_desc(g_addr, CP, 128), smem_desc(g_addr + XA_BYTES, CP, 128), 2 * CP, du, du, 2 * CP, cols);
-        mma_commit(&dw_full);
-        // half hf of the keys of Z_r = (P hi + P lo) K
-        const auto issue_z = [&](int r, int hf) {
-          w.wait(&p_full[hf], r & 1, 0x21);
-          if (hf == 0 && r >= 2) w.wait(&z_free[r & 1], ((r >> 1) - 1) & 1, 0x22);
-          fence_after_sync();
-          const uint32_t z = tmem + BQ_Z + (r & 1) * HD, idesc = instr_desc_bf16(128, HD, 0, 1);
-          const int k0 = hf ? 4 : 0, k1 = hf ? 4 + nb2 / 16 : na / 16;
-          for (int ks = k0; ks < k1; ++ks) {
-            mma_bf16_ts(z, tmem + BQ_P + 8 * ks, desc_advance(dk, ks * 256), idesc, ks > 0);
-            mma_bf16_ts(z, tmem + BQ_PLO + 8 * ks, desc_advance(dk, ks * 256), idesc, 1);
-          }
-          mma_commit(&z_half[hf]);
-        };
-        for (int r = 0; r < rank; ++r) {
-          const uint32_t slot = tmem + BQ_TERM + (r & 1) * TERM_COLS;
-          w.wait(&term_full[r & 1], (r >> 1) & 1, 0x23);
-          if (r > 0) w.wait(&u_free[0], (r - 1) & 1, 0x24);
-          else w.wait(&dw_free, 0, 0x25);
-          fence_after_sync();
-          issue_term(tmem + BQ_U, slot, k_addr, na);
-          mma_commit(&u_full[0]);
-          if (r > 0) {
-            issue_z(r - 1, 0);
-            w.wait(&u_free[1], (r - 1) & 1, 0x26);
-          }
-          if (nb2) {
-            fence_after_sync();
-            issue_term(tmem + BQ_U + 64, slot, k_addr + 64 * 16, nb2);
-          }
-          mma_commit(&u_full[1]);            // also: the term's slot has been read
-          if (r > 0) issue_z(r - 1, 1);
+  if (warp >= BQ_ISSUER) {
+    registers_down_to<40>();
+    if (warp == BQ_ISSUER && elect_one()) {
+      const uint32_t k_addr = smem_u32(smem + BQ_K), g_addr = smem_u32(smem + BQ_G), u_addr = smem_u32(smem + BQ_U);
+      const uint64_t du = smem_desc(u_addr, ROW_PLANE, 128), dk_rows = smem_desc(k_addr, ROW_PLANE, 128), dk_dims = smem_desc(k_addr, 128, ROW_PLANE);
+      const uint32_t idesc_s = instr_desc_bf16(128, cols, 0, 0), idesc_z = instr_desc_bf16(128, HD, 0, 1);
+      issue_dw(tmem + BQ_S, smem_desc(g_addr, ROW_PLANE, 128), smem_desc(g_addr + SLAB_S_BYTES, ROW_PLANE, 128), 2 * ROW_PLANE, du, du,
+               2 * ROW_PLANE, cols);
+      mma_commit(&dw_full);
+      for (int r = 0; r <= G; ++r) {
+        w.wait(&x_full, r & 1, 0x21);
+        fence_after_sync();
+        if (r < G) {
+          const uint32_t slot = tmem + BQ_ROWS + ((r + 1) & 1) * BQ_ROW_COLS;
+#pragma unroll
+          for (int ks = 0; ks < HD / 16; ++ks)
+            mma_bf16_ts(tmem + BQ_S, slot + 8 * ks, desc_advance(dk_rows, ks * 2 * ROW_PLANE), idesc_s, ks > 0);
+          mma_commit(&s_full);
         }
-        issue_z(rank - 1, 0);
-        issue_z(rank - 1, 1);
+        const uint32_t z = tmem + BQ_Z + (r & 1) * HD;
+        for (int ks = 0; ks < cols / 16; ++ks) {
+          mma_bf16_ts(z, tmem + BQ_X + 8 * ks, desc_advance(dk_dims, ks * 256), idesc_z, ks > 0);
+          mma_bf16_ts(z, tmem + BQ_XLO + 8 * ks, desc_advance(dk_dims, ks * 256), idesc_z, 1);
+        }
+        mma_commit(&z_full);
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else {
-    registers_up_to<112>();
-    const unsigned char* xrow = Qimg + row * 16;
-    const float* l = lq + qd * RMAX_ALL * HD;
-    const int rpos = uniform(sc[qd].rpos);
-    const int last_key = 32 * my_rb + 31, my_key = 32 * my_rb + lane;
-    const int d0 = 16 * sub;
+    registers_up_to<224>();
+    const int sub = warp >> 2, m = lane & 3, d0 = 32 * sub;
+    const int my_key = 32 * my_rb + lane;
+    // this warp's keys: half of every 32, in blocks of 16; blocks behind the diagonal stay zero in X
+    const auto key_of = [&](int x) { return 32 * x + 16 * sub; };
+    const auto on = [&](int x) { return 32 * x < cols && x <= my_rb; };
+    // rows of q with only the dims of group r - 1, as the A operand: 32 dims per warp
     const auto build = [&](int r) {
-      build_term16(tmem + BQ_TERM + (r & 1) * TERM_COLS + lane_off, xrow, l + r * HD, d0);
+      const uint32_t* mask = mask_s + (qd * GMAX + r - 1) * (HD / 2) + d0 / 2;
+      const uint32_t slot = tmem + BQ_ROWS + (r & 1) * BQ_ROW_COLS + lane_off + d0 / 2;
+      uint32_t o[16];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint4 x = *reinterpret_cast<const uint4*>(Qimg + (d0 / 8 + c) * ROW_PLANE + row * 16);
+        const uint4 k = *reinterpret_cast<const uint4*>(mask + 4 * c);
+        o[4 * c] = x.x & k.x; o[4 * c + 1] = x.y & k.y; o[4 * c + 2] = x.z & k.z; o[4 * c + 3] = x.w & k.w;
+      }
+      tmem_st16(slot, o);
+    };
+    // eight pairs of products as bf16 value and remainder, into the columns of one block of 16 keys
+    const auto store_x = [&](int x, const uint32_t (&hi)[8], const uint32_t (&lo)[8]) {
+      tmem_st8(tmem + BQ_X + lane_off + key_of(x) / 2, hi);
+      tmem_st8(tmem + BQ_XLO + lane_off + key_of(x) / 2, lo);
+    };
+    const auto split = [&](const f32x2 (&t)[8], uint32_t (&hi)[8], uint32_t (&lo)[8]) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float t0, t1;
+        f2_unpack(t[j], t0, t1);
+        hi[j] = pack_bf16(t0, t1);
+        lo[j] = pack_bf16(t0 - bf16_lo(hi[j]), t1 - bf16_hi(hi[j]));
+      }
+    };
+    // q rows lane / 4 + 8 t, dims d0 + 8 i + 2 m, + 1: the arrangement in which Z is drained
+    uint32_t qp[4][4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        qp[t][i] = *reinterpret_cast<const uint32_t*>(Qimg + (d0 / 8 + i) * ROW_PLANE + (32 * qd + (lane >> 2) + 8 * t) * 16 + 4 * m);
+    // the dimension whose sum this lane ends up with, in group order
+    const HeadOrder& order = *reinterpret_cast<const HeadOrder*>(smem + BQ_ORDER + qd * (int)sizeof(HeadOrder));
+    float* y_out = ys + qd * RMAX_ALL * HD + order.pos[d0 + 16 * (lane >> 4) + 8 * ((lane >> 3) & 1) + 2 * m + ((lane >> 2) & 1)];
+    build(1);
+    {
+      const uint32_t zero[8] = {};
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (32 * x < cols && !on(x)) store_x(x, zero, zero);
+    }
+    f32x2 dw[4][8];
+    f32x2 sum2 = 0ull;
+    w.wait(&dw_full, 0, 0x22);
+    __syncwarp();
+    fence_after_sync();
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (on(x)) {
+        float d[16];
+        tmem_ld16(tmem + BQ_S + lane_off + key_of(x), d);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int kj = key_of(x) + 2 * j;
+          dw[x][j] = f2_pack(kj <= my_key ? d[2 * j] : 0.f, kj + 1 <= my_key ? d[2 * j + 1] : 0.f);
+          sum2 = f2_add(sum2, dw[x][j]);
+        }
+        uint32_t hi[8], lo[8];
+        split(dw[x], hi, lo);
+        store_x(x, hi, lo);
+      }
+    tmem_st_wait();
+    fence_before_sync();
+    warp_arrive(&x_full, lane);
+    f32x2 dq[4][4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dq[t][i] = 0ull;
+    // Z_r: dq, and the sums over the 32 rows of q * Z (one warp holds all rows of its block)
+    const auto drain = [&](int r) {
+      float z[2][16];
+      const uint32_t at = tmem + BQ_Z + (r & 1) * HD + lane_off + d0;
+      tmem_ld_rows16(at, z[0]);
+      tmem_ld_rows16(at + (16u << 16), z[1]);
+      const float* e = e_s + (qd * RMAX_ALL + r) * HD + d0 + 2 * m;
+      f32x2 ev[4], y[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ev[i] = *reinterpret_cast<const f32x2*>(e + 8 * i);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const f32x2 z2 = f2_pack(z[t >> 1][4 * i + 2 * (t & 1)], z[t >> 1][4 * i + 2 * (t & 1) + 1]);
+          dq[t][i] = f2_fma(ev[i], z2, dq[t][i]);
+          const f32x2 q2 = f2_pack(bf16_lo(qp[t][i]), bf16_hi(qp[t][i]));
+          y[i] = t ? f2_fma(q2, z2, y[i]) : f2_mul(q2, z2);
+        }
+      if (!want_coef) return;
+      // over the eight lanes with the same dims, halving what is carried: lane bit 4 picks i / 2, bit 3 i % 2, bit 2 the element
+      const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+      const f32x2 u0 = f2_add(b4 ? y[2] : y[0], f2_shfl_xor(b4 ? y[0] : y[2], 16));
+      const f32x2 u1 = f2_add(b4 ? y[3] : y[1], f2_shfl_xor(b4 ? y[1] : y[3], 16));
+      const f32x2 u = f2_add(b3 ? u1 : u0, f2_shfl_xor(b3 ? u0 : u1, 8));
+      float v0, v1;
+      f2_unpack(u, v0, v1);
+      const float v = (b2 ? v1 : v0) + __shfl_xor_sync(0xffffffffu, b2 ? v0 : v1, 4);
+      y_out[r * HD] = v;
+    };
+    for (int r = 1; r <= G; ++r) {
+      // the next rows' slot was last read for the scores of r - 1, which have arrived
+      if (r < G) build(r + 1);
+      w.wait(&s_full, (r - 1) & 1, 0x23);
+      __syncwarp();
+      fence_after_sync();
+      float sc[2][16];
+      uint32_t hi[2][8], lo[2][8];
+      const auto products = [&](int x, int k) {
+        f32x2 t[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t[j] = f2_mul(dw[x][j], f2_pack(sc[k][2 * j], sc[k][2 * j + 1]));
+        split(t, hi[k], lo[k]);
+      };
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+        if (on(x)) tmem_ld16(tmem + BQ_S + lane_off + key_of(x), sc[x]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+        if (on(x)) products(x, x);
+#pragma unroll
+      for (int x = 2; x < 4; ++x)
+        if (on(x)) tmem_ld16(tmem + BQ_S + lane_off + key_of(x), sc[x - 2]);
+      tmem_ld_wait();
+      w.wait(&z_full, (r - 1) & 1, 0x24);            // X of r - 1 has been read
+      __syncwarp();
+      fence_after_sync();
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+        if (on(x)) store_x(x, hi[x], lo[x]);
+#pragma unroll
+      for (int x = 2; x < 4; ++x)
+        if (on(x)) {
+          products(x, x - 2);
+          store_x(x, hi[x - 2], lo[x - 2]);
+        }
       tmem_st_wait();
       fence_before_sync();
-      warp_arrive(&term_full[r & 1], lane);
-    };
-    build(0);
-    // this warp's keys: a quarter of each half, in blocks of 8; blocks behind the diagonal stay zero in P
-    const auto key_of = [&](int hf, int x) { return 64 * hf + sub * ((hf ? nb2 : na) / 4) + 8 * x; };
-    const auto exists = [&](int hf, int x) { return 32 * x < (hf ? nb2 : na); };
-    const auto on = [&](int hf, int x) { return exists(hf, x) && key_of(hf, x) <= last_key; };
-    f32x2 dw[2][2][4];
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-      for (int x = 0; x < 2; ++x)
-        if (exists(hf, x) && !on(hf, x)) {
-          tmem_st4(tmem + BQ_P + lane_off + key_of(hf, x) / 2, 0u, 0u, 0u, 0u);
-          tmem_st4(tmem + BQ_PLO + lane_off + key_of(hf, x) / 2, 0u, 0u, 0u, 0u);
-        }
-    w.wait(&dw_full, 0, 0x27);
-    fence_after_sync();
-    f32x2 sum2 = 0ull;
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-      for (int x = 0; x < 2; ++x)
-        if (on(hf, x)) {
-          float d[8];
-          tmem_ld8(tmem + BQ_U + lane_off + key_of(hf, x), d);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int kj = key_of(hf, x) + 2 * j;
-            dw[hf][x][j] = f2_pack(kj <= my_key ? 2.f * d[2 * j] : 0.f, kj + 1 <= my_key ? 2.f * d[2 * j + 1] : 0.f);
-            sum2 = f2_add(sum2, dw[hf][x][j]);
-          }
-        }
-    fence_before_sync();
-    warp_arrive(&dw_free, lane);
-    f32x2 dq[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dq[j] = 0ull;
-    // Z of term r: dq, and the sums over the 32 rows of q * Z (one warp holds all rows of its block)
-    const auto drain = [&](int r) {
-      float z[16];
-      tmem_ld16(tmem + BQ_Z + (r & 1) * HD + lane_off + d0, z);
-      tmem_ld_wait();
-      fence_before_sync();
-      warp_arrive(&z_free[r & 1], lane);
-      const f32x2 sgn = f2_bcast(r < rpos ? 1.f : -1.f);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const ulonglong2 lv = *reinterpret_cast<const ulonglong2*>(l + r * HD + d0 + 4 * j);
-        dq[2 * j] = f2_fma(f2_mul(lv.x, sgn), f2_pack(z[4 * j], z[4 * j + 1]), dq[2 * j]);
-        dq[2 * j + 1] = f2_fma(f2_mul(lv.y, sgn), f2_pack(z[4 * j + 2], z[4 * j + 3]), dq[2 * j + 1]);
-      }
-      if (!want_coef) return;
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(xrow + (d0 / 8 + k) * CP);
-        const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          z[8 * k + 2 * j] *= bf16_lo(rw[j]);
-          z[8 * k + 2 * j + 1] *= bf16_hi(rw[j]);
-        }
-      }
-      // butterfly that halves the values it carries: 16 shuffles for 16 sums over 32 lanes
-#pragma unroll
-      for (int o = 16; o >= 2; o >>= 1) {
-        const bool up = lane & o;
-#pragma unroll
-        for (int j = 0; j < o / 2; ++j) {
-          const float send = up ? z[j] : z[j + o / 2], keep = up ? z[j + o / 2] : z[j];
-          z[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-      }
-      z[0] += __shfl_xor_sync(0xffffffffu, z[0], 1);
-      if ((lane & 1) == 0) ys[(qd * RMAX_ALL + r) * HD + d0 + (lane >> 1)] = z[0];
-    };
-    for (int r = 0; r < rank; ++r) {
-      // the next term is built while the MMAs of this one run; its slot's last reader was term r - 1, complete
-      // since u_full[1](r - 1)
-      if (r + 1 < rank) build(r + 1);
-      const f32x2 c2 = f2_bcast(sc[qd].c[r]);
-      f32x2 n2 = 0ull;
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        w.wait(&u_full[hf], r & 1, 0x28 + hf);
-        fence_after_sync();
-        float u[2][8];
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (on(hf, x)) tmem_ld8(tmem + BQ_U + lane_off + key_of(hf, x), u[x]);
-        tmem_ld_wait();
-        fence_before_sync();
-        warp_arrive(&u_free[hf], lane);
-        uint32_t hi[2][4], lo[2][4];
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (on(hf, x)) {
-            f32x2 t[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              t[j] = f2_mul(dw[hf][x][j], f2_add(f2_pack(u[x][2 * j], u[x][2 * j + 1]), c2));
-              n2 = f2_add(n2, t[j]);
-            }
-            split8(t, hi[x], lo[x]);
-          }
-        if (r > 0) {                           // the previous term's P has been read
-          w.wait(&z_half[hf], (r - 1) & 1, 0x2A + hf);
-          fence_after_sync();
-        }
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (on(hf, x)) {
-            tmem_st4(tmem + BQ_P + lane_off + key_of(hf, x) / 2, hi[x][0], hi[x][1], hi[x][2], hi[x][3]);
-            tmem_st4(tmem + BQ_PLO + lane_off + key_of(hf, x) / 2, lo[x][0], lo[x][1], lo[x][2], lo[x][3]);
-          }
-        tmem_st_wait();
-        fence_before_sync();
-        warp_arrive(&p_full[hf], lane);
-      }
-      if (r > 0) drain(r - 1);
-      if (want_coef) {
-        float n, n1;
-        f2_unpack(n2, n, n1);
-        n += n1;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-        if (lane == 0) nq[warp][r] = n;
-      }
+      warp_arrive(&x_full, lane);
+      drain(r - 1);
     }
-    w.wait(&z_half[0], (rank - 1) & 1, 0x2C);
-    w.wait(&z_half[1], (rank - 1) & 1, 0x2D);
+    const int rows = max(tile.nc - 32 * my_rb, 0);            // of the row block that exist
+    const size_t out0 = (((size_t)tile.b * a.Hq + my_head) * a.N + tok0 + 32 * my_rb + (lane >> 2)) * HD + d0 + 2 * m;
+    float2 cross[4][4];
+    const bool add_cross = a.dq && a.dq_init && tile.c >= a.cross_from;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        cross[t][i] = add_cross && (lane >> 2) + 8 * t < rows ? *reinterpret_cast<const float2*>(a.dq_init + out0 + 8 * t * HD + 8 * i)
+                                                               : make_float2(0.f, 0.f);
+    w.wait(&z_full, G & 1, 0x25);
+    __syncwarp();
     fence_after_sync();
-    drain(rank - 1);
+    drain(G);
+    if (a.dq && !dead) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if ((lane >> 2) + 8 * t < rows) {
+            float v0, v1;
+            f2_unpack(dq[t][i], v0, v1);
+            *reinterpret_cast<uint32_t*>(a.dq + out0 + 8 * t * HD + 8 * i) = pack_bf16(v0 + cross[t][i].x, v1 + cross[t][i].y);
+          }
+    }
     if (want_coef) {
       float s0, s1;
       f2_unpack(sum2, s0, s1);
       s0 += s1;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-      if (lane == 0) sq[warp] = s0;
-    }
-    if (a.dq && my_key < tile.nc && !dead) {
-      // 16 consecutive dims of a row per thread: whole 32- and 64-byte sectors
-      const size_t o = (((size_t)tile.b * a.Hq + my_head) * a.N + tok0 + my_key) * HD + d0;
-      float v[16];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f2_unpack(dq[j], v[2 * j], v[2 * j + 1]);
-      if (a.dq_init && tile.c >= a.cross_from) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 t = *reinterpret_cast<const float4*>(a.dq_init + o + 4 * j);
-          v[4 * j] += t.x; v[4 * j + 1] += t.y; v[4 * j + 2] += t.z; v[4 * j + 3] += t.w;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        *reinterpret_cast<uint4*>(a.dq + o + 8 * j) =
-            make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
-                       pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
-    }
-    if (want_coef) {
-      // the quadrant's four warps turn its sums into D' (symmetrised: both orders are the same sum), n', s'
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + qd) : "memory");
-      const auto n_of = [&](int r) { return (nq[qd][r] + nq[4 + qd][r]) + (nq[8 + qd][r] + nq[12 + qd][r]); };
-      const int nu = rank * (rank + 1) / 2, stride = nu + rank + 1, blocks = (a.N + 31) / 32;
-      float* dst = a.coef_partial + (((size_t)tile.b * a.Hq + my_head) * blocks + tile.c * 4 + my_rb) * stride;
+      if (lane == 0) sum_s[warp] = s0;
+      // the quadrant's two warps: sums of y over the dims of each group, then dA, dB and dC (symmetrised: both orders are
+      // the same sum)
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + qd) : "memory");
       const float* y = ys + qd * RMAX_ALL * HD;
-      for (int x = sub * 32 + lane; x < stride && 32 * my_rb < tile.nc; x += 128) {
-        float t;
-        if (x < nu) {
-          int r = 0, rest = x;
-          while (rest >= rank - r) { rest -= rank - r; ++r; }
-          const int r2 = r + rest;
-          t = fmaf(sc[qd].c[r2], n_of(r), sc[qd].c[r] * n_of(r2));
+      for (int x = sub * 32 + lane; x < a.rank * G; x += 64) {
+        const int r = x / G, g = x % G, end = order.start[g + 1];
+        float t = 0.f;
 #pragma unroll 4
-          for (int d = 0; d < HD; d += 4) {
-            const float4 la = *reinterpret_cast<const float4*>(l + r * HD + d), lb = *reinterpret_cast<const float4*>(l + r2 * HD + d);
-            const float4 ya = *reinterpret_cast<const float4*>(y + r * HD + d), yb = *reinterpret_cast<const float4*>(y + r2 * HD + d);
-            t = fmaf(lb.x, ya.x, fmaf(lb.y, ya.y, fmaf(lb.z, ya.z, fmaf(lb.w, ya.w, t))));
-            t = fmaf(la.x, yb.x, fmaf(la.y, yb.y, fmaf(la.z, yb.z, fmaf(la.w, yb.w, t))));
-          }
-          t *= 0.5f;
-        } else if (x < nu + rank) {
-          t = n_of(x - nu);
+        for (int p = order.start[g]; p < end; ++p) t += y[r * HD + p];
+        cls_s[qd][x] = t;
+      }
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + qd) : "memory");
+      const int slots = 1 + G + G * (G + 1) / 2, blocks = (a.N + 31) / 32;
+      float* dst = a.coef_partial + (((size_t)tile.b * a.Hq + my_head) * blocks + tile.c * 4 + my_rb) * slots;
+      for (int x = sub * 32 + lane; x < slots && rows > 0; x += 64) {
+        float t;
+        if (x == 0) {
+          t = sum_s[qd] + sum_s[4 + qd];
+        } else if (x <= G) {
+          t = a.scale * cls_s[qd][x - 1];
         } else {
-          t = (sq[qd] + sq[4 + qd]) + (sq[8 + qd] + sq[12 + qd]);
+          int g = 0, rest = x - 1 - G;
+          while (rest >= G - g) { rest -= G - g; ++g; }
+          t = 0.5f * a.scale * a.scale * (cls_s[qd][(1 + g) * G + g + rest] + cls_s[qd][(1 + g + rest) * G + g]);
         }
         dst[x] = t;
       }
@@ -410,8 +409,8 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_q_kernel(const IntraB
 constexpr uint32_t BK_U = 0, BK_P = 128, BK_PLO = 192, BK_Z = 256, BK_V = 320, BK_TERM = 384;
 static_assert(BK_TERM + 2 * TERM_COLS <= 512, "tensor-memory columns of the key/value-side kernel");
 constexpr int BK_HEAD_L = RMAX_ALL * HD * 4;
-constexpr int BK_HEAD_BYTES = X_BYTES + 2 * SLAB_S_BYTES + BK_HEAD_L;       // Q image, G hi, G lo, l: one head's operands
-constexpr int BK_SMEM = X_BYTES + XA_BYTES + 2 * BK_HEAD_BYTES;
+constexpr int BK_HEAD_BYTES = ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES + BK_HEAD_L;       // Q image, G hi, G lo, l: one head's operands
+constexpr int BK_SMEM = ROW_IMAGE_BYTES + SLAB_S_BYTES + 2 * BK_HEAD_BYTES;
 static_assert(BK_HEAD_BYTES % 16 == 0 && BK_SMEM <= 227 * 1024, "shared memory of the key/value-side kernel");
 
 // FINE: P^T with its remainders and W^T against both images of G, for heads of more than 8 groups.  Their weights were
@@ -422,10 +421,10 @@ template <bool FINE>
 __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const IntraBwdArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* Kimg = smem;
-  unsigned char* Uimg = Kimg + X_BYTES;
-  unsigned char* heads = Uimg + XA_BYTES;                       // two sets of a head's operands
+  unsigned char* Uimg = Kimg + ROW_IMAGE_BYTES;
+  unsigned char* heads = Uimg + SLAB_S_BYTES;                   // two sets of a head's operands
   __shared__ __align__(16) HeadScalars sc[2];
-  __shared__ uint64_t q_full[2], g_full[2], dw_full, dw_free, u_full[2], u_free[2], term_full[2], p_full[2], z_half[2], z_free, w_full, v_full;
+  __shared__ uint64_t u_in, g_full[2], dw_full, dw_free, u_full[2], u_free[2], term_full[2], p_full[2], z_half[2], z_free, w_full, v_full;
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -435,20 +434,9 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
   const int tok0 = c * CT, nc = min(CT, a.N - tok0), cols = (nc + 31) & ~31;
   const size_t koff = ((size_t)b * a.Hkv + kvh) * a.N + tok0;
   const auto head_of = [&](int i) { return kvh * a.rep + h0 + i; };
-  // Q image, l and scalars of head i: asynchronous copies by threads tid of n
-  const auto fetch_q = [&](int i, int n) {
-    unsigned char* set = heads + (i & 1) * BK_HEAD_BYTES;
-    load_rows(set, 0, a.q + (((size_t)b * a.Hq + head_of(i)) * a.N + tok0) * HD, cols, nc, tid, n);
-    load_head(reinterpret_cast<float*>(set + X_BYTES + 2 * SLAB_S_BYTES), &sc[i & 1], a.factors + head_of(i), rank, tid, n);
-  };
-  load_rows(Kimg, 0, a.k + koff * HD, CT, nc, tid, BW_THREADS);
-  load_rows(Uimg, 0, a.v + koff * VD, CT, nc, tid, BW_THREADS);
-  if (warp < BW_COMPUTE) fetch_q(0, BW_COMPUTE * 32);
-  augment_rows(Uimg, nc, tid, BW_THREADS);
   if (warp == 0) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&q_full[s], BW_COMPUTE);
       mbar_init(&g_full[s], 1);
       mbar_init(&u_full[s], 1);
       mbar_init(&u_free[s], BW_COMPUTE);
@@ -461,11 +449,10 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
     mbar_init(&z_free, BW_COMPUTE);
     mbar_init(&w_full, BW_COMPUTE);
     mbar_init(&v_full, 1);
+    mbar_init(&u_in, 1);
     mbar_fence_init();
     dead = 0;
   }
-  async_copies_wait();
-  fence_async_smem();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -479,34 +466,43 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
     if (warp == BW_ISSUER) {
       if (elect_one()) {
         const uint32_t u_addr = smem_u32(Uimg);
-        const auto fetch_g = [&](int i) {                     // both G images of head i (bulk copies)
-          unsigned char* dst = heads + (i & 1) * BK_HEAD_BYTES + X_BYTES;
-          const unsigned char* src = reinterpret_cast<const unsigned char*>(a.gimg) + (((size_t)b * a.Hq + head_of(i)) * a.NB + c) * SLAB_S_BYTES;
-          mbar_arrive_expect_tx(&g_full[i & 1], 2 * SLAB_S_BYTES);
-          bulk_g2s(dst, src, SLAB_S_BYTES, &g_full[i & 1]);
-          bulk_g2s(dst + SLAB_S_BYTES, src + a.gimg_lo_offset, SLAB_S_BYTES, &g_full[i & 1]);
+        const size_t unit = ((size_t)b * a.Hkv + kvh) * a.NB + c;
+        mbar_arrive_expect_tx(&u_in, ROW_IMAGE_BYTES + SLAB_S_BYTES);
+        bulk_g2s(Kimg, a.k_image + unit * ROW_IMAGE_BYTES, ROW_IMAGE_BYTES, &u_in);
+        bulk_g2s(Uimg, a.u_image + unit * SLAB_S_BYTES, SLAB_S_BYTES, &u_in);
+        const auto fetch_head = [&](int i) {                  // rows of q, both images of G, l and scalars of head i
+          unsigned char* dst = heads + (i & 1) * BK_HEAD_BYTES;
+          const size_t at = ((size_t)b * a.Hq + head_of(i)) * a.NB + c;
+          const HeadFactor* f = a.factors + head_of(i);
+          uint64_t* bar = &g_full[i & 1];
+          mbar_arrive_expect_tx(bar, ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES + rank * HD * 4 + (int)sizeof(HeadScalars));
+          bulk_g2s(dst, a.q_image + at * ROW_IMAGE_BYTES, ROW_IMAGE_BYTES, bar);
+          bulk_g2s(dst + ROW_IMAGE_BYTES, a.gimg + at * SLAB_S_BYTES, SLAB_S_BYTES, bar);
+          bulk_g2s(dst + ROW_IMAGE_BYTES + SLAB_S_BYTES, a.gimg + a.gimg_lo_offset + at * SLAB_S_BYTES, SLAB_S_BYTES, bar);
+          bulk_g2s(dst + ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES, &f->l[0][0], rank * HD * 4, bar);
+          bulk_g2s(&sc[i & 1], &f->s, (int)sizeof(HeadScalars), bar);
         };
-        fetch_g(0);
+        fetch_head(0);
+        w.wait(&u_in, 0, 0x32);
         int T = 0;                                            // terms issued so far, over all heads
         for (int i = 0; i < n_heads; ++i) {
-          const uint32_t q_addr = smem_u32(heads + (i & 1) * BK_HEAD_BYTES), g_addr = q_addr + X_BYTES;
+          const uint32_t q_addr = smem_u32(heads + (i & 1) * BK_HEAD_BYTES), g_addr = q_addr + ROW_IMAGE_BYTES;
           if (i + 1 < n_heads) {
             if (i > 0) w.wait(&v_full, (i - 1) & 1, 0x30);    // head i - 1 no longer reads the set that head i + 1 takes
-            fetch_g(i + 1);
+            fetch_head(i + 1);
           }
           w.wait(&g_full[i & 1], (i >> 1) & 1, 0x31);
-          w.wait(&q_full[i & 1], (i >> 1) & 1, 0x32);
           if (T > 0) {
             w.wait(&u_free[0], (T - 1) & 1, 0x33);
             w.wait(&u_free[1], (T - 1) & 1, 0x34);
           }
           fence_after_sync();
           // dW^T[j, i] = [v|1]_j . g_i: rows from the U image, columns from the hi and lo images of G
-          const uint64_t du = smem_desc(u_addr, CP, 128);
-          issue_dw(tmem + BK_U, du, du, 2 * CP, smem_desc(g_addr, CT * 16, 128), smem_desc(g_addr + SLAB_S_BYTES, CT * 16, 128),
+          const uint64_t du = smem_desc(u_addr, ROW_PLANE, 128);
+          issue_dw(tmem + BK_U, du, du, 2 * ROW_PLANE, smem_desc(g_addr, CT * 16, 128), smem_desc(g_addr + SLAB_S_BYTES, CT * 16, 128),
                    2 * CT * 16, cols);
           mma_commit(&dw_full);
-          const uint64_t dq = smem_desc(q_addr, 128, CP), dg = smem_desc(g_addr, 128, CT * 16);
+          const uint64_t dq = smem_desc(q_addr, 128, ROW_PLANE), dg = smem_desc(g_addr, 128, CT * 16);
           const uint64_t dg_lo = smem_desc(g_addr + SLAB_S_BYTES, 128, CT * 16);
           const auto issue_z = [&](int t, int hf) {
             w.wait(&p_full[hf], t & 1, 0x35);
@@ -525,7 +521,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
             if (r > 0) w.wait(&u_free[0], (T - 1) & 1, 0x38);
             else w.wait(&dw_free, i & 1, 0x39);
             fence_after_sync();
-            issue_term(tmem + BK_U, slot, q_addr, na);
+            issue_term<ROW_PLANE>(tmem + BK_U, slot, q_addr, na);
             mma_commit(&u_full[0]);
             if (r > 0) {
               issue_z(T - 1, 0);
@@ -533,7 +529,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
             }
             if (nb2) {
               fence_after_sync();
-              issue_term(tmem + BK_U + 64, slot, q_addr + 64 * 16, nb2);
+              issue_term<ROW_PLANE>(tmem + BK_U + 64, slot, q_addr + 64 * 16, nb2);
             }
             mma_commit(&u_full[1]);            // also: the term's slot has been read
             if (r > 0) issue_z(T - 1, 1);
@@ -568,23 +564,20 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
           tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, 0u, 0u, 0u, 0u);
           tmem_st4(tmem + BK_PLO + lane_off + col_of(hf, x) / 2, 0u, 0u, 0u, 0u);
         }
+    w.wait(&u_in, 0, 0x3F);
     f32x2 dk[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) dk[j] = 0ull;
     int T = 0;
     for (int i = 0; i < n_heads; ++i) {
-      const float* l = reinterpret_cast<const float*>(heads + (i & 1) * BK_HEAD_BYTES + X_BYTES + 2 * SLAB_S_BYTES);
+      const float* l = reinterpret_cast<const float*>(heads + (i & 1) * BK_HEAD_BYTES + ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES);
       const HeadScalars& hs = sc[i & 1];
-      async_copies_wait();
-      fence_async_smem();
-      warp_arrive(&q_full[i & 1], lane);
-      // every warp reads l and the scalars below: all copies have arrived
-      w.wait(&q_full[i & 1], (i >> 1) & 1, 0x3C);
-      if (i > 0) w.wait(&v_full, (i - 1) & 1, 0x3D);          // W^T of the previous head has been read; so has its operand set
-      if (i + 1 < n_heads) fetch_q(i + 1, BW_COMPUTE * 32);
+      w.wait(&g_full[i & 1], (i >> 1) & 1, 0x3C);             // l and the scalars are read below
+      if (i > 0) w.wait(&v_full, (i - 1) & 1, 0x3D);          // W^T of the previous head has been read
+      __syncwarp();
       const int rpos = uniform(hs.rpos);
       const auto build = [&](int r) {
-        build_term16(tmem + BK_TERM + ((T + r) & 1) * TERM_COLS + lane_off, xrow, l + r * HD, d0);
+        build_term16<ROW_PLANE>(tmem + BK_TERM + ((T + r) & 1) * TERM_COLS + lane_off, xrow, l + r * HD, d0);
         tmem_st_wait();
         fence_before_sync();
         warp_arrive(&term_full[(T + r) & 1], lane);
@@ -769,11 +762,11 @@ __global__ void __launch_bounds__(256) kv_head_reduce_kernel(const KvReduceArgs 
   *reinterpret_cast<uint2*>(out + tok * HD + 4 * d4) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
 }
 
-IntraBwdArgs bwd_args(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
+IntraBwdArgs bwd_args(const RowImages& rows, const void* gimg, const void* factors,
                       int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups) {
   IntraBwdArgs a{};
-  a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k);
-  a.v = static_cast<const __nv_bfloat16*>(v); a.gimg = static_cast<const __nv_bfloat16*>(gimg);
+  a.q_image = static_cast<const unsigned char*>(rows.q_image); a.k_image = static_cast<const unsigned char*>(rows.k_image);
+  a.u_image = static_cast<const unsigned char*>(rows.u_image); a.gimg = static_cast<const unsigned char*>(gimg);
   a.factors = static_cast<const HeadFactor*>(factors);
   a.status = status;
   a.N = N; a.NB = NB; a.Hq = Hq; a.Hkv = Hkv; a.rep = Hq / Hkv; a.rank = groups + 1;
@@ -785,15 +778,15 @@ IntraBwdArgs bwd_args(const void* q, const void* k, const void* v, const void* g
 
 int intra_row_blocks(int N) { return (N + 31) / 32; }
 
-cudaError_t intra_backward_q(const void* q, const void* k, const void* v, const void* gimg,
-                             const void* factors, void* dq, const float* dq_init, float* coef_partial,
-                             int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups, int cross_from,
-                             cudaStream_t st) {
+cudaError_t intra_backward_q(const RowImages& rows, const void* gimg, const void* factors, void* dq, const float* dq_init,
+                             float* coef_partial, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups, float scale,
+                             int cross_from, cudaStream_t st) {
   cudaError_t e = allow_smem<intra_bwd_q_kernel>(BQ_SMEM);
   if (e != cudaSuccess) return e;
-  IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB, groups);
+  IntraBwdArgs a = bwd_args(rows, gimg, factors, status, B, Hq, Hkv, N, NB, groups);
+  a.scale = scale;
   a.dq = static_cast<__nv_bfloat16*>(dq); a.dq_init = dq_init; a.coef_partial = coef_partial; a.cross_from = cross_from;
-  intra_bwd_q_kernel<<<dim3(NB, B * Hkv, Hq / Hkv), BW_THREADS, BQ_SMEM, st>>>(a);
+  intra_bwd_q_kernel<<<dim3(NB, B * Hkv, Hq / Hkv), BQ_THREADS, BQ_SMEM, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -814,14 +807,14 @@ int intra_kv_parts(int B, int Hq, int Hkv, int NB) {
   return best;
 }
 
-cudaError_t intra_backward_kv(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
+cudaError_t intra_backward_kv(const RowImages& rows, const void* gimg, const void* factors,
                               void* dk, void* dv, const float* dk_cross, const float* dv_cross, int cross_end, float* dk_part,
                               float* dv_part, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups,
                               cudaStream_t st) {
   const bool fine = groups > 8;
   cudaError_t e = fine ? allow_smem<intra_bwd_kv_kernel<true>>(BK_SMEM) : allow_smem<intra_bwd_kv_kernel<false>>(BK_SMEM);
   if (e != cudaSuccess) return e;
-  IntraBwdArgs a = bwd_args(q, k, v, gimg, factors, status, B, Hq, Hkv, N, NB, groups);
+  IntraBwdArgs a = bwd_args(rows, gimg, factors, status, B, Hq, Hkv, N, NB, groups);
   a.parts = intra_kv_parts(B, Hq, Hkv, NB);
   a.heads_per_cta = (Hq / Hkv + a.parts - 1) / a.parts;
   a.cross_end = cross_end;

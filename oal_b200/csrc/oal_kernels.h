@@ -83,18 +83,25 @@ cudaError_t cross_read(bool query, const void* x, const void* image, const float
 
 // ---- tensor-core backward kernels (oal_state_bwd.cu): chunks [c0, c0 + NC) of every sequence ----------
 // carry_img / carry_lo: the saved state image and its remainder image (both or neither)
-cudaError_t dstate_heads(const void* q, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
+cudaError_t dstate_heads(const void* q_image, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
                          float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, int c0, int NC, float scale,
                          int32_t* status, cudaStream_t st);
-cudaError_t feature_grad(bool query, const void* x, const void* gimg, const void* v, const void* image,
+// query: x_image, a_image = images of q and G; else of k and [v | 1]
+cudaError_t feature_grad(bool query, const void* x_image, const void* a_image, const void* image,
                          const float* coef_table, float* dx, int B, int H, int rep, int N, int NB, int c0, int NC,
                          int32_t* status, cudaStream_t st);
 cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, int G, const int32_t* dim_perm,
                          const int32_t* group_start, float* dcoef, float* slots, cudaStream_t st);
+// Operand images of the rows of q and k [B*H, NB, 8, 128, 8] and of [v | 1 | 0] [B*Hkv, NB, 10, 128, 8]; k == null: q only
+struct RowImages {
+  const void *q, *k, *v;
+  void *q_image, *k_image, *u_image;
+};
+// heads = B * Hq (0: only the images of k and v), kv_heads = B * Hkv
 cudaError_t norm_vjp_image(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                            const float* num, const float* den, float floor_v, void* gimg, int heads,
-                           int N, int NB, int token_major_heads /* > 0: grad_out is [B, N, Hq, 64] */,
-                           int32_t* clear_status, cudaStream_t st);
+                           int N, int NB, int token_major_heads /* > 0: grad_out is [B, N, Hq, 64] */, const RowImages& rows,
+                           int kv_heads, int32_t* clear_status, cudaStream_t st);
 
 
 // ---- factored intra-chunk weight (oal_factor.cu) -----------------------------------------
@@ -107,11 +114,10 @@ cudaError_t expand_factor_grad(const float* factor, int factor_rows, int Hq, int
                                const float* dC, float* dfactor, cudaStream_t st);
 cudaError_t build_head_factors(const int32_t* dim_perm, const int32_t* group_start, const float* A, const float* Bc,
                                const float* Cc, int Hq, int G, float scale, void* table, cudaStream_t st);
-// dA, dB, dC = back-transformed sum of the query-side partial sums [B][Hq][tiles][nu_stride] (rm terms,
-// upper triangle) + extra ([Hq][NCOEF] slots of the cross-chunk term, or null).
-cudaError_t intra_coef_finish(const float* partial, int tiles, int nu_stride, int rm, const void* table,
-                              const float* extra, int B, int Hq, int G, float* dA, float* dB, float* dC,
-                              const float* factor, float* dfactor, cudaStream_t st);
+// dA, dB, dC = sum of the query-side partial sums [B][Hq][tiles][1 + G + G (G + 1) / 2] (dA, dB, upper triangle of dC) +
+// extra ([Hq][NCOEF] slots of the cross-chunk term, or null); dfactor (optional): the gradient of `factor`, a row per head.
+cudaError_t intra_coef_finish(const float* partial, int tiles, const float* extra, int B, int Hq, int G, float* dA, float* dB,
+                              float* dC, const float* factor, float* dfactor, cudaStream_t st);
 cudaError_t launch_head_prologue(const PrologueArgs& a, int Hq, cudaStream_t st);
 // writes *status | STATUS_DELIVERED to the sink's host word
 cudaError_t deliver_status(const int32_t* status, StatusSink sink, cudaStream_t st);
@@ -122,13 +128,13 @@ cudaError_t intra_forward(const void* q, const void* k, const void* v, const voi
                           float* den, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups, int out_dt,
                           float floor_v, bool out_token_major, int cross_from, StatusSink sink, cudaStream_t st);
 int intra_row_blocks(int N);     // row blocks per head: partial sums of the coefficient gradient
-cudaError_t intra_backward_q(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
+cudaError_t intra_backward_q(const RowImages& rows, const void* gimg, const void* factors,
                              void* dq, const float* dq_init, float* coef_partial, int32_t* status, int B, int Hq,
-                             int Hkv, int N, int NB, int groups, int cross_from, cudaStream_t st);
+                             int Hkv, int N, int NB, int groups, float scale, int cross_from, cudaStream_t st);
 int intra_kv_parts(int B, int Hq, int Hkv, int NB);     // CTAs the heads of a KV head are spread over
 // dk, dv: null where not requested; *_cross: fp32 cross-chunk parts of the tokens before cross_end; *_part: scratch of
 // B * Hq * N * 64 floats
-cudaError_t intra_backward_kv(const void* q, const void* k, const void* v, const void* gimg, const void* factors,
+cudaError_t intra_backward_kv(const RowImages& rows, const void* gimg, const void* factors,
                               void* dk, void* dv, const float* dk_cross, const float* dv_cross, int cross_end, float* dk_part,
                               float* dv_part, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups, cudaStream_t st);
 

@@ -33,7 +33,7 @@ __device__ __forceinline__ void unpack_bf16x8(const uint4 t, float (&o)[8]) {
 // dstate_heads
 // ---------------------------------------------------------------------------
 struct DStateArgs {
-  const __nv_bfloat16* q;          // [B,Hq,N,64]
+  const unsigned char* q_image;    // [B*Hq, NB, 8, 128, 8]
   const __nv_bfloat16* gimg;       // [B*Hq, NB, 10, 128, 8]
   const __nv_bfloat16* carry_img;  // [units, NB, 19, 10, 128, 8] or null (no coefficient gradients)
   const __nv_bfloat16* carry_lo;   // same layout: bf16(state - bf16(state)); the dot products below see hi + lo,
@@ -65,7 +65,7 @@ constexpr int DS_GEN_WARPS = 8, DS_EPI_WARPS = 8;
 constexpr int DS_ISSUER = DS_GEN_WARPS + DS_EPI_WARPS, DS_LOADER = DS_ISSUER + 1;
 // What bounds it: the drain (about 1400 clocks per iteration) and the generators, latency rather than issue slots.  The carry
 // rows were loaded by the drain warps at the head of an item, 5000 of its 15000 clocks.  14 / 2 heads, B = 4, N = 4096:
-// 268 -> 221 us.
+// 268 -> 188 us (221 with the pieces of q from the rows themselves).
 // Two warps more only fill the issuer's warpgroup, whose registers the drain warps take: 640 threads x 96 at launch =
 // 256 x 80 + 256 x 144 + 128 x 24 and 1024 to spare.
 constexpr int DS_THREADS = (DS_LOADER + 3) * 32;
@@ -137,36 +137,30 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
   if (warp < DS_GEN_WARPS) {
     // ---------------- generators ----------------
     registers_down_to<80>();
-    // The two pieces of its token's row that a thread needs for (item, head) come straight from global memory, an
-    // iteration ahead.  (The whole row, once per slab: 32 cache lines for each of eight loads, 1000 clocks.  Through shared
-    // memory with cp.async, coalesced: about 1000 clocks too, which the copies of 16 bytes take to issue.)
+    // The two pieces of its token's row that a thread needs for (item, head) come from the row image, an iteration ahead.
+    // (From the rows themselves: 32 cache lines per load, 1000 clocks.  Through shared memory with cp.async: as long.)
     const int half = warp >> 2, token = 32 * (warp & 3) + lane;
     DsCursor cur;
     cur.start(a.c0, a.NC, a.Hkv, rep);
-    const __nv_bfloat16* row = nullptr;        // the token's row, or null past the end of the sequence
+    const uint4* row = nullptr;                // the token's pieces, ROW_PLANE apart
     uint4 r4 = make_uint4(0u, 0u, 0u, 0u), c4 = r4;
     const auto fetch = [&]() {
-      const int i = cur.c * CT + token, hs = 2 * cur.slab + half;
-      const HalfBlock blk = half_block(min(hs, F_PAIR_BLOCKS - 1));
-      row = i < a.N ? a.q + ((size_t)(cur.b * a.Hq + cur.h0 + cur.hh) * a.N + i) * HD : nullptr;
-      if (row) {
-        r4 = __ldg(reinterpret_cast<const uint4*>(row) + blk.rb);
-        c4 = __ldg(reinterpret_cast<const uint4*>(row) + blk.cb);
-      } else {
-        r4 = c4 = make_uint4(0u, 0u, 0u, 0u);
-      }
+      const HalfBlock blk = half_block(min(2 * cur.slab + half, F_PAIR_BLOCKS - 1));
+      row = reinterpret_cast<const uint4*>(a.q_image + ((size_t)(cur.b * a.Hq + cur.h0 + cur.hh) * a.NB + cur.c) * ROW_IMAGE_BYTES) + token;
+      r4 = __ldg(row + blk.rb * CT);
+      c4 = __ldg(row + blk.cb * CT);
     };
     if (T > 0) fetch();
     int s = 0, use = 0;                       // ring slot of `it` and how often it has been used before
     for (int it = 0; it < T; ++it) {
       const int hs = 2 * cur.slab + half;
       const uint4 r_now = r4, c_now = c4;
-      const __nv_bfloat16* row_now = row;
+      const uint4* row_now = row;
       cur.next(rep, a.c0, a.NC, a.Hkv);
       if (it + 1 < T) fetch();
       if (use > 0) w.wait(&mma_done[s], (use - 1) & 1, 0x31);   // the MMA that read A[s] has completed
       uint4* tile = reinterpret_cast<uint4*>(Abuf + s * SLAB_A_BYTES) + 8 * half * CT + token;
-      raw_half_slab(hs, r_now, c_now, [&](int j) { return row_now ? __ldg(reinterpret_cast<const uint4*>(row_now) + j) : make_uint4(0u, 0u, 0u, 0u); },
+      raw_half_slab(hs, r_now, c_now, [&](int j) { return __ldg(row_now + j * CT); },
                     [&](int j, uint4 f) { tile[j * CT] = f; });
       fence_async_smem();
       warp_arrive(&ready[s], lane);
@@ -387,7 +381,7 @@ __device__ __forceinline__ void fold_half_slab(int hs, uint32_t taddr, const uns
   if (blk.cb != col.cb) {
     if (col.cb >= 0) fold_add8(dx_token, col.cb, col.dx);
     col.cb = blk.cb;
-    const uint4 c4 = *reinterpret_cast<const uint4*>(xrow + blk.cb * CP);
+    const uint4 c4 = *reinterpret_cast<const uint4*>(xrow + blk.cb * ROW_PLANE);
     const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -395,7 +389,7 @@ __device__ __forceinline__ void fold_half_slab(int hs, uint32_t taddr, const uns
       col.dx[k] = 0ull;
     }
   }
-  const uint4 r4 = *reinterpret_cast<const uint4*>(xrow + blk.rb * CP);
+  const uint4 r4 = *reinterpret_cast<const uint4*>(xrow + blk.rb * ROW_PLANE);
   const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
   f32x2 xr[8], sum[8];
 #pragma unroll
@@ -434,16 +428,14 @@ __device__ __forceinline__ void fold_half_slab(int hs, uint32_t taddr, const uns
 //              tensor memory (four buffers) into its dx row in shared memory; halves are combined per item
 //   warp  8    lane 0 issues  dphi[s] = A . S[s]^T  (M = tokens, N = 128 features, K = 80)
 //   warp  9    lane 0 streams the state slab images (four slots) and, per item, the A operand
-//              image (QUERY: the image of G) and the head's coefficient table (two buffers each)
+//              image (G, or [v | 1] for keys) and, for queries, the head's coefficient table (two buffers each)
 // A state slot and a dphi buffer share their index and one barrier per direction (see cross_read_kernel).
 // What bounds it: the fold's instruction latency (two warps per scheduler, 1500 clocks per slab; the MMAs are four slabs
-// ahead).  14 / 2 heads, B = 4, N = 4096: 187 -> 166 us (QUERY), 38 -> 33 (not).
-// KEY: the A operand [v | 1] is built in shared memory by the fold warps.
+// ahead).  14 / 2 heads, B = 4, N = 4096: 187 -> 164 us (QUERY), 38 -> 29 (not).
 // ---------------------------------------------------------------------------
 struct FeatGradArgs {
-  const __nv_bfloat16* x;        // q [B,Hq,N,64] (QUERY) or k [B,Hkv,N,64]
-  const __nv_bfloat16* gimg;     // QUERY: A-operand image of G  [B*Hq, NB, 10, 128, 8]
-  const __nv_bfloat16* v;        // KEY: values, the A operand [v | 1] is built in shared memory
+  const unsigned char* x_image;  // rows of q (QUERY) or k  [B*H, NB, 8, 128, 8]
+  const unsigned char* a_image;  // A operand: image of G (QUERY) or [v | 1]  [B*H, NB, 10, 128, 8]
   const __nv_bfloat16* image;    // state image [units, NB, 19, 10, 128, 8]: carry (QUERY) / dT (KEY)
   const float* coef_table;       // QUERY
   float* dx;                     // [B,H,N,64] fp32
@@ -476,7 +468,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
   unsigned char* Aimg = Sbuf + FG_RING * SLAB_S_BYTES;              // 2 x SLAB_S_BYTES: [10][128 tokens][8 e]
   float* coef_s = reinterpret_cast<float*>(Aimg + 2 * SLAB_S_BYTES); // 2 x F_ROWS
   unsigned char* ximg = reinterpret_cast<unsigned char*>(coef_s + 2 * F_ROWS);     // rows of x
-  unsigned char* dx_s = ximg + X_BYTES;                              // per half: [16][128 tokens][4] fp32, plane pitch CP
+  unsigned char* dx_s = ximg + ROW_IMAGE_BYTES;                              // per half: [16][128 tokens][4] fp32, plane pitch CP
   __shared__ uint64_t ready[FG_RING], done[FG_RING], a_full[2], a_free[2], coef_full[2], coef_free[2];
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
@@ -490,7 +482,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
       mbar_init(&done[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&a_full[s], QUERY ? 1 : FG_FOLD_WARPS);
+      mbar_init(&a_full[s], 1);
       mbar_init(&a_free[s], 1);
       mbar_init(&coef_full[s], 1);
       mbar_init(&coef_free[s], FG_FOLD_WARPS);
@@ -518,19 +510,13 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
     uint4 next[PIECES];                                   // this thread's share of the next item's rows
     const auto fetch = [&](int k) {
       const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
-      const __nv_bfloat16* src = a.x + ((size_t)(it.b * a.H + it.h) * a.N + it.c * CT) * HD;
+      const uint4* src = reinterpret_cast<const uint4*>(a.x_image + ((size_t)(it.b * a.H + it.h) * a.NB + it.c) * ROW_IMAGE_BYTES);
 #pragma unroll
-      for (int j = 0; j < PIECES; ++j) {
-        const int x = tid + j * T;
-        next[j] = (x >> 3) < a.N - it.c * CT ? *reinterpret_cast<const uint4*>(src + 8 * x) : make_uint4(0u, 0u, 0u, 0u);
-      }
+      for (int j = 0; j < PIECES; ++j) next[j] = __ldg(src + tid + j * T);
     };
     const auto store_rows = [&]() {
 #pragma unroll
-      for (int j = 0; j < PIECES; ++j) {
-        const int x = tid + j * T;
-        *reinterpret_cast<uint4*>(ximg + (x & 7) * CP + (x >> 3) * 16) = next[j];
-      }
+      for (int j = 0; j < PIECES; ++j) reinterpret_cast<uint4*>(ximg)[tid + j * T] = next[j];
     };
     if (my_items > 0) fetch(0);
     store_rows();
@@ -542,17 +528,6 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
     for (int k = 0; k < my_items; ++k) {
       const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
       const size_t head_off = (size_t)(it.b * a.H + it.h) * a.N;
-      if (!QUERY) {
-        // A operand [v | 1] of this item, once the MMAs of item k-2 have left the buffer
-        if (k >= 2) w.wait(&a_free[k & 1], ((k >> 1) - 1) & 1, 0x51);
-        uint4* dst = reinterpret_cast<uint4*>(Aimg + (k & 1) * SLAB_S_BYTES);
-        for (int idx = tid; idx < (EP / 8) * CT; idx += T) {
-          const int ec = idx >> 7, t = idx & 127, j = it.c * CT + t;
-          dst[idx] = u_image_chunk(a.v + (head_off + j) * VD, ec, j < a.N);
-        }
-        fence_async_smem();
-        warp_arrive(&a_full[k & 1], lane);
-      }
       if (k + 1 < my_items) fetch(k + 1);
       const float* coef = coef_s + (k & 1) * F_ROWS;
       if (QUERY) w.wait(&coef_full[k & 1], (k >> 1) & 1, 0x52);
@@ -617,17 +592,17 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
         const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         if (k >= 2) {
           w.wait(&a_free[k & 1], ((k >> 1) - 1) & 1, 0x57);
-          w.wait(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x58);
+          if (QUERY) w.wait(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x58);
         }
         mbar_arrive_expect_tx(&a_full[k & 1], SLAB_U_BYTES);
-        bulk_g2s(Aimg + (k & 1) * SLAB_S_BYTES,
-                 reinterpret_cast<const unsigned char*>(a.gimg) + ((size_t)(it.b * a.H + it.h) * a.NB + it.c) * SLAB_S_BYTES,
-                 SLAB_U_BYTES, &a_full[k & 1]);
+        bulk_g2s(Aimg + (k & 1) * SLAB_S_BYTES, a.a_image + ((size_t)(it.b * a.H + it.h) * a.NB + it.c) * SLAB_S_BYTES, SLAB_U_BYTES,
+                 &a_full[k & 1]);
+        if (!QUERY) return;
         mbar_arrive_expect_tx(&coef_full[k & 1], F_ROWS * (uint32_t)sizeof(float));
         bulk_g2s(coef_s + (k & 1) * F_ROWS, a.coef_table + (size_t)it.h * F_ROWS, F_ROWS * (uint32_t)sizeof(float),
                  &coef_full[k & 1]);
       };
-      if (QUERY && my_items > 0) fetch_item(0);
+      if (my_items > 0) fetch_item(0);
       for (int k = 0; k < my_items; ++k) {
         const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         const int unit = (it.b * a.H + it.h) / a.rep;
@@ -635,7 +610,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
                                    ((size_t)unit * a.NB + it.c) * F_SLABS * SLAB_S_BYTES;
         for (int s = 0; s < F_SLABS; ++s) {
           // the next item's operand and table while there is time: their buffers' last reader was item k-1
-          if (QUERY && s == 2 * F_SLABS / 3 && k + 1 < my_items) fetch_item(k + 1);
+          if (s == 2 * F_SLABS / 3 && k + 1 < my_items) fetch_item(k + 1);
           if (use > 0) w.wait(&done[s4], (use - 1) & 1, 0x59);
           mbar_arrive_expect_tx(&ready[s4], SLAB_U_BYTES);
           bulk_g2s(Sbuf + s4 * SLAB_S_BYTES, img + (size_t)s * SLAB_S_BYTES, SLAB_U_BYTES, &ready[s4]);
@@ -729,19 +704,33 @@ __global__ void __launch_bounds__(32 * SLOT_WARPS) dcoef_slots_kernel(const floa
   }
 }
 
-// normalisation VJP writing the bf16 operand images of G (hi, lo)
+// normalisation VJP writing the bf16 operand images of G (hi, lo), and the images of the rows that the backward kernels
+// fetch with bulk copies (RowImages; copied by threads, 16 bytes each with cp.async, a tile's rows took 5000 clocks)
 //   CTA = 32 consecutive tokens of one (head, chunk); warp = 8 consecutive columns, lane = token, so a
 //   warp stores 512 contiguous bytes of an image chunk.  Rows are enumerated over padded chunks so
 //   that tail tokens of the last chunk are zeroed.
 __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_out, int out_dt, const float* grad_num,
                                                              const float* grad_den, const float* num,
                                                              const float* den, float floor_v, __nv_bfloat16* gimg, int N, int NB, int heads,
-                                                             int tm_heads, int32_t* status) {
+                                                             int tm_heads, const RowImages img_rows, int q_blocks, int32_t* status) {
   __shared__ float part[8][32];
   if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;     // first kernel of the backward
   const int ec = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t per_head = (size_t)NB * CT;
-  const size_t r = (size_t)blockIdx.x * 32 + lane;          // grid covers heads * per_head rows exactly
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  if ((int)blockIdx.x >= q_blocks) {                        // rows of k and of [v | 1 | 0]
+    const size_t r = (size_t)(blockIdx.x - q_blocks) * 32 + lane, bh = r / per_head;
+    const int t = (int)(r % per_head), tl = t % CT;
+    const bool live = t < N;
+    const size_t at = (bh * N + t) * HD + 8 * ec, chunk = bh * NB + t / CT;
+    uint4* k_out = reinterpret_cast<uint4*>(static_cast<unsigned char*>(img_rows.k_image) + chunk * ROW_IMAGE_BYTES);
+    uint4* u_out = reinterpret_cast<uint4*>(static_cast<unsigned char*>(img_rows.u_image) + chunk * SLAB_S_BYTES);
+    k_out[ec * CT + tl] = live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(img_rows.k) + at) : zero;
+    u_out[ec * CT + tl] = live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(img_rows.v) + at) : zero;
+    if (ec < 2) u_out[(VD / 8 + ec) * CT + tl] = make_uint4(ec == 0 && live ? 0x00003F80u : 0u, 0u, 0u, 0u);
+    return;
+  }
+  const size_t r = (size_t)blockIdx.x * 32 + lane;          // q_blocks cover heads * per_head rows exactly
   const size_t bh = r / per_head;
   const int t = (int)(r % per_head);
   const int cidx = t / CT, tl = t % CT;
@@ -781,6 +770,8 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
     }
   }
   part[ec][lane] = dot;
+  reinterpret_cast<uint4*>(static_cast<unsigned char*>(img_rows.q_image) + (bh * NB + cidx) * ROW_IMAGE_BYTES)[ec * CT + tl] =
+      live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(img_rows.q) + row * HD + 8 * ec) : zero;
   // hi image = bf16(g); lo image = bf16(g - hi): dW = g . [v|1] is formed from both, because its two
   // large terms (dout.v / den and dout.num / den^2) nearly cancel
   uint4* img = reinterpret_cast<uint4*>(gimg + (bh * NB + cidx) * (size_t)(SLAB_S_BYTES / 2));
@@ -814,26 +805,25 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
 
 }  // namespace
 
-cudaError_t dstate_heads(const void* q, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
+cudaError_t dstate_heads(const void* q_image, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
                          float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, int c0, int NC, float scale,
                          int32_t* status, cudaStream_t st) {
   cudaError_t e = allow_smem<dstate_heads_kernel>(DS_SMEM);
   if (e != cudaSuccess) return e;
   const int sms = sm_count(), items = F_SLABS * NC * B * Hkv;
-  DStateArgs a{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(gimg),
+  DStateArgs a{static_cast<const unsigned char*>(q_image), static_cast<const __nv_bfloat16*>(gimg),
                static_cast<const __nv_bfloat16*>(carry_img), static_cast<const __nv_bfloat16*>(carry_lo), coef_table,
                dcarry, dcoef_partial, N, NB, Hq, Hkv, B * Hkv, c0, NC, scale, status};
   dstate_heads_kernel<<<items < sms ? items : sms, DS_THREADS, DS_SMEM, st>>>(a);
   return cudaGetLastError();
 }
 
-cudaError_t feature_grad(bool query, const void* x, const void* gimg, const void* v, const void* image,
+cudaError_t feature_grad(bool query, const void* x_image, const void* a_image, const void* image,
                          const float* coef_table, float* dx, int B, int H, int rep, int N, int NB, int c0, int NC,
                          int32_t* status, cudaStream_t st) {
-  const int smem = FG_RING * SLAB_S_BYTES + 2 * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float) + X_BYTES + 2 * 16 * CP;
-  FeatGradArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gimg),
-                 static_cast<const __nv_bfloat16*>(v), static_cast<const __nv_bfloat16*>(image), coef_table, dx,
-                 N, NB, H, rep, B, c0, NC, status};
+  const int smem = FG_RING * SLAB_S_BYTES + 2 * SLAB_S_BYTES + 2 * F_ROWS * (int)sizeof(float) + ROW_IMAGE_BYTES + 2 * 16 * CP;
+  FeatGradArgs a{static_cast<const unsigned char*>(x_image), static_cast<const unsigned char*>(a_image),
+                 static_cast<const __nv_bfloat16*>(image), coef_table, dx, N, NB, H, rep, B, c0, NC, status};
   cudaError_t e;
   const int sms = sm_count(), items = B * H * NC, grid = items < sms ? items : sms;
   if (query) {
@@ -857,11 +847,12 @@ cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, int G, const i
 
 cudaError_t norm_vjp_image(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                            const float* num, const float* den, float floor_v, void* gimg, int heads,
-                           int N, int NB, int token_major_heads, int32_t* clear_status, cudaStream_t st) {
-  const size_t rows = (size_t)heads * NB * CT;      // a multiple of 32
-  norm_vjp_image_kernel<<<(unsigned)(rows / 32), 256, 0, st>>>(grad_out, out_dt, grad_num, grad_den, num, den,
-                                                                   floor_v, static_cast<__nv_bfloat16*>(gimg), N,
-                                                                   NB, heads, token_major_heads, clear_status);
+                           int N, int NB, int token_major_heads, const RowImages& rows, int kv_heads, int32_t* clear_status,
+                           cudaStream_t st) {
+  const int q_blocks = (int)((size_t)heads * NB * CT / 32), kv_blocks = rows.k ? (int)((size_t)kv_heads * NB * CT / 32) : 0;
+  norm_vjp_image_kernel<<<q_blocks + kv_blocks, 256, 0, st>>>(grad_out, out_dt, grad_num, grad_den, num, den, floor_v,
+                                                              static_cast<__nv_bfloat16*>(gimg), N, NB, heads, token_major_heads, rows,
+                                                              q_blocks, clear_status);
   return cudaGetLastError();
 }
 
