@@ -50,10 +50,6 @@ struct IntraBwdArgs {
   int cross_from;                   // first chunk that has a cross-chunk part in dq_init
 };
 
-// Warps 0..15 compute, warp 16 issues; 17..19 only fill the issuer's warpgroup, whose registers the compute warps
-// take: 640 threads x 96 at launch = 512 x 112 + 128 x 24 and 1024 to spare.
-constexpr int BW_COMPUTE = 16, BW_ISSUER = BW_COMPUTE, BW_THREADS = (BW_COMPUTE + 4) * 32;
-
 // dW[128, n] = rows . cols^T over the 80-long augmented value axis; the side given as hi + lo is walked twice.
 __device__ __forceinline__ void issue_dw(uint32_t tmem_dw, uint64_t rows_hi, uint64_t rows_lo, uint32_t rows_step, uint64_t cols_hi,
                                          uint64_t cols_lo, uint32_t cols_step, int n) {
@@ -76,14 +72,13 @@ __device__ __forceinline__ f32x2 f2_shfl_xor(f32x2 v, int o) {
 // query side
 // ---------------------------------------------------------------------------
 // What bounds it: the chain score chain -> products -> X -> Z of each r (about 2000 clocks; the MMAs of an r are 1250) and the
-// first and last phase of a tile.  Eight compute warps with 64 keys each, one barrier of theirs per r: it says at once that
+// first and last phase of a tile.  One barrier of the compute warps per r: it says at once that
 // the scores have been read, X is written, the next masked rows are in place and the Z before last has been drained.
-// 14 / 2 heads, 8 groups, B = 4, N = 4096: 353 -> 204 us against walking the terms of the factored weight (scaled rows as value +
-// remainder, twice the MMA steps, 16 warps with 32 keys each and six barriers per term); of a tile's 32000 clocks 20000 are the
-// loop.
-// Warps 0..7 compute, warp 8 issues; 9..11 only help to load and fill the issuer's warpgroup, whose registers the compute
-// warps take: 384 threads x 168 at launch = 256 x 224 + 128 x 40 and 2048 to spare.
-constexpr int BQ_COMPUTE = 8, BQ_ISSUER = BQ_COMPUTE, BQ_THREADS = (BQ_COMPUTE + 4) * 32;
+// 14 / 2 heads, 8 groups, B = 4, N = 4096: 353 -> 194 us against walking the terms of the factored weight (scaled rows as value +
+// remainder, twice the MMA steps and six barriers per term).
+// Warps 0..15 compute (with eight of twice the keys and dims 201 us), warp 16 issues; 17..19 only help to load and fill the
+// issuer's warpgroup, whose registers the compute warps take: 640 threads x 96 at launch = 512 x 112 + 128 x 32.
+constexpr int BQ_SUBS = 4, BQ_COMPUTE = 4 * BQ_SUBS, BQ_ISSUER = BQ_COMPUTE, BQ_THREADS = (BQ_COMPUTE + 4) * 32;
 // tensor memory: scores (128; first dW) | X hi (64) | X lo (64) | two Z (64) | two slots of masked rows (32)
 constexpr uint32_t BQ_S = 0, BQ_X = 128, BQ_XLO = 192, BQ_Z = 256, BQ_ROWS = 384, BQ_ROW_COLS = 32;
 static_assert(BQ_ROWS + 2 * BQ_ROW_COLS <= 512, "tensor-memory columns of the query-side kernel");
@@ -154,7 +149,7 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
   __syncwarp();
 
   if (warp >= BQ_ISSUER) {
-    registers_down_to<40>();
+    registers_down_to<32>();
     if (warp == BQ_ISSUER && elect_one()) {
       const uint32_t k_addr = smem_u32(smem + BQ_K), g_addr = smem_u32(smem + BQ_G), u_addr = smem_u32(smem + BQ_U);
       const uint64_t du = smem_desc(u_addr, ROW_PLANE, 128), dk_rows = smem_desc(k_addr, ROW_PLANE, 128), dk_dims = smem_desc(k_addr, 128, ROW_PLANE);
@@ -182,24 +177,30 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
     }
     __syncwarp();
   } else {
-    registers_up_to<224>();
-    const int sub = warp >> 2, m = lane & 3, d0 = 32 * sub;
+    registers_up_to<112>();
+    constexpr int BLOCKS = 8 / BQ_SUBS, DIMS = HD / BQ_SUBS, PIECES = DIMS / 8;     // of 16 keys, dims and pieces of 8 dims per warp
+    const int sub = warp >> 2, m = lane & 3, d0 = DIMS * sub;
     const int my_key = 32 * my_rb + lane;
-    // this warp's keys: half of every 32, in blocks of 16; blocks behind the diagonal stay zero in X
-    const auto key_of = [&](int x) { return 32 * x + 16 * sub; };
-    const auto on = [&](int x) { return 32 * x < cols && x <= my_rb; };
-    // rows of q with only the dims of group r - 1, as the A operand: 32 dims per warp
+    // this warp's keys: blocks of 16, half of some 32s; blocks behind the diagonal stay zero in X
+    const auto block_of = [&](int x) { return x * (BQ_SUBS / 2) + (sub >> 1); };
+    const auto key_of = [&](int x) { return 32 * block_of(x) + 16 * (sub & 1); };
+    const auto exists = [&](int x) { return 32 * block_of(x) < cols; };
+    const auto on = [&](int x) { return exists(x) && block_of(x) <= my_rb; };
+    // rows of q with only the dims of group r - 1, as the A operand
     const auto build = [&](int r) {
       const uint32_t* mask = mask_s + (qd * GMAX + r - 1) * (HD / 2) + d0 / 2;
       const uint32_t slot = tmem + BQ_ROWS + (r & 1) * BQ_ROW_COLS + lane_off + d0 / 2;
-      uint32_t o[16];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint4 x = *reinterpret_cast<const uint4*>(Qimg + (d0 / 8 + c) * ROW_PLANE + row * 16);
-        const uint4 k = *reinterpret_cast<const uint4*>(mask + 4 * c);
-        o[4 * c] = x.x & k.x; o[4 * c + 1] = x.y & k.y; o[4 * c + 2] = x.z & k.z; o[4 * c + 3] = x.w & k.w;
+      for (int c = 0; c < PIECES; c += 2) {
+        uint32_t o[8];
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const uint4 x = *reinterpret_cast<const uint4*>(Qimg + (d0 / 8 + c + y) * ROW_PLANE + row * 16);
+          const uint4 k = *reinterpret_cast<const uint4*>(mask + 4 * (c + y));
+          o[4 * y] = x.x & k.x; o[4 * y + 1] = x.y & k.y; o[4 * y + 2] = x.z & k.z; o[4 * y + 3] = x.w & k.w;
+        }
+        tmem_st8(slot + 4 * c, o);
       }
-      tmem_st16(slot, o);
     };
     // eight pairs of products as bf16 value and remainder, into the columns of one block of 16 keys
     const auto store_x = [&](int x, const uint32_t (&hi)[8], const uint32_t (&lo)[8]) {
@@ -216,29 +217,29 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
       }
     };
     // q rows lane / 4 + 8 t, dims d0 + 8 i + 2 m, + 1: the arrangement in which Z is drained
-    uint32_t qp[4][4];
+    uint32_t qp[4][PIECES];
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < PIECES; ++i)
         qp[t][i] = *reinterpret_cast<const uint32_t*>(Qimg + (d0 / 8 + i) * ROW_PLANE + (32 * qd + (lane >> 2) + 8 * t) * 16 + 4 * m);
     // the dimension whose sum this lane ends up with, in group order
     const HeadOrder& order = *reinterpret_cast<const HeadOrder*>(smem + BQ_ORDER + qd * (int)sizeof(HeadOrder));
-    float* y_out = ys + qd * RMAX_ALL * HD + order.pos[d0 + 16 * (lane >> 4) + 8 * ((lane >> 3) & 1) + 2 * m + ((lane >> 2) & 1)];
+    float* y_out = ys + qd * RMAX_ALL * HD + order.pos[d0 + 8 * (lane >> 4) + 2 * m + ((lane >> 3) & 1)];
     build(1);
     {
       const uint32_t zero[8] = {};
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-        if (32 * x < cols && !on(x)) store_x(x, zero, zero);
+      for (int x = 0; x < BLOCKS; ++x)
+        if (exists(x) && !on(x)) store_x(x, zero, zero);
     }
-    f32x2 dw[4][8];
+    f32x2 dw[BLOCKS][8];
     f32x2 sum2 = 0ull;
     w.wait(&dw_full, 0, 0x22);
     __syncwarp();
     fence_after_sync();
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
+    for (int x = 0; x < BLOCKS; ++x)
       if (on(x)) {
         float d[16];
         tmem_ld16(tmem + BQ_S + lane_off + key_of(x), d);
@@ -256,24 +257,24 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
     tmem_st_wait();
     fence_before_sync();
     warp_arrive(&x_full, lane);
-    f32x2 dq[4][4];
+    f32x2 dq[4][PIECES];
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dq[t][i] = 0ull;
+      for (int i = 0; i < PIECES; ++i) dq[t][i] = 0ull;
     // Z_r: dq, and the sums over the 32 rows of q * Z (one warp holds all rows of its block)
     const auto drain = [&](int r) {
-      float z[2][16];
+      float z[2][4 * PIECES];
       const uint32_t at = tmem + BQ_Z + (r & 1) * HD + lane_off + d0;
-      tmem_ld_rows16(at, z[0]);
-      tmem_ld_rows16(at + (16u << 16), z[1]);
+      tmem_ld_rows(at, z[0]);
+      tmem_ld_rows(at + (16u << 16), z[1]);
       const float* e = e_s + (qd * RMAX_ALL + r) * HD + d0 + 2 * m;
-      f32x2 ev[4], y[4];
+      f32x2 ev[PIECES], y[PIECES];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) ev[i] = *reinterpret_cast<const f32x2*>(e + 8 * i);
+      for (int i = 0; i < PIECES; ++i) ev[i] = *reinterpret_cast<const f32x2*>(e + 8 * i);
       tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < PIECES; ++i)
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
           const f32x2 z2 = f2_pack(z[t >> 1][4 * i + 2 * (t & 1)], z[t >> 1][4 * i + 2 * (t & 1) + 1]);
@@ -282,15 +283,14 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
           y[i] = t ? f2_fma(q2, z2, y[i]) : f2_mul(q2, z2);
         }
       if (!want_coef) return;
-      // over the eight lanes with the same dims, halving what is carried: lane bit 4 picks i / 2, bit 3 i % 2, bit 2 the element
-      const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-      const f32x2 u0 = f2_add(b4 ? y[2] : y[0], f2_shfl_xor(b4 ? y[0] : y[2], 16));
-      const f32x2 u1 = f2_add(b4 ? y[3] : y[1], f2_shfl_xor(b4 ? y[1] : y[3], 16));
-      const f32x2 u = f2_add(b3 ? u1 : u0, f2_shfl_xor(b3 ? u0 : u1, 8));
+      // over the eight lanes with the same dims, halving what is carried: first the pieces, then the two elements
+      const bool b4 = lane & 16, b3 = lane & 8;
       float v0, v1;
-      f2_unpack(u, v0, v1);
-      const float v = (b2 ? v1 : v0) + __shfl_xor_sync(0xffffffffu, b2 ? v0 : v1, 4);
-      y_out[r * HD] = v;
+      static_assert(PIECES == 2, "lane bit 4 picks the piece, bit 3 the element");
+      f2_unpack(f2_add(b4 ? y[1] : y[0], f2_shfl_xor(b4 ? y[0] : y[1], 16)), v0, v1);
+      float v = (b3 ? v1 : v0) + __shfl_xor_sync(0xffffffffu, b3 ? v0 : v1, 8);
+      v += __shfl_xor_sync(0xffffffffu, v, 4);
+      if ((lane & 4) == 0) y_out[r * HD] = v;
     };
     for (int r = 1; r <= G; ++r) {
       // the next rows' slot was last read for the scores of r - 1, which have arrived
@@ -298,36 +298,30 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
       w.wait(&s_full, (r - 1) & 1, 0x23);
       __syncwarp();
       fence_after_sync();
-      float sc[2][16];
-      uint32_t hi[2][8], lo[2][8];
+      uint32_t hi[BLOCKS / 2][8], lo[BLOCKS / 2][8];
       const auto products = [&](int x, int k) {
+        float sc[16];
+        tmem_ld16(tmem + BQ_S + lane_off + key_of(x), sc);
+        tmem_ld_wait();
         f32x2 t[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t[j] = f2_mul(dw[x][j], f2_pack(sc[k][2 * j], sc[k][2 * j + 1]));
+        for (int j = 0; j < 8; ++j) t[j] = f2_mul(dw[x][j], f2_pack(sc[2 * j], sc[2 * j + 1]));
         split(t, hi[k], lo[k]);
       };
 #pragma unroll
-      for (int x = 0; x < 2; ++x)
-        if (on(x)) tmem_ld16(tmem + BQ_S + lane_off + key_of(x), sc[x]);
-      tmem_ld_wait();
-#pragma unroll
-      for (int x = 0; x < 2; ++x)
+      for (int x = 0; x < BLOCKS / 2; ++x)
         if (on(x)) products(x, x);
-#pragma unroll
-      for (int x = 2; x < 4; ++x)
-        if (on(x)) tmem_ld16(tmem + BQ_S + lane_off + key_of(x), sc[x - 2]);
-      tmem_ld_wait();
       w.wait(&z_full, (r - 1) & 1, 0x24);            // X of r - 1 has been read
       __syncwarp();
       fence_after_sync();
 #pragma unroll
-      for (int x = 0; x < 2; ++x)
+      for (int x = 0; x < BLOCKS / 2; ++x)
         if (on(x)) store_x(x, hi[x], lo[x]);
 #pragma unroll
-      for (int x = 2; x < 4; ++x)
+      for (int x = BLOCKS / 2; x < BLOCKS; ++x)
         if (on(x)) {
-          products(x, x - 2);
-          store_x(x, hi[x - 2], lo[x - 2]);
+          products(x, x - BLOCKS / 2);
+          store_x(x, hi[x - BLOCKS / 2], lo[x - BLOCKS / 2]);
         }
       tmem_st_wait();
       fence_before_sync();
@@ -336,12 +330,12 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
     }
     const int rows = max(tile.nc - 32 * my_rb, 0);            // of the row block that exist
     const size_t out0 = (((size_t)tile.b * a.Hq + my_head) * a.N + tok0 + 32 * my_rb + (lane >> 2)) * HD + d0 + 2 * m;
-    float2 cross[4][4];
+    float2 cross[4][PIECES];
     const bool add_cross = a.dq && a.dq_init && tile.c >= a.cross_from;
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < PIECES; ++i)
         cross[t][i] = add_cross && (lane >> 2) + 8 * t < rows ? *reinterpret_cast<const float2*>(a.dq_init + out0 + 8 * t * HD + 8 * i)
                                                                : make_float2(0.f, 0.f);
     w.wait(&z_full, G & 1, 0x25);
@@ -352,7 +346,7 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
 #pragma unroll
       for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < PIECES; ++i)
           if ((lane >> 2) + 8 * t < rows) {
             float v0, v1;
             f2_unpack(dq[t][i], v0, v1);
@@ -366,24 +360,26 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
       if (lane == 0) sum_s[warp] = s0;
-      // the quadrant's two warps: sums of y over the dims of each group, then dA, dB and dC (symmetrised: both orders are
+      // the quadrant's warps: sums of y over the dims of each group, then dA, dB and dC (symmetrised: both orders are
       // the same sum)
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + qd) : "memory");
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + qd), "n"(BQ_SUBS * 32) : "memory");
       const float* y = ys + qd * RMAX_ALL * HD;
-      for (int x = sub * 32 + lane; x < a.rank * G; x += 64) {
+      for (int x = sub * 32 + lane; x < a.rank * G; x += BQ_SUBS * 32) {
         const int r = x / G, g = x % G, end = order.start[g + 1];
         float t = 0.f;
 #pragma unroll 4
         for (int p = order.start[g]; p < end; ++p) t += y[r * HD + p];
         cls_s[qd][x] = t;
       }
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + qd) : "memory");
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + qd), "n"(BQ_SUBS * 32) : "memory");
       const int slots = 1 + G + G * (G + 1) / 2, blocks = (a.N + 31) / 32;
       float* dst = a.coef_partial + (((size_t)tile.b * a.Hq + my_head) * blocks + tile.c * 4 + my_rb) * slots;
-      for (int x = sub * 32 + lane; x < slots && rows > 0; x += 64) {
+      for (int x = sub * 32 + lane; x < slots && rows > 0; x += BQ_SUBS * 32) {
         float t;
         if (x == 0) {
-          t = sum_s[qd] + sum_s[4 + qd];
+          t = 0.f;
+#pragma unroll
+          for (int y = 0; y < BQ_SUBS; ++y) t += sum_s[4 * y + qd];
         } else if (x <= G) {
           t = a.scale * cls_s[qd][x - 1];
         } else {
@@ -404,8 +400,20 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
 // ---------------------------------------------------------------------------
 // key / value side: one CTA per (chunk, KV head, batch row) and group of query heads; rows are keys
 // ---------------------------------------------------------------------------
-// tensor memory: U (two halves of 64; first dW^T of a head) | P^T (64), later W^T | their remainders (64) | Z (64) | dU (64) |
-// two term slots (64)
+// What bounds it: as on the query side, the chain of a term (products, hand-over, Z), most of all on the quadrant of keys 0 to
+// 31, which meets all queries (its scheduler issues 1.8 times the mean).  One barrier of the compute warps per term says that U has been read, P^T is written, the next
+// term's rows are in place and the Z before last is drained; the next head's dW^T is computed while W^T of this one is stored.
+//
+// Compute warps: four per quadrant, or two where P^T has remainders (with 112 registers a thread these spill: 16 groups, B = 1,
+// N = 4096: 159 us against 148; 8 groups, B = 4: 242 against 248).  The next warp issues, three more only fill its warpgroup, whose
+// registers the compute warps take: 640 threads x 96 at launch = 512 x 112 + 128 x 32, 384 x 168 = 256 x 232 + 128 x 40.
+template <bool FINE>
+struct KvWarps {
+  static constexpr int SUBS = FINE ? 2 : 4, COMPUTE = 4 * SUBS, ISSUER = COMPUTE, THREADS = (COMPUTE + 4) * 32;
+  static constexpr int REGS = FINE ? 232 : 112, REGS_REST = FINE ? 40 : 32;
+};
+// tensor memory: U (128; first dW^T of a head) | P^T (64), later W^T | their remainders (64) | Z (64) | dU (64) | two term
+// slots (64).  Where P^T has no remainders their columns are a second Z until W^T is stored.
 constexpr uint32_t BK_U = 0, BK_P = 128, BK_PLO = 192, BK_Z = 256, BK_V = 320, BK_TERM = 384;
 static_assert(BK_TERM + 2 * TERM_COLS <= 512, "tensor-memory columns of the key/value-side kernel");
 constexpr int BK_HEAD_L = RMAX_ALL * HD * 4;
@@ -418,38 +426,33 @@ static_assert(BK_HEAD_BYTES % 16 == 0 && BK_SMEM <= 227 * 1024, "shared memory o
 // times as far from 64 bits in dv and 1.18 times in dk (14 / 2 heads, N = 347, 16 groups: 2.13e-3 -> 2.64e-3 and 2.14e-3 ->
 // 2.52e-3); up to 8 groups the bf16 values are nearer than the tiles that they replaced (dk 3.3e-3 -> 2.8e-3).
 template <bool FINE>
-__global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const IntraBwdArgs a) {
+__global__ void __launch_bounds__(KvWarps<FINE>::THREADS, 1) intra_bwd_kv_kernel(const IntraBwdArgs a) {
+  constexpr int SUBS = KvWarps<FINE>::SUBS;
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* Kimg = smem;
   unsigned char* Uimg = Kimg + ROW_IMAGE_BYTES;
   unsigned char* heads = Uimg + SLAB_S_BYTES;                   // two sets of a head's operands
   __shared__ __align__(16) HeadScalars sc[2];
-  __shared__ uint64_t u_in, g_full[2], dw_full, dw_free, u_full[2], u_free[2], term_full[2], p_full[2], z_half[2], z_free, w_full, v_full;
+  __shared__ uint64_t u_in, head_in[2], dw_full, ready, u_full, z_full, w_full, v_full;
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int part = blockIdx.z, c = blockIdx.x, b = blockIdx.y / a.Hkv, kvh = blockIdx.y - b * a.Hkv;
   const int h0 = part * a.heads_per_cta, n_heads = min(a.heads_per_cta, a.rep - h0), rank = a.rank;
-  const int qd = warp & 3, sub = (warp >> 2) & 3, row = 32 * qd + lane;     // row: key index inside the chunk
+  const int qd = warp & 3, row = 32 * qd + lane;     // row: key index inside the chunk
   const int tok0 = c * CT, nc = min(CT, a.N - tok0), cols = (nc + 31) & ~31;
-  const size_t koff = ((size_t)b * a.Hkv + kvh) * a.N + tok0;
   const auto head_of = [&](int i) { return kvh * a.rep + h0 + i; };
   if (warp == 0) tmem_alloc(&tmem_base, 512);
   if (tid == 0) {
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&g_full[s], 1);
-      mbar_init(&u_full[s], 1);
-      mbar_init(&u_free[s], BW_COMPUTE);
-      mbar_init(&term_full[s], BW_COMPUTE);
-      mbar_init(&p_full[s], BW_COMPUTE);
-      mbar_init(&z_half[s], 1);
-    }
-    mbar_init(&dw_full, 1);
-    mbar_init(&dw_free, BW_COMPUTE);
-    mbar_init(&z_free, BW_COMPUTE);
-    mbar_init(&w_full, BW_COMPUTE);
-    mbar_init(&v_full, 1);
     mbar_init(&u_in, 1);
+    mbar_init(&head_in[0], 1);
+    mbar_init(&head_in[1], 1);
+    mbar_init(&dw_full, 1);
+    mbar_init(&ready, KvWarps<FINE>::COMPUTE);
+    mbar_init(&u_full, 1);
+    mbar_init(&z_full, 1);
+    mbar_init(&w_full, KvWarps<FINE>::COMPUTE);
+    mbar_init(&v_full, 1);
     mbar_fence_init();
     dead = 0;
   }
@@ -459,275 +462,268 @@ __global__ void __launch_bounds__(BW_THREADS, 1) intra_bwd_kv_kernel(const Intra
   Waiter w{&dead};
   const uint32_t tmem = uniform(tmem_base);
   const uint32_t lane_off = (uint32_t)(32 * qd) << 16;
-  const int na = min(cols, 64), nb2 = cols - na;              // columns of the two halves
+  // the last Z of a head is in its own columns: those of the remainders are free for W^T
+  const auto z_at = [&](int r) { return tmem + (FINE || ((rank - 1 - r) & 1) == 0 ? BK_Z : BK_PLO); };
 
-  if (warp >= BW_ISSUER) {
-    registers_down_to<24>();
-    if (warp == BW_ISSUER) {
-      if (elect_one()) {
-        const uint32_t u_addr = smem_u32(Uimg);
-        const size_t unit = ((size_t)b * a.Hkv + kvh) * a.NB + c;
-        mbar_arrive_expect_tx(&u_in, ROW_IMAGE_BYTES + SLAB_S_BYTES);
-        bulk_g2s(Kimg, a.k_image + unit * ROW_IMAGE_BYTES, ROW_IMAGE_BYTES, &u_in);
-        bulk_g2s(Uimg, a.u_image + unit * SLAB_S_BYTES, SLAB_S_BYTES, &u_in);
-        const auto fetch_head = [&](int i) {                  // rows of q, both images of G, l and scalars of head i
-          unsigned char* dst = heads + (i & 1) * BK_HEAD_BYTES;
-          const size_t at = ((size_t)b * a.Hq + head_of(i)) * a.NB + c;
-          const HeadFactor* f = a.factors + head_of(i);
-          uint64_t* bar = &g_full[i & 1];
-          mbar_arrive_expect_tx(bar, ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES + rank * HD * 4 + (int)sizeof(HeadScalars));
-          bulk_g2s(dst, a.q_image + at * ROW_IMAGE_BYTES, ROW_IMAGE_BYTES, bar);
-          bulk_g2s(dst + ROW_IMAGE_BYTES, a.gimg + at * SLAB_S_BYTES, SLAB_S_BYTES, bar);
-          bulk_g2s(dst + ROW_IMAGE_BYTES + SLAB_S_BYTES, a.gimg + a.gimg_lo_offset + at * SLAB_S_BYTES, SLAB_S_BYTES, bar);
-          bulk_g2s(dst + ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES, &f->l[0][0], rank * HD * 4, bar);
-          bulk_g2s(&sc[i & 1], &f->s, (int)sizeof(HeadScalars), bar);
-        };
-        fetch_head(0);
-        w.wait(&u_in, 0, 0x32);
-        int T = 0;                                            // terms issued so far, over all heads
-        for (int i = 0; i < n_heads; ++i) {
-          const uint32_t q_addr = smem_u32(heads + (i & 1) * BK_HEAD_BYTES), g_addr = q_addr + ROW_IMAGE_BYTES;
-          if (i + 1 < n_heads) {
-            if (i > 0) w.wait(&v_full, (i - 1) & 1, 0x30);    // head i - 1 no longer reads the set that head i + 1 takes
+  if (warp >= KvWarps<FINE>::ISSUER) {
+    registers_down_to<KvWarps<FINE>::REGS_REST>();
+    if (warp == KvWarps<FINE>::ISSUER && elect_one()) {
+      const uint32_t u_addr = smem_u32(Uimg);
+      const size_t unit = ((size_t)b * a.Hkv + kvh) * a.NB + c;
+      mbar_arrive_expect_tx(&u_in, ROW_IMAGE_BYTES + SLAB_S_BYTES);
+      bulk_g2s(Kimg, a.k_image + unit * ROW_IMAGE_BYTES, ROW_IMAGE_BYTES, &u_in);
+      bulk_g2s(Uimg, a.u_image + unit * SLAB_S_BYTES, SLAB_S_BYTES, &u_in);
+      const auto fetch_head = [&](int i) {                  // rows of q, both images of G, l and scalars of head i
+        unsigned char* dst = heads + (i & 1) * BK_HEAD_BYTES;
+        const size_t at = ((size_t)b * a.Hq + head_of(i)) * a.NB + c;
+        const HeadFactor* f = a.factors + head_of(i);
+        uint64_t* bar = &head_in[i & 1];
+        mbar_arrive_expect_tx(bar, ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES + rank * HD * 4 + (int)sizeof(HeadScalars));
+        bulk_g2s(dst, a.q_image + at * ROW_IMAGE_BYTES, ROW_IMAGE_BYTES, bar);
+        bulk_g2s(dst + ROW_IMAGE_BYTES, a.gimg + at * SLAB_S_BYTES, SLAB_S_BYTES, bar);
+        bulk_g2s(dst + ROW_IMAGE_BYTES + SLAB_S_BYTES, a.gimg + a.gimg_lo_offset + at * SLAB_S_BYTES, SLAB_S_BYTES, bar);
+        bulk_g2s(dst + ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES, &f->l[0][0], rank * HD * 4, bar);
+        bulk_g2s(&sc[i & 1], &f->s, (int)sizeof(HeadScalars), bar);
+      };
+      const uint64_t du = smem_desc(u_addr, ROW_PLANE, 128);
+      // dW^T[j, i] = [v|1]_j . g_i: rows from the U image, columns from the hi and lo images of G
+      const auto head_dw = [&](int i) {
+        const uint32_t g_addr = smem_u32(heads + (i & 1) * BK_HEAD_BYTES) + ROW_IMAGE_BYTES;
+        w.wait(&head_in[i & 1], (i >> 1) & 1, 0x31);
+        fence_after_sync();
+        issue_dw(tmem + BK_U, du, du, 2 * ROW_PLANE, smem_desc(g_addr, ROW_PLANE, 128), smem_desc(g_addr + SLAB_S_BYTES, ROW_PLANE, 128),
+                 2 * ROW_PLANE, cols);
+        mma_commit(&dw_full);
+      };
+      fetch_head(0);
+      if (n_heads > 1) fetch_head(1);
+      w.wait(&u_in, 0, 0x32);
+      head_dw(0);
+      int T = 0, phase = 0;                                 // terms so far, over all heads; phases of `ready`
+      for (int i = 0; i < n_heads; ++i) {
+        const uint32_t q_addr = smem_u32(heads + (i & 1) * BK_HEAD_BYTES), g_addr = q_addr + ROW_IMAGE_BYTES;
+        const uint64_t dq = smem_desc(q_addr, 128, ROW_PLANE), dg = smem_desc(g_addr, 128, ROW_PLANE);
+        const uint64_t dg_lo = smem_desc(g_addr + SLAB_S_BYTES, 128, ROW_PLANE);
+        for (int r = -1; r < rank; ++r) {
+          w.wait(&ready, phase++ & 1, 0x33);
+          fence_after_sync();
+          if (r + 1 < rank) {
+            issue_term<ROW_PLANE>(tmem + BK_U, tmem + BK_TERM + ((T + r + 1) & 1) * TERM_COLS, q_addr, cols);
+            mma_commit(&u_full);
+          }
+          if (r < 0) continue;
+          const uint32_t z = z_at(r);
+          for (int part = 0; part < (FINE ? 2 : 1); ++part)
+            for (int ks = 0; ks < cols / 16; ++ks)
+              mma_bf16_ts(z, tmem + (part ? BK_PLO : BK_P) + 8 * ks, desc_advance(dq, ks * 256), instr_desc_bf16(128, HD, 0, 1), part + ks > 0);
+          mma_commit(&z_full);
+          if (r == 0 && i > 0 && i + 1 < n_heads) {
+            w.wait(&v_full, (i - 1) & 1, 0x34);             // head i - 1 no longer reads the set that head i + 1 takes
             fetch_head(i + 1);
           }
-          w.wait(&g_full[i & 1], (i >> 1) & 1, 0x31);
-          if (T > 0) {
-            w.wait(&u_free[0], (T - 1) & 1, 0x33);
-            w.wait(&u_free[1], (T - 1) & 1, 0x34);
-          }
-          fence_after_sync();
-          // dW^T[j, i] = [v|1]_j . g_i: rows from the U image, columns from the hi and lo images of G
-          const uint64_t du = smem_desc(u_addr, ROW_PLANE, 128);
-          issue_dw(tmem + BK_U, du, du, 2 * ROW_PLANE, smem_desc(g_addr, CT * 16, 128), smem_desc(g_addr + SLAB_S_BYTES, CT * 16, 128),
-                   2 * CT * 16, cols);
-          mma_commit(&dw_full);
-          const uint64_t dq = smem_desc(q_addr, 128, ROW_PLANE), dg = smem_desc(g_addr, 128, CT * 16);
-          const uint64_t dg_lo = smem_desc(g_addr + SLAB_S_BYTES, 128, CT * 16);
-          const auto issue_z = [&](int t, int hf) {
-            w.wait(&p_full[hf], t & 1, 0x35);
-            if (hf == 0 && t > 0) w.wait(&z_free, (t - 1) & 1, 0x36);
-            fence_after_sync();
-            const int k0 = hf ? 4 : 0, k1 = hf ? 4 + nb2 / 16 : na / 16;
-            for (int part = 0; part < (FINE ? 2 : 1); ++part)
-              for (int ks = k0; ks < k1; ++ks)
-                mma_bf16_ts(tmem + BK_Z, tmem + (part ? BK_PLO : BK_P) + 8 * ks, desc_advance(dq, ks * 256),
-                            instr_desc_bf16(128, HD, 0, 1), part + ks > 0);
-            mma_commit(&z_half[hf]);
-          };
-          for (int r = 0; r < rank; ++r, ++T) {
-            const uint32_t slot = tmem + BK_TERM + (T & 1) * TERM_COLS;
-            w.wait(&term_full[T & 1], (T >> 1) & 1, 0x37);
-            if (r > 0) w.wait(&u_free[0], (T - 1) & 1, 0x38);
-            else w.wait(&dw_free, i & 1, 0x39);
-            fence_after_sync();
-            issue_term<ROW_PLANE>(tmem + BK_U, slot, q_addr, na);
-            mma_commit(&u_full[0]);
-            if (r > 0) {
-              issue_z(T - 1, 0);
-              w.wait(&u_free[1], (T - 1) & 1, 0x3A);
-            }
-            if (nb2) {
-              fence_after_sync();
-              issue_term<ROW_PLANE>(tmem + BK_U + 64, slot, q_addr + 64 * 16, nb2);
-            }
-            mma_commit(&u_full[1]);            // also: the term's slot has been read
-            if (r > 0) issue_z(T - 1, 1);
-          }
-          issue_z(T - 1, 0);
-          issue_z(T - 1, 1);
-          w.wait(&w_full, i & 1, 0x3B);
-          fence_after_sync();
-          // dU (+)= W^T G: the weights' bf16 values, then their remainders, then the values against G's remainders
-          for (int part = 0; part < (FINE ? 3 : 2); ++part)
-            for (int ks = 0; ks < cols / 16; ++ks)
-              mma_bf16_ts(tmem + BK_V, tmem + (part == 1 ? BK_PLO : BK_P) + 8 * ks, desc_advance(part == 2 ? dg_lo : dg, ks * 256),
-                          instr_desc_bf16(128, HD, 0, 1), i + part + ks > 0);
-          mma_commit(&v_full);
         }
+        T += rank;
+        if (i + 1 < n_heads) head_dw(i + 1);
+        w.wait(&w_full, i & 1, 0x35);
+        fence_after_sync();
+        // dU (+)= W^T G: the weights' bf16 values, then their remainders, then the values against G's remainders
+        for (int part = 0; part < (FINE ? 3 : 2); ++part)
+          for (int ks = 0; ks < cols / 16; ++ks)
+            mma_bf16_ts(tmem + BK_V, tmem + (part == 1 ? BK_PLO : BK_P) + 8 * ks, desc_advance(part == 2 ? dg_lo : dg, ks * 256),
+                        instr_desc_bf16(128, HD, 0, 1), i + part + ks > 0);
+        mma_commit(&v_full);
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else {
-    registers_up_to<112>();
+    registers_up_to<KvWarps<FINE>::REGS>();
+    constexpr int BLOCKS = 8 / SUBS, DIMS = HD / SUBS, PIECES = DIMS / 8;     // 16 queries, dims and pieces of 8 dims per warp
+    const int sub = warp >> 2, m = lane & 3, d0 = DIMS * sub;
     const unsigned char* xrow = Kimg + row * 16;
-    const int d0 = 16 * sub;
-    // this warp's queries: a quarter of each half, in blocks of 8; blocks before the diagonal stay zero in P^T and W^T
-    const auto col_of = [&](int hf, int x) { return 64 * hf + sub * ((hf ? nb2 : na) / 4) + 8 * x; };
-    const auto exists = [&](int hf, int x) { return 32 * x < (hf ? nb2 : na); };
-    const auto on = [&](int hf, int x) { return exists(hf, x) && col_of(hf, x) + 7 >= 32 * qd; };
+    // this warp's queries: blocks of 16, half of some 32s; blocks before the diagonal stay zero in P^T and W^T
+    const auto block_of = [&](int x) { return x * (SUBS / 2) + (sub >> 1); };
+    const auto col_of = [&](int x) { return 32 * block_of(x) + 16 * (sub & 1); };
+    const auto exists = [&](int x) { return 32 * block_of(x) < cols; };
+    const auto on = [&](int x) { return exists(x) && block_of(x) >= qd; };
+    const uint32_t zero[8] = {};
 #pragma unroll
-    for (int hf = 0; hf < 2; ++hf)
+    for (int x = 0; x < BLOCKS; ++x)
+      if (exists(x) && !on(x)) {
+        tmem_st8(tmem + BK_P + lane_off + col_of(x) / 2, zero);
+        if (FINE) tmem_st8(tmem + BK_PLO + lane_off + col_of(x) / 2, zero);
+      }
+    // keys lane / 4 + 8 t, dims d0 + 8 j + 2 m, + 1: the arrangement in which Z is drained
+    f32x2 dk[4][PIECES];
 #pragma unroll
-      for (int x = 0; x < 2; ++x)
-        if (exists(hf, x) && !on(hf, x)) {
-          tmem_st4(tmem + BK_P + lane_off + col_of(hf, x) / 2, 0u, 0u, 0u, 0u);
-          tmem_st4(tmem + BK_PLO + lane_off + col_of(hf, x) / 2, 0u, 0u, 0u, 0u);
-        }
-    w.wait(&u_in, 0, 0x3F);
-    f32x2 dk[8];
+    for (int t = 0; t < 4; ++t)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dk[j] = 0ull;
+      for (int j = 0; j < PIECES; ++j) dk[t][j] = 0ull;
+    const auto load_rows_of = [&](uint32_t at, f32x2 (&v)[4][PIECES]) {
+      float z[2][4 * PIECES];
+      tmem_ld_rows(at + lane_off + d0, z[0]);
+      tmem_ld_rows(at + lane_off + d0 + (16u << 16), z[1]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j) v[t][j] = f2_pack(z[t >> 1][4 * j + 2 * (t & 1)], z[t >> 1][4 * j + 2 * (t & 1) + 1]);
+    };
+    w.wait(&u_in, 0, 0x36);
     int T = 0;
     for (int i = 0; i < n_heads; ++i) {
       const float* l = reinterpret_cast<const float*>(heads + (i & 1) * BK_HEAD_BYTES + ROW_IMAGE_BYTES + 2 * SLAB_S_BYTES);
       const HeadScalars& hs = sc[i & 1];
-      w.wait(&g_full[i & 1], (i >> 1) & 1, 0x3C);             // l and the scalars are read below
-      if (i > 0) w.wait(&v_full, (i - 1) & 1, 0x3D);          // W^T of the previous head has been read
+      w.wait(&head_in[i & 1], (i >> 1) & 1, 0x37);
       __syncwarp();
       const int rpos = uniform(hs.rpos);
       const auto build = [&](int r) {
-        build_term16<ROW_PLANE>(tmem + BK_TERM + ((T + r) & 1) * TERM_COLS + lane_off, xrow, l + r * HD, d0);
-        tmem_st_wait();
-        fence_before_sync();
-        warp_arrive(&term_full[(T + r) & 1], lane);
+        const uint32_t slot = tmem + BK_TERM + ((T + r) & 1) * TERM_COLS + lane_off;
+#pragma unroll
+        for (int d = 0; d < DIMS; d += 16) build_term16<ROW_PLANE>(slot, xrow, l + r * HD, d0 + d);
       };
       build(0);
-      f32x2 dw[2][2][4], wt[2][2][4];
-      w.wait(&dw_full, i & 1, 0x3E);
+      f32x2 dw[BLOCKS][8], wt[BLOCKS][8];
+      const f32x2 w0 = f2_bcast(hs.w0);
+      w.wait(&dw_full, i & 1, 0x38);
+      __syncwarp();
       fence_after_sync();
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf)
+      for (int x = 0; x < BLOCKS; ++x)
+        if (on(x)) {
+          float d[16];
+          tmem_ld16(tmem + BK_U + lane_off + col_of(x), d);
+          tmem_ld_wait();
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (on(hf, x)) {
-            float d[8];
-            tmem_ld8(tmem + BK_U + lane_off + col_of(hf, x), d);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int i0 = col_of(hf, x) + 2 * j;             // query not earlier than the key
-              dw[hf][x][j] = f2_pack(i0 >= row ? 2.f * d[2 * j] : 0.f, i0 + 1 >= row ? 2.f * d[2 * j + 1] : 0.f);
-              wt[hf][x][j] = f2_bcast(hs.w0);
-            }
+          for (int j = 0; j < 8; ++j) {
+            const int i0 = col_of(x) + 2 * j;                 // query not earlier than the key
+            dw[x][j] = f2_pack(i0 >= row ? 2.f * d[2 * j] : 0.f, i0 + 1 >= row ? 2.f * d[2 * j + 1] : 0.f);
+            wt[x][j] = w0;
           }
+        }
+      tmem_st_wait();
       fence_before_sync();
-      warp_arrive(&dw_free, lane);
+      warp_arrive(&ready, lane);
       const auto drain = [&](int r) {
-        float z[16];
-        tmem_ld16(tmem + BK_Z + lane_off + d0, z);
-        tmem_ld_wait();
-        fence_before_sync();
-        warp_arrive(&z_free, lane);
+        f32x2 z[4][PIECES], lv[PIECES];
         const f32x2 sgn = f2_bcast(r < rpos ? 1.f : -1.f);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const ulonglong2 lv = *reinterpret_cast<const ulonglong2*>(l + r * HD + d0 + 4 * j);
-          dk[2 * j] = f2_fma(f2_mul(lv.x, sgn), f2_pack(z[4 * j], z[4 * j + 1]), dk[2 * j]);
-          dk[2 * j + 1] = f2_fma(f2_mul(lv.y, sgn), f2_pack(z[4 * j + 2], z[4 * j + 3]), dk[2 * j + 1]);
-        }
+        for (int j = 0; j < PIECES; ++j) lv[j] = f2_mul(*reinterpret_cast<const f32x2*>(l + r * HD + d0 + 2 * m + 8 * j), sgn);
+        load_rows_of(z_at(r), z);
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j)
+#pragma unroll
+          for (int t = 0; t < 4; ++t) dk[t][j] = f2_fma(lv[j], z[t][j], dk[t][j]);
       };
       for (int r = 0; r < rank; ++r) {
-        // the next term is built while the MMAs of this one run; its slot's last reader was term r - 1, complete
-        // since u_full[1](r - 1)
+        // the next term's slot was last read for U of r - 1, which has arrived
         if (r + 1 < rank) build(r + 1);
         const f32x2 c2 = f2_bcast(hs.c[r]), sgn = f2_bcast(r < rpos ? 1.f : -1.f);
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          w.wait(&u_full[hf], (T + r) & 1, 0x40 + hf);
-          fence_after_sync();
-          float u[2][8];
-#pragma unroll
-          for (int x = 0; x < 2; ++x)
-            if (on(hf, x)) tmem_ld8(tmem + BK_U + lane_off + col_of(hf, x), u[x]);
+        w.wait(&u_full, (T + r) & 1, 0x39);
+        __syncwarp();
+        fence_after_sync();
+        uint32_t p[BLOCKS / 2][8], rest[BLOCKS / 2][8];
+        const auto products = [&](int x, int k) {
+          float u[16];
+          tmem_ld16(tmem + BK_U + lane_off + col_of(x), u);
           tmem_ld_wait();
-          fence_before_sync();
-          warp_arrive(&u_free[hf], lane);
-          uint32_t p[2][4], rest[2][4];
 #pragma unroll
-          for (int x = 0; x < 2; ++x)
-            if (on(hf, x)) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const f32x2 u2 = f2_add(f2_pack(u[x][2 * j], u[x][2 * j + 1]), c2);
-                float t0, t1;
-                f2_unpack(f2_mul(dw[hf][x][j], u2), t0, t1);
-                p[x][j] = pack_bf16(t0, t1);
-                if (FINE) rest[x][j] = pack_bf16(t0 - bf16_lo(p[x][j]), t1 - bf16_hi(p[x][j]));
-                wt[hf][x][j] = f2_fma(rpos == rank ? u2 : f2_mul(u2, sgn), u2, wt[hf][x][j]);
-              }
-            }
-          if (r > 0) {                         // the previous term's P^T has been read
-            w.wait(&z_half[hf], (T + r - 1) & 1, 0x42 + hf);
-            fence_after_sync();
+          for (int j = 0; j < 8; ++j) {
+            const f32x2 u2 = f2_add(f2_pack(u[2 * j], u[2 * j + 1]), c2);
+            float t0, t1;
+            f2_unpack(f2_mul(dw[x][j], u2), t0, t1);
+            p[k][j] = pack_bf16(t0, t1);
+            if (FINE) rest[k][j] = pack_bf16(t0 - bf16_lo(p[k][j]), t1 - bf16_hi(p[k][j]));
+            wt[x][j] = f2_fma(rpos == rank ? u2 : f2_mul(u2, sgn), u2, wt[x][j]);
           }
+        };
+        const auto store = [&](int x, int k) {
+          tmem_st8(tmem + BK_P + lane_off + col_of(x) / 2, p[k]);
+          if (FINE) tmem_st8(tmem + BK_PLO + lane_off + col_of(x) / 2, rest[k]);
+        };
 #pragma unroll
-          for (int x = 0; x < 2; ++x)
-            if (on(hf, x)) {
-              const uint32_t at = lane_off + col_of(hf, x) / 2;
-              tmem_st4(tmem + BK_P + at, p[x][0], p[x][1], p[x][2], p[x][3]);
-              if (FINE) tmem_st4(tmem + BK_PLO + at, rest[x][0], rest[x][1], rest[x][2], rest[x][3]);
-            }
-          tmem_st_wait();
-          fence_before_sync();
-          // the whole Z of the previous term is complete: out of the way before the next one starts
-          if (hf == 1 && r > 0) drain(r - 1);
-          warp_arrive(&p_full[hf], lane);
-        }
+        for (int x = 0; x < BLOCKS / 2; ++x)
+          if (on(x)) products(x, x);
+        // P^T of the previous term, or W^T of the previous head, has been read
+        if (r > 0) w.wait(&z_full, (T + r - 1) & 1, 0x3A);
+        else if (i > 0) w.wait(&v_full, (i - 1) & 1, 0x3B);
+        __syncwarp();
+        fence_after_sync();
+#pragma unroll
+        for (int x = 0; x < BLOCKS / 2; ++x)
+          if (on(x)) store(x, x);
+#pragma unroll
+        for (int x = BLOCKS / 2; x < BLOCKS; ++x)
+          if (on(x)) {
+            products(x, x - BLOCKS / 2);
+            store(x, x - BLOCKS / 2);
+          }
+        if (FINE && r > 0) drain(r - 1);
+        tmem_st_wait();
+        fence_before_sync();
+        warp_arrive(&ready, lane);
+        if (!FINE && r > 0) drain(r - 1);
       }
-      w.wait(&z_half[0], (T + rank - 1) & 1, 0x44);
-      w.wait(&z_half[1], (T + rank - 1) & 1, 0x45);
+      w.wait(&z_full, (T + rank - 1) & 1, 0x3C);
+      __syncwarp();
       fence_after_sync();
       drain(rank - 1);
-      // W^T and its remainders in the place of P^T and its, whose last readers are complete
+      // W^T and its remainders in the place of P^T and its, or of the second Z, whose readers of this quadrant are done
+      fence_before_sync();
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + qd), "n"(SUBS * 32) : "memory");
+      fence_after_sync();
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf)
+      for (int x = 0; x < BLOCKS; ++x)
+        if (on(x)) {
+          uint32_t o[8], rest[8];
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (on(hf, x)) {
-            uint32_t o[4], rest[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float w_a, w_b;
-              f2_unpack(wt[hf][x][j], w_a, w_b);
-              const int i0 = col_of(hf, x) + 2 * j;
-              if (i0 < row) w_a = 0.f;
-              if (i0 + 1 < row) w_b = 0.f;
-              o[j] = pack_bf16(w_a, w_b);
-              rest[j] = pack_bf16(w_a - bf16_lo(o[j]), w_b - bf16_hi(o[j]));
-            }
-            const uint32_t at = lane_off + col_of(hf, x) / 2;
-            tmem_st4(tmem + BK_P + at, o[0], o[1], o[2], o[3]);
-            tmem_st4(tmem + BK_PLO + at, rest[0], rest[1], rest[2], rest[3]);
+          for (int j = 0; j < 8; ++j) {
+            float w_a, w_b;
+            f2_unpack(wt[x][j], w_a, w_b);
+            const int i0 = col_of(x) + 2 * j;
+            if (i0 < row) w_a = 0.f;
+            if (i0 + 1 < row) w_b = 0.f;
+            o[j] = pack_bf16(w_a, w_b);
+            rest[j] = pack_bf16(w_a - bf16_lo(o[j]), w_b - bf16_hi(o[j]));
           }
+          tmem_st8(tmem + BK_P + lane_off + col_of(x) / 2, o);
+          tmem_st8(tmem + BK_PLO + lane_off + col_of(x) / 2, rest);
+        } else if (!FINE && exists(x)) {
+          tmem_st8(tmem + BK_PLO + lane_off + col_of(x) / 2, zero);
+        }
       tmem_st_wait();
       fence_before_sync();
       warp_arrive(&w_full, lane);
       T += rank;
     }
-    w.wait(&v_full, (n_heads - 1) & 1, 0x46);
-    fence_after_sync();
-    float z[16], v[16];
-    tmem_ld16(tmem + BK_V + lane_off + d0, z);
-    tmem_ld_wait();
+    const int rows = max(nc - 32 * qd, 0);                    // of the quadrant that exist
+    const size_t tok = (size_t)tok0 + 32 * qd + (lane >> 2);
+    const size_t out0 = (((size_t)b * a.Hkv + kvh) * a.N + tok) * HD + d0 + 2 * m;
+    const size_t part0 = ((((size_t)b * a.Hkv + kvh) * a.parts + part) * a.N + tok) * HD + d0 + 2 * m;
+    const auto write = [&](const f32x2 (&v)[4][PIECES], float* partial, const float* cross, __nv_bfloat16* out) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f2_unpack(dk[j], v[2 * j], v[2 * j + 1]);
-    if (row < nc && !dead) {
-      // 16 consecutive dims of a row per thread: whole sectors
-      const auto write = [&](float (&x)[16], float* partial, const float* cross, __nv_bfloat16* out) {
-        if (partial) {
-          float* dst = partial + ((((size_t)b * a.Hkv + kvh) * a.parts + part) * a.N + tok0 + row) * HD + d0;
+      for (int t = 0; t < 4; ++t) {
+        if ((lane >> 2) + 8 * t >= rows) continue;
+        const bool add = cross && (int)tok + 8 * t < a.cross_end;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(dst + 4 * j) = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
-        } else if (out) {
-          const size_t o = (koff + row) * HD + d0;
-          if (cross && tok0 + row < a.cross_end) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float4 t = *reinterpret_cast<const float4*>(cross + o + 4 * j);
-              x[4 * j] += t.x; x[4 * j + 1] += t.y; x[4 * j + 2] += t.z; x[4 * j + 3] += t.w;
-            }
+        for (int j = 0; j < PIECES; ++j) {
+          float x0, x1;
+          f2_unpack(v[t][j], x0, x1);
+          const size_t at = 8 * t * HD + 8 * j;
+          if (partial) {
+            *reinterpret_cast<float2*>(partial + part0 + at) = make_float2(x0, x1);
+          } else if (out) {
+            const float2 z = add ? *reinterpret_cast<const float2*>(cross + out0 + at) : make_float2(0.f, 0.f);
+            *reinterpret_cast<uint32_t*>(out + out0 + at) = pack_bf16(x0 + z.x, x1 + z.y);
           }
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-            *reinterpret_cast<uint4*>(out + o + 8 * j) =
-                make_uint4(pack_bf16(x[8 * j], x[8 * j + 1]), pack_bf16(x[8 * j + 2], x[8 * j + 3]),
-                           pack_bf16(x[8 * j + 4], x[8 * j + 5]), pack_bf16(x[8 * j + 6], x[8 * j + 7]));
         }
-      };
-      write(v, a.dk_part, a.dk_cross, a.dk);
-      write(z, a.dv_part, a.dv_cross, a.dv);
-    }
+      }
+    };
+    if (!dead) write(dk, a.dk_part, a.dk_cross, a.dk);
+    w.wait(&v_full, (n_heads - 1) & 1, 0x3D);
+    __syncwarp();
+    fence_after_sync();
+    load_rows_of(tmem + BK_V, dk);
+    if (!dead) write(dk, a.dv_part, a.dv_cross, a.dv);
   }
   fence_before_sync();
   __syncthreads();
@@ -826,8 +822,8 @@ cudaError_t intra_backward_kv(const RowImages& rows, const void* gimg, const voi
     a.dk_cross = dk_cross; a.dv_cross = dv_cross;
   }
   const dim3 grid(NB, B * Hkv, a.parts);
-  if (fine) intra_bwd_kv_kernel<true><<<grid, BW_THREADS, BK_SMEM, st>>>(a);
-  else intra_bwd_kv_kernel<false><<<grid, BW_THREADS, BK_SMEM, st>>>(a);
+  if (fine) intra_bwd_kv_kernel<true><<<grid, KvWarps<true>::THREADS, BK_SMEM, st>>>(a);
+  else intra_bwd_kv_kernel<false><<<grid, KvWarps<false>::THREADS, BK_SMEM, st>>>(a);
   if (a.parts == 1 || (e = cudaGetLastError()) != cudaSuccess) return cudaGetLastError();
   KvReduceArgs r{{dk_part, dv_part}, {dk_cross, dv_cross}, {static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv)},
                  B, Hkv, a.parts, N, cross_end};

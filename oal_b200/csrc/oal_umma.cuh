@@ -190,7 +190,7 @@ __device__ __forceinline__ void tmem_st_rows16(uint32_t taddr, const uint32_t (&
       : "memory");
 }
 // 16 lanes x 32 columns, the same arrangement, tensor memory -> registers.
-__device__ __forceinline__ void tmem_ld_rows16(uint32_t taddr, float (&v)[16]) {
+__device__ __forceinline__ void tmem_ld_rows(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
   asm volatile(
       "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -200,6 +200,16 @@ __device__ __forceinline__ void tmem_ld_rows16(uint32_t taddr, float (&v)[16]) {
       : "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+// 16 lanes x 16 columns of that arrangement.
+__device__ __forceinline__ void tmem_ld_rows(uint32_t taddr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
