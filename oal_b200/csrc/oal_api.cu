@@ -412,7 +412,6 @@ ChunkRange chunk_range(const OalProblem* p, const void* state_in, const void* ds
 
 struct ForwardSpaceTC {
   float* ds;
-  int32_t* update_status;
   size_t bytes;
 };
 
@@ -429,7 +428,6 @@ ForwardSpaceTC carve_forward_tc(const OalProblem* p, void* ws) {
   ForwardSpaceTC s;
   const size_t units = (size_t)p->batch * p->kv_heads;
   s.ds = c.take<float>(units * chunk_count(p) * oal::state_rows() * oal::EP);
-  s.update_status = c.take<int32_t>(oal::state_update_blocks((int)units, chunk_count(p)));
   s.bytes = c.off;
   return s;
 }
@@ -437,13 +435,17 @@ ForwardSpaceTC carve_forward_tc(const OalProblem* p, void* ws) {
 // The buffer the forward hands to the backward: the bf16 carry images of every chunk (the MMA operand),
 // the images of their rounding remainders (read only by the coefficient-gradient dot products), then the
 // per-head factor table of the intra-chunk kernels and the per-feature coefficient table of the state kernels
-// (the backward of the same call sees the same coefficients).
+// (the backward of the same call sees the same coefficients), then the images of the rows of k and [v | 1].
 size_t saved_images_bytes_tc(const OalProblem* p) {
   return align_up((size_t)p->batch * p->kv_heads * chunk_count(p) * oal::state_image_bytes_per_chunk());
 }
 size_t saved_factors_bytes_tc(const OalProblem* p) { return align_up(oal::head_factor_bytes(p->q_heads)); }
-size_t saved_state_bytes_tc(const OalProblem* p) {
+size_t saved_rows_offset_tc(const OalProblem* p) {
   return 2 * saved_images_bytes_tc(p) + saved_factors_bytes_tc(p) + align_up((size_t)p->q_heads * oal::state_rows() * sizeof(float));
+}
+size_t k_image_bytes_tc(const OalProblem* p) { return align_up((size_t)p->batch * p->kv_heads * chunk_count(p) * oal::ROW_IMAGE_BYTES); }
+size_t saved_state_bytes_tc(const OalProblem* p) {
+  return saved_rows_offset_tc(p) + k_image_bytes_tc(p) + align_up((size_t)p->batch * p->kv_heads * chunk_count(p) * oal::state_slab_image_bytes());
 }
 char* saved_at(const void* saved_state, size_t offset) {
   return const_cast<char*>(static_cast<const char*>(saved_state)) + offset;
@@ -454,10 +456,15 @@ float* saved_coef_table(const OalProblem* p, const void* saved_state) {
   return reinterpret_cast<float*>(saved_at(saved_state, 2 * saved_images_bytes_tc(p) + saved_factors_bytes_tc(p)));
 }
 
+oal::RowImages row_images(const OalProblem* p, const void* saved_state, const void* q, const void* k, const void* v, void* q_image) {
+  char* rows = saved_at(saved_state, saved_rows_offset_tc(p));
+  return oal::RowImages{q, k, v, q_image, rows, rows + k_image_bytes_tc(p)};
+}
+
 struct BackwardSpaceTC {
   float* coef_blocks;            // coefficient partial sums of the query row blocks
   void* gimg;
-  void *q_image, *k_image, *u_image;      // rows of q, k and [v | 1] as operand images
+  void* q_image;                 // rows of q as operand images
   float* dcarry;
   void* dt_img;
   float* dcoef_partial;
@@ -479,8 +486,6 @@ BackwardSpaceTC carve_backward_tc(const OalProblem* p, void* ws) {
   s.coef_blocks = c.take<float>((size_t)p->batch * p->q_heads * oal::intra_row_blocks(p->seq_len) * (1 + p->groups + p->groups * (p->groups + 1) / 2));
   s.gimg = c.take<char>(2 * (size_t)p->batch * p->q_heads * nb * slab_image);   // hi image, then lo image
   s.q_image = c.take<char>((size_t)p->batch * p->q_heads * nb * oal::ROW_IMAGE_BYTES);
-  s.k_image = c.take<char>(units * nb * oal::ROW_IMAGE_BYTES);
-  s.u_image = c.take<char>(units * nb * slab_image);
   s.dcarry = c.take<float>(units * nb * oal::state_rows() * oal::EP);
   s.dt_img = c.take<char>(units * nb * oal::state_image_bytes_per_chunk());
   s.dcoef_partial = c.take<float>(2 * (size_t)p->batch * nb * p->q_heads * oal::state_rows());   // two column halves
@@ -498,16 +503,12 @@ BackwardSpaceTC carve_backward_tc(const OalProblem* p, void* ws) {
 
 // Stage A of the tensor-core backward: everything that does not depend on later tokens' state
 // gradient (normalisation VJP, per-chunk dCarry and coefficient partial sums).
-oal::RowImages row_images(const BackwardSpaceTC& s, const void* q, const void* k, const void* v) {
-  return oal::RowImages{q, k, v, s.q_image, s.k_image, s.u_image};
-}
 int backward_vjp(const OalProblem* p, const float* num, const float* den, const void* grad_out, const float* grad_num,
                  const float* grad_den, const BackwardSpaceTC& s, const oal::RowImages& rows, int32_t* clear_status, cudaStream_t st) {
   LaunchScope scope("norm_vjp", st);
   const cudaError_t e = oal::norm_vjp_image(grad_out, p->out_dtype, grad_num, grad_den, num, den, p->floor, s.gimg,
-                                            rows.q ? p->batch * p->q_heads : 0, p->seq_len, chunk_count(p),
-                                            (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) ? p->q_heads : 0, rows, p->batch * p->kv_heads,
-                                            clear_status, st);
+                                            p->batch * p->q_heads, p->seq_len, chunk_count(p),
+                                            (p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) ? p->q_heads : 0, rows, clear_status, st);
   return e == cudaSuccess ? OAL_OK : fail_cuda(e, "normalisation VJP kernel");
 }
 int backward_dstate(const OalProblem* p, const void* saved_state, const ChunkRange& cr, const BackwardSpaceTC& s,
@@ -539,7 +540,7 @@ oal::PairArgs base_args(const OalProblem* p, const void* q, const void* k, const
 // ---- forward ------------------------------------------------------------------------------------
 int forward_core(const OalProblem* p, const void* q, const void* k, const void* v, const int32_t* dim_perm,
                  const int32_t* group_start, const CoefSource& src, void* out, float* num, float* den, void* saved_state,
-                 const float* state_in, float* ds, int32_t* update_status, int32_t* status, oal::StatusSink sink, bool timing,
+                 const float* state_in, float* ds, int32_t* status, oal::StatusSink sink, bool timing,
                  cudaStream_t st) {
   cudaError_t e;
   const bool tc = p->precision == OAL_PRECISION_BF16_TENSORCORE;
@@ -554,14 +555,15 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
   SideWork beside;
   cudaStream_t s0 = st;
   oal::PrologueArgs pro{};
+  const oal::RowImages rows = tc ? row_images(p, saved_state, q, k, v, nullptr) : oal::RowImages{};
   if (src.factor) {
     pro = prologue_args(p, src, dim_perm, group_start, coef_table, factors, status, sink.host ? sink.counter : nullptr);
-    if (!update) {
+    if (!tc) {
       LaunchScope scope("head_prologue", st, 1, timing);
       if ((e = oal::launch_head_prologue(pro, p->q_heads, st)) != cudaSuccess) return fail_cuda(e, "prologue kernel");
-    } else if (timing && (side = side_streams(side_lock))) {
+    } else if (cr.n > 0 && timing && (side = side_streams(side_lock))) {
       // The rotations (11 us at 8 groups, 45 at 16) are needed by the call's last kernel only, the coefficients by the
-      // next but one: with both in the state kernel's launch the scan waited for the rotations.  Beside the state
+      // next but one: with both in one launch the state kernels waited for the rotations.  Beside the state
       // kernels they cost the host a launch and two events.  14 / 2 heads, B = 1, both forms in us: forward + backward
       // N = 256 169 -> 160, N = 1024 198 -> 190, replayed 203 -> 192, 16 groups N = 4096 663 -> 647.
       s0 = beside.fork(side, 0, st);
@@ -584,17 +586,27 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
     e = oal::build_coef_table(dim_perm, group_start, src.A, src.B, src.C, p->q_heads, p->groups, p->scale, coef_table, st);
     if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
   }
-  if (update) {
+  if (tc) {
+    LaunchScope scope("rows_prologue", st, 1, timing);
+    e = oal::rows_prologue(rows, units, p->seq_len, nb, src.factor ? &pro : nullptr, p->q_heads, st);
+    if (e != cudaSuccess) return fail_cuda(e, "row image kernel");
+  }
+  const bool walk = update && timing && oal::state_walk_pays(units, nb);
+  if (walk) {
+    LaunchScope scope("state_walk", st, 1, timing);
+    e = oal::state_walk(rows, saved_state, saved_remainders(p, saved_state), state_in, units, p->seq_len, nb, cr.trim, status, st);
+    if (e != cudaSuccess) return fail_cuda(e, "state walk kernel");
+  } else if (update) {
     LaunchScope scope("state_update", st, 1, timing);
-    e = oal::state_update(k, v, ds, units, p->seq_len, nb, cr.n, src.factor ? &pro : nullptr, p->q_heads, status,
-                          src.factor ? update_status : nullptr, st);
+    e = oal::state_update(k, v, ds, units, p->seq_len, nb, cr.n, status, st);
     if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
   }
   if (tc && cr.n > 0) {
-    { LaunchScope scope("state_scan", st, 1, timing);
-      e = oal::state_scan(ds, saved_state, saved_remainders(p, saved_state), state_in, nullptr, units, nb, 0, cr.trim,
-                          update && src.factor ? update_status : nullptr, oal::state_update_blocks(units, cr.n), status, st); }
-    if (e != cudaSuccess) return fail_cuda(e, "state scan kernel");
+    if (!walk) {
+      LaunchScope scope("state_scan", st, 1, timing);
+      e = oal::state_scan(ds, saved_state, saved_remainders(p, saved_state), state_in, nullptr, units, nb, 0, cr.trim, st);
+      if (e != cudaSuccess) return fail_cuda(e, "state scan kernel");
+    }
     { LaunchScope scope("cross_read_q", st, 1, timing);
       e = oal::cross_read(true, q, saved_state, coef_table, num, den, p->batch, p->q_heads, p->q_heads / p->kv_heads,
                           p->seq_len, nb, cr.first, cr.n, status, st); }
@@ -712,14 +724,11 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   const ChunkRange cr = chunk_range(p, nullptr, x.dstate_in);
   const void* factors = saved_factors(p, x.saved_state);      // written by the forward of this call
   const float* coef_table = saved_coef_table(p, x.saved_state);
-  const oal::RowImages rows = row_images(s, x.q, x.k, x.v);
+  const oal::RowImages rows = row_images(p, x.saved_state, x.q, x.k, x.v, s.q_image);
   cudaError_t e;
   if (!reuse) {
     if (int rc = backward_vjp(p, x.num, x.den, x.grad_out, x.grad_num, x.grad_den, s, rows, x.clear_status ? x.status : nullptr, st)) return rc;
     if (int rc = backward_dstate(p, x.saved_state, cr, s, x.status, st)) return rc;
-  } else {
-    // oal_backward_local_state left the images of q and G; it has not seen k and v
-    if (int rc = backward_vjp(p, x.num, x.den, nullptr, nullptr, nullptr, s, row_images(s, nullptr, x.k, x.v), nullptr, st)) return rc;
   }
   // Three chains leave the state stage: the query side (on the caller's stream), the key/value side and
   // the reduction of the cross-chunk coefficient gradient.  They share no buffer, so the last two run on
@@ -738,11 +747,11 @@ int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& 
   }
   if (want_kv && cross) {
     { LaunchScope scope("state_scan_reverse", skv);
-      e = oal::state_scan(s.dcarry, s.dt_img, nullptr, x.dstate_in, nullptr, units, nb, 1, cr.trim, nullptr, 0, nullptr, skv); }
+      e = oal::state_scan(s.dcarry, s.dt_img, nullptr, x.dstate_in, nullptr, units, nb, 1, cr.trim, skv); }
     if (e != cudaSuccess) return fail_cuda(e, "reverse state scan kernel");
     if (want_k) {
       { LaunchScope scope("feature_grad_k", skv);
-        e = oal::feature_grad(false, s.k_image, s.u_image, s.dt_img, nullptr, s.dk_cross, p->batch, p->kv_heads, 1,
+        e = oal::feature_grad(false, rows.k_image, rows.u_image, s.dt_img, nullptr, s.dk_cross, p->batch, p->kv_heads, 1,
                               p->seq_len, nb, 0, cr.n, x.status, skv); }
       if (e != cudaSuccess) return fail_cuda(e, "key feature gradient kernel");
     }
@@ -888,7 +897,6 @@ static int forward_entry(const OalProblem* p, const void* q, const void* k, cons
   if (!q || !k || !v || !dim_perm || !group_start || !src.A || !src.B || !src.C || !out || !num || !den || !status)
     return fail(OAL_ERR_ARGUMENT, "oal_forward: NULL tensor pointer");
   float* ds = nullptr;
-  int32_t* update_status = nullptr;
   if (p->precision == OAL_PRECISION_FP32_IEEE) {
     if (state_in) return fail(OAL_ERR_ARGUMENT, "fp32_ieee mode keeps no chunk state: state_in must be NULL");
   } else {
@@ -897,9 +905,8 @@ static int forward_entry(const OalProblem* p, const void* q, const void* k, cons
     if (!workspace || workspace_bytes < s.bytes) return fail(OAL_ERR_WORKSPACE, "oal_forward: workspace too small");
     if (!saved_state) return fail(OAL_ERR_ARGUMENT, "oal_forward: saved_state is NULL");
     ds = s.ds;
-    update_status = s.update_status;
   }
-  return forward_core(p, q, k, v, dim_perm, group_start, src, out, num, den, saved_state, state_in, ds, update_status, status, sink, true,
+  return forward_core(p, q, k, v, dim_perm, group_start, src, out, num, den, saved_state, state_in, ds, status, sink, true,
                       static_cast<cudaStream_t>(stream));
 }
 
@@ -1081,9 +1088,9 @@ int oal_forward_local_state(const OalProblem* p, const void* k, const void* v, f
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int units = p->batch * p->kv_heads, nb = chunk_count(p);
   cudaError_t e;
-  { LaunchScope scope("state_update", st); e = oal::state_update(k, v, s.ds, units, p->seq_len, nb, nb, nullptr, 0, status, nullptr, st); }
+  { LaunchScope scope("state_update", st); e = oal::state_update(k, v, s.ds, units, p->seq_len, nb, nb, status, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state update kernel");
-  { LaunchScope scope("state_total", st); e = oal::state_scan(s.ds, nullptr, nullptr, nullptr, state_total, units, nb, 0, false, nullptr, 0, nullptr, st); }
+  { LaunchScope scope("state_total", st); e = oal::state_scan(s.ds, nullptr, nullptr, nullptr, state_total, units, nb, 0, false, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state total kernel");
   return OAL_OK;
 }
@@ -1106,12 +1113,11 @@ int oal_backward_local_state(const OalProblem* p, const void* q, const int32_t* 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   OalProblem local = *p;
   local.grad_mask |= OAL_GRAD_K;      // dCarry is needed whatever the caller finally asks for
-  if ((rc = backward_vjp(&local, num, den, grad_out, grad_num, grad_den, s, row_images(s, q, nullptr, nullptr), nullptr, st))) return rc;
+  if ((rc = backward_vjp(&local, num, den, grad_out, grad_num, grad_den, s, row_images(&local, saved_state, q, nullptr, nullptr, s.q_image), nullptr, st))) return rc;
   if ((rc = backward_dstate(&local, saved_state, ChunkRange{false, chunk_count(p), 0}, s, status, st))) return rc;
   cudaError_t e;
   { LaunchScope scope("state_total", st);
-    e = oal::state_scan(s.dcarry, nullptr, nullptr, nullptr, dstate_total, p->batch * p->kv_heads, chunk_count(p), 1, false, nullptr, 0,
-                        nullptr, st); }
+    e = oal::state_scan(s.dcarry, nullptr, nullptr, nullptr, dstate_total, p->batch * p->kv_heads, chunk_count(p), 1, false, st); }
   if (e != cudaSuccess) return fail_cuda(e, "state gradient total kernel");
   return OAL_OK;
 }
@@ -1177,7 +1183,7 @@ int oal_forward_static_scratch(const OalProblem* p, const void* q, const void* k
   rc = static_scratch_address(&scratch);
   if (rc) return rc;
   return forward_core(p, q, k, v, dim_perm, group_start, explicit_coefs(coef_a, coef_b, coef_c), out, num, den, saved_state,
-                      nullptr, scratch, nullptr, status, oal::StatusSink{nullptr, nullptr}, false, static_cast<cudaStream_t>(stream));
+                      nullptr, scratch, status, oal::StatusSink{nullptr, nullptr}, false, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

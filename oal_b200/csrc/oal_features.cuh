@@ -254,6 +254,14 @@ __device__ __forceinline__ void store_half_slab(int hs, const unsigned char* xla
   umma::tmem_st_rows16(slot + (16u << 16), o[1]);
 }
 
+// 16 bytes through the read-only path, issued where it stands: the compiler may move an ordinary load down to its first use,
+// behind the waits that it was meant to overlap.
+__device__ __forceinline__ uint4 load_ahead(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // Bounded mbarrier waits for one CTA: the first wait that expires raises a shared flag and every
 // later wait returns at once, so a kernel always terminates; the flag ends up in the status word.
 struct Waiter {

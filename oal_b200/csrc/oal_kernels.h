@@ -67,15 +67,23 @@ size_t state_slab_image_bytes();           // bytes of one slab image [10][128][
 cudaError_t build_coef_table(const int32_t* dim_perm, const int32_t* group_start, const float* A,
                              const float* Bc, const float* Cc, int Hq, int G, float scale, float* table,
                              cudaStream_t st);
-// increments of the first NC chunks; `prologue` (optional): its blocks ride in the same launch.  block_status: words
-// [state_update_blocks] for state_scan to merge, or null where no prologue clears `status` in this launch
-int state_update_blocks(int units, int NC);
-cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, const PrologueArgs* prologue,
-                         int q_heads, int32_t* status, int32_t* block_status, cudaStream_t st);
+// increments of the first NC chunks
+cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, int32_t* status, cudaStream_t st);
+// Operand images of the rows of q and k [B*H, NB, 8, 128, 8] and of [v | 1 | 0] [B*Hkv, NB, 10, 128, 8].
+struct RowImages {
+  const void *q, *k, *v;
+  void *q_image, *k_image, *u_image;
+};
+// images of k and [v | 1]; `prologue` (optional): its blocks ride in the same launch
+cudaError_t rows_prologue(const RowImages& rows, int units, int N, int NB, const PrologueArgs* prologue, int q_heads, cudaStream_t st);
+// both images of every chunk (trim: but the first), the running state kept on chip; state_walk_pays: faster than state_update
+// and state_scan
+bool state_walk_pays(int units, int NB);
+cudaError_t state_walk(const RowImages& rows, void* image, void* image_lo, const float* state_in, int units, int N, int NB, bool trim,
+                       int32_t* status, cudaStream_t st);
 // image_lo: optional second image holding bf16(state - bf16(state)); trim: see state_scan_kernel
 cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float* state_in, float* state_total,
-                       int units, int NB, int reverse, bool trim, const int32_t* block_status, int n_status, int32_t* status,
-                       cudaStream_t st);
+                       int units, int NB, int reverse, bool trim, cudaStream_t st);
 // chunks [c0, c0 + NC) of every sequence; the other rows of out64 / out1 are not written
 cudaError_t cross_read(bool query, const void* x, const void* image, const float* coef_table, float* out64,
                        float* out1, int B, int H, int rep, int N, int NB, int c0, int NC, int32_t* status, cudaStream_t st);
@@ -92,16 +100,11 @@ cudaError_t feature_grad(bool query, const void* x_image, const void* a_image, c
                          int32_t* status, cudaStream_t st);
 cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, int G, const int32_t* dim_perm,
                          const int32_t* group_start, float* dcoef, float* slots, cudaStream_t st);
-// Operand images of the rows of q and k [B*H, NB, 8, 128, 8] and of [v | 1 | 0] [B*Hkv, NB, 10, 128, 8]; k == null: q only
-struct RowImages {
-  const void *q, *k, *v;
-  void *q_image, *k_image, *u_image;
-};
-// heads = B * Hq (0: only the images of k and v), kv_heads = B * Hkv
+// writes the images of G and of q
 cudaError_t norm_vjp_image(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                            const float* num, const float* den, float floor_v, void* gimg, int heads,
                            int N, int NB, int token_major_heads /* > 0: grad_out is [B, N, Hq, 64] */, const RowImages& rows,
-                           int kv_heads, int32_t* clear_status, cudaStream_t st);
+                           int32_t* clear_status, cudaStream_t st);
 
 
 // ---- factored intra-chunk weight (oal_factor.cu) -----------------------------------------

@@ -3,9 +3,11 @@
 // Chunked causal scan of the reference (oal_attention/hd_block_gemm_runtime.py:271-320
 // block totals and exclusive cumsum, :552-560 cross contraction phi_q x carry) with 128-token
 // chunks:
-//   state_update : dS[u,c] = phi_k(chunk c)^T [v | 1]          (features are the MMA M dimension)
-//   state_scan   : carry[u,c] = state_in + sum_{c'<c} dS[u,c'] (fp32), stored as the bf16
+//   state_walk   : dS[u,c] = phi_k(chunk c)^T [v | 1]          (features are the MMA M dimension),
+//                  carry[u,c] = state_in + sum_{c'<c} dS[u,c'] (fp32), stored as the bf16
 //                  operand image the MMAs read
+//   state_update, state_scan : the same in two steps, increments in memory between them, for a range of a longer sequence
+//                  (the totals of the ranges are exchanged between the two) and as the reverse scan of the backward
 //   cross_read   : Y[i,:] = phi_q(i) . carry[u,c(i)]           (tokens are the MMA M dimension)
 // Feature tiles are generated on chip (oal_features.cuh), in shared memory or, for the cross read, straight in tensor
 // memory, and never touch HBM.
@@ -56,28 +58,45 @@ __global__ void coef_table_kernel(const int32_t* dim_perm, const int32_t* group_
 }
 
 // ---------------------------------------------------------------------------
+// First launch of a forward: the first `n_prologue` blocks compute the per-head prologue (oal_prologue.cuh), the others write
+// the rows of k and of [v | 1 | 0] as operand images, which the state walk and the backward kernels fetch with bulk copies.
+//   Image blocks: 32 consecutive tokens of one (unit, chunk); warp = 8 consecutive columns, lane = token, so a warp stores 512
+//   contiguous bytes.  Rows are enumerated over padded chunks: zeros past the end of the sequence.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) rows_prologue_kernel(const PrologueArgs pro, int n_prologue, const RowImages rows, int N, int NB) {
+  __shared__ PrologueSmem smem;
+  if ((int)blockIdx.x < n_prologue) {
+    head_prologue(pro, blockIdx.x, smem, threadIdx.x, 256);
+    return;
+  }
+  const int ec = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t per_unit = (size_t)NB * CT, r = (size_t)(blockIdx.x - n_prologue) * 32 + lane, u = r / per_unit;
+  const int t = (int)(r % per_unit), tl = t % CT;
+  const bool live = t < N;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const size_t at = (u * N + t) * HD + 8 * ec, chunk = u * NB + t / CT;
+  uint4* k_out = reinterpret_cast<uint4*>(static_cast<unsigned char*>(rows.k_image) + chunk * ROW_IMAGE_BYTES);
+  uint4* u_out = reinterpret_cast<uint4*>(static_cast<unsigned char*>(rows.u_image) + chunk * SLAB_S_BYTES);
+  k_out[ec * CT + tl] = live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(rows.k) + at) : zero;
+  u_out[ec * CT + tl] = live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(rows.v) + at) : zero;
+  if (ec < 2) u_out[(VD / 8 + ec) * CT + tl] = make_uint4(ec == 0 && live ? 0x00003F80u : 0u, 0u, 0u, 0u);
+}
+
+// ---------------------------------------------------------------------------
 // state_update: dS[u,c][slab rows] = phi_k^T U
-//   one block per (slab group of 4, chunk, unit); 256 threads, thread = (token, half of the slab's chunks).
-//   The first `n_prologue` blocks compute the per-head prologue instead (oal_prologue.cuh): it has no input in
-//   common with this kernel, both are needed next, and one launch costs less than two and a fork.
+//   one block per (slab group of 4, chunk, unit); 256 threads, thread = (token, half of the slab)
 // ---------------------------------------------------------------------------
 struct StateUpdateArgs {
   const __nv_bfloat16 *k, *v;   // [units, N, 64]
   float* ds;                    // [units, NB] chunks of F_ROWS x EP floats in state_inc_offset order
   int N, NB, NC;                // chunks of the sequence; chunks whose increment is computed (the first NC)
   int32_t* status;
-  int32_t* block_status;        // with a prologue that clears `status` in this launch: a word per block instead, see state_scan
 };
 
 constexpr int GEN_THREADS = 256;      // (token, half of a slab)
 
-__global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const StateUpdateArgs a, const PrologueArgs pro,
-                                                                      int n_prologue) {
+__global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const StateUpdateArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  if ((int)blockIdx.x < n_prologue) {
-    head_prologue(pro, blockIdx.x, *reinterpret_cast<PrologueSmem*>(smem), threadIdx.x, GEN_THREADS);
-    return;
-  }
   unsigned char* Abuf = smem;                          // 2 x SLAB_A_BYTES
   unsigned char* Uimg = smem + 2 * SLAB_A_BYTES;       // [10][128 tokens][8 e]
   unsigned char* Ximg = Uimg + SLAB_S_BYTES;           // rows of k
@@ -85,7 +104,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
-  const int item = (int)blockIdx.x - n_prologue;
+  const int item = blockIdx.x;
   const int grp = item % SU_GROUPS, c = (item / SU_GROUPS) % a.NC, u = item / SU_GROUPS / a.NC;
   const int token = tid & 127, half = tid >> 7;
   if (warp == 0) tmem_alloc(&tmem_base, 256);
@@ -154,11 +173,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   epilogue(ns - 1);
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, 256);
-  if (tid == 0) {
-    const int32_t bits = dead ? w.status_bits() : 0;
-    if (a.block_status) a.block_status[item] = bits;
-    else if (bits) atomicOr(a.status, bits);
-  }
+  if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
 
 // ---------------------------------------------------------------------------
@@ -170,23 +185,18 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
 //   nothing reads its image, and the increment of the last one visited reaches no image: neither is touched.
 // image_lo (optional): a second image of the rounding remainders, bf16(state - bf16(state)); the
 // coefficient-gradient dot products of the backward read state = image + image_lo.
-// block_status (optional): words left by the blocks of a state update whose launch also cleared `status`; nothing orders
-// that store against an atomic of the same launch, so they are merged into it here.
 // ---------------------------------------------------------------------------
 constexpr int SCAN_AHEAD = 4;
 
 __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_bfloat16* image,
                                                          __nv_bfloat16* image_lo, const float* state_in,
-                                                         float* state_total, int NB, int reverse, int trim,
-                                                         const int32_t* block_status, int n_status, int32_t* status) {
+                                                         float* state_total, int NB, int reverse, int trim) {
   constexpr size_t CHUNK = (size_t)F_ROWS * EP;
   const int slab = blockIdx.x / (EU / 8), e8 = blockIdx.x % (EU / 8), within = threadIdx.x * 4;
   const size_t x = (size_t)(slab * (EP / 8) + e8) * 1024 + within;    // element inside a chunk, image order
   const size_t u = blockIdx.y;
   // row-major position of the same element in state_in / state_total
   const size_t rm = (size_t)(slab * 128 + (within >> 3)) * EP + e8 * 8 + (within & 7);
-  for (size_t b = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x; b < (size_t)n_status; b += (size_t)gridDim.y * gridDim.x * 256)
-    if (block_status[b]) atomicOr(status, block_status[b]);
   float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
   if (state_in) run = *reinterpret_cast<const float4*>(state_in + u * CHUNK + rm);
   const float* src = ds + u * NB * CHUNK + x;
@@ -219,6 +229,161 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_b
     *reinterpret_cast<float4*>(state_total + u * CHUNK + rm) = run;
     if (e8 == EU / 8 - 1) *reinterpret_cast<float4*>(state_total + u * CHUNK + rm + 8) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
+}
+
+// ---------------------------------------------------------------------------
+// state_walk: the carry images of every chunk, one block per (unit, slab), which walks the chunks with its 128 x 72 state in
+// registers.
+//   warps 0-3   thread = token: features of chunk c into A[c % 2], the pieces of k two chunks ahead in registers; warp 0 issues
+//               the MMA  Z[c % 2] = A^T [v | 1]
+//   warps 4-15  thread = (feature row, 24 columns): image c written while the MMA runs, then the increment of chunk c added;
+//               warp 4 has the image of [v | 1] two chunks on copied in
+// What bounds it: the stores of a block's SM, 37 KB per chunk at 16 bytes per clock (2350 clocks per chunk, whatever the
+// generators do: eight warps, or all in one set of warps, are no faster).  In two kernels the increments, twice the images'
+// bytes, go to memory and back: 135 -> 77 us at B = 4, N = 4096, 2 KV heads (152 blocks: two on four SMs); with 2 units the walk
+// takes 51 us against 42, so state_walk_pays() asks for three, or a short sequence.
+// ---------------------------------------------------------------------------
+struct StateWalkArgs {
+  const unsigned char *k_image, *u_image;
+  unsigned char *image, *image_lo; // [units, NB, 19, 10, 128, 8]: state, and bf16(state - bf16(state))
+  const float* state_in;           // [units, F_ROWS, EP] row-major, or null
+  int N, NB;
+  int first_image;                 // 1: nothing reads the image of the first chunk (a zero state)
+  int32_t* status;
+};
+constexpr int SW_GEN_WARPS = 4, SW_DRAIN_WARPS = 12, SW_THREADS = (SW_GEN_WARPS + SW_DRAIN_WARPS) * 32;
+constexpr int SW_BLOCKS = EU / 8 / (SW_DRAIN_WARPS / 4);      // blocks of 8 columns per drain warp
+static_assert(SW_BLOCKS * (SW_DRAIN_WARPS / 4) * 8 == EU, "the drain warps share the used columns evenly");
+// shared memory: two feature slabs, two images of [v | 1] (the MMA reads 8 columns past the used ones: in bounds, into columns
+// of Z that no one reads)
+constexpr int SW_U = 2 * SLAB_A_BYTES, SW_SMEM = SW_U + SLAB_U_BYTES + SLAB_S_BYTES;
+
+__global__ void __launch_bounds__(SW_THREADS, 2) state_walk_kernel(const StateWalkArgs a) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint64_t z_full[2], z_free[2], u_full[2];
+  __shared__ uint32_t tmem_base;
+  __shared__ int dead;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
+  const int slab = blockIdx.x % F_SLABS, u = blockIdx.x / F_SLABS;
+  const int n = a.NB - 1;                              // the increment of the last chunk reaches no image
+  if (warp == 0) tmem_alloc(&tmem_base, 256);
+  const auto fetch_u = [&](int c) {                    // one thread
+    mbar_arrive_expect_tx(&u_full[c & 1], SLAB_U_BYTES);
+    bulk_g2s(smem + SW_U + (c & 1) * SLAB_U_BYTES, a.u_image + ((size_t)u * a.NB + c) * SLAB_S_BYTES, SLAB_U_BYTES, &u_full[c & 1]);
+  };
+  if (tid == 0) {
+    for (int x = 0; x < 2; ++x) {
+      mbar_init(&z_full[x], 1);
+      mbar_init(&z_free[x], SW_DRAIN_WARPS);
+      mbar_init(&u_full[x], 1);
+    }
+    mbar_fence_init();
+    dead = 0;
+    for (int c = 0; c < 2 && c < n; ++c) fetch_u(c);
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  Waiter w{&dead};
+  const uint32_t tmem = uniform(tmem_base);
+
+  if (warp < SW_GEN_WARPS) {
+    // ---------------- generators ----------------
+    const HalfBlock blk[2] = {half_block(min(2 * slab, F_PAIR_BLOCKS - 1)), half_block(min(2 * slab + 1, F_PAIR_BLOCKS - 1))};
+    const unsigned char* base = a.k_image + (size_t)u * a.NB * ROW_IMAGE_BYTES + tid * 16;
+    uint4 r4[2][2], c4[2][2];                          // [chunk parity][half of the slab]
+    const auto fetch_k = [&](int c, int x) {
+      const unsigned char* at = base + (size_t)min(c, a.NB - 1) * ROW_IMAGE_BYTES;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        r4[x][h] = load_ahead(at + blk[h].rb * ROW_PLANE);
+        c4[x][h] = load_ahead(at + blk[h].cb * ROW_PLANE);
+      }
+    };
+    fetch_k(0, 0);
+    fetch_k(1, 1);
+    const uint32_t idesc = instr_desc_bf16(128, EP, 1, 1);
+    for (int c0 = 0; c0 < n; c0 += 2) {
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {                    // parity: a register set and a buffer each
+        const int c = c0 + x;
+        if (c >= n) break;
+        if (c >= 2) w.wait(&z_full[x], ((c >> 1) - 1) & 1, 0x11);      // the MMA that read A[x] has completed
+        __syncwarp();
+        uint4* tile = reinterpret_cast<uint4*>(smem + x * SLAB_A_BYTES) + tid;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          raw_half_slab(2 * slab + h, r4[x][h], c4[x][h],
+                        [&](int j) { return __ldg(reinterpret_cast<const uint4*>(base + (size_t)c * ROW_IMAGE_BYTES + j * ROW_PLANE)); },
+                        [&](int j, uint4 f) { tile[(8 * h + j) * CT] = f; });
+        fetch_k(c + 2, x);
+        fence_async_smem();
+        asm volatile("bar.sync 1, %0;" ::"n"(SW_GEN_WARPS * 32) : "memory");
+        if (warp == 0 && elect_one()) {
+          w.wait(&u_full[x], (c >> 1) & 1, 0x12);
+          if (c >= 2) w.wait(&z_free[x], ((c >> 1) - 1) & 1, 0x13);
+          fence_after_sync();
+          const uint64_t da = smem_desc(smem_u32(smem + x * SLAB_A_BYTES), 128, CT * 16);
+          const uint64_t du = smem_desc(smem_u32(smem + SW_U + x * SLAB_U_BYTES), 128, ROW_PLANE);
+#pragma unroll
+          for (int ks = 0; ks < CT / 16; ++ks)
+            mma_bf16_ss(tmem + x * EP, desc_advance(da, ks * 256), desc_advance(du, ks * 256), idesc, ks > 0);
+          mma_commit(&z_full[x]);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // ---------------- state ----------------
+    const int fr = 32 * (warp & 3) + lane, e0 = SW_BLOCKS * ((warp - SW_GEN_WARPS) >> 2);       // feature row, first block of 8 columns
+    float run[8 * SW_BLOCKS];
+#pragma unroll
+    for (int e = 0; e < 8 * SW_BLOCKS; ++e) run[e] = 0.f;
+    if (a.state_in) {
+      const float* src = a.state_in + ((size_t)u * F_ROWS + slab * 128 + fr) * EP + 8 * e0;
+#pragma unroll
+      for (int e = 0; e < 8 * SW_BLOCKS; e += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(src + e);
+        run[e] = t.x; run[e + 1] = t.y; run[e + 2] = t.z; run[e + 3] = t.w;
+      }
+    }
+    const size_t at0 = ((size_t)u * a.NB * F_SLABS + slab) * SLAB_S_BYTES + e0 * ROW_PLANE + fr * 16;
+    for (int c = 0; c < a.NB; ++c) {
+      if (c >= a.first_image) {
+        const size_t at = at0 + (size_t)c * F_SLABS * SLAB_S_BYTES;
+#pragma unroll
+        for (int e8 = 0; e8 < SW_BLOCKS; ++e8) {
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float x = run[8 * e8 + 2 * j], y = run[8 * e8 + 2 * j + 1];
+            hi[j] = pack_bf16(x, y);
+            lo[j] = pack_bf16(x - bf16_lo(hi[j]), y - bf16_hi(hi[j]));
+          }
+          *reinterpret_cast<uint4*>(a.image + at + e8 * ROW_PLANE) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<uint4*>(a.image_lo + at + e8 * ROW_PLANE) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+      }
+      if (c >= n) break;
+      w.wait(&z_full[c & 1], (c >> 1) & 1, 0x14);
+      if (warp == SW_GEN_WARPS && lane == 0 && c + 2 < n) fetch_u(c + 2);
+      __syncwarp();
+      fence_after_sync();
+      const uint32_t t = tmem + (c & 1) * EP + ((uint32_t)(32 * (warp & 3)) << 16) + 8 * e0;
+      float z[SW_BLOCKS][8];
+#pragma unroll
+      for (int e8 = 0; e8 < SW_BLOCKS; ++e8) tmem_ld8(t + 8 * e8, z[e8]);
+      tmem_ld_wait();
+      fence_before_sync();
+      warp_arrive(&z_free[c & 1], lane);
+#pragma unroll
+      for (int e = 0; e < 8 * SW_BLOCKS; ++e) run[e] += z[e >> 3][e & 7];
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem_base, 256);
+  if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
 
 // ---------------------------------------------------------------------------
@@ -458,25 +623,43 @@ cudaError_t build_coef_table(const int32_t* dim_perm, const int32_t* group_start
   return cudaGetLastError();
 }
 
-int state_update_blocks(int units, int NC) { return SU_GROUPS * NC * units; }
-
-cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, const PrologueArgs* prologue,
-                         int q_heads, int32_t* status, int32_t* block_status, cudaStream_t st) {
+cudaError_t state_update(const void* k, const void* v, float* ds, int units, int N, int NB, int NC, int32_t* status, cudaStream_t st) {
   const int smem = 2 * SLAB_A_BYTES + SLAB_S_BYTES + X_BYTES;
   cudaError_t e = allow_smem<state_update_kernel>(smem);
   if (e != cudaSuccess) return e;
-  StateUpdateArgs a{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ds, N, NB, NC, status, block_status};
+  StateUpdateArgs a{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ds, N, NB, NC, status};
+  state_update_kernel<<<SU_GROUPS * NC * units, GEN_THREADS, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+// The walk's time by chunks, against what the two kernels need for increments to memory and back: 1.25 us per chunk and
+// block of an SM, 0.53 us per chunk and unit and 6 us for the second launch and its first loads.
+bool state_walk_pays(int units, int NB) {
+  const int sms = sm_count(), per_sm = (F_SLABS * units + sms - 1) / sms;
+  return 1.25 * per_sm * NB < 0.53 * units * NB + 6.;
+}
+
+cudaError_t rows_prologue(const RowImages& rows, int units, int N, int NB, const PrologueArgs* prologue, int q_heads, cudaStream_t st) {
   const int n_pro = prologue ? q_heads : 0;
-  state_update_kernel<<<n_pro + state_update_blocks(units, NC), GEN_THREADS, smem, st>>>(a, prologue ? *prologue : PrologueArgs{}, n_pro);
+  rows_prologue_kernel<<<n_pro + units * NB * (CT / 32), 256, 0, st>>>(prologue ? *prologue : PrologueArgs{}, n_pro, rows, N, NB);
+  return cudaGetLastError();
+}
+
+cudaError_t state_walk(const RowImages& rows, void* image, void* image_lo, const float* state_in, int units, int N, int NB, bool trim,
+                       int32_t* status, cudaStream_t st) {
+  cudaError_t e = allow_smem<state_walk_kernel>(SW_SMEM);
+  if (e != cudaSuccess) return e;
+  StateWalkArgs a{static_cast<const unsigned char*>(rows.k_image), static_cast<const unsigned char*>(rows.u_image),
+                  static_cast<unsigned char*>(image), static_cast<unsigned char*>(image_lo), state_in, N, NB, trim ? 1 : 0, status};
+  state_walk_kernel<<<F_SLABS * units, SW_THREADS, SW_SMEM, st>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float* state_in, float* state_total,
-                       int units, int NB, int reverse, bool trim, const int32_t* block_status, int n_status, int32_t* status,
-                       cudaStream_t st) {
+                       int units, int NB, int reverse, bool trim, cudaStream_t st) {
   state_scan_kernel<<<dim3(F_SLABS * (EU / 8), units), 256, 0, st>>>(
       ds, static_cast<__nv_bfloat16*>(image), static_cast<__nv_bfloat16*>(image_lo), state_in, state_total, NB, reverse,
-      trim ? 1 : 0, block_status, block_status ? n_status : 0, status);
+      trim ? 1 : 0);
   return cudaGetLastError();
 }
 

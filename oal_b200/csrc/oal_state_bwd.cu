@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
     const auto fetch = [&]() {
       const HalfBlock blk = half_block(min(2 * cur.slab + half, F_PAIR_BLOCKS - 1));
       row = reinterpret_cast<const uint4*>(a.q_image + ((size_t)(cur.b * a.Hq + cur.h0 + cur.hh) * a.NB + cur.c) * ROW_IMAGE_BYTES) + token;
-      r4 = __ldg(row + blk.rb * CT);
-      c4 = __ldg(row + blk.cb * CT);
+      r4 = load_ahead(row + blk.rb * CT);
+      c4 = load_ahead(row + blk.cb * CT);
     };
     if (T > 0) fetch();
     int s = 0, use = 0;                       // ring slot of `it` and how often it has been used before
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
       const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
       const uint4* src = reinterpret_cast<const uint4*>(a.x_image + ((size_t)(it.b * a.H + it.h) * a.NB + it.c) * ROW_IMAGE_BYTES);
 #pragma unroll
-      for (int j = 0; j < PIECES; ++j) next[j] = __ldg(src + tid + j * T);
+      for (int j = 0; j < PIECES; ++j) next[j] = load_ahead(src + tid + j * T);
     };
     const auto store_rows = [&]() {
 #pragma unroll
@@ -704,33 +704,20 @@ __global__ void __launch_bounds__(32 * SLOT_WARPS) dcoef_slots_kernel(const floa
   }
 }
 
-// normalisation VJP writing the bf16 operand images of G (hi, lo), and the images of the rows that the backward kernels
-// fetch with bulk copies (RowImages; copied by threads, 16 bytes each with cp.async, a tile's rows took 5000 clocks)
+// normalisation VJP writing the bf16 operand images of G (hi, lo), and the image of the rows of q that the backward
+// kernels fetch with bulk copies (copied by threads, 16 bytes each with cp.async, a tile's rows took 5000 clocks)
 //   CTA = 32 consecutive tokens of one (head, chunk); warp = 8 consecutive columns, lane = token, so a
 //   warp stores 512 contiguous bytes of an image chunk.  Rows are enumerated over padded chunks so
 //   that tail tokens of the last chunk are zeroed.
 __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_out, int out_dt, const float* grad_num,
                                                              const float* grad_den, const float* num,
                                                              const float* den, float floor_v, __nv_bfloat16* gimg, int N, int NB, int heads,
-                                                             int tm_heads, const RowImages img_rows, int q_blocks, int32_t* status) {
+                                                             int tm_heads, const RowImages img_rows, int32_t* status) {
   __shared__ float part[8][32];
   if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;     // first kernel of the backward
   const int ec = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t per_head = (size_t)NB * CT;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  if ((int)blockIdx.x >= q_blocks) {                        // rows of k and of [v | 1 | 0]
-    const size_t r = (size_t)(blockIdx.x - q_blocks) * 32 + lane, bh = r / per_head;
-    const int t = (int)(r % per_head), tl = t % CT;
-    const bool live = t < N;
-    const size_t at = (bh * N + t) * HD + 8 * ec, chunk = bh * NB + t / CT;
-    uint4* k_out = reinterpret_cast<uint4*>(static_cast<unsigned char*>(img_rows.k_image) + chunk * ROW_IMAGE_BYTES);
-    uint4* u_out = reinterpret_cast<uint4*>(static_cast<unsigned char*>(img_rows.u_image) + chunk * SLAB_S_BYTES);
-    k_out[ec * CT + tl] = live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(img_rows.k) + at) : zero;
-    u_out[ec * CT + tl] = live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(img_rows.v) + at) : zero;
-    if (ec < 2) u_out[(VD / 8 + ec) * CT + tl] = make_uint4(ec == 0 && live ? 0x00003F80u : 0u, 0u, 0u, 0u);
-    return;
-  }
-  const size_t r = (size_t)blockIdx.x * 32 + lane;          // q_blocks cover heads * per_head rows exactly
+  const size_t r = (size_t)blockIdx.x * 32 + lane;          // grid covers heads * per_head rows exactly
   const size_t bh = r / per_head;
   const int t = (int)(r % per_head);
   const int cidx = t / CT, tl = t % CT;
@@ -771,7 +758,7 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
   }
   part[ec][lane] = dot;
   reinterpret_cast<uint4*>(static_cast<unsigned char*>(img_rows.q_image) + (bh * NB + cidx) * ROW_IMAGE_BYTES)[ec * CT + tl] =
-      live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(img_rows.q) + row * HD + 8 * ec) : zero;
+      live ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(img_rows.q) + row * HD + 8 * ec) : make_uint4(0u, 0u, 0u, 0u);
   // hi image = bf16(g); lo image = bf16(g - hi): dW = g . [v|1] is formed from both, because its two
   // large terms (dout.v / den and dout.num / den^2) nearly cancel
   uint4* img = reinterpret_cast<uint4*>(gimg + (bh * NB + cidx) * (size_t)(SLAB_S_BYTES / 2));
@@ -847,12 +834,11 @@ cudaError_t dcoef_reduce(const float* partial, int outer, int Hq, int G, const i
 
 cudaError_t norm_vjp_image(const void* grad_out, int out_dt, const float* grad_num, const float* grad_den,
                            const float* num, const float* den, float floor_v, void* gimg, int heads,
-                           int N, int NB, int token_major_heads, const RowImages& rows, int kv_heads, int32_t* clear_status,
+                           int N, int NB, int token_major_heads, const RowImages& rows, int32_t* clear_status,
                            cudaStream_t st) {
-  const int q_blocks = (int)((size_t)heads * NB * CT / 32), kv_blocks = rows.k ? (int)((size_t)kv_heads * NB * CT / 32) : 0;
-  norm_vjp_image_kernel<<<q_blocks + kv_blocks, 256, 0, st>>>(grad_out, out_dt, grad_num, grad_den, num, den, floor_v,
-                                                              static_cast<__nv_bfloat16*>(gimg), N, NB, heads, token_major_heads, rows,
-                                                              q_blocks, clear_status);
+  norm_vjp_image_kernel<<<(unsigned)((size_t)heads * NB * CT / 32), 256, 0, st>>>(grad_out, out_dt, grad_num, grad_den, num, den, floor_v,
+                                                                                  static_cast<__nv_bfloat16*>(gimg), N, NB, heads,
+                                                                                  token_major_heads, rows, clear_status);
   return cudaGetLastError();
 }
 
