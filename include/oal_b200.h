@@ -84,7 +84,9 @@ enum {
   /* the sequences start here (no state_in, no dstate_in in this call or its counterpart): the forward and the
    * backward of a call, which must both carry the flag or both not, leave out the state work of the chunks that
    * only meet a zero state */
-  OAL_FLAG_ZERO_STATE_IN = 2
+  OAL_FLAG_ZERO_STATE_IN = 2,
+  /* forward entry points only: no oal_backward follows, what only a backward reads is not written to saved_state */
+  OAL_FLAG_NO_BACKWARD = 4
 };
 
 typedef struct OalProblem {

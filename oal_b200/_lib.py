@@ -24,6 +24,7 @@ GRAD_Q, GRAD_K, GRAD_V, GRAD_COEF, GRAD_REUSE_STATE_STAGE = 1, 2, 4, 8, 16
 STATE_ROWS = 2432
 FLAG_OUT_TOKEN_MAJOR = 1
 FLAG_ZERO_STATE_IN = 2
+FLAG_NO_BACKWARD = 4
 STATUS_NONFINITE, STATUS_DENOMINATOR, STATUS_WAIT_TIMEOUT, STATUS_BAD_LAYOUT = 1, 2, 4, 8
 
 # every symbol include/oal_b200.h declares

@@ -321,7 +321,7 @@ int check_problem(const OalProblem* p) {
     if (p->chunk != 128) return fail(OAL_ERR_ARGUMENT, "bf16_tensorcore requires chunk == 128");
   }
   if (!(p->floor > 0.f)) return fail(OAL_ERR_ARGUMENT, "floor must be positive");
-  if (p->flags & ~(OAL_FLAG_OUT_TOKEN_MAJOR | OAL_FLAG_ZERO_STATE_IN)) return fail(OAL_ERR_ARGUMENT, "unknown bits in flags");
+  if (p->flags & ~(OAL_FLAG_OUT_TOKEN_MAJOR | OAL_FLAG_ZERO_STATE_IN | OAL_FLAG_NO_BACKWARD)) return fail(OAL_ERR_ARGUMENT, "unknown bits in flags");
   if ((p->flags & OAL_FLAG_OUT_TOKEN_MAJOR) && (p->precision != OAL_PRECISION_BF16_TENSORCORE || p->groups > 8))
     // (the limit of 8 groups is the flag's contract; the kernels have none)
     return fail(OAL_ERR_ARGUMENT, "token-major out needs bf16_tensorcore and at most 8 groups per head");
@@ -586,15 +586,17 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
     e = oal::build_coef_table(dim_perm, group_start, src.A, src.B, src.C, p->q_heads, p->groups, p->scale, coef_table, st);
     if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
   }
-  if (tc) {
+  const bool walk = update && timing && oal::state_walk_pays(units, nb);
+  const bool backward = !(p->flags & OAL_FLAG_NO_BACKWARD);
+  if (tc && (src.factor || walk || backward)) {
     LaunchScope scope("rows_prologue", st, 1, timing);
-    e = oal::rows_prologue(rows, units, p->seq_len, nb, src.factor ? &pro : nullptr, p->q_heads, st);
+    e = oal::rows_prologue(rows, walk || backward ? units : 0, p->seq_len, nb, src.factor ? &pro : nullptr, p->q_heads, st);
     if (e != cudaSuccess) return fail_cuda(e, "row image kernel");
   }
-  const bool walk = update && timing && oal::state_walk_pays(units, nb);
+  void* remainders = tc && backward ? saved_remainders(p, saved_state) : nullptr;
   if (walk) {
     LaunchScope scope("state_walk", st, 1, timing);
-    e = oal::state_walk(rows, saved_state, saved_remainders(p, saved_state), state_in, units, p->seq_len, nb, cr.trim, status, st);
+    e = oal::state_walk(rows, saved_state, remainders, state_in, units, p->seq_len, nb, cr.trim, status, st);
     if (e != cudaSuccess) return fail_cuda(e, "state walk kernel");
   } else if (update) {
     LaunchScope scope("state_update", st, 1, timing);
@@ -604,7 +606,7 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
   if (tc && cr.n > 0) {
     if (!walk) {
       LaunchScope scope("state_scan", st, 1, timing);
-      e = oal::state_scan(ds, saved_state, saved_remainders(p, saved_state), state_in, nullptr, units, nb, 0, cr.trim, st);
+      e = oal::state_scan(ds, saved_state, remainders, state_in, nullptr, units, nb, 0, cr.trim, st);
       if (e != cudaSuccess) return fail_cuda(e, "state scan kernel");
     }
     { LaunchScope scope("cross_read_q", st, 1, timing);
@@ -707,6 +709,7 @@ int backward_core_fp32(const OalProblem* p, const BackwardArgs& x, const CoefSou
 }
 
 int backward_core(const OalProblem* p, const BackwardArgs& x, const CoefSource& src, CoefSink sink, cudaStream_t st) {
+  if (p->flags & OAL_FLAG_NO_BACKWARD) return fail(OAL_ERR_ARGUMENT, "oal_backward: the problem says that no backward follows");
   if (p->precision == OAL_PRECISION_FP32_IEEE) return backward_core_fp32(p, x, src, sink, st);
   if (!x.saved_state) return fail(OAL_ERR_ARGUMENT, "oal_backward: saved_state is NULL");
   if (misaligned({x.q, x.k, x.v, x.num, x.saved_state, x.grad_out, x.grad_num, x.dq, x.dk, x.dv, x.dstate_in, x.workspace}))

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_b
 // ---------------------------------------------------------------------------
 struct StateWalkArgs {
   const unsigned char *k_image, *u_image;
-  unsigned char *image, *image_lo; // [units, NB, 19, 10, 128, 8]: state, and bf16(state - bf16(state))
+  unsigned char *image, *image_lo; // [units, NB, 19, 10, 128, 8]: state, and bf16(state - bf16(state)) or null
   const float* state_in;           // [units, F_ROWS, EP] row-major, or null
   int N, NB;
   int first_image;                 // 1: nothing reads the image of the first chunk (a zero state)
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(SW_THREADS, 2) state_walk_kernel(const StateWa
             lo[j] = pack_bf16(x - bf16_lo(hi[j]), y - bf16_hi(hi[j]));
           }
           *reinterpret_cast<uint4*>(a.image + at + e8 * ROW_PLANE) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(a.image_lo + at + e8 * ROW_PLANE) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          if (a.image_lo) *reinterpret_cast<uint4*>(a.image_lo + at + e8 * ROW_PLANE) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         }
       }
       if (c >= n) break;

@@ -171,7 +171,8 @@ def _native_call(prepared):
                            out_dtype=out_dtype if out_dtype != torch.float64 else torch.float32, precision=plan.precision,
                            chunk=plan.chunk_tokens, scale=prepared.scale, floor=prepared.normalization_floor,
                            grad_mask=_grad_bits(mask),
-                           flags=_lib.FLAG_ZERO_STATE_IN | (_lib.FLAG_OUT_TOKEN_MAJOR if token_major else 0))
+                           flags=_lib.FLAG_ZERO_STATE_IN | (_lib.FLAG_OUT_TOKEN_MAJOR if token_major else 0)
+                           | (0 if any(mask) else _lib.FLAG_NO_BACKWARD))
     if token_major and plan.geometry[5] != _lib.HEAD_DIM:
         return None                     # refused where the call runs
     return _lib.host().prepare(bytes(problem), list(plan.geometry), tables.group_count, io_dtype, out_dtype, device.index,
