@@ -332,6 +332,9 @@ std::shared_ptr<Prepared> prepare(py::bytes problem, std::vector<int64_t> geomet
   p->dim_perm = dim_perm;
   p->group_start = group_start;
   p->eps = (float)eps;
+  // at least what this library needs, whatever a preparation that was stored by another build says: a forward call has no
+  // length of the saved state to check
+  for (int phase = 0; phase < 3; ++phase) bytes[phase] = std::max(bytes[phase], (int64_t)oal_workspace_bytes(&p->problem, phase));
   p->forward_bytes = bytes[0]; p->backward_bytes = bytes[1]; p->saved_bytes = bytes[2];
   p->coef_floats = p->Hq * (1 + groups + groups * groups);
   for (int i = 0; i < 4; ++i) p->grad[i] = grad[i];

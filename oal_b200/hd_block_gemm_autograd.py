@@ -270,10 +270,12 @@ def forward_impl(q, k, v, a, b, c, tables: GroupTables, scale: float, floor: flo
     num = torch.empty(B, Hq, N, _lib.HEAD_DIM, dtype=torch.float32, device=dev)
     den = torch.empty(B, Hq, N, dtype=torch.float32, device=dev)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
-    ws = workspace if workspace is not None else torch.empty(max(plan.forward_workspace_bytes, 16),
+    ws = workspace if workspace is not None else torch.empty(max(plan.forward_workspace_bytes,
+                                                                 _lib.workspace_bytes(problem, 0), 16),
                                                              dtype=torch.uint8, device=dev)
-    saved = (torch.empty(plan.saved_state_bytes, dtype=torch.uint8, device=dev)
-             if plan.saved_state_bytes else None)
+    # what this library needs, whatever a plan that was stored by another build says: oal_forward has no length to check
+    saved_bytes = max(plan.saved_state_bytes, _lib.workspace_bytes(problem, 2))
+    saved = torch.empty(saved_bytes, dtype=torch.uint8, device=dev) if saved_bytes else None
     a32, b32, c32 = (t.detach().to(torch.float32).contiguous() for t in (a, b, c))
     with _lib.device_guard(qp):
         rc = lib.oal_forward(ctypes.byref(problem), _lib.ptr(qp), _lib.ptr(kp), _lib.ptr(vp),
@@ -346,7 +348,8 @@ def backward_impl(saved_inputs, num, den, saved_state, tables: GroupTables, scal
     dB = torch.empty(Hq, G, dtype=torch.float32, device=dev) if bits & _lib.GRAD_COEF else None
     dC = torch.empty(Hq, G, G, dtype=torch.float32, device=dev) if bits & _lib.GRAD_COEF else None
     status = torch.zeros(1, dtype=torch.int32, device=dev)
-    ws = workspace if workspace is not None else torch.empty(max(plan.backward_workspace_bytes, 16),
+    ws = workspace if workspace is not None else torch.empty(max(plan.backward_workspace_bytes,
+                                                                 _lib.workspace_bytes(problem, 1), 16),
                                                              dtype=torch.uint8, device=dev)
     with _lib.device_guard(qp):
         rc = lib.oal_backward(ctypes.byref(problem), _lib.ptr(qp), _lib.ptr(kp), _lib.ptr(vp),

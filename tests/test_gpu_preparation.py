@@ -31,6 +31,28 @@ def test_copies_and_pickles_run_the_same_call():
             assert torch.equal(got, x)
 
 
+@pytest.mark.parametrize("general", [False, True])
+def test_a_plan_with_the_sizes_of_another_build_gets_room_enough(general):
+    """Stored sizes only ever raise what a call allocates: a forward call cannot check the length of its saved state."""
+    from oal_b200.hd_block_gemm_adapters import run_grouped_coefficients
+
+    make, live = _prepared()
+    q, k, v, factor = (t.clone().requires_grad_(True) for t in live)
+    groups = (torch.arange(64) % 4).to(torch.int32).cuda()
+    prepared = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, factor, precision="bf16_tensorcore")
+    plan = dataclasses.replace(prepared.plan, forward_workspace_bytes=16, backward_workspace_bytes=16, saved_state_bytes=16)
+    coefficients = [torch.rand(shape, device="cuda").requires_grad_(True) for shape in ((4,), (4, 4), (4, 4, 4))]
+    results = []
+    for each in (prepared, dataclasses.replace(prepared, plan=plan)):
+        inputs = (q, k, v, *coefficients) if general else (q, k, v, factor)
+        out = (run_grouped_coefficients(*inputs, tables=each.tables, plan=each.plan, scale=each.scale,
+                                        normalization_floor=each.normalization_floor) if general
+               else oal_b200.run_prepared_grouped_hd_block_gemm(each, *inputs))
+        results.append([*out, *torch.autograd.grad(out[0].float().sum(), inputs)])
+    for got, want in zip(results[1], results[0]):
+        assert torch.equal(got, want)
+
+
 def test_a_changed_copy_runs_its_own_options():
     make, live = _prepared()
     prepared = make()
