@@ -573,6 +573,7 @@ def run_gpu_arm(args) -> None:
         intra = w["hq"] * (D + e) * 65 * tok
         kernel_flops = {
             "state_update": w["hkv"] * 2 * f * e * tok,
+            "state_walk": w["hkv"] * 2 * f * e * tok,
             "cross_read_q": w["hq"] * 2 * f * e * tok,
             "dstate_heads": w["hq"] * 2 * f * e * tok,
             "feature_grad_q": w["hq"] * 2 * f * e * tok,
@@ -582,16 +583,17 @@ def run_gpu_arm(args) -> None:
             "intra_backward_q": intra,         # dW and dq
             "intra_backward_kv": intra,        # dk and dv
         }
-        # MMA FLOPs the intra-chunk kernels really execute per launch, per 128-token chunk: G + 1 terms, each a chain
-        # over K = 64 of value + remainder against the other side's rows.  Query-side tiles hold four 32-row blocks
-        # and see only the keys of the last one; the key/value side walks all 128 queries of a head.  The weights meet
-        # the values (80 columns) and G (64) as value + remainder.
+        # MMA FLOPs the intra-chunk kernels really execute per launch, per 128-token chunk: forward and key/value side G + 1
+        # terms, each a chain over K = 64 of value + remainder against the other side's rows; query side of the backward G
+        # chains over K = 64 (rows of one group's dims) and G + 1 products as value + remainder.  Query-side tiles hold four
+        # 32-row blocks and see only the keys of the last one; the key/value side walks all 128 queries of a head.  The
+        # weights meet the values (80 columns) and G (64) as value + remainder.
         terms, rep, chunks = w["g"] + 1, w["hq"] // w["hkv"], w["batch"] * w["hkv"] * (w["n"] // KERNEL_CHUNK)
         seen = chunks * sum(32 * (4 - 4 * x // rep) for x in range(rep))       # key columns of all query-side tiles
         rows = chunks * rep * 128                                             # query columns of the key/value side
         executed_flops = {
             "intra_forward": seen * 2 * 128 * (terms * 128 + 2 * 80),
-            "intra_backward_q": seen * 2 * 128 * (2 * 80 + terms * (128 + 2 * 64)),
+            "intra_backward_q": seen * 2 * 128 * (2 * 80 + w["g"] * 64 + terms * 2 * 64),
             "intra_backward_kv": rows * 2 * 128 * (2 * 80 + terms * (128 + 64) + 2 * 64),
         }
         kernels = {name: dict(launches=cnt, ms_per_launch=ms / max(cnt, 1), share=None)
