@@ -41,7 +41,7 @@ def test_a_plan_with_the_sizes_of_another_build_gets_room_enough(general):
     groups = (torch.arange(64) % 4).to(torch.int32).cuda()
     prepared = oal_b200.prepare_grouped_hd_block_gemm(q, k, v, groups, factor, precision="bf16_tensorcore")
     plan = dataclasses.replace(prepared.plan, forward_workspace_bytes=16, backward_workspace_bytes=16, saved_state_bytes=16)
-    coefficients = [torch.rand(shape, device="cuda").requires_grad_(True) for shape in ((4,), (4, 4), (4, 4, 4))]
+    coefficients = [t.cuda().requires_grad_(True) for t in (torch.ones(4), torch.full((4, 4), 0.5), torch.eye(4).expand(4, 4, 4).clone())]
     results = []
     for each in (prepared, dataclasses.replace(prepared, plan=plan)):
         inputs = (q, k, v, *coefficients) if general else (q, k, v, factor)
