@@ -4,7 +4,7 @@
 // diagonalised by cyclic Jacobi rotations (fp32; the eigenvalues are re-evaluated as Rayleigh quotients
 // of the untouched matrix), one warp per query head, the rotations of a round (disjoint index pairs of
 // a round-robin tournament) applied together.  The result is stored as the
-// table the intra-chunk kernels read (oal_intra.cuh): c_r, l_r[d] and the count of positive terms.  Replaces nothing in the reference, which evaluates the direct form
+// table the intra-chunk kernels read (oal_intra.cuh): c_r, l_r[d], the back-transform t and the count of positive terms.  Replaces nothing in the reference, which evaluates the direct form
 // (oal_attention/grouped_reference.py:61-99); the values of w are the same.
 //
 // intra_coef_finish_kernel: sums the per-(batch row, row block) partial sums of the query-side backward in
@@ -175,6 +175,7 @@ __global__ void __launch_bounds__(32) head_factor_kernel(const int32_t* dim_perm
     const int col = live ? order[r] : 0;
     out.l[r][lane] = live ? sl * V[1 + gdim[lane]][col] : 0.f;
     out.l[r][lane + 32] = live ? sl * V[1 + gdim[lane + 32]][col] : 0.f;
+    if (lane < RMAX_ALL) out.t[lane][r] = (live && lane < n) ? V[lane][col] / lam[r] : 0.f;
   }
 }
 

@@ -25,6 +25,7 @@
 namespace oal {
 
 constexpr int RMAX_ALL = OAL_MAX_GROUPS + 1;         // 17: extent of the per-head factor table
+constexpr int T_PITCH = 20;
 constexpr int XA_BYTES = 10 * CP;                    // [v | 1 | 0]
 
 // What a kernel keeps of a head's table besides l.
@@ -68,7 +69,9 @@ struct alignas(16) HeadFactor {
   float e[RMAX_ALL][HD];             // of the dimension's group g: e_0 = scale B_g, e_r = scale^2 (C_rg + C_gr)
   uint32_t mask[GMAX][HD / 2];       // the dimensions of a group, as words of two bf16
   HeadOrder order;
+  float t[RMAX_ALL][T_PITCH];        // t[a][r] = V[a][r] / lambda_r  (v = t u)
 };
+static_assert(offsetof(HeadFactor, t) % 16 == 0 && sizeof(HeadFactor::t) % 16 == 0, "copied in 16-byte pieces");
 
 // Chunks 8 and 9 of the image of [v | 1 | 0]: one in the first element of rows below `valid`, zeros elsewhere.
 __device__ __forceinline__ void augment_rows(unsigned char* img, int valid, int tid, int nthreads) {

@@ -9,6 +9,14 @@
 // s_g is one MMA chain over the rows of q with the other groups' dims set to zero, exact in bf16.  dB_g and dC_rg are
 // sums of y_0 and y_r over the dims of g: 64 sums per r instead of G (G + 1) / 2 products per pair.  X_r's remainder
 // keeps these strongly cancelling sums (sum_j dW_ij w_ij = 0 for every row) at 16 bits.
+// A call of one chunk that wants coefficient gradients takes the terms of the factored weight instead (oal_intra.cuh; u_r as
+// the forward formed it, from the scaled rows of q):
+//   X_r = dW u_r,  dq += 2 sgn_r l_r * Z_r,  D[r][r'] = sum dW u_r u_r' from y_r,  dC = t D t^T,  dB = t sum dW u_r
+// The forward's weights carry the rounding of its scaled rows, about 5e-6 of a row's numerator and denominator, and so does
+// dW.  With the same terms sum_j dW_ij w_ij still cancels; with exact scores it does not, and where no bf16 features (2e-3 of
+// dfactor from 129 tokens on) hide it what is left was the largest error.  dfactor against 64 bits, 14 heads, 33 to 128
+// tokens, geometric mean of 40 inputs, terms / scores: 8 groups 1.13 / 1.22e-5, 12 groups 0.92 / 1.08e-5, 16 groups 0.94 /
+// 1.19e-5; from 129 tokens on the same within 0.2 %.  The kernel at N = 128: 8 groups 22 / 17 us, 16 groups 38 / 26 us.
 //
 // Key / value side (rows are keys, columns are the queries of one head): per head and term r of the factored weight
 // (oal_intra.cuh; the scaled rows as bf16 value + remainder: the rounding of the scaled keys alone would act like a
@@ -79,24 +87,28 @@ __device__ __forceinline__ f32x2 f2_shfl_xor(f32x2 v, int o) {
 // Warps 0..15 compute (with eight of twice the keys and dims 201 us), warp 16 issues; 17..19 only help to load and fill the
 // issuer's warpgroup, whose registers the compute warps take: 640 threads x 96 at launch = 512 x 112 + 128 x 32.
 constexpr int BQ_SUBS = 4, BQ_COMPUTE = 4 * BQ_SUBS, BQ_ISSUER = BQ_COMPUTE, BQ_THREADS = (BQ_COMPUTE + 4) * 32;
-// tensor memory: scores (128; first dW) | X hi (64) | X lo (64) | two Z (64) | two slots of masked rows (32)
+// tensor memory: scores (128; first dW) | X hi (64) | X lo (64) | two Z (64) | two slots of masked rows (32) or terms (64)
 constexpr uint32_t BQ_S = 0, BQ_X = 128, BQ_XLO = 192, BQ_Z = 256, BQ_ROWS = 384, BQ_ROW_COLS = 32;
-static_assert(BQ_ROWS + 2 * BQ_ROW_COLS <= 512, "tensor-memory columns of the query-side kernel");
+static_assert(BQ_ROWS + 2 * TERM_COLS <= 512, "tensor-memory columns of the query-side kernel");
 // shared memory: images of q, k, [v | 1] and G (hi, lo), then of each quadrant's head
 constexpr int BQ_K = ROW_IMAGE_BYTES, BQ_U = BQ_K + ROW_IMAGE_BYTES, BQ_G = BQ_U + SLAB_S_BYTES;
 constexpr int BQ_E = BQ_G + 2 * SLAB_S_BYTES;                           // e_r[d], [quadrant][r][64] fp32
 constexpr int BQ_MASK = BQ_E + 4 * RMAX_ALL * HD * 4;                   // dims of a group, [quadrant][group][32] words of two bf16
 constexpr int BQ_ORDER = BQ_MASK + 4 * GMAX * (HD / 2) * 4;
 constexpr int BQ_SMEM = BQ_ORDER + 4 * (int)sizeof(HeadOrder);
-static_assert(4 * RMAX_ALL * HD * 4 <= 2 * SLAB_S_BYTES, "the y sums take the place of the images of G");
+// TERMS: l, t and the scalars in the places of e, the masks and the order
+constexpr int BQ_Y = 4 * RMAX_ALL * HD, BQ_D = RMAX_ALL * RMAX_ALL;       // floats: y sums; D or t D of a quadrant
+static_assert((BQ_Y + 8 * BQ_D) * 4 <= 2 * SLAB_S_BYTES, "the y sums, D and t D take the place of the images of G");
+static_assert(sizeof(HeadFactor::t) <= GMAX * (HD / 2) * 4 && sizeof(HeadScalars) <= sizeof(HeadOrder), "a quadrant's tables of either form");
 
+template <bool TERMS>
 __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraBwdArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* Qimg = smem;
   float* e_s = reinterpret_cast<float*>(smem + BQ_E);
   uint32_t* mask_s = reinterpret_cast<uint32_t*>(smem + BQ_MASK);
   float* ys = reinterpret_cast<float*>(smem + BQ_G);            // [quadrant][r][64], dims sorted by group; G is dead once dW is complete
-  __shared__ float sum_s[BQ_COMPUTE], cls_s[4][RMAX_ALL * GMAX];
+  __shared__ float sum_s[BQ_COMPUTE], cls_s[TERMS ? 1 : 4][RMAX_ALL * GMAX], n_s[TERMS ? BQ_COMPUTE : 1][RMAX_ALL];
   __shared__ uint64_t in_full, dw_full, s_full, x_full, z_full;
   __shared__ uint32_t tmem_base;
   __shared__ int dead;
@@ -115,7 +127,8 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
     mbar_init(&z_full, 1);
     mbar_fence_init();
     mbar_arrive_expect_tx(&in_full, ROW_IMAGE_BYTES + SLAB_S_BYTES +
-                                        4 * ((8 + 2 * (EP / 8)) * 512 + a.rank * HD * 4 + G * (HD / 2) * 4 + (int)sizeof(HeadOrder)));
+                                        4 * ((8 + 2 * (EP / 8)) * 512 + a.rank * HD * 4 +
+                                             (TERMS ? (int)(sizeof(HeadFactor::t) + sizeof(HeadScalars)) : G * (HD / 2) * 4 + (int)sizeof(HeadOrder))));
     dead = 0;
   }
   fence_before_sync();
@@ -135,16 +148,24 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
       const int lo = y - 8 >= EP / 8, e = y - 8 - lo * (EP / 8);
       bulk_g2s(smem + BQ_G + lo * SLAB_S_BYTES + e * ROW_PLANE + dst, a.gimg + lo * a.gimg_lo_offset + head * SLAB_S_BYTES + e * ROW_PLANE + rows,
                512, &in_full);
-    } else if (y == PER - 3) bulk_g2s(e_s + quadrant * RMAX_ALL * HD, &f->e[0][0], a.rank * HD * 4, &in_full);
-    else if (y == PER - 2) bulk_g2s(mask_s + quadrant * GMAX * (HD / 2), &f->mask[0][0], G * (HD / 2) * 4, &in_full);
-    else if (y == PER - 1) bulk_g2s(smem + BQ_ORDER + quadrant * (int)sizeof(HeadOrder), &f->order, (int)sizeof(HeadOrder), &in_full);
+    } else if (y == PER - 3) bulk_g2s(e_s + quadrant * RMAX_ALL * HD, TERMS ? &f->l[0][0] : &f->e[0][0], a.rank * HD * 4, &in_full);
+    else if (y == PER - 2) {
+      if (TERMS) bulk_g2s(mask_s + quadrant * GMAX * (HD / 2), &f->t[0][0], (int)sizeof(f->t), &in_full);
+      else bulk_g2s(mask_s + quadrant * GMAX * (HD / 2), &f->mask[0][0], G * (HD / 2) * 4, &in_full);
+    } else if (y == PER - 1) {
+      unsigned char* dst_head = smem + BQ_ORDER + quadrant * (int)sizeof(HeadOrder);
+      if (TERMS) bulk_g2s(dst_head, &f->s, (int)sizeof(HeadScalars), &in_full);
+      else bulk_g2s(dst_head, &f->order, (int)sizeof(HeadOrder), &in_full);
+    }
     else if (x == 4 * PER) bulk_g2s(smem + BQ_K, a.k_image + unit * ROW_IMAGE_BYTES, ROW_IMAGE_BYTES, &in_full);
     else if (x == 4 * PER + 1) bulk_g2s(smem + BQ_U, a.u_image + unit * SLAB_S_BYTES, SLAB_S_BYTES, &in_full);
   }
   Waiter w{&dead};
   const uint32_t tmem = uniform(tmem_base);
   const uint32_t lane_off = (uint32_t)(32 * qd) << 16;
-  const bool want_coef = a.coef_partial != nullptr;
+  const bool want_coef = TERMS || a.coef_partial != nullptr;
+  constexpr int FIRST = TERMS ? 0 : 1;                // first r whose X is a product with scores
+  constexpr uint32_t SLOT_COLS = TERMS ? TERM_COLS : BQ_ROW_COLS;
   w.wait(&in_full, 0, 0x20);
   __syncwarp();
 
@@ -157,16 +178,21 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
       issue_dw(tmem + BQ_S, smem_desc(g_addr, ROW_PLANE, 128), smem_desc(g_addr + SLAB_S_BYTES, ROW_PLANE, 128), 2 * ROW_PLANE, du, du,
                2 * ROW_PLANE, cols);
       mma_commit(&dw_full);
-      for (int r = 0; r <= G; ++r) {
-        w.wait(&x_full, r & 1, 0x21);
+      for (int r = FIRST - 1, phase = 0; r <= G; ++r) {
+        w.wait(&x_full, phase++ & 1, 0x21);
         fence_after_sync();
         if (r < G) {
-          const uint32_t slot = tmem + BQ_ROWS + ((r + 1) & 1) * BQ_ROW_COLS;
+          const uint32_t slot = tmem + BQ_ROWS + ((r + 1) & 1) * SLOT_COLS;
+          if (TERMS) {
+            issue_term<ROW_PLANE>(tmem + BQ_S, slot, k_addr, cols);
+          } else {
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks)
-            mma_bf16_ts(tmem + BQ_S, slot + 8 * ks, desc_advance(dk_rows, ks * 2 * ROW_PLANE), idesc_s, ks > 0);
+            for (int ks = 0; ks < HD / 16; ++ks)
+              mma_bf16_ts(tmem + BQ_S, slot + 8 * ks, desc_advance(dk_rows, ks * 2 * ROW_PLANE), idesc_s, ks > 0);
+          }
           mma_commit(&s_full);
         }
+        if (r < 0) continue;
         const uint32_t z = tmem + BQ_Z + (r & 1) * HD;
         for (int ks = 0; ks < cols / 16; ++ks) {
           mma_bf16_ts(z, tmem + BQ_X + 8 * ks, desc_advance(dk_dims, ks * 256), idesc_z, ks > 0);
@@ -186,8 +212,17 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
     const auto key_of = [&](int x) { return 32 * block_of(x) + 16 * (sub & 1); };
     const auto exists = [&](int x) { return 32 * block_of(x) < cols; };
     const auto on = [&](int x) { return exists(x) && block_of(x) <= my_rb; };
-    // rows of q with only the dims of group r - 1, as the A operand
+    // TERMS: c_r, signs, l and t of the quadrant's head
+    const HeadScalars& hs = *reinterpret_cast<const HeadScalars*>(smem + BQ_ORDER + qd * (int)sizeof(HeadOrder));
+    const float* l = e_s + qd * RMAX_ALL * HD;
+    const int rpos = TERMS ? uniform(hs.rpos) : 0;
+    // rows of q with only the dims of group r - 1, or scaled by l_r, as the A operand
     const auto build = [&](int r) {
+      if constexpr (TERMS) {
+        static_assert(DIMS == 16, "a piece of a term");
+        build_term16<ROW_PLANE>(tmem + BQ_ROWS + (r & 1) * SLOT_COLS + lane_off, Qimg + row * 16, l + r * HD, d0);
+        return;
+      }
       const uint32_t* mask = mask_s + (qd * GMAX + r - 1) * (HD / 2) + d0 / 2;
       const uint32_t slot = tmem + BQ_ROWS + (r & 1) * BQ_ROW_COLS + lane_off + d0 / 2;
 #pragma unroll
@@ -225,8 +260,9 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
         qp[t][i] = *reinterpret_cast<const uint32_t*>(Qimg + (d0 / 8 + i) * ROW_PLANE + (32 * qd + (lane >> 2) + 8 * t) * 16 + 4 * m);
     // the dimension whose sum this lane ends up with, in group order
     const HeadOrder& order = *reinterpret_cast<const HeadOrder*>(smem + BQ_ORDER + qd * (int)sizeof(HeadOrder));
-    float* y_out = ys + qd * RMAX_ALL * HD + order.pos[d0 + 8 * (lane >> 4) + 2 * m + ((lane >> 3) & 1)];
-    build(1);
+    const int my_dim = d0 + 8 * (lane >> 4) + 2 * m + ((lane >> 3) & 1);
+    float* y_out = ys + qd * RMAX_ALL * HD + (TERMS ? my_dim : order.pos[my_dim]);
+    build(FIRST);
     {
       const uint32_t zero[8] = {};
 #pragma unroll
@@ -250,6 +286,7 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
           dw[x][j] = f2_pack(kj <= my_key ? d[2 * j] : 0.f, kj + 1 <= my_key ? d[2 * j + 1] : 0.f);
           sum2 = f2_add(sum2, dw[x][j]);
         }
+        if constexpr (TERMS) continue;
         uint32_t hi[8], lo[8];
         split(dw[x], hi, lo);
         store_x(x, hi, lo);
@@ -271,7 +308,10 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
       const float* e = e_s + (qd * RMAX_ALL + r) * HD + d0 + 2 * m;
       f32x2 ev[PIECES], y[PIECES];
 #pragma unroll
-      for (int i = 0; i < PIECES; ++i) ev[i] = *reinterpret_cast<const f32x2*>(e + 8 * i);
+      for (int i = 0; i < PIECES; ++i) {
+        ev[i] = *reinterpret_cast<const f32x2*>(e + 8 * i);
+        if (TERMS) ev[i] = f2_mul(ev[i], f2_bcast(r < rpos ? 2.f : -2.f));
+      }
       tmem_ld_wait();
 #pragma unroll
       for (int i = 0; i < PIECES; ++i)
@@ -292,10 +332,12 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
       v += __shfl_xor_sync(0xffffffffu, v, 4);
       if ((lane & 4) == 0) y_out[r * HD] = v;
     };
-    for (int r = 1; r <= G; ++r) {
+    for (int r = FIRST; r <= G; ++r) {
       // the next rows' slot was last read for the scores of r - 1, which have arrived
       if (r < G) build(r + 1);
-      w.wait(&s_full, (r - 1) & 1, 0x23);
+      const f32x2 c2 = f2_bcast(TERMS ? hs.c[r] : 0.f);
+      f32x2 n2 = 0ull;
+      w.wait(&s_full, (r - FIRST) & 1, 0x23);
       __syncwarp();
       fence_after_sync();
       uint32_t hi[BLOCKS / 2][8], lo[BLOCKS / 2][8];
@@ -305,13 +347,17 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
         tmem_ld_wait();
         f32x2 t[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t[j] = f2_mul(dw[x][j], f2_pack(sc[2 * j], sc[2 * j + 1]));
+        for (int j = 0; j < 8; ++j) {
+          const f32x2 s2 = f2_pack(sc[2 * j], sc[2 * j + 1]);
+          t[j] = f2_mul(dw[x][j], TERMS ? f2_add(s2, c2) : s2);
+          if (TERMS) n2 = f2_add(n2, t[j]);
+        }
         split(t, hi[k], lo[k]);
       };
 #pragma unroll
       for (int x = 0; x < BLOCKS / 2; ++x)
         if (on(x)) products(x, x);
-      w.wait(&z_full, (r - 1) & 1, 0x24);            // X of r - 1 has been read
+      if (r > 0) w.wait(&z_full, (r - 1) & 1, 0x24);            // X of r - 1 has been read
       __syncwarp();
       fence_after_sync();
 #pragma unroll
@@ -326,7 +372,15 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
       tmem_st_wait();
       fence_before_sync();
       warp_arrive(&x_full, lane);
-      drain(r - 1);
+      if (r > 0) drain(r - 1);
+      if constexpr (TERMS) {
+        float n0, n1;
+        f2_unpack(n2, n0, n1);
+        n0 += n1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) n0 += __shfl_xor_sync(0xffffffffu, n0, o);
+        if (lane == 0) n_s[warp][r] = n0;
+      }
     }
     const int rows = max(tile.nc - 32 * my_rb, 0);            // of the row block that exist
     const size_t out0 = (((size_t)tile.b * a.Hq + my_head) * a.N + tok0 + 32 * my_rb + (lane >> 2)) * HD + d0 + 2 * m;
@@ -360,34 +414,83 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
       if (lane == 0) sum_s[warp] = s0;
-      // the quadrant's warps: sums of y over the dims of each group, then dA, dB and dC (symmetrised: both orders are
-      // the same sum)
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + qd), "n"(BQ_SUBS * 32) : "memory");
+      // the quadrant's warps: dA, dB and the upper triangle of dC from the sums (symmetrised: both orders are the same sum)
+      const auto quadrant_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + qd), "n"(BQ_SUBS * 32) : "memory"); };
+      const auto triangle = [](int x, int n, int& i, int& j) {      // x-th entry of an upper triangle, row-major
+        i = 0;
+        while (x >= n - i) { x -= n - i; ++i; }
+        j = i + x;
+      };
+      quadrant_sync();
       const float* y = ys + qd * RMAX_ALL * HD;
-      for (int x = sub * 32 + lane; x < a.rank * G; x += BQ_SUBS * 32) {
-        const int r = x / G, g = x % G, end = order.start[g + 1];
-        float t = 0.f;
-#pragma unroll 4
-        for (int p = order.start[g]; p < end; ++p) t += y[r * HD + p];
-        cls_s[qd][x] = t;
-      }
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + qd), "n"(BQ_SUBS * 32) : "memory");
-      const int slots = 1 + G + G * (G + 1) / 2, blocks = (a.N + 31) / 32;
+      const int slots = 1 + G + G * (G + 1) / 2, blocks = (a.N + 31) / 32, first = sub * 32 + lane;
       float* dst = a.coef_partial + (((size_t)tile.b * a.Hq + my_head) * blocks + tile.c * 4 + my_rb) * slots;
-      for (int x = sub * 32 + lane; x < slots && rows > 0; x += BQ_SUBS * 32) {
-        float t;
-        if (x == 0) {
-          t = 0.f;
-#pragma unroll
-          for (int y = 0; y < BQ_SUBS; ++y) t += sum_s[4 * y + qd];
-        } else if (x <= G) {
-          t = a.scale * cls_s[qd][x - 1];
-        } else {
-          int g = 0, rest = x - 1 - G;
-          while (rest >= G - g) { rest -= G - g; ++g; }
-          t = 0.5f * a.scale * a.scale * (cls_s[qd][(1 + g) * G + g + rest] + cls_s[qd][(1 + g + rest) * G + g]);
+      if constexpr (TERMS) {
+        const auto n_of = [&](int r) { return (n_s[qd][r] + n_s[4 + qd][r]) + (n_s[8 + qd][r] + n_s[12 + qd][r]); };
+        const float* t = reinterpret_cast<const float*>(mask_s + qd * GMAX * (HD / 2));
+        float *D = ys + BQ_Y + 2 * qd * BQ_D, *tD = D + BQ_D;
+        const int rank = a.rank;
+        for (int x = first; x < rank * (rank + 1) / 2; x += BQ_SUBS * 32) {
+          int r, r2;
+          triangle(x, rank, r, r2);
+          float s = fmaf(hs.c[r2], n_of(r), hs.c[r] * n_of(r2));
+#pragma unroll 4
+          for (int k = 0; k < HD; k += 4) {
+            const int d = (k + 4 * lane) % HD;                      // rows start in the same bank: every lane elsewhere
+            const float4 la = *reinterpret_cast<const float4*>(l + r * HD + d), lb = *reinterpret_cast<const float4*>(l + r2 * HD + d);
+            const float4 ya = *reinterpret_cast<const float4*>(y + r * HD + d), yb = *reinterpret_cast<const float4*>(y + r2 * HD + d);
+            s = fmaf(lb.x, ya.x, fmaf(lb.y, ya.y, fmaf(lb.z, ya.z, fmaf(lb.w, ya.w, s))));
+            s = fmaf(la.x, yb.x, fmaf(la.y, yb.y, fmaf(la.z, yb.z, fmaf(la.w, yb.w, s))));
+          }
+          D[r * RMAX_ALL + r2] = D[r2 * RMAX_ALL + r] = 0.5f * s;
         }
-        dst[x] = t;
+        quadrant_sync();
+        for (int x = first; x < G * rank; x += BQ_SUBS * 32) {
+          const int g = x / rank, r2 = x % rank;
+          float s = 0.f;
+#pragma unroll 4
+          for (int r = 0; r < rank; ++r) s = fmaf(t[(1 + g) * T_PITCH + r], D[r * RMAX_ALL + r2], s);
+          tD[g * RMAX_ALL + r2] = s;
+        }
+        quadrant_sync();
+        for (int x = first; x < slots && rows > 0; x += BQ_SUBS * 32) {
+          float s = 0.f;
+          if (x == 0) {
+            s = (sum_s[qd] + sum_s[4 + qd]) + (sum_s[8 + qd] + sum_s[12 + qd]);
+          } else if (x <= G) {
+            for (int r = 0; r < rank; ++r) s = fmaf(t[x * T_PITCH + r], n_of(r), s);
+          } else {
+            int g, g2;
+            triangle(x - 1 - G, G, g, g2);
+#pragma unroll 4
+            for (int r = 0; r < rank; ++r) s = fmaf(tD[g * RMAX_ALL + r], t[(1 + g2) * T_PITCH + r], s);
+          }
+          dst[x] = s;
+        }
+      } else {
+        for (int x = first; x < a.rank * G; x += BQ_SUBS * 32) {     // sums of y over the dims of each group
+          const int r = x / G, g = x % G, end = order.start[g + 1];
+          float t = 0.f;
+#pragma unroll 4
+          for (int p = order.start[g]; p < end; ++p) t += y[r * HD + p];
+          cls_s[qd][x] = t;
+        }
+        quadrant_sync();
+        for (int x = first; x < slots && rows > 0; x += BQ_SUBS * 32) {
+          float t;
+          if (x == 0) {
+            t = 0.f;
+#pragma unroll
+            for (int y = 0; y < BQ_SUBS; ++y) t += sum_s[4 * y + qd];
+          } else if (x <= G) {
+            t = a.scale * cls_s[qd][x - 1];
+          } else {
+            int g, g2;
+            triangle(x - 1 - G, G, g, g2);
+            t = 0.5f * a.scale * a.scale * (cls_s[qd][(1 + g) * G + g2] + cls_s[qd][(1 + g2) * G + g]);
+          }
+          dst[x] = t;
+        }
       }
     }
   }
@@ -777,12 +880,15 @@ int intra_row_blocks(int N) { return (N + 31) / 32; }
 cudaError_t intra_backward_q(const RowImages& rows, const void* gimg, const void* factors, void* dq, const float* dq_init,
                              float* coef_partial, int32_t* status, int B, int Hq, int Hkv, int N, int NB, int groups, float scale,
                              int cross_from, cudaStream_t st) {
-  cudaError_t e = allow_smem<intra_bwd_q_kernel>(BQ_SMEM);
+  const bool terms = coef_partial && NB == 1;
+  cudaError_t e = terms ? allow_smem<intra_bwd_q_kernel<true>>(BQ_SMEM) : allow_smem<intra_bwd_q_kernel<false>>(BQ_SMEM);
   if (e != cudaSuccess) return e;
   IntraBwdArgs a = bwd_args(rows, gimg, factors, status, B, Hq, Hkv, N, NB, groups);
   a.scale = scale;
   a.dq = static_cast<__nv_bfloat16*>(dq); a.dq_init = dq_init; a.coef_partial = coef_partial; a.cross_from = cross_from;
-  intra_bwd_q_kernel<<<dim3(NB, B * Hkv, Hq / Hkv), BQ_THREADS, BQ_SMEM, st>>>(a);
+  const dim3 grid(NB, B * Hkv, Hq / Hkv);
+  if (terms) intra_bwd_q_kernel<true><<<grid, BQ_THREADS, BQ_SMEM, st>>>(a);
+  else intra_bwd_q_kernel<false><<<grid, BQ_THREADS, BQ_SMEM, st>>>(a);
   return cudaGetLastError();
 }
 

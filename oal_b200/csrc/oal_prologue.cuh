@@ -96,8 +96,8 @@ __device__ __forceinline__ void one_sided_jacobi(PrologueSmem& s, int n, int lan
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
   if (lane < n) {
-    // a vanishing term keeps its direction at a negligible weight; a NaN (which fmaxf would drop) stays one and reaches
-    // weights and status
+    // a vanishing term keeps its direction at a negligible weight, so that the coefficient gradient of a
+    // singular factor can be rotated back; a NaN (which fmaxf would drop) stays one and reaches weights and status
     const float least = fmaxf(1e-12f * top, 1e-30f);
     s.lam[lane] = sqrtf(norm < least ? least : norm);
 #pragma unroll
@@ -158,6 +158,7 @@ __device__ __forceinline__ void head_prologue(const PrologueArgs& a, int h, Prol
     const int r = x / HD, d = x % HD;
     out.l[r][d] = r < n ? a.scale * s.lam[r] * s.V[1 + s.gdim[d]][r] : 0.f;
   }
+  for (int x = tid; x < n * n; x += nthreads) out.t[x / n][x % n] = s.V[x / n][x % n] / s.lam[x % n];
   const float (*M)[RMAX_ALL + 1] = s.M;
   write_head_groups(out.e, out.mask, out.order, s.gdim, a.dim_perm + h * HD, a.group_start + h * (GMAX + 1), a.G, a.scale,
                     [&](int g) { return 2.f * M[0][1 + g]; }, [&](int g, int g2) { return 2.f * M[1 + g][1 + g2]; }, tid, nthreads);
