@@ -80,3 +80,30 @@ def assert_close(res, ref, tol, keys=None, label=""):
     bad = {k: v for k, v in worst.items() if not v <= tol}
     assert not bad, f"{label} normalized max error above {tol}: {bad} (all: {worst})"
     return worst
+
+
+def saved_state_parts(saved, *, batch, q_heads, kv_heads, n, groups):
+    """The bytes of a saved state (CPU uint8) that a forward writes, by name: an image's last block of 8 columns, table rows
+    beyond the groups and the gaps between the parts are never written or read."""
+    units_chunks, at, parts = batch * kv_heads * -(-n // 128), 0, {}
+
+    def take(size):
+        nonlocal at
+        piece = saved[at:at + size]
+        at += -(-size // 256) * 256
+        return piece
+
+    for name in ("image", "remainders"):
+        parts[name] = take(units_chunks * 19 * 10 * 2048).view(units_chunks, 19, 10, 2048)[:, :, :9]
+    table = take(q_heads * 12288).view(q_heads, 12288)
+    floats = lambda lo, rows, width, used: table[:, lo:lo + rows * width * 4].reshape(q_heads, rows, width * 4)[..., :used * 4]
+    parts["scalars"] = table[:, :80]
+    parts["l"] = floats(80, 17, 64, 64)
+    parts["e"] = floats(4432, groups + 1, 64, 64)
+    parts["mask"] = floats(8784, groups, 32, 32)
+    parts["order"] = table[:, 10832:10928]
+    parts["t"] = floats(10928, groups + 1, 20, groups + 1)
+    parts["coefficients"] = take(q_heads * 2432 * 4)
+    parts["k"] = take(units_chunks * 8 * 2048)
+    parts["u"] = take(units_chunks * 10 * 2048)
+    return parts

@@ -17,11 +17,14 @@ from oal_b200 import _lib, synthetic
 from oal_b200.hd_block_gemm import make_problem
 from oal_b200.hd_block_gemm_autograd import build_group_tables
 from oracle import oal_oracle as orc
+from tests.helpers import saved_state_parts
 
 pytestmark = pytest.mark.gpu
 
 
 def _call(entry, case, use_static):
+    """(out, num, den, parts of the saved state); a saved state starts as a pattern of its entry's own, so that equal parts were
+    written by both."""
     lib = _lib.load()
     dev = torch.device("cuda")
     q, k, v = (t.to(dev, torch.bfloat16).contiguous() for t in (case.q, case.k, case.v))
@@ -37,7 +40,7 @@ def _call(entry, case, use_static):
     out = torch.empty(b, hq, n, 64, dtype=torch.bfloat16, device=dev)
     num = torch.empty(b, hq, n, 64, dtype=torch.float32, device=dev)
     den = torch.empty(b, hq, n, dtype=torch.float32, device=dev)
-    saved = torch.empty(_lib.workspace_bytes(problem, 2), dtype=torch.uint8, device=dev)
+    saved = torch.full((_lib.workspace_bytes(problem, 2),), 0x5A if use_static else 0xA5, dtype=torch.uint8, device=dev)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
     stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
     common = [ctypes.byref(problem), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(tables.dim_perm),
@@ -51,7 +54,8 @@ def _call(entry, case, use_static):
     _lib.check(rc)
     torch.cuda.synchronize()
     assert int(status.item()) == 0
-    return out.float().cpu(), num.cpu(), den.cpu(), saved.cpu()
+    parts = saved_state_parts(saved.cpu(), batch=b, q_heads=hq, kv_heads=hkv, n=n, groups=g)
+    return out.float().cpu(), num.cpu(), den.cpu(), parts
 
 
 def test_static_scratch_forward_matches_workspace_forward_twice():
@@ -62,7 +66,8 @@ def test_static_scratch_forward_matches_workspace_forward_twice():
         got = _call("static", case, use_static=True)
         for name, x, y in zip(("out", "num", "den", "saved_state"), got, want):
             if name == "saved_state":
-                assert torch.equal(x, y), name
+                for part in x:
+                    assert torch.equal(x[part], y[part]), part
             else:
                 assert orc.normalized_max_error(x, y) <= 1e-6, name
 
@@ -138,7 +143,8 @@ def test_static_scratch_limits_are_exact(batch, hkv, n, hq, accepted):
             scale=0.125, factor=torch.rand(hq, 6, generator=g) * 0.9 + 0.1)
         want = _call("workspace", case, use_static=False)
         got = _call("static", case, use_static=True)
-        assert torch.equal(got[3], want[3])
+        for part in got[3]:
+            assert torch.equal(got[3][part], want[3][part]), part
         assert orc.normalized_max_error(got[0], want[0]) <= 1e-6
         return
     problem = make_problem((batch, hq, hkv, n, 64, 64), groups=2, io_dtype=torch.bfloat16, out_dtype=torch.bfloat16,
