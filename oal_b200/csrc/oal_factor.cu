@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(32) head_factor_kernel(const int32_t* dim_perm
 
 __device__ __forceinline__ int tri_all(int g, int g2) { return g * GMAX - (g * (g - 1)) / 2 + (g2 - g); }
 
-// The prologue on its own, where no state kernel runs whose launch it could share (state_update_kernel).
+// The prologue on its own: on a side stream, or for calls without row images (rows_prologue_kernel shares its launch with it).
 __global__ void __launch_bounds__(256) head_prologue_kernel(const PrologueArgs a) {
   __shared__ PrologueSmem s;
   head_prologue(a, blockIdx.x, s, threadIdx.x, 256);
