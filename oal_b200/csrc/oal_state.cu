@@ -13,6 +13,8 @@
 // memory, and never touch HBM.
 // The fp32 accumulators live in tensor memory; state images are streamed with 1-D bulk
 // async copies.  Every mbarrier wait is bounded (oal_umma.cuh).
+#include <algorithm>
+
 #include "oal_features.cuh"
 #include "oal_kernels.h"
 #include "oal_prologue.cuh"
@@ -238,10 +240,11 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const float* ds, __nv_b
 //               the MMA  Z[c % 2] = A^T [v | 1]
 //   warps 4-15  thread = (feature row, 24 columns): image c written while the MMA runs, then the increment of chunk c added;
 //               warp 4 has the image of [v | 1] two chunks on copied in
-// What bounds it: the stores of a block's SM, 37 KB per chunk at 16 bytes per clock (2350 clocks per chunk, whatever the
-// generators do: eight warps, or all in one set of warps, are no faster).  In two kernels the increments, twice the images'
-// bytes, go to memory and back: 135 -> 77 us at B = 4, N = 4096, 2 KV heads (152 blocks: two on four SMs); with 2 units the walk
-// takes 51 us against 42, so state_walk_pays() asks for three, or a short sequence.
+// What bounds it: the chain of a chunk (features, MMA, drain) for a block alone on its SM, 1.4 us per chunk with remainder images
+// and 1.2 without; with two blocks the stores of an SM, 37 KB per chunk and block at 16 bytes per clock (2350 clocks, whatever
+// the generators do: eight warps, or all in one set of warps, are no faster).  In two kernels the increments, twice the images'
+// bytes, go to memory and back: 135 -> 77 us at B = 4, N = 4096, 2 KV heads (152 blocks: two on four SMs); one or two units leave
+// most SMs without a block, see state_walk_pays().
 // ---------------------------------------------------------------------------
 struct StateWalkArgs {
   const unsigned char *k_image, *u_image;
@@ -632,11 +635,20 @@ cudaError_t state_update(const void* k, const void* v, float* ds, int units, int
   return cudaGetLastError();
 }
 
-// The walk's time by chunks, against what the two kernels need for increments to memory and back: 1.25 us per chunk and
-// block of an SM, 0.53 us per chunk and unit and 6 us for the second launch and its first loads.
+// The walk against the two kernels, whose increments go to memory and back: a chunk costs the walk 1.3 us (its blocks' chain)
+// and the two kernels 0.36 us per unit and, once, 7.6 us for the second launch and its first loads; a walk of a few units that
+// writes more than about 1000 chunks in all loses another 0.9 us per chunk.  Whole forwards as recorded graphs, walk less two
+// steps in us, with (without) remainder images:
+//   units      4 chunks    8             16            32           64           128          256          512
+//     1       -6 (-6)     0 (-2)       +10 (+6)      +30 (+24)    +60 (+48)   +115 (+98)   +231 (+184)  +478 (+393)
+//     2       -6 (-5)    -2 (-2)        +7 (+3)      +16 (+12)    +36 (+26)    +67 (+47)   +154 (+111)  +407 (+274)
+//     3       -6 (-7)    -3 (-4)        -3 (-4)       -4 (-6)      +3 (-1)      +3 (+1)     +44 (+19)   +185 (+159)
+//     4       -7 (-7)    -2 (-4)        -6 (-5)       -7 (-10)    -24 (-20)    -40 (-36)    -25 (-30)    +53 (+73)
+//     6       -7 (-7)   -11 (-13)      -22 (-22)     -41 (-32)    -80 (-72)   -108 (-114)  -173 (-138)  -305 (-211)
+//    14      -14 (-15)  -30 (-30)      -63 (-54)    -121 (-121)  -221 (-220)  -422 (-387)  -823 (-736)
+//    32      -25 (-25)  -71 (-62)     -134 (-126)   -261 (-240)  -532 (-463) -1051 (-906)
 bool state_walk_pays(int units, int NB) {
-  const int sms = sm_count(), per_sm = (F_SLABS * units + sms - 1) / sms;
-  return 1.25 * per_sm * NB < 0.53 * units * NB + 6.;
+  return NB * (1.3 - 0.36 * units) + 0.9 * std::max(0, NB - 1000 / units) < 7.6;
 }
 
 cudaError_t rows_prologue(const RowImages& rows, int units, int N, int NB, const PrologueArgs* prologue, int q_heads, cudaStream_t st) {
