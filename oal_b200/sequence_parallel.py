@@ -61,6 +61,16 @@ def exclusive_prefix_over_ranks(local: torch.Tensor, group=None, *, reverse: boo
     return total
 
 
+def _workspace(prepared, phase: int, like: torch.Tensor) -> torch.Tensor:
+    """Forward (0) or backward (1) workspace of a call: what this library needs, whatever a plan that was stored by another
+    build says."""
+    plan = prepared.plan
+    problem = make_problem(plan.geometry, groups=prepared.tables.group_count, io_dtype=like.dtype, out_dtype=like.dtype,
+                           precision=plan.precision, chunk=plan.chunk_tokens, scale=1.0, floor=1e-38)
+    stored = (plan.forward_workspace_bytes, plan.backward_workspace_bytes)[phase]
+    return torch.empty(max(stored, _lib.workspace_bytes(problem, phase), 16), dtype=torch.uint8, device=like.device)
+
+
 def local_state_total(k: torch.Tensor, v: torch.Tensor, plan, groups: int = 1, workspace=None) -> torch.Tensor:
     """fp32 ``[B*Hkv, 2432, 80]``: this rank's contribution to the running state.  With ``workspace``
     (``plan.forward_workspace_bytes`` bytes) the chunk-state increments stay there for the forward."""
@@ -112,7 +122,7 @@ class _SequenceParallelFunction(torch.autograd.Function):
         plan = prepared.plan
         mask = tuple(bool(x) for x in ctx.needs_input_grad[:6])
         ctx.set_materialize_grads(False)
-        ws = torch.empty(max(plan.forward_workspace_bytes, 16), dtype=torch.uint8, device=q.device)
+        ws = _workspace(prepared, 0, k)
         state_in = exclusive_prefix_over_ranks(local_state_total(k, v, plan, prepared.gmax, workspace=ws), group)
         out, num, den, saved_state, padded = forward_impl(q, k, v, a, b, c, prepared.tables, prepared.scale,
                                                           prepared.normalization_floor, plan, state_in=state_in,
@@ -137,7 +147,7 @@ class _SequenceParallelFunction(torch.autograd.Function):
         if ctx.forward_status is not None:
             if not torch.cuda.is_current_stream_capturing():
                 ctx.forward_status.check(block=False)    # this call's own forward, if it has finished
-        ws = torch.empty(max(plan.backward_workspace_bytes, 16), dtype=torch.uint8, device=num.device)
+        ws = _workspace(prepared, 1, padded[0])
         local = local_dstate_total(padded, num, den, state, prepared.tables, prepared.scale,
                                    prepared.normalization_floor, plan, mask, grad_output, grad_numerator,
                                    grad_denominator, ws)

@@ -53,6 +53,22 @@ def test_a_plan_with_the_sizes_of_another_build_gets_room_enough(general):
         assert torch.equal(got, want)
 
 
+def test_a_sequence_parallel_call_with_the_sizes_of_another_build_gets_room_enough():
+    from oal_b200.sequence_parallel import sequence_parallel_attention
+
+    make, live = _prepared()
+    q, k, v, factor = (t.clone().requires_grad_(True) for t in live)
+    groups = (torch.arange(64) % 4).to(torch.int32).cuda()
+    prepared = make()
+    plan = dataclasses.replace(prepared.plan, forward_workspace_bytes=16, backward_workspace_bytes=16, saved_state_bytes=16)
+    results = []
+    for each in (prepared, dataclasses.replace(prepared, plan=plan)):
+        out = sequence_parallel_attention(q, k, v, groups, factor, prepared=each)
+        results.append([*out, *torch.autograd.grad(out[0].float().sum(), (q, k, v, factor))])
+    for got, want in zip(results[1], results[0]):
+        assert torch.equal(got, want)
+
+
 def test_a_changed_copy_runs_its_own_options():
     make, live = _prepared()
     prepared = make()
