@@ -1107,6 +1107,7 @@ int oal_backward_local_state(const OalProblem* p, const void* q, const int32_t* 
   if (rc) return rc;
   if (p->precision != OAL_PRECISION_BF16_TENSORCORE)
     return fail(OAL_ERR_DTYPE, "oal_backward_local_state: chunk states exist only in bf16_tensorcore mode");
+  if (p->flags & OAL_FLAG_NO_BACKWARD) return fail(OAL_ERR_ARGUMENT, "oal_backward_local_state: the problem says that no backward follows");
   if (!q || !dim_perm || !group_start || !coef_a || !coef_b || !coef_c || !num || !den || !saved_state || !dstate_total || !status)
     return fail(OAL_ERR_ARGUMENT, "oal_backward_local_state: NULL tensor pointer");
   if (misaligned({q, num, saved_state, grad_out, grad_num, dstate_total, workspace}))

@@ -60,3 +60,16 @@ def test_contract_violations_map_to_reference_exception_types():
     lib = _lib.load()
     rc = lib.oal_forward(ctypes.byref(bad), *([None] * 14), 0, None, None)
     assert rc < 0
+
+
+def test_backward_entries_refuse_a_problem_without_backward():
+    import torch
+
+    lib = _lib.load()
+    p = make_problem((1, 2, 2, 300, 64, 64), groups=4, io_dtype=torch.bfloat16, out_dtype=torch.bfloat16, precision="bf16_tensorcore",
+                     chunk=128, scale=1.0, floor=1e-38, flags=_lib.FLAG_NO_BACKWARD)
+    one = ctypes.c_void_p(256)      # never read: nothing is launched (no room in the workspace either)
+    assert lib.oal_backward(ctypes.byref(p), *([one] * 22), 0, one, None) == -1
+    assert b"no backward follows" in lib.oal_last_error_string()
+    assert lib.oal_backward_local_state(ctypes.byref(p), *([one] * 14), 0, one, None) == -1
+    assert b"no backward follows" in lib.oal_last_error_string()
