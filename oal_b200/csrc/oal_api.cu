@@ -586,7 +586,7 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
     e = oal::build_coef_table(dim_perm, group_start, src.A, src.B, src.C, p->q_heads, p->groups, p->scale, coef_table, st);
     if (e != cudaSuccess) return fail_cuda(e, "coefficient table kernel");
   }
-  const bool walk = update && timing && oal::state_walk_pays(units, nb);
+  const bool walk = update && oal::state_walk_pays(units, nb);
   const bool backward = !(p->flags & OAL_FLAG_NO_BACKWARD);
   if (tc && (src.factor || walk || backward)) {
     LaunchScope scope("rows_prologue", st, 1, timing);

@@ -72,6 +72,18 @@ def test_static_scratch_forward_matches_workspace_forward_twice():
                 assert orc.normalized_max_error(x, y) <= 1e-6, name
 
 
+@pytest.mark.parametrize("hkv,n", [(2, 300), (1, 1700), (2, 120)])
+def test_static_scratch_forward_queues_the_launches_of_the_regular_one(hkv, n):
+    """The same route to the carry images, on both sides of the rule that picks it."""
+    case = synthetic.qwen_head_case(34, batch=1, n=n, hq=4, hkv=hkv, g=4, bf16=True)
+    counts = []
+    for static in (False, True):
+        before = _lib.launch_count()
+        _call("static" if static else "workspace", case, use_static=static)
+        counts.append(_lib.launch_count() - before)
+    assert counts[0] == counts[1]
+
+
 def _static_call_on_device_tensors(case):
     """Everything the call needs is created first; returns a closure that only makes the library call."""
     lib = _lib.load()
