@@ -255,8 +255,9 @@ int oal_selftest_umma(int mode, int n, int k, const void* a, const void* b, floa
 /*
  * Self-test of the bounded-wait path every tensor-core kernel relies on (no counterpart in the reference,
  * which has no device-side waits).  One warp waits on a barrier that nothing arrives on, with a limit of
- * `limit_clocks` SM clocks (1 .. 1 000 000, i.e. at most about half a millisecond); the wait gives up and
- * the kernel ORs OAL_STATUS_WAIT_TIMEOUT | (0x7E << 8) into *status and returns normally, exactly as the
+ * `limit_clocks` SM clocks (1 .. 1 000 000, i.e. at most about half a millisecond); the wait gives up, the kernel
+ * pauses for 2 ms (copies in flight would land meanwhile) and
+ * ORs OAL_STATUS_WAIT_TIMEOUT | (0x7E << 8) into *status and returns normally, exactly as the
  * production kernels do after their 50 M-clock limit.  Nothing hangs or faults; the context stays usable.
  */
 int oal_selftest_wait_timeout(int64_t limit_clocks, int32_t* status, void* stream);

@@ -264,13 +264,29 @@ __device__ __forceinline__ uint4 load_ahead(const void* p) {
 
 // Bounded mbarrier waits for one CTA: the first wait that expires raises a shared flag and every
 // later wait returns at once, so a kernel always terminates; the flag ends up in the status word.
+// A thread that issues bulk copies stops at its first wait that was not met, and a CTA that gave up settles before it frees
+// its tensor memory and leaves: a bulk copy that lands in the shared memory of a CTA that has left is a launch failure, and
+// the barriers that would tell when the last one is in have lost their phases.  (MMAs touch the CTA's own memory only and
+// queue a few deep: their thread runs its loop to the end.  With a check there the cross read took 111 us instead of 108.)
 struct Waiter {
   int* dead;          // shared flag: a wait expired somewhere in this CTA (holds the site id, >= 1)
-  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, int site = 1) {
-    if (umma::mbar_test(bar, parity)) return;           // already complete: the common case costs one probe
-    if (*reinterpret_cast<volatile int*>(dead)) return;
-    if (!umma::mbar_wait(bar, parity)) *reinterpret_cast<volatile int*>(dead) = site;
+  __device__ __forceinline__ bool gave_up() const { return *reinterpret_cast<volatile int*>(dead) != 0; }
+  // whether the phase has completed; false: this or another thread's wait expired
+  __device__ __forceinline__ bool met(uint64_t* bar, uint32_t parity, int site) {
+    if (umma::mbar_test(bar, parity)) return true;      // already complete: the common case costs one probe
+    if (gave_up()) return false;
+    if (umma::mbar_wait(bar, parity)) return true;
+    *reinterpret_cast<volatile int*>(dead) = site;
+    return false;
   }
+  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, int site = 1) { met(bar, parity, site); }
+  // Every thread, after the last barrier of the CTA.  What is still in flight then (at most the shared memory of an SM, and
+  // the queue of MMAs) takes microseconds; the pause is a thousand times that.
+  __device__ __forceinline__ void settle() const {
+    if (!gave_up()) return;
+    for (const long long t0 = clock64(); clock64() - t0 < SETTLE_CLOCKS;) __nanosleep(1000);
+  }
+  static constexpr long long SETTLE_CLOCKS = 4000000;      // 2 ms
   // status bits to OR into the caller's word: the timeout flag plus the site id in bits 8..15
   __device__ __forceinline__ int status_bits() const {
     const int d = *reinterpret_cast<volatile int*>(dead);

@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(FW_THREADS, 2) intra_fwd_kernel(const IntraFwd
   }
   if (flags) atomicOr(a.status, flags);
   __syncthreads();
+  w.settle();
   if (warp == 0) tmem_dealloc(tmem_base, 256);
   if (tid == 0) {
     if (dead) atomicOr(a.status, w.status_bits());

@@ -496,6 +496,7 @@ __global__ void __launch_bounds__(BQ_THREADS, 1) intra_bwd_q_kernel(const IntraB
   }
   fence_before_sync();
   __syncthreads();
+  w.settle();
   if (warp == 0) tmem_dealloc(tmem_base, 512);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
@@ -621,8 +622,8 @@ __global__ void __launch_bounds__(KvWarps<FINE>::THREADS, 1) intra_bwd_kv_kernel
               mma_bf16_ts(z, tmem + (part ? BK_PLO : BK_P) + 8 * ks, desc_advance(dq, ks * 256), instr_desc_bf16(128, HD, 0, 1), part + ks > 0);
           mma_commit(&z_full);
           if (r == 0 && i > 0 && i + 1 < n_heads) {
-            w.wait(&v_full, (i - 1) & 1, 0x34);             // head i - 1 no longer reads the set that head i + 1 takes
-            fetch_head(i + 1);
+            // head i - 1 no longer reads the set that head i + 1 takes
+            if (w.met(&v_full, (i - 1) & 1, 0x34)) fetch_head(i + 1);
           }
         }
         T += rank;
@@ -830,6 +831,7 @@ __global__ void __launch_bounds__(KvWarps<FINE>::THREADS, 1) intra_bwd_kv_kernel
   }
   fence_before_sync();
   __syncthreads();
+  w.settle();
   if (warp == 0) tmem_dealloc(tmem_base, 512);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }

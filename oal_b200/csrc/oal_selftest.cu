@@ -3,6 +3,7 @@
 // It exists so that a wrong descriptor encoding shows up as a failed unit test with
 // a small, readable error instead of as a parity failure of the whole operator.
 #include "oal_common.cuh"
+#include "oal_features.cuh"
 #include "oal_umma.cuh"
 
 namespace oal {
@@ -105,9 +106,9 @@ __global__ void __launch_bounds__(128) umma_selftest_kernel(const __nv_bfloat16*
   if (warp == 0) tmem_dealloc(tmem_base, 512);
 }
 
-// One warp waits on an mbarrier that nothing ever arrives on, with a short limit: the wait gives up,
-// the kernel records the status word exactly as the production kernels do (timeout flag + site id)
-// and returns normally.  Nothing hangs, traps or faults; the context stays usable.
+// One thread waits on an mbarrier that nothing ever arrives on, with a short limit: the wait gives up, the other threads'
+// wait on it returns at once, the kernel settles, records the status word exactly as the production kernels do (timeout flag
+// + site id) and returns normally.  Nothing hangs, traps or faults; the context stays usable.
 constexpr int SELFTEST_WAIT_SITE = 0x7E;
 __global__ void __launch_bounds__(32) wait_timeout_selftest_kernel(long long limit_clocks, int* status) {
   __shared__ uint64_t bar;
@@ -118,10 +119,13 @@ __global__ void __launch_bounds__(32) wait_timeout_selftest_kernel(long long lim
     dead = 0;
   }
   __syncwarp();
-  if (threadIdx.x == 0) {
-    if (!mbar_wait(&bar, 0, limit_clocks)) dead = SELFTEST_WAIT_SITE;
-    if (dead) atomicOr(status, OAL_STATUS_WAIT_TIMEOUT | ((dead & 0xFF) << 8));
-  }
+  if (threadIdx.x == 0 && !mbar_wait(&bar, 0, limit_clocks)) dead = SELFTEST_WAIT_SITE;
+  __syncthreads();
+  Waiter w{&dead};
+  const bool met = w.met(&bar, 0, SELFTEST_WAIT_SITE + 1);
+  __syncthreads();
+  w.settle();
+  if (threadIdx.x == 31 && !met) atomicOr(status, w.status_bits());
 }
 
 }  // namespace

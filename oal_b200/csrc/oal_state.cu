@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) state_update_kernel(const Stat
   }
   epilogue(ns - 1);
   __syncthreads();
+  w.settle();
   if (warp == 0) tmem_dealloc(tmem_base, 256);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(SW_THREADS, 2) state_walk_kernel(const StateWa
       }
       if (c >= n) break;
       w.wait(&z_full[c & 1], (c >> 1) & 1, 0x14);
-      if (warp == SW_GEN_WARPS && lane == 0 && c + 2 < n) fetch_u(c + 2);
+      if (warp == SW_GEN_WARPS && lane == 0 && c + 2 < n && !w.gave_up()) fetch_u(c + 2);
       __syncwarp();
       fence_after_sync();
       const uint32_t t = tmem + (c & 1) * EP + ((uint32_t)(32 * (warp & 3)) << 16) + 8 * e0;
@@ -385,6 +386,7 @@ __global__ void __launch_bounds__(SW_THREADS, 2) state_walk_kernel(const StateWa
   }
   fence_before_sync();
   __syncthreads();
+  w.settle();
   if (warp == 0) tmem_dealloc(tmem_base, 256);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
@@ -584,13 +586,13 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
       int slot = 0, use = 0;
       const auto fetch_coef = [&](int k) {
         const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
-        if (k >= 2) w.wait(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x48);   // item k-2 no longer reads this buffer
+        if (k >= 2 && !w.met(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x48)) return;   // item k-2 no longer reads this buffer
         mbar_arrive_expect_tx(&coef_full[k & 1], F_ROWS * (uint32_t)sizeof(float));
         bulk_g2s(smem + CR_COEF + (k & 1) * F_ROWS * sizeof(float), a.coef_table + (size_t)it.h * F_ROWS,
                  F_ROWS * (uint32_t)sizeof(float), &coef_full[k & 1]);
       };
       if (QUERY && my_items > 0) fetch_coef(0);
-      for (int k = 0; k < my_items; ++k) {
+      for (int k = 0; k < my_items && !w.gave_up(); ++k) {
         const CrItem it = cr_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         const int unit = (it.b * a.H + it.h) / a.rep;
         const unsigned char* img = reinterpret_cast<const unsigned char*>(a.image) +
@@ -598,7 +600,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
         for (int s = 0; s < F_SLABS; ++s) {
           // the next item's table while there is time: its buffer's last reader was item k-1
           if (QUERY && s == 2 * F_SLABS / 3 && k + 1 < my_items) fetch_coef(k + 1);
-          if (use > 0) w.wait(&done[slot], (use - 1) & 1, 0x46);
+          if (use > 0 && !w.met(&done[slot], (use - 1) & 1, 0x46)) break;
           // the unused columns of an image only reach unused columns of the accumulator
           mbar_arrive_expect_tx(&full[slot], SLAB_U_BYTES);
           bulk_g2s(smem + slot * SLAB_S_BYTES, img + (size_t)s * SLAB_S_BYTES, SLAB_U_BYTES, &full[slot]);
@@ -610,6 +612,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1) cross_read_kernel(const CrossRe
   }
   fence_before_sync();
   __syncthreads();
+  w.settle();
   if (warp == CR_ISSUER) tmem_dealloc(tmem_base, 512);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }

@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
       int s = 0, use = 0, fetched = 0;
       const auto fetch_carry = [&](const DsCursor& x) {
         const size_t at = (((size_t)x.u * a.NB + x.c) * F_SLABS + x.slab) * SLAB_S_BYTES;
-        if (fetched > 0) w.wait(&carry_free, (fetched - 1) & 1, 0x38);      // in registers of the drain warps
+        if (fetched > 0 && !w.met(&carry_free, (fetched - 1) & 1, 0x38)) return;      // in registers of the drain warps
         ++fetched;
         mbar_arrive_expect_tx(&carry_full, 2 * SLAB_U_BYTES);
         bulk_g2s(smem + DS_CARRY, reinterpret_cast<const unsigned char*>(a.carry_img) + at, SLAB_U_BYTES, &carry_full);
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
         const int h = d.h0 + d.hh;
         const unsigned char* src =
             reinterpret_cast<const unsigned char*>(a.gimg) + ((size_t)(d.b * a.Hq + h) * a.NB + d.c) * SLAB_S_BYTES;
-        if (use > 0) w.wait(&mma_done[s], (use - 1) & 1, 0x36);
+        if (use > 0 && !w.met(&mma_done[s], (use - 1) & 1, 0x36)) break;
         mbar_arrive_expect_tx(&ready[s], SLAB_U_BYTES + 128 * 4);
         bulk_g2s(Gbuf + s * SLAB_U_BYTES, src, SLAB_U_BYTES, &ready[s]);
         bulk_g2s(smem + DS_COEF + it % DS_CRING * 128 * 4, a.coef_table + (size_t)h * F_ROWS + d.slab * 128, 128 * 4, &ready[s]);
@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dstate_heads_kernel(const DStat
   }
   fence_before_sync();
   __syncthreads();
+  w.settle();
   if (warp == DS_ISSUER) tmem_dealloc(tmem_base, 256);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }
@@ -591,8 +592,8 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
       const auto fetch_item = [&](int k) {
         const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         if (k >= 2) {
-          w.wait(&a_free[k & 1], ((k >> 1) - 1) & 1, 0x57);
-          if (QUERY) w.wait(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x58);
+          if (!w.met(&a_free[k & 1], ((k >> 1) - 1) & 1, 0x57)) return;
+          if (QUERY && !w.met(&coef_free[k & 1], ((k >> 1) - 1) & 1, 0x58)) return;
         }
         mbar_arrive_expect_tx(&a_full[k & 1], SLAB_U_BYTES);
         bulk_g2s(Aimg + (k & 1) * SLAB_S_BYTES, a.a_image + ((size_t)(it.b * a.H + it.h) * a.NB + it.c) * SLAB_S_BYTES, SLAB_U_BYTES,
@@ -603,7 +604,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
                  &coef_full[k & 1]);
       };
       if (my_items > 0) fetch_item(0);
-      for (int k = 0; k < my_items; ++k) {
+      for (int k = 0; k < my_items && !w.gave_up(); ++k) {
         const FgItem it = fg_item(blockIdx.x + k * gridDim.x, a.H, a.rep, a.NC, a.c0);
         const int unit = (it.b * a.H + it.h) / a.rep;
         const unsigned char* img = reinterpret_cast<const unsigned char*>(a.image) +
@@ -611,7 +612,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
         for (int s = 0; s < F_SLABS; ++s) {
           // the next item's operand and table while there is time: their buffers' last reader was item k-1
           if (s == 2 * F_SLABS / 3 && k + 1 < my_items) fetch_item(k + 1);
-          if (use > 0) w.wait(&done[s4], (use - 1) & 1, 0x59);
+          if (use > 0 && !w.met(&done[s4], (use - 1) & 1, 0x59)) break;
           mbar_arrive_expect_tx(&ready[s4], SLAB_U_BYTES);
           bulk_g2s(Sbuf + s4 * SLAB_S_BYTES, img + (size_t)s * SLAB_S_BYTES, SLAB_U_BYTES, &ready[s4]);
           if (++s4 == FG_RING) { s4 = 0; ++use; }
@@ -622,6 +623,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) feature_grad_kernel(const FeatG
   }
   fence_before_sync();
   __syncthreads();
+  w.settle();
   if (warp == FG_ISSUER) tmem_dealloc(tmem_base, 512);
   if (tid == 0 && dead) atomicOr(a.status, w.status_bits());
 }

@@ -207,6 +207,23 @@ def test_bounded_wait_that_runs_out_reports_a_status_and_leaves_the_context_usab
     assert ERR(out, want) < 1e-5
 
 
+def test_a_kernel_that_gave_up_settles_before_it_leaves():
+    """After the wait (0.1 ms) the kernel pauses for 4 000 000 clocks, at most 2 GHz, so that copies in flight would have landed."""
+    import ctypes
+
+    from oal_b200 import _lib
+
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    begin.record()
+    _lib.check(_lib.load().oal_selftest_wait_timeout(200_000, _lib.ptr(status), stream))
+    end.record()
+    end.synchronize()
+    assert begin.elapsed_time(end) > 1.9
+    assert int(status) == _lib.STATUS_WAIT_TIMEOUT | (0x7E << 8)
+
+
 def test_every_library_call_runs_under_the_tensors_device(monkeypatch):
     """The kernels launch on the current device; the wrapper makes the tensors' device current around
     each call (the reference is plain torch code and follows its tensors)."""
