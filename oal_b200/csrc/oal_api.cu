@@ -519,7 +519,7 @@ int backward_dstate(const OalProblem* p, const void* saved_state, const ChunkRan
   const cudaError_t e = oal::dstate_heads(s.q_image, s.gimg, want_c ? saved_state : nullptr,
                                           want_c ? saved_remainders(p, saved_state) : nullptr, saved_coef_table(p, saved_state),
                                           s.dcarry, want_c ? s.dcoef_partial : nullptr, p->batch, p->q_heads, p->kv_heads,
-                                          p->seq_len, chunk_count(p), cr.first, cr.n, p->scale, status, st);
+                                          chunk_count(p), cr.first, cr.n, p->scale, status, st);
   return e == cudaSuccess ? OAL_OK : fail_cuda(e, "state gradient kernel");
 }
 
@@ -596,7 +596,7 @@ int forward_core(const OalProblem* p, const void* q, const void* k, const void* 
   void* remainders = tc && backward ? saved_remainders(p, saved_state) : nullptr;
   if (walk) {
     LaunchScope scope("state_walk", st, 1, timing);
-    e = oal::state_walk(rows, saved_state, remainders, state_in, units, p->seq_len, nb, cr.trim, status, st);
+    e = oal::state_walk(rows, saved_state, remainders, state_in, units, nb, cr.trim, status, st);
     if (e != cudaSuccess) return fail_cuda(e, "state walk kernel");
   } else if (update) {
     LaunchScope scope("state_update", st, 1, timing);

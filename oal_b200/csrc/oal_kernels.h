@@ -79,7 +79,7 @@ cudaError_t rows_prologue(const RowImages& rows, int units, int N, int NB, const
 // both images of every chunk (trim: but the first), the running state kept on chip; state_walk_pays: faster than state_update
 // and state_scan
 bool state_walk_pays(int units, int NB);
-cudaError_t state_walk(const RowImages& rows, void* image, void* image_lo, const float* state_in, int units, int N, int NB, bool trim,
+cudaError_t state_walk(const RowImages& rows, void* image, void* image_lo, const float* state_in, int units, int NB, bool trim,
                        int32_t* status, cudaStream_t st);
 // image_lo: optional second image holding bf16(state - bf16(state)); trim: see state_scan_kernel
 cudaError_t state_scan(const float* ds, void* image, void* image_lo, const float* state_in, float* state_total,
@@ -92,7 +92,7 @@ cudaError_t cross_read(bool query, const void* x, const void* image, const float
 // ---- tensor-core backward kernels (oal_state_bwd.cu): chunks [c0, c0 + NC) of every sequence ----------
 // carry_img / carry_lo: the saved state image and its remainder image (both or neither)
 cudaError_t dstate_heads(const void* q_image, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
-                         float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, int c0, int NC, float scale,
+                         float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int NB, int c0, int NC, float scale,
                          int32_t* status, cudaStream_t st);
 // query: x_image, a_image = images of q and G; else of k and [v | 1]
 cudaError_t feature_grad(bool query, const void* x_image, const void* a_image, const void* image,

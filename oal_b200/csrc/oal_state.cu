@@ -251,7 +251,7 @@ struct StateWalkArgs {
   const unsigned char *k_image, *u_image;
   unsigned char *image, *image_lo; // [units, NB, 19, 10, 128, 8]: state, and bf16(state - bf16(state)) or null
   const float* state_in;           // [units, F_ROWS, EP] row-major, or null
-  int N, NB;
+  int NB;
   int first_image;                 // 1: nothing reads the image of the first chunk (a zero state)
   int32_t* status;
 };
@@ -660,12 +660,12 @@ cudaError_t rows_prologue(const RowImages& rows, int units, int N, int NB, const
   return cudaGetLastError();
 }
 
-cudaError_t state_walk(const RowImages& rows, void* image, void* image_lo, const float* state_in, int units, int N, int NB, bool trim,
+cudaError_t state_walk(const RowImages& rows, void* image, void* image_lo, const float* state_in, int units, int NB, bool trim,
                        int32_t* status, cudaStream_t st) {
   cudaError_t e = allow_smem<state_walk_kernel>(SW_SMEM);
   if (e != cudaSuccess) return e;
   StateWalkArgs a{static_cast<const unsigned char*>(rows.k_image), static_cast<const unsigned char*>(rows.u_image),
-                  static_cast<unsigned char*>(image), static_cast<unsigned char*>(image_lo), state_in, N, NB, trim ? 1 : 0, status};
+                  static_cast<unsigned char*>(image), static_cast<unsigned char*>(image_lo), state_in, NB, trim ? 1 : 0, status};
   state_walk_kernel<<<F_SLABS * units, SW_THREADS, SW_SMEM, st>>>(a);
   return cudaGetLastError();
 }

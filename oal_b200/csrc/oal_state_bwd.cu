@@ -41,7 +41,7 @@ struct DStateArgs {
   const float* coef_table;         // [Hq, F_ROWS]
   float* dcarry;                   // [units, NB] chunks of F_ROWS x EP floats in state_inc_offset order
   float* dcoef_partial;            // [B, NC, 2 column halves, Hq, F_ROWS] or null
-  int N, NB, Hq, Hkv, units;
+  int NB, Hq, Hkv, units;
   int c0, NC;                      // chunks [c0, c0 + NC) of each sequence (no one reads dCarry of the others)
   float scale;
   int32_t* status;
@@ -795,14 +795,14 @@ __global__ void __launch_bounds__(256) norm_vjp_image_kernel(const void* grad_ou
 }  // namespace
 
 cudaError_t dstate_heads(const void* q_image, const void* gimg, const void* carry_img, const void* carry_lo, const float* coef_table,
-                         float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int N, int NB, int c0, int NC, float scale,
+                         float* dcarry, float* dcoef_partial, int B, int Hq, int Hkv, int NB, int c0, int NC, float scale,
                          int32_t* status, cudaStream_t st) {
   cudaError_t e = allow_smem<dstate_heads_kernel>(DS_SMEM);
   if (e != cudaSuccess) return e;
   const int sms = sm_count(), items = F_SLABS * NC * B * Hkv;
   DStateArgs a{static_cast<const unsigned char*>(q_image), static_cast<const __nv_bfloat16*>(gimg),
                static_cast<const __nv_bfloat16*>(carry_img), static_cast<const __nv_bfloat16*>(carry_lo), coef_table,
-               dcarry, dcoef_partial, N, NB, Hq, Hkv, B * Hkv, c0, NC, scale, status};
+               dcarry, dcoef_partial, NB, Hq, Hkv, B * Hkv, c0, NC, scale, status};
   dstate_heads_kernel<<<items < sms ? items : sms, DS_THREADS, DS_SMEM, st>>>(a);
   return cudaGetLastError();
 }

@@ -176,10 +176,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                : "memory");
 }
 // 4 consecutive 32-bit columns per thread, registers -> TMEM.
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
-               : "memory");
-}
 // 16 lanes x 32 columns (.16x256b.x4): of every 8 columns i a thread holds columns 2 (lane % 4), + 1 of row lane / 4 in
 // r[4 i], r[4 i + 1] and of row lane / 4 + 8 in r[4 i + 2], r[4 i + 3].
 __device__ __forceinline__ void tmem_st_rows16(uint32_t taddr, const uint32_t (&r)[16]) {
