@@ -631,7 +631,7 @@ def run_gpu_arm(args) -> None:
                             note="algorithmic MMA FLOPs of the kernel (unpadded, causal half, chunk 64 as in "
                                  "flop_per_token) / its mean launch time",
                             executed_mma_tflops=tc[top].get("executed_mma_tflops"),
-                            executed_note="MMA FLOPs the kernel really issues (stacked tile, remainder chain, full tiles "
+                            executed_note="MMA FLOPs the kernel really issues (value and remainder chains, full tiles "
                                           "under the causal mask); the achieved figure counts the reference's GEMMs for "
                                           "the same term",
                             frac_of_burst_peak=round(achieved / peaks["tflops_burst"], 4), burst_peak=peaks["tflops_burst"],
